@@ -263,6 +263,29 @@ typedef struct mk_stage_args {
 /* Launch.  Asynchronous on `stream`. */
 int mk_stage_launch(const mk_stage_args* args, void* stream);
 
+/* A prompt through `program`, all positions at once: what `positions` decode steps with given tokens leave in the
+ * states, caches and `pos`, computed as matrix products over batch x positions token rows (tcgen05) instead of step by
+ * step.  The LM head is not run: feed the prompt's last token to mk_stage_launch.  `program` is a HOST copy of the
+ * records.  Programs with two-piece inputs, int8 weights, an fp32 KV cache or all-reduces are MK_ERR_UNSUPPORTED.
+ * The reference takes a prompt in by one `step` per position (qwen3.8-27b-gfx942/mk/reference.py:378-386). */
+typedef struct mk_stage_prefill_args {
+    uint64_t program;        /* host address of mk_stage_desc[n_stages]                             */
+    int32_t n_stages;
+    int32_t batch;           /* M, 1..8                                                            */
+    int32_t positions;       /* L: prompt tokens per sequence                                      */
+    int32_t device;
+    uint64_t tokens;         /* int32[positions][batch] in device memory                           */
+    uint64_t pos;            /* int32[M]: positions of the first token; advanced by `positions`    */
+    uint64_t status;         /* int32[4] as in mk_stage_args                                       */
+    uint64_t workspace;      /* device scratch of mk_stage_prefill_bytes                           */
+    int64_t workspace_bytes;
+    int64_t spin_limit_ns;   /* bound on every device-side wait; 0 = 2 s                           */
+} mk_stage_prefill_args;
+int mk_stage_prefill(const mk_stage_prefill_args* args, void* stream);
+
+/* Bytes of workspace it needs; negative (MK_ERR_UNSUPPORTED) for a program it cannot run. */
+int64_t mk_stage_prefill_bytes(const mk_stage_desc* program, int n_stages, int batch, int positions, int device);
+
 /* Checks a host copy of a program against the kernel's structural limits (ring slot, input staging
  * area, MMA columns, mailbox size) before it is uploaded; MK_ERR_BADARG names the stage. */
 int mk_stage_validate(const mk_stage_desc* program, int n_stages, int batch);

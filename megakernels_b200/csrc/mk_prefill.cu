@@ -1,0 +1,562 @@
+// Prompts through a stage program, all positions at once (declarations: include/mk_stage.h).
+//
+// `mk_stage_prefill` walks the same program the decode kernel runs, but executes every stage for M x L token rows with
+// the kernels of mk_prefill.cuh.  The program's per-step activation buffers ([M][width]) become arrays of M x L rows in
+// the caller's workspace; weights, states and caches are used where they are.  Everything the LM head needs is left to
+// one ordinary decode step with the prompt's last token, so the caller sees exactly what stepping through would leave.
+#include <cstdarg>
+#include <cstdio>
+#include <cstring>
+#include <vector>
+
+#include "../../include/mk_b200.h"
+#include "mk_prefill.cuh"
+
+using namespace mkp;
+
+int mk_set_error(int code, const char* text);
+
+namespace {
+
+int pfail(int code, const char* fmt, ...) {
+    char buf[512];
+    va_list ap;
+    va_start(ap, fmt);
+    vsnprintf(buf, sizeof buf, fmt, ap);
+    va_end(ap);
+    return mk_set_error(code, buf);
+}
+#define MKP_CUDA(call)                                                                      \
+    do {                                                                                    \
+        cudaError_t err__ = (call);                                                         \
+        if (err__ != cudaSuccess)                                                           \
+            return pfail(MK_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(err__));   \
+    } while (0)
+
+constexpr int SMEM_MAX = 232448;
+
+// Hands out the workspace; with base == nullptr it only counts.
+struct Arena {
+    uint8_t* base;
+    size_t off = 0;
+    template <class T>
+    T* take(size_t n) {
+        off = (off + 1023) & ~(size_t)1023;
+        T* p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+        off += n * sizeof(T);
+        return p;
+    }
+};
+
+template <int FMT, int PX>
+int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaStream_t st) {
+    constexpr int PW = FMT == W_FP8_BLOCK ? 2 : 1;
+    const int stage = PW * A_BYTES + PX * A.nt * 128, fixed = (int)sizeof(GemmBars) + 1024;
+    // two CTAs per SM while both keep three stages, else one with as many as fit
+    int stages = (SMEM_MAX / 2 - 1024 - fixed) / stage;
+    if (stages < 3) stages = (SMEM_MAX - fixed) / stage;
+    if (stages > 6) stages = 6;
+    if (stages < 2) return pfail(MK_ERR_BADARG, "prefill: %d tokens per tile leave no room for two stages", A.nt);
+    A.stages = stages;
+    const int smem = stages * stage + fixed;
+    auto fn = out == OUT_STORE ? rows_gemm<FMT, PX, OUT_STORE> : (out == OUT_ADD ? rows_gemm<FMT, PX, OUT_ADD> : rows_gemm<FMT, PX, OUT_GLU>);
+    MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const dim3 grid = items ? dim3(blocks, items, 1) : dim3(tiles_x, blocks, A.ksplit);
+    fn<<<grid, GEMM_THREADS, smem, st>>>(A);
+    MKP_CUDA(cudaGetLastError());
+    if (A.ksplit > 1) {
+        const dim3 fgrid(out == OUT_GLU ? (A.act_cols + 255) / 256 : (A.n_valid + 1023) / 1024, A.rows);
+        if (out == OUT_STORE) rows_finish<PX, OUT_STORE><<<fgrid, 256, 0, st>>>(A);
+        else if (out == OUT_ADD) rows_finish<PX, OUT_ADD><<<fgrid, 256, 0, st>>>(A);
+        else rows_finish<PX, OUT_GLU><<<fgrid, 256, 0, st>>>(A);
+        MKP_CUDA(cudaGetLastError());
+    }
+    return MK_OK;
+}
+
+// Token tiles of `rows` rows: equal tiles of at most 256, multiples of 16.
+void token_tiles(int rows, int* n, int* nt) {
+    *n = (rows + 255) / 256;
+    *nt = ((rows + *n - 1) / *n + 15) / 16 * 16;
+}
+
+// CTAs that share the K range of one tile: the count with the shortest schedule (rounds of one CTA per SM, each 64-column
+// block counted once and the start and end of a CTA as six), at least eight blocks each.
+int pick_ksplit(int ctas, int kbs, int sms) {
+    int best = 1;
+    double cost = 1e30;
+    for (int z = 1; z <= 8 && (z == 1 || kbs / z >= 8); z++) {
+        const double c = (double)((ctas * z + sms - 1) / sms) * ((kbs + z - 1) / z + 6) + (z > 1 ? 4 + z : 0);
+        if (c < cost) {
+            cost = c;
+            best = z;
+        }
+    }
+    return best;
+}
+
+struct Buffer { uint64_t base; int width; float* rows; };
+struct Slab { uint64_t key; const void* norm; float in_scale; uint8_t* x; int rows, width; };
+
+struct Exec {
+    const mk_stage_desc* prog;
+    int n_stages, M, L, rows, xrows, ntiles, nt, sms;
+    const int* tokens;
+    int* pos;
+    int* status;
+    long long spin;
+    cudaStream_t st;
+    bool dry;
+    Arena arena;
+    std::vector<Buffer> bufs;
+    std::vector<Slab> slabs;
+    uint8_t* x_scratch = nullptr;        // slabs made from fp32 rows; reused by every stage that needs new ones
+    Slab x_have = {0, nullptr, 0.f, nullptr, 0, 0};
+    float* part = nullptr;
+    size_t part_floats = 0;
+    // DeltaNet / attention / routing scratch
+    float *qkv = nullptr, *o = nullptr;
+    float4* scal = nullptr;
+    __nv_bfloat16* q = nullptr;
+    RouteArgs route;
+    uint8_t* xg = nullptr;               // gathered slabs
+    int slot_rows = 0, max_items = 0;
+    float *yg = nullptr, *ys = nullptr;
+    uint8_t *act_g = nullptr, *act_s = nullptr;
+
+    Buffer* find(uint64_t p) {
+        for (auto& b : bufs)
+            if (p >= b.base && p < b.base + (uint64_t)b.width * 4) return &b;
+        return nullptr;
+    }
+    // the row array behind a per-step buffer, at the same column offset
+    float* at(uint64_t p) {
+        Buffer* b = find(p);
+        return b ? b->rows + (p - b->base) / 4 : nullptr;
+    }
+    void add(uint64_t p, int width) {
+        if (p && !find(p)) bufs.push_back({p, width, nullptr});
+    }
+    Slab* slab(uint64_t key) {
+        for (auto& s : slabs)
+            if (s.key == key) return &s;
+        return nullptr;
+    }
+    void need_slab(uint64_t key, int width) {
+        Slab* s = slab(key);
+        if (!s) slabs.push_back({key, nullptr, 0.f, nullptr, xrows, width});
+        else if (width > s->width) s->width = width;
+    }
+    void written(uint64_t p) {           // fp32 rows change: slabs made from them are stale
+        if (find(x_have.key) == find(p)) x_have.key = 0;
+    }
+
+    static int format(const mk_stage_desc& d) {
+        switch (d.i[MKS_I_FMT]) {
+            case MKS_FMT_MXFP4: return W_MXFP4;
+            case MKS_FMT_FP8: return d.i[MKS_I_BLOCK_SCALES] ? W_FP8_BLOCK : W_FP8;
+            case MKS_FMT_BF16: return W_BF16;
+            default: return -1;
+        }
+    }
+
+    // What this path cannot do is refused as a whole, and the caller steps through the prompt instead.
+    const char* refuse() const {
+        if (prog[0].op != MKS_OP_EMBED) return "the program does not start with the embedding";
+        for (int s = 0; s < n_stages; s++) {
+            const mk_stage_desc& d = prog[s];
+            if (d.op == MKS_OP_GEMV) {
+                if (d.i[MKS_I_PIECES] != 1) return "two-piece inputs";
+                if (d.i[MKS_I_ALLREDUCE]) return "tensor parallelism";
+                if (format(d) < 0) return "int8 weights";
+                if (d.i[MKS_I_KC] % 64) return "columns per split are not whole 64-column blocks";
+                if (d.i[MKS_I_GROUPS] != 1 && d.i[MKS_I_GROUPS] != -1) return "fixed groups";
+                if (d.i[MKS_I_GROUPS] < 0 && d.i[MKS_I_SPLITS] != 1) return "split experts";
+                if (d.i[MKS_I_FMT] == MKS_FMT_BF16 && d.i[MKS_I_KC] / 16 % 4) return "bf16 blocks";
+                if (d.i[MKS_I_EPILOGUE] != MKS_E_LOGITS && d.i[MKS_I_OUT_STRIDE] % 4) return "unaligned outputs";
+                if (d.i[MKS_I_X_STRIDE] % 4) return "unaligned inputs";
+            } else if (d.op == MKS_OP_ATTN) {
+                if (d.i[MKS_I_KV_F32] || !d.i[MKS_I_Q_BF16]) return "fp32 attention";
+                if (d.i[MKS_I_NQ] / d.i[MKS_I_NKV] > 8) return "query heads per KV head";
+            }
+        }
+        return nullptr;
+    }
+
+    void layout() {
+        for (int s = 0; s < n_stages; s++) {
+            const mk_stage_desc& d = prog[s];
+            if (d.op == MKS_OP_EMBED) add(d.p[MKS_P_H], d.i[MKS_I_HIDDEN]);
+            else if (d.op == MKS_OP_GEMV && d.i[MKS_I_EPILOGUE] != MKS_E_LOGITS && d.i[MKS_I_EPILOGUE] != MKS_E_GLU) add(d.p[MKS_P_OUT], d.i[MKS_I_OUT_STRIDE]);
+            else if (d.op == MKS_OP_VEC && d.i[MKS_I_VEC_N]) add(d.p[MKS_P_VEC_OUT], d.i[MKS_I_VEC_N]);
+        }
+        for (auto& b : bufs) b.rows = arena.take<float>((size_t)rows * b.width);
+        int kmax = 0, experts = 0, topk = 0;
+        size_t conv = 0, heads = 0, vals = 0, q_w = 0, ex_k = 0, ex_n = 0, ex_f = 0, sh = 0;
+        for (int s = 0; s < n_stages; s++) {
+            const mk_stage_desc& d = prog[s];
+            auto up = [](size_t& a, size_t b) { if (b > a) a = b; };
+            if (d.op == MKS_OP_GEMV && d.i[MKS_I_EPILOGUE] != MKS_E_LOGITS) {
+                const int K = d.i[MKS_I_KC] * d.i[MKS_I_SPLITS];
+                const bool routed = d.i[MKS_I_GROUPS] < 0;
+                if (d.i[MKS_I_EPILOGUE] == MKS_E_GLU) {
+                    if (routed) {
+                        up(ex_k, K);
+                        up(ex_f, d.i[MKS_I_N_VALID]);
+                        sh |= d.p[MKS_P_W_SHARED] != 0;
+                    } else need_slab(d.p[MKS_P_OUT], d.i[MKS_I_N_VALID]);
+                }
+                if (routed && d.i[MKS_I_EPILOGUE] != MKS_E_GLU) up(ex_n, d.i[MKS_I_N_VALID]);
+                if (K > kmax) kmax = K;
+                if (!routed) {
+                    const int blocks = (d.i[MKS_I_TILES] + 7) / 8, z = pick_ksplit(blocks * ntiles, K / 64, sms);
+                    if (z > 1) up(part_floats, (size_t)z * rows * (d.i[MKS_I_EPILOGUE] == MKS_E_GLU ? d.i[MKS_I_TILES] * 16 : d.i[MKS_I_N_VALID]));
+                }
+            } else if (d.op == MKS_OP_GDN) {
+                up(conv, d.i[MKS_I_CONV_DIM]);
+                up(heads, d.i[MKS_I_NVH]);
+                need_slab(d.p[MKS_P_Y2], d.i[MKS_I_NVH] * 128);
+            } else if (d.op == MKS_OP_ATTN) {
+                up(q_w, (size_t)d.i[MKS_I_NQ] * d.i[MKS_I_HD]);
+                need_slab(d.p[MKS_P_A_Y2], d.i[MKS_I_NQ] * d.i[MKS_I_HD]);
+            } else if (d.op == MKS_OP_ROUTE) {
+                experts = d.i[MKS_I_EXPERTS];
+                topk = d.i[MKS_I_TOPK];
+            }
+        }
+        for (auto& s : slabs) s.x = arena.take<uint8_t>((size_t)(s.width + 63) / 64 * xrows * 128);
+        vals = heads * 128;
+        x_scratch = arena.take<uint8_t>((size_t)kmax / 64 * xrows * 128);
+        if (part_floats) part = arena.take<float>(part_floats);
+        if (conv) {
+            qkv = arena.take<float>((size_t)rows * conv);
+            scal = arena.take<float4>((size_t)rows * heads);
+            o = arena.take<float>((size_t)rows * vals);
+        }
+        if (q_w) q = arena.take<__nv_bfloat16>((size_t)rows * q_w);
+        if (experts) {
+            // tile width of the routed products: about twice the mean load, so that most experts are one tile
+            const int mean = (int)((long long)rows * topk / experts);
+            memset(&route, 0, sizeof route);
+            route.nt = mean > 96 ? 256 : (mean > 40 ? 128 : (mean > 16 ? 64 : 32));
+            slot_rows = (rows * topk + experts * 15 + route.nt + 15) / 16 * 16;
+            max_items = experts + rows * topk / route.nt + 1;
+            if (max_items > rows * topk) max_items = rows * topk;
+            route.items = arena.take<int4>(max_items);
+            route.counts = arena.take<int>(3 * experts + 1);
+            route.n_items = route.counts ? route.counts + 3 * experts : nullptr;
+            route.slot = arena.take<int>((size_t)rows * 8);
+            route.weight = arena.take<float>((size_t)rows * 8);
+            route.gate = arena.take<float>(rows);
+            xg = arena.take<uint8_t>(ex_k / 64 * slot_rows * 128);
+            act_g = arena.take<uint8_t>((ex_f + 63) / 64 * slot_rows * 128);
+            yg = arena.take<float>((size_t)slot_rows * ex_n);
+            if (sh) {
+                act_s = arena.take<uint8_t>((ex_f + 63) / 64 * xrows * 128);
+                ys = arena.take<float>((size_t)rows * ex_n);
+            }
+        }
+    }
+
+    int gemm(const mk_stage_desc& d, GemmArgs& A, int out, int items) {
+        const int blocks = (d.i[MKS_I_TILES] + 7) / 8;
+        switch (format(d)) {
+            case W_MXFP4: return launch_gemm<W_MXFP4, 1>(A, out, blocks, ntiles, items, st);
+            case W_FP8: return launch_gemm<W_FP8, 1>(A, out, blocks, ntiles, items, st);
+            case W_FP8_BLOCK: return launch_gemm<W_FP8_BLOCK, 1>(A, out, blocks, ntiles, items, st);
+            default: return launch_gemm<W_BF16, 1>(A, out, blocks, ntiles, items, st);
+        }
+    }
+    GemmArgs args(const mk_stage_desc& d) {
+        GemmArgs A;
+        memset(&A, 0, sizeof A);
+        A.w = reinterpret_cast<const uint8_t*>(d.p[MKS_P_W]);
+        A.tiles = d.i[MKS_I_TILES];
+        A.unit_steps = d.i[MKS_I_UNIT_STEPS];
+        A.chunk_steps = d.i[MKS_I_CHUNK_STEPS];
+        A.chunk_bytes = d.i[MKS_I_CHUNK_BYTES];
+        A.kc = d.i[MKS_I_KC];
+        A.row_scale = reinterpret_cast<const float*>(d.p[MKS_P_ROW_SCALE]);
+        A.kbs = d.i[MKS_I_KC] * d.i[MKS_I_SPLITS] / 64;
+        A.ksplit = 1;
+        A.rows = rows;
+        A.nt = nt;
+        A.gelu = d.i[MKS_I_ACT] == MKS_ACT_GELU_TANH;
+        A.n_valid = d.i[MKS_I_EPILOGUE] == MKS_E_GLU ? d.i[MKS_I_TILES] * 16 : d.i[MKS_I_N_VALID];
+        A.act_cols = d.i[MKS_I_N_VALID];
+        A.status = status;
+        A.spin_limit_ns = spin;
+        return A;
+    }
+
+    // The token operand of a stage: what its producer left as slabs, or its fp32 rows brought into that form.
+    int operand(const mk_stage_desc& d, const uint8_t** x, int* x_rows) {
+        if (Slab* s = slab(d.p[MKS_P_X])) {
+            *x = s->x;
+            *x_rows = s->rows;
+            return MK_OK;
+        }
+        const bool norm = d.i[MKS_I_PROLOGUE] == MKS_P_NORM;
+        const void* nw = norm ? reinterpret_cast<const void*>(d.p[MKS_P_NORM_W]) : nullptr;
+        const float in_scale = d.f[MKS_F_IN_SCALE] != 0.f ? d.f[MKS_F_IN_SCALE] : 1.f;
+        if (x_have.key != d.p[MKS_P_X] || x_have.norm != nw || x_have.in_scale != in_scale) {
+            const float* src = at(d.p[MKS_P_X]);
+            if (!src) return pfail(MK_ERR_BADARG, "prefill: a stage reads a buffer no earlier stage writes");
+            rows_in<1><<<rows, 256, 0, st>>>(src, d.i[MKS_I_X_STRIDE], d.i[MKS_I_KC] * d.i[MKS_I_SPLITS], reinterpret_cast<const float*>(nw), d.f[MKS_F_NORM_OFF],
+                                             d.f[MKS_F_EPS], in_scale, x_scratch, 0, xrows);
+            MKP_CUDA(cudaGetLastError());
+            x_have = {d.p[MKS_P_X], nw, in_scale, x_scratch, xrows, 0};
+        }
+        *x = x_scratch;
+        *x_rows = xrows;
+        return MK_OK;
+    }
+
+    int dense(const mk_stage_desc& d) {
+        GemmArgs A = args(d);
+        int rc = operand(d, &A.x, &A.x_rows);
+        if (rc != MK_OK) return rc;
+        A.ksplit = pick_ksplit((d.i[MKS_I_TILES] + 7) / 8 * ntiles, A.kbs, sms);
+        A.part = part;
+        A.part_rows = rows;
+        int out;
+        if (d.i[MKS_I_EPILOGUE] == MKS_E_GLU) {
+            out = OUT_GLU;
+            Slab* s = slab(d.p[MKS_P_OUT]);
+            A.act = s->x;
+            A.act_rows = s->rows;
+        } else {
+            out = d.i[MKS_I_EPILOGUE] == MKS_E_RESID ? OUT_ADD : OUT_STORE;
+            A.out = at(d.p[MKS_P_OUT]);
+            A.out_stride = d.i[MKS_I_OUT_STRIDE];
+            written(d.p[MKS_P_OUT]);
+        }
+        return gemm(d, A, out, 0);
+    }
+
+    int routed(const mk_stage_desc& d) {
+        const bool shared = d.p[MKS_P_W_SHARED] != 0, up = d.i[MKS_I_EPILOGUE] == MKS_E_GLU;
+        GemmArgs A = args(d);
+        int rc;
+        if (up) {
+            rc = operand(d, &A.x, &A.x_rows);
+            if (rc != MK_OK) return rc;
+            if (shared) {                // the shared expert: a dense product on the rows as they are
+                GemmArgs S = A;
+                S.w = reinterpret_cast<const uint8_t*>(d.p[MKS_P_W_SHARED]);
+                S.row_scale = reinterpret_cast<const float*>(d.p[MKS_P_RS_SHARED]);
+                S.act = act_s;
+                S.act_rows = xrows;
+                rc = gemm(d, S, OUT_GLU, 0);
+                if (rc != MK_OK) return rc;
+            }
+            gather_rows<<<rows, 256, 0, st>>>(A.x, A.x_rows, route.slot, route.topk, A.kbs, xg, slot_rows);
+            MKP_CUDA(cudaGetLastError());
+            A.x = xg;
+            A.act = act_g;
+            A.act_rows = slot_rows;
+        } else {
+            if (shared) {
+                GemmArgs S = A;
+                S.w = reinterpret_cast<const uint8_t*>(d.p[MKS_P_W_SHARED]);
+                S.row_scale = reinterpret_cast<const float*>(d.p[MKS_P_RS_SHARED]);
+                S.x = act_s;
+                S.x_rows = xrows;
+                S.out = ys;
+                S.out_stride = d.i[MKS_I_N_VALID];
+                rc = gemm(d, S, OUT_STORE, 0);
+                if (rc != MK_OK) return rc;
+            }
+            A.x = act_g;
+            A.out = yg;
+            A.out_stride = d.i[MKS_I_N_VALID];
+        }
+        A.x_rows = slot_rows;
+        A.w_gstride = d.p[MKS_P_W_GSTRIDE];
+        A.rs_gstride = d.p[MKS_P_RS_GSTRIDE];
+        A.nt = route.nt;
+        A.items = route.items;
+        A.n_items = route.n_items;
+        rc = gemm(d, A, up ? OUT_GLU : OUT_STORE, max_items);
+        if (rc != MK_OK || up) return rc;
+        combine_rows<<<rows, 256, 0, st>>>(yg, d.i[MKS_I_N_VALID], route.slot, route.weight, route.topk, shared ? ys : nullptr, route.gate,
+                                           d.i[MKS_I_EPILOGUE] == MKS_E_RESID, at(d.p[MKS_P_OUT]), d.i[MKS_I_OUT_STRIDE]);
+        MKP_CUDA(cudaGetLastError());
+        written(d.p[MKS_P_OUT]);
+        return MK_OK;
+    }
+
+    int gdn(const mk_stage_desc& d) {
+        GdnArgs G;
+        memset(&G, 0, sizeof G);
+        G.y = at(d.p[MKS_P_Y]);
+        if (!G.y) return pfail(MK_ERR_BADARG, "prefill: the DeltaNet stage reads a buffer no earlier stage writes");
+        G.y_stride = d.i[MKS_I_Y_STRIDE];
+        G.M = M; G.L = L;
+        G.nkh = d.i[MKS_I_NKH]; G.nvh = d.i[MKS_I_NVH]; G.conv_dim = d.i[MKS_I_CONV_DIM];
+        G.q_off = d.i[MKS_I_Q_OFF]; G.k_off = d.i[MKS_I_K_OFF]; G.v_off = d.i[MKS_I_V_OFF]; G.z_off = d.i[MKS_I_Z_OFF];
+        G.b_off = d.i[MKS_I_B_OFF]; G.a_off = d.i[MKS_I_A_OFF];
+        G.conv_w = reinterpret_cast<const float*>(d.p[MKS_P_CONV_W]);
+        G.A_log = reinterpret_cast<const float*>(d.p[MKS_P_A_LOG]);
+        G.dt_bias = reinterpret_cast<const float*>(d.p[MKS_P_DT_BIAS]);
+        G.norm_w = reinterpret_cast<const float*>(d.p[MKS_P_GDN_NORM]);
+        G.conv_state = reinterpret_cast<float*>(d.p[MKS_P_CONV_STATE]);
+        G.ring = 4;
+        G.ssm = reinterpret_cast<float*>(d.p[MKS_P_SSM_STATE]);
+        G.pos = pos;
+        G.conv_bf16 = d.i[MKS_I_CONV_BF16];
+        G.l2_clamp = d.i[MKS_I_L2_CLAMP];
+        G.eps = d.f[MKS_F_EPS];
+        G.qkv = qkv; G.scal = scal; G.o = o;
+        Slab* s = slab(d.p[MKS_P_Y2]);
+        G.out = s->x;
+        G.out_rows = s->rows;
+        gdn_conv<<<dim3((G.conv_dim / 128 + 7) / 8, rows), 256, 0, st>>>(G);
+        gdn_history<<<dim3((G.conv_dim + 255) / 256, M), 256, 0, st>>>(G);
+        gdn_scan<<<dim3(4, G.nvh, M), 256, 0, st>>>(G);
+        gdn_gate<1><<<dim3((G.nvh + 15) / 16, rows), 256, 0, st>>>(G);
+        MKP_CUDA(cudaGetLastError());
+        return MK_OK;
+    }
+
+    template <int HD>
+    int attn_hd(const AttnArgs& T) {
+        const int bq = AT_ROWS / (T.nq / T.nkv);
+        attn_prepare<HD><<<dim3((T.nq + 2 * T.nkv + 7) / 8, rows), 256, 0, st>>>(T);
+        MKP_CUDA(cudaFuncSetAttribute(attn_rows<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem<HD>()));
+        attn_rows<HD><<<dim3((L + bq - 1) / bq, T.nkv, M), 256, attn_smem<HD>(), st>>>(T);
+        MKP_CUDA(cudaGetLastError());
+        return MK_OK;
+    }
+    int attn(const mk_stage_desc& d) {
+        AttnArgs T;
+        memset(&T, 0, sizeof T);
+        const int HD = d.i[MKS_I_HD];
+        T.y = at(d.p[MKS_P_A_Y]);
+        if (!T.y) return pfail(MK_ERR_BADARG, "prefill: the attention stage reads a buffer no earlier stage writes");
+        T.y_stride = d.i[MKS_I_A_Y_STRIDE];
+        T.M = M; T.L = L; T.nq = d.i[MKS_I_NQ]; T.nkv = d.i[MKS_I_NKV];
+        T.q_off = d.i[MKS_I_A_Q_OFF]; T.q_hs = d.i[MKS_I_A_Q_HSTRIDE]; T.gate_off = d.i[MKS_I_A_GATE_OFF];
+        T.k_off = d.i[MKS_I_A_K_OFF]; T.v_off = d.i[MKS_I_A_V_OFF];
+        T.rot = d.i[MKS_I_ROT]; T.pairs = d.i[MKS_I_ROPE_PAIRS]; T.window = d.i[MKS_I_WINDOW];
+        T.norm_plain = d.i[MKS_I_NORM_PLAIN]; T.v_norm = d.i[MKS_I_V_NORM];
+        T.eps = d.f[MKS_F_EPS]; T.scale = d.f[MKS_F_SCALE];
+        T.q_norm = reinterpret_cast<const float*>(d.p[MKS_P_Q_NORM]);
+        T.k_norm = reinterpret_cast<const float*>(d.p[MKS_P_K_NORM]);
+        T.cos = reinterpret_cast<const float*>(d.p[MKS_P_ROPE_COS]);
+        T.sin = reinterpret_cast<const float*>(d.p[MKS_P_ROPE_SIN]);
+        T.k_cache = reinterpret_cast<void*>(d.p[MKS_P_K_CACHE]);
+        T.v_cache = reinterpret_cast<void*>(d.p[MKS_P_V_CACHE]);
+        T.bt = reinterpret_cast<const int*>(d.p[MKS_P_BLOCK_TABLE]);
+        T.max_pages = d.i[MKS_I_MAX_PAGES];
+        const int kvb = d.i[MKS_I_KV_BLOCK] > 0 ? d.i[MKS_I_KV_BLOCK] : 64;
+        T.kv_shift = 31 - __builtin_clz(kvb);
+        const bool own = d.i[MKS_I_KV_S_PAGE] == 0;
+        T.s_page = own ? (uint32_t)(T.nkv * kvb * HD) : (uint32_t)d.i[MKS_I_KV_S_PAGE];
+        T.s_head = own ? (uint32_t)(kvb * HD) : (uint32_t)d.i[MKS_I_KV_S_HEAD];
+        T.s_pos = own ? (uint32_t)HD : (uint32_t)d.i[MKS_I_KV_S_POS];
+        T.pos = pos;
+        T.q = q;
+        Slab* s = slab(d.p[MKS_P_A_Y2]);
+        T.out = s->x;
+        T.out_rows = s->rows;
+        return HD == 512 ? attn_hd<512>(T) : attn_hd<256>(T);
+    }
+
+    int routing(const mk_stage_desc& d) {
+        route.logits = at(d.p[MKS_P_LOGITS]);
+        if (!route.logits) return pfail(MK_ERR_BADARG, "prefill: the routing stage reads a buffer no earlier stage writes");
+        route.rows = rows;
+        route.stride = d.i[MKS_I_LOGIT_STRIDE];
+        route.experts = d.i[MKS_I_EXPERTS];
+        route.topk = d.i[MKS_I_TOPK];
+        route.kind = d.i[MKS_I_ROUTE_KIND];
+        route.expert_scale = reinterpret_cast<const float*>(d.p[MKS_P_EXPERT_SCALE]);
+        MKP_CUDA(cudaMemsetAsync(route.counts, 0, (3 * route.experts + 1) * sizeof(int), st));
+        route_rows<<<(rows + 7) / 8, 256, 0, st>>>(route);
+        route_plan<<<1, 256, 0, st>>>(route);
+        route_slots<<<(rows * 8 + 255) / 256, 256, 0, st>>>(route);
+        MKP_CUDA(cudaGetLastError());
+        return MK_OK;
+    }
+
+    int vec(const mk_stage_desc& d) {
+        if (!d.i[MKS_I_VEC_N]) return MK_OK;
+        vec_rows<<<rows, 256, 0, st>>>(d.i[MKS_I_VEC_N], at(d.p[MKS_P_VEC_BASE]), at(d.p[MKS_P_VEC_A]), reinterpret_cast<const float*>(d.p[MKS_P_VEC_A_W]),
+                                       at(d.p[MKS_P_VEC_B]), reinterpret_cast<const float*>(d.p[MKS_P_VEC_B_W]), d.f[MKS_F_NORM_OFF], d.f[MKS_F_EPS],
+                                       d.f[MKS_F_SCALE] != 0.f ? d.f[MKS_F_SCALE] : 1.f, at(d.p[MKS_P_VEC_OUT]));
+        MKP_CUDA(cudaGetLastError());
+        written(d.p[MKS_P_VEC_OUT]);
+        return MK_OK;
+    }
+
+    int run() {
+        for (int s = 0; s < n_stages; s++) {
+            const mk_stage_desc& d = prog[s];
+            int rc = MK_OK;
+            switch (d.op) {
+                case MKS_OP_EMBED:
+                    embed_rows<<<rows, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(d.p[MKS_P_TABLE]), tokens, M, L, d.i[MKS_I_HIDDEN], d.i[MKS_I_VOCAB],
+                                                     d.f[MKS_F_SCALE], at(d.p[MKS_P_H]));
+                    MKP_CUDA(cudaGetLastError());
+                    written(d.p[MKS_P_H]);
+                    break;
+                case MKS_OP_GEMV:
+                    if (d.i[MKS_I_EPILOGUE] == MKS_E_LOGITS) break;            // the last token's step computes logits
+                    rc = d.i[MKS_I_GROUPS] < 0 ? routed(d) : dense(d);
+                    break;
+                case MKS_OP_GDN: rc = gdn(d); break;
+                case MKS_OP_ATTN: rc = attn(d); break;
+                case MKS_OP_ROUTE: rc = routing(d); break;
+                case MKS_OP_VEC: rc = vec(d); break;
+                default: return pfail(MK_ERR_BADARG, "prefill: unknown op %d", d.op);
+            }
+            if (rc != MK_OK) return rc;
+        }
+        advance_pos<<<1, 32, 0, st>>>(pos, M, L);
+        MKP_CUDA(cudaGetLastError());
+        return MK_OK;
+    }
+};
+
+int prepare(Exec& E, const mk_stage_desc* prog, int n_stages, int batch, int positions, int device, void* workspace) {
+    E.prog = prog;
+    E.n_stages = n_stages;
+    E.M = batch;
+    E.L = positions;
+    E.rows = batch * positions;
+    token_tiles(E.rows, &E.ntiles, &E.nt);
+    E.xrows = E.ntiles * E.nt;
+    if (cudaDeviceGetAttribute(&E.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return pfail(MK_ERR_CUDA, "prefill: no device %d", device);
+    E.arena.base = static_cast<uint8_t*>(workspace);
+    if (const char* why = E.refuse()) return pfail(MK_ERR_UNSUPPORTED, "prefill: %s", why);
+    E.layout();
+    return MK_OK;
+}
+
+}  // namespace
+
+extern "C" int64_t mk_stage_prefill_bytes(const mk_stage_desc* program, int n_stages, int batch, int positions, int device) {
+    if (!program || n_stages < 1 || batch < 1 || batch > MKS_MAX_BATCH || positions < 1) return pfail(MK_ERR_BADARG, "mk_stage_prefill_bytes: bad argument");
+    Exec E;
+    const int rc = prepare(E, program, n_stages, batch, positions, device, nullptr);
+    return rc == MK_OK ? (int64_t)E.arena.off + 1024 : rc;
+}
+
+extern "C" int mk_stage_prefill(const mk_stage_prefill_args* a, void* stream) {
+    if (!a || !a->program || a->n_stages < 1) return pfail(MK_ERR_BADARG, "mk_stage_prefill: no program");
+    if (a->batch < 1 || a->batch > MKS_MAX_BATCH || a->positions < 1) return pfail(MK_ERR_BADARG, "mk_stage_prefill: batch %d, positions %d", a->batch, a->positions);
+    if (!a->tokens || !a->pos || !a->status || !a->workspace) return pfail(MK_ERR_BADARG, "mk_stage_prefill: tokens / pos / status / workspace missing");
+    MKP_CUDA(cudaSetDevice(a->device));
+    Exec E;
+    uint8_t* ws = reinterpret_cast<uint8_t*>((a->workspace + 1023) & ~(uint64_t)1023);
+    const int rc = prepare(E, reinterpret_cast<const mk_stage_desc*>(a->program), a->n_stages, a->batch, a->positions, a->device, ws);
+    if (rc != MK_OK) return rc;
+    if ((int64_t)E.arena.off + 1024 > a->workspace_bytes) return pfail(MK_ERR_BADARG, "mk_stage_prefill: workspace of %lld bytes, %lld needed", (long long)a->workspace_bytes, (long long)E.arena.off + 1024);
+    E.tokens = reinterpret_cast<const int*>(a->tokens);
+    E.pos = reinterpret_cast<int*>(a->pos);
+    E.status = reinterpret_cast<int*>(a->status);
+    E.spin = a->spin_limit_ns > 0 ? a->spin_limit_ns : 2000000000ll;
+    E.st = static_cast<cudaStream_t>(stream);
+    return E.run();
+}

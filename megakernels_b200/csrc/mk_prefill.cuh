@@ -1,0 +1,1209 @@
+// Token-parallel kernels of the prompt path (mk_prefill.cu): what a decode program does for the eight columns of
+// one step, done for all positions of a prompt at once.
+//
+// The contractions are matrix products here, so they run on the 5th-generation tensor cores: `rows_gemm` keeps 128
+// weight rows as the A operand of tcgen05.mma and up to 256 token rows as its N columns, accumulators in tensor
+// memory.  The weights stay in the decode kernel's packed tiles: eight warps read a tile step each with one 128-bit
+// load per lane, convert it to bf16 (exact for every format) and write the swizzled operand into shared memory, so
+// a prompt reads the same bytes from HBM as a decode step does and no second copy of the model exists.
+//
+// Operand layout in global memory ("slabs"): a matrix of R token rows and K columns is stored as K / 64 slabs of R
+// rows x 128 bytes, the 16-byte pieces of a row swizzled with its number (piece p of row r sits at p ^ (r & 7)).
+// Any run of rows that starts at a multiple of eight is then one contiguous, ready-to-use K-major SWIZZLE_128B tile:
+// the producer brings it with one untiled bulk copy, and no tensor map is needed.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "../../include/mk_stage.h"
+#include "mk_device.cuh"
+
+namespace mkp {
+using mk::bf_hi;
+using mk::bf_lo;
+using mk::mbar_arrive;
+using mk::mbar_expect_tx;
+using mk::mbar_init;
+using mk::mbar_try_wait;
+using mk::sigmoid_f;
+using mk::silu_f;
+using mk::smem_u32;
+using mk::softplus_f;
+using mk::u64;
+using mk::warp_max;
+using mk::warp_sum;
+
+constexpr int ERR_TIMEOUT = -2;
+enum { WP_EMPTY = 301, WP_FULL, WP_DONE, WP_DRAIN };
+
+// Byte offset of column `c` of row `row` inside a slab array with `rows` rows per slab (bf16 elements).
+__host__ __device__ __forceinline__ size_t slab_offset(int rows, int row, int c) {
+    return ((size_t)(c >> 6) * rows + row) * 128 + (size_t)((((c >> 3) & 7) ^ (row & 7)) << 4) + (size_t)(c & 7) * 2;
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+// Eight consecutive columns c .. c + 7 of a row into PIECES slabs (piece i + 1 is what the pieces before it lost).
+template <int PIECES>
+__device__ __forceinline__ void store_slab8(uint8_t* x, size_t piece_stride, int rows, int row, int c, float (&v)[8]) {
+    uint8_t* dst = x + slab_offset(rows, row, c);
+#pragma unroll
+    for (int p = 0; p < PIECES; p++) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            w[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+            if (p + 1 < PIECES) {
+                v[2 * i] -= bf_lo(w[i]);
+                v[2 * i + 1] -= bf_hi(w[i]);
+            }
+        }
+        *reinterpret_cast<uint4*>(dst + (size_t)p * piece_stride) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// ---- matrix product ----------------------------------------------------------------------------------------
+enum { W_MXFP4 = 0, W_FP8, W_FP8_BLOCK, W_BF16, W_SLAB };      // how the weights come: packed tiles of a format, or bf16 slabs
+enum { OUT_STORE = 0, OUT_ADD, OUT_GLU };
+
+struct GemmArgs {
+    // weights: [group][split][tile][chunk] blocks (stage/pack.py), or slabs
+    const uint8_t* w;
+    size_t w_gstride;            // bytes between groups
+    int tiles, unit_steps, chunk_steps, chunk_bytes, kc;
+    int w_rows;                  // W_SLAB: rows per slab
+    const float* row_scale;      // per weight row, or null
+    size_t rs_gstride;
+    // token operand
+    const uint8_t* x;
+    size_t x_piece;              // bytes between its pieces
+    int x_rows;                  // rows per slab
+    // output
+    float* out;
+    long long out_stride;        // floats between token rows
+    uint8_t* act;                // OUT_GLU: slab array of the activations
+    size_t act_piece;
+    int act_rows, act_cols;      // activation columns (n_valid pairs)
+    int n_valid;                 // weight rows that exist
+    int rows;                    // token rows that exist (dense)
+    int nt;                      // tokens per tile (a multiple of 16, <= 256)
+    int kbs;                     // 64-column blocks of K
+    int ksplit;                  // CTAs that share K; > 1: fp32 partials [split][part_rows][n_valid] in `part`
+    float* part;
+    int part_rows;
+    int gelu;
+    // routed groups: items[i] = {group, first row, rows, 0}, n_items on the device
+    const int4* items;
+    const int* n_items;
+    int stages;
+    int* status;
+    long long spin_limit_ns;
+};
+
+constexpr int CONV_WARPS = 8, GEMM_THREADS = (CONV_WARPS + 2) * 32;
+constexpr int A_BYTES = 128 * 128;                     // one 64-column block of 128 weight rows
+constexpr int MAX_STAGES = 8;
+struct GemmBars {
+    uint64_t full[MAX_STAGES], empty[MAX_STAGES], done;
+    uint32_t tmem;
+    volatile int dead;
+};
+
+__device__ __noinline__ bool wait_slow(GemmBars& B, const GemmArgs& A, uint64_t* b, uint32_t parity, int site) {
+    u64 t0 = 0;
+#pragma unroll 1
+    for (unsigned it = 0;; it++) {
+        if (mbar_try_wait(b, parity)) return true;
+        if ((it & 63u) == 63u) {
+            if (B.dead) return false;
+            const u64 now = mk::globaltimer();
+            if (!t0) t0 = now;
+            else if (now - t0 > (u64)A.spin_limit_ns) {
+                B.dead = 1;
+                if (atomicCAS(A.status, 0, ERR_TIMEOUT) == 0) {
+                    A.status[1] = site;
+                    A.status[2] = (int)blockIdx.x;
+                    A.status[3] = (int)threadIdx.x;
+                }
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ bool wait(GemmBars& B, const GemmArgs& A, uint64_t* b, uint32_t parity, int site) {
+    return mbar_try_wait(b, parity) || wait_slow(B, A, b, parity, site);
+}
+
+// K-major SWIZZLE_128B operand: rows of 128 bytes, eight-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t operand_desc(uint32_t saddr) {
+    return (uint64_t)((saddr >> 4) & 0x3FFF) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t e2m1x2_f16(uint32_t b) {
+    uint32_t r;
+    asm("{\n .reg .b8 t;\n .reg .b16 h;\n cvt.u16.u32 h, %1;\n cvt.u8.u16 t, h;\n cvt.rn.f16x2.e2m1x2 %0, t;\n}\n" : "=r"(r) : "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t e4m3x2_f16(uint32_t b) {
+    uint32_t r;
+    asm("{\n .reg .b16 h;\n cvt.u16.u32 h, %1;\n cvt.rn.f16x2.e4m3x2 %0, h;\n}\n" : "=r"(r) : "r"(b));
+    return r;
+}
+// The bits of a half moved to the bf16 fields: the value times 2^-112 (halves of at most 7 mantissa bits, no subnormals).
+__device__ __forceinline__ uint32_t f16_as_bf16(uint32_t h) { return (h & 0x80008000u) | ((h >> 3) & 0x0FFF0FFFu); }
+
+// Raw bytes of one 64-column block of a 16-row tile, as lane (g, q) holds them.
+template <int FMT> struct Raw { uint4 q[FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2)]; uint32_t s[FMT == W_FP8_BLOCK ? 2 : 1]; };
+
+// Walks the 64-column blocks of one tile through its units.
+template <int FMT>
+struct Walk {
+    static constexpr int STEPS = FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2);      // 512-byte steps per 64 columns
+    const uint8_t* p;          // the current chunk
+    int within, st;            // step inside the chunk, step inside the unit
+    __device__ __forceinline__ void start(const GemmArgs& A, const uint8_t* w, int tile, int kb) {
+        constexpr int STEP_K = 64 / STEPS;
+        const int split = kb * 64 / A.kc;
+        st = (kb * 64 - split * A.kc) / STEP_K;
+        const size_t unit = (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
+        within = st % A.chunk_steps;
+        p = w + ((size_t)split * A.tiles + tile) * unit + (size_t)(st / A.chunk_steps) * A.chunk_bytes;
+    }
+    __device__ __forceinline__ void load(const GemmArgs& A, int lane, Raw<FMT>& r) {
+        if (FMT == W_MXFP4) r.s[0] = __ldg(reinterpret_cast<const uint32_t*>(p + A.chunk_steps * 512 + within * 32 + (lane >> 2) * 4));
+        if (FMT == W_FP8_BLOCK) {
+            const uint2 s = __ldg(reinterpret_cast<const uint2*>(p + A.chunk_steps * 512 + (within >> 2) * 8));
+            r.s[0] = s.x;
+            r.s[FMT == W_FP8_BLOCK ? 1 : 0] = s.y;
+        }
+#pragma unroll
+        for (int i = 0; i < STEPS; i++) {
+            r.q[i] = __ldg(reinterpret_cast<const uint4*>(p + within * 512) + lane);
+            st++;
+            if (++within == A.chunk_steps) {
+                within = 0;
+                p += A.chunk_bytes;
+            }
+        }
+        if (st == A.unit_steps) {          // the same tile of the next split
+            st = 0;
+            p += (size_t)(A.tiles - 1) * (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
+        }
+    }
+};
+
+// One lane's share of a block as bf16: v[row half][j] holds columns 16 j + 4 q + {0 .. 3}; for block-scaled weights
+// `lo` takes what the product of a value (4 bits) and its bf16 scale (8 bits) keeps behind the first eight bits, so that
+// the two pieces together are exact.
+template <int FMT>
+__device__ __forceinline__ void convert(const Raw<FMT>& r, uint2 (&v)[2][4], uint2 (&lo)[2][4]) {
+    if constexpr (FMT == W_BF16) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            v[0][j] = make_uint2(r.q[j].x, r.q[j].y);
+            v[1][j] = make_uint2(r.q[j].z, r.q[j].w);
+        }
+    } else if constexpr (FMT == W_MXFP4) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            // scale group 0 (j = 0, 1): bits pre-arranged by the packer; three magnitude bits at 8..6 of a half are the
+            // value times 2^-126.  Group 1 (j = 2, 3): plain nibbles, through f16: the value times 2^-112.
+            const uint32_t w = h == 0 ? r.q[0].x : r.q[0].z, n = h == 0 ? r.q[0].y : r.q[0].w;
+            const uint32_t s0 = (r.s[0] >> (16 * h)) & 0xFFu, s1 = (r.s[0] >> (16 * h + 8)) & 0xFFu;
+            const uint32_t f0 = (min(s0, 128u) + 126u) << 7, f1 = (min(s1, 142u) + 112u) << 7;     // 2^(s - 1), 2^(s - 15)
+            const uint32_t m0 = f0 | (f0 << 16), m1 = f1 | (f1 << 16);
+            v[h][0].x = mul_bf16x2((w & 0x80008000u) | ((w >> 3) & 0x01C001C0u), m0);
+            v[h][0].y = mul_bf16x2(((w << 3) & 0x80008000u) | (w & 0x01C001C0u), m0);
+            v[h][1].x = mul_bf16x2(((w << 1) & 0x80008000u) | ((w << 3) & 0x01C001C0u), m0);
+            v[h][1].y = mul_bf16x2(((w << 2) & 0x80008000u) | ((w << 6) & 0x01C001C0u), m0);
+            v[h][2].x = mul_bf16x2(f16_as_bf16(e2m1x2_f16(n)), m1);
+            v[h][2].y = mul_bf16x2(f16_as_bf16(e2m1x2_f16(n >> 8)), m1);
+            v[h][3].x = mul_bf16x2(f16_as_bf16(e2m1x2_f16(n >> 16)), m1);
+            v[h][3].y = mul_bf16x2(f16_as_bf16(e2m1x2_f16(n >> 24)), m1);
+            if (s0 > 128u || s1 > 142u) {          // weights beyond +-12: the factors above would leave the range of a bf16
+                const uint32_t g0 = (127u + (s0 > 128u ? s0 - 128u : 0u)) << 7, g1 = (127u + (s1 > 142u ? s1 - 142u : 0u)) << 7;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const uint32_t m = j < 2 ? (g0 | (g0 << 16)) : (g1 | (g1 << 16));
+                    v[h][j].x = mul_bf16x2(v[h][j].x, m);
+                    v[h][j].y = mul_bf16x2(v[h][j].y, m);
+                }
+            }
+        }
+    } else {
+        constexpr uint32_t UP = 0x77807780u;       // 2^112
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const uint32_t w[4] = {r.q[i].x, r.q[i].y, r.q[i].z, r.q[i].w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int h = k >> 1, j = 2 * i + (k & 1);
+                v[h][j].x = mul_bf16x2(f16_as_bf16(e4m3x2_f16(w[k])), UP);
+                v[h][j].y = mul_bf16x2(f16_as_bf16(e4m3x2_f16(w[k] >> 16)), UP);
+                if constexpr (FMT == W_FP8_BLOCK) {
+                    const uint32_t s = r.s[h] >> 16, ss = s | (s << 16), neg = 0xBF80BF80u;
+                    const uint2 e = v[h][j];
+                    v[h][j].x = mul_bf16x2(e.x, ss);
+                    v[h][j].y = mul_bf16x2(e.y, ss);
+                    lo[h][j].x = fma_bf16x2(e.x, ss, mul_bf16x2(v[h][j].x, neg));
+                    lo[h][j].y = fma_bf16x2(e.y, ss, mul_bf16x2(v[h][j].y, neg));
+                }
+            }
+        }
+    }
+}
+
+// Writes a lane's share of tile `tile` into the swizzled operand.  Lanes of odd rows store their columns in the order
+// j = 2, 3, 0, 1: the sixteen 8-byte stores of a half warp then fall into different banks.
+__device__ __forceinline__ void store_operand(uint8_t* a, int tile, int lane, const uint2 (&v)[2][4]) {
+    const int g = lane >> 2, q = lane & 3;
+    const bool odd = g & 1;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        uint8_t* row = a + (size_t)(16 * tile + 8 * h + g) * 128 + (q & 1) * 8;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint2 x = odd ? v[h][i ^ 2] : v[h][i];
+            const int j = odd ? i ^ 2 : i;
+            *reinterpret_cast<uint2*>(row + (((2 * j + (q >> 1)) ^ g) << 4)) = x;
+        }
+    }
+}
+
+// One CTA: 128 weight rows x nt token rows over a range of K.
+//   warps 0..7  convert weight tiles into the A operand, then read the accumulators back (epilogue);
+//   warp 8      one lane brings the token operand (and, for slab weights, the A operand) with bulk copies;
+//   warp 9      one lane issues the MMAs.
+// grid: x = token tile (neighbouring CTAs share weights, so HBM reads them once), y = 128-row weight block, z = K split;
+// routed groups: x = weight block, y = work item.
+// PX: bf16 pieces of the token operand (3: fp32-exact inputs), weight pieces: 2 for block-scaled FP8, else 1.
+template <int FMT, int PX, int OUT>
+__global__ void __launch_bounds__(GEMM_THREADS, 2) rows_gemm(const __grid_constant__ GemmArgs A) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    constexpr int PW = FMT == W_FP8_BLOCK ? 2 : 1;
+    constexpr int DIST = FMT == W_BF16 ? 2 : (FMT == W_MXFP4 ? 6 : 4);        // blocks a lane requests ahead
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int group = 0, row0, rows, block, z = 0;
+    if (A.items) {
+        if ((int)blockIdx.y >= __ldg(A.n_items)) return;
+        const int4 it = __ldg(A.items + blockIdx.y);
+        group = it.x;
+        row0 = it.y;
+        rows = it.z;
+        block = blockIdx.x;
+    } else {
+        row0 = (int)blockIdx.x * A.nt;
+        rows = min(A.nt, A.rows - row0);
+        block = blockIdx.y;
+        z = blockIdx.z;
+    }
+    const int nt = A.items ? (rows + 15) & ~15 : A.nt;         // columns this CTA multiplies
+    const int kb0 = (int)((long long)A.kbs * z / A.ksplit), kb1 = (int)((long long)A.kbs * (z + 1) / A.ksplit);
+    const uint32_t x_bytes = (uint32_t)nt * 128u, stage_bytes = PW * A_BYTES + PX * (uint32_t)A.nt * 128u;
+    GemmBars& B = *reinterpret_cast<GemmBars*>(smem + (size_t)A.stages * stage_bytes);
+    int cols = 32;
+    while (cols < A.nt) cols *= 2;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < A.stages; i++) {
+            mbar_init(&B.full[i], FMT == W_SLAB ? 1 : CONV_WARPS + 1);
+            mbar_init(&B.empty[i], 1);
+        }
+        mbar_init(&B.done, 1);
+        B.dead = 0;
+        mk::fence_barrier_init();
+    }
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&B.tmem)), "r"(cols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = B.tmem;
+
+    if (warp == CONV_WARPS) {
+        if (lane == 0) {
+            int i = 0;
+            uint32_t slot = 0, phase = 0;
+#pragma unroll 1
+            for (int kb = kb0; kb < kb1; kb++, i++) {
+                if (!wait(B, A, &B.empty[slot], phase ^ 1u, WP_EMPTY)) break;
+                uint8_t* st = smem + (size_t)slot * stage_bytes;
+                mbar_expect_tx(&B.full[slot], PX * x_bytes + (FMT == W_SLAB ? A_BYTES : 0));
+                if (FMT == W_SLAB)
+                    mk::bulk_load(st, A.w + (size_t)group * A.w_gstride + ((size_t)kb * A.w_rows + (size_t)block * 128) * 128, A_BYTES, &B.full[slot], mk::policy_evict_first());
+#pragma unroll
+                for (int p = 0; p < PX; p++)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 ::"r"(smem_u32(st + PW * A_BYTES + (size_t)p * A.nt * 128)),
+                                   "l"(A.x + (size_t)p * A.x_piece + ((size_t)kb * A.x_rows + row0) * 128), "r"(x_bytes), "r"(smem_u32(&B.full[slot])) : "memory");
+                if (++slot == (uint32_t)A.stages) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+            }
+            if (B.dead) {
+                // a role gave up: copies in flight must land before the CTA leaves (their barrier may still await others,
+                // so this waits a bounded time instead)
+                const u64 t0 = mk::globaltimer();
+                while (mk::globaltimer() - t0 < 1000000ull) {}
+            }
+        }
+    } else if (warp == CONV_WARPS + 1) {
+        if (lane == 0) {
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | (8u << 24);   // f32 <- bf16 x bf16, M 128
+            uint32_t slot = 0, phase = 0, accumulate = 0;
+            bool ok = true;
+#pragma unroll 1
+            for (int kb = kb0; kb < kb1; kb++) {
+                if (!wait(B, A, &B.full[slot], phase, WP_FULL)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t st = smem_u32(smem + (size_t)slot * stage_bytes);
+#pragma unroll
+                for (int pw = 0; pw < PW; pw++)
+#pragma unroll
+                    for (int px = 0; px < PX; px++) {
+                        const uint64_t da = operand_desc(st + pw * A_BYTES), db = operand_desc(st + PW * A_BYTES + px * (uint32_t)A.nt * 128u);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                                         ::"r"(tmem), "l"(da + 2 * k), "l"(db + 2 * k), "r"(idesc), "r"(accumulate));
+                            accumulate = 1;
+                        }
+                    }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&B.empty[slot])) : "memory");
+                if (++slot == (uint32_t)A.stages) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+            }
+            if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&B.done)) : "memory");
+        }
+    } else {
+        if constexpr (FMT != W_SLAB) {
+            // warp = tile: its bytes are requested DIST blocks ahead, straight into registers
+            const int tile = block * 8 + warp;
+            const bool have = tile < A.tiles;
+            Walk<FMT> walk;
+            walk.start(A, A.w + (size_t)group * A.w_gstride, min(tile, A.tiles - 1), kb0);
+            Raw<FMT> raw[DIST];
+            int asked = kb0;
+#pragma unroll
+            for (int i = 0; i < DIST; i++)
+                if (asked < kb1) {
+                    walk.load(A, lane, raw[i]);
+                    asked++;
+                }
+            uint32_t slot = 0, phase = 0;
+            bool ok = true;
+#pragma unroll 1
+            for (int kb = kb0; kb < kb1 && ok; kb += DIST) {
+#pragma unroll
+                for (int i = 0; i < DIST; i++) {
+                    if (kb + i < kb1 && ok) {
+                        uint2 v[2][4], lo[2][4];
+                        convert<FMT>(raw[i], v, lo);
+                        if (!have) {
+#pragma unroll
+                            for (int j = 0; j < 4; j++) v[0][j] = v[1][j] = lo[0][j] = lo[1][j] = make_uint2(0u, 0u);
+                        }
+                        if (asked < kb1) {
+                            walk.load(A, lane, raw[i]);
+                            asked++;
+                        }
+                        ok = __all_sync(0xffffffffu, wait(B, A, &B.empty[slot], phase ^ 1u, WP_EMPTY));   // the warp leaves together
+                        if (ok) {
+                            uint8_t* st = smem + (size_t)slot * stage_bytes;
+                            store_operand(st, warp, lane, v);
+                            if (PW == 2) store_operand(st + A_BYTES, warp, lane, lo);
+                            mk::fence_proxy_async();
+                        }
+                        __syncwarp();
+                        if (ok && lane == 0) mbar_arrive(&B.full[slot]);
+                        if (++slot == (uint32_t)A.stages) {
+                            slot = 0;
+                            phase ^= 1u;
+                        }
+                    }
+                }
+            }
+        }
+        // ---- epilogue: lane = weight row, columns = tokens; warps 0-3 and 4-7 take alternate groups of 16 tokens
+        const bool ok = __all_sync(0xffffffffu, wait(B, A, &B.done, 0, WP_DONE));
+        if (ok) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int sub = warp & 3, n = block * 128 + sub * 32 + lane;
+            float rs = 1.f;
+            if (A.row_scale && n < A.tiles * 16) rs = __ldg(A.row_scale + (size_t)group * A.rs_gstride + n);
+#pragma unroll 1
+            for (int c0 = (warp >> 2) * 16; c0 < nt; c0 += 32) {
+                uint32_t r[16];
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                               "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                             : "r"(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)c0));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const float v = __uint_as_float(r[i]) * rs;
+                    const int t = row0 + c0 + i;
+                    const bool live = c0 + i < rows;
+                    if (A.ksplit > 1) {
+                        if (live && n < A.n_valid) A.part[((size_t)z * A.part_rows + t) * A.n_valid + n] = v;
+                    } else if (OUT == OUT_GLU) {
+                        // rows 0-7 of a 16-row tile are gates, rows 8-15 their up rows
+                        const float up = __shfl_down_sync(0xffffffffu, v, 8);
+                        const int col = (n >> 4) * 8 + (n & 7);
+                        if (live && !(n & 8) && col < A.act_cols) {
+                            float y = A.gelu ? 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v))) : silu_f(v);
+                            y *= up;
+                            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(A.act + slab_offset(A.act_rows, t, col));
+#pragma unroll
+                            for (int p = 0; p < PX; p++) {
+                                const __nv_bfloat16 b = __float2bfloat16_rn(y);
+                                *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<uint8_t*>(dst) + (size_t)p * A.act_piece) = b;
+                                y -= __bfloat162float(b);
+                            }
+                        }
+                    } else if (live && n < A.n_valid) {
+                        float* o = A.out + (size_t)t * A.out_stride + n;
+                        *o = OUT == OUT_ADD ? *o + v : v;
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        }
+    }
+    __syncthreads();
+    if (warp == 9) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
+    }
+}
+
+// Adds the K splits' partials in split order and runs the epilogue.
+template <int PX, int OUT>
+__global__ void __launch_bounds__(256) rows_finish(const __grid_constant__ GemmArgs A) {
+    const int t = blockIdx.y;
+    const float* p = A.part + (size_t)t * A.n_valid;
+    const size_t ss = (size_t)A.part_rows * A.n_valid;
+    if (OUT == OUT_GLU) {
+        const int col = blockIdx.x * 256 + threadIdx.x;
+        if (col >= A.act_cols) return;
+        const int n = (col >> 3) * 16 + (col & 7);
+        float g = 0.f, u = 0.f;
+        for (int z = 0; z < A.ksplit; z++) {
+            g += p[z * ss + n];
+            u += p[z * ss + n + 8];
+        }
+        float y = (A.gelu ? 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) : silu_f(g)) * u;
+        uint8_t* dst = A.act + slab_offset(A.act_rows, t, col);
+#pragma unroll
+        for (int q = 0; q < PX; q++) {
+            const __nv_bfloat16 b = __float2bfloat16_rn(y);
+            *reinterpret_cast<__nv_bfloat16*>(dst + (size_t)q * A.act_piece) = b;
+            y -= __bfloat162float(b);
+        }
+    } else {
+        const int n = (blockIdx.x * 256 + threadIdx.x) * 4;
+        if (n >= A.n_valid) return;
+        float* o = A.out + (size_t)t * A.out_stride + n;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (((A.n_valid | (int)A.out_stride) & 3) == 0) {
+            for (int z = 0; z < A.ksplit; z++) {
+                const float4 a = *reinterpret_cast<const float4*>(p + z * ss + n);
+                v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+            }
+            float4* o4 = reinterpret_cast<float4*>(o);
+            if (OUT == OUT_ADD) {
+                const float4 b = *o4;
+                v[0] += b.x; v[1] += b.y; v[2] += b.z; v[3] += b.w;
+            }
+            *o4 = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+            for (int i = 0; i < 4 && n + i < A.n_valid; i++) {
+                for (int z = 0; z < A.ksplit; z++) v[i] += p[z * ss + n + i];
+                o[i] = OUT == OUT_ADD ? o[i] + v[i] : v[i];
+            }
+        }
+    }
+}
+
+// ---- element-wise steps ------------------------------------------------------------------------------------
+__device__ __forceinline__ float block_sum(float v, float* red) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float s = 0.f;
+    for (int i = 0; i < (int)blockDim.x / 32; i++) s += red[i];
+    __syncthreads();
+    return s;
+}
+
+// fp32 rows -> slabs: optional RMSNorm, rounding to bf16 (PIECES = 1, the model's activation type) or fp32-exact pieces.
+template <int PIECES>
+__global__ void __launch_bounds__(256) rows_in(const float* x, long long stride, int K, const float* norm_w, float norm_off, float eps, float in_scale,
+                                               uint8_t* out, size_t piece, int out_rows) {
+    __shared__ float red[8];
+    const int row = blockIdx.x;
+    const float* src = x + (size_t)row * stride;
+    float r = 1.f;
+    if (norm_w) {
+        float s = 0.f;
+        for (int c = threadIdx.x * 4; c < K; c += 1024) {
+            const float4 a = *reinterpret_cast<const float4*>(src + c);
+            s += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+        }
+        s = block_sum(s, red);
+        r = rsqrtf(s / (float)K + eps) * in_scale;
+    }
+    for (int c = threadIdx.x * 8; c < K; c += 2048) {
+        const float4 a = *reinterpret_cast<const float4*>(src + c), b = *reinterpret_cast<const float4*>(src + c + 4);
+        float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        if (norm_w) {
+            const float4 wa = __ldg(reinterpret_cast<const float4*>(norm_w + c)), wb = __ldg(reinterpret_cast<const float4*>(norm_w + c + 4));
+            const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = v[i] * r * (norm_off + w[i]);
+        }
+        store_slab8<PIECES>(out, piece, out_rows, row, c, v);
+    }
+}
+
+// Row r = sequence * L + position of every array below; tokens are [L][M] (step-major, as mk_stage_args.tokens_in).
+__global__ void __launch_bounds__(256) embed_rows(const __nv_bfloat16* table, const int* tokens, int M, int L, int H, int vocab, float scale, float* h) {
+    const int row = blockIdx.x, m = row / L, l = row - m * L;
+    const int tok = max(0, min(vocab - 1, tokens[(size_t)l * M + m]));
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(table + (size_t)tok * H);
+    float2* dst = reinterpret_cast<float2*>(h + (size_t)row * H);
+    for (int c = threadIdx.x; c < H / 2; c += 256) {
+        const uint32_t w = __ldg(src + c);
+        float lo = bf_lo(w), hi = bf_hi(w);
+        if (scale != 0.f) {
+            lo = round_bf16(lo * scale);
+            hi = round_bf16(hi * scale);
+        }
+        dst[c] = make_float2(lo, hi);
+    }
+}
+
+__global__ void advance_pos(int* pos, int M, int L) {
+    if ((int)threadIdx.x < M) pos[threadIdx.x] += L;
+}
+
+// out = (base + rms(a) w_a [+ rms(b) w_b]) * scale
+__global__ void __launch_bounds__(256) vec_rows(int N, const float* base, const float* a, const float* wa, const float* b, const float* wb, float off, float eps,
+                                                float scale, float* out) {
+    __shared__ float red[8];
+    const size_t o = (size_t)blockIdx.x * N;
+    float sa = 0.f, sb = 0.f;
+    for (int c = threadIdx.x; c < N; c += 256) {
+        sa += a[o + c] * a[o + c];
+        if (b) sb += b[o + c] * b[o + c];
+    }
+    const float ra = rsqrtf(block_sum(sa, red) / (float)N + eps);
+    const float rb = b ? rsqrtf(block_sum(sb, red) / (float)N + eps) : 0.f;
+    for (int c = threadIdx.x; c < N; c += 256) {
+        float r = a[o + c] * ra * (off + wa[c]);
+        if (b) r += b[o + c] * rb * (off + wb[c]);
+        if (base) r += base[o + c];
+        out[o + c] = r * scale;
+    }
+}
+
+// ---- Gated DeltaNet ----------------------------------------------------------------------------------------
+struct GdnArgs {
+    const float* y;              // in-projection rows
+    long long y_stride;
+    int M, L, nkh, nvh, conv_dim;
+    int q_off, k_off, v_off, z_off, b_off, a_off;
+    const float *conv_w, *A_log, *dt_bias, *norm_w;
+    float* conv_state;           // history rings; see `conv_slot`
+    int ring, layout;            // ring length; 0: [M][conv_dim][ring], 1: the 0.8B kernel's per-task copies, 2: its per-head batched layout
+    float* ssm;                  // [M][nvh][128 v][128 k]
+    const int* pos;              // position of each sequence's first row
+    int conv_bf16, l2_clamp;
+    float eps;
+    // scratch
+    float* qkv;                  // [rows][conv_dim]: normalised q, k, and v
+    float4* scal;                // [rows][nvh]: decay, beta, q . k of the head
+    float* o;                    // [rows][nvh * 128]
+    uint8_t* out;                // slabs of the gated output
+    size_t out_piece;
+    int out_rows;
+};
+
+// Where the history of channel `ch` (q | k | v order) of sequence m lives; the 0.8B kernels keep q and k once per
+// recurrence task of the head (8 of them), of which task `copy` is meant.
+__device__ __forceinline__ float* conv_slot(const GdnArgs& G, int m, int ch, int copy) {
+    const int qk = G.nkh * 128;
+    if (G.layout == 0) return G.conv_state + ((size_t)m * G.conv_dim + ch) * G.ring;
+    const int part = ch < qk ? 0 : (ch < 2 * qk ? 1 : 2), c = ch - part * qk, h = c >> 7, i = c & 127;
+    if (G.layout == 2) return G.conv_state + (((size_t)m * G.nvh + h) * 384 + part * 128 + i) * G.ring;
+    const int task = h * 8 + (part == 2 ? i >> 4 : copy);
+    return G.conv_state + ((size_t)task * 272 + (part == 2 ? 256 + (i & 15) : part * 128 + i)) * G.ring;
+}
+
+// Causal conv1d + SiLU of every channel, L2 norms of q and k, and the scalars of the recurrence.  One warp per 128
+// channels of a row, four channels per lane.
+__global__ void __launch_bounds__(256) gdn_conv(const __grid_constant__ GdnArgs G) {
+    const int row = blockIdx.y, m = row / G.L, l = row - m * G.L, lane = threadIdx.x & 31;
+    const int blk = blockIdx.x * 8 + (threadIdx.x >> 5);                    // 128-channel block: q heads, k heads, v heads
+    if (blk * 128 >= G.conv_dim) return;
+    const int part = blk < G.nkh ? 0 : (blk < 2 * G.nkh ? 1 : 2);
+    const int head = blk - part * G.nkh;
+    const int col = (part == 0 ? G.q_off : (part == 1 ? G.k_off : G.v_off)) + head * 128 + 4 * lane;
+    const int ch = blk * 128 + 4 * lane;
+    const float* y = G.y + (size_t)row * G.y_stride + col;
+    const int pos = G.pos[m] + l;
+    float x[4][4];                                                          // [tap][channel], oldest first
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+        const int back = 3 - d;
+        if (l >= back) {
+            const float4 a = *reinterpret_cast<const float4*>(y - (long long)back * G.y_stride);
+            x[d][0] = a.x; x[d][1] = a.y; x[d][2] = a.z; x[d][3] = a.w;
+            if (back && G.conv_bf16) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) x[d][i] = round_bf16(x[d][i]);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[d][i] = conv_slot(G, m, ch + i, 0)[(pos - back) & (G.ring - 1)];
+        }
+    }
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float4 w = __ldg(reinterpret_cast<const float4*>(G.conv_w) + ch + i);
+        float a = x[0][i] * w.x;
+        a = fmaf(x[1][i], w.y, a);
+        a = fmaf(x[2][i], w.z, a);
+        a = fmaf(x[3][i], w.w, a);
+        v[i] = silu_f(a);
+    }
+    if (part < 2) {
+        const float s = warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
+        float inv = G.l2_clamp ? 1.f / fmaxf(sqrtf(s), G.eps) : 1.f / sqrtf(s + G.eps);
+        if (part == 0) inv *= 0.08838834764831845f;                         // 128^-0.5
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] *= inv;
+    }
+    *reinterpret_cast<float4*>(G.qkv + (size_t)row * G.conv_dim + ch) = make_float4(v[0], v[1], v[2], v[3]);
+    if (part == 2 && lane == 0) {
+        const float b = G.y[(size_t)row * G.y_stride + G.b_off + head], a = G.y[(size_t)row * G.y_stride + G.a_off + head];
+        G.scal[(size_t)row * G.nvh + head] = make_float4(expf(-expf(G.A_log[head]) * softplus_f(a + G.dt_bias[head])), sigmoid_f(b), 0.f, 0.f);
+    }
+}
+
+// The last `ring` inputs of every channel go back into the history rings.  Runs after gdn_conv has read them.
+__global__ void __launch_bounds__(256) gdn_history(const __grid_constant__ GdnArgs G) {
+    const int ch = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y;
+    if (ch >= G.conv_dim) return;
+    const int qk = G.nkh * 128, part = ch < qk ? 0 : (ch < 2 * qk ? 1 : 2);
+    const int col = (part == 0 ? G.q_off : (part == 1 ? G.k_off : G.v_off)) + ch - part * qk;
+    for (int l = max(0, G.L - G.ring); l < G.L; l++) {
+        float v = G.y[((size_t)m * G.L + l) * G.y_stride + col];
+        if (G.conv_bf16) v = round_bf16(v);
+        const int slot = (G.pos[m] + l) & (G.ring - 1);
+        const int copies = G.layout == 1 && part < 2 ? 8 : 1;
+        for (int c = 0; c < copies; c++) conv_slot(G, m, ch, c)[slot] = v;
+    }
+}
+
+// The recurrence of 32 value rows of one head of one sequence, position after position: state rows never interact, so a
+// head is four CTAs.  Eight threads share a row (16 keys each, in registers); the inputs of the next SCAN_BLOCK
+// positions arrive in shared memory while the current ones run.  Both dot products are taken against the state before
+// the update (o = decay (S q) + delta (k . q)), so they reduce together and only one of them is on the critical path.
+constexpr int SCAN_BLOCK = 8;
+__global__ void __launch_bounds__(256) gdn_scan(const __grid_constant__ GdnArgs G) {
+    __shared__ __align__(16) float in_s[2][SCAN_BLOCK][256 + 32];            // q | k | 32 values
+    __shared__ float4 sc_s[2][SCAN_BLOCK];
+    const int rep = G.nvh / G.nkh;
+    const int m = blockIdx.z, h = blockIdx.y, v0 = blockIdx.x * 32, kh = h / rep;
+    const int tid = threadIdx.x, vr = tid >> 3, part = tid & 7;
+    float* st = G.ssm + (((size_t)m * G.nvh + h) * 128 + v0 + vr) * 128 + part * 4;     // keys part * 4 + 32 i + {0..3}
+    float s[16];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float4 a = *reinterpret_cast<const float4*>(st + 32 * i);
+        s[4 * i] = a.x; s[4 * i + 1] = a.y; s[4 * i + 2] = a.z; s[4 * i + 3] = a.w;
+    }
+    const size_t row0 = (size_t)m * G.L;
+    const int key_dim = G.nkh * 128;
+    auto request = [&](int buf, int l0) {
+        // 72 16-byte pieces per position: 32 of q, 32 of k, 8 of v
+        for (int i = tid; i < SCAN_BLOCK * 72; i += 256) {
+            const int b = i / 72, c = i - b * 72, l = l0 + b;
+            if (l < G.L) {
+                const float* src = G.qkv + (row0 + l) * G.conv_dim + (c < 32 ? kh * 128 + 4 * c : (c < 64 ? key_dim + kh * 128 + 4 * (c - 32) : 2 * key_dim + h * 128 + v0 + 4 * (c - 64)));
+                mk::cp_async16(&in_s[buf][b][4 * c], src);
+            }
+        }
+        if (tid < SCAN_BLOCK && l0 + tid < G.L) mk::cp_async16(&sc_s[buf][tid], G.scal + (row0 + l0 + tid) * G.nvh + h);
+        mk::cp_async_commit();
+    };
+    request(0, 0);
+    float* o = G.o + row0 * (size_t)(G.nvh * 128) + h * 128 + v0 + vr;
+#pragma unroll 1
+    for (int l0 = 0, buf = 0; l0 < G.L; l0 += SCAN_BLOCK, buf ^= 1) {
+        mk::cp_async_wait_all();
+        __syncthreads();
+        if (l0 + SCAN_BLOCK < G.L) request(buf ^ 1, l0 + SCAN_BLOCK);
+        const int nb = min(SCAN_BLOCK, G.L - l0);
+#pragma unroll 1
+        for (int b = 0; b < nb; b++) {
+            const float* q = in_s[buf][b] + part * 4;
+            const float* k = q + 128;
+            float kk[16], dk = 0.f, dq = 0.f, kq = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 a = *reinterpret_cast<const float4*>(k + 32 * i), c = *reinterpret_cast<const float4*>(q + 32 * i);
+                kk[4 * i] = a.x; kk[4 * i + 1] = a.y; kk[4 * i + 2] = a.z; kk[4 * i + 3] = a.w;
+                dk = fmaf(s[4 * i], a.x, dk); dk = fmaf(s[4 * i + 1], a.y, dk); dk = fmaf(s[4 * i + 2], a.z, dk); dk = fmaf(s[4 * i + 3], a.w, dk);
+                dq = fmaf(s[4 * i], c.x, dq); dq = fmaf(s[4 * i + 1], c.y, dq); dq = fmaf(s[4 * i + 2], c.z, dq); dq = fmaf(s[4 * i + 3], c.w, dq);
+                kq = fmaf(a.x, c.x, kq); kq = fmaf(a.y, c.y, kq); kq = fmaf(a.z, c.z, kq); kq = fmaf(a.w, c.w, kq);
+            }
+#pragma unroll
+            for (int x = 1; x < 8; x <<= 1) {
+                dk += __shfl_xor_sync(0xffffffffu, dk, x);
+                dq += __shfl_xor_sync(0xffffffffu, dq, x);
+                kq += __shfl_xor_sync(0xffffffffu, kq, x);
+            }
+            const float4 sc = sc_s[buf][b];
+            const float delta = (in_s[buf][b][256 + vr] - sc.x * dk) * sc.y;
+#pragma unroll
+            for (int i = 0; i < 16; i++) s[i] = fmaf(kk[i], delta, s[i] * sc.x);
+            if (part == 0) o[(size_t)(l0 + b) * (G.nvh * 128)] = fmaf(sc.x, dq, delta * kq);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) *reinterpret_cast<float4*>(st + 32 * i) = make_float4(s[4 * i], s[4 * i + 1], s[4 * i + 2], s[4 * i + 3]);
+}
+
+// Gated RMSNorm per head, into slabs: one half warp per head and row (eight columns per lane).
+template <int PIECES>
+__global__ void __launch_bounds__(256) gdn_gate(const __grid_constant__ GdnArgs G) {
+    const int row = blockIdx.y, h = blockIdx.x * 16 + (threadIdx.x >> 4), i = (threadIdx.x & 15) * 8;
+    if (h >= G.nvh) return;
+    const float* o = G.o + (size_t)row * (G.nvh * 128) + h * 128 + i;
+    const float* z = G.y + (size_t)row * G.y_stride + G.z_off + h * 128 + i;
+    float v[8], s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        v[j] = o[j];
+        s = fmaf(v[j], v[j], s);
+    }
+    const unsigned mask = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+    for (int x = 8; x; x >>= 1) s += __shfl_xor_sync(mask, s, x);
+    const float r = rsqrtf(s / 128.f + G.eps);
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = v[j] * r * __ldg(G.norm_w + i + j) * (z[j] * sigmoid_f(z[j]));
+    store_slab8<PIECES>(G.out, G.out_piece, G.out_rows, row, h * 128 + i, v);
+}
+
+// ---- attention -----------------------------------------------------------------------------------------------
+struct AttnArgs {
+    const float* y;
+    long long y_stride;
+    int M, L, nq, nkv;
+    int q_off, q_hs, gate_off, k_off, v_off;
+    int rot, pairs, window, q_bf16, norm_plain, v_norm;
+    float eps, scale;
+    const float *q_norm, *k_norm, *cos, *sin;
+    void *k_cache, *v_cache;
+    const int* bt;
+    int max_pages, kv_shift;
+    uint32_t s_page, s_head, s_pos;
+    const int* pos;
+    __nv_bfloat16* q;            // [rows][nq][HD] prepared queries
+    uint8_t* out;                // slabs of the (gated) output
+    int out_rows;
+};
+
+__device__ __forceinline__ size_t kv_offset(const AttnArgs& T, int m, int kvh, int p) {
+    const int page = __ldg(T.bt + (size_t)m * T.max_pages + (p >> T.kv_shift));
+    return (size_t)((uint32_t)page * T.s_page + (uint32_t)kvh * T.s_head + (uint32_t)(p & ((1 << T.kv_shift) - 1)) * T.s_pos);
+}
+
+// Norm, rotation and rounding of every head vector of a row: queries to `q`, keys and values into the paged cache.
+// One warp per head vector; lane i holds dims i + 32 j, so both halves of a rotated pair are in one lane.
+template <int HD>
+__global__ void __launch_bounds__(256) attn_prepare(const __grid_constant__ AttnArgs T) {
+    constexpr int N = HD / 32;
+    const int row = blockIdx.y, m = row / T.L, lane = threadIdx.x & 31;
+    const int hv = blockIdx.x * 8 + (threadIdx.x >> 5);                 // q heads, k heads, v heads
+    if (hv >= T.nq + 2 * T.nkv) return;
+    const int kind = hv < T.nq ? 0 : (hv < T.nq + T.nkv ? 1 : 2);
+    const int head = kind == 0 ? hv : (kind == 1 ? hv - T.nq : hv - T.nq - T.nkv);
+    const float* y = T.y + (size_t)row * T.y_stride;
+    const float* src = kind == 0 ? y + T.q_off + (size_t)head * T.q_hs
+                                 : (kind == 1 || T.v_off < 0 ? y + T.k_off + (size_t)head * HD : y + T.v_off + (size_t)head * HD);
+    const int pos = T.pos[m] + (row - m * T.L);
+    float v[N], s = 0.f;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        v[j] = src[lane + 32 * j];
+        s = fmaf(v[j], v[j], s);
+    }
+    const float* nw = kind == 0 ? T.q_norm : (kind == 1 ? T.k_norm : nullptr);
+    const float off = T.norm_plain ? 0.f : 1.f;
+    if (kind < 2 || T.v_norm) {
+        const float r = rsqrtf(warp_sum(s) / (float)HD + T.eps);
+#pragma unroll
+        for (int j = 0; j < N; j++) v[j] = v[j] * r * (nw ? off + __ldg(nw + lane + 32 * j) : 1.f);
+    }
+    if (kind < 2) {
+        const int pd = T.rot == HD ? HD / 64 : T.rot / 64;               // distance of a pair in units of 32 dims
+#pragma unroll
+        for (int j = 0; j < N / 2; j++)
+            if (j < pd && lane + 32 * j < T.pairs) {
+                const size_t o = (size_t)pos * T.pairs + lane + 32 * j;
+                const float c = __ldg(T.cos + o), sn = __ldg(T.sin + o);
+#pragma unroll
+                for (int d = 1; d <= N / 2; d++)                          // static register indexes
+                    if (d == pd) {
+                        const float a = v[j], b = v[j + d];
+                        v[j] = a * c - b * sn;
+                        v[j + d] = b * c + a * sn;
+                    }
+            }
+    }
+    if (kind == 0) {
+        __nv_bfloat16* dst = T.q + ((size_t)row * T.nq + head) * HD;
+#pragma unroll
+        for (int j = 0; j < N; j++) dst[lane + 32 * j] = __float2bfloat16_rn(v[j]);
+    } else {
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(kind == 1 ? T.k_cache : T.v_cache) + kv_offset(T, m, head, pos);
+#pragma unroll
+        for (int j = 0; j < N; j++) dst[lane + 32 * j] = __float2bfloat16_rn(v[j]);
+    }
+}
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cp16_zfill(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Causal attention of a block of positions over the paged bf16 cache.  A CTA owns one KV head of one sequence and
+// 64 query rows (position, head of the group); blocks of 64 keys pass through shared memory.  Warp (r, d): rows 16 r ..
+// 16 r + 15; it scores keys 32 d .. 32 d + 31 of the block and accumulates head dims [d HD / 2, (d + 1) HD / 2).
+// Probabilities enter the second product as three bf16 pieces (24 bits), so only Q, K and V carry bf16 roundings, as in
+// the decode step.  V arrives while the scores are computed, the next K while P x V runs.
+constexpr int AT_ROWS = 64, AT_KEYS = 64, AT_PIECES = 3;
+template <int HD> constexpr int attn_smem() { return 3 * AT_ROWS * HD * 2 + AT_PIECES * AT_ROWS * AT_KEYS * 2 + 4 * AT_ROWS * 4; }
+template <int HD>
+__global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant__ AttnArgs T) {
+    extern __shared__ __align__(128) uint8_t sm[];
+    constexpr int RB = HD * 2, CH = RB / 16;                             // bytes and 16-byte pieces of a row
+    uint8_t *q_s = sm, *k_s = q_s + AT_ROWS * RB, *v_s = k_s + AT_KEYS * RB, *p_s = v_s + AT_KEYS * RB;
+    float* st_s = reinterpret_cast<float*>(p_s + AT_PIECES * AT_ROWS * AT_KEYS * 2);   // [2][64] maxima, [2][64] sums
+    const int qpk = T.nq / T.nkv, bq = AT_ROWS / qpk;
+    const int m = blockIdx.z, kvh = blockIdx.y, l0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * bq;      // long ones first
+    const int np = min(bq, T.L - l0), pos0 = T.pos[m] + l0;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp & 3, dh = warp >> 2, g = lane >> 2, t = lane & 3;
+    const int last = pos0 + np - 1, first = (T.window ? max(0, pos0 - T.window + 1) : 0) & ~(AT_KEYS - 1);
+    const __nv_bfloat16 *kc = reinterpret_cast<const __nv_bfloat16*>(T.k_cache), *vc = reinterpret_cast<const __nv_bfloat16*>(T.v_cache);
+    auto load_kv = [&](uint8_t* dst, const __nv_bfloat16* cache, int k0) {
+#pragma unroll 4
+        for (int i = tid; i < AT_KEYS * CH; i += 256) {
+            const int key = i / CH, c = i - key * CH, p = k0 + key;
+            cp16_zfill(smem_u32(dst + (size_t)key * RB + (((c & ~7) | ((c ^ key) & 7)) << 4)), cache + kv_offset(T, m, kvh, min(p, last)) + c * 8, p <= last);
+        }
+        mk::cp_async_commit();
+    };
+    for (int i = tid; i < AT_ROWS * CH; i += 256) {
+        const int r = i / CH, c = i - r * CH, p = r / qpk, hq = r - p * qpk;
+        const bool live = p < np;
+        const __nv_bfloat16* src = T.q + (((size_t)m * T.L + l0 + (live ? p : 0)) * T.nq + kvh * qpk + hq) * HD + c * 8;
+        cp16_zfill(smem_u32(q_s + (size_t)r * RB + (((c & ~7) | ((c ^ r) & 7)) << 4)), src, live);
+    }
+    load_kv(k_s, kc, first);
+    float o[HD / 16][4], mx[2] = {-3.0e38f, -3.0e38f}, sum[2] = {0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < HD / 16; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    int qp[2];                                                           // positions of this lane's two rows
+#pragma unroll
+    for (int i = 0; i < 2; i++) qp[i] = pos0 + min((16 * rg + g + 8 * i) / qpk, np - 1);
+    const uint32_t qa = smem_u32(q_s) + (uint32_t)(16 * rg + (lane & 15)) * RB, qx = (lane & 7);
+#pragma unroll 1
+    for (int k0 = first; k0 <= last; k0 += AT_KEYS) {
+        cp_wait<0>();
+        __syncthreads();                                                 // K is here; everybody is done with V and P
+        load_kv(v_s, vc, k0);
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+#pragma unroll 4
+        for (int kk = 0; kk < HD / 16; kk++) {
+            uint32_t a[4];
+            const uint32_t ca = 2 * kk + (lane >> 4);
+            ldsm4(a, qa + (((ca & ~7u) | ((ca ^ qx) & 7)) << 4));
+#pragma unroll
+            for (int n = 0; n < 2; n++) {
+                const uint32_t key = 32 * dh + 16 * n + (lane & 7) + ((lane >> 4) << 3), cb = 2 * kk + ((lane >> 3) & 1);
+                uint32_t b[4];
+                ldsm4(b, smem_u32(k_s) + key * RB + (((cb & ~7u) | ((cb ^ key) & 7)) << 4));
+                mma16816(s[2 * n], a, b[0], b[1]);
+                mma16816(s[2 * n + 1], a, b[2], b[3]);
+            }
+        }
+        // mask, scale, running maximum over both key halves
+        float bm[2] = {-3.0e38f, -3.0e38f};
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int p = k0 + 32 * dh + 8 * n + 2 * t + (i & 1), r = i >> 1;
+                const bool seen = p <= qp[r] && (!T.window || p > qp[r] - T.window);
+                s[n][i] = seen ? s[n][i] * T.scale : -3.0e38f;
+                bm[r] = fmaxf(bm[r], s[n][i]);
+            }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 1));
+            bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 2));
+            if (t == 0) st_s[dh * AT_ROWS + 16 * rg + g + 8 * r] = bm[r];
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + rg) : "memory");        // the two warps of these rows
+        float f[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const float nm = fmaxf(mx[r], fmaxf(bm[r], st_s[(dh ^ 1) * AT_ROWS + 16 * rg + g + 8 * r]));
+            f[r] = __expf(mx[r] - nm);
+            mx[r] = nm;
+            sum[r] *= f[r];
+        }
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                float p0 = s[n][2 * r] > -2.9e38f ? __expf(s[n][2 * r] - mx[r]) : 0.f, p1 = s[n][2 * r + 1] > -2.9e38f ? __expf(s[n][2 * r + 1] - mx[r]) : 0.f;
+                sum[r] += p0 + p1;
+                const uint32_t row = 16 * rg + g + 8 * r, c = 4 * dh + n;
+#pragma unroll
+                for (int q = 0; q < AT_PIECES; q++) {
+                    const uint32_t w = pack_bf16(p0, p1);
+                    *reinterpret_cast<uint32_t*>(p_s + q * AT_ROWS * AT_KEYS * 2 + row * 128 + ((c ^ (row & 7)) << 4) + t * 4) = w;
+                    p0 -= bf_lo(w);
+                    p1 -= bf_hi(w);
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < HD / 16; i++) {
+            o[i][0] *= f[0]; o[i][1] *= f[0];
+            o[i][2] *= f[1]; o[i][3] *= f[1];
+        }
+        cp_wait<0>();
+        __syncthreads();                                                 // V and P are here; everybody is done with K
+        if (k0 + AT_KEYS <= last) load_kv(k_s, kc, k0 + AT_KEYS);
+#pragma unroll
+        for (int kk = 0; kk < AT_KEYS / 16; kk++) {
+            uint32_t a[AT_PIECES][4];
+#pragma unroll
+            for (int q = 0; q < AT_PIECES; q++)
+                ldsm4(a[q], smem_u32(p_s) + q * AT_ROWS * AT_KEYS * 2 + (uint32_t)(16 * rg + (lane & 15)) * 128 + (((2 * kk + (lane >> 4)) ^ qx) << 4));
+#pragma unroll
+            for (int n = 0; n < HD / 32; n++) {
+                const uint32_t key = 16 * kk + (lane & 15), c = dh * (CH / 2) + 2 * n + (lane >> 4);
+                uint32_t b[4];
+                ldsm4_t(b, smem_u32(v_s) + key * RB + (((c & ~7u) | ((c ^ key) & 7)) << 4));
+#pragma unroll
+                for (int q = 0; q < AT_PIECES; q++) {
+                    mma16816(o[2 * n], a[q], b[0], b[1]);
+                    mma16816(o[2 * n + 1], a[q], b[2], b[3]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
+        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
+        if (t == 0) st_s[(2 + dh) * AT_ROWS + 16 * rg + g + 8 * r] = sum[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const int rr = 16 * rg + g + 8 * r, p = rr / qpk, hq = kvh * qpk + rr - p * qpk;
+        if (p >= np) continue;
+        const float inv = 1.f / (st_s[2 * AT_ROWS + rr] + st_s[3 * AT_ROWS + rr]);
+        const int row = m * T.L + l0 + p;
+        const float* gate = T.gate_off >= 0 ? T.y + (size_t)row * T.y_stride + T.q_off + (size_t)hq * T.q_hs + T.gate_off : nullptr;
+#pragma unroll
+        for (int n = 0; n < HD / 16; n++) {
+            const int dim = dh * (HD / 2) + 8 * n + 2 * t;
+            float a = o[n][2 * r] * inv, b = o[n][2 * r + 1] * inv;
+            if (gate) {
+                a *= sigmoid_f(gate[dim]);
+                b *= sigmoid_f(gate[dim + 1]);
+            }
+            *reinterpret_cast<uint32_t*>(T.out + slab_offset(T.out_rows, row, hq * HD + dim)) = pack_bf16(a, b);
+        }
+    }
+}
+
+// ---- expert routing --------------------------------------------------------------------------------------------
+struct RouteArgs {
+    const float* logits;
+    int rows, stride, experts, topk, kind;
+    const float* expert_scale;
+    int4* items;                 // {expert, first row, rows, 0}
+    int* n_items;
+    int* counts;                 // [experts] tokens per expert, then [experts] fill counters, then [experts] first rows
+    int* slot;                   // [rows][8] row of the token's k-th expert (ascending expert id) in the gathered order
+    float* weight;               // [rows][8]
+    float* gate;                 // [rows] shared expert's gate
+    int nt;
+};
+
+// One warp per token: the top-k experts (ties to the lower id), their weights, and the count per expert.
+__global__ void __launch_bounds__(256) route_rows(const __grid_constant__ RouteArgs R) {
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= R.rows) return;
+    const float* lg = R.logits + (size_t)row * R.stride;
+    const int per = R.experts / 32;
+    float v[8];
+    bool used[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        v[i] = i < per ? lg[lane + 32 * i] : 0.f;
+        used[i] = i >= per;
+    }
+    float top0 = 0.f, wsum = 0.f, myw = 0.f;
+    int myid = 0x7fffffff;
+#pragma unroll 1
+    for (int k = 0; k < R.topk; k++) {
+        u64 best = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (!used[i]) {
+                const u64 key = mk::score_key(v[i], lane + 32 * i);
+                best = key > best ? key : best;
+            }
+        best = mk::warp_max_u64(best);
+        const int id = max(0, min(R.experts - 1, mk::key_index(best)));
+        float mine = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (i == (id >> 5)) {
+                mine = v[i];
+                if (lane == (id & 31)) used[i] = true;
+            }
+        const float sc = __shfl_sync(0xffffffffu, mine, id & 31);
+        if (k == 0) top0 = sc;
+        const float w = __expf(sc - top0);
+        wsum += w;
+        if (lane == k) {
+            myw = w;
+            myid = id;
+        }
+    }
+    // rank among the token's experts: ascending id, the order in which their products are added
+    int rank = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) rank += __shfl_sync(0xffffffffu, myid, k) < myid;
+    if (lane < R.topk) {
+        R.slot[(size_t)row * 8 + rank] = myid;                           // the expert for now; route_slots turns it into a row
+        R.weight[(size_t)row * 8 + rank] = myw / wsum * (R.kind == 1 && R.expert_scale ? R.expert_scale[myid] : 1.f);
+        atomicAdd(R.counts + myid, 1);
+    }
+    if (R.kind == 0 && lane == 0) R.gate[row] = sigmoid_f(lg[R.experts]);
+}
+
+// Lays the experts' tokens out one after the other (each expert from a multiple of 16 rows) and lists the tiles.
+__global__ void __launch_bounds__(256) route_plan(const __grid_constant__ RouteArgs R) {
+    __shared__ int rows_s[256], tiles_s[256];
+    const int e = threadIdx.x, n = e < R.experts ? R.counts[e] : 0;
+    const int rows = (n + 15) & ~15, tiles = (n + R.nt - 1) / R.nt;
+    rows_s[e] = rows;
+    tiles_s[e] = tiles;
+    __syncthreads();
+    for (int d = 1; d < 256; d <<= 1) {
+        const int a = e >= d ? rows_s[e - d] : 0, b = e >= d ? tiles_s[e - d] : 0;
+        __syncthreads();
+        rows_s[e] += a;
+        tiles_s[e] += b;
+        __syncthreads();
+    }
+    const int first = rows_s[e] - rows, item = tiles_s[e] - tiles;
+    if (e < R.experts) {
+        R.counts[2 * R.experts + e] = first;
+        for (int i = 0; i < tiles; i++) R.items[item + i] = make_int4(e, first + i * R.nt, min(R.nt, n - i * R.nt), 0);
+    }
+    if (e == 255) *R.n_items = tiles_s[255];
+}
+
+__global__ void __launch_bounds__(256) route_slots(const __grid_constant__ RouteArgs R) {
+    const int i = blockIdx.x * 256 + threadIdx.x, row = i >> 3, k = i & 7;
+    if (row >= R.rows || k >= R.topk) return;
+    const int e = R.slot[i];
+    R.slot[i] = R.counts[2 * R.experts + e] + atomicAdd(R.counts + R.experts + e, 1);
+}
+
+// Copies every token's slab row to the rows of its experts.
+__global__ void __launch_bounds__(256) gather_rows(const uint8_t* x, int x_rows, const int* slot, int topk, int kbs, uint8_t* out, int out_rows) {
+    const int row = blockIdx.x;
+    for (int i = threadIdx.x; i < kbs * 8; i += 256) {
+        const int kb = i >> 3, c = i & 7;
+        const uint4 v = *reinterpret_cast<const uint4*>(x + ((size_t)kb * x_rows + row) * 128 + ((c ^ (row & 7)) << 4));
+        for (int k = 0; k < topk; k++) {
+            const int s = slot[(size_t)row * 8 + k];
+            *reinterpret_cast<uint4*>(out + ((size_t)kb * out_rows + s) * 128 + ((c ^ (s & 7)) << 4)) = v;
+        }
+    }
+}
+
+// Weighted sum of a token's expert outputs (ascending expert id, then the shared expert), stored or added.
+__global__ void __launch_bounds__(256) combine_rows(const float* y, int N, const int* slot, const float* weight, int topk, const float* shared, const float* gate,
+                                                    int add, float* out, long long out_stride) {
+    const int row = blockIdx.x;
+    for (int c = threadIdx.x * 4; c < N; c += 1024) {
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < topk; k++) {
+            const float w = weight[(size_t)row * 8 + k];
+            const float4 v = *reinterpret_cast<const float4*>(y + (size_t)slot[(size_t)row * 8 + k] * N + c);
+            s.x = fmaf(v.x, w, s.x); s.y = fmaf(v.y, w, s.y); s.z = fmaf(v.z, w, s.z); s.w = fmaf(v.w, w, s.w);
+        }
+        if (shared) {
+            const float w = gate[row];
+            const float4 v = *reinterpret_cast<const float4*>(shared + (size_t)row * N + c);
+            s.x = fmaf(v.x, w, s.x); s.y = fmaf(v.y, w, s.y); s.z = fmaf(v.z, w, s.z); s.w = fmaf(v.w, w, s.w);
+        }
+        float4* o = reinterpret_cast<float4*>(out + (size_t)row * out_stride + c);
+        if (add) {
+            const float4 b = *o;
+            s.x += b.x; s.y += b.y; s.z += b.z; s.w += b.w;
+        }
+        *o = s;
+    }
+}
+
+}  // namespace mkp

@@ -192,13 +192,15 @@ class Engine:
         return out
 
     def prefill(self, prompts):
-        """Feeds the prompts (M lists of equal length) position by position in ONE launch and returns the logits
-        after the last position: what the reference does with one `step` per position (`mk/reference.py:378-386`)."""
+        """Takes the prompts (M lists of equal length) in and returns the logits after the last position: what the
+        reference does with one `step` per position (`mk/reference.py:378-386`).  All positions but the last go through
+        the token-parallel path (`Runtime.prefill`), the last one and short prompts through the decode kernel."""
         if len(prompts) != self.M or len({len(p) for p in prompts}) != 1 or not prompts[0]:
             raise ValueError(f"prefill takes {self.M} prompts of one common, non-zero length")
         toks = torch.tensor(prompts, dtype=torch.int32).t().contiguous().to(self.device)      # [L, M]
-        self.rt.tok[: self.M].copy_(toks[0])
-        self.rt.launch(toks.shape[0], tokens_in=toks)
+        taken = self.rt.prefill(toks)                        # all positions at once, but the last
+        self.rt.tok[: self.M].copy_(toks[taken])
+        self.rt.launch(toks.shape[0] - taken, tokens_in=toks[taken:])
         self._prompt = toks                                  # alive until the launch has run
         return self.logits
 

@@ -58,7 +58,14 @@ class StageArgs(ctypes.Structure):
                 ("row_valid", ctypes.c_uint64)]
 
 
-STAGE_EXPORTS = ["mk_stage_launch", "mk_stage_validate", "mk_stage_count", "mk_stage_query", "mk_stage_scratch_bytes", "mk_sync_probe", "mk_peer_alloc", "mk_peer_open",
+class PrefillArgs(ctypes.Structure):
+    _fields_ = [("program", ctypes.c_uint64), ("n_stages", ctypes.c_int32), ("batch", ctypes.c_int32),
+                ("positions", ctypes.c_int32), ("device", ctypes.c_int32), ("tokens", ctypes.c_uint64), ("pos", ctypes.c_uint64),
+                ("status", ctypes.c_uint64), ("workspace", ctypes.c_uint64), ("workspace_bytes", ctypes.c_int64),
+                ("spin_limit_ns", ctypes.c_int64)]
+
+
+STAGE_EXPORTS = ["mk_stage_launch", "mk_stage_prefill", "mk_stage_prefill_bytes", "mk_stage_validate", "mk_stage_count", "mk_stage_query", "mk_stage_scratch_bytes", "mk_sync_probe", "mk_peer_alloc", "mk_peer_open",
                  "mk_peer_close", "mk_peer_free"]
 STAGE_QUERIES = ["SMEM_BYTES", "N_THREADS", "SLOT_BYTES", "XS_BYTES", "DESC_BYTES", "MAX_GROUPS", "MAILBOX_BYTES", "ATTN_MAX_CHUNK"]
 
@@ -72,6 +79,9 @@ def lib():
     if not _bound:
         P = ctypes.POINTER
         L.mk_stage_launch.argtypes = [P(StageArgs), ctypes.c_void_p]
+        L.mk_stage_prefill.argtypes = [P(PrefillArgs), ctypes.c_void_p]
+        L.mk_stage_prefill_bytes.argtypes = [P(StageDesc), ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int]
+        L.mk_stage_prefill_bytes.restype = ctypes.c_int64
         L.mk_stage_validate.argtypes = [P(StageDesc), ctypes.c_int, ctypes.c_int]
         L.mk_stage_count.argtypes = [P(StageDesc), ctypes.c_int, P(ctypes.c_int64), P(ctypes.c_int64)]
         L.mk_stage_query.argtypes = [ctypes.c_int]
@@ -84,7 +94,7 @@ def lib():
         L.mk_peer_close.argtypes = [ctypes.c_uint64]
         L.mk_peer_free.argtypes = [ctypes.c_uint64]
         for name in STAGE_EXPORTS:
-            if name not in ("mk_stage_query", "mk_stage_scratch_bytes"):
+            if name not in ("mk_stage_query", "mk_stage_scratch_bytes", "mk_stage_prefill_bytes"):
                 getattr(L, name).restype = ctypes.c_int
         _bound = True
     return L

@@ -15,6 +15,16 @@ from . import desc as D
 from . import pack as P
 
 
+# Prompts shorter than this go through the decode kernel position by position, bit for bit what `step` computes.  The
+# token-parallel path is faster from two or three positions on (it passes over the weights once); the line lies a little
+# higher so that a handful of tokens appended to a conversation rounds like generated ones.
+MIN_ROWS_PATH = 12
+# Token rows (sequences x positions) of one pass of the token-parallel path: large enough that the tensor cores, not the
+# weight stream, bound a pass (4096 rows: about 8000 operations per weight byte), small enough that its workspace stays
+# near a gigabyte for the widest model.
+MAX_ROWS = 4096
+
+
 class Program:
     """Stage records plus everything that must stay alive while they are used."""
 
@@ -145,7 +155,7 @@ class Runtime:
         self.prog = program
         dev = program.device
         self.device, self.M, self.grid = dev, program.batch, program.grid
-        host = program.host_array()
+        host = self.host = program.host_array()
         _lib.check(self.lib.mk_stage_validate(host, len(program.stages), self.M))
         nb, na = ctypes.c_int64(), ctypes.c_int64()
         _lib.check(self.lib.mk_stage_count(host, len(program.stages), ctypes.byref(nb), ctypes.byref(na)))
@@ -162,6 +172,7 @@ class Runtime:
         self.tp, self.rank, self.mailbox = tp, rank, mailbox
         self.spin_limit_ns = int(spin_limit_ms * 1e6)
         self.launches = 0
+        self._workspace = None          # of the token-parallel prompt path, grown to the largest pass so far
 
     def reset(self):
         self.pos.zero_()
@@ -195,6 +206,32 @@ class Runtime:
         self.bar_base += nb * n_steps * self.grid
         self.ar_base += na * n_steps
         self.launches += 1
+
+    def prefill(self, tokens):
+        """Takes in all positions of `tokens` (int32 [L, M] on the device) but the last through the token-parallel path, in
+        passes of at most MAX_ROWS rows, and returns how many: 0 for a short prompt or a program that path cannot run
+        (two-piece inputs, tensor parallelism).  The caller feeds the rest to `launch`."""
+        todo = tokens.shape[0] - 1
+        if todo < MIN_ROWS_PATH - 1 or self.tp > 1:
+            return 0
+        passes = -(-todo * self.M // MAX_ROWS)
+        each = -(-todo // passes)
+        need = int(self.lib.mk_stage_prefill_bytes(self.host, self.n_stages, self.M, each, self.device.index))
+        if need == _lib.MK_ERR_UNSUPPORTED:
+            return 0
+        if need < 0:
+            _lib.check(need)
+        if self._workspace is None or self._workspace.numel() < need:
+            self._workspace = None
+            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        for lo in range(0, todo, each):
+            part = tokens[lo: min(lo + each, todo)]
+            a = D.PrefillArgs(program=ctypes.addressof(self.host), n_stages=self.n_stages, batch=self.M, positions=part.shape[0],
+                              device=self.device.index, tokens=part.data_ptr(), pos=self.pos.data_ptr(), status=self.status.data_ptr(),
+                              workspace=self._workspace.data_ptr(), workspace_bytes=self._workspace.numel(), spin_limit_ns=self.spin_limit_ns)
+            _lib.check(self.lib.mk_stage_prefill(ctypes.byref(a), ctypes.c_void_p(stream)))
+        return todo
 
     def check(self):
         """Synchronise and raise if a device-side wait ran out in any launch so far."""

@@ -1,0 +1,81 @@
+"""The token-parallel prompt path against the decode kernel that steps through the same prompt.
+
+The first layer's recurrent state sees no earlier bf16 rounding, so there the two must agree to fp32 sums; behind it
+roundings of GEMV inputs flip, so logits and states are held to the bars the decode tests use.  Lengths: the shortest
+this path takes, one row short of / past a 16-row tile and a 256-row tile, several passes, and a start behind a context."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from megakernels_b200 import gemma26b, qwen27b, qwen35moe
+from megakernels_b200.gemma26b.dims import FULL as FULL26
+from megakernels_b200.qwen27b.dims import FULL as FULL27
+from megakernels_b200.qwen35moe.dims import FULL as FULL35
+from megakernels_b200.stage import runtime
+
+SHAPES = {
+    "27b": (qwen27b, FULL27.with_(hidden=1024, ffn=2048, vocab=4096, layers=4, nkh=4, nvh=12, nq=8, nkv=2)),
+    "35b": (qwen35moe, FULL35.with_(hidden=1024, vocab=4096, layers=4, nkh=4, nvh=8, nq=8, nkv=2, fi=128, sfi=128)),
+    "26b": (gemma26b, FULL26.with_(hidden=512, vocab=4096, layers=6, ffn=256, experts=128, eff=128, window=64)),
+}
+CASES = [("27b", {}, 1, 12, 0), ("27b", {}, 1, 258, 0), ("27b", {}, 3, 86, 37), ("27b", {"fmt": "bf16"}, 2, 41, 0),
+         ("35b", {}, 1, 18, 0), ("35b", {}, 2, 129, 21), ("26b", {}, 1, 17, 0), ("26b", {}, 3, 150, 21)]
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+@pytest.fixture(scope="module")
+def packed():
+    made = {}
+
+    def get(model, fmt):
+        key = (model, tuple(fmt.items()))
+        if key not in made:
+            pkg, shape = SHAPES[model]
+            made[key] = pkg.Packed(pkg.SynthWeights(shape, layers=shape.layers, init="realistic", device="cuda", **fmt), "cuda")
+        return made[key]
+    return get
+
+
+@pytest.mark.parametrize("model,fmt,M,length,context", CASES)
+def test_prompt_rows_equal_stepping(packed, monkeypatch, model, fmt, M, length, context):
+    pkg, shape = SHAPES[model]
+    prompts = [pkg.make_prompt(shape.vocab, context + length, seed=j) for j in range(M)]
+    engines = []
+    for rows in (True, False):
+        eng = pkg.Engine(packed(model, fmt), M, maxlen=context + length + 64)
+        for p in range(context):
+            eng.step(torch.tensor([q[p] for q in prompts], device="cuda"))
+        with monkeypatch.context() as mp:
+            mp.setattr(runtime, "MAX_ROWS", 200)            # several passes for the longer prompts
+            if not rows:
+                mp.setattr(runtime, "MIN_ROWS_PATH", 1 << 30)
+            launches = eng.rt.launches
+            logits = eng.prefill([q[context:] for q in prompts]).clone()
+            assert eng.rt.launches == launches + 1
+        eng.check()
+        engines.append((eng, logits))
+    (a, la), (b, lb) = engines
+    assert a.pos[:M].tolist() == b.pos[:M].tolist() == [context + length] * M
+    assert rel(la, lb) < 3e-2
+    if model == "26b":
+        assert rel(a.ks[0], b.ks[0]) < 1e-3 and rel(a.vs[0], b.vs[0]) < 1e-3
+        assert rel(a.kf, b.kf) < 3e-2 and rel(a.vf, b.vf) < 3e-2
+    else:
+        assert rel(a.ssm[0], b.ssm[0]) < 2e-4 and rel(a.ssm, b.ssm) < 1e-2 and rel(a.conv, b.conv) < 1e-2
+        assert rel(a.k_cache, b.k_cache) < 2e-2 and rel(a.v_cache, b.v_cache) < 2e-2
+
+
+def test_programs_without_the_row_path_step(packed):
+    pkg, shape = SHAPES["35b"]
+    eng = pkg.Engine(packed("35b", {}), 1, maxlen=64, exact_inputs=True)
+    prompt = pkg.make_prompt(shape.vocab, 20, seed=3)
+    got = eng.prefill([prompt]).clone()
+    eng.reset()
+    for t in prompt:
+        want = eng.step(torch.tensor([t], device="cuda"))
+    assert torch.equal(got, want)
