@@ -214,6 +214,24 @@ typedef struct mk_batch_args {
 } mk_batch_args;
 int mk_launch_batch(mk_engine* e, const mk_batch_args* args, void* stream);
 
+/* A prompt, all positions at once: leaves in the states, conv histories and KV cache what feeding `positions` tokens one
+ * by one leaves (to fp32 rounding), computed as matrix products over the positions (tcgen05) instead of one pass over
+ * the weights per token.  No LM head: feed the prompt's last token to mk_launch / mk_launch_batch.  The reference feeds
+ * a prompt token by token inside its kernel (qwen3.5-0.8b/qwen_mk/engine.py:296-301). */
+typedef struct mk_prefill_args {
+    uint64_t tokens;         /* int32[positions] in device memory                                  */
+    int32_t positions;
+    int32_t start_pos;       /* position of the first token                                        */
+    int32_t sequence;        /* which of the engine's sequences (0 for single-sequence launches)   */
+    int32_t batched;         /* 1: for mk_launch_batch (MK_L_CONV_HIST_B), 0: for mk_launch        */
+    uint64_t resid_out;      /* optional fp32 [positions, hidden]: residual after the last layer   */
+    uint64_t workspace;      /* device scratch of mk_prefill_bytes                                 */
+    int64_t workspace_bytes;
+    int64_t spin_limit_ns;   /* bound on every device-side wait; 0 = 2 s                           */
+} mk_prefill_args;
+int mk_prefill(mk_engine* e, const mk_prefill_args* args, void* stream);
+int64_t mk_prefill_bytes(int positions);
+
 /* Replaces `watchdog_fired` (qwen3.5-0.8b/csrc/megakernel.cu:1284-1289): synchronises the device,
  * reads the status words of the last launch and returns MK_OK or MK_ERR_TIMEOUT.  Unlike the
  * reference, waits are bounded in every build, not only with -DMK_WATCHDOG. */

@@ -27,7 +27,7 @@ GLOBAL_FIELDS = ["embed", "embed_scale", "lm_head", "lm_scale", "final_norm", "r
 QUERIES = ["SMEM_BYTES", "N_THREADS", "CONV_RING", "KV_BLOCK", "MAX_SPLITS", "PART_STRIDE", "OPS_PER_LAYER",
            "PROF_MAX_OPS", "PROF_FIELDS", "SPEC_T", "MAX_LAYERS", "LAYER_FIELDS", "GLOBAL_FIELDS", "SLOT_BYTES",
            "STAGES", "MAX_LM_ROWS", "MAX_BATCH", "BATCH_SMEM_BYTES"]
-EXPORTS = ["mk_create", "mk_destroy", "mk_set_params", "mk_launch", "mk_launch_static", "mk_launch_batch", "mk_status", "mk_query", "mk_bw_probe",
+EXPORTS = ["mk_create", "mk_destroy", "mk_set_params", "mk_launch", "mk_launch_static", "mk_launch_batch", "mk_prefill", "mk_prefill_bytes", "mk_status", "mk_query", "mk_bw_probe",
            "mk_plan_rows", "mk_plan_attn_chunk", "mk_last_error"]
 
 
@@ -67,6 +67,12 @@ class BatchArgs(ctypes.Structure):
                 ("out_info", ctypes.c_uint64), ("prof", ctypes.c_uint64), ("spin_limit_ns", ctypes.c_int64)]
 
 
+class PrefillArgs(ctypes.Structure):
+    _fields_ = [("tokens", ctypes.c_uint64), ("positions", ctypes.c_int32), ("start_pos", ctypes.c_int32),
+                ("sequence", ctypes.c_int32), ("batched", ctypes.c_int32), ("resid_out", ctypes.c_uint64),
+                ("workspace", ctypes.c_uint64), ("workspace_bytes", ctypes.c_int64), ("spin_limit_ns", ctypes.c_int64)]
+
+
 _lib = None
 
 
@@ -87,6 +93,9 @@ def load():
     lib.mk_launch.argtypes = [ctypes.c_void_p, P(LaunchArgs), ctypes.c_void_p]
     lib.mk_launch_static.argtypes = [ctypes.c_void_p, P(LaunchArgs), ctypes.c_void_p]
     lib.mk_launch_batch.argtypes = [ctypes.c_void_p, P(BatchArgs), ctypes.c_void_p]
+    lib.mk_prefill.argtypes = [ctypes.c_void_p, P(PrefillArgs), ctypes.c_void_p]
+    lib.mk_prefill_bytes.argtypes = [ctypes.c_int]
+    lib.mk_prefill_bytes.restype = ctypes.c_int64
     lib.mk_status.argtypes = [ctypes.c_void_p, P(ctypes.c_int32)]
     lib.mk_query.argtypes = [ctypes.c_int]
     lib.mk_query.restype = ctypes.c_int64
@@ -96,7 +105,7 @@ def load():
     lib.mk_plan_attn_chunk.argtypes = [ctypes.c_int, ctypes.c_int]
     lib.mk_plan_attn_chunk.restype = ctypes.c_int
     lib.mk_last_error.restype = ctypes.c_char_p
-    for name in ("mk_create", "mk_destroy", "mk_set_params", "mk_launch", "mk_launch_static", "mk_launch_batch", "mk_status", "mk_bw_probe", "mk_plan_rows"):
+    for name in ("mk_create", "mk_destroy", "mk_set_params", "mk_launch", "mk_launch_static", "mk_launch_batch", "mk_prefill", "mk_status", "mk_bw_probe", "mk_plan_rows"):
         getattr(lib, name).restype = ctypes.c_int
     _lib = lib
     return lib

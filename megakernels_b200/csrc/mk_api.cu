@@ -36,6 +36,13 @@ int mk_set_error(int code, const char* text) {
     snprintf(g_err, sizeof g_err, "%s", text);
     return code;
 }
+// the library's other translation units see an engine through this
+int mk_engine_view(mk_engine* e, const mk_model_desc** desc, const Params** params) {
+    if (!e->params_set) return MK_ERR_BADARG;
+    *desc = &e->desc;
+    *params = &e->host;
+    return MK_OK;
+}
 #define MK_CUDA(call)                                                                      \
     do {                                                                                   \
         cudaError_t err__ = (call);                                                        \

@@ -4,96 +4,13 @@
 // the kernels of mk_prefill.cuh.  The program's per-step activation buffers ([M][width]) become arrays of M x L rows in
 // the caller's workspace; weights, states and caches are used where they are.  Everything the LM head needs is left to
 // one ordinary decode step with the prompt's last token, so the caller sees exactly what stepping through would leave.
-#include <cstdarg>
-#include <cstdio>
-#include <cstring>
 #include <vector>
 
-#include "../../include/mk_b200.h"
-#include "mk_prefill.cuh"
+#include "mk_prefill_host.h"
 
 using namespace mkp;
 
-int mk_set_error(int code, const char* text);
-
 namespace {
-
-int pfail(int code, const char* fmt, ...) {
-    char buf[512];
-    va_list ap;
-    va_start(ap, fmt);
-    vsnprintf(buf, sizeof buf, fmt, ap);
-    va_end(ap);
-    return mk_set_error(code, buf);
-}
-#define MKP_CUDA(call)                                                                      \
-    do {                                                                                    \
-        cudaError_t err__ = (call);                                                         \
-        if (err__ != cudaSuccess)                                                           \
-            return pfail(MK_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(err__));   \
-    } while (0)
-
-constexpr int SMEM_MAX = 232448;
-
-// Hands out the workspace; with base == nullptr it only counts.
-struct Arena {
-    uint8_t* base;
-    size_t off = 0;
-    template <class T>
-    T* take(size_t n) {
-        off = (off + 1023) & ~(size_t)1023;
-        T* p = base ? reinterpret_cast<T*>(base + off) : nullptr;
-        off += n * sizeof(T);
-        return p;
-    }
-};
-
-template <int FMT, int PX>
-int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaStream_t st) {
-    constexpr int PW = FMT == W_FP8_BLOCK ? 2 : 1;
-    const int stage = PW * A_BYTES + PX * A.nt * 128, fixed = (int)sizeof(GemmBars) + 1024;
-    // two CTAs per SM while both keep three stages, else one with as many as fit
-    int stages = (SMEM_MAX / 2 - 1024 - fixed) / stage;
-    if (stages < 3) stages = (SMEM_MAX - fixed) / stage;
-    if (stages > 6) stages = 6;
-    if (stages < 2) return pfail(MK_ERR_BADARG, "prefill: %d tokens per tile leave no room for two stages", A.nt);
-    A.stages = stages;
-    const int smem = stages * stage + fixed;
-    auto fn = out == OUT_STORE ? rows_gemm<FMT, PX, OUT_STORE> : (out == OUT_ADD ? rows_gemm<FMT, PX, OUT_ADD> : rows_gemm<FMT, PX, OUT_GLU>);
-    MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const dim3 grid = items ? dim3(blocks, items, 1) : dim3(tiles_x, blocks, A.ksplit);
-    fn<<<grid, GEMM_THREADS, smem, st>>>(A);
-    MKP_CUDA(cudaGetLastError());
-    if (A.ksplit > 1) {
-        const dim3 fgrid(out == OUT_GLU ? (A.act_cols + 255) / 256 : (A.n_valid + 1023) / 1024, A.rows);
-        if (out == OUT_STORE) rows_finish<PX, OUT_STORE><<<fgrid, 256, 0, st>>>(A);
-        else if (out == OUT_ADD) rows_finish<PX, OUT_ADD><<<fgrid, 256, 0, st>>>(A);
-        else rows_finish<PX, OUT_GLU><<<fgrid, 256, 0, st>>>(A);
-        MKP_CUDA(cudaGetLastError());
-    }
-    return MK_OK;
-}
-
-// Token tiles of `rows` rows: equal tiles of at most 256, multiples of 16.
-void token_tiles(int rows, int* n, int* nt) {
-    *n = (rows + 255) / 256;
-    *nt = ((rows + *n - 1) / *n + 15) / 16 * 16;
-}
-
-// CTAs that share the K range of one tile: the count with the shortest schedule (rounds of one CTA per SM, each 64-column
-// block counted once and the start and end of a CTA as six), at least eight blocks each.
-int pick_ksplit(int ctas, int kbs, int sms) {
-    int best = 1;
-    double cost = 1e30;
-    for (int z = 1; z <= 8 && (z == 1 || kbs / z >= 8); z++) {
-        const double c = (double)((ctas * z + sms - 1) / sms) * ((kbs + z - 1) / z + 6) + (z > 1 ? 4 + z : 0);
-        if (c < cost) {
-            cost = c;
-            best = z;
-        }
-    }
-    return best;
-}
 
 struct Buffer { uint64_t base; int width; float* rows; };
 struct Slab { uint64_t key; const void* norm; float in_scale; uint8_t* x; int rows, width; };
@@ -115,7 +32,7 @@ struct Exec {
     float* part = nullptr;
     size_t part_floats = 0;
     // DeltaNet / attention / routing scratch
-    float *qkv = nullptr, *o = nullptr;
+    float *qkv = nullptr, *o = nullptr, *gram = nullptr;
     float4* scal = nullptr;
     __nv_bfloat16* q = nullptr;
     RouteArgs route;
@@ -192,7 +109,7 @@ struct Exec {
         }
         for (auto& b : bufs) b.rows = arena.take<float>((size_t)rows * b.width);
         int kmax = 0, experts = 0, topk = 0;
-        size_t conv = 0, heads = 0, vals = 0, q_w = 0, ex_k = 0, ex_n = 0, ex_f = 0, sh = 0;
+        size_t conv = 0, heads = 0, kheads = 0, vals = 0, q_w = 0, ex_k = 0, ex_n = 0, ex_f = 0, sh = 0;
         for (int s = 0; s < n_stages; s++) {
             const mk_stage_desc& d = prog[s];
             auto up = [](size_t& a, size_t b) { if (b > a) a = b; };
@@ -215,6 +132,7 @@ struct Exec {
             } else if (d.op == MKS_OP_GDN) {
                 up(conv, d.i[MKS_I_CONV_DIM]);
                 up(heads, d.i[MKS_I_NVH]);
+                up(kheads, d.i[MKS_I_NKH]);
                 need_slab(d.p[MKS_P_Y2], d.i[MKS_I_NVH] * 128);
             } else if (d.op == MKS_OP_ATTN) {
                 up(q_w, (size_t)d.i[MKS_I_NQ] * d.i[MKS_I_HD]);
@@ -232,6 +150,7 @@ struct Exec {
             qkv = arena.take<float>((size_t)rows * conv);
             scal = arena.take<float4>((size_t)rows * heads);
             o = arena.take<float>((size_t)rows * vals);
+            gram = arena.take<float>((size_t)M * ((L + SCAN - 1) / SCAN) * kheads * 64);
         }
         if (q_w) q = arena.take<__nv_bfloat16>((size_t)rows * q_w);
         if (experts) {
@@ -406,23 +325,19 @@ struct Exec {
         G.pos = pos;
         G.conv_bf16 = d.i[MKS_I_CONV_BF16];
         G.l2_clamp = d.i[MKS_I_L2_CLAMP];
-        G.eps = d.f[MKS_F_EPS];
+        G.eps = G.norm_eps = d.f[MKS_F_EPS];
         G.qkv = qkv; G.scal = scal; G.o = o;
         Slab* s = slab(d.p[MKS_P_Y2]);
         G.out = s->x;
         G.out_rows = s->rows;
-        gdn_conv<<<dim3((G.conv_dim / 128 + 7) / 8, rows), 256, 0, st>>>(G);
-        gdn_history<<<dim3((G.conv_dim + 255) / 256, M), 256, 0, st>>>(G);
-        gdn_scan<<<dim3(4, G.nvh, M), 256, 0, st>>>(G);
-        gdn_gate<1><<<dim3((G.nvh + 15) / 16, rows), 256, 0, st>>>(G);
-        MKP_CUDA(cudaGetLastError());
-        return MK_OK;
+        G.gram = gram;
+        return launch_gdn(G, gdn_gate<1>, sms, st);
     }
 
     template <int HD>
     int attn_hd(const AttnArgs& T) {
         const int bq = AT_ROWS / (T.nq / T.nkv);
-        attn_prepare<HD><<<dim3((T.nq + 2 * T.nkv + 7) / 8, rows), 256, 0, st>>>(T);
+        attn_prepare<HD, false, false><<<dim3((T.nq + 2 * T.nkv + 7) / 8, rows), 256, 0, st>>>(T);
         MKP_CUDA(cudaFuncSetAttribute(attn_rows<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem<HD>()));
         attn_rows<HD><<<dim3((L + bq - 1) / bq, T.nkv, M), 256, attn_smem<HD>(), st>>>(T);
         MKP_CUDA(cudaGetLastError());

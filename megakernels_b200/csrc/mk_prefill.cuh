@@ -75,6 +75,7 @@ struct GemmArgs {
     int w_rows;                  // W_SLAB: rows per slab
     const float* row_scale;      // per weight row, or null
     size_t rs_gstride;
+    int rs_pairs;                // OUT_GLU: the scales alternate gate, up (the 0.8B layout) instead of following the tiles
     // token operand
     const uint8_t* x;
     size_t x_piece;              // bytes between its pieces
@@ -101,7 +102,6 @@ struct GemmArgs {
     long long spin_limit_ns;
 };
 
-constexpr int CONV_WARPS = 8, GEMM_THREADS = (CONV_WARPS + 2) * 32;
 constexpr int A_BYTES = 128 * 128;                     // one 64-column block of 128 weight rows
 constexpr int MAX_STAGES = 8;
 struct GemmBars {
@@ -110,7 +110,7 @@ struct GemmBars {
     volatile int dead;
 };
 
-__device__ __noinline__ bool wait_slow(GemmBars& B, const GemmArgs& A, uint64_t* b, uint32_t parity, int site) {
+static __device__ __noinline__ bool wait_slow(GemmBars& B, const GemmArgs& A, uint64_t* b, uint32_t parity, int site) {
     u64 t0 = 0;
 #pragma unroll 1
     for (unsigned it = 0;; it++) {
@@ -170,35 +170,50 @@ template <int FMT> struct Raw { uint4 q[FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 
 template <int FMT>
 struct Walk {
     static constexpr int STEPS = FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2);      // 512-byte steps per 64 columns
-    const uint8_t* p;          // the current chunk
-    int within, st;            // step inside the chunk, step inside the unit
-    __device__ __forceinline__ void start(const GemmArgs& A, const uint8_t* w, int tile, int kb) {
+    const uint8_t *p, *s;      // this lane's bytes of the next step; the current chunk's scales
+    int left, st;              // steps left in the chunk and in the unit
+    __device__ __forceinline__ void start(const GemmArgs& A, const uint8_t* w, int tile, int kb, int lane) {
         constexpr int STEP_K = 64 / STEPS;
-        const int split = kb * 64 / A.kc;
-        st = (kb * 64 - split * A.kc) / STEP_K;
+        const int split = kb * 64 / A.kc, at = (kb * 64 - split * A.kc) / STEP_K;
         const size_t unit = (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
-        within = st % A.chunk_steps;
-        p = w + ((size_t)split * A.tiles + tile) * unit + (size_t)(st / A.chunk_steps) * A.chunk_bytes;
+        const int within = at % A.chunk_steps;
+        const uint8_t* chunk = w + ((size_t)split * A.tiles + tile) * unit + (size_t)(at / A.chunk_steps) * A.chunk_bytes;
+        st = A.unit_steps - at;
+        left = A.chunk_steps - within;
+        p = chunk + within * 512 + lane * 16;
+        s = chunk + A.chunk_steps * 512 + (FMT == W_MXFP4 ? within * 32 + (lane >> 2) * 4 : (within >> 2) * 8);
     }
-    __device__ __forceinline__ void load(const GemmArgs& A, int lane, Raw<FMT>& r) {
-        if (FMT == W_MXFP4) r.s[0] = __ldg(reinterpret_cast<const uint32_t*>(p + A.chunk_steps * 512 + within * 32 + (lane >> 2) * 4));
+    __device__ __forceinline__ void load(const GemmArgs& A, Raw<FMT>& r) {
+        if (FMT == W_MXFP4) r.s[0] = __ldg(reinterpret_cast<const uint32_t*>(s));
         if (FMT == W_FP8_BLOCK) {
-            const uint2 s = __ldg(reinterpret_cast<const uint2*>(p + A.chunk_steps * 512 + (within >> 2) * 8));
-            r.s[0] = s.x;
-            r.s[FMT == W_FP8_BLOCK ? 1 : 0] = s.y;
+            const uint2 x = __ldg(reinterpret_cast<const uint2*>(s));
+            r.s[0] = x.x;
+            r.s[FMT == W_FP8_BLOCK ? 1 : 0] = x.y;
         }
 #pragma unroll
         for (int i = 0; i < STEPS; i++) {
-            r.q[i] = __ldg(reinterpret_cast<const uint4*>(p + within * 512) + lane);
-            st++;
-            if (++within == A.chunk_steps) {
-                within = 0;
-                p += A.chunk_bytes;
-            }
+            r.q[i] = __ldg(reinterpret_cast<const uint4*>(p));
+            step(A);
         }
-        if (st == A.unit_steps) {          // the same tile of the next split
-            st = 0;
-            p += (size_t)(A.tiles - 1) * (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
+    }
+    __device__ __forceinline__ void skip(const GemmArgs& A) {
+#pragma unroll
+        for (int i = 0; i < STEPS; i++) step(A);
+    }
+    __device__ __forceinline__ void step(const GemmArgs& A) {
+        p += 512;
+        if (FMT == W_MXFP4) s += 32;
+        if (FMT == W_FP8_BLOCK && (left & 3) == 1) s += 8;
+        if (--left == 0) {
+            left = A.chunk_steps;
+            p += A.chunk_bytes - A.chunk_steps * 512;
+            s += A.chunk_bytes - (FMT == W_MXFP4 ? A.chunk_steps * 32 : A.chunk_steps * 2);
+        }
+        if (--st == 0) {                   // the same tile of the next split
+            st = A.unit_steps;
+            const size_t jump = (size_t)(A.tiles - 1) * (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
+            p += jump;
+            s += jump;
         }
     }
 };
@@ -215,14 +230,15 @@ __device__ __forceinline__ void convert(const Raw<FMT>& r, uint2 (&v)[2][4], uin
             v[1][j] = make_uint2(r.q[j].z, r.q[j].w);
         }
     } else if constexpr (FMT == W_MXFP4) {
+        const uint32_t sc = r.s[0] & 0x7F7F7F7Fu;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             // scale group 0 (j = 0, 1): bits pre-arranged by the packer; three magnitude bits at 8..6 of a half are the
             // value times 2^-126.  Group 1 (j = 2, 3): plain nibbles, through f16: the value times 2^-112.
             const uint32_t w = h == 0 ? r.q[0].x : r.q[0].z, n = h == 0 ? r.q[0].y : r.q[0].w;
-            const uint32_t s0 = (r.s[0] >> (16 * h)) & 0xFFu, s1 = (r.s[0] >> (16 * h + 8)) & 0xFFu;
-            const uint32_t f0 = (min(s0, 128u) + 126u) << 7, f1 = (min(s1, 142u) + 112u) << 7;     // 2^(s - 1), 2^(s - 15)
-            const uint32_t m0 = f0 | (f0 << 16), m1 = f1 | (f1 << 16);
+            // factors 2^(s - 1) and 2^(s - 15) in both halves: the scale byte moved to the exponent field, plus a constant
+            const uint32_t m0 = __byte_perm(sc, 0u, h == 0 ? 0x4040 : 0x4242) * 128u + 0x3F003F00u;
+            const uint32_t m1 = __byte_perm(sc, 0u, h == 0 ? 0x4141 : 0x4343) * 128u + 0x38003800u;
             v[h][0].x = mul_bf16x2((w & 0x80008000u) | ((w >> 3) & 0x01C001C0u), m0);
             v[h][0].y = mul_bf16x2(((w << 3) & 0x80008000u) | (w & 0x01C001C0u), m0);
             v[h][1].x = mul_bf16x2(((w << 1) & 0x80008000u) | ((w << 3) & 0x01C001C0u), m0);
@@ -231,15 +247,16 @@ __device__ __forceinline__ void convert(const Raw<FMT>& r, uint2 (&v)[2][4], uin
             v[h][2].y = mul_bf16x2(f16_as_bf16(e2m1x2_f16(n >> 8)), m1);
             v[h][3].x = mul_bf16x2(f16_as_bf16(e2m1x2_f16(n >> 16)), m1);
             v[h][3].y = mul_bf16x2(f16_as_bf16(e2m1x2_f16(n >> 24)), m1);
-            if (s0 > 128u || s1 > 142u) {          // weights beyond +-12: the factors above would leave the range of a bf16
-                const uint32_t g0 = (127u + (s0 > 128u ? s0 - 128u : 0u)) << 7, g1 = (127u + (s1 > 142u ? s1 - 142u : 0u)) << 7;
+        }
+        if (r.s[0] & 0x80808080u) {            // scales of 2 and more: the top bit is worth 2^128, twice 2^64
+#pragma unroll
+            for (int h = 0; h < 2; h++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const uint32_t m = j < 2 ? (g0 | (g0 << 16)) : (g1 | (g1 << 16));
-                    v[h][j].x = mul_bf16x2(v[h][j].x, m);
-                    v[h][j].y = mul_bf16x2(v[h][j].y, m);
+                    const uint32_t m = (r.s[0] >> (16 * h + 8 * (j >> 1) + 7)) & 1u ? 0x5F805F80u : 0x3F803F80u;
+                    v[h][j].x = mul_bf16x2(mul_bf16x2(v[h][j].x, m), m);
+                    v[h][j].y = mul_bf16x2(mul_bf16x2(v[h][j].y, m), m);
                 }
-            }
         }
     } else {
         constexpr uint32_t UP = 0x77807780u;       // 2^112
@@ -264,34 +281,37 @@ __device__ __forceinline__ void convert(const Raw<FMT>& r, uint2 (&v)[2][4], uin
     }
 }
 
-// Writes a lane's share of tile `tile` into the swizzled operand.  Lanes of odd rows store their columns in the order
+// Writes a lane's share of a tile into the swizzled operand.  Lanes of odd rows store their columns in the order
 // j = 2, 3, 0, 1: the sixteen 8-byte stores of a half warp then fall into different banks.
-__device__ __forceinline__ void store_operand(uint8_t* a, int tile, int lane, const uint2 (&v)[2][4]) {
-    const int g = lane >> 2, q = lane & 3;
-    const bool odd = g & 1;
+__device__ __forceinline__ void store_operand(uint8_t* a, const uint32_t (&off)[4], bool odd, const uint2 (&v)[2][4]) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        uint8_t* row = a + (size_t)(16 * tile + 8 * h + g) * 128 + (q & 1) * 8;
+    for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint2 x = odd ? v[h][i ^ 2] : v[h][i];
-            const int j = odd ? i ^ 2 : i;
-            *reinterpret_cast<uint2*>(row + (((2 * j + (q >> 1)) ^ g) << 4)) = x;
-        }
-    }
+        for (int i = 0; i < 4; i++) *reinterpret_cast<uint2*>(a + off[i] + h * 1024) = odd ? v[h][i ^ 2] : v[h][i];
+}
+// Sixteen accumulator columns of this lane's row.
+__device__ __forceinline__ void load16(uint32_t tmem, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(tmem));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // One CTA: 128 weight rows x nt token rows over a range of K.
-//   warps 0..7  convert weight tiles into the A operand, then read the accumulators back (epilogue);
-//   warp 8      one lane brings the token operand (and, for slab weights, the A operand) with bulk copies;
-//   warp 9      one lane issues the MMAs.
+//   warps 0 .. 8 CG - 1  CG groups of eight convert weight tiles into the A operand (group c takes every CG-th block of 64
+//                        columns, warp w of a group tile w), then read the accumulators back (epilogue);
+//   warp 8 CG            one lane brings the token operand (and, for slab weights, the A operand) with bulk copies;
+//   warp 8 CG + 1        one lane issues the MMAs.
 // grid: x = token tile (neighbouring CTAs share weights, so HBM reads them once), y = 128-row weight block, z = K split;
 // routed groups: x = weight block, y = work item.
 // PX: bf16 pieces of the token operand (3: fp32-exact inputs), weight pieces: 2 for block-scaled FP8, else 1.
-template <int FMT, int PX, int OUT>
-__global__ void __launch_bounds__(GEMM_THREADS, 2) rows_gemm(const __grid_constant__ GemmArgs A) {
+// Three-piece inputs keep the products of the first piece in an accumulator of their own: an accumulation rounds its sum
+// towards zero, and the small terms of pieces 2 and 3 would add two more such roundings per step to the large sum.
+template <int FMT, int PX, int OUT, int CG>
+static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) rows_gemm(const __grid_constant__ GemmArgs A) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    constexpr int PW = FMT == W_FP8_BLOCK ? 2 : 1;
+    constexpr int PW = FMT == W_FP8_BLOCK ? 2 : 1, CW = 8 * CG;
     constexpr int DIST = FMT == W_BF16 ? 2 : (FMT == W_MXFP4 ? 6 : 4);        // blocks a lane requests ahead
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -314,17 +334,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) rows_gemm(const __grid_consta
     const uint32_t x_bytes = (uint32_t)nt * 128u, stage_bytes = PW * A_BYTES + PX * (uint32_t)A.nt * 128u;
     GemmBars& B = *reinterpret_cast<GemmBars*>(smem + (size_t)A.stages * stage_bytes);
     int cols = 32;
-    while (cols < A.nt) cols *= 2;
+    while (cols < A.nt * (PX > 1 ? 2 : 1)) cols *= 2;
     if (threadIdx.x == 0) {
         for (int i = 0; i < A.stages; i++) {
-            mbar_init(&B.full[i], FMT == W_SLAB ? 1 : CONV_WARPS + 1);
+            mbar_init(&B.full[i], FMT == W_SLAB ? 1 : 8 + 1);
             mbar_init(&B.empty[i], 1);
         }
         mbar_init(&B.done, 1);
         B.dead = 0;
         mk::fence_barrier_init();
     }
-    if (warp == 9) {
+    if (warp == CW + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&B.tmem)), "r"(cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
@@ -333,12 +353,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) rows_gemm(const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = B.tmem;
 
-    if (warp == CONV_WARPS) {
+    if (warp == CW) {
         if (lane == 0) {
-            int i = 0;
             uint32_t slot = 0, phase = 0;
 #pragma unroll 1
-            for (int kb = kb0; kb < kb1; kb++, i++) {
+            for (int kb = kb0; kb < kb1; kb++) {
                 if (!wait(B, A, &B.empty[slot], phase ^ 1u, WP_EMPTY)) break;
                 uint8_t* st = smem + (size_t)slot * stage_bytes;
                 mbar_expect_tx(&B.full[slot], PX * x_bytes + (FMT == W_SLAB ? A_BYTES : 0));
@@ -361,10 +380,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) rows_gemm(const __grid_consta
                 while (mk::globaltimer() - t0 < 1000000ull) {}
             }
         }
-    } else if (warp == CONV_WARPS + 1) {
+    } else if (warp == CW + 1) {
         if (lane == 0) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | (8u << 24);   // f32 <- bf16 x bf16, M 128
-            uint32_t slot = 0, phase = 0, accumulate = 0;
+            uint32_t slot = 0, phase = 0, first = 1;
             bool ok = true;
 #pragma unroll 1
             for (int kb = kb0; kb < kb1; kb++) {
@@ -375,17 +394,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) rows_gemm(const __grid_consta
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t st = smem_u32(smem + (size_t)slot * stage_bytes);
 #pragma unroll
-                for (int pw = 0; pw < PW; pw++)
+                for (int px = 0; px < PX; px++)
 #pragma unroll
-                    for (int px = 0; px < PX; px++) {
+                    for (int pw = 0; pw < PW; pw++) {
                         const uint64_t da = operand_desc(st + pw * A_BYTES), db = operand_desc(st + PW * A_BYTES + px * (uint32_t)A.nt * 128u);
+                        const uint32_t d = tmem + (px ? (uint32_t)A.nt : 0u);
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
+                            const uint32_t accumulate = !(first && k == 0 && pw == 0 && px <= 1);
                             asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                                         ::"r"(tmem), "l"(da + 2 * k), "l"(db + 2 * k), "r"(idesc), "r"(accumulate));
-                            accumulate = 1;
+                                         ::"r"(d), "l"(da + 2 * k), "l"(db + 2 * k), "r"(idesc), "r"(accumulate));
                         }
                     }
+                first = 0;
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&B.empty[slot])) : "memory");
                 if (++slot == (uint32_t)A.stages) {
                     slot = 0;
@@ -397,100 +418,126 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) rows_gemm(const __grid_consta
     } else {
         if constexpr (FMT != W_SLAB) {
             // warp = tile: its bytes are requested DIST blocks ahead, straight into registers
-            const int tile = block * 8 + warp;
+            const int w8 = warp & 7, tile = block * 8 + w8, kb_first = kb0 + (warp >> 3);
             const bool have = tile < A.tiles;
-            Walk<FMT> walk;
-            walk.start(A, A.w + (size_t)group * A.w_gstride, min(tile, A.tiles - 1), kb0);
-            Raw<FMT> raw[DIST];
-            int asked = kb0;
+            if (!have)                       // rows past the matrix: zero in every slot, never written again
+                for (int i = lane; i < A.stages * 128; i += 32) {
+                    uint8_t* a = smem + (size_t)(i >> 7) * stage_bytes + (size_t)w8 * 2048 + (i & 127) * 16;
 #pragma unroll
-            for (int i = 0; i < DIST; i++)
-                if (asked < kb1) {
-                    walk.load(A, lane, raw[i]);
-                    asked++;
+                    for (int p = 0; p < PW; p++) *reinterpret_cast<uint4*>(a + p * A_BYTES) = make_uint4(0u, 0u, 0u, 0u);
                 }
-            uint32_t slot = 0, phase = 0;
+            const int g = lane >> 2, q = lane & 3;
+            // offsets of the lane's 8-byte pieces j = 0 .. 3 of a row: odd rows take j = 2, 3, 0, 1 (see store_operand)
+            uint32_t off[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) off[i] = (uint32_t)(w8 * 2048 + g * 128 + (q & 1) * 8) + (((2 * (g & 1 ? i ^ 2 : i) + (q >> 1)) ^ g) << 4);
+            Walk<FMT> walk;
+            walk.start(A, A.w + (size_t)group * A.w_gstride, min(tile, A.tiles - 1), min(kb_first, kb1 - 1), lane);
+            Raw<FMT> raw[DIST];
+            int asked = kb_first;
+            auto request = [&](Raw<FMT>& r) {
+                if (asked < kb1) {
+                    walk.load(A, r);
+                    if (CG == 2) walk.skip(A);
+                    asked += CG;
+                }
+            };
+#pragma unroll
+            for (int i = 0; i < DIST; i++) request(raw[i]);
+            uint32_t slot = (uint32_t)(warp >> 3), phase = 0;
             bool ok = true;
 #pragma unroll 1
-            for (int kb = kb0; kb < kb1 && ok; kb += DIST) {
+            for (int kb = kb_first; kb < kb1 && ok; kb += DIST * CG) {
 #pragma unroll
                 for (int i = 0; i < DIST; i++) {
-                    if (kb + i < kb1 && ok) {
+                    if (kb + i * CG < kb1 && ok) {
                         uint2 v[2][4], lo[2][4];
                         convert<FMT>(raw[i], v, lo);
-                        if (!have) {
-#pragma unroll
-                            for (int j = 0; j < 4; j++) v[0][j] = v[1][j] = lo[0][j] = lo[1][j] = make_uint2(0u, 0u);
-                        }
-                        if (asked < kb1) {
-                            walk.load(A, lane, raw[i]);
-                            asked++;
-                        }
+                        request(raw[i]);
                         ok = __all_sync(0xffffffffu, wait(B, A, &B.empty[slot], phase ^ 1u, WP_EMPTY));   // the warp leaves together
-                        if (ok) {
+                        if (ok && have) {
                             uint8_t* st = smem + (size_t)slot * stage_bytes;
-                            store_operand(st, warp, lane, v);
-                            if (PW == 2) store_operand(st + A_BYTES, warp, lane, lo);
-                            mk::fence_proxy_async();
+                            store_operand(st, off, g & 1, v);
+                            if (PW == 2) store_operand(st + A_BYTES, off, g & 1, lo);
                         }
+                        mk::fence_proxy_async();
                         __syncwarp();
                         if (ok && lane == 0) mbar_arrive(&B.full[slot]);
-                        if (++slot == (uint32_t)A.stages) {
-                            slot = 0;
+                        slot += CG;
+                        if (slot >= (uint32_t)A.stages) {
+                            slot -= A.stages;
                             phase ^= 1u;
                         }
                     }
                 }
             }
         }
-        // ---- epilogue: lane = weight row, columns = tokens; warps 0-3 and 4-7 take alternate groups of 16 tokens
+        // ---- epilogue: lane = weight row, columns = tokens; each set of four warps takes every 2 CG-th group of 16 tokens
         const bool ok = __all_sync(0xffffffffu, wait(B, A, &B.done, 0, WP_DONE));
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int sub = warp & 3, n = block * 128 + sub * 32 + lane;
             float rs = 1.f;
-            if (A.row_scale && n < A.tiles * 16) rs = __ldg(A.row_scale + (size_t)group * A.rs_gstride + n);
+            if (A.row_scale && n < A.n_valid) rs = __ldg(A.row_scale + (size_t)group * A.rs_gstride + (A.rs_pairs ? 2 * ((n >> 4) * 8 + (n & 7)) + ((n >> 3) & 1) : n));
 #pragma unroll 1
-            for (int c0 = (warp >> 2) * 16; c0 < nt; c0 += 32) {
-                uint32_t r[16];
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                               "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                             : "r"(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)c0));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int c0 = (warp >> 2) * 16; c0 < nt; c0 += 32 * CG) {
+                float v[16];
+                {
+                    uint32_t r[16];
+                    load16(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)c0, r);
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const float v = __uint_as_float(r[i]) * rs;
-                    const int t = row0 + c0 + i;
-                    const bool live = c0 + i < rows;
-                    if (A.ksplit > 1) {
-                        if (live && n < A.n_valid) A.part[((size_t)z * A.part_rows + t) * A.n_valid + n] = v;
-                    } else if (OUT == OUT_GLU) {
-                        // rows 0-7 of a 16-row tile are gates, rows 8-15 their up rows
-                        const float up = __shfl_down_sync(0xffffffffu, v, 8);
-                        const int col = (n >> 4) * 8 + (n & 7);
-                        if (live && !(n & 8) && col < A.act_cols) {
-                            float y = A.gelu ? 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v))) : silu_f(v);
-                            y *= up;
-                            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(A.act + slab_offset(A.act_rows, t, col));
+                    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+                    if (PX > 1) {
+                        load16(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)(A.nt + c0), r);
 #pragma unroll
-                            for (int p = 0; p < PX; p++) {
-                                const __nv_bfloat16 b = __float2bfloat16_rn(y);
-                                *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<uint8_t*>(dst) + (size_t)p * A.act_piece) = b;
-                                y -= __bfloat162float(b);
-                            }
-                        }
-                    } else if (live && n < A.n_valid) {
-                        float* o = A.out + (size_t)t * A.out_stride + n;
-                        *o = OUT == OUT_ADD ? *o + v : v;
+                        for (int i = 0; i < 16; i++) v[i] += __uint_as_float(r[i]);
                     }
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i++) v[i] *= rs;
+                if (A.ksplit > 1) {
+#pragma unroll
+                    for (int i = 0; i < 16; i++)
+                        if (c0 + i < rows && n < A.n_valid) A.part[((size_t)z * A.part_rows + row0 + c0 + i) * A.n_valid + n] = v[i];
+                } else if (OUT == OUT_GLU) {
+                    // Rows 0-7 of a 16-row tile are gates, rows 8-15 their up rows.  The two lanes of a pair share the tokens:
+                    // the gate's lane computes tokens 0-7, the up row's lane tokens 8-15; then the eight lanes of a half
+                    // tile exchange, so that each holds eight neighbouring columns of one token and stores 16 bytes.
+                    const bool hi = n & 8;
+                    float y[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const float other = __shfl_xor_sync(0xffffffffu, hi ? v[i] : v[i + 8], 8);
+                        const float gate = hi ? other : v[i], up = hi ? v[i + 8] : other;
+                        y[i] = (A.gelu ? 0.5f * gate * (1.f + tanhf(0.7978845608028654f * (gate + 0.044715f * gate * gate * gate))) : silu_f(gate)) * up;
+                    }
+#pragma unroll
+                    for (int o = 4; o; o >>= 1) {          // 8 x 8 transpose: afterwards y[c] is column c of token (lane & 7)
+                        const bool u = lane & o;
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+                            if (!(i & o)) {
+                                const float got = __shfl_xor_sync(0xffffffffu, u ? y[i] : y[i + o], o);
+                                if (u) y[i] = got;
+                                else y[i + o] = got;
+                            }
+                    }
+                    const int t = c0 + (hi ? 8 : 0) + (lane & 7), col = (n >> 4) * 8;
+                    if (t < rows && col < A.act_cols) store_slab8<PX>(A.act, A.act_piece, A.act_rows, row0 + t, col, y);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; i++)
+                        if (c0 + i < rows && n < A.n_valid) {
+                            float* o = A.out + (size_t)(row0 + c0 + i) * A.out_stride + n;
+                            *o = OUT == OUT_ADD ? *o + v[i] : v[i];
+                        }
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         }
     }
     __syncthreads();
-    if (warp == 9) {
+    if (warp == CW + 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
     }
@@ -498,7 +545,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) rows_gemm(const __grid_consta
 
 // Adds the K splits' partials in split order and runs the epilogue.
 template <int PX, int OUT>
-__global__ void __launch_bounds__(256) rows_finish(const __grid_constant__ GemmArgs A) {
+static __global__ void __launch_bounds__(256) rows_finish(const __grid_constant__ GemmArgs A) {
     const int t = blockIdx.y;
     const float* p = A.part + (size_t)t * A.n_valid;
     const size_t ss = (size_t)A.part_rows * A.n_valid;
@@ -557,7 +604,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 
 // fp32 rows -> slabs: optional RMSNorm, rounding to bf16 (PIECES = 1, the model's activation type) or fp32-exact pieces.
 template <int PIECES>
-__global__ void __launch_bounds__(256) rows_in(const float* x, long long stride, int K, const float* norm_w, float norm_off, float eps, float in_scale,
+static __global__ void __launch_bounds__(256) rows_in(const float* x, long long stride, int K, const float* norm_w, float norm_off, float eps, float in_scale,
                                                uint8_t* out, size_t piece, int out_rows) {
     __shared__ float red[8];
     const int row = blockIdx.x;
@@ -586,7 +633,7 @@ __global__ void __launch_bounds__(256) rows_in(const float* x, long long stride,
 }
 
 // Row r = sequence * L + position of every array below; tokens are [L][M] (step-major, as mk_stage_args.tokens_in).
-__global__ void __launch_bounds__(256) embed_rows(const __nv_bfloat16* table, const int* tokens, int M, int L, int H, int vocab, float scale, float* h) {
+static __global__ void __launch_bounds__(256) embed_rows(const __nv_bfloat16* table, const int* tokens, int M, int L, int H, int vocab, float scale, float* h) {
     const int row = blockIdx.x, m = row / L, l = row - m * L;
     const int tok = max(0, min(vocab - 1, tokens[(size_t)l * M + m]));
     const uint32_t* src = reinterpret_cast<const uint32_t*>(table + (size_t)tok * H);
@@ -602,12 +649,12 @@ __global__ void __launch_bounds__(256) embed_rows(const __nv_bfloat16* table, co
     }
 }
 
-__global__ void advance_pos(int* pos, int M, int L) {
+static __global__ void advance_pos(int* pos, int M, int L) {
     if ((int)threadIdx.x < M) pos[threadIdx.x] += L;
 }
 
 // out = (base + rms(a) w_a [+ rms(b) w_b]) * scale
-__global__ void __launch_bounds__(256) vec_rows(int N, const float* base, const float* a, const float* wa, const float* b, const float* wb, float off, float eps,
+static __global__ void __launch_bounds__(256) vec_rows(int N, const float* base, const float* a, const float* wa, const float* b, const float* wb, float off, float eps,
                                                 float scale, float* out) {
     __shared__ float red[8];
     const size_t o = (size_t)blockIdx.x * N;
@@ -638,10 +685,11 @@ struct GdnArgs {
     float* ssm;                  // [M][nvh][128 v][128 k]
     const int* pos;              // position of each sequence's first row
     int conv_bf16, l2_clamp;
-    float eps;
+    float eps, norm_eps;         // of the L2 norms, of the gated norm
     // scratch
     float* qkv;                  // [rows][conv_dim]: normalised q, k, and v
-    float4* scal;                // [rows][nvh]: decay, beta, q . k of the head
+    float4* scal;                // [rows][nvh]: decay, beta
+    float* gram;                 // [M][blocks of 8 positions][nkh][8][8] products of the block's keys and queries
     float* o;                    // [rows][nvh * 128]
     uint8_t* out;                // slabs of the gated output
     size_t out_piece;
@@ -661,7 +709,7 @@ __device__ __forceinline__ float* conv_slot(const GdnArgs& G, int m, int ch, int
 
 // Causal conv1d + SiLU of every channel, L2 norms of q and k, and the scalars of the recurrence.  One warp per 128
 // channels of a row, four channels per lane.
-__global__ void __launch_bounds__(256) gdn_conv(const __grid_constant__ GdnArgs G) {
+static __global__ void __launch_bounds__(256) gdn_conv(const __grid_constant__ GdnArgs G) {
     const int row = blockIdx.y, m = row / G.L, l = row - m * G.L, lane = threadIdx.x & 31;
     const int blk = blockIdx.x * 8 + (threadIdx.x >> 5);                    // 128-channel block: q heads, k heads, v heads
     if (blk * 128 >= G.conv_dim) return;
@@ -712,94 +760,236 @@ __global__ void __launch_bounds__(256) gdn_conv(const __grid_constant__ GdnArgs 
 }
 
 // The last `ring` inputs of every channel go back into the history rings.  Runs after gdn_conv has read them.
-__global__ void __launch_bounds__(256) gdn_history(const __grid_constant__ GdnArgs G) {
-    const int ch = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y;
-    if (ch >= G.conv_dim) return;
+static __global__ void __launch_bounds__(256) gdn_history(const __grid_constant__ GdnArgs G) {
+    const int ch = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y, l = G.L - 1 - (int)blockIdx.z;
+    if (ch >= G.conv_dim || l < 0) return;
     const int qk = G.nkh * 128, part = ch < qk ? 0 : (ch < 2 * qk ? 1 : 2);
     const int col = (part == 0 ? G.q_off : (part == 1 ? G.k_off : G.v_off)) + ch - part * qk;
-    for (int l = max(0, G.L - G.ring); l < G.L; l++) {
-        float v = G.y[((size_t)m * G.L + l) * G.y_stride + col];
-        if (G.conv_bf16) v = round_bf16(v);
-        const int slot = (G.pos[m] + l) & (G.ring - 1);
-        const int copies = G.layout == 1 && part < 2 ? 8 : 1;
-        for (int c = 0; c < copies; c++) conv_slot(G, m, ch, c)[slot] = v;
-    }
+    float v = G.y[((size_t)m * G.L + l) * G.y_stride + col];
+    if (G.conv_bf16) v = round_bf16(v);
+    const int slot = (G.pos[m] + l) & (G.ring - 1), copies = G.layout == 1 && part < 2 ? 8 : 1;
+    for (int c = 0; c < copies; c++) conv_slot(G, m, ch, c)[slot] = v;
 }
 
-// The recurrence of 32 value rows of one head of one sequence, position after position: state rows never interact, so a
-// head is four CTAs.  Eight threads share a row (16 keys each, in registers); the inputs of the next SCAN_BLOCK
-// positions arrive in shared memory while the current ones run.  Both dot products are taken against the state before
-// the update (o = decay (S q) + delta (k . q)), so they reduce together and only one of them is on the critical path.
-constexpr int SCAN_BLOCK = 8;
-__global__ void __launch_bounds__(256) gdn_scan(const __grid_constant__ GdnArgs G) {
-    __shared__ __align__(16) float in_s[2][SCAN_BLOCK][256 + 32];            // q | k | 32 values
-    __shared__ float4 sc_s[2][SCAN_BLOCK];
-    const int rep = G.nvh / G.nkh;
-    const int m = blockIdx.z, h = blockIdx.y, v0 = blockIdx.x * 32, kh = h / rep;
-    const int tid = threadIdx.x, vr = tid >> 3, part = tid & 7;
-    float* st = G.ssm + (((size_t)m * G.nvh + h) * 128 + v0 + vr) * 128 + part * 4;     // keys part * 4 + 32 i + {0..3}
-    float s[16];
+// The recurrence  s <- d s + beta (v - d s k) k,  o = s q  runs in blocks of SCAN = 8 positions.  With s the state before
+// the block, P_t the product of its first t decays and delta_t = beta_t (v_t - the state's recall of k_t),
+//     recall_t = P_t (s k_t) + sum_{i < t} (P_t / P_i) delta_i (k_i k_t)      o_t = P_t (s q_t) + sum_{i <= t} (P_t / P_i) delta_i (k_i q_t)
+//     s       <- P_8 s + sum_i (P_8 / P_i) delta_i k_i,
+// so the sixteen products s k_t, s q_t of a block reduce together instead of one by one, and what is sequential are eight
+// scalar steps.
+constexpr int SCAN = 8;
+// k_i k_t (i < t) and q_i k_t (i >= t) of every block and key head: gram[t * 8 + i].  One warp each.
+static __global__ void __launch_bounds__(128) gdn_gram(const __grid_constant__ GdnArgs G) {
+    const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, chunks = (G.L + SCAN - 1) / SCAN;
+    if (w >= G.M * chunks * G.nkh) return;
+    const int kh = w % G.nkh, c = (w / G.nkh) % chunks, m = w / (G.nkh * chunks);
+    float4 q[SCAN], k[SCAN];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float4 a = *reinterpret_cast<const float4*>(st + 32 * i);
-        s[4 * i] = a.x; s[4 * i + 1] = a.y; s[4 * i + 2] = a.z; s[4 * i + 3] = a.w;
-    }
-    const size_t row0 = (size_t)m * G.L;
-    const int key_dim = G.nkh * 128;
-    auto request = [&](int buf, int l0) {
-        // 72 16-byte pieces per position: 32 of q, 32 of k, 8 of v
-        for (int i = tid; i < SCAN_BLOCK * 72; i += 256) {
-            const int b = i / 72, c = i - b * 72, l = l0 + b;
-            if (l < G.L) {
-                const float* src = G.qkv + (row0 + l) * G.conv_dim + (c < 32 ? kh * 128 + 4 * c : (c < 64 ? key_dim + kh * 128 + 4 * (c - 32) : 2 * key_dim + h * 128 + v0 + 4 * (c - 64)));
-                mk::cp_async16(&in_s[buf][b][4 * c], src);
-            }
+    for (int t = 0; t < SCAN; t++) {
+        q[t] = k[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int l = c * SCAN + t;
+        if (l < G.L) {
+            const float4* src = reinterpret_cast<const float4*>(G.qkv + ((size_t)m * G.L + l) * G.conv_dim + kh * 128) + lane;
+            q[t] = src[0];
+            k[t] = src[G.nkh * 32];
         }
-        if (tid < SCAN_BLOCK && l0 + tid < G.L) mk::cp_async16(&sc_s[buf][tid], G.scal + (row0 + l0 + tid) * G.nvh + h);
+    }
+    float v[SCAN * SCAN];
+#pragma unroll
+    for (int t = 0; t < SCAN; t++)
+#pragma unroll
+        for (int i = 0; i < SCAN; i++) {
+            const float4 a = k[t], b = i < t ? k[i] : q[i];
+            v[t * SCAN + i] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w)));
+        }
+#pragma unroll
+    for (int o = 16, n = 32; o; o >>= 1, n >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            if (j < n) {
+                const float send = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
+                v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+    }
+    *reinterpret_cast<float2*>(G.gram + (size_t)w * 64 + 2 * lane) = make_float2(v[0], v[1]);
+}
+
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 both(float a) { return ((u64)__float_as_uint(a) << 32) | __float_as_uint(a); }
+__device__ __forceinline__ float sum2(u64 a) { return __uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32)); }
+
+// Four warps; eight lanes share R value rows of one head of one sequence (16 keys each, in registers, packed in pairs), so
+// a CTA holds 16 R rows and a head is 8 / R CTAs: R = 1 spreads a few heads over the chip, R = 2 reads shared memory once
+// for two rows when there are enough heads.
+template <int R>
+static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ GdnArgs G) {
+    constexpr int ROWS = 16 * R, IN = 256 + ROWS;
+    __shared__ __align__(16) float in_s[2][SCAN][IN];        // q | k | values
+    __shared__ __align__(16) float4 sc_s[2][SCAN];           // decay, beta
+    __shared__ __align__(16) float gram_s[2][64];
+    __shared__ __align__(16) float mat_s[64];                // gram with the decays between the two positions
+    __shared__ float p_s[SCAN], e_s[SCAN];                   // P_t, P_8 / P_t
+    const int rep = G.nvh / G.nkh;
+    const int m = blockIdx.z, h = blockIdx.y, v0 = blockIdx.x * ROWS, kh = h / rep;
+    const int tid = threadIdx.x, part = tid & 7, rr = (tid >> 3) * R;
+    const int chunks = (G.L + SCAN - 1) / SCAN, key_dim = G.nkh * 128;
+    float* st = G.ssm + (((size_t)m * G.nvh + h) * 128 + v0 + rr) * 128 + part * 4;     // keys part * 4 + 32 i + {0..3}
+    u64 s[R][8];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(st + r * 128 + 32 * i);
+            s[r][2 * i] = a.x;
+            s[r][2 * i + 1] = a.y;
+        }
+    const size_t row0 = (size_t)m * G.L;
+    auto request = [&](int buf, int c) {
+        constexpr int PIECES = IN / 4;
+        for (int i = tid; i < SCAN * PIECES; i += 128) {
+            const int b = i / PIECES, x = i - b * PIECES, l = min(c * SCAN + b, G.L - 1);
+            const float* src = G.qkv + (row0 + l) * G.conv_dim + (x < 32 ? kh * 128 + 4 * x : (x < 64 ? key_dim + kh * 128 + 4 * (x - 32) : 2 * key_dim + h * 128 + v0 + 4 * (x - 64)));
+            mk::cp_async16(&in_s[buf][b][4 * x], src);
+        }
+        if (tid < SCAN) mk::cp_async16(&sc_s[buf][tid], G.scal + (row0 + min(c * SCAN + tid, G.L - 1)) * G.nvh + h);
+        if (tid >= 32 && tid < 48) mk::cp_async16(&gram_s[buf][4 * (tid - 32)], G.gram + (((size_t)m * chunks + c) * G.nkh + kh) * 64 + 4 * (tid - 32));
         mk::cp_async_commit();
     };
     request(0, 0);
-    float* o = G.o + row0 * (size_t)(G.nvh * 128) + h * 128 + v0 + vr;
+    float* o = G.o + row0 * (size_t)(G.nvh * 128) + h * 128 + v0 + rr;
 #pragma unroll 1
-    for (int l0 = 0, buf = 0; l0 < G.L; l0 += SCAN_BLOCK, buf ^= 1) {
+    for (int c = 0, buf = 0; c < chunks; c++, buf ^= 1) {
         mk::cp_async_wait_all();
         __syncthreads();
-        if (l0 + SCAN_BLOCK < G.L) request(buf ^ 1, l0 + SCAN_BLOCK);
-        const int nb = min(SCAN_BLOCK, G.L - l0);
-#pragma unroll 1
-        for (int b = 0; b < nb; b++) {
-            const float* q = in_s[buf][b] + part * 4;
-            const float* k = q + 128;
-            float kk[16], dk = 0.f, dq = 0.f, kq = 0.f;
+        if (c + 1 < chunks) request(buf ^ 1, c + 1);
+        const int nb = min(SCAN, G.L - c * SCAN);
+        // a position past the end decays by 1 and corrects by 0
+        if (tid < 64) {
+            const int t = tid >> 3, i = tid & 7, lo = min(t, i), hi = max(t, i);
+            float d = 1.f;
+#pragma unroll
+            for (int j = 0; j < SCAN; j++)
+                if (j > lo && j <= hi && j < nb) d *= sc_s[buf][j].x;
+            mat_s[tid] = gram_s[buf][tid] * d;
+        } else if (tid < 64 + 2 * SCAN) {
+            const int t = (tid - 64) & 7;
+            float d = 1.f;
+#pragma unroll
+            for (int j = 0; j < SCAN; j++)
+                if ((tid < 72 ? j <= t : j > t) && j < nb) d *= sc_s[buf][j].x;
+            (tid < 72 ? p_s : e_s)[t] = d;
+        }
+        // s k_t, s q_t over this lane's keys
+        float u[R][16];
+#pragma unroll
+        for (int t = 0; t < SCAN; t++) {
+            const float* q = in_s[buf][t] + part * 4;
+            u64 a[R], b[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) a[r] = b[r] = 0ull;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const float4 a = *reinterpret_cast<const float4*>(k + 32 * i), c = *reinterpret_cast<const float4*>(q + 32 * i);
-                kk[4 * i] = a.x; kk[4 * i + 1] = a.y; kk[4 * i + 2] = a.z; kk[4 * i + 3] = a.w;
-                dk = fmaf(s[4 * i], a.x, dk); dk = fmaf(s[4 * i + 1], a.y, dk); dk = fmaf(s[4 * i + 2], a.z, dk); dk = fmaf(s[4 * i + 3], a.w, dk);
-                dq = fmaf(s[4 * i], c.x, dq); dq = fmaf(s[4 * i + 1], c.y, dq); dq = fmaf(s[4 * i + 2], c.z, dq); dq = fmaf(s[4 * i + 3], c.w, dq);
-                kq = fmaf(a.x, c.x, kq); kq = fmaf(a.y, c.y, kq); kq = fmaf(a.z, c.z, kq); kq = fmaf(a.w, c.w, kq);
+                const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(q + 128 + 32 * i), qv = *reinterpret_cast<const ulonglong2*>(q + 32 * i);
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    a[r] = fma2(s[r][2 * i], kv.x, a[r]);
+                    b[r] = fma2(s[r][2 * i], qv.x, b[r]);
+                    a[r] = fma2(s[r][2 * i + 1], kv.y, a[r]);
+                    b[r] = fma2(s[r][2 * i + 1], qv.y, b[r]);
+                }
             }
 #pragma unroll
-            for (int x = 1; x < 8; x <<= 1) {
-                dk += __shfl_xor_sync(0xffffffffu, dk, x);
-                dq += __shfl_xor_sync(0xffffffffu, dq, x);
-                kq += __shfl_xor_sync(0xffffffffu, kq, x);
+            for (int r = 0; r < R; r++) {
+                u[r][2 * t] = sum2(a[r]);
+                u[r][2 * t + 1] = sum2(b[r]);
             }
-            const float4 sc = sc_s[buf][b];
-            const float delta = (in_s[buf][b][256 + vr] - sc.x * dk) * sc.y;
+        }
+        // lane t of the eight ends up with s k_t and s q_t
 #pragma unroll
-            for (int i = 0; i < 16; i++) s[i] = fmaf(kk[i], delta, s[i] * sc.x);
-            if (part == 0) o[(size_t)(l0 + b) * (G.nvh * 128)] = fmaf(sc.x, dq, delta * kq);
+        for (int x = 4, n = 8; x; x >>= 1, n >>= 1) {
+            const bool up = part & x;
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (j < n) {
+                        const float send = up ? u[r][j] : u[r][j + n], keep = up ? u[r][j + n] : u[r][j];
+                        u[r][j] = keep + __shfl_xor_sync(0xffffffffu, send, x);
+                    }
+        }
+        __syncthreads();                                     // mat_s, p_s, e_s
+        float delta[R][SCAN];
+#pragma unroll
+        for (int t = 0; t < SCAN; t++) {
+            float mrow[SCAN];
+#pragma unroll
+            for (int i = 0; i < SCAN; i += 4) {
+                if (i >= t) continue;
+                const float4 a = *reinterpret_cast<const float4*>(mat_s + t * 8 + i);
+                mrow[i] = a.x; mrow[i + 1] = a.y; mrow[i + 2] = a.z; mrow[i + 3] = a.w;
+            }
+            const float beta = t < nb ? sc_s[buf][t].y : 0.f, p = p_s[t];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                float recall = __shfl_sync(0xffffffffu, u[r][0], (tid & 24) | t) * p;
+#pragma unroll
+                for (int i = 0; i < SCAN; i++)
+                    if (i < t) recall = fmaf(mrow[i], delta[r][i], recall);
+                delta[r][t] = (in_s[buf][t][256 + rr + r] - recall) * beta;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            float y = u[r][1] * p_s[part];
+#pragma unroll
+            for (int i = 0; i < SCAN; i++)
+                if (i <= part) y = fmaf(mat_s[i * 8 + part], delta[r][i], y);
+            if (part < nb) o[(size_t)(c * SCAN + part) * (G.nvh * 128) + r] = y;
+        }
+        {
+            const u64 p = both(p_s[SCAN - 1]);
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int i = 0; i < 8; i++) s[r][i] = mul2(s[r][i], p);
+        }
+#pragma unroll
+        for (int t = 0; t < SCAN; t++) {
+            const float* k = in_s[buf][t] + 128 + part * 4;
+            u64 f[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) f[r] = both(delta[r][t] * e_s[t]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k + 32 * i);
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    s[r][2 * i] = fma2(kv.x, f[r], s[r][2 * i]);
+                    s[r][2 * i + 1] = fma2(kv.y, f[r], s[r][2 * i + 1]);
+                }
+            }
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) *reinterpret_cast<float4*>(st + 32 * i) = make_float4(s[4 * i], s[4 * i + 1], s[4 * i + 2], s[4 * i + 3]);
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) *reinterpret_cast<ulonglong2*>(st + r * 128 + 32 * i) = make_ulonglong2(s[r][2 * i], s[r][2 * i + 1]);
 }
 
 // Gated RMSNorm per head, into slabs: one half warp per head and row (eight columns per lane).
 template <int PIECES>
-__global__ void __launch_bounds__(256) gdn_gate(const __grid_constant__ GdnArgs G) {
+static __global__ void __launch_bounds__(256) gdn_gate(const __grid_constant__ GdnArgs G) {
     const int row = blockIdx.y, h = blockIdx.x * 16 + (threadIdx.x >> 4), i = (threadIdx.x & 15) * 8;
     if (h >= G.nvh) return;
     const float* o = G.o + (size_t)row * (G.nvh * 128) + h * 128 + i;
@@ -813,7 +1003,7 @@ __global__ void __launch_bounds__(256) gdn_gate(const __grid_constant__ GdnArgs 
     const unsigned mask = 0xffffu << (threadIdx.x & 16);
 #pragma unroll
     for (int x = 8; x; x >>= 1) s += __shfl_xor_sync(mask, s, x);
-    const float r = rsqrtf(s / 128.f + G.eps);
+    const float r = rsqrtf(s / 128.f + G.norm_eps);
 #pragma unroll
     for (int j = 0; j < 8; j++) v[j] = v[j] * r * __ldg(G.norm_w + i + j) * (z[j] * sigmoid_f(z[j]));
     store_slab8<PIECES>(G.out, G.out_piece, G.out_rows, row, h * 128 + i, v);
@@ -833,8 +1023,10 @@ struct AttnArgs {
     int max_pages, kv_shift;
     uint32_t s_page, s_head, s_pos;
     const int* pos;
-    __nv_bfloat16* q;            // [rows][nq][HD] prepared queries
+    void* q;                     // [rows][nq][HD] prepared queries, bf16 (attn_rows) or fp32 (attn_rows_f32)
+    float q_scale;               // fp32 queries: factor applied after the rotation
     uint8_t* out;                // slabs of the (gated) output
+    size_t out_piece;
     int out_rows;
 };
 
@@ -845,8 +1037,8 @@ __device__ __forceinline__ size_t kv_offset(const AttnArgs& T, int m, int kvh, i
 
 // Norm, rotation and rounding of every head vector of a row: queries to `q`, keys and values into the paged cache.
 // One warp per head vector; lane i holds dims i + 32 j, so both halves of a rotated pair are in one lane.
-template <int HD>
-__global__ void __launch_bounds__(256) attn_prepare(const __grid_constant__ AttnArgs T) {
+template <int HD, bool QF32, bool KVF32>
+static __global__ void __launch_bounds__(256) attn_prepare(const __grid_constant__ AttnArgs T) {
     constexpr int N = HD / 32;
     const int row = blockIdx.y, m = row / T.L, lane = threadIdx.x & 31;
     const int hv = blockIdx.x * 8 + (threadIdx.x >> 5);                 // q heads, k heads, v heads
@@ -886,14 +1078,15 @@ __global__ void __launch_bounds__(256) attn_prepare(const __grid_constant__ Attn
                     }
             }
     }
-    if (kind == 0) {
-        __nv_bfloat16* dst = T.q + ((size_t)row * T.nq + head) * HD;
+    const size_t o = kind == 0 ? ((size_t)row * T.nq + head) * HD : kv_offset(T, m, head, pos);
+    void* dst = kind == 0 ? T.q : (kind == 1 ? T.k_cache : T.v_cache);
+    if (kind == 0 ? QF32 : KVF32) {
+        const float f = kind == 0 ? T.q_scale : 1.f;
 #pragma unroll
-        for (int j = 0; j < N; j++) dst[lane + 32 * j] = __float2bfloat16_rn(v[j]);
+        for (int j = 0; j < N; j++) reinterpret_cast<float*>(dst)[o + lane + 32 * j] = v[j] * f;
     } else {
-        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(kind == 1 ? T.k_cache : T.v_cache) + kv_offset(T, m, head, pos);
 #pragma unroll
-        for (int j = 0; j < N; j++) dst[lane + 32 * j] = __float2bfloat16_rn(v[j]);
+        for (int j = 0; j < N; j++) reinterpret_cast<__nv_bfloat16*>(dst)[o + lane + 32 * j] = __float2bfloat16_rn(v[j]);
     }
 }
 
@@ -920,7 +1113,7 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 constexpr int AT_ROWS = 64, AT_KEYS = 64, AT_PIECES = 3;
 template <int HD> constexpr int attn_smem() { return 3 * AT_ROWS * HD * 2 + AT_PIECES * AT_ROWS * AT_KEYS * 2 + 4 * AT_ROWS * 4; }
 template <int HD>
-__global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant__ AttnArgs T) {
+static __global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant__ AttnArgs T) {
     extern __shared__ __align__(128) uint8_t sm[];
     constexpr int RB = HD * 2, CH = RB / 16;                             // bytes and 16-byte pieces of a row
     uint8_t *q_s = sm, *k_s = q_s + AT_ROWS * RB, *v_s = k_s + AT_KEYS * RB, *p_s = v_s + AT_KEYS * RB;
@@ -942,7 +1135,7 @@ __global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant__ Attn
     for (int i = tid; i < AT_ROWS * CH; i += 256) {
         const int r = i / CH, c = i - r * CH, p = r / qpk, hq = r - p * qpk;
         const bool live = p < np;
-        const __nv_bfloat16* src = T.q + (((size_t)m * T.L + l0 + (live ? p : 0)) * T.nq + kvh * qpk + hq) * HD + c * 8;
+        const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(T.q) + (((size_t)m * T.L + l0 + (live ? p : 0)) * T.nq + kvh * qpk + hq) * HD + c * 8;
         cp16_zfill(smem_u32(q_s + (size_t)r * RB + (((c & ~7) | ((c ^ r) & 7)) << 4)), src, live);
     }
     load_kv(k_s, kc, first);
@@ -1070,6 +1263,194 @@ __global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant__ Attn
     }
 }
 
+// The same for the 0.8B model, whose attention is exact to fp32: queries, probabilities and an fp32 cache enter the
+// tensor cores as three bf16 pieces each, and of the nine piece products the six that reach above 2^-24 are formed (a
+// bf16 cache is one piece: three products).  Blocks of 32 keys; the fp32 rows of the next block wait in registers.
+constexpr int AF_KEYS = 32, AF_HD = 256, AF_RB = AF_HD * 2;
+template <bool KVF32> constexpr int attn_f32_smem() { return 3 * AT_ROWS * AF_RB + 2 * (KVF32 ? 3 : 1) * AF_KEYS * AF_RB + 3 * AT_ROWS * AF_KEYS * 2 + 4 * AT_ROWS * 4; }
+// Four consecutive columns c .. c + 3 of a row, as NP pieces of swizzled rows
+template <int NP>
+__device__ __forceinline__ void split4(uint8_t* base, size_t piece, int row, int c, float4 v) {
+    uint8_t* dst = base + (size_t)row * AF_RB + ((((c >> 3) & ~7) | (((c >> 3) ^ row) & 7)) << 4) + (c & 4) * 2;
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+        const uint32_t a = pack_bf16(v.x, v.y), b = pack_bf16(v.z, v.w);
+        *reinterpret_cast<uint2*>(dst + p * piece) = make_uint2(a, b);
+        v.x -= bf_lo(a); v.y -= bf_hi(a); v.z -= bf_lo(b); v.w -= bf_hi(b);
+    }
+}
+template <bool KVF32>
+static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_constant__ AttnArgs T) {
+    extern __shared__ __align__(128) uint8_t sm[];
+    constexpr int KP = KVF32 ? 3 : 1, QB = AT_ROWS * AF_RB, KB = AF_KEYS * AF_RB, PB = AT_ROWS * AF_KEYS * 2;
+    constexpr int PER = AF_KEYS * AF_HD / 4 / 256;                        // groups of four columns per thread and block
+    uint8_t *q_s = sm, *k_s = q_s + 3 * QB, *v_s = k_s + KP * KB, *p_s = v_s + KP * KB;
+    float* st_s = reinterpret_cast<float*>(p_s + 3 * PB);
+    const int qpk = T.nq / T.nkv, bq = AT_ROWS / qpk;
+    const int m = blockIdx.z, kvh = blockIdx.y, l0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * bq;
+    const int np = min(bq, T.L - l0), pos0 = T.pos[m] + l0, last = pos0 + np - 1;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp & 3, dh = warp >> 2, g = lane >> 2, t = lane & 3;
+    auto fetch = [&](const void* cache, int k0, float4 (&r)[PER]) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int key = (tid >> 6) + 4 * i, c = (tid & 63) * 4, p = k0 + key;
+            r[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (p <= last) {
+                const size_t o = kv_offset(T, m, kvh, p) + c;
+                if (KVF32) r[i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(cache) + o);
+                else {
+                    const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(cache) + o);
+                    r[i] = make_float4(bf_lo(w.x), bf_hi(w.x), bf_lo(w.y), bf_hi(w.y));
+                }
+            }
+        }
+    };
+    auto place = [&](uint8_t* dst, const float4 (&r)[PER]) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) split4<KP>(dst, KB, (tid >> 6) + 4 * i, (tid & 63) * 4, r[i]);
+    };
+    float4 kr[PER];
+    fetch(T.k_cache, 0, kr);
+    for (int i = tid; i < AT_ROWS * AF_HD / 4; i += 256) {
+        const int r = i / (AF_HD / 4), c = (i - r * (AF_HD / 4)) * 4, p = r / qpk, hq = r - p * qpk;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p < np) v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(T.q) + (((size_t)m * T.L + l0 + p) * T.nq + kvh * qpk + hq) * AF_HD + c);
+        split4<3>(q_s, QB, r, c, v);
+    }
+    float o[AF_HD / 16][4], mx[2] = {-3.0e38f, -3.0e38f}, sum[2] = {0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < AF_HD / 16; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    int qp[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) qp[i] = pos0 + min((16 * rg + g + 8 * i) / qpk, np - 1);
+    const uint32_t qa = smem_u32(q_s) + (uint32_t)(16 * rg + (lane & 15)) * AF_RB, qx = lane & 7;
+#pragma unroll 1
+    for (int k0 = 0; k0 <= last; k0 += AF_KEYS) {
+        __syncthreads();                                                 // everybody is done with the previous block
+        place(k_s, kr);
+        float4 vr[PER];
+        fetch(T.v_cache, k0, vr);
+        __syncthreads();
+        float s[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+#pragma unroll 2
+        for (int kk = 0; kk < AF_HD / 16; kk++) {
+            uint32_t a[3][4], b[KP][4];
+            const uint32_t ca = 2 * kk + (lane >> 4), key = 16 * dh + (lane & 7) + ((lane >> 4) << 3), cb = 2 * kk + ((lane >> 3) & 1);
+#pragma unroll
+            for (int p = 0; p < 3; p++) ldsm4(a[p], qa + p * QB + (((ca & ~7u) | ((ca ^ qx) & 7)) << 4));
+#pragma unroll
+            for (int p = 0; p < KP; p++) ldsm4(b[p], smem_u32(k_s) + p * KB + key * AF_RB + (((cb & ~7u) | ((cb ^ key) & 7)) << 4));
+#pragma unroll
+            for (int p = 2; p >= 0; p--)                                  // small products first
+#pragma unroll
+                for (int r = KP - 1; r >= 0; r--)
+                    if (p + r < 3) {
+                        mma16816(s[0], a[p], b[r][0], b[r][1]);
+                        mma16816(s[1], a[p], b[r][2], b[r][3]);
+                    }
+        }
+        float bm[2] = {-3.0e38f, -3.0e38f};
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int p = k0 + 16 * dh + 8 * n + 2 * t + (i & 1), r = i >> 1;
+                s[n][i] = p <= qp[r] ? s[n][i] : -3.0e38f;
+                bm[r] = fmaxf(bm[r], s[n][i]);
+            }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 1));
+            bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 2));
+            if (t == 0) st_s[dh * AT_ROWS + 16 * rg + g + 8 * r] = bm[r];
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + rg) : "memory");
+        float f[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const float nm = fmaxf(mx[r], fmaxf(bm[r], st_s[(dh ^ 1) * AT_ROWS + 16 * rg + g + 8 * r]));
+            f[r] = __expf(mx[r] - nm);
+            mx[r] = nm;
+            sum[r] *= f[r];
+        }
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                float p0 = s[n][2 * r] > -2.9e38f ? __expf(s[n][2 * r] - mx[r]) : 0.f, p1 = s[n][2 * r + 1] > -2.9e38f ? __expf(s[n][2 * r + 1] - mx[r]) : 0.f;
+                sum[r] += p0 + p1;
+                const uint32_t row = 16 * rg + g + 8 * r, c = 2 * dh + n;
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    const uint32_t w = pack_bf16(p0, p1);
+                    *reinterpret_cast<uint32_t*>(p_s + q * PB + row * 64 + ((c ^ ((row >> 1) & 3)) << 4) + t * 4) = w;
+                    p0 -= bf_lo(w);
+                    p1 -= bf_hi(w);
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < AF_HD / 16; i++) {
+            o[i][0] *= f[0]; o[i][1] *= f[0];
+            o[i][2] *= f[1]; o[i][3] *= f[1];
+        }
+        place(v_s, vr);
+        if (k0 + AF_KEYS <= last) fetch(T.k_cache, k0 + AF_KEYS, kr);
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < AF_KEYS / 16; kk++) {
+            uint32_t a[3][4];
+            const uint32_t row = 16 * rg + (lane & 15);
+#pragma unroll
+            for (int p = 0; p < 3; p++) ldsm4(a[p], smem_u32(p_s) + p * PB + row * 64 + (((2 * kk + (lane >> 4)) ^ ((row >> 1) & 3)) << 4));
+#pragma unroll
+            for (int n = 0; n < AF_HD / 32; n++) {
+                const uint32_t key = 16 * kk + (lane & 15), c = dh * 16 + 2 * n + (lane >> 4);
+                uint32_t b[KP][4];
+#pragma unroll
+                for (int p = 0; p < KP; p++) ldsm4_t(b[p], smem_u32(v_s) + p * KB + key * AF_RB + (((c & ~7u) | ((c ^ key) & 7)) << 4));
+#pragma unroll
+                for (int p = 2; p >= 0; p--)
+#pragma unroll
+                    for (int r = KP - 1; r >= 0; r--)
+                        if (p + r < 3) {
+                            mma16816(o[2 * n], a[p], b[r][0], b[r][1]);
+                            mma16816(o[2 * n + 1], a[p], b[r][2], b[r][3]);
+                        }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
+        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
+        if (t == 0) st_s[(2 + dh) * AT_ROWS + 16 * rg + g + 8 * r] = sum[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const int rr = 16 * rg + g + 8 * r, p = rr / qpk, hq = kvh * qpk + rr - p * qpk;
+        if (p >= np) continue;
+        const float inv = 1.f / (st_s[2 * AT_ROWS + rr] + st_s[3 * AT_ROWS + rr]);
+        const int row = m * T.L + l0 + p;
+        const float* gate = T.y + (size_t)row * T.y_stride + T.q_off + (size_t)hq * T.q_hs + T.gate_off;
+#pragma unroll
+        for (int n = 0; n < AF_HD / 16; n++) {
+            const int dim = dh * (AF_HD / 2) + 8 * n + 2 * t;
+            float a = o[n][2 * r] * inv * sigmoid_f(gate[dim]), b = o[n][2 * r + 1] * inv * sigmoid_f(gate[dim + 1]);
+            uint8_t* dst = T.out + slab_offset(T.out_rows, row, hq * AF_HD + dim);
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const uint32_t w = pack_bf16(a, b);
+                *reinterpret_cast<uint32_t*>(dst + q * T.out_piece) = w;
+                a -= bf_lo(w);
+                b -= bf_hi(w);
+            }
+        }
+    }
+}
+
 // ---- expert routing --------------------------------------------------------------------------------------------
 struct RouteArgs {
     const float* logits;
@@ -1085,7 +1466,7 @@ struct RouteArgs {
 };
 
 // One warp per token: the top-k experts (ties to the lower id), their weights, and the count per expert.
-__global__ void __launch_bounds__(256) route_rows(const __grid_constant__ RouteArgs R) {
+static __global__ void __launch_bounds__(256) route_rows(const __grid_constant__ RouteArgs R) {
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= R.rows) return;
     const float* lg = R.logits + (size_t)row * R.stride;
@@ -1139,7 +1520,7 @@ __global__ void __launch_bounds__(256) route_rows(const __grid_constant__ RouteA
 }
 
 // Lays the experts' tokens out one after the other (each expert from a multiple of 16 rows) and lists the tiles.
-__global__ void __launch_bounds__(256) route_plan(const __grid_constant__ RouteArgs R) {
+static __global__ void __launch_bounds__(256) route_plan(const __grid_constant__ RouteArgs R) {
     __shared__ int rows_s[256], tiles_s[256];
     const int e = threadIdx.x, n = e < R.experts ? R.counts[e] : 0;
     const int rows = (n + 15) & ~15, tiles = (n + R.nt - 1) / R.nt;
@@ -1161,7 +1542,7 @@ __global__ void __launch_bounds__(256) route_plan(const __grid_constant__ RouteA
     if (e == 255) *R.n_items = tiles_s[255];
 }
 
-__global__ void __launch_bounds__(256) route_slots(const __grid_constant__ RouteArgs R) {
+static __global__ void __launch_bounds__(256) route_slots(const __grid_constant__ RouteArgs R) {
     const int i = blockIdx.x * 256 + threadIdx.x, row = i >> 3, k = i & 7;
     if (row >= R.rows || k >= R.topk) return;
     const int e = R.slot[i];
@@ -1169,7 +1550,7 @@ __global__ void __launch_bounds__(256) route_slots(const __grid_constant__ Route
 }
 
 // Copies every token's slab row to the rows of its experts.
-__global__ void __launch_bounds__(256) gather_rows(const uint8_t* x, int x_rows, const int* slot, int topk, int kbs, uint8_t* out, int out_rows) {
+static __global__ void __launch_bounds__(256) gather_rows(const uint8_t* x, int x_rows, const int* slot, int topk, int kbs, uint8_t* out, int out_rows) {
     const int row = blockIdx.x;
     for (int i = threadIdx.x; i < kbs * 8; i += 256) {
         const int kb = i >> 3, c = i & 7;
@@ -1182,7 +1563,7 @@ __global__ void __launch_bounds__(256) gather_rows(const uint8_t* x, int x_rows,
 }
 
 // Weighted sum of a token's expert outputs (ascending expert id, then the shared expert), stored or added.
-__global__ void __launch_bounds__(256) combine_rows(const float* y, int N, const int* slot, const float* weight, int topk, const float* shared, const float* gate,
+static __global__ void __launch_bounds__(256) combine_rows(const float* y, int N, const int* slot, const float* weight, int topk, const float* shared, const float* gate,
                                                     int add, float* out, long long out_stride) {
     const int row = blockIdx.x;
     for (int c = threadIdx.x * 4; c < N; c += 1024) {

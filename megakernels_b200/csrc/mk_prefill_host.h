@@ -1,0 +1,114 @@
+// Host helpers shared by the two prompt paths (mk_prefill.cu: stage programs, mk_prefill_08b.cu: the 0.8B model).
+#pragma once
+#include <cstdarg>
+#include <cstdio>
+#include <cstring>
+
+#include "../../include/mk_b200.h"
+#include "mk_prefill.cuh"
+
+int mk_set_error(int code, const char* text);       // mk_api.cu: the text behind mk_last_error()
+
+namespace mkp {
+
+inline int pfail(int code, const char* fmt, ...) {
+    char buf[512];
+    va_list ap;
+    va_start(ap, fmt);
+    vsnprintf(buf, sizeof buf, fmt, ap);
+    va_end(ap);
+    return mk_set_error(code, buf);
+}
+#define MKP_CUDA(call)                                                                      \
+    do {                                                                                    \
+        cudaError_t err__ = (call);                                                         \
+        if (err__ != cudaSuccess)                                                           \
+            return pfail(MK_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(err__));   \
+    } while (0)
+
+constexpr int SMEM_MAX = 232448;
+
+// Hands out the workspace; with base == nullptr it only counts.
+struct Arena {
+    uint8_t* base;
+    size_t off = 0;
+    template <class T>
+    T* take(size_t n) {
+        off = (off + 1023) & ~(size_t)1023;
+        T* p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+        off += n * sizeof(T);
+        return p;
+    }
+};
+
+template <int FMT, int PX, int CG>
+int launch_gemm_cg(GemmArgs& A, int out, dim3 grid, int smem, cudaStream_t st) {
+    auto fn = out == OUT_STORE ? rows_gemm<FMT, PX, OUT_STORE, CG> : (out == OUT_ADD ? rows_gemm<FMT, PX, OUT_ADD, CG> : rows_gemm<FMT, PX, OUT_GLU, CG>);
+    MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    fn<<<grid, (8 * CG + 2) * 32, smem, st>>>(A);
+    MKP_CUDA(cudaGetLastError());
+    return MK_OK;
+}
+
+template <int FMT, int PX>
+int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaStream_t st) {
+    constexpr int PW = FMT == W_FP8_BLOCK ? 2 : 1;
+    const int stage = PW * A_BYTES + PX * A.nt * 128, fixed = (int)sizeof(GemmBars) + 1024;
+    // Narrow tiles leave room for two CTAs per SM with three stages each: one's start and end hide behind the other.  Wide
+    // ones have the SM to themselves, with sixteen warps to convert weights (eight cannot keep up with the MMAs).
+    int stages = (SMEM_MAX / 2 - 1024 - fixed) / stage;
+    const bool two = stages >= 3;
+    if (!two) stages = (SMEM_MAX - fixed) / stage;
+    if (stages > MAX_STAGES) stages = MAX_STAGES;
+    if (stages < 2) return pfail(MK_ERR_BADARG, "prefill: %d tokens per tile leave no room for two stages", A.nt);
+    A.stages = stages;
+    const int smem = stages * stage + fixed;
+    const dim3 grid = items ? dim3(blocks, items, 1) : dim3(tiles_x, blocks, A.ksplit);
+    const int rc = two || FMT == W_SLAB ? launch_gemm_cg<FMT, PX, 1>(A, out, grid, smem, st) : launch_gemm_cg<FMT, PX, FMT == W_SLAB ? 1 : 2>(A, out, grid, smem, st);
+    if (rc != MK_OK) return rc;
+    if (A.ksplit > 1) {
+        const dim3 fgrid(out == OUT_GLU ? (A.act_cols + 255) / 256 : (A.n_valid + 1023) / 1024, A.rows);
+        if (out == OUT_STORE) rows_finish<PX, OUT_STORE><<<fgrid, 256, 0, st>>>(A);
+        else if (out == OUT_ADD) rows_finish<PX, OUT_ADD><<<fgrid, 256, 0, st>>>(A);
+        else rows_finish<PX, OUT_GLU><<<fgrid, 256, 0, st>>>(A);
+        MKP_CUDA(cudaGetLastError());
+    }
+    return MK_OK;
+}
+
+// The DeltaNet mixer of M sequences of L rows; `gate` is gdn_gate of the wanted number of pieces.
+inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), int sms, cudaStream_t st) {
+    const int rows = G.M * G.L, chunks = (G.L + SCAN - 1) / SCAN;
+    gdn_conv<<<dim3((G.conv_dim / 128 + 7) / 8, rows), 256, 0, st>>>(G);
+    gdn_history<<<dim3((G.conv_dim + 255) / 256, G.M, G.ring), 256, 0, st>>>(G);
+    gdn_gram<<<(G.M * chunks * G.nkh + 3) / 4, 128, 0, st>>>(G);
+    // two rows per lane once that leaves two CTAs per SM
+    if (G.M * G.nvh * 4 >= 2 * sms) gdn_scan<2><<<dim3(4, G.nvh, G.M), 128, 0, st>>>(G);
+    else gdn_scan<1><<<dim3(8, G.nvh, G.M), 128, 0, st>>>(G);
+    gate<<<dim3((G.nvh + 15) / 16, rows), 256, 0, st>>>(G);
+    MKP_CUDA(cudaGetLastError());
+    return MK_OK;
+}
+
+// Token tiles of `rows` rows: equal tiles of at most 256, multiples of 16.
+inline void token_tiles(int rows, int* n, int* nt) {
+    *n = (rows + 255) / 256;
+    *nt = ((rows + *n - 1) / *n + 15) / 16 * 16;
+}
+
+// CTAs that share the K range of one tile: the count with the shortest schedule (rounds of one CTA per SM, each 64-column
+// block counted once and the start and end of a CTA as six), at least eight blocks each.
+inline int pick_ksplit(int ctas, int kbs, int sms) {
+    int best = 1;
+    double cost = 1e30;
+    for (int z = 1; z <= 8 && (z == 1 || kbs / z >= 8); z++) {
+        const double c = (double)((ctas * z + sms - 1) / sms) * ((kbs + z - 1) / z + 6) + (z > 1 ? 4 + z : 0);
+        if (c < cost) {
+            cost = c;
+            best = z;
+        }
+    }
+    return best;
+}
+
+}  // namespace mkp

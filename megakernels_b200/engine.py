@@ -32,6 +32,11 @@ from .quant import is_gemv_weight, quantize_int8_rows, roundtrip_int8_rows
 # Steps per launch.  A step takes well under a millisecond on a B200, so this only bounds the size
 # of the per-launch output buffers.
 MAX_STEPS_PER_LAUNCH = 1024
+# Prompt tokens from which the token-parallel path takes a prompt in: it passes over the weights once (about 2 ms with its
+# launches) where stepping costs 0.4 ms per token.  Shorter ones keep the step path and its bits.
+MIN_PROMPT_ROWS = 16
+# Positions of one pass of that path: bounds its workspace (about 150 KB per position).
+MAX_PROMPT_ROWS = 4096
 
 
 def rope_tables(cfg, max_seq, device):
@@ -270,6 +275,7 @@ class Megakernel:
         self.weight_bytes = self._weight_bytes()
         self.last_step_ns = []
         self.launches = 0
+        self._workspace = None          # of the token-parallel prompt path, grown to the largest pass so far
         self.reset()
 
     # ------------------------------------------------------------------------------------------
@@ -373,6 +379,24 @@ class Megakernel:
         return dict(seed=seed & 0xFFFFFFFF, inv_temperature=(1.0 / temperature) if temperature > 0 else 0.0,
                     n_stop=len(stop_ids)), stops
 
+    def _take_in(self, tokens, start, hidden=None, seq=0, batched=False):
+        """`tokens` enter positions start, start + 1, ... of sequence `seq`, all at once (`mk_prefill`); `hidden` [n, hidden]
+        fp32 receives the residuals after the last layer.  Asynchronous; positions are the caller's to advance."""
+        n = len(tokens)
+        need = int(self.lib.mk_prefill_bytes(min(n, MAX_PROMPT_ROWS)))
+        if self._workspace is None or self._workspace.numel() < need:
+            self._workspace = None
+            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
+        ids = torch.tensor(tokens, dtype=torch.int32).to(self.device)
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        for lo in range(0, n, MAX_PROMPT_ROWS):
+            rows = min(MAX_PROMPT_ROWS, n - lo)
+            a = _lib.PrefillArgs(tokens=ids.data_ptr() + 4 * lo, positions=rows, start_pos=start + lo, sequence=seq, batched=int(batched),
+                                 resid_out=hidden[lo:].data_ptr() if hidden is not None else 0, workspace=self._workspace.data_ptr(),
+                                 workspace_bytes=self._workspace.numel(), spin_limit_ns=self.spin_limit_ns)
+            _lib.check(self.lib.mk_prefill(self._h, ctypes.byref(a), ctypes.c_void_p(stream)))
+            self.launches += 1
+
     @torch.no_grad()
     def run(self, tokens, n_generate=1, temperature=0.0, seed=0, stop_ids=(), return_logits=False, prof=None,
             prof_step=0, timing=False, all_logits=False, track_mtp=False, return_resid=False):
@@ -395,21 +419,30 @@ class Megakernel:
             raise ValueError(f"sequence would exceed max_seq={self.max_seq}")
         dev, cfg = self.device, self.cfg
         want_hidden = track_mtp or return_resid
+        hidden = torch.empty(n_steps, cfg.hidden, device=dev) if want_hidden else None
+        # a long prompt goes in all at once, except its last token (whoever wants logits or times per token gets steps)
+        taken = 0
+        if n_given > MIN_PROMPT_ROWS and not all_logits and not timing and prof is None:
+            taken = n_given - 1
+            self._take_in(given[:taken], self.pos, hidden)
+            self.pos += taken
+        left, n_left = n_given - taken, n_steps - taken
         how, stops = self._sampling(temperature, seed, stop_ids, dev)
-        bufs = dict(forced=torch.tensor(given, dtype=torch.int32).pin_memory().to(dev, non_blocking=True),
-                    stop_ids=stops, tokens_out=torch.zeros(n_steps, dtype=torch.int64, device=dev),
-                    logits_out=torch.empty(n_steps, cfg.vocab, device=dev) if (return_logits or all_logits) else None,
-                    resid_out=torch.empty(n_steps, cfg.hidden, device=dev) if want_hidden else None, prof=prof)
-        first_choice = 0 if all_logits else n_given - 1            # the first step whose LM head runs
-        words = self._submit(n_steps, dict(how, n_forced=n_given, lm_from=first_choice, prof_step=prof_step), bufs, timing)
+        bufs = dict(forced=torch.tensor(given[taken:], dtype=torch.int32).pin_memory().to(dev, non_blocking=True),
+                    stop_ids=stops, tokens_out=torch.zeros(n_left, dtype=torch.int64, device=dev),
+                    logits_out=torch.empty(n_left, cfg.vocab, device=dev) if (return_logits or all_logits) else None,
+                    resid_out=hidden[taken:] if want_hidden else None, prof=prof)
+        first_choice = 0 if all_logits else left - 1               # the first step whose LM head runs
+        words = self._submit(n_left, dict(how, n_forced=left, lm_from=first_choice, prof_step=prof_step), bufs, timing)
         ran = words[0]
         # tokens_out holds keys (ordered score << 32 | ~id): the low word, complemented, is the id
-        chosen = (0xFFFFFFFF - (bufs["tokens_out"][n_given - 1: ran] & 0xFFFFFFFF)).tolist()
-        hidden = bufs["resid_out"][:ran] if want_hidden else None
-        if ran:
+        chosen = (0xFFFFFFFF - (bufs["tokens_out"][left - 1: ran] & 0xFFFFFFFF)).tolist()
+        if want_hidden:
+            hidden = hidden[: taken + ran]
+        if taken + ran:
             if track_mtp and self.mtp is not None:
-                entered = (given + chosen)[:ran]                   # what positions pos .. pos + ran - 1 were fed
-                self.mtp_fed(self.pos, mtp_mod.rmsnorm(hidden, self.final_norm, cfg.eps), entered)
+                entered = (given + chosen)[: taken + ran]          # what positions pos - taken .. pos + ran - 1 were fed
+                self.mtp_fed(self.pos - taken, mtp_mod.rmsnorm(hidden, self.final_norm, cfg.eps), entered)
             else:
                 self.mtp_h = None                                  # the draft head's cache no longer follows the sequence
         self.pos += ran
@@ -417,7 +450,7 @@ class Megakernel:
         if all_logits:
             return chosen, bufs["logits_out"][:ran]
         if return_logits:
-            return chosen, bufs["logits_out"][n_given - 1: ran]
+            return chosen, bufs["logits_out"][left - 1: ran]
         return chosen
 
     # ------------------------------------------------------------------------------------------
@@ -448,6 +481,15 @@ class Megakernel:
         if any(self.bpos[j] + n_steps > self.max_seq for j in range(B)):
             raise ValueError(f"a sequence would exceed max_seq={self.max_seq}")
         dev = self.device
+        # long prompts go in all at once, except their last tokens (times per step are times of steps)
+        for j, p in enumerate(prompts):
+            if len(p) > MIN_PROMPT_ROWS and not timing and prof is None:
+                self._take_in(p[:-1], self.bpos[j], seq=j, batched=True)
+                self.bpos[j] += len(p) - 1
+                prompts[j] = p[-1:]
+        n_forced = [len(p) for p in prompts]
+        n_total = [n + n_generate - 1 for n in n_forced]
+        n_steps = max(n_total)
         forced = torch.zeros(max(n_forced), NBW, dtype=torch.int32)
         for j, p in enumerate(prompts):
             forced[: len(p), j] = torch.tensor(p, dtype=torch.int32)
@@ -511,10 +553,24 @@ class Megakernel:
                            device=self.device)
 
     def prefill(self, tokens, chunk=512):
-        """Take a prompt in: everything but its last token goes through the kernel (in launches of `chunk` steps,
-        keeping the draft head's cache in step); the last token is handed back for the caller to feed with the
-        first generation launch, as the reference's `prefill` does (`qwen_mk/engine.py:296-301`)."""
-        *body, tail = list(tokens)
+        """Take a prompt in: everything but its last token goes through the kernels (all at once, or a short prompt in
+        launches of `chunk` steps), keeping the draft head's cache in step; the last token is handed back for the caller to
+        feed with the first generation launch, as the reference's `prefill` does (`qwen_mk/engine.py:296-301`)."""
+        *body, tail = [int(t) for t in tokens]
+        if len(body) >= MIN_PROMPT_ROWS:
+            self._enter_mode("single")
+            n, start = len(body), self.pos
+            if start + n > self.max_seq:
+                raise ValueError(f"sequence would exceed max_seq={self.max_seq}")
+            hidden = torch.empty(n, self.cfg.hidden, device=self.device) if self.mtp is not None else None
+            self._take_in(body, start, hidden)
+            self.pos += n
+            if hidden is not None:
+                self.mtp_fed(start, mtp_mod.rmsnorm(hidden, self.final_norm, self.cfg.eps), body)
+            else:
+                self.mtp_h = None
+            self.last_resid = hidden
+            return tail
         for lo in range(0, len(body), chunk):
             self.run(body[lo: lo + chunk], track_mtp=True)
         return tail

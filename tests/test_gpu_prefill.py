@@ -79,3 +79,52 @@ def test_programs_without_the_row_path_step(packed):
     for t in prompt:
         want = eng.step(torch.tensor([t], device="cuda"))
     assert torch.equal(got, want)
+
+
+# ---- the 0.8B model: fp32-exact, so ids are equal and states agree to fp32 sums -------------------------------------------
+@pytest.fixture(scope="module")
+def small():
+    from megakernels_b200.config import qwen35_08b
+    from megakernels_b200.synth import make_mtp_weights, make_weights
+    cfg = qwen35_08b(n_layers=4, vocab=4096)
+    return cfg, make_weights(cfg, 0, init="realistic"), make_mtp_weights(cfg, 0)
+
+
+@pytest.mark.parametrize("quant,kv,length,context", [("bf16", "fp32", 17, 0), ("bf16", "fp32", 130, 5), ("int8", "fp32", 17, 3),
+                                                     ("int8", "fp32", 300, 33), ("int8", "bf16", 90, 0)])
+def test_small_model_prompt_equals_stepping(small, monkeypatch, quant, kv, length, context):
+    from megakernels_b200 import engine as E
+    from megakernels_b200.synth import make_prompt
+    prompt, got = make_prompt(small[0], context + length), []
+    for rows in (True, False):
+        mk = E.Megakernel(small, max_seq=512, quant=quant, kv_dtype=kv, mtp=quant == "int8")
+        with monkeypatch.context() as mp:
+            mp.setattr(E, "MIN_PROMPT_ROWS", 1 << 30)
+            if context:
+                mk.run(prompt[:context])
+            mp.setattr(E, "MIN_PROMPT_ROWS", 16 if rows else 1 << 30)
+            mp.setattr(E, "MAX_PROMPT_ROWS", 120)            # several passes
+            ids, logits = mk.run(prompt[context:], n_generate=6, return_logits=True, track_mtp=True)
+        got.append((mk, ids, logits))
+    (a, ia, la), (b, ib, lb) = got
+    tol = 2e-5 if kv == "fp32" else 2e-4                      # a bf16 cache rounds
+    assert ia == ib and a.pos == b.pos and rel(la, lb) < tol
+    for x, y in zip(a.bstate + a.conv_hist, b.bstate + b.conv_hist):
+        assert rel(x, y) < tol
+    assert rel(a.k_cache[0], b.k_cache[0]) < 50 * tol and rel(a.v_cache[0], b.v_cache[0]) < 50 * tol
+    if a.mtp is not None:
+        assert rel(a.mtp_k_cache, b.mtp_k_cache) < 50 * tol and a.mtp_h[0] == b.mtp_h[0]
+
+
+def test_small_model_batched_prompts_equal_stepping(small, monkeypatch):
+    from megakernels_b200 import engine as E
+    from megakernels_b200.synth import make_prompt
+    prompts, got = [make_prompt(small[0], n, seed=n) for n in (60, 9, 17, 100)], []
+    for rows in (16, 1 << 30):
+        mk = E.Megakernel(small[:2], max_seq=256, quant="int8", batch=4)
+        monkeypatch.setattr(E, "MIN_PROMPT_ROWS", rows)
+        got.append((mk.run_batch(prompts, n_generate=8), mk))
+    (ia, a), (ib, b) = got
+    assert ia == ib and a.bpos == b.bpos
+    for x, y in zip(a.bstate + a.bconv_hist, b.bstate + b.bconv_hist):
+        assert rel(x, y) < 2e-5
