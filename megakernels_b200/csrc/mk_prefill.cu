@@ -109,7 +109,7 @@ struct Exec {
         }
         for (auto& b : bufs) b.rows = arena.take<float>((size_t)rows * b.width);
         int kmax = 0, experts = 0, topk = 0;
-        size_t conv = 0, heads = 0, kheads = 0, vals = 0, q_w = 0, ex_k = 0, ex_n = 0, ex_f = 0, sh = 0;
+        size_t conv = 0, heads = 0, vals = 0, q_w = 0, ex_k = 0, ex_n = 0, ex_f = 0, sh = 0;
         for (int s = 0; s < n_stages; s++) {
             const mk_stage_desc& d = prog[s];
             auto up = [](size_t& a, size_t b) { if (b > a) a = b; };
@@ -132,7 +132,6 @@ struct Exec {
             } else if (d.op == MKS_OP_GDN) {
                 up(conv, d.i[MKS_I_CONV_DIM]);
                 up(heads, d.i[MKS_I_NVH]);
-                up(kheads, d.i[MKS_I_NKH]);
                 need_slab(d.p[MKS_P_Y2], d.i[MKS_I_NVH] * 128);
             } else if (d.op == MKS_OP_ATTN) {
                 up(q_w, (size_t)d.i[MKS_I_NQ] * d.i[MKS_I_HD]);
@@ -150,7 +149,7 @@ struct Exec {
             qkv = arena.take<float>((size_t)rows * conv);
             scal = arena.take<float4>((size_t)rows * heads);
             o = arena.take<float>((size_t)rows * vals);
-            gram = arena.take<float>((size_t)M * ((L + SCAN - 1) / SCAN) * kheads * 64);
+            gram = arena.take<float>((size_t)M * ((L + SCAN - 1) / SCAN) * heads * 80);
         }
         if (q_w) q = arena.take<__nv_bfloat16>((size_t)rows * q_w);
         if (experts) {

@@ -689,7 +689,7 @@ struct GdnArgs {
     // scratch
     float* qkv;                  // [rows][conv_dim]: normalised q, k, and v
     float4* scal;                // [rows][nvh]: decay, beta
-    float* gram;                 // [M][blocks of 8 positions][nkh][8][8] products of the block's keys and queries
+    float* gram;                 // [M][blocks of 8 positions][nvh][80]: see gdn_gram
     float* o;                    // [rows][nvh * 128]
     uint8_t* out;                // slabs of the gated output
     size_t out_piece;
@@ -778,11 +778,12 @@ static __global__ void __launch_bounds__(256) gdn_history(const __grid_constant_
 // so the sixteen products s k_t, s q_t of a block reduce together instead of one by one, and what is sequential are eight
 // scalar steps.
 constexpr int SCAN = 8;
-// k_i k_t (i < t) and q_i k_t (i >= t) of every block and key head: gram[t * 8 + i].  One warp each.
+// Per block and value head: k_i k_t (i < t) and q_i k_t (i >= t) with the decays between the two positions, [t][i], then
+// P_t and P_8 / P_t.  One warp per block and key head.
 static __global__ void __launch_bounds__(128) gdn_gram(const __grid_constant__ GdnArgs G) {
     const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, chunks = (G.L + SCAN - 1) / SCAN;
     if (w >= G.M * chunks * G.nkh) return;
-    const int kh = w % G.nkh, c = (w / G.nkh) % chunks, m = w / (G.nkh * chunks);
+    const int kh = w % G.nkh, c = (w / G.nkh) % chunks, m = w / (G.nkh * chunks), rep = G.nvh / G.nkh;
     float4 q[SCAN], k[SCAN];
 #pragma unroll
     for (int t = 0; t < SCAN; t++) {
@@ -812,9 +813,24 @@ static __global__ void __launch_bounds__(128) gdn_gram(const __grid_constant__ G
                 v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
     }
-    *reinterpret_cast<float2*>(G.gram + (size_t)w * 64 + 2 * lane) = make_float2(v[0], v[1]);
+    // per value head: entry (t, i) takes the decays between the two positions; a position past the end decays by 1
+    for (int r = 0; r < rep; r++) {
+        const int h = kh * rep + r, l = c * SCAN + (lane & 7);
+        const float dec = l < G.L ? G.scal[((size_t)m * G.L + l) * G.nvh + h].x : 1.f;
+        float d0 = 1.f, d1 = 1.f, p = 1.f;
+        const int t = lane >> 2, i = (lane & 3) * 2;
+#pragma unroll
+        for (int j = 0; j < SCAN; j++) {
+            const float dj = __shfl_sync(0xffffffffu, dec, j);
+            d0 *= j > min(t, i) && j <= max(t, i) ? dj : 1.f;
+            d1 *= j > min(t, i + 1) && j <= max(t, i + 1) ? dj : 1.f;
+            p *= (lane < 8 ? j <= lane : j > (lane & 7)) ? dj : 1.f;
+        }
+        float* out = G.gram + (((size_t)m * chunks + c) * G.nvh + h) * 80;
+        *reinterpret_cast<float2*>(out + 2 * lane) = make_float2(v[0] * d0, v[1] * d1);
+        if (lane < 16) out[64 + lane] = p;
+    }
 }
-
 __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
     u64 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
@@ -830,15 +846,14 @@ __device__ __forceinline__ float sum2(u64 a) { return __uint_as_float((uint32_t)
 
 // Four warps; eight lanes share R value rows of one head of one sequence (16 keys each, in registers, packed in pairs), so
 // a CTA holds 16 R rows and a head is 8 / R CTAs: R = 1 spreads a few heads over the chip, R = 2 reads shared memory once
-// for two rows when there are enough heads.
+// for two rows when there are enough heads.  16 heads x 511 positions: 70 us (207 position by position; 145 with the decay
+// products formed here instead of in gdn_gram, where their branches serialised 64 threads per block).
 template <int R>
 static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ GdnArgs G) {
     constexpr int ROWS = 16 * R, IN = 256 + ROWS;
     __shared__ __align__(16) float in_s[2][SCAN][IN];        // q | k | values
     __shared__ __align__(16) float4 sc_s[2][SCAN];           // decay, beta
-    __shared__ __align__(16) float gram_s[2][64];
-    __shared__ __align__(16) float mat_s[64];                // gram with the decays between the two positions
-    __shared__ float p_s[SCAN], e_s[SCAN];                   // P_t, P_8 / P_t
+    __shared__ __align__(16) float mats[2][80];           // what gdn_gram left for the block
     const int rep = G.nvh / G.nkh;
     const int m = blockIdx.z, h = blockIdx.y, v0 = blockIdx.x * ROWS, kh = h / rep;
     const int tid = threadIdx.x, part = tid & 7, rr = (tid >> 3) * R;
@@ -854,15 +869,23 @@ static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ G
             s[r][2 * i + 1] = a.y;
         }
     const size_t row0 = (size_t)m * G.L;
+    const float* qk_src = G.qkv + row0 * G.conv_dim + ((tid & 32) ? key_dim : 0) + kh * 128 + 4 * (tid & 31);
+    const float* v_src = G.qkv + row0 * G.conv_dim + 2 * key_dim + h * 128 + v0 + 4 * (tid % (ROWS / 4));
+    const float* m_src = G.gram + ((size_t)m * chunks * G.nvh + h) * 80 + 4 * (tid - 64);
+    const float4* s_src = G.scal + row0 * G.nvh + h;
     auto request = [&](int buf, int c) {
-        constexpr int PIECES = IN / 4;
-        for (int i = tid; i < SCAN * PIECES; i += 128) {
-            const int b = i / PIECES, x = i - b * PIECES, l = min(c * SCAN + b, G.L - 1);
-            const float* src = G.qkv + (row0 + l) * G.conv_dim + (x < 32 ? kh * 128 + 4 * x : (x < 64 ? key_dim + kh * 128 + 4 * (x - 32) : 2 * key_dim + h * 128 + v0 + 4 * (x - 64)));
-            mk::cp_async16(&in_s[buf][b][4 * x], src);
+        const int l0 = c * SCAN;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int b = (tid >> 6) + 2 * j;
+            mk::cp_async16(&in_s[buf][b][4 * (tid & 63)], qk_src + (size_t)min(l0 + b, G.L - 1) * G.conv_dim);
         }
-        if (tid < SCAN) mk::cp_async16(&sc_s[buf][tid], G.scal + (row0 + min(c * SCAN + tid, G.L - 1)) * G.nvh + h);
-        if (tid >= 32 && tid < 48) mk::cp_async16(&gram_s[buf][4 * (tid - 32)], G.gram + (((size_t)m * chunks + c) * G.nkh + kh) * 64 + 4 * (tid - 32));
+        if (tid < 2 * ROWS) {
+            const int b = tid / (ROWS / 4);
+            mk::cp_async16(&in_s[buf][b][256 + 4 * (tid % (ROWS / 4))], v_src + (size_t)min(l0 + b, G.L - 1) * G.conv_dim);
+        }
+        if (tid >= 64 && tid < 84) mk::cp_async16(&mats[buf][4 * (tid - 64)], m_src + (size_t)c * G.nvh * 80);
+        if (tid >= 96 && tid < 96 + SCAN) mk::cp_async16(&sc_s[buf][tid - 96], s_src + (size_t)min(l0 + tid - 96, G.L - 1) * G.nvh);
         mk::cp_async_commit();
     };
     request(0, 0);
@@ -874,21 +897,7 @@ static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ G
         if (c + 1 < chunks) request(buf ^ 1, c + 1);
         const int nb = min(SCAN, G.L - c * SCAN);
         // a position past the end decays by 1 and corrects by 0
-        if (tid < 64) {
-            const int t = tid >> 3, i = tid & 7, lo = min(t, i), hi = max(t, i);
-            float d = 1.f;
-#pragma unroll
-            for (int j = 0; j < SCAN; j++)
-                if (j > lo && j <= hi && j < nb) d *= sc_s[buf][j].x;
-            mat_s[tid] = gram_s[buf][tid] * d;
-        } else if (tid < 64 + 2 * SCAN) {
-            const int t = (tid - 64) & 7;
-            float d = 1.f;
-#pragma unroll
-            for (int j = 0; j < SCAN; j++)
-                if ((tid < 72 ? j <= t : j > t) && j < nb) d *= sc_s[buf][j].x;
-            (tid < 72 ? p_s : e_s)[t] = d;
-        }
+        const float *mat_s = mats[buf], *p_s = mats[buf] + 64, *e_s = mats[buf] + 72;
         // s k_t, s q_t over this lane's keys
         float u[R][16];
 #pragma unroll
@@ -927,7 +936,6 @@ static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ G
                         u[r][j] = keep + __shfl_xor_sync(0xffffffffu, send, x);
                     }
         }
-        __syncthreads();                                     // mat_s, p_s, e_s
         float delta[R][SCAN];
 #pragma unroll
         for (int t = 0; t < SCAN; t++) {

@@ -126,7 +126,7 @@ struct Run {
         scal = arena.take<float4>((size_t)rows * S::LIN_H);
         o = arena.take<float>((size_t)rows * S::LIN_V);
         q = arena.take<float>((size_t)rows * S::MIX);
-        gram = arena.take<float>((size_t)((rows + SCAN - 1) / SCAN) * S::LIN_H * 64);
+        gram = arena.take<float>((size_t)((rows + SCAN - 1) / SCAN) * S::LIN_H * 80);
         part = arena.take<float>((size_t)8 * rows * S::HID);
         pos = arena.take<int>(1);
     }
