@@ -225,12 +225,17 @@ typedef struct mk_prefill_args {
     int32_t sequence;        /* which of the engine's sequences (0 for single-sequence launches)   */
     int32_t batched;         /* 1: for mk_launch_batch (MK_L_CONV_HIST_B), 0: for mk_launch        */
     uint64_t resid_out;      /* optional fp32 [positions, hidden]: residual after the last layer   */
+    uint64_t weights;        /* what mk_prefill_weights has written                                */
     uint64_t workspace;      /* device scratch of mk_prefill_bytes                                 */
     int64_t workspace_bytes;
     int64_t spin_limit_ns;   /* bound on every device-side wait; 0 = 2 s                           */
 } mk_prefill_args;
 int mk_prefill(mk_engine* e, const mk_prefill_args* args, void* stream);
 int64_t mk_prefill_bytes(int positions);
+/* The engine's matrices as bf16 operand tiles, written once into `bytes` (mk_prefill_weight_bytes) of device memory that
+ * the caller keeps as long as the engine takes prompts in. */
+int mk_prefill_weights(mk_engine* e, uint64_t weights, int64_t bytes, void* stream);
+int64_t mk_prefill_weight_bytes(mk_engine* e);
 
 /* Replaces `watchdog_fired` (qwen3.5-0.8b/csrc/megakernel.cu:1284-1289): synchronises the device,
  * reads the status words of the last launch and returns MK_OK or MK_ERR_TIMEOUT.  Unlike the

@@ -265,8 +265,8 @@ int mk_stage_launch(const mk_stage_args* args, void* stream);
 
 /* A prompt through `program`, all positions at once: what `positions` decode steps with given tokens leave in the
  * states, caches and `pos`, computed as matrix products over batch x positions token rows (tcgen05) instead of step by
- * step.  The LM head is not run: feed the prompt's last token to mk_stage_launch.  `program` is a HOST copy of the
- * records.  Programs with two-piece inputs, int8 weights, an fp32 KV cache or all-reduces are MK_ERR_UNSUPPORTED.
+ * step.  The LM head is not run: either feed the prompt's last token to mk_stage_launch, or let this call take it in too
+ * (`last`) and launch the LM head's record alone.  `program` is a HOST copy of the records.  Programs with two-piece inputs, int8 weights, an fp32 KV cache or all-reduces are MK_ERR_UNSUPPORTED.
  * The reference takes a prompt in by one `step` per position (qwen3.8-27b-gfx942/mk/reference.py:378-386). */
 typedef struct mk_stage_prefill_args {
     uint64_t program;        /* host address of mk_stage_desc[n_stages]                             */
@@ -280,6 +280,10 @@ typedef struct mk_stage_prefill_args {
     uint64_t workspace;      /* device scratch of mk_stage_prefill_bytes                           */
     int64_t workspace_bytes;
     int64_t spin_limit_ns;   /* bound on every device-side wait; 0 = 2 s                           */
+    int32_t last;            /* 1: the prompt ends here.  The last position's residual and its sums of squares go to the
+                                program's own buffers and `pos` is advanced by positions - 1: a launch of an embedding
+                                record of width 0 and the LM head's record completes the step      */
+    int32_t reserved;
 } mk_stage_prefill_args;
 int mk_stage_prefill(const mk_stage_prefill_args* args, void* stream);
 

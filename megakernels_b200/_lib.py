@@ -27,7 +27,7 @@ GLOBAL_FIELDS = ["embed", "embed_scale", "lm_head", "lm_scale", "final_norm", "r
 QUERIES = ["SMEM_BYTES", "N_THREADS", "CONV_RING", "KV_BLOCK", "MAX_SPLITS", "PART_STRIDE", "OPS_PER_LAYER",
            "PROF_MAX_OPS", "PROF_FIELDS", "SPEC_T", "MAX_LAYERS", "LAYER_FIELDS", "GLOBAL_FIELDS", "SLOT_BYTES",
            "STAGES", "MAX_LM_ROWS", "MAX_BATCH", "BATCH_SMEM_BYTES"]
-EXPORTS = ["mk_create", "mk_destroy", "mk_set_params", "mk_launch", "mk_launch_static", "mk_launch_batch", "mk_prefill", "mk_prefill_bytes", "mk_status", "mk_query", "mk_bw_probe",
+EXPORTS = ["mk_create", "mk_destroy", "mk_set_params", "mk_launch", "mk_launch_static", "mk_launch_batch", "mk_prefill", "mk_prefill_bytes", "mk_prefill_weights", "mk_prefill_weight_bytes", "mk_status", "mk_query", "mk_bw_probe",
            "mk_plan_rows", "mk_plan_attn_chunk", "mk_last_error"]
 
 
@@ -69,7 +69,7 @@ class BatchArgs(ctypes.Structure):
 
 class PrefillArgs(ctypes.Structure):
     _fields_ = [("tokens", ctypes.c_uint64), ("positions", ctypes.c_int32), ("start_pos", ctypes.c_int32),
-                ("sequence", ctypes.c_int32), ("batched", ctypes.c_int32), ("resid_out", ctypes.c_uint64),
+                ("sequence", ctypes.c_int32), ("batched", ctypes.c_int32), ("resid_out", ctypes.c_uint64), ("weights", ctypes.c_uint64),
                 ("workspace", ctypes.c_uint64), ("workspace_bytes", ctypes.c_int64), ("spin_limit_ns", ctypes.c_int64)]
 
 
@@ -94,6 +94,10 @@ def load():
     lib.mk_launch_static.argtypes = [ctypes.c_void_p, P(LaunchArgs), ctypes.c_void_p]
     lib.mk_launch_batch.argtypes = [ctypes.c_void_p, P(BatchArgs), ctypes.c_void_p]
     lib.mk_prefill.argtypes = [ctypes.c_void_p, P(PrefillArgs), ctypes.c_void_p]
+    lib.mk_prefill_weights.argtypes = [ctypes.c_void_p, ctypes.c_uint64, ctypes.c_int64, ctypes.c_void_p]
+    lib.mk_prefill_weights.restype = ctypes.c_int
+    lib.mk_prefill_weight_bytes.argtypes = [ctypes.c_void_p]
+    lib.mk_prefill_weight_bytes.restype = ctypes.c_int64
     lib.mk_prefill_bytes.argtypes = [ctypes.c_int]
     lib.mk_prefill_bytes.restype = ctypes.c_int64
     lib.mk_status.argtypes = [ctypes.c_void_p, P(ctypes.c_int32)]

@@ -23,7 +23,7 @@ struct Exec {
     int* status;
     long long spin;
     cudaStream_t st;
-    bool dry;
+    bool h_last = false;
     Arena arena;
     std::vector<Buffer> bufs;
     std::vector<Slab> slabs;
@@ -71,7 +71,7 @@ struct Exec {
     static int format(const mk_stage_desc& d) {
         switch (d.i[MKS_I_FMT]) {
             case MKS_FMT_MXFP4: return W_MXFP4;
-            case MKS_FMT_FP8: return d.i[MKS_I_BLOCK_SCALES] ? W_FP8_BLOCK : W_FP8;
+            case MKS_FMT_FP8: return d.i[MKS_I_BLOCK_SCALES] ? W_FP8_PIECES : W_FP8;
             case MKS_FMT_BF16: return W_BF16;
             default: return -1;
         }
@@ -181,7 +181,9 @@ struct Exec {
         switch (format(d)) {
             case W_MXFP4: return launch_gemm<W_MXFP4, 1>(A, out, blocks, ntiles, items, st);
             case W_FP8: return launch_gemm<W_FP8, 1>(A, out, blocks, ntiles, items, st);
-            case W_FP8_BLOCK: return launch_gemm<W_FP8_BLOCK, 1>(A, out, blocks, ntiles, items, st);
+            case W_FP8_PIECES:
+                if (A.ksplit == 1 && A.nt * (A.kbs / 2) <= 512 && A.kbs % 2 == 0) return launch_gemm<W_FP8_BLOCK, 1>(A, out, blocks, ntiles, items, st);
+                return launch_gemm<W_FP8_PIECES, 1>(A, out, blocks, ntiles, items, st);
             default: return launch_gemm<W_BF16, 1>(A, out, blocks, ntiles, items, st);
         }
     }
@@ -387,6 +389,8 @@ struct Exec {
         route.kind = d.i[MKS_I_ROUTE_KIND];
         route.expert_scale = reinterpret_cast<const float*>(d.p[MKS_P_EXPERT_SCALE]);
         MKP_CUDA(cudaMemsetAsync(route.counts, 0, (3 * route.experts + 1) * sizeof(int), st));
+        route.ids_out = h_last ? reinterpret_cast<int*>(d.p[MKS_P_ROUTE_OUT]) : nullptr;
+        route.L = L;
         route_rows<<<(rows + 7) / 8, 256, 0, st>>>(route);
         route_plan<<<1, 256, 0, st>>>(route);
         route_slots<<<(rows * 8 + 255) / 256, 256, 0, st>>>(route);
@@ -427,7 +431,11 @@ struct Exec {
             }
             if (rc != MK_OK) return rc;
         }
-        advance_pos<<<1, 32, 0, st>>>(pos, M, L);
+        if (h_last) {
+            const mk_stage_desc& d = prog[0];
+            last_rows<<<M, 256, 0, st>>>(at(d.p[MKS_P_H]), L, d.i[MKS_I_HIDDEN], reinterpret_cast<float*>(d.p[MKS_P_H]), reinterpret_cast<float*>(d.p[MKS_P_H_SSQ]));
+        }
+        advance_pos<<<1, 32, 0, st>>>(pos, M, h_last ? L - 1 : L);
         MKP_CUDA(cudaGetLastError());
         return MK_OK;
     }
@@ -470,6 +478,7 @@ extern "C" int mk_stage_prefill(const mk_stage_prefill_args* a, void* stream) {
     E.tokens = reinterpret_cast<const int*>(a->tokens);
     E.pos = reinterpret_cast<int*>(a->pos);
     E.status = reinterpret_cast<int*>(a->status);
+    E.h_last = a->last != 0;
     E.spin = a->spin_limit_ns > 0 ? a->spin_limit_ns : 2000000000ll;
     E.st = static_cast<cudaStream_t>(stream);
     return E.run();

@@ -64,7 +64,11 @@ __device__ __forceinline__ void store_slab8(uint8_t* x, size_t piece_stride, int
 }
 
 // ---- matrix product ----------------------------------------------------------------------------------------
-enum { W_MXFP4 = 0, W_FP8, W_FP8_BLOCK, W_BF16, W_SLAB };      // how the weights come: packed tiles of a format, or bf16 slabs
+// How the weights come: packed tiles of a format, or bf16 slabs.  Block-scaled FP8 has two forms: few tokens per tile leave
+// room in tensor memory for an accumulator per 128-column block, and the epilogue adds them with their scales
+// (W_FP8_BLOCK, the decode kernel's arithmetic); many tokens do not, and the scaled weights enter as two exact bf16 pieces
+// (W_FP8_PIECES), at twice the MMAs.
+enum { W_MXFP4 = 0, W_FP8, W_FP8_BLOCK, W_FP8_PIECES, W_BF16, W_SLAB };
 enum { OUT_STORE = 0, OUT_ADD, OUT_GLU };
 
 struct GemmArgs {
@@ -155,16 +159,16 @@ __device__ __forceinline__ uint32_t e2m1x2_f16(uint32_t b) {
     asm("{\n .reg .b8 t;\n .reg .b16 h;\n cvt.u16.u32 h, %1;\n cvt.u8.u16 t, h;\n cvt.rn.f16x2.e2m1x2 %0, t;\n}\n" : "=r"(r) : "r"(b));
     return r;
 }
-__device__ __forceinline__ uint32_t e4m3x2_f16(uint32_t b) {
-    uint32_t r;
-    asm("{\n .reg .b16 h;\n cvt.u16.u32 h, %1;\n cvt.rn.f16x2.e4m3x2 %0, h;\n}\n" : "=r"(r) : "r"(b));
-    return r;
+// Two e4m3 values (bytes `sel` picks) moved to the bf16 fields: the values times 2^-120, subnormals included.
+__device__ __forceinline__ uint32_t e4m3_as_bf16(uint32_t w, uint32_t sel) {
+    const uint32_t b = __byte_perm(w, 0u, sel);                      // each byte in the upper half of its 16 bits
+    return (b & 0x80008000u) | ((b >> 4) & 0x07F007F0u);
 }
 // The bits of a half moved to the bf16 fields: the value times 2^-112 (halves of at most 7 mantissa bits, no subnormals).
 __device__ __forceinline__ uint32_t f16_as_bf16(uint32_t h) { return (h & 0x80008000u) | ((h >> 3) & 0x0FFF0FFFu); }
 
 // Raw bytes of one 64-column block of a 16-row tile, as lane (g, q) holds them.
-template <int FMT> struct Raw { uint4 q[FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2)]; uint32_t s[FMT == W_FP8_BLOCK ? 2 : 1]; };
+template <int FMT> struct Raw { uint4 q[FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2)]; uint32_t s[FMT == W_FP8_PIECES ? 2 : 1]; };
 
 // Walks the 64-column blocks of one tile through its units.
 template <int FMT>
@@ -185,10 +189,10 @@ struct Walk {
     }
     __device__ __forceinline__ void load(const GemmArgs& A, Raw<FMT>& r) {
         if (FMT == W_MXFP4) r.s[0] = __ldg(reinterpret_cast<const uint32_t*>(s));
-        if (FMT == W_FP8_BLOCK) {
+        if (FMT == W_FP8_PIECES) {
             const uint2 x = __ldg(reinterpret_cast<const uint2*>(s));
             r.s[0] = x.x;
-            r.s[FMT == W_FP8_BLOCK ? 1 : 0] = x.y;
+            r.s[FMT == W_FP8_PIECES ? 1 : 0] = x.y;
         }
 #pragma unroll
         for (int i = 0; i < STEPS; i++) {
@@ -203,7 +207,7 @@ struct Walk {
     __device__ __forceinline__ void step(const GemmArgs& A) {
         p += 512;
         if (FMT == W_MXFP4) s += 32;
-        if (FMT == W_FP8_BLOCK && (left & 3) == 1) s += 8;
+        if (FMT == W_FP8_PIECES && (left & 3) == 1) s += 8;
         if (--left == 0) {
             left = A.chunk_steps;
             p += A.chunk_bytes - A.chunk_steps * 512;
@@ -259,16 +263,16 @@ __device__ __forceinline__ void convert(const Raw<FMT>& r, uint2 (&v)[2][4], uin
                 }
         }
     } else {
-        constexpr uint32_t UP = 0x77807780u;       // 2^112
+        constexpr uint32_t UP = 0x7B807B80u;       // 2^120
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const uint32_t w[4] = {r.q[i].x, r.q[i].y, r.q[i].z, r.q[i].w};
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int h = k >> 1, j = 2 * i + (k & 1);
-                v[h][j].x = mul_bf16x2(f16_as_bf16(e4m3x2_f16(w[k])), UP);
-                v[h][j].y = mul_bf16x2(f16_as_bf16(e4m3x2_f16(w[k] >> 16)), UP);
-                if constexpr (FMT == W_FP8_BLOCK) {
+                v[h][j].x = mul_bf16x2(e4m3_as_bf16(w[k], 0x1404), UP);
+                v[h][j].y = mul_bf16x2(e4m3_as_bf16(w[k], 0x3424), UP);
+                if constexpr (FMT == W_FP8_PIECES) {
                     const uint32_t s = r.s[h] >> 16, ss = s | (s << 16), neg = 0xBF80BF80u;
                     const uint2 e = v[h][j];
                     v[h][j].x = mul_bf16x2(e.x, ss);
@@ -298,6 +302,15 @@ __device__ __forceinline__ void load16(uint32_t tmem, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Scale of weight row n in 128-column block b of block-scaled FP8: behind the chunk's steps, one for the upper and one for
+// the lower eight rows of a tile.
+__device__ __forceinline__ float block_scale(const GemmArgs& A, int group, int n, int b) {
+    const int tile = min(n >> 4, A.tiles - 1), split = b * 128 / A.kc, in = b - split * (A.kc / 128), per = A.chunk_steps / 4;
+    const size_t unit = (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
+    const uint8_t* chunk = A.w + (size_t)group * A.w_gstride + ((size_t)split * A.tiles + tile) * unit + (size_t)(in / per) * A.chunk_bytes;
+    return __ldg(reinterpret_cast<const float*>(chunk + A.chunk_steps * 512 + (in % per) * 8) + ((n >> 3) & 1));
+}
+
 // One CTA: 128 weight rows x nt token rows over a range of K.
 //   warps 0 .. 8 CG - 1  CG groups of eight convert weight tiles into the A operand (group c takes every CG-th block of 64
 //                        columns, warp w of a group tile w), then read the accumulators back (epilogue);
@@ -305,13 +318,13 @@ __device__ __forceinline__ void load16(uint32_t tmem, uint32_t (&r)[16]) {
 //   warp 8 CG + 1        one lane issues the MMAs.
 // grid: x = token tile (neighbouring CTAs share weights, so HBM reads them once), y = 128-row weight block, z = K split;
 // routed groups: x = weight block, y = work item.
-// PX: bf16 pieces of the token operand (3: fp32-exact inputs), weight pieces: 2 for block-scaled FP8, else 1.
+// PX: bf16 pieces of the token operand (3: fp32-exact inputs); weight pieces: 2 for W_FP8_PIECES, else 1.
 // Three-piece inputs keep the products of the first piece in an accumulator of their own: an accumulation rounds its sum
 // towards zero, and the small terms of pieces 2 and 3 would add two more such roundings per step to the large sum.
 template <int FMT, int PX, int OUT, int CG>
 static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) rows_gemm(const __grid_constant__ GemmArgs A) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    constexpr int PW = FMT == W_FP8_BLOCK ? 2 : 1, CW = 8 * CG;
+    constexpr int PW = FMT == W_FP8_PIECES ? 2 : 1, CW = 8 * CG;
     constexpr int DIST = FMT == W_BF16 ? 2 : (FMT == W_MXFP4 ? 6 : 4);        // blocks a lane requests ahead
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -333,8 +346,9 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
     const int kb0 = (int)((long long)A.kbs * z / A.ksplit), kb1 = (int)((long long)A.kbs * (z + 1) / A.ksplit);
     const uint32_t x_bytes = (uint32_t)nt * 128u, stage_bytes = PW * A_BYTES + PX * (uint32_t)A.nt * 128u;
     GemmBars& B = *reinterpret_cast<GemmBars*>(smem + (size_t)A.stages * stage_bytes);
+    const int blocks128 = FMT == W_FP8_BLOCK ? A.kbs / 2 : 1;   // (K splits do not occur with per-block accumulators)
     int cols = 32;
-    while (cols < A.nt * (PX > 1 ? 2 : 1)) cols *= 2;
+    while (cols < nt * (PX > 1 ? 2 : blocks128)) cols *= 2;
     if (threadIdx.x == 0) {
         for (int i = 0; i < A.stages; i++) {
             mbar_init(&B.full[i], FMT == W_SLAB ? 1 : 8 + 1);
@@ -398,10 +412,10 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
 #pragma unroll
                     for (int pw = 0; pw < PW; pw++) {
                         const uint64_t da = operand_desc(st + pw * A_BYTES), db = operand_desc(st + PW * A_BYTES + px * (uint32_t)A.nt * 128u);
-                        const uint32_t d = tmem + (px ? (uint32_t)A.nt : 0u);
+                        const uint32_t d = tmem + (px ? (uint32_t)nt : 0u) + (FMT == W_FP8_BLOCK ? (uint32_t)((kb >> 1) * nt) : 0u);
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
-                            const uint32_t accumulate = !(first && k == 0 && pw == 0 && px <= 1);
+                            const uint32_t accumulate = !((FMT == W_FP8_BLOCK ? !(kb & 1) : first != 0) && k == 0 && pw == 0 && px <= 1);
                             asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
                                          ::"r"(d), "l"(da + 2 * k), "l"(db + 2 * k), "r"(idesc), "r"(accumulate));
                         }
@@ -485,10 +499,20 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
                 {
                     uint32_t r[16];
                     load16(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)c0, r);
+                    const float s0 = FMT == W_FP8_BLOCK ? block_scale(A, group, n, 0) : 1.f;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+                    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]) * s0;
+                    if (FMT == W_FP8_BLOCK) {
+#pragma unroll 2
+                        for (int b = 1; b < blocks128; b++) {
+                            const float s = block_scale(A, group, n, b);
+                            load16(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)(b * nt + c0), r);
+#pragma unroll
+                            for (int i = 0; i < 16; i++) v[i] = fmaf(__uint_as_float(r[i]), s, v[i]);
+                        }
+                    }
                     if (PX > 1) {
-                        load16(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)(A.nt + c0), r);
+                        load16(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)(nt + c0), r);
 #pragma unroll
                         for (int i = 0; i < 16; i++) v[i] += __uint_as_float(r[i]);
                     }
@@ -649,6 +673,21 @@ static __global__ void __launch_bounds__(256) embed_rows(const __nv_bfloat16* ta
     }
 }
 
+// The last position of every sequence: its residual and the sums of squares per 16 elements, where a decode step leaves them.
+static __global__ void __launch_bounds__(256) last_rows(const float* h, int L, int H, float* out, float* ssq) {
+    const int m = blockIdx.x;
+    const float* src = h + ((size_t)m * L + L - 1) * H;
+    for (int g = threadIdx.x; g < H / 16; g += 256) {
+        float s = 0.f;
+        for (int i = 0; i < 16; i++) {
+            const float v = src[g * 16 + i];
+            out[(size_t)m * H + g * 16 + i] = v;
+            s += v * v;
+        }
+        ssq[(size_t)m * (H / 16) + g] = s;
+    }
+}
+
 static __global__ void advance_pos(int* pos, int M, int L) {
     if ((int)threadIdx.x < M) pos[threadIdx.x] += L;
 }
@@ -708,54 +747,70 @@ __device__ __forceinline__ float* conv_slot(const GdnArgs& G, int m, int ch, int
 }
 
 // Causal conv1d + SiLU of every channel, L2 norms of q and k, and the scalars of the recurrence.  One warp per 128
-// channels of a row, four channels per lane.
+// channels and CONV_ROWS consecutive rows, four channels per lane: the window slides through registers, so an input is read
+// once per CONV_ROWS + 3 rows instead of four times.
+constexpr int CONV_ROWS = 8;
 static __global__ void __launch_bounds__(256) gdn_conv(const __grid_constant__ GdnArgs G) {
-    const int row = blockIdx.y, m = row / G.L, l = row - m * G.L, lane = threadIdx.x & 31;
+    const int groups = (G.L + CONV_ROWS - 1) / CONV_ROWS, m = blockIdx.y / groups, l0 = (blockIdx.y - m * groups) * CONV_ROWS, lane = threadIdx.x & 31;
     const int blk = blockIdx.x * 8 + (threadIdx.x >> 5);                    // 128-channel block: q heads, k heads, v heads
     if (blk * 128 >= G.conv_dim) return;
     const int part = blk < G.nkh ? 0 : (blk < 2 * G.nkh ? 1 : 2);
     const int head = blk - part * G.nkh;
     const int col = (part == 0 ? G.q_off : (part == 1 ? G.k_off : G.v_off)) + head * 128 + 4 * lane;
-    const int ch = blk * 128 + 4 * lane;
-    const float* y = G.y + (size_t)row * G.y_stride + col;
-    const int pos = G.pos[m] + l;
-    float x[4][4];                                                          // [tap][channel], oldest first
-#pragma unroll
-    for (int d = 0; d < 4; d++) {
-        const int back = 3 - d;
-        if (l >= back) {
-            const float4 a = *reinterpret_cast<const float4*>(y - (long long)back * G.y_stride);
-            x[d][0] = a.x; x[d][1] = a.y; x[d][2] = a.z; x[d][3] = a.w;
-            if (back && G.conv_bf16) {
-#pragma unroll
-                for (int i = 0; i < 4; i++) x[d][i] = round_bf16(x[d][i]);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; i++) x[d][i] = conv_slot(G, m, ch + i, 0)[(pos - back) & (G.ring - 1)];
-        }
-    }
-    float v[4];
+    const int ch = blk * 128 + 4 * lane, pos = G.pos[m];
+    const float* y = G.y + (size_t)m * G.L * G.y_stride + col;
+    float w[4][4], x[4][4];                                                 // [tap][channel], oldest first
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const float4 w = __ldg(reinterpret_cast<const float4*>(G.conv_w) + ch + i);
-        float a = x[0][i] * w.x;
-        a = fmaf(x[1][i], w.y, a);
-        a = fmaf(x[2][i], w.z, a);
-        a = fmaf(x[3][i], w.w, a);
-        v[i] = silu_f(a);
+        const float4 a = __ldg(reinterpret_cast<const float4*>(G.conv_w) + ch + i);
+        w[0][i] = a.x; w[1][i] = a.y; w[2][i] = a.z; w[3][i] = a.w;
     }
-    if (part < 2) {
-        const float s = warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
-        float inv = G.l2_clamp ? 1.f / fmaxf(sqrtf(s), G.eps) : 1.f / sqrtf(s + G.eps);
-        if (part == 0) inv *= 0.08838834764831845f;                         // 128^-0.5
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[i] *= inv;
+    for (int d = 0; d < 3; d++) {
+        const int l = l0 - 3 + d;
+        if (l >= 0) {
+            const float4 a = *reinterpret_cast<const float4*>(y + (size_t)l * G.y_stride);
+            x[d + 1][0] = a.x; x[d + 1][1] = a.y; x[d + 1][2] = a.z; x[d + 1][3] = a.w;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (G.conv_bf16) x[d + 1][i] = round_bf16(x[d + 1][i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[d + 1][i] = conv_slot(G, m, ch + i, 0)[(pos + l) & (G.ring - 1)];
+        }
     }
-    *reinterpret_cast<float4*>(G.qkv + (size_t)row * G.conv_dim + ch) = make_float4(v[0], v[1], v[2], v[3]);
-    if (part == 2 && lane == 0) {
-        const float b = G.y[(size_t)row * G.y_stride + G.b_off + head], a = G.y[(size_t)row * G.y_stride + G.a_off + head];
-        G.scal[(size_t)row * G.nvh + head] = make_float4(expf(-expf(G.A_log[head]) * softplus_f(a + G.dt_bias[head])), sigmoid_f(b), 0.f, 0.f);
+    float4 in[CONV_ROWS];
+#pragma unroll
+    for (int r = 0; r < CONV_ROWS; r++)
+        if (l0 + r < G.L) in[r] = *reinterpret_cast<const float4*>(y + (size_t)(l0 + r) * G.y_stride);
+#pragma unroll
+    for (int r = 0; r < CONV_ROWS; r++) {
+        if (l0 + r >= G.L) break;
+        const size_t row = (size_t)m * G.L + l0 + r;
+        const float now[4] = {in[r].x, in[r].y, in[r].z, in[r].w};
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            x[0][i] = x[1][i]; x[1][i] = x[2][i]; x[2][i] = x[3][i];
+            float a = x[0][i] * w[0][i];
+            a = fmaf(x[1][i], w[1][i], a);
+            a = fmaf(x[2][i], w[2][i], a);
+            a = fmaf(now[i], w[3][i], a);
+            x[3][i] = G.conv_bf16 ? round_bf16(now[i]) : now[i];
+            v[i] = silu_f(a);
+        }
+        if (part < 2) {
+            const float s = warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
+            float inv = G.l2_clamp ? 1.f / fmaxf(sqrtf(s), G.eps) : 1.f / sqrtf(s + G.eps);
+            if (part == 0) inv *= 0.08838834764831845f;                     // 128^-0.5
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] *= inv;
+        }
+        *reinterpret_cast<float4*>(G.qkv + row * G.conv_dim + ch) = make_float4(v[0], v[1], v[2], v[3]);
+        if (part == 2 && lane == 0) {
+            const float b = G.y[row * G.y_stride + G.b_off + head], a = G.y[row * G.y_stride + G.a_off + head];
+            G.scal[row * G.nvh + head] = make_float4(expf(-expf(G.A_log[head]) * softplus_f(a + G.dt_bias[head])), sigmoid_f(b), 0.f, 0.f);
+        }
     }
 }
 
@@ -1273,9 +1328,11 @@ static __global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant
 
 // The same for the 0.8B model, whose attention is exact to fp32: queries, probabilities and an fp32 cache enter the
 // tensor cores as three bf16 pieces each, and of the nine piece products the six that reach above 2^-24 are formed (a
-// bf16 cache is one piece: three products).  Blocks of 32 keys; the fp32 rows of the next block wait in registers.
-constexpr int AF_KEYS = 32, AF_HD = 256, AF_RB = AF_HD * 2;
-template <bool KVF32> constexpr int attn_f32_smem() { return 3 * AT_ROWS * AF_RB + 2 * (KVF32 ? 3 : 1) * AF_KEYS * AF_RB + 3 * AT_ROWS * AF_KEYS * 2 + 4 * AT_ROWS * 4; }
+// bf16 cache is one piece: three products).  32 query rows per CTA (a 500-token prompt is then one CTA per SM), blocks of 32
+// keys: warp (r, d) takes rows 16 r .. 16 r + 15, scores keys 8 d .. 8 d + 7 and accumulates head dims 64 d .. 64 d + 63.
+// The fp32 rows of the next block wait in registers.
+constexpr int AF_ROWS = 32, AF_KEYS = 32, AF_HD = 256, AF_RB = AF_HD * 2;
+template <bool KVF32> constexpr int attn_f32_smem() { return 3 * AF_ROWS * AF_RB + 2 * (KVF32 ? 3 : 1) * AF_KEYS * AF_RB + 3 * AF_ROWS * AF_KEYS * 2 + 8 * AF_ROWS * 4; }
 // Four consecutive columns c .. c + 3 of a row, as NP pieces of swizzled rows
 template <int NP>
 __device__ __forceinline__ void split4(uint8_t* base, size_t piece, int row, int c, float4 v) {
@@ -1290,14 +1347,14 @@ __device__ __forceinline__ void split4(uint8_t* base, size_t piece, int row, int
 template <bool KVF32>
 static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_constant__ AttnArgs T) {
     extern __shared__ __align__(128) uint8_t sm[];
-    constexpr int KP = KVF32 ? 3 : 1, QB = AT_ROWS * AF_RB, KB = AF_KEYS * AF_RB, PB = AT_ROWS * AF_KEYS * 2;
+    constexpr int KP = KVF32 ? 3 : 1, QB = AF_ROWS * AF_RB, KB = AF_KEYS * AF_RB, PB = AF_ROWS * AF_KEYS * 2;
     constexpr int PER = AF_KEYS * AF_HD / 4 / 256;                        // groups of four columns per thread and block
     uint8_t *q_s = sm, *k_s = q_s + 3 * QB, *v_s = k_s + KP * KB, *p_s = v_s + KP * KB;
     float* st_s = reinterpret_cast<float*>(p_s + 3 * PB);
-    const int qpk = T.nq / T.nkv, bq = AT_ROWS / qpk;
+    const int qpk = T.nq / T.nkv, bq = AF_ROWS / qpk;
     const int m = blockIdx.z, kvh = blockIdx.y, l0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * bq;
     const int np = min(bq, T.L - l0), pos0 = T.pos[m] + l0, last = pos0 + np - 1;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp & 3, dh = warp >> 2, g = lane >> 2, t = lane & 3;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp & 1, dh = warp >> 1, g = lane >> 2, t = lane & 3;
     auto fetch = [&](const void* cache, int k0, float4 (&r)[PER]) {
 #pragma unroll
         for (int i = 0; i < PER; i++) {
@@ -1319,15 +1376,15 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
     };
     float4 kr[PER];
     fetch(T.k_cache, 0, kr);
-    for (int i = tid; i < AT_ROWS * AF_HD / 4; i += 256) {
+    for (int i = tid; i < AF_ROWS * AF_HD / 4; i += 256) {
         const int r = i / (AF_HD / 4), c = (i - r * (AF_HD / 4)) * 4, p = r / qpk, hq = r - p * qpk;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (p < np) v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(T.q) + (((size_t)m * T.L + l0 + p) * T.nq + kvh * qpk + hq) * AF_HD + c);
         split4<3>(q_s, QB, r, c, v);
     }
-    float o[AF_HD / 16][4], mx[2] = {-3.0e38f, -3.0e38f}, sum[2] = {0.f, 0.f};
+    float o[AF_HD / 32][4], mx[2] = {-3.0e38f, -3.0e38f}, sum[2] = {0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < AF_HD / 16; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    for (int i = 0; i < AF_HD / 32; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
     int qp[2];
 #pragma unroll
     for (int i = 0; i < 2; i++) qp[i] = pos0 + min((16 * rg + g + 8 * i) / qpk, np - 1);
@@ -1339,15 +1396,18 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
         float4 vr[PER];
         fetch(T.v_cache, k0, vr);
         __syncthreads();
-        float s[2][4];
-#pragma unroll
-        for (int i = 0; i < 2; i++) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};                               // 16 rows x 8 keys
 #pragma unroll 2
-        for (int kk = 0; kk < AF_HD / 16; kk++) {
-            uint32_t a[3][4], b[KP][4];
-            const uint32_t ca = 2 * kk + (lane >> 4), key = 16 * dh + (lane & 7) + ((lane >> 4) << 3), cb = 2 * kk + ((lane >> 3) & 1);
+        for (int kk = 0; kk < AF_HD / 32; kk++) {
+            uint32_t a[2][3][4], b[KP][4];
+            const uint32_t key = 8 * dh + (lane & 7), cb = 4 * kk + (lane >> 3);
 #pragma unroll
-            for (int p = 0; p < 3; p++) ldsm4(a[p], qa + p * QB + (((ca & ~7u) | ((ca ^ qx) & 7)) << 4));
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int p = 0; p < 3; p++) {
+                    const uint32_t ca = 4 * kk + 2 * h + (lane >> 4);
+                    ldsm4(a[h][p], qa + p * QB + (((ca & ~7u) | ((ca ^ qx) & 7)) << 4));
+                }
 #pragma unroll
             for (int p = 0; p < KP; p++) ldsm4(b[p], smem_u32(k_s) + p * KB + key * AF_RB + (((cb & ~7u) | ((cb ^ key) & 7)) << 4));
 #pragma unroll
@@ -1355,51 +1415,49 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
 #pragma unroll
                 for (int r = KP - 1; r >= 0; r--)
                     if (p + r < 3) {
-                        mma16816(s[0], a[p], b[r][0], b[r][1]);
-                        mma16816(s[1], a[p], b[r][2], b[r][3]);
+                        mma16816(s, a[0][p], b[r][0], b[r][1]);
+                        mma16816(s, a[1][p], b[r][2], b[r][3]);
                     }
         }
         float bm[2] = {-3.0e38f, -3.0e38f};
 #pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int p = k0 + 16 * dh + 8 * n + 2 * t + (i & 1), r = i >> 1;
-                s[n][i] = p <= qp[r] ? s[n][i] : -3.0e38f;
-                bm[r] = fmaxf(bm[r], s[n][i]);
-            }
+        for (int i = 0; i < 4; i++) {
+            const int p = k0 + 8 * dh + 2 * t + (i & 1), r = i >> 1;
+            s[i] = p <= qp[r] ? s[i] : -3.0e38f;
+            bm[r] = fmaxf(bm[r], s[i]);
+        }
 #pragma unroll
         for (int r = 0; r < 2; r++) {
             bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 1));
             bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 2));
-            if (t == 0) st_s[dh * AT_ROWS + 16 * rg + g + 8 * r] = bm[r];
+            if (t == 0) st_s[dh * AF_ROWS + 16 * rg + g + 8 * r] = bm[r];
         }
-        asm volatile("bar.sync %0, 64;" ::"r"(1 + rg) : "memory");
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + rg) : "memory");
         float f[2];
 #pragma unroll
         for (int r = 0; r < 2; r++) {
-            const float nm = fmaxf(mx[r], fmaxf(bm[r], st_s[(dh ^ 1) * AT_ROWS + 16 * rg + g + 8 * r]));
+            float nm = mx[r];
+#pragma unroll
+            for (int d = 0; d < 4; d++) nm = fmaxf(nm, st_s[d * AF_ROWS + 16 * rg + g + 8 * r]);
             f[r] = __expf(mx[r] - nm);
             mx[r] = nm;
             sum[r] *= f[r];
         }
 #pragma unroll
-        for (int n = 0; n < 2; n++)
+        for (int r = 0; r < 2; r++) {
+            float p0 = s[2 * r] > -2.9e38f ? __expf(s[2 * r] - mx[r]) : 0.f, p1 = s[2 * r + 1] > -2.9e38f ? __expf(s[2 * r + 1] - mx[r]) : 0.f;
+            sum[r] += p0 + p1;
+            const uint32_t row = 16 * rg + g + 8 * r;
 #pragma unroll
-            for (int r = 0; r < 2; r++) {
-                float p0 = s[n][2 * r] > -2.9e38f ? __expf(s[n][2 * r] - mx[r]) : 0.f, p1 = s[n][2 * r + 1] > -2.9e38f ? __expf(s[n][2 * r + 1] - mx[r]) : 0.f;
-                sum[r] += p0 + p1;
-                const uint32_t row = 16 * rg + g + 8 * r, c = 2 * dh + n;
-#pragma unroll
-                for (int q = 0; q < 3; q++) {
-                    const uint32_t w = pack_bf16(p0, p1);
-                    *reinterpret_cast<uint32_t*>(p_s + q * PB + row * 64 + ((c ^ ((row >> 1) & 3)) << 4) + t * 4) = w;
-                    p0 -= bf_lo(w);
-                    p1 -= bf_hi(w);
-                }
+            for (int q = 0; q < 3; q++) {
+                const uint32_t w = pack_bf16(p0, p1);
+                *reinterpret_cast<uint32_t*>(p_s + q * PB + row * 64 + ((dh ^ ((row >> 1) & 3)) << 4) + t * 4) = w;
+                p0 -= bf_lo(w);
+                p1 -= bf_hi(w);
             }
+        }
 #pragma unroll
-        for (int i = 0; i < AF_HD / 16; i++) {
+        for (int i = 0; i < AF_HD / 32; i++) {
             o[i][0] *= f[0]; o[i][1] *= f[0];
             o[i][2] *= f[1]; o[i][3] *= f[1];
         }
@@ -1413,8 +1471,8 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
 #pragma unroll
             for (int p = 0; p < 3; p++) ldsm4(a[p], smem_u32(p_s) + p * PB + row * 64 + (((2 * kk + (lane >> 4)) ^ ((row >> 1) & 3)) << 4));
 #pragma unroll
-            for (int n = 0; n < AF_HD / 32; n++) {
-                const uint32_t key = 16 * kk + (lane & 15), c = dh * 16 + 2 * n + (lane >> 4);
+            for (int n = 0; n < AF_HD / 64; n++) {
+                const uint32_t key = 16 * kk + (lane & 15), c = dh * 8 + 2 * n + (lane >> 4);
                 uint32_t b[KP][4];
 #pragma unroll
                 for (int p = 0; p < KP; p++) ldsm4_t(b[p], smem_u32(v_s) + p * KB + key * AF_RB + (((c & ~7u) | ((c ^ key) & 7)) << 4));
@@ -1433,19 +1491,19 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
     for (int r = 0; r < 2; r++) {
         sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
         sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
-        if (t == 0) st_s[(2 + dh) * AT_ROWS + 16 * rg + g + 8 * r] = sum[r];
+        if (t == 0) st_s[(4 + dh) * AF_ROWS + 16 * rg + g + 8 * r] = sum[r];
     }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < 2; r++) {
         const int rr = 16 * rg + g + 8 * r, p = rr / qpk, hq = kvh * qpk + rr - p * qpk;
         if (p >= np) continue;
-        const float inv = 1.f / (st_s[2 * AT_ROWS + rr] + st_s[3 * AT_ROWS + rr]);
+        const float inv = 1.f / ((st_s[4 * AF_ROWS + rr] + st_s[5 * AF_ROWS + rr]) + (st_s[6 * AF_ROWS + rr] + st_s[7 * AF_ROWS + rr]));
         const int row = m * T.L + l0 + p;
         const float* gate = T.y + (size_t)row * T.y_stride + T.q_off + (size_t)hq * T.q_hs + T.gate_off;
 #pragma unroll
-        for (int n = 0; n < AF_HD / 16; n++) {
-            const int dim = dh * (AF_HD / 2) + 8 * n + 2 * t;
+        for (int n = 0; n < AF_HD / 32; n++) {
+            const int dim = dh * (AF_HD / 4) + 8 * n + 2 * t;
             float a = o[n][2 * r] * inv * sigmoid_f(gate[dim]), b = o[n][2 * r + 1] * inv * sigmoid_f(gate[dim + 1]);
             uint8_t* dst = T.out + slab_offset(T.out_rows, row, hq * AF_HD + dim);
 #pragma unroll
@@ -1470,6 +1528,8 @@ struct RouteArgs {
     int* slot;                   // [rows][8] row of the token's k-th expert (ascending expert id) in the gathered order
     float* weight;               // [rows][8]
     float* gate;                 // [rows] shared expert's gate
+    int* ids_out;                // [sequences][topk] the last position's experts in rank order, or null
+    int L;
     int nt;
 };
 
@@ -1523,6 +1583,7 @@ static __global__ void __launch_bounds__(256) route_rows(const __grid_constant__
         R.slot[(size_t)row * 8 + rank] = myid;                           // the expert for now; route_slots turns it into a row
         R.weight[(size_t)row * 8 + rank] = myw / wsum * (R.kind == 1 && R.expert_scale ? R.expert_scale[myid] : 1.f);
         atomicAdd(R.counts + myid, 1);
+        if (R.ids_out && row % R.L == R.L - 1) R.ids_out[(row / R.L) * R.topk + lane] = myid;
     }
     if (R.kind == 0 && lane == 0) R.gate[row] = sigmoid_f(lg[R.experts]);
 }

@@ -3,8 +3,8 @@
 // The kernels are those of mk_prefill.cuh with fp32-exact operands: token rows enter the tensor cores as three bf16
 // pieces (24 bits), weights are exact in bf16 (int8 values need eight bits), sums are fp32 and the row scales of int8
 // weights are applied to them, so a prompt's state agrees with stepping to fp32 rounding.  The decode kernels' weight
-// layouts depend on the grid, so each layer's four matrices are first rewritten as bf16 slabs in scratch: 42 MB that
-// stay in L2 until the products that follow have read them.
+// layouts depend on the grid and are not operand tiles, so an engine that takes prompts in keeps a second copy of its
+// matrices as bf16 slabs (mk_prefill_weights, 1 GB; rewriting them in every pass cost a tenth of a 512-token prompt).
 #include "mk_prefill_host.h"
 
 using namespace mkp;
@@ -96,6 +96,30 @@ __global__ void __launch_bounds__(256) embed_rows_08b(const uint8_t* table, cons
 
 __global__ void put_pos(int* p, int v) { *p = v; }
 
+// Where a layer's four matrices lie among the slabs (rows rounded up to whole 128-row blocks).
+struct LayerSlabs {
+    const uint8_t *in, *out, *gu, *down, *end;
+    static size_t bytes(int rows, int k) { return (size_t)((rows + 127) / 128 * 128) * k * 2; }
+    LayerSlabs(const uint8_t* base, const mk::Params* P, int layer) {
+        for (int l = 0; l <= layer; l++) {
+            in = l ? end : base;
+            out = in + bytes(P->layer[l].kind ? S::ATT_IN : S::GDN_IN, S::HID);
+            gu = out + bytes(S::HID, S::MIX);
+            down = gu + bytes(2 * S::INTER, S::HID);
+            end = down + bytes(S::HID, S::INTER);
+        }
+    }
+};
+
+int to_slabs(const mk_model_desc* desc, const uint8_t* src, int N, int K, int unit, bool glu, const uint8_t* dst, cudaStream_t st) {
+    const bool q8 = desc->quant == MK_QUANT_INT8;
+    const int rb = q8 ? K : 2 * K, n = (int)(((long long)((N + 7) / 8) * (rb / 64) * 32 + 255) / 256);
+    auto fn = q8 ? slabs_from_rows<true> : slabs_from_rows<false>;
+    fn<<<n, 256, 0, st>>>(src, N, rb, unit, desc->grid, glu, const_cast<uint8_t*>(dst), (N + 127) / 128 * 128);
+    MKP_CUDA(cudaGetLastError());
+    return MK_OK;
+}
+
 struct Run {
     const mk_model_desc* desc;
     const mk::Params* P;
@@ -106,7 +130,8 @@ struct Run {
     Arena arena;
     float *h, *y, *part, *qkv, *o, *q, *gram;
     float4* scal;
-    uint8_t *x, *mix, *act, *w;
+    uint8_t *x, *mix, *act;
+    const uint8_t* slabs;
     size_t x_piece, mix_piece, act_piece;
     int* pos;
 
@@ -121,7 +146,6 @@ struct Run {
         x = arena.take<uint8_t>(PX * x_piece);
         mix = arena.take<uint8_t>(PX * mix_piece);
         act = arena.take<uint8_t>(PX * act_piece);
-        w = arena.take<uint8_t>((size_t)(S::PROJ_MAX + 127) / 128 * 128 * S::HID * 2);     // the in-projection is the largest matrix
         qkv = arena.take<float>((size_t)rows * S::CONV_DIM);
         scal = arena.take<float4>((size_t)rows * S::LIN_H);
         o = arena.take<float>((size_t)rows * S::LIN_V);
@@ -131,16 +155,7 @@ struct Run {
         pos = arena.take<int>(1);
     }
 
-    int convert(const uint8_t* src, int N, int K, int unit, bool glu) {
-        const bool q8 = desc->quant == MK_QUANT_INT8;
-        const int rb = q8 ? K : 2 * K;
-        const long long n = (long long)((N + 7) / 8) * (rb / 64) * 32;
-        if (q8) slabs_from_rows<true><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src, N, rb, unit, desc->grid, glu, w, (N + 127) / 128 * 128);
-        else slabs_from_rows<false><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src, N, rb, unit, desc->grid, glu, w, (N + 127) / 128 * 128);
-        MKP_CUDA(cudaGetLastError());
-        return MK_OK;
-    }
-    int product(int N, int K, const uint8_t* xs, size_t piece, const float* scale, int out, float* dst, int dst_stride) {
+    int product(const uint8_t* w, int N, int K, const uint8_t* xs, size_t piece, const float* scale, int out, float* dst, int dst_stride) {
         GemmArgs A;
         memset(&A, 0, sizeof A);
         A.w = w;
@@ -182,8 +197,8 @@ struct Run {
             const bool attn = L.kind != 0;
             const int in_rows = attn ? S::ATT_IN : S::GDN_IN;
             rows_in<PX><<<rows, 256, 0, st>>>(h, S::HID, S::HID, L.in_norm, 1.f, S::EPS, 1.f, x, x_piece, xrows);
-            if ((rc = convert(L.w_in, in_rows, S::HID, 1, false)) != MK_OK) return rc;
-            if ((rc = product(in_rows, S::HID, x, x_piece, L.s_in, OUT_STORE, y, S::PROJ_MAX)) != MK_OK) return rc;
+            const LayerSlabs W(slabs, P, l);
+            if ((rc = product(W.in, in_rows, S::HID, x, x_piece, L.s_in, OUT_STORE, y, S::PROJ_MAX)) != MK_OK) return rc;
             if (attn) {
                 AttnArgs T;
                 memset(&T, 0, sizeof T);
@@ -198,7 +213,7 @@ struct Run {
                 T.max_pages = P->max_seq / mk::KV_BLOCK; T.kv_shift = 6;
                 T.s_page = S::NKV * mk::KV_BLOCK * S::HD; T.s_head = mk::KV_BLOCK * S::HD; T.s_pos = S::HD;
                 T.pos = pos; T.q = q; T.out = mix; T.out_piece = mix_piece; T.out_rows = xrows;
-                const dim3 pg((S::NQ + 2 * S::NKV + 7) / 8, rows), ag((rows + AT_ROWS / S::QPK - 1) / (AT_ROWS / S::QPK), S::NKV, 1);
+                const dim3 pg((S::NQ + 2 * S::NKV + 7) / 8, rows), ag((rows + AF_ROWS / S::QPK - 1) / (AF_ROWS / S::QPK), S::NKV, 1);
                 if (kv32) {
                     attn_prepare<256, true, true><<<pg, 256, 0, st>>>(T);
                     MKP_CUDA(cudaFuncSetAttribute(attn_rows_f32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_f32_smem<true>()));
@@ -223,31 +238,49 @@ struct Run {
                 if ((rc = launch_gdn(G, gdn_gate<PX>, sms, st)) != MK_OK) return rc;
             }
             MKP_CUDA(cudaGetLastError());
-            // out-projection: rows where the engine keeps them, else the recurrence tasks' column slices
-            const uint8_t* w_out = attn ? L.w_out : L.w_out_rows;
-            if (w_out) {
-                if ((rc = convert(w_out, S::HID, S::MIX, 1, false)) != MK_OK) return rc;
-            } else {
-                slabs_from_cols<1><<<S::GDN_TASKS * (S::HID / 16) * 32 / 256, 256, 0, st>>>(L.w_out, S::GDN_TASKS, 0, w, S::HID);
-                MKP_CUDA(cudaGetLastError());
-            }
-            if ((rc = product(S::HID, S::MIX, mix, mix_piece, L.s_out, OUT_ADD, h, S::HID)) != MK_OK) return rc;
+            if ((rc = product(W.out, S::HID, S::MIX, mix, mix_piece, L.s_out, OUT_ADD, h, S::HID)) != MK_OK) return rc;
             rows_in<PX><<<rows, 256, 0, st>>>(h, S::HID, S::HID, L.post_norm, 1.f, S::EPS, 1.f, x, x_piece, xrows);
-            if ((rc = convert(L.w_gu, 2 * S::INTER, S::HID, 2, true)) != MK_OK) return rc;
-            if ((rc = product(2 * S::INTER, S::HID, x, x_piece, L.s_gu, OUT_GLU, nullptr, 0)) != MK_OK) return rc;
-            if (L.w_down_rows) {
-                if ((rc = convert(L.w_down_rows, S::HID, S::INTER, 1, false)) != MK_OK) return rc;
-            } else {
-                slabs_from_cols<2><<<(desc->grid * (S::HID / 16) * 32 + 255) / 256, 256, 0, st>>>(L.w_down, desc->grid, S::INTER, w, S::HID);
-                MKP_CUDA(cudaGetLastError());
-            }
-            if ((rc = product(S::HID, S::INTER, act, act_piece, L.s_down, OUT_ADD, h, S::HID)) != MK_OK) return rc;
+            if ((rc = product(W.gu, 2 * S::INTER, S::HID, x, x_piece, L.s_gu, OUT_GLU, nullptr, 0)) != MK_OK) return rc;
+            if ((rc = product(W.down, S::HID, S::INTER, act, act_piece, L.s_down, OUT_ADD, h, S::HID)) != MK_OK) return rc;
         }
         return MK_OK;
     }
 };
 
 }  // namespace
+
+extern "C" int64_t mk_prefill_weight_bytes(mk_engine* e) {
+    const mk_model_desc* desc;
+    const mk::Params* P;
+    if (!e || mk_engine_view(e, &desc, &P) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill_weight_bytes: mk_set_params has not succeeded on this engine");
+    return (int64_t)(LayerSlabs(nullptr, P, P->n_layers - 1).end - static_cast<const uint8_t*>(nullptr)) + 1024;
+}
+
+extern "C" int mk_prefill_weights(mk_engine* e, uint64_t weights, int64_t bytes, void* stream) {
+    const mk_model_desc* desc;
+    const mk::Params* P;
+    if (!e || !weights || mk_engine_view(e, &desc, &P) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill_weights: null argument or no parameters");
+    if (bytes < mk_prefill_weight_bytes(e)) return pfail(MK_ERR_BADARG, "mk_prefill_weights: %lld bytes, %lld needed", (long long)bytes, (long long)mk_prefill_weight_bytes(e));
+    const uint8_t* base = reinterpret_cast<const uint8_t*>((weights + 1023) & ~(uint64_t)1023);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    MKP_CUDA(cudaSetDevice(desc->device));
+    for (int l = 0; l < P->n_layers; l++) {
+        const mk::LayerP& L = P->layer[l];
+        const LayerSlabs W(base, P, l);
+        int rc = to_slabs(desc, L.w_in, L.kind ? S::ATT_IN : S::GDN_IN, S::HID, 1, false, W.in, st);
+        // the out- and down-projection: rows where the engine keeps them, else the column slices of the tasks / CTAs
+        const uint8_t* w_out = L.kind ? L.w_out : L.w_out_rows;
+        if (rc == MK_OK && w_out) rc = to_slabs(desc, w_out, S::HID, S::MIX, 1, false, W.out, st);
+        else if (rc == MK_OK) slabs_from_cols<1><<<S::GDN_TASKS * (S::HID / 16) * 32 / 256, 256, 0, st>>>(L.w_out, S::GDN_TASKS, 0, const_cast<uint8_t*>(W.out), S::HID);
+        if (rc == MK_OK) rc = to_slabs(desc, L.w_gu, 2 * S::INTER, S::HID, 2, true, W.gu, st);
+        if (rc == MK_OK && L.w_down_rows) rc = to_slabs(desc, L.w_down_rows, S::HID, S::INTER, 1, false, W.down, st);
+        else if (rc == MK_OK)
+            slabs_from_cols<2><<<(desc->grid * (S::HID / 16) * 32 + 255) / 256, 256, 0, st>>>(L.w_down, desc->grid, S::INTER, const_cast<uint8_t*>(W.down), S::HID);
+        if (rc != MK_OK) return rc;
+        MKP_CUDA(cudaGetLastError());
+    }
+    return MK_OK;
+}
 
 extern "C" int64_t mk_prefill_bytes(int positions) {
     if (positions < 1) return pfail(MK_ERR_BADARG, "mk_prefill_bytes: %d positions", positions);
@@ -263,7 +296,7 @@ extern "C" int mk_prefill(mk_engine* e, const mk_prefill_args* a, void* stream) 
     Run R;
     memset(&R, 0, sizeof R);
     if (mk_engine_view(e, &R.desc, &R.P) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill: mk_set_params has not succeeded on this engine");
-    if (a->positions < 1 || !a->tokens || !a->workspace) return pfail(MK_ERR_BADARG, "mk_prefill: positions %d, tokens / workspace missing", a->positions);
+    if (a->positions < 1 || !a->tokens || !a->workspace || !a->weights) return pfail(MK_ERR_BADARG, "mk_prefill: positions %d, tokens / weights / workspace missing", a->positions);
     if (a->start_pos < 0 || (int64_t)a->start_pos + a->positions > R.desc->max_seq) return pfail(MK_ERR_BADARG, "mk_prefill: sequence would exceed max_seq=%d", R.desc->max_seq);
     if (a->sequence < 0 || a->sequence >= (R.desc->max_batch > 1 ? R.desc->max_batch : 1)) return pfail(MK_ERR_BADARG, "mk_prefill: sequence %d", a->sequence);
     for (int l = 0; l < R.P->n_layers; l++)
@@ -275,6 +308,7 @@ extern "C" int mk_prefill(mk_engine* e, const mk_prefill_args* a, void* stream) 
     R.seq = a->sequence;
     R.batched = a->batched;
     R.tokens = reinterpret_cast<const int*>(a->tokens);
+    R.slabs = reinterpret_cast<const uint8_t*>((a->weights + 1023) & ~(uint64_t)1023);
     R.spin = a->spin_limit_ns > 0 ? a->spin_limit_ns : 2000000000ll;
     R.st = static_cast<cudaStream_t>(stream);
     R.arena.base = reinterpret_cast<uint8_t*>((a->workspace + 1023) & ~(uint64_t)1023);

@@ -52,7 +52,7 @@ int launch_gemm_cg(GemmArgs& A, int out, dim3 grid, int smem, cudaStream_t st) {
 
 template <int FMT, int PX>
 int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaStream_t st) {
-    constexpr int PW = FMT == W_FP8_BLOCK ? 2 : 1;
+    constexpr int PW = FMT == W_FP8_PIECES ? 2 : 1;
     const int stage = PW * A_BYTES + PX * A.nt * 128, fixed = (int)sizeof(GemmBars) + 1024;
     // Narrow tiles leave room for two CTAs per SM with three stages each: one's start and end hide behind the other.  Wide
     // ones have the SM to themselves, with sixteen warps to convert weights (eight cannot keep up with the MMAs).
@@ -79,11 +79,11 @@ int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaSt
 // The DeltaNet mixer of M sequences of L rows; `gate` is gdn_gate of the wanted number of pieces.
 inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), int sms, cudaStream_t st) {
     const int rows = G.M * G.L, chunks = (G.L + SCAN - 1) / SCAN;
-    gdn_conv<<<dim3((G.conv_dim / 128 + 7) / 8, rows), 256, 0, st>>>(G);
+    gdn_conv<<<dim3((G.conv_dim / 128 + 7) / 8, G.M * ((G.L + CONV_ROWS - 1) / CONV_ROWS)), 256, 0, st>>>(G);
     gdn_history<<<dim3((G.conv_dim + 255) / 256, G.M, G.ring), 256, 0, st>>>(G);
     gdn_gram<<<(G.M * chunks * G.nkh + 3) / 4, 128, 0, st>>>(G);
-    // two rows per lane once that leaves two CTAs per SM
-    if (G.M * G.nvh * 4 >= 2 * sms) gdn_scan<2><<<dim3(4, G.nvh, G.M), 128, 0, st>>>(G);
+    // one row per lane while that is about one CTA per SM (latency decides); with more, shared-memory reads do: two rows
+    if (2 * G.M * G.nvh * 8 > 3 * sms) gdn_scan<2><<<dim3(4, G.nvh, G.M), 128, 0, st>>>(G);
     else gdn_scan<1><<<dim3(8, G.nvh, G.M), 128, 0, st>>>(G);
     gate<<<dim3((G.nvh + 15) / 16, rows), 256, 0, st>>>(G);
     MKP_CUDA(cudaGetLastError());

@@ -276,6 +276,7 @@ class Megakernel:
         self.last_step_ns = []
         self.launches = 0
         self._workspace = None          # of the token-parallel prompt path, grown to the largest pass so far
+        self._prompt_weights = None     # the matrices as that path reads them, laid out at the first prompt
         self.reset()
 
     # ------------------------------------------------------------------------------------------
@@ -324,8 +325,8 @@ class Megakernel:
 
     def reset(self):
         """Start a new sequence (cached K/V need no clearing: positions are rewritten)."""
-        for t in self.conv_hist + self.bconv_hist + self.bstate + self.ll:
-            t.zero_()
+        torch._foreach_zero_(self.conv_hist + self.bconv_hist + self.bstate)      # a handful of launches for 54 tensors
+        torch._foreach_zero_(self.ll)
         self._mode = None              # "single" or "batch": the two kinds of launch keep separate conv histories
         self.bpos = [0] * self.batch   # position of every sequence; `pos` is that of sequence 0
         self.attn_part.zero_()
@@ -389,10 +390,16 @@ class Megakernel:
             self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
         ids = torch.tensor(tokens, dtype=torch.int32).to(self.device)
         stream = torch.cuda.current_stream(self.device).cuda_stream
+        if self._prompt_weights is None:
+            w = torch.empty(int(self.lib.mk_prefill_weight_bytes(self._h)), dtype=torch.uint8, device=self.device)
+            _lib.check(self.lib.mk_prefill_weights(self._h, w.data_ptr(), w.numel(), ctypes.c_void_p(stream)))
+            torch.cuda.current_stream(self.device).synchronize()      # complete before a launch on any stream reads it
+            self._prompt_weights = w
         for lo in range(0, n, MAX_PROMPT_ROWS):
             rows = min(MAX_PROMPT_ROWS, n - lo)
             a = _lib.PrefillArgs(tokens=ids.data_ptr() + 4 * lo, positions=rows, start_pos=start + lo, sequence=seq, batched=int(batched),
-                                 resid_out=hidden[lo:].data_ptr() if hidden is not None else 0, workspace=self._workspace.data_ptr(),
+                                 resid_out=hidden[lo:].data_ptr() if hidden is not None else 0,
+                                 weights=self._prompt_weights.data_ptr(), workspace=self._workspace.data_ptr(),
                                  workspace_bytes=self._workspace.numel(), spin_limit_ns=self.spin_limit_ns)
             _lib.check(self.lib.mk_prefill(self._h, ctypes.byref(a), ctypes.c_void_p(stream)))
             self.launches += 1
@@ -729,7 +736,6 @@ class Megakernel:
 
     def restore(self, snap):
         tensors, pos, mode = snap
-        for dst, src in zip(self.conv_hist + self.bconv_hist + self.bstate, tensors):
-            dst.copy_(src)
+        torch._foreach_copy_(self.conv_hist + self.bconv_hist + self.bstate, tensors)
         self.bpos = list(pos)
         self._mode = mode

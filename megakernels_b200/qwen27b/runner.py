@@ -193,14 +193,12 @@ class Engine:
 
     def prefill(self, prompts):
         """Takes the prompts (M lists of equal length) in and returns the logits after the last position: what the
-        reference does with one `step` per position (`mk/reference.py:378-386`).  All positions but the last go through
-        the token-parallel path (`Runtime.prefill`), the last one and short prompts through the decode kernel."""
+        reference does with one `step` per position (`mk/reference.py:378-386`).  Long prompts go through the
+        token-parallel path, short ones through the decode kernel (`Runtime.prefill`)."""
         if len(prompts) != self.M or len({len(p) for p in prompts}) != 1 or not prompts[0]:
             raise ValueError(f"prefill takes {self.M} prompts of one common, non-zero length")
         toks = torch.tensor(prompts, dtype=torch.int32).t().contiguous().to(self.device)      # [L, M]
-        taken = self.rt.prefill(toks)                        # all positions at once, but the last
-        self.rt.tok[: self.M].copy_(toks[taken])
-        self.rt.launch(toks.shape[0] - taken, tokens_in=toks[taken:])
+        self.rt.prefill(toks)
         self._prompt = toks                                  # alive until the launch has run
         return self.logits
 

@@ -187,9 +187,7 @@ class Engine:
         if len(prompts) != self.M or len({len(p) for p in prompts}) != 1 or not prompts[0]:
             raise ValueError(f"prefill takes {self.M} prompts of one common, non-zero length")
         toks = torch.tensor(prompts, dtype=torch.int32).t().contiguous().to(self.device)
-        taken = self.rt.prefill(toks)                        # all positions at once, but the last
-        self.rt.tok[: self.M].copy_(toks[taken])
-        self.rt.launch(toks.shape[0] - taken, tokens_in=toks[taken:])
+        self.rt.prefill(toks)
         self._prompt = toks
         return self.logits
 

@@ -62,7 +62,7 @@ class PrefillArgs(ctypes.Structure):
     _fields_ = [("program", ctypes.c_uint64), ("n_stages", ctypes.c_int32), ("batch", ctypes.c_int32),
                 ("positions", ctypes.c_int32), ("device", ctypes.c_int32), ("tokens", ctypes.c_uint64), ("pos", ctypes.c_uint64),
                 ("status", ctypes.c_uint64), ("workspace", ctypes.c_uint64), ("workspace_bytes", ctypes.c_int64),
-                ("spin_limit_ns", ctypes.c_int64)]
+                ("spin_limit_ns", ctypes.c_int64), ("last", ctypes.c_int32), ("reserved", ctypes.c_int32)]
 
 
 STAGE_EXPORTS = ["mk_stage_launch", "mk_stage_prefill", "mk_stage_prefill_bytes", "mk_stage_validate", "mk_stage_count", "mk_stage_query", "mk_stage_scratch_bytes", "mk_sync_probe", "mk_peer_alloc", "mk_peer_open",

@@ -173,6 +173,7 @@ class Runtime:
         self.spin_limit_ns = int(spin_limit_ms * 1e6)
         self.launches = 0
         self._workspace = None          # of the token-parallel prompt path, grown to the largest pass so far
+        self._head = None
 
     def reset(self):
         self.pos.zero_()
@@ -180,12 +181,13 @@ class Runtime:
             if t.dtype == torch.int32:
                 t.zero_()
 
-    def launch(self, n_steps=1, tokens_out=None, prof=None, stream=None, n_stages=None, prof_cta=0, tokens_in=None, row_valid=None):
-        """`n_stages` runs only a prefix of the program (one step; for stage-by-stage checks in tests)."""
-        full = n_stages is None
-        n_stages = self.n_stages if full else n_stages
+    def launch(self, n_steps=1, tokens_out=None, prof=None, stream=None, n_stages=None, prof_cta=0, tokens_in=None, row_valid=None, program=None):
+        """`n_stages` runs only a prefix of the program (one step; for stage-by-stage checks in tests); `program`, a (device
+        copy, records) pair whose records all end in a barrier, another one."""
+        full = n_stages is None and program is None
+        n_stages = program[1] if program is not None else (self.n_stages if full else n_stages)
         assert full or n_steps == 1
-        a = D.StageArgs(program=self.program_dev.data_ptr(), n_stages=n_stages, batch=self.M, n_steps=n_steps,
+        a = D.StageArgs(program=(program[0] if program is not None else self.program_dev).data_ptr(), n_stages=n_stages, batch=self.M, n_steps=n_steps,
                         device=self.device.index, tok=self.tok.data_ptr(), pos=self.pos.data_ptr(),
                         tokens_out=tokens_out.data_ptr() if tokens_out is not None else 0, barrier=self.bar.data_ptr(),
                         barrier_base=self.bar_base, status=self.status.data_ptr(), spin_limit_ns=self.spin_limit_ns,
@@ -200,7 +202,9 @@ class Runtime:
         st = stream if stream is not None else torch.cuda.current_stream(self.device)
         _lib.check(self.lib.mk_stage_launch(ctypes.byref(a), ctypes.c_void_p(st.cuda_stream)))
         nb, na = self.barriers_per_step, self.allreduces_per_step
-        if not full:
+        if program is not None:
+            nb, na = n_stages, 0
+        elif not full:
             nb = sum(1 for d in self.prog.stages[:n_stages] if not d.flags & D.MKS_FLAG_NO_BARRIER)
             na = sum(1 for d in self.prog.stages[:n_stages] if d.op == D.MKS_OP_GEMV and d.i[D.MKS_I_ALLREDUCE])
         self.bar_base += nb * n_steps * self.grid
@@ -208,30 +212,43 @@ class Runtime:
         self.launches += 1
 
     def prefill(self, tokens):
-        """Takes in all positions of `tokens` (int32 [L, M] on the device) but the last through the token-parallel path, in
-        passes of at most MAX_ROWS rows, and returns how many: 0 for a short prompt or a program that path cannot run
-        (two-piece inputs, tensor parallelism).  The caller feeds the rest to `launch`."""
-        todo = tokens.shape[0] - 1
-        if todo < MIN_ROWS_PATH - 1 or self.tp > 1:
-            return 0
-        passes = -(-todo * self.M // MAX_ROWS)
-        each = -(-todo // passes)
-        need = int(self.lib.mk_stage_prefill_bytes(self.host, self.n_stages, self.M, each, self.device.index))
-        if need == _lib.MK_ERR_UNSUPPORTED:
-            return 0
+        """A prompt of every sequence: `tokens` int32 [L, M] on the device.  Long ones go through the token-parallel path in
+        passes of at most MAX_ROWS rows, and only the LM head runs in the decode kernel; short ones, and programs that path
+        cannot run (two-piece inputs, tensor parallelism), step through the decode kernel."""
+        L = tokens.shape[0]
+        passes = -(-L * self.M // MAX_ROWS)
+        each = -(-L // passes)
+        need = _lib.MK_ERR_UNSUPPORTED
+        if L >= MIN_ROWS_PATH and self.tp == 1:
+            need = int(self.lib.mk_stage_prefill_bytes(self.host, self.n_stages, self.M, each, self.device.index))
+            if need < 0 and need != _lib.MK_ERR_UNSUPPORTED:
+                _lib.check(need)
+        self.tok[: self.M].copy_(tokens[0])
         if need < 0:
-            _lib.check(need)
+            return self.launch(L, tokens_in=tokens)
         if self._workspace is None or self._workspace.numel() < need:
             self._workspace = None
             self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
         stream = torch.cuda.current_stream(self.device).cuda_stream
-        for lo in range(0, todo, each):
-            part = tokens[lo: min(lo + each, todo)]
+        for lo in range(0, L, each):
+            part = tokens[lo: min(lo + each, L)]
             a = D.PrefillArgs(program=ctypes.addressof(self.host), n_stages=self.n_stages, batch=self.M, positions=part.shape[0],
                               device=self.device.index, tokens=part.data_ptr(), pos=self.pos.data_ptr(), status=self.status.data_ptr(),
-                              workspace=self._workspace.data_ptr(), workspace_bytes=self._workspace.numel(), spin_limit_ns=self.spin_limit_ns)
+                              workspace=self._workspace.data_ptr(), workspace_bytes=self._workspace.numel(), spin_limit_ns=self.spin_limit_ns,
+                              last=int(lo + each >= L))
             _lib.check(self.lib.mk_stage_prefill(ctypes.byref(a), ctypes.c_void_p(stream)))
-        return todo
+        self.launch(1, program=self._head_program())
+
+    def _head_program(self):
+        """The records that complete a step whose layers have run: an embedding of width 0 (which keeps the token choice at
+        the end of the launch) and, if there is one, the LM head."""
+        if self._head is None:
+            first, last = D.StageDesc.from_buffer_copy(self.host[0]), self.host[self.n_stages - 1]
+            first.i[D.K["MKS_I_HIDDEN"]] = 0
+            records = [first] + ([last] if last.op == D.MKS_OP_GEMV and last.i[D.MKS_I_EPILOGUE] == D.MKS_E_LOGITS else [])
+            arr = (D.StageDesc * len(records))(*records)
+            self._head = torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8).to(self.device), len(records)
+        return self._head
 
     def check(self):
         """Synchronise and raise if a device-side wait ran out in any launch so far."""
