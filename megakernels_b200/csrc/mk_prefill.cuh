@@ -170,19 +170,18 @@ __device__ __forceinline__ uint32_t f16_as_bf16(uint32_t h) { return (h & 0x8000
 // Raw bytes of one 64-column block of a 16-row tile, as lane (g, q) holds them.
 template <int FMT> struct Raw { uint4 q[FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2)]; uint32_t s[FMT == W_FP8_PIECES ? 2 : 1]; };
 
-// Walks the 64-column blocks of one tile through its units.
+// Walks the 64-column blocks of one tile: its units follow one another.
 template <int FMT>
 struct Walk {
     static constexpr int STEPS = FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2);      // 512-byte steps per 64 columns
     const uint8_t *p, *s;      // this lane's bytes of the next step; the current chunk's scales
-    int left, st;              // steps left in the chunk and in the unit
+    int left;                  // steps left in the chunk
     __device__ __forceinline__ void start(const GemmArgs& A, const uint8_t* w, int tile, int kb, int lane) {
         constexpr int STEP_K = 64 / STEPS;
         const int split = kb * 64 / A.kc, at = (kb * 64 - split * A.kc) / STEP_K;
         const size_t unit = (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
         const int within = at % A.chunk_steps;
-        const uint8_t* chunk = w + ((size_t)split * A.tiles + tile) * unit + (size_t)(at / A.chunk_steps) * A.chunk_bytes;
-        st = A.unit_steps - at;
+        const uint8_t* chunk = w + ((size_t)tile * (A.kbs * 64 / A.kc) + split) * unit + (size_t)(at / A.chunk_steps) * A.chunk_bytes;
         left = A.chunk_steps - within;
         p = chunk + within * 512 + lane * 16;
         s = chunk + A.chunk_steps * 512 + (FMT == W_MXFP4 ? within * 32 + (lane >> 2) * 4 : (within >> 2) * 8);
@@ -212,12 +211,6 @@ struct Walk {
             left = A.chunk_steps;
             p += A.chunk_bytes - A.chunk_steps * 512;
             s += A.chunk_bytes - (FMT == W_MXFP4 ? A.chunk_steps * 32 : A.chunk_steps * 2);
-        }
-        if (--st == 0) {                   // the same tile of the next split
-            st = A.unit_steps;
-            const size_t jump = (size_t)(A.tiles - 1) * (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
-            p += jump;
-            s += jump;
         }
     }
 };
@@ -307,7 +300,7 @@ __device__ __forceinline__ void load16(uint32_t tmem, uint32_t (&r)[16]) {
 __device__ __forceinline__ float block_scale(const GemmArgs& A, int group, int n, int b) {
     const int tile = min(n >> 4, A.tiles - 1), split = b * 128 / A.kc, in = b - split * (A.kc / 128), per = A.chunk_steps / 4;
     const size_t unit = (size_t)(A.unit_steps / A.chunk_steps) * A.chunk_bytes;
-    const uint8_t* chunk = A.w + (size_t)group * A.w_gstride + ((size_t)split * A.tiles + tile) * unit + (size_t)(in / per) * A.chunk_bytes;
+    const uint8_t* chunk = A.w + (size_t)group * A.w_gstride + ((size_t)tile * (A.kbs * 64 / A.kc) + split) * unit + (size_t)(in / per) * A.chunk_bytes;
     return __ldg(reinterpret_cast<const float*>(chunk + A.chunk_steps * 512 + (in % per) * 8) + ((n >> 3) & 1));
 }
 

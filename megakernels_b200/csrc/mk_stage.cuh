@@ -2,20 +2,22 @@
 // decode steps of up to eight sequences.
 //
 // What a step does is a program of mk_stage_desc records (include/mk_stage.h) in device memory.
-// Every CTA has 16 consumer warps and one producer warp:
+// Every CTA has 16 consumer warps and one scout warp:
 //
-//   * the producer's elected lane walks the program and, for every GEMV stage, issues this CTA's weight
-//     chunks (1-D bulk copies completing on mbarriers) into a shared-memory ring, in exactly the order
-//     the consumer warps will ask for them.  It never looks at activations (except the routed expert
-//     list), so weights of later stages land while the consumers wait at a grid barrier;
-//   * a GEMV stage is cut into units: (group, K split, 16-row tile).  A CTA owns a contiguous range of
-//     units; inside it each consumer warp takes whole units, converts the weight bytes to fp16 in
-//     registers (bf16 stays bf16) and multiplies with `mma.sync.m16n8k16`: the weight tile is the
-//     16-row A operand, the sequences are the eight B columns, so one to eight sequences cost the same
-//     number of instructions.  Nothing in the GEMV needs a CTA-wide barrier: a warp waits for its own
-//     chunks and releases them itself;
-//   * units that add up into one output tile (K splits, routed experts) meet through a counter: each
-//     writes its 16 x 8 partial tile, the last arrival adds them in a fixed order and runs the epilogue
+//   * every consumer warp owns a few slots of a shared-memory ring and feeds them itself: a lane copies (cp.async) the very
+//     bytes it will multiply, four tile steps ahead at a time, so a slot needs no barrier and no other warp has to notice
+//     that it is free.  The stream runs ahead across stage boundaries: weights of the next matrix land while the warp
+//     waits at a grid barrier.  It never depends on activations, except for the routed expert list;
+//   * the scout walks the program ahead of the consumers and leaves each GEMV stage's geometry (this CTA's tiles and
+//     columns) in shared memory, so that a warp that runs into the next stage does not wait for global memory;
+//   * a GEMV stage is cut into panels of input columns (usually one: the whole row) and 16-row tiles.  A CTA stages one
+//     panel's input and takes an even share of the panel's tiles; its sixteen warps take even shares of the CTA's weight
+//     chunks, in order, so a warp multiplies whole rows and at most shares its first and its last tile with its
+//     neighbours (summed through shared memory).  The weight bytes become fp16 in registers (bf16 stays bf16) and
+//     multiply with `mma.sync.m16n8k16`: the weight tile is the 16-row A operand, the sequences are the eight B columns,
+//     so one to eight sequences cost the same number of instructions;
+//   * with several panels every CTA publishes its 16 x 8 partial tiles as words that carry their own tag, and one CTA per
+//     tile (they take turns) polls the panels' words and adds them in a fixed order; then the epilogue runs
 //     (store, residual add with sums of squares for the next RMSNorm, GLU, logits + arg-max);
 //   * with tensor parallelism the epilogue of a row-parallel GEMV first pushes the tile into every
 //     rank's mailbox with plain peer stores (value and sequence tag in one 64-bit word), polls its own
@@ -23,8 +25,8 @@
 //   * stages meet at a grid barrier (one atomic counter in global memory, bounded wait).
 //
 // Every wait is bounded: a wait that runs out records MK_ERR_TIMEOUT and its site in the status words,
-// after which every wait in every CTA returns at once, the remaining stages are skipped, the producer
-// waits (bounded) for its copies in flight and the kernel returns.
+// after which every wait in every CTA returns at once, the remaining stages are skipped, every warp
+// waits for its copies in flight and the kernel returns.
 #pragma once
 #include <cuda_fp16.h>
 
@@ -34,20 +36,24 @@
 namespace mks {
 using namespace mk;
 
-constexpr int SLOT_BYTES = 4352;                  // one ring slot: 8 tile steps of 512 bytes + 256 bytes of scales
-constexpr int XS_BYTES = 50176;                   // staged GEMV input: 8 columns x 3072 fp16 + padding; also mixer scratch
+constexpr int SLOT_BYTES = 4352;                  // largest chunk of the packed format: 8 tile steps of 512 bytes + 256 bytes of scales
+constexpr int BLOCK_STEPS = 4;                    // one ring slot: four tile steps and their scales
+constexpr int BLOCK_BYTES = BLOCK_STEPS * 512 + 128;
+constexpr int XS_BYTES = 82432;                   // staged GEMV input: 8 columns x 5120 fp16 + padding; also mixer scratch and shared tiles
 constexpr int MAX_GROUPS = 72;                    // routed experts of one step (8 x 8) + shared / dense groups
-constexpr int MISC_BYTES = 8192;
+constexpr int MISC_BYTES = 10752;
 constexpr int SMEM_TOTAL = 232448;                // 227 KB
-constexpr int MAX_RING_DEPTH = 4;                 // ring slots per consumer warp: 2..4, as many as the launch's input staging area leaves room for
-constexpr int NS = 16 * MAX_RING_DEPTH;           // ring slots (upper bound): every consumer warp has its own
+constexpr int MIN_RING_DEPTH = 4, MAX_RING_DEPTH = 6;   // ring slots per consumer warp: as many as the launch's input staging area leaves room for
+constexpr int MAX_SEGS = 16;                      // K splits (of all groups) of one panel of a stage that adds its groups up
+constexpr int TILE_BYTES = 16 * 512;              // what each warp adds to a tile that the warp before it started
+constexpr int GEO_RING = 4;                       // stage records in shared memory: the scout is up to three stages ahead
 constexpr int ATTN_MAX_CHUNK = 256;               // positions per attention task (score buffer)
 constexpr int MAILBOX_TILES = 1024;               // output tiles of a row-parallel GEMV one all-reduce can carry
 constexpr int MAILBOX_BYTES = 2 * MAILBOX_TILES * MKS_MAX_RANKS * 128 * 8 + 2 * MKS_MAX_RANKS * MKS_MAX_BATCH * 16;
-static_assert((size_t)16 * 2 * SLOT_BYTES + XS_BYTES + MISC_BYTES <= SMEM_TOTAL, "shared memory of one SM");
+static_assert((size_t)16 * MIN_RING_DEPTH * BLOCK_BYTES + XS_BYTES + MISC_BYTES <= SMEM_TOTAL, "shared memory of one SM");
 
 // wait sites (status[1])
-enum { WS_FULL = 101, WS_EMPTY, WS_BARRIER, WS_ROUTE, WS_DRAIN, WS_MAILBOX, WS_KEYS };
+enum { WS_SCOUT = 101, WS_BARRIER, WS_MAILBOX, WS_KEYS, WS_TILE };
 
 struct Args {
     const mk_stage_desc* prog;
@@ -75,16 +81,63 @@ struct Args {
 // area; what is per thread (identity, ring position) travels in registers.  A per-thread context struct
 // handed to the stage functions by reference would sit in local memory: 544 threads' copies do not fit
 // the few KB of L1 that the shared-memory carve-out leaves, and every field access would cost an L2 trip.
+// One GEMV stage as this CTA sees it (written by the scout, read by every warp).
+struct Geo {
+    const uint8_t* w;              // weights of group 0 (or of expert 0)
+    const uint8_t* w_shared;       // weights of the last group of a routed stage, or null
+    u64 gstride, w_bytes;
+    int T, S, G;                   // tiles and K splits of a group, groups
+    int n_chunks, chunk_steps, chunk_bytes;
+    int ebps;                      // scale bytes per tile step
+    int reduce, routed;
+    int Q, P, panel;               // K splits a tile adds up, panels they are cut into, this CTA's panel (-1: all, one after another)
+    int t0, t1;                    // this CTA's tiles (of all groups, unless the groups are added up)
+    int g0, ng;                    // groups these tiles lie in, when every group has an input of its own (else 0, 1)
+    int nb;                        // batches: one staged input each
+    uint32_t stage;                // the stage this entry describes (counted over the launch)
+};
+// A warp's share of a batch: chunks [c, c1), tile by tile.
+struct Share {
+    const uint8_t* src;            // chunk c
+    int c, c1, n;                  // and all of the batch's chunks
+    int cpt, tl, k;                // chunks of one tile; chunk c as tile of the batch and chunk of the tile
+};
+// The stream's registers (the same in every lane).
+struct Feed {
+    const uint8_t* src;            // next step of the current chunk (of the whole run, where chunks carry no scales)
+    int steps, left;               // steps left in it, chunks left in the run behind it
+    int eoff;                      // from src to the scales of that step
+    int ebps, cs;                  // scale bytes per step, steps per chunk
+    int ahead;                     // blocks requested and not yet multiplied
+    uint32_t rd, wr;               // shared-memory addresses (this lane's part) of the next block to multiply, the next to request
+};
+// Where a consumer warp's weight stream stands: ahead of the multiplication by up to the ring's depth.
+struct Cur {
+    const uint8_t* src;            // the current run of consecutive chunks
+    int left;                      // its chunks
+    int rest;                      // chunks of the batch behind the run
+    int run, jump;                 // chunks of a whole run, bytes from one's end to the next
+    int chunk_bytes, chunk_steps;
+    int ebps;                      // scale bytes per tile step (behind a chunk's steps)
+    int tile, seg;                 // the run behind the current one, if the runs belong to several matrices
+    uint32_t gn, now;              // stages entered; the stage the warp multiplies in
+    int b, nb;                     // batches of the stage begun, all of them
+    // the registers of the stream between two GEMV stages
+    Feed f;                        // (rd, wr without the lane's part)
+};
+
 struct Shared {
-    uint64_t full[NS];
-    uint64_t empty[NS];
     u64 keys_s[8];                 // best key per sequence
-    volatile u64 pf_pos;           // bytes of the weight stream the issuing lane has requested (read by the prefetch lane)
+    mk_stage_desc desc[GEO_RING];  // stage n's record in entry n % GEO_RING
+    Geo geo[GEO_RING];             // and, for a GEMV stage, its geometry
+    Share share[GEO_RING][NCW];    // its first batch's
+    Cur cur[NCW];
     unsigned long long* prof;      // this stage's timestamp row (CTA 0, last step) or null
-    mk_stage_desc desc[2];         // this stage's record and the next one's
     Args A;                        // the launch arguments
+    uint32_t tag0;                 // stage barriers passed before this launch
     float red[16 + 17 * 8];        // block-reduction scratch
-    float xinv[8];                 // factor that undoes the power-of-two scaling of a staged column
+    float xinv[MAX_SEGS * 8];      // factor that undoes the power-of-two scaling of a staged column (of every K split, when groups are added up)
+    int xmax[MAX_SEGS * 8];        // its largest magnitude, then its scale
     float rstd[8];                 // 1/rms of the staged input
     int tok_s[8];
     int pos_s[8];
@@ -97,6 +150,8 @@ struct Shared {
     int n_groups;
     volatile int abort_flag;
     volatile unsigned route_seq;
+    volatile unsigned described;   // stages the scout has described
+    volatile unsigned completed;   // stages all warps of this CTA have left
     int flag;
     // dynamic shared memory: [this block | staging area of A.xs_bytes | 16 x A.ring_depth ring slots]
     __device__ __forceinline__ uint8_t* xs() { return reinterpret_cast<uint8_t*>(this) + MISC_BYTES; }
@@ -110,11 +165,6 @@ __device__ __forceinline__ int warp_() { return (int)(threadIdx.x >> 5); }
 __device__ __forceinline__ int lane_() { return (int)(threadIdx.x & 31); }
 __device__ __forceinline__ int cta_() { return (int)blockIdx.x; }
 __device__ __forceinline__ int grid_() { return (int)gridDim.x; }
-struct Mut {
-    uint32_t chunk_n;        // ring chunks this consumer warp has taken so far
-    bool dead;               // this thread saw a wait run out
-};
-
 constexpr int PROF_FIELDS = 8;  // per stage: entered, input staged, units done, barrier passed, ring-wait ns of warp 0
 __device__ __forceinline__ void prof_mark(Shared& S, int field) {
     if (S.prof && tid_() == 0) S.prof[field] = globaltimer();
@@ -148,20 +198,6 @@ __device__ __noinline__ u64 spin_slow2(volatile int* abort_flag, int* status, u6
 #define MKS_SPIN_FAIL(S, s, where) \
     ((((++(s).it) & 255u) == 0) && (((s).t0 = spin_slow2(&(S).abort_flag, (S).A.status, (u64)(S).A.spin_limit_ns, (s).t0, (where))) == ~0ull))
 
-// Wait of a whole warp for one barrier phase.  The warp leaves together: a lane that returned alone
-// would never reach the `__syncwarp` the others go on to.
-__device__ __forceinline__ bool mbar_wait2(Shared& S, uint64_t* b, uint32_t parity, int where) {
-    Spin2 s;
-    bool fail = false;
-#pragma unroll 1
-    for (;;) {
-        const bool ok = mbar_try_wait(b, parity);
-        if (__all_sync(0xffffffffu, ok)) return true;
-        if (!ok && MKS_SPIN_FAIL(S, s, where)) fail = true;
-        if (__any_sync(0xffffffffu, fail)) return false;       // the abort flag is set: the stage loop stops at its next check
-    }
-}
-
 __device__ __forceinline__ u64 ld_acquire_u64(const unsigned long long* p) {
     u64 v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -185,7 +221,8 @@ __device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsig
     asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-__device__ __forceinline__ void grid_barrier(Shared& S, Mut& mu, const Args& A, u64& bar_n) {
+// Only thread 0 waits here; the CTA barrier in front of the next stage holds the others.
+__device__ __forceinline__ void grid_barrier(Shared& S, const Args& A, u64& bar_n) {
     bar_n++;
     consumer_sync();
     if (tid_() == 0 && !S.abort_flag) {
@@ -196,7 +233,7 @@ __device__ __forceinline__ void grid_barrier(Shared& S, Mut& mu, const Args& A, 
             if (MKS_SPIN_FAIL(S, s, WS_BARRIER)) break;
         }
     }
-    consumer_sync();
+    __syncwarp();
 }
 
 // ---- conversions -----------------------------------------------------------------------------------------
@@ -238,43 +275,65 @@ __device__ __forceinline__ float gelu_tanh_f(float x) {
 }
 __device__ __forceinline__ float ldcg_f(const float* p) { return __ldcg(p); }
 
-// ---- geometry of a GEMV stage (shared by producer and consumers) ----------------------------------------------
-struct Gemv {
-    int T, S, G, unit_steps, chunk_steps, chunk_bytes, n_chunks;
-    int u0, u1;                  // this CTA's unit range; unit = (group * S + split) * T + tile (32-bit: 64-bit division costs hundreds of cycles)
-};
-__device__ __forceinline__ Gemv gemv_geometry(const Shared& S, const mk_stage_desc& d) {
-    Gemv g;
-    g.T = d.i[MKS_I_TILES];
-    g.S = d.i[MKS_I_SPLITS];
-    g.G = d.i[MKS_I_GROUPS] >= 0 ? d.i[MKS_I_GROUPS] : *reinterpret_cast<const volatile int*>(&S.n_groups);
-    g.unit_steps = d.i[MKS_I_UNIT_STEPS];
-    g.chunk_steps = d.i[MKS_I_CHUNK_STEPS];
-    g.chunk_bytes = d.i[MKS_I_CHUNK_BYTES];
-    g.n_chunks = g.unit_steps / g.chunk_steps;
-    const unsigned P = (unsigned)(g.G * g.S), grid = (unsigned)grid_(), cta = (unsigned)cta_();
-    if (P <= grid) {
-        // every CTA stays inside one panel (one staged input): panel p gets the CTAs [ceil(p grid / P), ceil((p + 1) grid / P))
-        // and they share its T tiles evenly.  A CTA that straddled two panels would stage its input twice and
-        // keep the whole grid waiting at the stage's barrier.
-        const unsigned p = cta * P / grid;
-        const unsigned c0 = (p * grid + P - 1) / P, c1 = ((p + 1) * grid + P - 1) / P;
-        const unsigned n = c1 - c0, k = cta - c0;
-        g.u0 = (int)(p * (unsigned)g.T + (unsigned)g.T * k / n);
-        g.u1 = (int)(p * (unsigned)g.T + (unsigned)g.T * (k + 1) / n);
-    } else {
-        const unsigned U = P * (unsigned)g.T;                      // < 2^24: U * grid fits 32 bits
-        g.u0 = (int)(U * cta / grid);
-        g.u1 = (int)(U * (cta + 1) / grid);
+// ---- geometry of a GEMV stage (shared by scout, weight streams and multiplication) ---------------------------------
+// Column stride of the staged input in bytes: a multiple of 128 plus 32, so that the eight columns'
+// 8-byte fragment reads of a half warp fall into different banks.
+__host__ __device__ __forceinline__ int xs_stride_bytes(int cols) { return ((cols * 2 + 127) / 128) * 128 + 32; }
+// K splits of `kc` columns of `ncols` staged columns (sequences x pieces) that fit `xs_bytes`.
+__host__ __device__ __forceinline__ int max_panel_splits(int xs_bytes, int kc, int ncols, int pieces, bool reduce) {
+    int w = (xs_bytes / ncols - 32) / 128 * 64 / kc;
+    if (reduce) w = min(w, MAX_SEGS);
+    return max(w, 1);
+}
+// What a stage costs the busiest CTA, in bytes of weight stream (about 83 per ns), if its R tiles x Q splits are cut into P
+// panels: the weights of its tiles (whole chunks per warp count half: the other warps keep the memory busy); the input it
+// stages (every CTA reads its panel's fp32 columns from L2: about 0.12 ns a value); and with more than one panel the exchange:
+// one round trip through L2 (about 1.5 us) and 16-byte words of partial tiles, written once and read once.
+__host__ __device__ __forceinline__ u64 panel_cost(int R, int Q, int P, int n_chunks, int chunk_bytes, int kc, int M, int grid) {
+    const u64 tiles = ((u64)R * P + grid - 1) / grid, w = (Q + P - 1) / P;
+    const u64 chunks = tiles * w * n_chunks, even = (chunks + NCW - 1) / NCW * NCW;
+    return (chunks + even) / 2 * chunk_bytes + w * kc * M * 10 + (P > 1 ? 120000 + tiles * M * 256 : 0);
+}
+
+// Every lane of the scout calls this: the number of panels, from P0 (what the staging area allows) up to half the grid
+// (each panel then has a CTA).
+__device__ __forceinline__ int pick_panels(int R, int Q, int P0, int n_chunks, int chunk_bytes, int kc, int M, int grid) {
+    u64 best = ~0ull;
+    for (int P = P0 + lane_(); P <= min(Q, grid / 2); P += 32) {
+        const u64 k = panel_cost(R, Q, P, n_chunks, chunk_bytes, kc, M, grid) << 8 | (u64)P;
+        best = k < best ? k : best;
     }
-    return g;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other < best ? other : best;
+    }
+    return best == ~0ull ? 0 : (int)(best & 255u);
+}
+
+// One batch of a stage: a staged input (K splits [seg0, seg1) of a panel) and the tiles [t0, t1) it multiplies.
+struct Batch {
+    int panel, seg0, seg1, t0, t1, grp;
+};
+__device__ __forceinline__ Batch geo_batch(const Geo& g, int b) {
+    Batch r;
+    const int pb = g.ng == 1 ? b : b / g.ng, gb = b - pb * g.ng;
+    r.panel = g.panel >= 0 ? g.panel : pb;
+    r.seg0 = g.P == 1 ? 0 : g.Q * r.panel / g.P;
+    r.seg1 = g.P == 1 ? g.Q : g.Q * (r.panel + 1) / g.P;
+    r.t0 = g.t0; r.t1 = g.t1; r.grp = 0;
+    if (g.ng > 1 || g.g0 > 0) {
+        r.grp = g.g0 + gb;
+        r.t0 = max(r.t0, r.grp * g.T);
+        r.t1 = min(r.t1, (r.grp + 1) * g.T);
+    }
+    return r;
 }
 // Weight bytes of group `grp`: experts of a routed stage come from the routing list, the shared expert last.
-__device__ __forceinline__ const uint8_t* group_weights(const Shared& S, const mk_stage_desc& d, int grp, int G) {
-    const uint8_t* w = reinterpret_cast<const uint8_t*>(d.p[MKS_P_W]);
-    if (d.i[MKS_I_GROUPS] >= 0) return w + (size_t)grp * d.p[MKS_P_W_GSTRIDE];
-    if (d.p[MKS_P_W_SHARED] && grp == G - 1) return reinterpret_cast<const uint8_t*>(d.p[MKS_P_W_SHARED]);
-    return w + (size_t)reinterpret_cast<const volatile int*>(S.glist)[grp] * d.p[MKS_P_W_GSTRIDE];
+__device__ __forceinline__ const uint8_t* group_weights(const Shared& S, const Geo& g, int grp) {
+    if (!g.routed) return g.w + (size_t)grp * g.gstride;
+    if (g.w_shared && grp == g.G - 1) return g.w_shared;
+    return g.w + (size_t)reinterpret_cast<const volatile int*>(S.glist)[grp] * g.gstride;
 }
 __device__ __forceinline__ const float* group_row_scale(const Shared& S, const mk_stage_desc& d, int grp, int G) {
     const float* s = reinterpret_cast<const float*>(d.p[MKS_P_ROW_SCALE]);
@@ -284,366 +343,505 @@ __device__ __forceinline__ const float* group_row_scale(const Shared& S, const m
     return s + (size_t)S.glist[grp] * d.p[MKS_P_RS_GSTRIDE];
 }
 
-// ---- producer --------------------------------------------------------------------------------------------
-// The whole producer warp walks the program.  In every round of up to 16 units lane j issues the chunks
-// of the round's j-th unit (the unit consumer warp j will multiply), one 1-D bulk copy per chunk: a single
-// lane needs about a quarter of a microsecond of dependent instructions per copy, which caps one SM at a few
-// chunks per microsecond -- a sixth of its share of the HBM stream.
+// ---- the weight stream of a consumer warp --------------------------------------------------------------------
+// A warp requests its own weights, block by block (four tile steps), in the order it multiplies them: lane j copies the 16
+// bytes per step that lane j will read, and right after a block has been read the slot takes the next request.  Earlier,
+// a producer warp filled two slots of a whole chunk per consumer warp and polled sixteen release barriers for free ones; with
+// half of the ring in flight at most, and the polls sharing issue slots with the multiplication, a 95 MB MXFP4 matrix
+// streamed at 3.0 TB/s where the same loop with the data in place runs at 5.9.
 //
-// Every consumer warp has its own ring_depth slots.  A slot is therefore filled and drained by the same pair
-// (lane j, warp j) in strict alternation, and a waiter is never more than one phase ahead of its barrier:
-// with slots shared between warps a fast warp could ask for the next-but-one phase of a slot that still
-// served another warp, and a parity wait cannot tell that phase from the one before it.
-__device__ __forceinline__ void prefetch_desc_l1(const mk_stage_desc* d) {
-    const char* p = reinterpret_cast<const char*>(d);
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 96));
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 192));
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 287));
+__device__ __noinline__ void stream_error(Shared& S, uint32_t stage, int where) {
+    if (atomicCAS(S.A.status, 0, -5) == 0) {
+        S.A.status[1] = (int)stage;
+        S.A.status[2] = cta_();
+        S.A.status[3] = where;
+    }
+    S.abort_flag = 1;
+}
+// Weights of K split `seg` (of all groups, if they are added up) of tile `tile` (of all groups, if they are not).
+__device__ __forceinline__ const uint8_t* split_weights(const Shared& S, const Geo& g, int tile, int seg) {
+    int grp = 0;
+    if (g.reduce) {
+        grp = g.S == 1 ? seg : seg / g.S;
+        seg -= grp * g.S;
+    } else if (g.G > 1) {
+        grp = tile / g.T;
+        tile -= grp * g.T;
+    }
+    return group_weights(S, g, grp) + (size_t)((tile * g.S + seg) * g.n_chunks) * g.chunk_bytes;
+}
+// Warp w's share of batch b.
+__device__ __forceinline__ Share batch_share(const Shared& S, const Geo& g, const Batch& bt, int w) {
+    Share r;
+    r.cpt = (bt.seg1 - bt.seg0) * g.n_chunks;
+    r.n = (bt.t1 - bt.t0) * r.cpt;
+    r.c = r.n * w / NCW;
+    r.c1 = r.n * (w + 1) / NCW;
+    r.tl = r.c / r.cpt;
+    r.k = r.c - r.tl * r.cpt;
+    const int sg = r.k / g.n_chunks;
+    r.src = r.c < r.c1 ? split_weights(S, g, bt.t0 + r.tl, bt.seg0 + sg) + (size_t)(r.k - sg * g.n_chunks) * g.chunk_bytes : nullptr;
+    return r;
+}
+// The next run of consecutive chunks; false if the scout has not described the stage it belongs to.  The whole warp calls it
+// and every lane computes the same; its first lane writes the cursor back.
+__device__ __noinline__ bool next_run(Shared& S) {
+    Cur& c = S.cur[warp_()];
+    const uint8_t* src = c.src;
+    int rest = c.rest, run = c.run, left = 0;
+    if (rest > 0) {
+        const Geo& g = S.geo[(c.gn - 1) % GEO_RING];
+        if (g.G == 1) {
+            src += c.left * c.chunk_bytes + c.jump;            // the same columns of the next tile
+        } else {
+            const int tile = c.tile, seg = c.seg;
+            src = split_weights(S, g, tile, seg);
+            __syncwarp();
+            if (lane_() == 0) {
+                const Batch bt = geo_batch(g, c.b - 1);
+                c.seg = !g.reduce || seg + 1 == bt.seg1 ? bt.seg0 : seg + 1;
+                c.tile = c.seg == bt.seg0 ? tile + 1 : tile;
+            }
+        }
+        left = min(run, rest);
+        rest -= left;
+    } else {
+        uint32_t gn = c.gn;
+        int b = c.b, nb = c.nb;
+        const unsigned described = __shfl_sync(0xffffffffu, S.described, 0);
+        __threadfence_block();
+        __syncwarp();
+#pragma unroll 1
+        while (left == 0) {
+            if (b == nb) {                                     // next stage
+                // (stages before the warp's own are over, and their entries may describe later ones by now)
+                if ((int)(c.now - gn) > 0) gn = c.now;
+                b = nb = 0;
+                if ((int)(described - gn) <= 0) break;
+                if (S.geo[gn % GEO_RING].stage != gn) {
+                    stream_error(S, gn, -1);
+                    break;
+                }
+                nb = S.geo[gn++ % GEO_RING].nb;
+                if (nb == 0) continue;
+            }
+            const Geo& g = S.geo[(gn - 1) % GEO_RING];
+            const Batch bt = geo_batch(g, b);
+            Share sh;
+            if (b == 0) sh = S.share[(gn - 1) % GEO_RING][warp_()];
+            else sh = batch_share(S, g, bt, warp_());
+            b++;
+            rest = sh.c1 - sh.c;
+            if (rest == 0) continue;
+            src = sh.src;
+            run = sh.cpt;
+            left = run - sh.k;
+            int seg = bt.seg0, tile = bt.t0 + sh.tl + 1;
+            if (g.reduce) {
+                run = g.n_chunks;                              // one K split of one matrix at a time
+                seg = sh.k / run;
+                left = run - (sh.k - seg * run);
+                seg += bt.seg0 + 1;
+                if (seg == bt.seg1) seg = bt.seg0;
+                else tile--;
+            }
+            left = min(left, rest);
+            rest -= left;
+            // self-check: the copies must be aligned and stay inside the matrix the record describes
+            if ((reinterpret_cast<size_t>(src) & 15) ||
+                (g.w_bytes && g.G == 1 && (size_t)(src - g.w) + (size_t)((long long)rest * g.chunk_bytes) > (size_t)g.w_bytes)) {
+                stream_error(S, gn, left);
+                left = rest = 0;
+                break;
+            }
+            __syncwarp();
+            if (lane_() == 0) {
+                c.run = run;
+                c.jump = (g.S * g.n_chunks - sh.cpt) * g.chunk_bytes;
+                c.chunk_bytes = g.chunk_bytes; c.chunk_steps = g.chunk_steps; c.ebps = g.ebps;
+                c.tile = tile; c.seg = seg;
+            }
+        }
+        __syncwarp();
+        if (lane_() == 0) {
+            c.gn = gn; c.b = b; c.nb = nb;
+        }
+    }
+    __syncwarp();
+    if (lane_() == 0) {
+        c.src = src; c.left = left; c.rest = rest;
+    }
+    __syncwarp();
+    return left > 0;
+}
+// Fill the warp's free slots.  The caller has ordered the warp's reads of the freed slots before this (a warp barrier).
+// Every free slot gets a group of copies, an empty one when there is nothing to request: then at least ring_depth - 1
+// groups lie behind the next block to multiply, and waiting for all but that many waits for the block.
+__device__ __forceinline__ void feed(Shared& S, Feed& f, int depth, uint32_t ring_end) {
+    int n_free = depth - f.ahead;
+#pragma unroll 1
+    for (; n_free > 0; n_free--) {
+        if (f.steps == 0) {
+            if (f.left > 0) {
+                f.src += f.cs * f.ebps;                        // past the scales of the chunk before
+                f.left--;
+            } else {
+                if (!next_run(S)) break;
+                const Cur& c = S.cur[warp_()];
+                f.src = c.src; f.ebps = c.ebps; f.cs = c.chunk_steps; f.left = c.left;
+                if (f.ebps == 0) f.cs *= f.left;
+                f.left = f.ebps == 0 ? 0 : f.left - 1;
+            }
+            f.steps = f.cs;
+            f.eoff = f.cs * 512;
+        }
+        const int n = min(BLOCK_STEPS, f.steps);
+        const uint8_t* src = f.src + lane_() * 16;
+#pragma unroll
+        for (int u = 0; u < BLOCK_STEPS; u++)
+            if (u < n) cp_async16(f.wr + u * 512, src + u * 512);
+        if (lane_() * 4 < n * f.ebps) cp_async4(f.wr + BLOCK_STEPS * 512 - lane_() * 12, f.src + f.eoff + lane_() * 4);
+        cp_async_commit();
+        f.src += n * 512;
+        f.steps -= n;
+        f.eoff += n * (f.ebps - 512);
+        f.ahead++;
+        f.wr += BLOCK_BYTES;
+        if (f.wr >= ring_end) f.wr -= depth * BLOCK_BYTES;
+    }
+#pragma unroll 1
+    for (; n_free > 0; n_free--) cp_async_commit();
+}
+// All but depth - 1 groups of copies have landed.
+__device__ __forceinline__ void wait_block(int depth) {
+    static_assert(MIN_RING_DEPTH == 4 && MAX_RING_DEPTH == 6, "one wait per ring depth");
+    if (depth == 4) cp_async_wait<3>();
+    else if (depth == 5) cp_async_wait<4>();
+    else cp_async_wait<5>();
 }
 
-// Lane j of the producer warp feeds consumer warp j and nobody else: it has its own cursor over the program
-// (stage, panel, round, chunk) and never waits inside the loop.  Every turn of the warp-wide loop each lane
-// looks whether the slot its next chunk goes to has been released, issues the copy if so and moves on; a lane
-// whose consumer is busy (a long unit tail, a barrier) costs the others nothing.  Lanes may be in different
-// rounds, panels and stages at the same time, exactly as far ahead as their own two slots allow.
-struct Cursor {
-    int step, si;                 // position in the program (si = -1 before the first stage)
-    int T, S_, G, n_chunks, chunk_bytes, u0, u1;
-    int pu, pend, r0;             // next panel start, end of the current panel's units in this CTA, next round
-    int panel;
-    int ch;                       // next chunk of the current unit
-    const uint8_t* w;             // the current panel's units
-    const uint8_t* wg;            // the current group's matrix
-    const uint8_t* src;           // the current unit
-    unsigned long long w_bytes;
-    unsigned routes;
-    bool have, done;
-};
-
-__device__ __noinline__ void producer_main(Shared& S, const Args& A) {
-    const int lane = lane_();
-    const u64 policy = policy_evict_first();
-    const uint32_t depth = (uint32_t)A.ring_depth;
-    uint32_t q = 0;              // chunks this lane has issued: chunk q of consumer warp `lane` lives in slot
-                                 // lane * depth + q % depth, phase q / depth
-    Cursor c;
-    c.step = 0; c.si = -1; c.u0 = c.u1 = c.pu = c.pend = c.r0 = 0; c.ch = 0; c.routes = 0;
-    c.have = false; c.done = lane >= NCW;
-    c.T = c.S_ = c.G = 1; c.n_chunks = 1; c.chunk_bytes = 0; c.panel = 0; c.w = c.wg = c.src = nullptr; c.w_bytes = 0;
+// ---- scout ---------------------------------------------------------------------------------------------------
+__device__ __forceinline__ bool scout_wait(Shared& S, volatile unsigned* word, unsigned at_least) {
     Spin2 sp;
     bool stop = false;
 #pragma unroll 1
-    while (!stop) {
-        bool progress = false;
-        if (!c.done && !c.have) {
-            // move the cursor: at most a few transitions per turn, so that the lanes stay roughly together
-#pragma unroll 1
-            for (int k = 0; k < 6 && !c.have && !c.done; k++) {
-                if (c.r0 < c.pend) {                                   // next round of the current panel
-                    const int nj = min(NCW, c.pend - c.r0);
-                    if (lane < nj) {
-                        c.src = c.w + (size_t)((c.r0 + lane) - c.panel * c.T) * ((size_t)c.n_chunks * c.chunk_bytes);
-                        c.ch = 0;
-                        c.have = true;
-                    }
-                    c.r0 += NCW;
-                    progress = true;
-                } else if (c.pu < c.u1) {                               // next panel of the current stage
-                    const mk_stage_desc& d = A.prog[c.si];
-                    c.panel = c.pu / c.T;
-                    c.pend = min(c.u1, (c.panel + 1) * c.T);
-                    const int grp = c.panel / c.S_, split = c.panel - grp * c.S_;
-                    c.wg = group_weights(S, d, grp, c.G);
-                    c.w = c.wg + (size_t)split * c.T * ((size_t)c.n_chunks * c.chunk_bytes);
-                    c.r0 = c.pu;
-                    c.pu = c.pend;
-                    progress = true;
-                } else {                                                // next stage
-                    int nsi = c.si + 1, nstep = c.step;
-                    if (nsi >= A.n_stages) {
-                        nsi = 0;
-                        nstep++;
-                    }
-                    if (nstep >= A.n_steps) {
-                        c.done = true;
-                        break;
-                    }
-                    const mk_stage_desc& d = A.prog[nsi];
-                    if (d.op == MKS_OP_ROUTE && S.route_seq < c.routes + 1) break;   // the expert list is not there yet
-                    if (d.op == MKS_OP_ROUTE) c.routes++;
-                    c.si = nsi;
-                    c.step = nstep;
-                    progress = true;
-                    if (d.op == MKS_OP_GEMV) {
-                        const Gemv g = gemv_geometry(S, d);
-                        c.T = g.T; c.S_ = g.S; c.G = g.G; c.n_chunks = g.n_chunks; c.chunk_bytes = g.chunk_bytes;
-                        c.u0 = g.u0; c.u1 = g.u1;
-                        c.pu = g.u0; c.pend = 0; c.r0 = 0;
-                        c.w_bytes = d.p[MKS_P_W_BYTES];
-                    } else {
-                        c.u0 = c.u1 = c.pu = c.pend = c.r0 = 0;
-                    }
-                }
-            }
-        }
-        if (c.have) {
-            const int slot = lane * (int)depth + (int)(q % depth);
-            const bool is_free = q < depth || mbar_try_wait(&S.empty[slot], ((q / depth) - 1) & 1);
-            if (is_free) {
-                // self-check: the copy must stay inside the matrix the record describes
-                const size_t off = (size_t)(c.src - c.wg) + (size_t)c.ch * c.chunk_bytes;
-                if (c.w_bytes && off + (size_t)c.chunk_bytes > (size_t)c.w_bytes) {
-                    if (atomicCAS(S.A.status, 0, -5) == 0) {
-                        S.A.status[1] = c.si;
-                        S.A.status[2] = cta_();
-                        S.A.status[3] = (int)(off >> 12);
-                    }
-                    S.abort_flag = 1;
-                } else if (!S.abort_flag) {
-                    mbar_expect_tx(&S.full[slot], (uint32_t)c.chunk_bytes);
-                    bulk_load(S.ring() + (size_t)slot * SLOT_BYTES, c.src + (size_t)c.ch * c.chunk_bytes, (uint32_t)c.chunk_bytes,
-                              &S.full[slot], policy);
-                    q++;
-                    c.ch++;
-                    if (c.ch == c.n_chunks) c.have = false;
-                    progress = true;
-                }
-            }
-        }
-        // the warp leaves together: when every lane is done, or a wait ran out somewhere
-        if (__all_sync(0xffffffffu, c.done)) break;
-        if (__any_sync(0xffffffffu, progress)) {
-            sp.it = 0;
-            sp.t0 = 0;
-        } else if (lane == 0 && MKS_SPIN_FAIL(S, sp, WS_EMPTY)) {
-            stop = true;
-        }
-        stop = __any_sync(0xffffffffu, stop || S.abort_flag != 0);
+    while (!__all_sync(0xffffffffu, (int)(*word - at_least) >= 0)) {      // (the warp leaves together)
+        // (the consumers' own waits end a launch that is stuck; this bound is only the scout's last resort)
+        if (lane_() == 0 && ((++sp.it) & 255u) == 0 &&
+            (sp.t0 = spin_slow2(&S.abort_flag, S.A.status, 8 * (u64)S.A.spin_limit_ns, sp.t0, WS_SCOUT)) == ~0ull) stop = true;
+        stop = stop || S.abort_flag != 0;
+        if (__any_sync(0xffffffffu, stop)) return false;
+        __nanosleep(40);
     }
-    // before the CTA may exit every copy that was issued must have landed (not abortable: the copies write shared memory)
-    if (lane < NCW) {
-        const uint32_t first = q > depth ? q - depth : 0;
+    __threadfence_block();
+    __syncwarp();
+    return true;
+}
+__device__ __noinline__ void scout_main(Shared& S, const Args& A) {
+    constexpr int DESC_WORDS = (int)(sizeof(mk_stage_desc) / 4);
+    unsigned n = 0, routes = 0;
+    const int grid = grid_(), cta = cta_();
 #pragma unroll 1
-        for (uint32_t i = first; i < q; i++) {
-            uint32_t it = 0;
-            u64 t0 = 0;
-            while (!mbar_try_wait(&S.full[lane * (int)depth + (int)(i % depth)], (i / depth) & 1)) {
-                if (((++it) & 1023u) == 0) {
-                    const u64 now = globaltimer();
-                    if (!t0) t0 = now;
-                    else if (now - t0 > (u64)S.A.spin_limit_ns) {
-                        if (atomicCAS(S.A.status, 0, -2) == 0) S.A.status[1] = WS_DRAIN;
-                        break;
-                    }
+    for (int step = 0; step < A.n_steps; step++) {
+#pragma unroll 1
+        for (int si = 0; si < A.n_stages; si++, n++) {
+            uint32_t words[(DESC_WORDS + 31) / 32];
+#pragma unroll
+            for (int i = 0; i < (DESC_WORDS + 31) / 32; i++)
+                if (lane_() + 32 * i < DESC_WORDS) words[i] = __ldg(reinterpret_cast<const uint32_t*>(&A.prog[si]) + lane_() + 32 * i);
+            // the stage that had this entry is over
+            if (n >= GEO_RING && !scout_wait(S, &S.completed, n - GEO_RING + 1)) return;
+            mk_stage_desc& d = S.desc[n % GEO_RING];
+            Geo& g = S.geo[n % GEO_RING];
+#pragma unroll
+            for (int i = 0; i < (DESC_WORDS + 31) / 32; i++)
+                if (lane_() + 32 * i < DESC_WORDS) reinterpret_cast<uint32_t*>(&d)[lane_() + 32 * i] = words[i];
+            __syncwarp();
+            if (d.op == MKS_OP_ROUTE) routes++;
+            if (d.op != MKS_OP_GEMV) {
+                if (lane_() == 0) {
+                    g.nb = 0;
+                    g.stage = n;
+                    __threadfence_block();
+                    S.described = n + 1;
                 }
+                continue;
             }
+            if (d.i[MKS_I_GROUPS] < 0 && !scout_wait(S, &S.route_seq, routes)) return;       // the expert list
+            const int T = d.i[MKS_I_TILES], Sp = d.i[MKS_I_SPLITS], kc = d.i[MKS_I_KC], pieces = d.i[MKS_I_PIECES];
+            const bool routed = d.i[MKS_I_GROUPS] < 0, reduce = d.i[MKS_I_REDUCE_GROUPS] != 0;
+            const int G = routed ? *reinterpret_cast<const volatile int*>(&S.n_groups) : d.i[MKS_I_GROUPS];
+            const int n_chunks = d.i[MKS_I_UNIT_STEPS] / d.i[MKS_I_CHUNK_STEPS], cb = d.i[MKS_I_CHUNK_BYTES];
+            const int R = reduce ? T : G * T, Q = reduce ? G * Sp : Sp;
+            const int w = max_panel_splits(A.xs_bytes, kc, A.M * pieces, pieces, reduce);
+            int P = 1, panel = 0, c0 = 0, nc = grid, nb = 0, t0 = 0, t1 = 0;
+            if (R > 0 && Q > 0) {
+                const int P0 = (Q + w - 1) / w;
+                P = pick_panels(R, Q, P0, n_chunks, cb, kc, A.M, grid);
+                if (P == 0) {
+                    P = P0;                                    // more panels than half the CTAs: every CTA goes through all of them
+                    panel = P > 1 ? -1 : 0;
+                }
+                if (P > 1 && panel >= 0) {
+                    // panel p has the CTAs [grid q0 / Q, grid q1 / Q), q0 and q1 its first split and the next panel's
+                    panel = (int)((long long)cta * P / grid);
+                    auto first = [&](int p) { return (grid * (Q * p / P) + Q - 1) / Q; };
+                    while (panel > 0 && first(panel) > cta) panel--;
+                    while (panel + 1 < P && first(panel + 1) <= cta) panel++;
+                    c0 = first(panel);
+                    nc = first(panel + 1) - c0;
+                }
+                const int k = cta - c0;
+                t0 = (int)((long long)R * k / nc);
+                t1 = (int)((long long)R * (k + 1) / nc);
+                nb = t1 > t0 ? (panel < 0 ? P : 1) : 0;
+            }
+            if (lane_() == 0) {
+                g.w = reinterpret_cast<const uint8_t*>(d.p[MKS_P_W]);
+                g.w_shared = reinterpret_cast<const uint8_t*>(d.p[MKS_P_W_SHARED]);
+                g.gstride = d.p[MKS_P_W_GSTRIDE];
+                g.w_bytes = d.p[MKS_P_W_BYTES];
+                g.T = T; g.S = Sp; g.G = G;
+                g.n_chunks = n_chunks; g.chunk_steps = d.i[MKS_I_CHUNK_STEPS]; g.chunk_bytes = cb;
+                g.ebps = d.i[MKS_I_FMT] == MKS_FMT_MXFP4 ? 32 : (d.i[MKS_I_BLOCK_SCALES] ? 2 : 0);
+                g.reduce = reduce; g.routed = routed;
+                g.Q = Q; g.P = P; g.panel = panel;
+                g.t0 = t0; g.t1 = t1;
+                g.g0 = 0; g.ng = 1;
+                if (!reduce && d.i[MKS_I_X_GSTRIDE] != 0 && nb) {   // a staged input per group
+                    g.g0 = t0 / T;
+                    g.ng = (t1 - 1) / T - g.g0 + 1;
+                }
+                g.nb = nb * g.ng;
+                g.stage = n;
+            }
+            __syncwarp();
+            if (g.nb && lane_() < NCW) S.share[n % GEO_RING][lane_()] = batch_share(S, g, geo_batch(g, 0), lane_());
+            __threadfence_block();
+            __syncwarp();
+            if (lane_() == 0) S.described = n + 1;
         }
     }
 }
 
 // ---- GEMV input staging ------------------------------------------------------------------------------------
-// Column stride of the staged input in bytes: a multiple of 128 plus 32, so that the eight columns'
-// 8-byte fragment reads of a half warp fall into different banks.
-__device__ __forceinline__ int xs_stride_bytes(int kc) { return ((kc * 2 + 127) / 128) * 128 + 32; }
-
-// Stage columns [split * kc, (split + 1) * kc) of every sequence's input of group `grp`: normalise, round
-// to bf16 (the model's activation type) and store as fp16 scaled by a power of two per column (bf16
-// weights: as bf16, unscaled).  Column `m` of the staged matrix is sequence m; with two pieces column
-// M + m holds what fp16 lost of sequence m, so that the products see an fp32-exact input.
+// Stage K splits [seg0, seg1) of every sequence's input: normalise, round to bf16 (the model's activation type) and
+// store as fp16 scaled by a power of two per column (bf16 weights: as bf16, unscaled).  Column `m` of the staged matrix
+// is sequence m; with two pieces column M + m holds what fp16 lost of sequence m, so that the products see an
+// fp32-exact input.  When groups are added up, consecutive splits belong to different groups: each has its own input,
+// its own scale, and nothing to stage for a sequence that gives it no weight.
 //
-// What matters here is the number of dependent L2 round trips (about 0.7 us each on this part), not
-// bytes: the first batch of input loads, the norm weights and the sums of squares behind 1/rms are all
-// requested before anything is awaited; the values go to shared memory as bf16 and are rescaled there.
-constexpr int XB = 2;       // float4 groups of one batch; two batches are in flight
+// What matters here is the number of dependent L2 round trips (about 0.7 us each on this part), not bytes: XB input
+// loads and their norm weights per thread are in flight at once, the first of them together with the sums of squares
+// behind 1/rms.  And the size of the code: every stage runs through it once, at the speed of instruction fetch.
+constexpr int XB = 4;       // float4 groups per thread and round
 
-__device__ __noinline__ void stage_x(Shared& S, Mut& mu, const mk_stage_desc& d, int grp, int split) {
-    const int kc = d.i[MKS_I_KC], fmt = d.i[MKS_I_FMT], pieces = d.i[MKS_I_PIECES], M = S.A.M;
-    const int stride = xs_stride_bytes(kc);
-    const bool norm = d.i[MKS_I_PROLOGUE] == MKS_P_NORM;
-    const float* x = reinterpret_cast<const float*>(d.p[MKS_P_X]) + (size_t)grp * d.i[MKS_I_X_GSTRIDE] + (size_t)split * kc;
-    const float* nw = reinterpret_cast<const float*>(d.p[MKS_P_NORM_W]) + (size_t)split * kc;
+// Exponent of the scale of a column whose largest magnitude has these bits: a = f * 2^e with f in [0.5, 1), the scale 2^(14 - e).
+__device__ __forceinline__ int scale_exponent(int bits) {
+    const int e = bits > 0 && bits < 0x7f800000 ? ((bits >> 23) & 0xff) - 126 : 0;
+    return max(-100, min(100, 14 - e));
+}
+// (PLAIN: one piece, no adding up of groups: nearly every stage)
+template <bool PLAIN>
+__device__ __forceinline__ void stage_x(Shared& S, const mk_stage_desc& d, int seg0, int seg1, int grp0, int n_splits) {
+    const int kc = d.i[MKS_I_KC], M = S.A.M;
+    const bool reduce = !PLAIN && d.i[MKS_I_REDUCE_GROUPS] != 0, norm = d.i[MKS_I_PROLOGUE] == MKS_P_NORM;
+    const bool bf16 = d.i[MKS_I_FMT] == MKS_FMT_BF16, two = !PLAIN && d.i[MKS_I_PIECES] == 2;
+    const int nseg = seg1 - seg0, cols = nseg * kc, stride = xs_stride_bytes(cols);
+    const float* x = reinterpret_cast<const float*>(d.p[MKS_P_X]);
+    const float* nw = reinterpret_cast<const float*>(d.p[MKS_P_NORM_W]);
+    const int xstride = d.i[MKS_I_X_STRIDE], gstride = d.i[MKS_I_X_GSTRIDE];
     const float noff = d.f[MKS_F_NORM_OFF];
-    const float in_scale = d.f[MKS_F_IN_SCALE] != 0.f ? d.f[MKS_F_IN_SCALE] : 1.f;
-    const int xstride = d.i[MKS_I_X_STRIDE];
-    const int k4n = kc >> 2, total = M * k4n;
-    int* red_i = reinterpret_cast<int*>(S.red);
-    if (tid_() < MKS_MAX_BATCH) red_i[tid_()] = 0;
-    // two batches in flight: the next one is requested before the current one is used, so a panel of eight
-    // sequences costs one exposed round trip, not one per batch
-    float4 xv[XB], xn[XB];
-    auto request = [&](int base, float4 (&dst)[XB]) {
-#pragma unroll
-        for (int u = 0; u < XB; u++) {
-            const int idx = base + u * NCT + tid_();
-            if (idx < total) {
-                const int m = idx / k4n, k4 = idx - m * k4n;
-                dst[u] = __ldcg(reinterpret_cast<const float4*>(x + (size_t)m * xstride) + k4);
-            }
-        }
-    };
-    request(0, xv);
-    if (XB * NCT < total) request(XB * NCT, xn);
-    if (norm) {
-        // 1/rms of every sequence from the 16-element sums of squares of the whole input vector: warp m adds up
-        // sequence m's sums (all loads of a lane in flight at once, fixed order) while the other warps only wait for x
-        const int K = d.i[MKS_I_K_TOTAL], n16 = K / 16;
-        const float* ssq = reinterpret_cast<const float*>(d.p[MKS_P_X_SSQ]);
-        if (warp_() < M) {
-            const float* row = ssq + (size_t)warp_() * n16;
-            float s = 0.f;
-#pragma unroll 8
-            for (int j = lane_(); j < n16; j += 32) s += ldcg_f(row + j);
-            s = warp_sum(s);
-            if (lane_() == 0) S.rstd[warp_()] = rsqrtf(s / (float)K + d.f[MKS_F_EPS]);
-        }
-    }
+    const int c4n = cols >> 2, k4n = kc >> 2;
+    const int total = (c4n + NCT - 1) / NCT * M;                      // a thread's groups: column group tid + i NCT of sequence m, m fastest
+    const int nscale = reduce ? nseg * 8 : 8;
     // A bound on |input| known to the host (a normed vector cannot exceed sqrt(K) max|weight|) fixes the power-of-two
     // scale of the fp16 copy up front: the values then go to shared memory in their final form in one pass.
     const float bound = d.f[MKS_F_IN_BOUND];
-    const bool fixed_scale = bound > 0.f && fmt != MKS_FMT_BF16 && pieces == 1;
+    const bool fixed_scale = bound > 0.f && !bf16 && !two;
+    // what a pass over the input leaves: final values; bf16 copies and their largest magnitudes; the latter alone
+    enum { FINAL, COPY, LARGEST };
+    int mode = bf16 || fixed_scale ? FINAL : (two ? LARGEST : COPY);
+    bool first = true;
+    const bool once = PLAIN && mode == COPY && total <= XB;           // the bf16 values of the only round wait in registers
+    float4 xv[XB], wv[XB];
     float fscale = 1.f;
+    if (tid_() < nscale) {
+        S.xmax[tid_()] = 0;
+        if (bf16) S.xinv[tid_()] = 1.f;
+    }
     if (fixed_scale) {
         const int be = ((__float_as_int(bound) >> 23) & 0xff) - 126;          // bound < 2^be
         const int e = max(-100, min(100, 15 - be));
         fscale = __int_as_float((127 + e) << 23);
-        if (tid_() < MKS_MAX_BATCH) S.xinv[tid_()] = __int_as_float((127 - e) << 23);
+        if (tid_() < nscale) S.xinv[tid_()] = __int_as_float((127 - e) << 23);
     }
-    consumer_sync();
-    prof_mark(S, 4);
 #pragma unroll 1
-    for (int base = 0; base < total; base += XB * NCT) {
-        if (base) {
+    for (;;) {
+        int li = tid_(), lm = 0, pi = tid_(), pm = 0;                 // the next group to request, to work on
+#pragma unroll 1
+        for (int base = 0; base < total; base += XB) {
 #pragma unroll
-            for (int u = 0; u < XB; u++) xv[u] = xn[u];
-            if (base + XB * NCT < total) request(base + XB * NCT, xn);
-        }
+            for (int u = 0; u < XB; u++) {
+                xv[u] = wv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (base + u < total && li < c4n) {
+                    int grp = grp0, o = seg0 * kc + li * 4;
+                    if (reduce) {
+                        const int sg = li / k4n;
+                        grp = n_splits == 1 ? seg0 + sg : (seg0 + sg) / n_splits;
+                        o = (seg0 + sg - grp * n_splits) * kc + (li - sg * k4n) * 4;
+                    }
+                    if (!reduce || S.coef[grp * 8 + lm] != 0.f) xv[u] = __ldcg(reinterpret_cast<const float4*>(x + (size_t)grp * gstride + lm * xstride + o));
+                    if (norm) wv[u] = __ldg(reinterpret_cast<const float4*>(nw + o));
+                }
+                if (++lm == M) {
+                    lm = 0;
+                    li += NCT;
+                }
+            }
+            if (first) {
+                first = false;
+                if (norm && warp_() < M) {
+                    // 1/rms of every sequence from the 16-element sums of squares of the whole input vector: warp m adds up
+                    // sequence m's sums (a lane's loads in flight together, fixed order) while the other warps only wait for x
+                    const int K = d.i[MKS_I_K_TOTAL], n16 = K / 16;
+                    const float* row = reinterpret_cast<const float*>(d.p[MKS_P_X_SSQ]) + (size_t)warp_() * n16;
+                    float s = 0.f;
+#pragma unroll 8
+                    for (int j = lane_(); j < n16; j += 32) s += ldcg_f(row + j);
+                    s = warp_sum(s);
+                    if (lane_() == 0)
+                        S.rstd[warp_()] = rsqrtf(s / (float)K + d.f[MKS_F_EPS]) * (d.f[MKS_F_IN_SCALE] != 0.f ? d.f[MKS_F_IN_SCALE] : 1.f);
+                }
+                __syncwarp();
+                consumer_sync();
+                prof_mark(S, 4);
+            }
 #pragma unroll
-        for (int u = 0; u < XB; u++) {
-            const int idx = base + u * NCT + tid_();
-            const bool live = idx < total;
-            int m = 0;
-            float mx = 0.f;
-            if (live) {
-                m = idx / k4n;
-                const int k4 = idx - m * k4n;
+            for (int u = 0; u < XB; u++) {
+                if (base + u >= total) break;
+                const int c4 = pi, m = pm;
+                const bool live = c4 < c4n;
+                if (++pm == M) {
+                    pm = 0;
+                    pi += NCT;
+                }
+                const int sg = reduce ? c4 / k4n : 0;
                 float v[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w};
                 if (norm) {
-                    // the norm weights are the same few KB for every sequence: after the first they come from L1
-                    const float4 wv = __ldg(reinterpret_cast<const float4*>(nw) + k4);
-                    const float r = S.rstd[m] * in_scale;
-                    v[0] = v[0] * r * (noff + wv.x); v[1] = v[1] * r * (noff + wv.y);
-                    v[2] = v[2] * r * (noff + wv.z); v[3] = v[3] * r * (noff + wv.w);
+                    const float r = S.rstd[m];
+                    v[0] = v[0] * r * (noff + wv[u].x); v[1] = v[1] * r * (noff + wv[u].y);
+                    v[2] = v[2] * r * (noff + wv[u].z); v[3] = v[3] * r * (noff + wv[u].w);
                 }
-                if (pieces == 2) {
-                    // fp32 copy, parked in the two columns that sequence m's pieces will occupy... of sequence pair slot m
-                    *reinterpret_cast<float4*>(S.xs() + (size_t)(2 * m) * stride + (size_t)k4 * 16) = make_float4(v[0], v[1], v[2], v[3]);
-                } else {
-                    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
-                    v[0] = __low2float(lo); v[1] = __high2float(lo); v[2] = __low2float(hi); v[3] = __high2float(hi);
-                    if (fixed_scale) {
-                        const __half2 a2 = __floats2half2_rn(v[0] * fscale, v[1] * fscale), b2 = __floats2half2_rn(v[2] * fscale, v[3] * fscale);
-                        *reinterpret_cast<uint2*>(S.xs() + (size_t)m * stride + (size_t)k4 * 8) =
-                            make_uint2(*reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&b2));
-                    } else {
-                        *reinterpret_cast<uint2*>(S.xs() + (size_t)m * stride + (size_t)k4 * 8) =
-                            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                if (!two) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v[i] = bf16_round(v[i]);
+                }
+                if (once) xv[u] = make_float4(v[0], v[1], v[2], v[3]);
+                if (mode != FINAL) {
+                    // (magnitudes compare like their bits) a warp's 32 groups are one sequence's and lie in at most two splits
+                    const int bits = live ? __float_as_int(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])))) : 0;
+                    const int s0 = PLAIN ? 0 : __shfl_sync(0xffffffffu, sg, 0);
+                    const int a = __reduce_max_sync(0xffffffffu, sg == s0 ? bits : 0);
+                    if (lane_() == 0 && a > 0) atomicMax(&S.xmax[s0 * 8 + m], a);
+                    if (!PLAIN) {
+                        const int b = __reduce_max_sync(0xffffffffu, sg != s0 ? bits : 0);
+                        if (lane_() == 0 && b > 0) atomicMax(&S.xmax[s0 * 8 + 8 + m], b);
                     }
                 }
-                mx = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-            }
-            if (fmt != MKS_FMT_BF16 && !fixed_scale) {
-                // a warp's 32 groups lie in at most two sequences
-                const int m0 = __shfl_sync(0xffffffffu, m, 0);
-                const float a = warp_max(live && m == m0 ? mx : 0.f), b = warp_max(live && m != m0 ? mx : 0.f);
-                if (lane_() == 0) {
-                    if (a > 0.f) atomicMax(&red_i[m0], __float_as_int(a));
-                    if (b > 0.f) atomicMax(&red_i[min(m0 + 1, MKS_MAX_BATCH - 1)], __float_as_int(b));
+                if (live && mode != LARGEST && !once) {
+                    uint8_t* dst = S.xs() + m * stride + c4 * 8;
+                    const bool as_bf16 = bf16 || mode == COPY;
+                    if (!as_bf16) {
+                        const float sc = two ? __int_as_float(S.xmax[sg * 8 + m]) : fscale;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) v[i] *= sc;
+                    }
+                    uint32_t hi[2];
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        const __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                        const __half2 h2 = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+                        hi[i] = as_bf16 ? *reinterpret_cast<const uint32_t*>(&b2) : *reinterpret_cast<const uint32_t*>(&h2);
+                        if (two) {                                 // what the first piece lost
+                            v[2 * i] -= bf16 ? __low2float(b2) : __low2float(h2);
+                            v[2 * i + 1] -= bf16 ? __high2float(b2) : __high2float(h2);
+                        }
+                    }
+                    *reinterpret_cast<uint2*>(dst) = make_uint2(hi[0], hi[1]);
+                    if (two) {
+#pragma unroll
+                        for (int i = 0; i < 2; i++) {
+                            const __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                            const __half2 h2 = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+                            hi[i] = bf16 ? *reinterpret_cast<const uint32_t*>(&b2) : *reinterpret_cast<const uint32_t*>(&h2);
+                        }
+                        *reinterpret_cast<uint2*>(dst + M * stride) = make_uint2(hi[0], hi[1]);
+                    }
                 }
             }
         }
-    }
-    if (fixed_scale) return;                                   // staged in final form; the caller's barrier publishes it
-    if (fmt == MKS_FMT_BF16) {
-        if (tid_() < 8) S.xinv[tid_()] = 1.f;
-        if (pieces == 2) {
-            // fp32-exact inputs for bf16 weights: x = hi + lo, both bf16 (16 significant bits), no scaling needed
-            consumer_sync();
-            float v[16];
-            int n = 0;
-#pragma unroll 1
-            for (int idx = tid_(); idx < M * kc && n < 16; idx += NCT, n++) {
-                const int m = idx / kc, k = idx - m * kc;
-                v[n] = *reinterpret_cast<const float*>(S.xs() + (size_t)(2 * m) * stride + (size_t)k * 4);
-            }
-            consumer_sync();
-            n = 0;
-#pragma unroll 1
-            for (int idx = tid_(); idx < M * kc && n < 16; idx += NCT, n++) {
-                const int m = idx / kc, k = idx - m * kc;
-                const __nv_bfloat16 hi = __float2bfloat16_rn(v[n]);
-                reinterpret_cast<__nv_bfloat16*>(S.xs() + (size_t)m * stride)[k] = hi;
-                reinterpret_cast<__nv_bfloat16*>(S.xs() + (size_t)(M + m) * stride)[k] = __float2bfloat16_rn(v[n] - __bfloat162float(hi));
-            }
-        }
-        return;
-    }
-    consumer_sync();
-    prof_mark(S, 5);
-    if (tid_() < M) {
-        // a = f * 2^e with f in [0.5, 1): the exponent field gives e; scale = 2^(14 - e), built from its bits
-        const int bits = red_i[tid_()];
-        int e = bits > 0 && bits < 0x7f800000 ? ((bits >> 23) & 0xff) - 126 : 0;
-        e = max(-100, min(100, 14 - e));
-        S.red[MKS_MAX_BATCH + tid_()] = __int_as_float((127 + e) << 23);
-        S.xinv[tid_()] = __int_as_float((127 - e) << 23);
-        if (pieces == 2) S.xinv[M + tid_()] = __int_as_float((127 - e) << 23);
-    }
-    consumer_sync();
-    prof_mark(S, 6);
-    if (pieces == 2) {
-        // at most 16 values per thread (checked by the host): read the fp32 copies, then overwrite them with the pieces
-        float v[16];
-        int n = 0;
-#pragma unroll 1
-        for (int idx = tid_(); idx < M * kc && n < 16; idx += NCT, n++) {
-            const int m = idx / kc, k = idx - m * kc;
-            v[n] = *reinterpret_cast<const float*>(S.xs() + (size_t)(2 * m) * stride + (size_t)k * 4) * S.red[MKS_MAX_BATCH + m];
-        }
+        if (mode == FINAL) return;                                 // the caller's barrier publishes it
+        __syncwarp();
         consumer_sync();
-        n = 0;
-#pragma unroll 1
-        for (int idx = tid_(); idx < M * kc && n < 16; idx += NCT, n++) {
-            const int m = idx / kc, k = idx - m * kc;
-            const __half hi = __float2half_rn(v[n]);
-            reinterpret_cast<__half*>(S.xs() + (size_t)m * stride)[k] = hi;
-            reinterpret_cast<__half*>(S.xs() + (size_t)(M + m) * stride)[k] = __float2half_rn(v[n] - __half2float(hi));
+        prof_mark(S, 5);
+        if (once) {
+            int m = 0, c4 = tid_();
+#pragma unroll
+            for (int u = 0; u < XB; u++) {
+                if (u >= total) break;
+                const int e = scale_exponent(S.xmax[m]);
+                const float sc = __int_as_float((127 + e) << 23);
+                if (c4 < c4n) {
+                    const __half2 a2 = __floats2half2_rn(xv[u].x * sc, xv[u].y * sc), b2 = __floats2half2_rn(xv[u].z * sc, xv[u].w * sc);
+                    *reinterpret_cast<uint2*>(S.xs() + m * stride + c4 * 8) =
+                        make_uint2(*reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&b2));
+                }
+                if (tid_() == 0) S.xinv[m] = __int_as_float((127 - e) << 23);
+                if (++m == M) {
+                    m = 0;
+                    c4 += NCT;
+                }
+            }
+            return;
         }
-        return;
+        if (tid_() < nscale && (tid_() & 7) < M) {
+            const int e = scale_exponent(S.xmax[tid_()]);
+            S.xmax[tid_()] = (127 + e) << 23;
+            S.xinv[tid_()] = __int_as_float((127 - e) << 23);
+            if (two) S.xinv[tid_() + M] = __int_as_float((127 - e) << 23);
+        }
+        __syncwarp();
+        consumer_sync();
+        prof_mark(S, 6);
+        if (mode == COPY) break;
+        mode = FINAL;
     }
     // bf16 -> scaled fp16 in place, eight values per thread and turn
-    const int k8n = kc >> 3;
+    const int c8n = cols >> 3, k8n = kc >> 3;
 #pragma unroll 1
-    for (int idx = tid_(); idx < M * k8n; idx += NCT) {
-        const int m = idx / k8n, k8 = idx - m * k8n;
-        uint4* pq = reinterpret_cast<uint4*>(S.xs() + (size_t)m * stride) + k8;
-        const uint4 q = *pq;
-        const float sc = S.red[MKS_MAX_BATCH + m];
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-        uint32_t o[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const __half2 h = __floats2half2_rn(bf_lo(w[i]) * sc, bf_hi(w[i]) * sc);
-            o[i] = *reinterpret_cast<const uint32_t*>(&h);
+    for (int c8 = tid_(); c8 < c8n; c8 += NCT) {
+        const int sg = reduce ? c8 / k8n : 0;
+#pragma unroll 1
+        for (int m = 0; m < M; m++) {
+            uint4* pq = reinterpret_cast<uint4*>(S.xs() + m * stride) + c8;
+            uint4 q = *pq;
+            const float sc = __int_as_float(S.xmax[sg * 8 + m]);
+            auto conv = [&](uint32_t w) {
+                const __half2 h = __floats2half2_rn(bf_lo(w) * sc, bf_hi(w) * sc);
+                return *reinterpret_cast<const uint32_t*>(&h);
+            };
+            q.x = conv(q.x); q.y = conv(q.y); q.z = conv(q.z); q.w = conv(q.w);
+            *pq = q;
         }
-        *pq = make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
 
 // ---- tensor-parallel all-reduce of one output tile -------------------------------------------------------------
 // Mailbox of a rank: [2 halves][MAILBOX_TILES][ranks][128] 64-bit words (value | tag << 32), then the key
 // exchange area [2][ranks][8][2].  Each lane owns four words of the tile.
-__device__ __forceinline__ bool allreduce_tile(Shared& S, Mut& mu, const Args& A, u64 seq, int tile, float (&acc)[4]) {
+__device__ __noinline__ float4 allreduce_tile(Shared& S, const Args& A, u64 seq, int tile, float4 in) {
+    const float acc[4] = {in.x, in.y, in.z, in.w};
     const uint32_t tag = (uint32_t)seq;
     const size_t base = (((size_t)(seq & 1) * MAILBOX_TILES + tile) * MKS_MAX_RANKS);
 #pragma unroll 1
@@ -669,361 +867,440 @@ __device__ __forceinline__ bool allreduce_tile(Shared& S, Mut& mu, const Args& A
             }
             if (__all_sync(0xffffffffu, ok)) break;
             if (!ok && MKS_SPIN_FAIL(S, s, WS_MAILBOX)) fail = true;
-            if (__any_sync(0xffffffffu, fail)) {
-                mu.dead = true;
-                return false;
-            }
+            if (__any_sync(0xffffffffu, fail)) return in;         // (the abort flag is set)
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) sum[i] += __uint_as_float((uint32_t)w[i]);
     }
-#pragma unroll
-    for (int i = 0; i < 4; i++) acc[i] = sum[i];
-    return true;
+    return make_float4(sum[0], sum[1], sum[2], sum[3]);
 }
 
 // ---- GEMV stage (consumers) ----------------------------------------------------------------------------------
-// Lane (g = lane / 4, t = lane % 4) of the warp that owns a unit holds, per tile step, 8 bytes of row g
-// and 8 bytes of row g + 8: the values that MMA j of the step multiplies with input columns
-// k0 + 16 j + 4 t + {0, 1, 2, 3}.  Its accumulators are rows g, g + 8 x sequences 2t, 2t + 1.
-struct Best2 {
-    u64 k0 = 0, k1 = 0;
-};
-
-// The hot loop is a function of its own with a handful of scalar arguments: inlined into the stage function it
-// shared that function's register budget (96 with 17 warps resident) and spilled inside the loop, and spilled
-// registers of 544 threads do not fit the L1 that the shared-memory carve-out leaves.
-struct UnitGeo {
-    int n_chunks, chunk_steps;
-};
+// Lane (g = lane / 4, t = lane % 4) of a warp holds, per tile step, 8 bytes of row g and 8 bytes of row g + 8: the
+// values that MMA j of the step multiplies with input columns k0 + 16 j + 4 t + {0, 1, 2, 3}.  Its accumulators are
+// rows g, g + 8 x sequences 2t, 2t + 1.
+//
+// (volatile: they stay behind the wait for the copies they read)
+__device__ __forceinline__ uint4 lds_u4(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float2 lds_f2(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
+// One tile step: accumulates into acc / acc2 (two chains: consecutive MMAs never wait for each other).
 template <int FMT>
-__device__ __noinline__ float4 unit_steps(Shared& S, UnitGeo gm, uint32_t chunk0, const uint8_t* xcol, bool col_live, bool blocks) {
-    constexpr int MMAS = FMT == MKS_FMT_MXFP4 ? 4 : (FMT == MKS_FMT_BF16 ? 1 : 2);
-    const int g = lane_() >> 2, t = lane_() & 3;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f}, acc2[4] = {0.f, 0.f, 0.f, 0.f};    // two chains: consecutive MMAs never wait for each other
-    float tmp[4] = {0.f, 0.f, 0.f, 0.f}, tmp2[4] = {0.f, 0.f, 0.f, 0.f};
-    const uint32_t depth = (uint32_t)S.A.ring_depth;
-    int kstep = 0;                                            // tile step inside the unit
-#pragma unroll 1
-    for (int ch = 0; ch < gm.n_chunks; ch++) {
-        const uint32_t qq = chunk0 + (uint32_t)ch;               // this warp's chunk counter
-        const int slot = warp_() * (int)depth + (int)(qq % depth);
-        if (!mbar_wait2(S, &S.full[slot], (qq / depth) & 1, WS_FULL)) break;
-        const uint8_t* sl = S.ring() + (size_t)slot * SLOT_BYTES;
-        const uint8_t* sc_base = sl + gm.chunk_steps * 512;
-#pragma unroll 4
-        for (int st = 0; st < gm.chunk_steps; st++, kstep++) {
-            const uint4 wq = *reinterpret_cast<const uint4*>(sl + st * 512 + lane_() * 16);
-            const uint8_t* xk = xcol + (size_t)kstep * (MMAS * 16) * 2 + t * 8;
-            if (FMT == MKS_FMT_MXFP4) {
-                // The conversion unit (cvt ... e2m1x2) is the scarcest pipe of this loop, so only half of the
-                // values go through it.  The 32 columns of scale group 0 (MMAs 0 and 1) arrive with their bits
-                // pre-arranged by the packer: every 32-bit word yields four f16x2 registers with shifts and masks
-                // alone (sign at bit 15, the three magnitude bits at 11..9 of each half: the value times 2^-14,
-                // which the group's scale takes back).  Scale group 1 (MMAs 2 and 3) keeps plain nibbles.
-                const uint32_t scw = *reinterpret_cast<const uint32_t*>(sc_base + st * 32 + g * 4);
-                float t0[4] = {0.f, 0.f, 0.f, 0.f}, t1[4] = {0.f, 0.f, 0.f, 0.f};      // scale group 0: MMAs 0, 1
-                float u0[4] = {0.f, 0.f, 0.f, 0.f}, u1[4] = {0.f, 0.f, 0.f, 0.f};      // scale group 1: MMAs 2, 3
-                uint2 b[4];
+__device__ __forceinline__ void tile_step(uint32_t sl, uint32_t sc, int st, const uint8_t* xk, float (&acc)[4], float (&acc2)[4]) {
+    const uint4 wq = lds_u4(sl);
+    if (FMT == MKS_FMT_MXFP4) {
+        // The conversion unit (cvt ... e2m1x2) is the scarcest pipe of this loop, so only half of the
+        // values go through it.  The 32 columns of scale group 0 (MMAs 0 and 1) arrive with their bits
+        // pre-arranged by the packer: every 32-bit word yields four f16x2 registers with shifts and masks
+        // alone (sign at bit 15, the three magnitude bits at 11..9 of each half: the value times 2^-14,
+        // which the group's scale takes back).  Scale group 1 (MMAs 2 and 3) keeps plain nibbles.
+        const uint32_t scw = lds_u32(sc);
+        float t0[4] = {0.f, 0.f, 0.f, 0.f};                                    // scale group 0: MMAs 0, 1
+        float u0[4] = {0.f, 0.f, 0.f, 0.f};                                    // scale group 1: MMAs 2, 3
+        uint2 b[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    b[j] = make_uint2(0u, 0u);
-                    if (col_live) b[j] = *reinterpret_cast<const uint2*>(xk + j * 32);
-                }
-                {
-                    const uint32_t lo = wq.x, hi = wq.z;                  // row g, row g + 8
-                    uint32_t a[4];
-                    a[0] = lo & 0x8E008E00u;
-                    a[1] = hi & 0x8E008E00u;
-                    a[2] = (lo << 3) & 0x8E008E00u;
-                    a[3] = (hi << 3) & 0x8E008E00u;
-                    mma_f16(t0, a, b[0].x, b[0].y);
-                    a[0] = ((lo << 1) & 0x80008000u) | ((lo << 6) & 0x0E000E00u);
-                    a[1] = ((hi << 1) & 0x80008000u) | ((hi << 6) & 0x0E000E00u);
-                    a[2] = ((lo << 2) & 0x80008000u) | ((lo << 9) & 0x0E000E00u);
-                    a[3] = ((hi << 2) & 0x80008000u) | ((hi << 9) & 0x0E000E00u);
-                    mma_f16(t1, a, b[1].x, b[1].y);
-                }
-                {
-                    const uint32_t lo = wq.y, hi = wq.w;
-                    uint32_t a[4];
-                    a[0] = cvt_e2m1x2(lo);
-                    a[2] = cvt_e2m1x2(lo >> 8);
-                    a[1] = cvt_e2m1x2(hi);
-                    a[3] = cvt_e2m1x2(hi >> 8);
-                    mma_f16(u0, a, b[2].x, b[2].y);
-                    a[0] = cvt_e2m1x2(lo >> 16);
-                    a[2] = cvt_e2m1x2(lo >> 24);
-                    a[1] = cvt_e2m1x2(hi >> 16);
-                    a[3] = cvt_e2m1x2(hi >> 24);
-                    mma_f16(u1, a, b[3].x, b[3].y);
-                }
-                // e8m0 scales: bytes [row g: group 0, group 1, row g + 8: group 0, group 1]; group 0 also takes 2^14
-                const float s00 = __uint_as_float(((scw & 0xFFu) + 14u) << 23), s01 = __uint_as_float(((scw >> 8) & 0xFFu) << 23);
-                const float s10 = __uint_as_float((((scw >> 16) & 0xFFu) + 14u) << 23), s11 = __uint_as_float((scw >> 24) << 23);
-                acc[0] = fmaf(t0[0] + t1[0], s00, acc[0]); acc[1] = fmaf(t0[1] + t1[1], s00, acc[1]);
-                acc[2] = fmaf(t0[2] + t1[2], s10, acc[2]); acc[3] = fmaf(t0[3] + t1[3], s10, acc[3]);
-                acc[0] = fmaf(u0[0] + u1[0], s01, acc[0]); acc[1] = fmaf(u0[1] + u1[1], s01, acc[1]);
-                acc[2] = fmaf(u0[2] + u1[2], s11, acc[2]); acc[3] = fmaf(u0[3] + u1[3], s11, acc[3]);
-            } else if (FMT == MKS_FMT_FP8) {
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const uint32_t lo = j == 0 ? wq.x : wq.y, hi = j == 0 ? wq.z : wq.w;
-                    uint32_t a[4];
-                    a[0] = cvt_e4m3x2(lo);
-                    a[2] = cvt_e4m3x2(lo >> 16);
-                    a[1] = cvt_e4m3x2(hi);
-                    a[3] = cvt_e4m3x2(hi >> 16);
-                    uint2 b = make_uint2(0u, 0u);
-                    if (col_live) b = *reinterpret_cast<const uint2*>(xk + j * 32);
-                    if (blocks) mma_f16(j == 0 ? tmp : tmp2, a, b.x, b.y);
-                    else mma_f16(j == 0 ? acc : acc2, a, b.x, b.y);
-                }
-                if (blocks && (kstep & 3) == 3) {
-                    // one scale per 128 k for rows 0-7 of the tile and one for rows 8-15 (a GLU tile pairs two matrices)
-                    const float2 bs = *reinterpret_cast<const float2*>(sc_base + (st >> 2) * 8);
-                    acc[0] = fmaf(tmp[0] + tmp2[0], bs.x, acc[0]); acc[1] = fmaf(tmp[1] + tmp2[1], bs.x, acc[1]);
-                    acc[2] = fmaf(tmp[2] + tmp2[2], bs.y, acc[2]); acc[3] = fmaf(tmp[3] + tmp2[3], bs.y, acc[3]);
-                    tmp[0] = tmp[1] = tmp[2] = tmp[3] = 0.f;
-                    tmp2[0] = tmp2[1] = tmp2[2] = tmp2[3] = 0.f;
-                }
-            } else if (FMT == MKS_FMT_INT8) {
-                const uint32_t x0 = wq.x ^ 0x80808080u, x1 = wq.y ^ 0x80808080u, x2 = wq.z ^ 0x80808080u, x3 = wq.w ^ 0x80808080u;
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const uint32_t lo = j == 0 ? x0 : x1, hi = j == 0 ? x2 : x3;
-                    uint32_t a[4];
-                    a[0] = cvt_s8x2(lo, 0x4140);
-                    a[2] = cvt_s8x2(lo, 0x4342);
-                    a[1] = cvt_s8x2(hi, 0x4140);
-                    a[3] = cvt_s8x2(hi, 0x4342);
-                    uint2 b = make_uint2(0u, 0u);
-                    if (col_live) b = *reinterpret_cast<const uint2*>(xk + j * 32);
-                    mma_f16(j == 0 ? acc : acc2, a, b.x, b.y);
-                }
-            } else {
-                uint32_t a[4] = {wq.x, wq.z, wq.y, wq.w};                 // row g: (x, y), row g + 8: (z, w)
-                uint2 b = make_uint2(0u, 0u);
-                if (col_live) b = *reinterpret_cast<const uint2*>(xk);
-                if (st & 1) mma_bf16(acc2, a, b.x, b.y);
-                else mma_bf16(acc, a, b.x, b.y);
-            }
+        for (int j = 0; j < 4; j++) b[j] = *reinterpret_cast<const uint2*>(xk + j * 32);
+        {
+            const uint32_t lo = wq.x, hi = wq.z;                  // row g, row g + 8
+            uint32_t a[4];
+            a[0] = lo & 0x8E008E00u;
+            a[1] = hi & 0x8E008E00u;
+            a[2] = (lo << 3) & 0x8E008E00u;
+            a[3] = (hi << 3) & 0x8E008E00u;
+            mma_f16(t0, a, b[0].x, b[0].y);
+            a[0] = ((lo << 1) & 0x80008000u) | ((lo << 6) & 0x0E000E00u);
+            a[1] = ((hi << 1) & 0x80008000u) | ((hi << 6) & 0x0E000E00u);
+            a[2] = ((lo << 2) & 0x80008000u) | ((lo << 9) & 0x0E000E00u);
+            a[3] = ((hi << 2) & 0x80008000u) | ((hi << 9) & 0x0E000E00u);
+            mma_f16(t0, a, b[1].x, b[1].y);
         }
-        __syncwarp();
-        if (lane_() == 0) mbar_arrive(&S.empty[slot]);
+        {
+            const uint32_t lo = wq.y, hi = wq.w;
+            uint32_t a[4];
+            a[0] = cvt_e2m1x2(lo);
+            a[2] = cvt_e2m1x2(lo >> 8);
+            a[1] = cvt_e2m1x2(hi);
+            a[3] = cvt_e2m1x2(hi >> 8);
+            mma_f16(u0, a, b[2].x, b[2].y);
+            a[0] = cvt_e2m1x2(lo >> 16);
+            a[2] = cvt_e2m1x2(lo >> 24);
+            a[1] = cvt_e2m1x2(hi >> 16);
+            a[3] = cvt_e2m1x2(hi >> 24);
+            mma_f16(u0, a, b[3].x, b[3].y);
+        }
+        // e8m0 scales: bytes [row g: group 0, group 1, row g + 8: group 0, group 1]; group 0 also takes 2^14
+        const float s00 = __uint_as_float(((scw & 0xFFu) + 14u) << 23), s01 = __uint_as_float(((scw >> 8) & 0xFFu) << 23);
+        const float s10 = __uint_as_float((((scw >> 16) & 0xFFu) + 14u) << 23), s11 = __uint_as_float((scw >> 24) << 23);
+        acc[0] = fmaf(t0[0], s00, acc[0]); acc[1] = fmaf(t0[1], s00, acc[1]);
+        acc[2] = fmaf(t0[2], s10, acc[2]); acc[3] = fmaf(t0[3], s10, acc[3]);
+        acc2[0] = fmaf(u0[0], s01, acc2[0]); acc2[1] = fmaf(u0[1], s01, acc2[1]);
+        acc2[2] = fmaf(u0[2], s11, acc2[2]); acc2[3] = fmaf(u0[3], s11, acc2[3]);
+    } else if (FMT == MKS_FMT_FP8) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const uint32_t lo = j == 0 ? wq.x : wq.y, hi = j == 0 ? wq.z : wq.w;
+            uint32_t a[4];
+            a[0] = cvt_e4m3x2(lo);
+            a[2] = cvt_e4m3x2(lo >> 16);
+            a[1] = cvt_e4m3x2(hi);
+            a[3] = cvt_e4m3x2(hi >> 16);
+            const uint2 b = *reinterpret_cast<const uint2*>(xk + j * 32);
+            mma_f16(j == 0 ? acc : acc2, a, b.x, b.y);
+        }
+    } else if (FMT == MKS_FMT_INT8) {
+        const uint32_t x0 = wq.x ^ 0x80808080u, x1 = wq.y ^ 0x80808080u, x2 = wq.z ^ 0x80808080u, x3 = wq.w ^ 0x80808080u;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const uint32_t lo = j == 0 ? x0 : x1, hi = j == 0 ? x2 : x3;
+            uint32_t a[4];
+            a[0] = cvt_s8x2(lo, 0x4140);
+            a[2] = cvt_s8x2(lo, 0x4342);
+            a[1] = cvt_s8x2(hi, 0x4140);
+            a[3] = cvt_s8x2(hi, 0x4342);
+            const uint2 b = *reinterpret_cast<const uint2*>(xk + j * 32);
+            mma_f16(j == 0 ? acc : acc2, a, b.x, b.y);
+        }
+    } else {
+        uint32_t a[4] = {wq.x, wq.z, wq.y, wq.w};                 // row g: (x, y), row g + 8: (z, w)
+        const uint2 b = *reinterpret_cast<const uint2*>(xk);
+        if (st & 1) mma_bf16(acc2, a, b.x, b.y);
+        else mma_bf16(acc, a, b.x, b.y);
     }
-    return make_float4(acc[0] + acc2[0], acc[1] + acc2[1], acc[2] + acc2[2], acc[3] + acc2[3]);
 }
 
-__device__ __noinline__ void gemv_stage(Shared& S, Mut& mu, const mk_stage_desc& d, const Args& A, u64& ar_seq) {
-    const Gemv gm = gemv_geometry(S, d);
-    const int fmt = d.i[MKS_I_FMT], epi = d.i[MKS_I_EPILOGUE], pieces = d.i[MKS_I_PIECES];
-    const int kc = d.i[MKS_I_KC];
-    const int stride = xs_stride_bytes(kc);
-    const int g = lane_() >> 2, t = lane_() & 3;
-    const int ncols = S.A.M * pieces;
-    const bool reduce_groups = d.i[MKS_I_REDUCE_GROUPS] != 0;
-    const int arrivals = reduce_groups ? gm.G * gm.S : gm.S;
-    const bool ar = d.i[MKS_I_ALLREDUCE] != 0 && A.tp > 1;
-    if (ar) ar_seq++;
-    unsigned* cnt = reinterpret_cast<unsigned*>(d.p[MKS_P_CNT]);
-    float* part = reinterpret_cast<float*>(d.p[MKS_P_PART]);
-    Best2 best;
+// Partial tiles of a stage with several panels: [tile][panel][8 sequences][8 row pairs][2] words (value | tag << 32); only
+// live sequences' columns are written and read.
+__device__ __forceinline__ unsigned long long* tile_words(unsigned long long* part, int tile_panel) {
+    return part + (size_t)tile_panel * 128 + (lane_() & 3) * 32 + (lane_() >> 2) * 2;
+}
+__device__ __forceinline__ void publish_tile(unsigned long long* dst, uint32_t tag, int M, const float (&v)[4]) {
+    chaos_delay();
+    const u64 t = (u64)tag << 32;
+    const int m0 = 2 * (lane_() & 3);
+    if (m0 < M) asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(dst), "l"(t | __float_as_uint(v[0])), "l"(t | __float_as_uint(v[2])) : "memory");
+    if (m0 + 1 < M) asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(dst + 16), "l"(t | __float_as_uint(v[1])), "l"(t | __float_as_uint(v[3])) : "memory");
+}
+// The sum of the P partial tiles at `src`, in panel order, four panels' words in flight.  False: a wait ran out.
+__device__ __forceinline__ bool collect_tile(Shared& S, const unsigned long long* src, uint32_t tag, int P, float (&acc)[4]) {
+    acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+    const int m0 = 2 * (lane_() & 3);
+    const bool l0 = m0 < S.A.M, l1 = m0 + 1 < S.A.M;
 #pragma unroll 1
-    for (int pu = gm.u0; pu < gm.u1;) {
-        const int panel = pu / gm.T;
-        const int pend = min(gm.u1, (panel + 1) * gm.T);
-        const int grp = (int)(panel / gm.S), split = (int)(panel % gm.S);
-        consumer_sync();                                     // everybody is done reading the previous panel's input
-        stage_x(S, mu, d, grp, split);
-        consumer_sync();
-        if (pu == gm.u0) prof_mark(S, 1);
-        const float* rs = group_row_scale(S, d, grp, gm.G);
+    for (int p0 = 0; p0 < P; p0 += 4) {
+        u64 w[4][4];
+        Spin2 s;
+        bool fail = false;
 #pragma unroll 1
-        for (int r0 = pu; r0 < pend; r0 += NCW) {
-            const int nj = min(NCW, pend - r0);
-            if (warp_() < nj && !mu.dead) {
-                const int tile = (int)((r0 + warp_()) - panel * gm.T);
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                const uint8_t* xcol = S.xs() + (size_t)g * stride;
-                const bool live = g < ncols;
-                const uint32_t chunk0 = mu.chunk_n;
-                UnitGeo ug;
-                ug.n_chunks = gm.n_chunks;
-                ug.chunk_steps = gm.chunk_steps;
-                const bool blocks = d.i[MKS_I_BLOCK_SCALES] != 0;
-                float4 r;
-                switch (fmt) {
-                    case MKS_FMT_MXFP4: r = unit_steps<MKS_FMT_MXFP4>(S, ug, chunk0, xcol, live, blocks); break;
-                    case MKS_FMT_FP8: r = unit_steps<MKS_FMT_FP8>(S, ug, chunk0, xcol, live, blocks); break;
-                    case MKS_FMT_INT8: r = unit_steps<MKS_FMT_INT8>(S, ug, chunk0, xcol, live, blocks); break;
-                    default: r = unit_steps<MKS_FMT_BF16>(S, ug, chunk0, xcol, live, blocks); break;
-                }
-                acc[0] = r.x; acc[1] = r.y; acc[2] = r.z; acc[3] = r.w;
-                // undo the input scaling, fold the second piece's columns onto the first
-                acc[0] *= S.xinv[2 * t]; acc[2] *= S.xinv[2 * t];
-                acc[1] *= S.xinv[2 * t + 1]; acc[3] *= S.xinv[2 * t + 1];
-                if (pieces == 2) {
-                    // columns [0, M) + columns [M, 2M): lane t holds columns 2t, 2t + 1
+        for (;;) {                                               // the warp leaves together
+            bool ok = true;
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int col = 2 * t + (i & 1);
-                        const int src_col = col + S.A.M;                      // the partner column, if col < M
-                        const float other = __shfl_sync(0xffffffffu, acc[i], (lane_() & ~3) | ((src_col >> 1) & 3));
-                        const float other1 = __shfl_sync(0xffffffffu, acc[i ^ 1], (lane_() & ~3) | ((src_col >> 1) & 3));
-                        const float add = (src_col & 1) == (i & 1) ? other : other1;
-                        if (col < S.A.M) acc[i] += add;
-                    }
-                }
-                if (rs) {
-                    const float s0 = rs[tile * 16 + g], s1 = rs[tile * 16 + g + 8];
-                    acc[0] *= s0; acc[1] *= s0; acc[2] *= s1; acc[3] *= s1;
-                }
-                bool finish = true;
-                const int cidx = reduce_groups ? tile : grp * gm.T + tile;
-                if (arrivals > 1) {
-                    const int aslot = reduce_groups ? grp * gm.S + split : split;
-                    float4* pp = reinterpret_cast<float4*>(part + ((size_t)cidx * arrivals + aslot) * 128) + lane_();
-                    __stcg(pp, make_float4(acc[0], acc[1], acc[2], acc[3]));
-                    fence_acq_rel_gpu();
-                    __syncwarp();
-                    unsigned old = 0;
-                    if (lane_() == 0) {
-                        chaos_delay();
-                        old = atomicAdd(cnt + cidx, 1u);
-                        // the last arriver puts the counter back: the number of arrivals of a routed stage changes
-                        // from step to step, and nobody touches the counter again before the stage's barrier
-                        if (old + 1u == (unsigned)arrivals) cnt[cidx] = 0u;
-                    }
-                    old = __shfl_sync(0xffffffffu, old, 0);
-                    finish = old + 1u == (unsigned)arrivals;
-                    if (finish) {
-                        fence_acq_rel_gpu();
-                        acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-                        // eight partial tiles are requested at a time, then added in arrival-slot order
-#pragma unroll 1
-                        for (int a0 = 0; a0 < arrivals; a0 += 8) {
-                            float4 v[8];
-#pragma unroll
-                            for (int u = 0; u < 8; u++)
-                                if (a0 + u < arrivals)
-                                    v[u] = __ldcg(reinterpret_cast<const float4*>(part + ((size_t)cidx * arrivals + a0 + u) * 128) + lane_());
-#pragma unroll
-                            for (int u = 0; u < 8; u++)
-                                if (a0 + u < arrivals) {
-                                    float c0 = 1.f, c1 = 1.f;
-                                    if (reduce_groups) {
-                                        c0 = S.coef[((a0 + u) / gm.S) * 8 + 2 * t];
-                                        c1 = S.coef[((a0 + u) / gm.S) * 8 + 2 * t + 1];
-                                    }
-                                    acc[0] = fmaf(v[u].x, c0, acc[0]); acc[1] = fmaf(v[u].y, c1, acc[1]);
-                                    acc[2] = fmaf(v[u].z, c0, acc[2]); acc[3] = fmaf(v[u].w, c1, acc[3]);
-                                }
-                        }
-                    }
-                } else if (reduce_groups) {
-                    acc[0] *= S.coef[2 * t]; acc[2] *= S.coef[2 * t];
-                    acc[1] *= S.coef[2 * t + 1]; acc[3] *= S.coef[2 * t + 1];
-                }
-                if (finish && ar) finish = allreduce_tile(S, mu, A, ar_seq, tile, acc);
-                if (finish) {
-                    // rows g, g + 8 of the tile x sequences 2t, 2t + 1
-                    const int ostride = d.i[MKS_I_OUT_STRIDE];
-                    const int ogrp = reduce_groups ? 0 : grp;
-                    float* out = reinterpret_cast<float*>(d.p[MKS_P_OUT]) + (size_t)ogrp * d.i[MKS_I_OUT_GSTRIDE];
-                    const int nvalid = d.i[MKS_I_N_VALID];
-                    const int m0 = 2 * t, m1 = 2 * t + 1;
-                    if (epi == MKS_E_STORE) {
-                        const int ra = tile * 16 + g, rb = ra + 8;
-                        if (m0 < S.A.M) {
-                            if (ra < nvalid) __stcg(out + (size_t)m0 * ostride + ra, acc[0]);
-                            if (rb < nvalid) __stcg(out + (size_t)m0 * ostride + rb, acc[2]);
-                        }
-                        if (m1 < S.A.M) {
-                            if (ra < nvalid) __stcg(out + (size_t)m1 * ostride + ra, acc[1]);
-                            if (rb < nvalid) __stcg(out + (size_t)m1 * ostride + rb, acc[3]);
-                        }
-                        float* ssq = reinterpret_cast<float*>(d.p[MKS_P_OUT_SSQ]);
-                        if (ssq) {                              // the sums of squares a later norm of this vector needs (whole tiles only)
-                            float q0 = acc[0] * acc[0] + acc[2] * acc[2], q1 = acc[1] * acc[1] + acc[3] * acc[3];
-#pragma unroll
-                            for (int o = 4; o < 32; o <<= 1) {
-                                q0 += __shfl_xor_sync(0xffffffffu, q0, o);
-                                q1 += __shfl_xor_sync(0xffffffffu, q1, o);
-                            }
-                            if (g == 0) {
-                                const int ntile = nvalid / 16;
-                                if (m0 < S.A.M) __stcg(ssq + (size_t)m0 * ntile + tile, q0);
-                                if (m1 < S.A.M) __stcg(ssq + (size_t)m1 * ntile + tile, q1);
-                            }
-                        }
-                    } else if (epi == MKS_E_RESID) {
-                        const int ra = tile * 16 + g, rb = ra + 8;
-                        float* ssq = reinterpret_cast<float*>(d.p[MKS_P_OUT_SSQ]);
-                        float q0 = 0.f, q1 = 0.f;
-                        if (m0 < S.A.M) {
-                            const float a = ldcg_f(out + (size_t)m0 * ostride + ra) + acc[0];
-                            const float b = ldcg_f(out + (size_t)m0 * ostride + rb) + acc[2];
-                            __stcg(out + (size_t)m0 * ostride + ra, a);
-                            __stcg(out + (size_t)m0 * ostride + rb, b);
-                            q0 = a * a + b * b;
-                        }
-                        if (m1 < S.A.M) {
-                            const float a = ldcg_f(out + (size_t)m1 * ostride + ra) + acc[1];
-                            const float b = ldcg_f(out + (size_t)m1 * ostride + rb) + acc[3];
-                            __stcg(out + (size_t)m1 * ostride + ra, a);
-                            __stcg(out + (size_t)m1 * ostride + rb, b);
-                            q1 = a * a + b * b;
-                        }
-                        // sum over the eight lanes that share t (the 16 rows of the tile), in a fixed order
-#pragma unroll
-                        for (int o = 4; o < 32; o <<= 1) {
-                            q0 += __shfl_xor_sync(0xffffffffu, q0, o);
-                            q1 += __shfl_xor_sync(0xffffffffu, q1, o);
-                        }
-                        if (g == 0 && ssq) {
-                            const int ntile = nvalid / 16;
-                            if (m0 < S.A.M) __stcg(ssq + (size_t)m0 * ntile + tile, q0);
-                            if (m1 < S.A.M) __stcg(ssq + (size_t)m1 * ntile + tile, q1);
-                        }
-                    } else if (epi == MKS_E_GLU) {
-                        const int r = tile * 8 + g;
-                        const bool gelu = d.i[MKS_I_ACT] == MKS_ACT_GELU_TANH;
-                        if (r < nvalid) {
-                            if (m0 < S.A.M) __stcg(out + (size_t)m0 * ostride + r, (gelu ? gelu_tanh_f(acc[0]) : silu_f(acc[0])) * acc[2]);
-                            if (m1 < S.A.M) __stcg(out + (size_t)m1 * ostride + r, (gelu ? gelu_tanh_f(acc[1]) : silu_f(acc[1])) * acc[3]);
-                        }
-                    } else {   // MKS_E_LOGITS
-                        const float cap = d.f[MKS_F_SOFTCAP];
-                        const int row_base = (int)d.p[MKS_P_ROW_BASE];
-                        const int ra = tile * 16 + g, rb = ra + 8;
-                        float v[4] = {acc[0], acc[1], acc[2], acc[3]};
-                        if (cap > 0.f) {
-#pragma unroll
-                            for (int i = 0; i < 4; i++) v[i] = cap * tanhf(v[i] / cap);
-                        }
-                        if (m0 < S.A.M) {
-                            if (ra < nvalid) { __stcg(out + (size_t)m0 * ostride + ra, v[0]); const u64 k = score_key(v[0], row_base + ra); best.k0 = k > best.k0 ? k : best.k0; }
-                            if (rb < nvalid) { __stcg(out + (size_t)m0 * ostride + rb, v[2]); const u64 k = score_key(v[2], row_base + rb); best.k0 = k > best.k0 ? k : best.k0; }
-                        }
-                        if (m1 < S.A.M) {
-                            if (ra < nvalid) { __stcg(out + (size_t)m1 * ostride + ra, v[1]); const u64 k = score_key(v[1], row_base + ra); best.k1 = k > best.k1 ? k : best.k1; }
-                            if (rb < nvalid) { __stcg(out + (size_t)m1 * ostride + rb, v[3]); const u64 k = score_key(v[3], row_base + rb); best.k1 = k > best.k1 ? k : best.k1; }
-                        }
-                    }
+            for (int u = 0; u < 4; u++) {
+                w[u][0] = w[u][1] = w[u][2] = w[u][3] = (u64)tag << 32;
+                if (p0 + u < P) {
+                    const unsigned long long* q = src + (size_t)(p0 + u) * 128;
+                    if (l0) asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[u][0]), "=l"(w[u][2]) : "l"(q) : "memory");
+                    if (l1) asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[u][1]), "=l"(w[u][3]) : "l"(q + 16) : "memory");
                 }
             }
-            if (warp_() < nj) mu.chunk_n += (uint32_t)gm.n_chunks;
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) ok = ok && (uint32_t)(w[u][i] >> 32) == tag;
+            if (__all_sync(0xffffffffu, ok)) break;
+            if (!ok && MKS_SPIN_FAIL(S, s, WS_TILE)) fail = true;
+            if (__any_sync(0xffffffffu, fail)) return false;
         }
-        pu = pend;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (p0 + u < P)
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[i] += __uint_as_float((uint32_t)w[u][i]);
     }
-    prof_mark(S, 2);
-    if (epi == MKS_E_LOGITS) {
-        // best key of every sequence over this CTA's rows -> keys[m][cta]
-        if (tid_() < 8) S.keys_s[tid_()] = 0;
+    return true;
+}
+
+// Epilogue of a finished tile (`row_tile` counts the tiles of all groups, unless the groups were added up).  False: a wait
+// ran out.
+__device__ __noinline__ bool finish_tile(Shared& S, const mk_stage_desc& d, u64 ar_seq, int row_tile, float4 in) {
+    float acc[4] = {in.x, in.y, in.z, in.w};
+    const int g = lane_() >> 2, t = lane_() & 3, epi = d.i[MKS_I_EPILOGUE];
+    const int T = d.i[MKS_I_TILES];
+    const int grp = row_tile < T ? 0 : row_tile / T, tile = row_tile - grp * T;
+    if (d.i[MKS_I_ALLREDUCE] != 0 && S.A.tp > 1) {
+        const float4 r = allreduce_tile(S, S.A, ar_seq, tile, make_float4(acc[0], acc[1], acc[2], acc[3]));
+        if (__any_sync(0xffffffffu, S.abort_flag != 0)) return false;
+        acc[0] = r.x; acc[1] = r.y; acc[2] = r.z; acc[3] = r.w;
+    }
+    // rows g, g + 8 of the tile x sequences 2t, 2t + 1
+    const int ostride = d.i[MKS_I_OUT_STRIDE], nvalid = d.i[MKS_I_N_VALID];
+    const int row = epi == MKS_E_GLU ? tile * 8 + g : tile * 16 + g;
+    float* out = reinterpret_cast<float*>(d.p[MKS_P_OUT]) + (size_t)grp * d.i[MKS_I_OUT_GSTRIDE] + (size_t)(2 * t) * ostride + row;
+    const bool l0 = 2 * t < S.A.M, l1 = 2 * t + 1 < S.A.M;
+    const bool va = row < nvalid, vb = epi != MKS_E_GLU && row + 8 < nvalid;
+    if (epi == MKS_E_RESID) {
+        if (l0) { acc[0] += ldcg_f(out); acc[2] += ldcg_f(out + 8); }
+        if (l1) { acc[1] += ldcg_f(out + ostride); acc[3] += ldcg_f(out + ostride + 8); }
+    }
+    float* ssq = epi == MKS_E_STORE || epi == MKS_E_RESID ? reinterpret_cast<float*>(d.p[MKS_P_OUT_SSQ]) : nullptr;
+    float a = acc[0], b = acc[2];
+    bool live = l0;
+#pragma unroll 1
+    for (int q = 0; q < 2; q++) {
+        if (epi == MKS_E_GLU) a = (d.i[MKS_I_ACT] == MKS_ACT_GELU_TANH ? gelu_tanh_f(a) : silu_f(a)) * b;
+        if (epi == MKS_E_LOGITS) {
+            const float cap = d.f[MKS_F_SOFTCAP];
+            if (cap > 0.f) {
+                a = cap * tanhf(a / cap);
+                b = cap * tanhf(b / cap);
+            }
+            const int r0 = (int)d.p[MKS_P_ROW_BASE] + row;
+            u64 k = va ? score_key(a, r0) : 0;
+            const u64 k2 = vb ? score_key(b, r0 + 8) : 0;
+            k = k2 > k ? k2 : k;
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                const u64 other = __shfl_xor_sync(0xffffffffu, k, o);
+                k = other > k ? other : k;
+            }
+            if (g == 0 && live) atomicMax(reinterpret_cast<unsigned long long*>(&S.keys_s[2 * t + q]), (unsigned long long)k);
+        }
+        if (live) {
+            if (va) __stcg(out, a);
+            if (vb) __stcg(out + 8, b);
+        }
+        if (ssq) {                                              // the sums of squares a later norm of this vector needs (whole tiles only)
+            float s2 = a * a + b * b;
+            // sum over the eight lanes that share t (the 16 rows of the tile), in a fixed order
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+            if (g == 0 && live) __stcg(ssq + (size_t)(2 * t + q) * (nvalid / 16) + tile, s2);
+        }
+        if (S.A.M == 1) break;
+        a = acc[1]; b = acc[3];
+        live = l1;
+        out += ostride;
+    }
+    return true;
+}
+
+// What happens to a tile's sum over this CTA's panel.  False: a wait ran out.
+__device__ __forceinline__ bool deliver(Shared& S, const mk_stage_desc& d, const Geo& gm, u64 ar_seq, uint32_t tag, int panel, int row_tile, const float (&v)[4]) {
+    if (gm.P == 1) return finish_tile(S, d, ar_seq, row_tile, make_float4(v[0], v[1], v[2], v[3]));
+    publish_tile(tile_words(reinterpret_cast<unsigned long long*>(d.p[MKS_P_PART]), row_tile * gm.P + panel), tag, S.A.M, v);
+    return true;
+}
+
+// A batch of a stage, input staged: this warp's chunks, tile by tile.  The first and the last tile may be shared with the
+// warps before and behind.  One call per batch: a call per tile spilled the caller's registers around each, and spills of
+// 544 threads do not fit the L1 that the shared-memory carve-out leaves.
+template <int FMT>
+__device__ __forceinline__ bool multiply(Shared& S, const mk_stage_desc& d, const Geo& gm, const Batch bt, int b, u64 ar_seq, uint32_t tag, uint32_t n_stage) {
+    constexpr int STEP_BYTES = (FMT == MKS_FMT_MXFP4 ? 4 : (FMT == MKS_FMT_BF16 ? 1 : 2)) * 32;   // staged input bytes of one tile step
+    const int depth = S.A.ring_depth;
+    Feed f = S.cur[warp_()].f;
+    f.rd += lane_() * 16;
+    f.wr += lane_() * 16;
+    const uint32_t ring_end = smem_u32(S.ring()) + (warp_() + 1) * depth * BLOCK_BYTES;
+    __syncwarp();
+    if (lane_() == 0) S.cur[warp_()].now = n_stage;
+    __syncwarp();
+    const int stride = xs_stride_bytes((bt.seg1 - bt.seg0) * d.i[MKS_I_KC]), chunk_steps = gm.chunk_steps, n_chunks = gm.n_chunks;
+    const Share sh = b == 0 ? S.share[n_stage % GEO_RING][warp_()] : batch_share(S, gm, bt, warp_());
+    const bool scales = FMT == MKS_FMT_MXFP4 || (FMT == MKS_FMT_FP8 && gm.ebps != 0);
+    const int cpt = sh.cpt, c1 = sh.c1;
+    int c = sh.c, tl = sh.tl, k = sh.k;
+    bool begun = k == 0, has_head = false, ok = true;
+    float sum[4] = {0.f, 0.f, 0.f, 0.f}, head[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    while (c < c1 && ok) {
+        // consecutive chunks of one tile: one K split's at a time when groups are added up
+        float s0 = 1.f, s1 = 1.f, f0 = 1.f, f1 = 1.f, x0, x1;
+        int ke = cpt;
+        {
+            int sg = 0, grp = 0, tile = bt.t0 + tl;
+            if (gm.reduce) {
+                sg = k / n_chunks;
+                ke = (sg + 1) * n_chunks;
+                grp = (bt.seg0 + sg) / gm.S;
+                f0 = S.coef[grp * 8 + 2 * (lane_() & 3)];
+                f1 = S.coef[grp * 8 + 2 * (lane_() & 3) + 1];
+            } else if (tile >= gm.T) {
+                grp = tile / gm.T;
+                tile -= grp * gm.T;
+            }
+            const float* rs = group_row_scale(S, d, grp, gm.G);
+            if (rs) {
+                s0 = __ldg(rs + tile * 16 + (lane_() >> 2));
+                s1 = __ldg(rs + tile * 16 + (lane_() >> 2) + 8);
+            }
+            x0 = S.xinv[sg * 8 + 2 * (lane_() & 3)];
+            x1 = S.xinv[sg * 8 + 2 * (lane_() & 3) + 1];
+        }
+        const int run = min(ke - k, c1 - c);
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        {
+            float acc2[4] = {0.f, 0.f, 0.f, 0.f};
+            float tot[4] = {0.f, 0.f, 0.f, 0.f};                // block-scaled FP8: the sum over 128-column blocks
+            // lanes beyond the staged columns read a live one (their accumulators are never used): predicated zeros cost a tenth of the loop
+            const uint8_t* xk = S.xs() + min(lane_() >> 2, S.A.M * d.i[MKS_I_PIECES] - 1) * stride + (lane_() & 3) * 8 + k * chunk_steps * STEP_BYTES;
+            // the stream's blocks end where a chunk with scales, or a run of chunks, ends
+            int chunks = run;
+#pragma unroll 1
+            while (chunks > 0 && ok) {
+                const int take = scales ? 1 : chunks;
+                int steps = take * chunk_steps;
+                chunks -= take;
+#pragma unroll 1
+                while (steps > 0) {
+                    __syncwarp();
+                    feed(S, f, depth, ring_end);
+                    if (f.ahead == 0) {                        // (a stream that was refused: the launch has failed)
+                        ok = false;
+                        break;
+                    }
+                    wait_block(depth);
+                    __syncwarp();
+                    const uint32_t sl = f.rd;
+                    if (steps >= BLOCK_STEPS) {
+#pragma unroll
+                        for (int st = 0; st < BLOCK_STEPS; st++, xk += STEP_BYTES) tile_step<FMT>(sl + st * 512, sl + BLOCK_STEPS * 512 + st * 32 - lane_() * 16 + (lane_() >> 2) * 4, st, xk, acc, acc2);
+                    } else {
+#pragma unroll 1
+                        for (int st = 0; st < steps; st++, xk += STEP_BYTES) tile_step<FMT>(sl + st * 512, sl + BLOCK_STEPS * 512 + st * 32 - lane_() * 16 + (lane_() >> 2) * 4, st, xk, acc, acc2);
+                    }
+                    if (FMT == MKS_FMT_FP8 && scales) {
+                        // one scale per 128 k for rows 0-7 of the tile and one for rows 8-15 (a GLU tile pairs two matrices)
+                        const float2 bs = lds_f2(sl + BLOCK_STEPS * 512 - lane_() * 16);
+                        tot[0] = fmaf(acc[0] + acc2[0], bs.x, tot[0]); tot[1] = fmaf(acc[1] + acc2[1], bs.x, tot[1]);
+                        tot[2] = fmaf(acc[2] + acc2[2], bs.y, tot[2]); tot[3] = fmaf(acc[3] + acc2[3], bs.y, tot[3]);
+                        acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+                        acc2[0] = acc2[1] = acc2[2] = acc2[3] = 0.f;
+                    }
+                    steps -= BLOCK_STEPS;
+                    f.ahead--;
+                    f.rd += BLOCK_BYTES;
+                    if (f.rd >= ring_end) f.rd -= depth * BLOCK_BYTES;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i] = acc[i] + acc2[i] + (FMT == MKS_FMT_FP8 ? tot[i] : 0.f);
+        }
+        __syncwarp();
+        // undo the input scaling, fold the second piece's columns onto the first
+        acc[0] *= x0; acc[1] *= x1; acc[2] *= x0; acc[3] *= x1;
+        if (d.i[MKS_I_PIECES] == 2) {
+            // columns [0, M) + columns [M, 2M): lane t holds columns 2t, 2t + 1
+            const int t = lane_() & 3;
+            float add[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int src_col = 2 * t + (i & 1) + S.A.M;              // the partner column
+                const int src = (lane_() & ~3) | ((src_col >> 1) & 3);
+                const float same = __shfl_sync(0xffffffffu, acc[i], src), other = __shfl_sync(0xffffffffu, acc[i ^ 1], src);
+                add[i] = (src_col & 1) == (i & 1) ? same : other;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (2 * t + (i & 1) < S.A.M) acc[i] += add[i];
+        }
+        sum[0] = fmaf(acc[0] * s0, f0, sum[0]); sum[1] = fmaf(acc[1] * s0, f1, sum[1]);
+        sum[2] = fmaf(acc[2] * s1, f0, sum[2]); sum[3] = fmaf(acc[3] * s1, f1, sum[3]);
+        c += run;
+        k += run;
+        if (k == cpt || c == c1) {
+            if (!begun) {
+                // the warp that has the tile's beginning adds this to it
+                has_head = true;
+#pragma unroll
+                for (int i = 0; i < 4; i++) head[i] = sum[i];
+            } else if (k == cpt) {
+                ok = deliver(S, d, gm, ar_seq, tag, bt.panel, bt.t0 + tl, sum) && ok;
+            } else {
+                break;                                             // c == c1, inside a tile that began here: `sum` is its first part
+            }
+            begun = true;
+            sum[0] = sum[1] = sum[2] = sum[3] = 0.f;
+            if (k == cpt) {
+                k = 0;
+                tl++;
+            } else {
+                k = 0;                                             // (the whole range lay inside another warp's tile)
+            }
+        }
+    }
+    __syncwarp();
+    feed(S, f, depth, ring_end);
+    if (lane_() == 0) {
+        f.rd -= lane_() * 16;
+        f.wr -= lane_() * 16;
+        S.cur[warp_()].f = f;
+    }
+    __syncwarp();
+    consumer_sync();                                             // the staging area is free: it takes the shared tiles
+    float4* tiles = reinterpret_cast<float4*>(S.xs()) + lane_();
+    tiles[warp_() * 32] = make_float4(head[0], head[1], head[2], head[3]);         // (zeros if there is none)
+    __syncwarp();
+    consumer_sync();
+    if (k > 0 && c == c1 && c > sh.c && ok) {
+        // the warps behind this one, up to the one that has the tile's last chunk
+        const int last = (16 * ((tl + 1) * cpt - 1) + 15) / sh.n;
+#pragma unroll 4
+        for (int v = warp_() + 1; v <= last; v++) {
+            const float4 x = tiles[v * 32];
+            sum[0] += x.x; sum[1] += x.y; sum[2] += x.z; sum[3] += x.w;
+        }
+        ok = deliver(S, d, gm, ar_seq, tag, bt.panel, bt.t0 + tl, sum);
+    }
+    __syncwarp();
+    return ok;
+}
+
+template <int FMT>
+__device__ __forceinline__ void gemv_stage(Shared& S, const mk_stage_desc& d, const Geo& gm, u64 ar_seq, uint32_t tag, uint32_t n_stage) {
+    const bool logits = d.i[MKS_I_EPILOGUE] == MKS_E_LOGITS;
+    if (logits && tid_() < 8) S.keys_s[tid_()] = 0;
+    bool ok = true;                                              // no wait of this warp ran out
+#pragma unroll 1
+    for (int b = 0; b < gm.nb; b++) {
+        const Batch bt = geo_batch(gm, b);
+        __syncwarp();
+        if (b) consumer_sync();                                  // everybody is done with the staging area
+        if (d.i[MKS_I_PIECES] == 1 && !gm.reduce) stage_x<true>(S, d, bt.seg0, bt.seg1, bt.grp, gm.S);
+        else stage_x<false>(S, d, bt.seg0, bt.seg1, bt.grp, gm.S);
+        __syncwarp();
         consumer_sync();
-        if (best.k0) atomicMax(reinterpret_cast<unsigned long long*>(&S.keys_s[2 * t]), best.k0);
-        if (best.k1) atomicMax(reinterpret_cast<unsigned long long*>(&S.keys_s[2 * t + 1]), best.k1);
+        if (b == 0) prof_mark(S, 1);
+        const bool good = multiply<FMT>(S, d, gm, bt, b, ar_seq, tag, n_stage);
+        ok = ok && good;
+    }
+    if (gm.P > 1 && gm.nb > 0) {
+        // every partial tile of this CTA is on its way; now the sums it is responsible for: each P-th tile of its range
+        const int step = gm.panel >= 0 ? gm.P : 1;
+        const int first = gm.panel >= 0 ? gm.t0 + ((gm.panel - gm.t0) % gm.P + gm.P) % gm.P : gm.t0;
+#pragma unroll 1
+        for (int tl = first + warp_() * step; tl < gm.t1 && ok; tl += NCW * step) {
+            float sum[4];
+            ok = collect_tile(S, tile_words(reinterpret_cast<unsigned long long*>(d.p[MKS_P_PART]), tl * gm.P), tag, gm.P, sum) &&
+                 finish_tile(S, d, ar_seq, tl, make_float4(sum[0], sum[1], sum[2], sum[3]));
+        }
+    }
+    __syncwarp();
+    prof_mark(S, 2);
+    if (logits) {
+        // best key of every sequence over this CTA's rows -> keys[m][cta]
+        __syncwarp();
         consumer_sync();
         u64* keys = reinterpret_cast<u64*>(d.p[MKS_P_KEYS]);
         if (tid_() < S.A.M) __stcg(reinterpret_cast<unsigned long long*>(keys + (size_t)tid_() * grid_() + cta_()), (unsigned long long)S.keys_s[tid_()]);

@@ -99,8 +99,18 @@ static int64_t scratch_bytes(const mk_stage_desc* prog, int n_stages, int batch)
         const mk_stage_desc& d = prog[s];
         int64_t b = 0;
         if (d.op == MKS_OP_GEMV) {
-            const int stride = ((d.i[MKS_I_KC] * 2 + 127) / 128) * 128 + 32;
-            b = (int64_t)stride * batch * d.i[MKS_I_PIECES];
+            // the panel width the kernel prefers on a whole B200; what it gets here bounds what it takes
+            const bool reduce = d.i[MKS_I_REDUCE_GROUPS] != 0;
+            const int G = d.i[MKS_I_GROUPS] > 0 ? d.i[MKS_I_GROUPS] : MAX_GROUPS, kc = d.i[MKS_I_KC], ncols = batch * d.i[MKS_I_PIECES];
+            const int R = reduce ? d.i[MKS_I_TILES] : d.i[MKS_I_TILES] * G, Q = reduce ? d.i[MKS_I_SPLITS] * G : d.i[MKS_I_SPLITS];
+            const int w = max_panel_splits(XS_BYTES, kc, ncols, d.i[MKS_I_PIECES], reduce), P0 = (Q + w - 1) / w;
+            int P = P0;
+            uint64_t best = ~0ull;
+            for (int p = P0; p <= Q && p <= 148 / 2; p++) {
+                const uint64_t k = panel_cost(R, Q, p, d.i[MKS_I_UNIT_STEPS] / d.i[MKS_I_CHUNK_STEPS], d.i[MKS_I_CHUNK_BYTES], kc, batch, 148);
+                if (k < best) { best = k; P = p; }
+            }
+            b = (int64_t)xs_stride_bytes((Q + P - 1) / P * kc) * ncols;
         } else if (d.op == MKS_OP_ATTN) {
             const int QPK = d.i[MKS_I_NQ] / d.i[MKS_I_NKV], HD = d.i[MKS_I_HD], CP = d.i[MKS_I_CHUNK_POS];
             b = (int64_t)(QPK * HD + 2 * HD + QPK * CP + QPK * ATTN_MAX_CHUNKS + 2 * QPK + CP + 4) * 4;
@@ -183,15 +193,16 @@ extern "C" int mk_stage_launch(const mk_stage_args* a, void* stream) {
     A.row_valid = reinterpret_cast<const int*>(a->row_valid);
     A.prof_cta = a->prof_cta;
     // shared memory: the staging area the program needs (the caller computes it with mk_stage_scratch_bytes), the rest ring slots
-    const int xs = a->xs_bytes > 0 ? (a->xs_bytes + 127) / 128 * 128 : XS_BYTES;
+    int xs = a->xs_bytes > 0 ? (a->xs_bytes + 127) / 128 * 128 : XS_BYTES;
+    xs = xs < TILE_BYTES ? TILE_BYTES : xs;
     if (xs > XS_BYTES) return sfail(MK_ERR_BADARG, "mk_stage_launch: staging area of %d bytes exceeds %d", xs, XS_BYTES);
-    int depth = (SMEM_TOTAL - MISC_BYTES - xs) / (16 * mks::SLOT_BYTES);
+    int depth = (SMEM_TOTAL - MISC_BYTES - xs) / (16 * BLOCK_BYTES);
     depth = depth > MAX_RING_DEPTH ? MAX_RING_DEPTH : depth;
-    if (depth < 2) return sfail(MK_ERR_BADARG, "mk_stage_launch: no room for two ring slots per warp");
+    if (depth < MIN_RING_DEPTH) return sfail(MK_ERR_BADARG, "mk_stage_launch: no room for %d ring slots per warp", MIN_RING_DEPTH);
     A.xs_bytes = xs;
     A.ring_depth = depth;
 
-    const int smem = MISC_BYTES + xs + 16 * depth * mks::SLOT_BYTES;
+    const int smem = MISC_BYTES + xs + 16 * depth * BLOCK_BYTES;
     MKS_CUDA(cudaFuncSetAttribute(stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     void* kargs[] = {&A};
     MKS_CUDA(cudaLaunchCooperativeKernel((const void*)stage_kernel, dim3(grid), dim3(mks::NTHREADS), kargs, smem, static_cast<cudaStream_t>(stream)));

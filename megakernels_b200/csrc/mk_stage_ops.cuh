@@ -11,7 +11,7 @@ constexpr size_t MAILBOX_KEY_WORDS = (size_t)2 * MAILBOX_TILES * MKS_MAX_RANKS *
 // Every sequence's arg-max over the keys the LM head's CTAs left in `keys` ([M][grid]); with tensor
 // parallelism each rank's CTA 0 pushes its best key into every rank's mailbox and every CTA takes the
 // maximum over ranks (a key carries the vocabulary row, so equal scores go to the lowest id on every rank).
-__device__ void choose_tokens(Shared& S, Mut& mu, const Args& A, const u64* keys, uint32_t tag, int vocab) {
+__device__ void choose_tokens(Shared& S, const Args& A, const u64* keys, uint32_t tag, int vocab) {
     if (warp_() < S.A.M) {
         const int m = warp_();
         u64 key = 0;
@@ -38,10 +38,7 @@ __device__ void choose_tokens(Shared& S, Mut& mu, const Args& A, const u64* keys
                 const bool ok = (uint32_t)(hi >> 32) == tag && (uint32_t)(lo >> 32) == tag;
                 if (__all_sync(0xffffffffu, ok)) break;
                 if (!ok && MKS_SPIN_FAIL(S, s, WS_KEYS)) fail = true;
-                if (__any_sync(0xffffffffu, fail)) {
-                    mu.dead = true;
-                    break;
-                }
+                if (__any_sync(0xffffffffu, fail)) break;          // (the abort flag is set)
             }
             key = warp_max_u64(((hi & 0xffffffffull) << 32) | (lo & 0xffffffffull));
         }
@@ -50,10 +47,10 @@ __device__ void choose_tokens(Shared& S, Mut& mu, const Args& A, const u64* keys
 }
 
 // ---- embedding ---------------------------------------------------------------------------------------------------
-__device__ __noinline__ void embed_stage(Shared& S, Mut& mu, const mk_stage_desc& d, const Args& A, int step, uint32_t tag) {
+__device__ __noinline__ void embed_stage(Shared& S, const mk_stage_desc& d, const Args& A, int step, uint32_t tag) {
     const int H = d.i[MKS_I_HIDDEN], vocab = d.i[MKS_I_VOCAB];
     if (step > 0 && d.i[MKS_I_KEYS_VALID] && d.p[MKS_P_E_KEYS]) {
-        choose_tokens(S, mu, A, reinterpret_cast<const u64*>(d.p[MKS_P_E_KEYS]), tag, vocab);
+        choose_tokens(S, A, reinterpret_cast<const u64*>(d.p[MKS_P_E_KEYS]), tag, vocab);
         consumer_sync();
         if (cta_() == 0 && tid_() < S.A.M) {
             A.tok[tid_()] = S.tok_s[tid_()];
@@ -104,7 +101,7 @@ __device__ __noinline__ void embed_stage(Shared& S, Mut& mu, const mk_stage_desc
 // ([v][k], fp32): decay, delta-rule update and output row by row, then the head's gated RMSNorm.
 // The conv history is a ring of four inputs per channel indexed by position & 3: this step's input
 // goes to one slot while the other three are read, so tasks that share q/k channels never collide.
-__device__ __noinline__ void gdn_stage(Shared& S, Mut& mu, const mk_stage_desc& d) {
+__device__ __noinline__ void gdn_stage(Shared& S, const mk_stage_desc& d) {
     const int nkh = d.i[MKS_I_NKH], nvh = d.i[MKS_I_NVH], rep = nvh / nkh;
     const int key_dim = nkh * 128, conv_dim = d.i[MKS_I_CONV_DIM];
     const int q_off = d.i[MKS_I_Q_OFF], k_off = d.i[MKS_I_K_OFF], v_off = d.i[MKS_I_V_OFF], z_off = d.i[MKS_I_Z_OFF];
@@ -226,7 +223,7 @@ __device__ __forceinline__ void load8(const void* row, int elem, float (&v)[8]) 
 
 // RMS-norm (optional), rotate and round one head vector; one warp.  `dst` receives HD <= 512 floats.  All of a
 // lane's loads are requested before the first is used (one L2 round trip for the vector, one for the weights).
-__device__ __noinline__ void head_prepare(Shared& S, Mut& mu, const float* src, float* dst, int HD, const float* nw, float norm_off, bool do_norm,
+__device__ __noinline__ void head_prepare(Shared& S, const float* src, float* dst, int HD, const float* nw, float norm_off, bool do_norm,
                                           float eps, const float* cs, const float* sn, int pairs, int pair_dist, bool round_bf16) {
     float v[16], w[16];
 #pragma unroll
@@ -272,7 +269,7 @@ __device__ __noinline__ void head_prepare(Shared& S, Mut& mu, const float* src, 
 constexpr int ATTN_MAX_CHUNKS = 256;      // split records per (sequence, kv head)
 
 template <bool KVF32>
-__device__ __noinline__ void attn_stage(Shared& S, Mut& mu, const mk_stage_desc& d) {
+__device__ __noinline__ void attn_stage(Shared& S, const mk_stage_desc& d) {
     const int NQ = d.i[MKS_I_NQ], NKV = d.i[MKS_I_NKV], HD = d.i[MKS_I_HD], ROT = d.i[MKS_I_ROT];
     const int QPK = NQ / NKV, CP = d.i[MKS_I_CHUNK_POS], window = d.i[MKS_I_WINDOW], maxpages = d.i[MKS_I_MAX_PAGES];
     const int kvb = d.i[MKS_I_KV_BLOCK] > 0 ? d.i[MKS_I_KV_BLOCK] : 64, kvb_shift = 31 - __clz(kvb);
@@ -337,12 +334,12 @@ __device__ __noinline__ void attn_stage(Shared& S, Mut& mu, const mk_stage_desc&
         // 1. queries (warps 0..QPK-1), new K (warp QPK), new V (warp QPK + 1), cache row offsets (the other warps)
         if (warp_() < QPK) {
             const int hq = kvh * QPK + warp_();
-            head_prepare(S, mu, y + q_off + (size_t)hq * q_hs, q_s + warp_() * HD, HD, qn, norm_off, true, eps, cs, sn, pairs, pair_dist, q_bf16);
+            head_prepare(S, y + q_off + (size_t)hq * q_hs, q_s + warp_() * HD, HD, qn, norm_off, true, eps, cs, sn, pairs, pair_dist, q_bf16);
         } else if (has_new && warp_() == QPK) {
-            head_prepare(S, mu, y + k_off + (size_t)kvh * HD, kn_s, HD, kn, norm_off, true, eps, cs, sn, pairs, pair_dist, !KVF32);
+            head_prepare(S, y + k_off + (size_t)kvh * HD, kn_s, HD, kn, norm_off, true, eps, cs, sn, pairs, pair_dist, !KVF32);
         } else if (has_new && warp_() == QPK + 1) {
             const float* vsrc = v_off >= 0 ? y + v_off + (size_t)kvh * HD : y + k_off + (size_t)kvh * HD;
-            head_prepare(S, mu, vsrc, vn_s, HD, nullptr, 0.f, d.i[MKS_I_V_NORM] != 0, eps, nullptr, nullptr, 0, 0, !KVF32);
+            head_prepare(S, vsrc, vn_s, HD, nullptr, 0.f, d.i[MKS_I_V_NORM] != 0, eps, nullptr, nullptr, 0, 0, !KVF32);
         } else if (warp_() >= QPK + 2) {
 #pragma unroll 1
             for (int i = tid_() - (QPK + 2) * 32; i < np; i += NCT - (QPK + 2) * 32) {
@@ -589,7 +586,7 @@ __device__ __noinline__ void attn_stage(Shared& S, Mut& mu, const mk_stage_desc&
 // Every CTA builds the same tables from the router logits: per sequence the top-k experts (ties to the
 // lower id) and their weights, the list of distinct experts in ascending id (the groups of the routed
 // GEMV stages) and coef[group][sequence], the weight with which a group's product enters a sequence.
-__device__ __noinline__ void route_stage(Shared& S, Mut& mu, const mk_stage_desc& d) {
+__device__ __noinline__ void route_stage(Shared& S, const mk_stage_desc& d) {
     const int E = d.i[MKS_I_EXPERTS], topk = d.i[MKS_I_TOPK], stride = d.i[MKS_I_LOGIT_STRIDE], kind = d.i[MKS_I_ROUTE_KIND];
     const float* logits = reinterpret_cast<const float*>(d.p[MKS_P_LOGITS]);
     const float* pes = reinterpret_cast<const float*>(d.p[MKS_P_EXPERT_SCALE]);
@@ -670,7 +667,7 @@ __device__ __noinline__ void route_stage(Shared& S, Mut& mu, const mk_stage_desc
 // out[m][i] = (base[m][i] + a[m][i] rstd_a[m] (off + w_a[i]) [+ b[m][i] rstd_b[m] (off + w_b[i])]) * scale, and the sums
 // of squares of the result per 16 elements.  rstd comes from the 16-element sums of squares the producing GEMV stage
 // left (every CTA adds them up itself, in a fixed order); a CTA then takes a slice of the 16-element groups.
-__device__ __noinline__ void vec_stage(Shared& S, Mut& mu, const mk_stage_desc& d) {
+__device__ __noinline__ void vec_stage(Shared& S, const mk_stage_desc& d) {
     const int N = d.i[MKS_I_VEC_N], ng = N / 16, M = S.A.M;
     if (N == 0) return;                                        // an empty stage: its barrier only
     const float* base = reinterpret_cast<const float*>(d.p[MKS_P_VEC_BASE]);
@@ -737,8 +734,6 @@ __device__ __noinline__ void vec_stage(Shared& S, Mut& mu, const mk_stage_desc& 
 __global__ void __launch_bounds__(NTHREADS, 1) stage_kernel(const __grid_constant__ Args A_in) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     Shared& S = *reinterpret_cast<Shared*>(smem_raw);
-    Mut mu;
-    mu.chunk_n = 0; mu.dead = false;
     {
         // the launch arguments, once, into shared memory
         constexpr int ARG_WORDS = (int)(sizeof(Args) / 4);
@@ -748,52 +743,58 @@ __global__ void __launch_bounds__(NTHREADS, 1) stage_kernel(const __grid_constan
     }
     if (tid_() == 0) S.prof = nullptr;
     if (tid_() == 0) {
-#pragma unroll 1
-        for (int i = 0; i < NS; i++) {
-            mbar_init(&S.full[i], 1);
-            mbar_init(&S.empty[i], 1);
-        }
         S.abort_flag = 0;
         S.route_seq = 0;
         S.n_groups = 0;
-        S.pf_pos = 0;
-        fence_barrier_init();
-        fence_proxy_async();
+        S.described = 0;
+        S.completed = 0;
+        S.tag0 = (uint32_t)(A_in.bar_base / grid_());
     }
     if (tid_() < 8) {
-        S.xinv[tid_()] = 1.f;
         S.rstd[tid_()] = 1.f;
         S.tok_s[tid_()] = 0;
         S.pos_s[tid_()] = tid_() < A_in.M ? A_in.pos[tid_()] : 0;
         S.valid_s[tid_()] = tid_() < A_in.M && (!A_in.row_valid || A_in.row_valid[tid_()] != 0);
     }
+    if (warp_() < NCW && lane_() == 0) {
+        Cur& c = S.cur[warp_()];
+        c.src = nullptr; c.left = c.rest = c.run = c.ebps = 0; c.gn = c.now = 0; c.b = 0; c.nb = 0;
+c.f.src = nullptr; c.f.steps = c.f.left = c.f.eoff = c.f.ebps = c.f.cs = c.f.ahead = 0;
+        c.f.rd = c.f.wr = smem_u32(smem_raw + MISC_BYTES + A_in.xs_bytes) + warp_() * A_in.ring_depth * BLOCK_BYTES;
+    }
     __syncthreads();
     const Args& A = S.A;
 
     if (warp_() == NCW) {
-        producer_main(S, A);
+        scout_main(S, A);
         return;
     }
-    // stage records travel through shared memory: the next one is requested while the current stage runs
-    constexpr int DESC_WORDS = (int)(sizeof(mk_stage_desc) / 4);
-    if (tid_() < DESC_WORDS) reinterpret_cast<uint32_t*>(&S.desc[0])[tid_()] = __ldg(reinterpret_cast<const uint32_t*>(&A.prog[0]) + tid_());
-    int cur = 0;
-
     u64 bar_n = 0, ar_seq = A.ar_base;
+    uint32_t n = 0;                                               // stages completed
     bool failed = false;
 #pragma unroll 1
     for (int step = 0; step < A.n_steps && !failed; step++) {
         if (tid_() < S.A.M) S.pos_s[tid_()] = A.pos[tid_()] + (S.valid_s[tid_()] ? step : 0);
-        consumer_sync();
 #pragma unroll 1
-        for (int si = 0; si < A.n_stages; si++) {
-            if (consumer_any(mu.dead || S.abort_flag != 0)) {
+        for (int si = 0; si < A.n_stages; si++, n++) {
+            // the scout has described this stage (normally long ago)
+            bool dead = false;
+            {
+                Spin2 sp;
+#pragma unroll 1
+                while (!__all_sync(0xffffffffu, S.described != n)) {       // (the warp leaves together: barriers follow)
+                    if (MKS_SPIN_FAIL(S, sp, WS_SCOUT)) dead = true;
+                    if (__any_sync(0xffffffffu, dead)) break;
+                }
+                __threadfence_block();
+                __syncwarp();
+            }
+            if (consumer_any(dead || S.abort_flag != 0)) {
                 failed = true;
                 break;
             }
-            const mk_stage_desc& d = S.desc[cur];
-            uint32_t next_word = 0;
-            if (tid_() < DESC_WORDS) next_word = __ldg(reinterpret_cast<const uint32_t*>(&A.prog[si + 1 < A.n_stages ? si + 1 : 0]) + tid_());
+            if (tid_() == 0) S.completed = n;                     // (every warp has left the stages before)
+            const mk_stage_desc& d = S.desc[n % GEO_RING];
             if (tid_() == 0) {
                 // prof_cta >= 0: that CTA's rows [stage][8]; prof_cta < 0: every CTA's rows [cta][stage][8]
                 if (A.prof && step == A.n_steps - 1 && (A.prof_cta < 0 || cta_() == A.prof_cta))
@@ -803,30 +804,36 @@ __global__ void __launch_bounds__(NTHREADS, 1) stage_kernel(const __grid_constan
             }
             prof_mark(S, 0);
             switch (d.op) {
-                case MKS_OP_EMBED: embed_stage(S, mu, d, A, step, (uint32_t)(A.bar_base / grid_() + bar_n) + 1u); break;
-                case MKS_OP_GEMV: gemv_stage(S, mu, d, A, ar_seq); break;
-                case MKS_OP_GDN: gdn_stage(S, mu, d); break;
-                case MKS_OP_ATTN:
-                    if (d.i[MKS_I_KV_F32]) attn_stage<true>(S, mu, d);
-                    else attn_stage<false>(S, mu, d);
+                case MKS_OP_EMBED: embed_stage(S, d, A, step, S.tag0 + (uint32_t)bar_n + 1u); break;
+                case MKS_OP_GEMV:
+                    if (d.i[MKS_I_ALLREDUCE] != 0 && A.tp > 1) ar_seq++;
+                    switch (d.i[MKS_I_FMT]) {
+                        case MKS_FMT_MXFP4: gemv_stage<MKS_FMT_MXFP4>(S, d, S.geo[n % GEO_RING], ar_seq, S.tag0 + (uint32_t)bar_n + 1u, n); break;
+                        case MKS_FMT_FP8: gemv_stage<MKS_FMT_FP8>(S, d, S.geo[n % GEO_RING], ar_seq, S.tag0 + (uint32_t)bar_n + 1u, n); break;
+                        case MKS_FMT_INT8: gemv_stage<MKS_FMT_INT8>(S, d, S.geo[n % GEO_RING], ar_seq, S.tag0 + (uint32_t)bar_n + 1u, n); break;
+                        default: gemv_stage<MKS_FMT_BF16>(S, d, S.geo[n % GEO_RING], ar_seq, S.tag0 + (uint32_t)bar_n + 1u, n); break;
+                    }
                     break;
-                case MKS_OP_ROUTE: route_stage(S, mu, d); break;
-                case MKS_OP_VEC: vec_stage(S, mu, d); break;
+                case MKS_OP_GDN: gdn_stage(S, d); break;
+                case MKS_OP_ATTN:
+                    if (d.i[MKS_I_KV_F32]) attn_stage<true>(S, d);
+                    else attn_stage<false>(S, d);
+                    break;
+                case MKS_OP_ROUTE: route_stage(S, d); break;
+                case MKS_OP_VEC: vec_stage(S, d); break;
                 default: break;
             }
             if (d.op != MKS_OP_GEMV) prof_mark(S, 2);
-            const bool barrier = !(d.flags & MKS_FLAG_NO_BARRIER);
-            if (tid_() < DESC_WORDS) reinterpret_cast<uint32_t*>(&S.desc[cur ^ 1])[tid_()] = next_word;
-            if (barrier) grid_barrier(S, mu, A, bar_n);
-            else consumer_sync();
-            cur ^= 1;
+            if (!(d.flags & MKS_FLAG_NO_BARRIER)) grid_barrier(S, A, bar_n);
             prof_mark(S, 3);
         }
     }
+    consumer_sync();
+    cp_async_wait_all();                                          // copies still under way write shared memory
     // the choice after the last step, and the positions (the program's first stage names the key buffer)
     const mk_stage_desc& d0 = A.prog[0];
     if (!failed && d0.op == MKS_OP_EMBED && d0.i[MKS_I_KEYS_VALID] && d0.p[MKS_P_E_KEYS]) {
-        choose_tokens(S, mu, A, reinterpret_cast<const u64*>(d0.p[MKS_P_E_KEYS]), (uint32_t)(A.bar_base / grid_() + bar_n) + 1u, d0.i[MKS_I_VOCAB]);
+        choose_tokens(S, A, reinterpret_cast<const u64*>(d0.p[MKS_P_E_KEYS]), S.tag0 + (uint32_t)bar_n + 1u, d0.i[MKS_I_VOCAB]);
         consumer_sync();
         if (cta_() == 0 && tid_() < S.A.M) {
             A.tok[tid_()] = S.tok_s[tid_()];

@@ -1,7 +1,7 @@
 """Tile layouts of the stage-machine megakernel's weight stream.
 
-A GEMV matrix [N, K] is cut into units: (K split s, 16-row tile t), stored unit after unit in the order
-(s, t).  A unit is a sequence of *tile steps* of 512 bytes: the bytes lane 0..31 of the consuming warp
+A GEMV matrix [N, K] is cut into units: (16-row tile t, K split s), stored unit after unit in the order
+(t, s), so that a whole tile is one run of bytes.  A unit is a sequence of *tile steps* of 512 bytes: the bytes lane 0..31 of the consuming warp
 load with one 128-bit read each.  Lane (g = lane // 4, q = lane % 4) holds 8 bytes of tile row g and
 8 bytes of tile row g + 8: the operands of the step's MMAs for input columns
 k0 + 16 j + 4 q + {0, 1, 2, 3}, j = 0 .. (64, 32 or 16 columns per step) / 16 - 1.  Steps are grouped
@@ -132,7 +132,7 @@ def pack_matrix(fmt, splits, w, scales=None, block_scales=None, row_order=None):
     used = sum(p.shape[-1] for p in parts)
     if used < cb:
         parts.append(torch.zeros(splits, T, nch, cb - used, dtype=torch.uint8, device=dev))
-    out = torch.cat(parts, dim=-1).reshape(-1)
+    out = torch.cat(parts, dim=-1).transpose(0, 1).reshape(-1)
     meta = dict(fmt=fmt, tiles=T, splits=splits, unit_steps=unit_steps, chunk_steps=cs, chunk_bytes=cb, kc=kc, rows=N,
                 block_scaled=block_scaled, bytes=out.numel())
     return out, meta
@@ -143,7 +143,7 @@ def unpack_matrix(packed, meta, K):
     returns (values fp32 [T*16, K] as the MMAs see them *before* scaling, scale bytes or floats)."""
     fmt, T, S, us, cs, cb = meta["fmt"], meta["tiles"], meta["splits"], meta["unit_steps"], meta["chunk_steps"], meta["chunk_bytes"]
     nch = us // cs
-    p = packed.reshape(S, T, nch, cb).cpu()
+    p = packed.reshape(T, S, nch, cb).cpu()
     out = torch.zeros(T * 16, K)
     step_k = STEP_K[fmt]
     kc = meta["kc"]
@@ -151,7 +151,7 @@ def unpack_matrix(packed, meta, K):
     for s in range(S):
         for t in range(T):
             for ch in range(nch):
-                blob = p[s, t, ch]
+                blob = p[t, s, ch]
                 for st in range(cs):
                     k0 = s * kc + (ch * cs + st) * step_k
                     for lane in range(32):

@@ -77,7 +77,7 @@ class Program:
         if arrivals > 1:
             ncnt = T if reduce_groups else gmax * T
             cnt = self.region(name + ".cnt", ncnt, torch.int32)
-            part = self.region(name + ".part", ncnt * arrivals * 128, torch.float32)
+            part = self.region(name + ".part", ncnt * arrivals * 256, torch.float32)
         ptr = lambda t: t.data_ptr() if t is not None else 0
         i = dict(FMT=meta["fmt"], TILES=T, SPLITS=S, GROUPS=groups, UNIT_STEPS=meta["unit_steps"], CHUNK_STEPS=meta["chunk_steps"],
                  CHUNK_BYTES=meta["chunk_bytes"], KC=meta["kc"], PROLOGUE=prologue, EPILOGUE=epilogue,
@@ -169,6 +169,8 @@ class Runtime:
         self.bar, self.status = z(1, torch.int64), z(4, torch.int32)
         self.bar_base = 0
         self.ar_base = 0
+        for t in program.shared.values():          # partial tiles carry tags that count from bar_base
+            t.zero_()
         self.tp, self.rank, self.mailbox = tp, rank, mailbox
         self.spin_limit_ns = int(spin_limit_ms * 1e6)
         self.launches = 0
