@@ -114,6 +114,7 @@ static int64_t scratch_bytes(const mk_stage_desc* prog, int n_stages, int batch)
         } else if (d.op == MKS_OP_ATTN) {
             const int QPK = d.i[MKS_I_NQ] / d.i[MKS_I_NKV], HD = d.i[MKS_I_HD], CP = d.i[MKS_I_CHUNK_POS];
             b = (int64_t)(QPK * HD + 2 * HD + QPK * CP + QPK * ATTN_MAX_CHUNKS + 2 * QPK + CP + 4) * 4;
+            if (!d.i[MKS_I_KV_F32] && d.i[MKS_I_Q_BF16]) b = attn_mma_bytes(QPK, HD);
         }
         need = b > need ? b : need;
     }

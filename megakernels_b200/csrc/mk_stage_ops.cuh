@@ -268,6 +268,77 @@ __device__ __noinline__ void head_prepare(Shared& S, const float* src, float* ds
 // memory, and the merge first turns the chunks' (max, sum) pairs into weights in shared memory.
 constexpr int ATTN_MAX_CHUNKS = 256;      // split records per (sequence, kv head)
 
+// A chunk's record is written: the last chunk of the (sequence, KV head) to arrive merges all of them, applies the output
+// gate and writes the mixer output.  wn_s: [QPK][ATTN_MAX_CHUNKS] floats of shared scratch.
+__device__ __noinline__ void attn_merge(Shared& S, const mk_stage_desc& d, int m, int kvh, int nch, const float* y, float* wn_s) {
+    const int NKV = d.i[MKS_I_NKV], HD = d.i[MKS_I_HD], QPK = d.i[MKS_I_NQ] / NKV;
+    const int q_off = d.i[MKS_I_A_Q_OFF], q_hs = d.i[MKS_I_A_Q_HSTRIDE], gate_off = d.i[MKS_I_A_GATE_OFF];
+    const int rec = (QPK * (HD + 2) + 3) & ~3, max_chunks = d.i[MKS_I_MAX_CHUNKS];
+    float* part = reinterpret_cast<float*>(d.p[MKS_P_A_PART]);
+    float* Y2 = reinterpret_cast<float*>(d.p[MKS_P_A_Y2]);
+    unsigned* cnt = reinterpret_cast<unsigned*>(d.p[MKS_P_A_CNT]);
+    fence_acq_rel_gpu();
+    consumer_sync();
+    prof_mark(S, 6);
+    if (tid_() == 0) {
+        chaos_delay();
+        const unsigned old = atomicAdd(cnt + m * NKV + kvh, 1u);
+        const int is_last = (int)(old + 1u == (unsigned)nch);
+        if (is_last) {
+            cnt[m * NKV + kvh] = 0u;
+            fence_acq_rel_gpu();
+        }
+        S.flag = is_last;
+    }
+    consumer_sync();
+    if (S.flag) {
+        const float* pbase = part + ((size_t)(m * NKV + kvh) * max_chunks) * rec;
+        // weights of the chunks: w[hq][j] = exp(max_j - max) / sum_j' exp(max_j' - max) l_j'
+#pragma unroll 1
+        for (int i = tid_(); i < QPK * nch; i += NCT) {
+            const int hq = i / nch, j = i - hq * nch;
+            wn_s[hq * ATTN_MAX_CHUNKS + j] = ldcg_f(pbase + (size_t)j * rec + QPK * HD + 2 * hq);
+        }
+        consumer_sync();
+        if (warp_() < QPK) {
+            float* w = wn_s + warp_() * ATTN_MAX_CHUNKS;
+            float mx = -3.0e38f;
+#pragma unroll 1
+            for (int j = lane_(); j < nch; j += 32) mx = fmaxf(mx, w[j]);
+            mx = warp_max(mx);
+            float den = 0.f;
+#pragma unroll 1
+            for (int j = lane_(); j < nch; j += 32) {
+                const float ex = __expf(w[j] - mx);
+                w[j] = ex;
+                den += ex * ldcg_f(pbase + (size_t)j * rec + QPK * HD + 2 * warp_() + 1);
+            }
+            den = warp_sum(den);
+            __syncwarp();
+#pragma unroll 1
+            for (int j = lane_(); j < nch; j += 32) w[j] = w[j] / den;
+        }
+        consumer_sync();
+#pragma unroll 1
+        for (int idx = tid_(); idx < QPK * (HD / 4); idx += NCT) {
+            const int hq = idx / (HD / 4), dd = (idx - hq * (HD / 4)) * 4;
+            const float* w = wn_s + hq * ATTN_MAX_CHUNKS;
+            float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+#pragma unroll 8
+            for (int j = 0; j < nch; j++) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(pbase + (size_t)j * rec + hq * HD + dd));
+                o0 = fmaf(w[j], v.x, o0); o1 = fmaf(w[j], v.y, o1); o2 = fmaf(w[j], v.z, o2); o3 = fmaf(w[j], v.w, o3);
+            }
+            const int hfull = kvh * QPK + hq;
+            if (gate_off >= 0) {
+                const float4 g = __ldcg(reinterpret_cast<const float4*>(y + q_off + (size_t)hfull * q_hs + gate_off + dd));
+                o0 *= sigmoid_f(g.x); o1 *= sigmoid_f(g.y); o2 *= sigmoid_f(g.z); o3 *= sigmoid_f(g.w);
+            }
+            __stcg(reinterpret_cast<float4*>(Y2 + (size_t)m * d.i[MKS_I_A_Y2_STRIDE] + (size_t)hfull * HD + dd), make_float4(o0, o1, o2, o3));
+        }
+    }
+}
+
 template <bool KVF32>
 __device__ __noinline__ void attn_stage(Shared& S, const mk_stage_desc& d) {
     const int NQ = d.i[MKS_I_NQ], NKV = d.i[MKS_I_NKV], HD = d.i[MKS_I_HD], ROT = d.i[MKS_I_ROT];
@@ -517,67 +588,281 @@ __device__ __noinline__ void attn_stage(Shared& S, const mk_stage_desc& d) {
             }
         }
         if (tid_() < 2 * QPK) __stcg(prec + QPK * HD + tid_(), stat_s[tid_()]);
-        // 5. arrival; the last chunk merges
-        fence_acq_rel_gpu();
+        attn_merge(S, d, m, kvh, nch, y, wn_s);
         consumer_sync();
-        prof_mark(S, 6);
-        if (tid_() == 0) {
-            chaos_delay();
-            const unsigned old = atomicAdd(cnt + m * NKV + kvh, 1u);
-            const int is_last = (int)(old + 1u == (unsigned)nch);
-            if (is_last) {
-                cnt[m * NKV + kvh] = 0u;
-                fence_acq_rel_gpu();
+    }
+}
+
+// bf16 caches and bf16 queries (every model's default): the same task on the tensor cores.  What bounded it: a task of 220
+// positions spent 65 us on fp32 FMAs with one shared-memory read per eight of them, three CTA barriers and two trips through
+// global scratch, and a chunk size fixed for the longest context left some CTAs a second task.  Here
+//   * the chunks of a (sequence, KV head) are as many as give every CTA one task at the present lengths;
+//   * a warp scores a tile of 16 positions: A = 16 rows of K straight from global memory (the dot product may take the dims in
+//     any order, so a lane's 16-byte loads are its fragments), B = the query heads;
+//   * a warp then owns 64 dims of the output and every nres-th tile: A = the heads' probabilities (rows 0-7 their first bf16
+//     piece, rows 8-15 the second; the third in an MMA of its own: fp32-exact), B = V, again from global memory with the dims
+//     of a lane's 16 bytes spread over eight MMAs; pairs of positions are put together with byte permutes;
+//   * 256 positions at a time with a running maximum; one CTA barrier per 256.
+constexpr int ATTN_SUB = 256;             // positions between two barriers: one tile per warp
+__host__ __device__ __forceinline__ int attn_mma_bytes(int QPK, int HD) {
+    // q fp32 [QPK][HD] | new K, V rows | q bf16 [8][HD + 8] | scores [2][8][ATTN_SUB + 4] | tile maxima [2][8][16] | rows [2][ATTN_SUB]
+    const int a = QPK * HD * 4 + 2 * HD * 4 + 8 * (HD + 8) * 2 + 2 * 8 * (ATTN_SUB + 4) * 4 + 2 * 8 * 16 * 4 + 2 * ATTN_SUB * 4;
+    // at the end: output pieces [16 warps][8][64] | sums [4][8] | merge weights
+    const int b = NCW * 8 * 64 * 4 + 4 * 8 * 4 + 8 * ATTN_MAX_CHUNKS * 4;
+    return a > b ? a : b;
+}
+__device__ __forceinline__ uint32_t bf16x2(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __noinline__ void attn_mma_stage(Shared& S, const mk_stage_desc& d) {
+    const int NKV = d.i[MKS_I_NKV], HD = d.i[MKS_I_HD], QPK = d.i[MKS_I_NQ] / NKV, ROT = d.i[MKS_I_ROT];
+    const int window = d.i[MKS_I_WINDOW], maxpages = d.i[MKS_I_MAX_PAGES], max_chunks = d.i[MKS_I_MAX_CHUNKS];
+    const int kvb = d.i[MKS_I_KV_BLOCK] > 0 ? d.i[MKS_I_KV_BLOCK] : 64, kvb_shift = 31 - __clz(kvb);
+    const bool own_layout = d.i[MKS_I_KV_S_PAGE] == 0;
+    const uint32_t kv_s_page = own_layout ? (uint32_t)(NKV * kvb * HD) : (uint32_t)d.i[MKS_I_KV_S_PAGE];
+    const uint32_t kv_s_head = own_layout ? (uint32_t)(kvb * HD) : (uint32_t)d.i[MKS_I_KV_S_HEAD];
+    const uint32_t kv_s_pos = own_layout ? (uint32_t)HD : (uint32_t)d.i[MKS_I_KV_S_POS];
+    __nv_bfloat16* kc = reinterpret_cast<__nv_bfloat16*>(d.p[MKS_P_K_CACHE]);
+    __nv_bfloat16* vc = reinterpret_cast<__nv_bfloat16*>(d.p[MKS_P_V_CACHE]);
+    const int* bt = reinterpret_cast<const int*>(d.p[MKS_P_BLOCK_TABLE]);
+    const float eps = d.f[MKS_F_EPS], scale = d.f[MKS_F_SCALE], norm_off = d.i[MKS_I_NORM_PLAIN] ? 0.f : 1.f;
+    const int rec = (QPK * (HD + 2) + 3) & ~3;
+    float* q_s = reinterpret_cast<float*>(S.xs());             // [QPK][HD]
+    float* kn_s = q_s + QPK * HD;                              // [2][HD]: the new K row, the new V row
+    uint8_t* qb = reinterpret_cast<uint8_t*>(kn_s + 2 * HD);   // [8][HD + 8] bf16
+    const int qb_stride = (HD + 8) * 2;
+    float* sc_s = reinterpret_cast<float*>(qb + 8 * qb_stride);   // [2][8][ATTN_SUB + 4]
+    float* wm_s = sc_s + 2 * 8 * (ATTN_SUB + 4);               // [2][8][16]
+    uint32_t* row_s = reinterpret_cast<uint32_t*>(wm_s + 2 * 8 * 16);   // [2][ATTN_SUB] element offsets of the cache rows
+    const int g = lane_() >> 2, t = lane_() & 3;
+    const int ndg = HD / 64, nres = NCW / ndg, dg = warp_() % ndg, res = warp_() / ndg;
+    int maxn = 1;
+#pragma unroll 1
+    for (int m = 0; m < S.A.M; m++) {
+        const int n = S.pos_s[m] + 1;
+        maxn = max(maxn, window ? min(n, window) : n);
+    }
+    // as many chunks per (sequence, KV head) as give every CTA at most one task, whole tiles each
+    const int pairs_all = S.A.M * NKV;
+    const int want = max(1, min(min(grid_() / pairs_all, max_chunks), (maxn + 15) / 16));
+    const int CP = ((maxn + want - 1) / want + 15) & ~15;
+    const int NCH = (maxn + CP - 1) / CP;
+#pragma unroll 1
+    for (int task = cta_(); task < pairs_all * NCH; task += grid_()) {
+        const int ch = task % NCH, kvh = (task / NCH) % NKV, m = task / (NCH * NKV);
+        if (!S.valid_s[m]) continue;                           // a padding row reads and writes no KV (uniform over the CTA)
+        const int pos = S.pos_s[m], n = pos + 1;
+        const int lo = window ? max(0, n - window) : 0;
+        const int first = lo + ch * CP;
+        if (first >= n) continue;                              // uniform over the CTA
+        const int last = min(first + CP, n), np = last - first;
+        const int nch = (n - lo + CP - 1) / CP;
+        const bool has_new = last == n;
+        const float* y = reinterpret_cast<const float*>(d.p[MKS_P_A_Y]) + (size_t)m * d.i[MKS_I_A_Y_STRIDE];
+        // cache rows of sub-chunk `sub` (past the end: its last row), by `nt` threads from `t0`; the first touch of a page after
+        // the weight stream costs microseconds (TLB), so one line per cache block is requested as soon as it is known
+        auto rows = [&](int sub, int i0, int step) {
+            uint32_t* r = row_s + (sub & 1) * ATTN_SUB;
+#pragma unroll 1
+            for (int i = i0; i < ATTN_SUB; i += step) {
+                const int p = min(first + sub * ATTN_SUB + i, last - 1);
+                const int page = __ldg(bt + (size_t)m * maxpages + (p >> kvb_shift));
+                const uint32_t off = (uint32_t)page * kv_s_page + (uint32_t)kvh * kv_s_head + (uint32_t)(p & (kvb - 1)) * kv_s_pos;
+                r[i] = off;
+                if (i == 0 || (p & (kvb - 1)) == 0) {
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(kc + off));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(vc + off));
+                }
             }
-            S.flag = is_last;
+        };
+        // queries (warps 0..QPK-1), new K and V (the next two), cache rows (the others)
+        {
+            const int pairs = d.i[MKS_I_ROPE_PAIRS], pair_dist = ROT == HD ? HD / 2 : ROT / 2;
+            const int w = warp_();
+            if (w < QPK || (has_new && w < QPK + 2)) {
+                const int which = w < QPK ? 0 : w - QPK + 1;   // 0: query, 1: K, 2: V
+                const int k_off = d.i[MKS_I_A_K_OFF], v_off = d.i[MKS_I_A_V_OFF];
+                const float* src = which == 0 ? y + d.i[MKS_I_A_Q_OFF] + (size_t)(kvh * QPK + w) * d.i[MKS_I_A_Q_HSTRIDE]
+                                              : y + (which == 2 && v_off >= 0 ? v_off : k_off) + (size_t)kvh * HD;
+                float* dst = which == 0 ? q_s + w * HD : kn_s + (which - 1) * HD;
+                const float* cs = which == 2 ? nullptr : reinterpret_cast<const float*>(d.p[MKS_P_ROPE_COS]) + (size_t)pos * pairs;
+                head_prepare(S, src, dst, HD, which == 2 ? nullptr : reinterpret_cast<const float*>(d.p[which == 0 ? MKS_P_Q_NORM : MKS_P_K_NORM]), norm_off,
+                             which != 2 || d.i[MKS_I_V_NORM] != 0, eps, cs, reinterpret_cast<const float*>(d.p[MKS_P_ROPE_SIN]) + (size_t)pos * pairs, pairs, pair_dist, false);
+                __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(qb + w * qb_stride);
+                if (which) {                                   // append the new row to the paged cache
+                    const int page = __ldg(bt + (size_t)m * maxpages + (pos >> kvb_shift));
+                    out = (which == 1 ? kc : vc) + ((size_t)page * kv_s_page + (size_t)kvh * kv_s_head + (size_t)(pos & (kvb - 1)) * kv_s_pos);
+                }
+#pragma unroll 1
+                for (int i = lane_() * 2; i < HD; i += 64) *reinterpret_cast<uint32_t*>(out + i) = bf16x2(dst[i], dst[i + 1]);
+            } else if (w >= QPK + 2) {
+                rows(0, tid_() - (QPK + 2) * 32, NCT - (QPK + 2) * 32);
+            }
+            if (w >= 8)                                        // heads that do not exist: zero columns
+#pragma unroll 1
+                for (int i = tid_() - 8 * 32; i < (8 - QPK) * (qb_stride / 4); i += 8 * 32) reinterpret_cast<uint32_t*>(qb + QPK * qb_stride)[i] = 0u;
         }
+        __syncwarp();
         consumer_sync();
-        if (S.flag) {
-            const float* pbase = part + ((size_t)(m * NKV + kvh) * max_chunks) * rec;
-            // weights of the chunks: w[hq][j] = exp(max_j - max) / sum_j' exp(max_j' - max) l_j'
+        prof_mark(S, 4);
+        float acc[8][4], mrun = -3.0e38f, lsum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+        const int nsub = (np + ATTN_SUB - 1) / ATTN_SUB;
 #pragma unroll 1
-            for (int i = tid_(); i < QPK * nch; i += NCT) {
-                const int hq = i / nch, j = i - hq * nch;
-                wn_s[hq * ATTN_MAX_CHUNKS + j] = ldcg_f(pbase + (size_t)j * rec + QPK * HD + 2 * hq);
+        for (int sub = 0; sub < nsub; sub++) {
+            const int ns = min(ATTN_SUB, np - sub * ATTN_SUB), ntile = (ns + 15) >> 4;
+            const uint32_t* row = row_s + (sub & 1) * ATTN_SUB;
+            float* sc = sc_s + (sub & 1) * 8 * (ATTN_SUB + 4);
+            float* wm = wm_s + (sub & 1) * 8 * 16;
+            {
+                // scores of tile `warp`
+                float c[4] = {0.f, 0.f, 0.f, 0.f};
+                const int ia = warp_() * 16 + g, ib = ia + 8;
+                if (warp_() < ntile) {
+                    const __nv_bfloat16* ra = kc + row[ia] + t * 8;
+                    const __nv_bfloat16* rb = kc + row[ib] + t * 8;
+                    const uint8_t* q = qb + g * qb_stride + t * 16;
+                    float c2[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+                    for (int e = 0; e < HD; e += 256) {
+                        uint4 ka[8], kb[8];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            ka[j] = __ldcg(reinterpret_cast<const uint4*>(ra + e + j * 32));
+                            kb[j] = __ldcg(reinterpret_cast<const uint4*>(rb + e + j * 32));
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            const uint4 qv = *reinterpret_cast<const uint4*>(q + (e + j * 32) * 2);
+                            const uint32_t a0[4] = {ka[j].x, kb[j].x, ka[j].y, kb[j].y}, a1[4] = {ka[j].z, kb[j].z, ka[j].w, kb[j].w};
+                            mma_bf16(c, a0, qv.x, qv.y);
+                            mma_bf16(c2, a1, qv.z, qv.w);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) c[i] = (c[i] + c2[i]) * scale;
+                }
+                if (ia >= ns) c[0] = c[1] = -3.0e38f;
+                if (ib >= ns) c[2] = c[3] = -3.0e38f;
+                sc[(2 * t) * (ATTN_SUB + 4) + ia] = c[0];
+                sc[(2 * t + 1) * (ATTN_SUB + 4) + ia] = c[1];
+                sc[(2 * t) * (ATTN_SUB + 4) + ib] = c[2];
+                sc[(2 * t + 1) * (ATTN_SUB + 4) + ib] = c[3];
+                float m0 = fmaxf(c[0], c[2]), m1 = fmaxf(c[1], c[3]);
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+                    m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+                }
+                if (g == 0) {
+                    wm[(2 * t) * 16 + warp_()] = m0;
+                    wm[(2 * t + 1) * 16 + warp_()] = m1;
+                }
             }
+            if (sub + 1 < nsub) rows(sub + 1, tid_(), NCT);
+            // the first tile's V rows are requested before the scores are exchanged
+            const __nv_bfloat16* vd = vc + dg * 64 + g * 8;
+            uint4 v[4];
+            auto request = [&](int tile) {
+                const uint32_t* r = row + tile * 16 + 2 * t;
+                v[0] = __ldcg(reinterpret_cast<const uint4*>(vd + r[0]));
+                v[1] = __ldcg(reinterpret_cast<const uint4*>(vd + r[1]));
+                v[2] = __ldcg(reinterpret_cast<const uint4*>(vd + r[8]));
+                v[3] = __ldcg(reinterpret_cast<const uint4*>(vd + r[9]));
+            };
+            if (res < ntile) request(res);
+            __syncwarp();
             consumer_sync();
-            if (warp_() < QPK) {
-                float* w = wn_s + warp_() * ATTN_MAX_CHUNKS;
-                float mx = -3.0e38f;
-#pragma unroll 1
-                for (int j = lane_(); j < nch; j += 32) mx = fmaxf(mx, w[j]);
-                mx = warp_max(mx);
-                float den = 0.f;
-#pragma unroll 1
-                for (int j = lane_(); j < nch; j += 32) {
-                    const float ex = __expf(w[j] - mx);
-                    w[j] = ex;
-                    den += ex * ldcg_f(pbase + (size_t)j * rec + QPK * HD + 2 * warp_() + 1);
-                }
-                den = warp_sum(den);
-                __syncwarp();
-#pragma unroll 1
-                for (int j = lane_(); j < nch; j += 32) w[j] = w[j] / den;
+            // this lane's head is g
+            float mnew = mrun;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 x = *reinterpret_cast<const float4*>(wm + g * 16 + i * 4);
+                mnew = fmaxf(mnew, fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)));
             }
-            consumer_sync();
+            if (sub) {
+                const float f = __expf(mrun - mnew);
+                lsum *= f;
+#pragma unroll
+                for (int j = 0; j < 8; j++) { acc[j][0] *= f; acc[j][1] *= f; acc[j][2] *= f; acc[j][3] *= f; }
+            }
+            mrun = mnew;
 #pragma unroll 1
-            for (int idx = tid_(); idx < QPK * (HD / 4); idx += NCT) {
-                const int hq = idx / (HD / 4), dd = (idx - hq * (HD / 4)) * 4;
-                const float* w = wn_s + hq * ATTN_MAX_CHUNKS;
-                float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
-#pragma unroll 8
-                for (int j = 0; j < nch; j++) {
-                    const float4 v = __ldcg(reinterpret_cast<const float4*>(pbase + (size_t)j * rec + hq * HD + dd));
-                    o0 = fmaf(w[j], v.x, o0); o1 = fmaf(w[j], v.y, o1); o2 = fmaf(w[j], v.z, o2); o3 = fmaf(w[j], v.w, o3);
+            for (int tile = res; tile < ntile; tile += nres) {
+                uint32_t b0[8], b1[8];
+                {
+                    const uint32_t* x = reinterpret_cast<const uint32_t*>(v);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        b0[2 * i] = __byte_perm(x[i], x[4 + i], 0x5410); b0[2 * i + 1] = __byte_perm(x[i], x[4 + i], 0x7632);
+                        b1[2 * i] = __byte_perm(x[8 + i], x[12 + i], 0x5410); b1[2 * i + 1] = __byte_perm(x[8 + i], x[12 + i], 0x7632);
+                    }
                 }
-                const int hfull = kvh * QPK + hq;
-                if (gate_off >= 0) {
-                    const float4 g = __ldcg(reinterpret_cast<const float4*>(y + q_off + (size_t)hfull * q_hs + gate_off + dd));
-                    o0 *= sigmoid_f(g.x); o1 *= sigmoid_f(g.y); o2 *= sigmoid_f(g.z); o3 *= sigmoid_f(g.w);
+                if (tile + nres < ntile) request(tile + nres);
+                const float* sp = sc + g * (ATTN_SUB + 4) + tile * 16 + 2 * t;
+                const float2 sa = *reinterpret_cast<const float2*>(sp), sb = *reinterpret_cast<const float2*>(sp + 8);
+                float pr[4] = {__expf(sa.x - mnew), __expf(sa.y - mnew), __expf(sb.x - mnew), __expf(sb.y - mnew)};
+                lsum += (pr[0] + pr[1]) + (pr[2] + pr[3]);
+                uint32_t hi[4], lw[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (int piece = 0; piece < 3; piece++) {
+                    const uint32_t w0 = bf16x2(pr[0], pr[1]), w1 = bf16x2(pr[2], pr[3]);
+                    pr[0] -= bf_lo(w0); pr[1] -= bf_hi(w0); pr[2] -= bf_lo(w1); pr[3] -= bf_hi(w1);
+                    if (piece == 0) { hi[0] = w0; hi[2] = w1; }
+                    if (piece == 1) { hi[1] = w0; hi[3] = w1; }
+                    if (piece == 2) { lw[0] = w0; lw[2] = w1; }
                 }
-                __stcg(reinterpret_cast<float4*>(Y2 + (size_t)m * d.i[MKS_I_A_Y2_STRIDE] + (size_t)hfull * HD + dd), make_float4(o0, o1, o2, o3));
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    mma_bf16(acc[j], hi, b0[j], b1[j]);
+                    mma_bf16(acc[j], lw, b0[j], b1[j]);
+                }
             }
         }
+        // the warps' pieces of the output meet in shared memory: [warp][head][64 dims]
+        __syncwarp();
+        consumer_sync();
+        float* red = reinterpret_cast<float*>(S.xs());
+        float* l_s = red + NCW * 8 * 64;                       // [residue][head]
+        float* wn_s = l_s + 4 * 8;
+        {
+            float* mine = red + (warp_() * 8 + g) * 64 + t * 16;      // column 2t holds dims 16 t + j, column 2t + 1 dims 16 t + 8 + j
+#pragma unroll
+            for (int j = 0; j < 8; j += 4) {
+                *reinterpret_cast<float4*>(mine + j) = make_float4(acc[j][0] + acc[j][2], acc[j + 1][0] + acc[j + 1][2], acc[j + 2][0] + acc[j + 2][2], acc[j + 3][0] + acc[j + 3][2]);
+                *reinterpret_cast<float4*>(mine + 8 + j) = make_float4(acc[j][1] + acc[j][3], acc[j + 1][1] + acc[j + 1][3], acc[j + 2][1] + acc[j + 2][3], acc[j + 3][1] + acc[j + 3][3]);
+            }
+            lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
+            lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
+            if (dg == 0 && t == 0) l_s[res * 8 + g] = lsum;
+        }
+        __syncwarp();
+        consumer_sync();
+        float* prec = reinterpret_cast<float*>(d.p[MKS_P_A_PART]) + ((size_t)(m * NKV + kvh) * max_chunks + ch) * rec;
+        const int hd4 = HD / 4, hd4_shift = 31 - __clz(hd4);
+#pragma unroll 1
+        for (int idx = tid_(); idx < QPK * hd4; idx += NCT) {
+            const int hq = idx >> hd4_shift, dd = (idx & (hd4 - 1)) * 4;
+            const float* src = red + ((dd >> 6) * 8 + hq) * 64 + (dd & 63);
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int r = 0; r < nres; r++) {
+                const float4 x = *reinterpret_cast<const float4*>(src + r * ndg * 8 * 64);
+                o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
+            }
+            __stcg(reinterpret_cast<float4*>(prec + hq * HD + dd), o);
+        }
+        if (warp_() == 0 && t == 0 && g < QPK) {
+            float l = 0.f;
+#pragma unroll 1
+            for (int r = 0; r < nres; r++) l += l_s[r * 8 + g];
+            __stcg(prec + QPK * HD + 2 * g, mrun);
+            __stcg(prec + QPK * HD + 2 * g + 1, l);
+        }
+        attn_merge(S, d, m, kvh, nch, y, wn_s);
+        __syncwarp();
         consumer_sync();
     }
 }
@@ -817,6 +1102,7 @@ c.f.src = nullptr; c.f.steps = c.f.left = c.f.eoff = c.f.ebps = c.f.cs = c.f.ahe
                 case MKS_OP_GDN: gdn_stage(S, d); break;
                 case MKS_OP_ATTN:
                     if (d.i[MKS_I_KV_F32]) attn_stage<true>(S, d);
+                    else if (d.i[MKS_I_Q_BF16]) attn_mma_stage(S, d);
                     else attn_stage<false>(S, d);
                     break;
                 case MKS_OP_ROUTE: route_stage(S, d); break;
