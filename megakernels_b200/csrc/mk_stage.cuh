@@ -43,7 +43,7 @@ constexpr int XS_BYTES = 82432;                   // staged GEMV input: 8 column
 constexpr int MAX_GROUPS = 72;                    // routed experts of one step (8 x 8) + shared / dense groups
 constexpr int MISC_BYTES = 10752;
 constexpr int SMEM_TOTAL = 232448;                // 227 KB
-constexpr int MIN_RING_DEPTH = 4, MAX_RING_DEPTH = 6;   // ring slots per consumer warp: as many as the launch's input staging area leaves room for
+constexpr int MIN_RING_DEPTH = 4, MAX_RING_DEPTH = 5;   // ring slots per consumer warp: as many as the launch's input staging area leaves room for
 constexpr int MAX_SEGS = 16;                      // K splits (of all groups) of one panel of a stage that adds its groups up
 constexpr int TILE_BYTES = 16 * 512;              // what each warp adds to a tile that the warp before it started
 constexpr int GEO_RING = 4;                       // stage records in shared memory: the scout is up to three stages ahead
@@ -102,14 +102,14 @@ struct Share {
     int c, c1, n;                  // and all of the batch's chunks
     int cpt, tl, k;                // chunks of one tile; chunk c as tile of the batch and chunk of the tile
 };
-// The stream's registers (the same in every lane).
+// The stream's registers (the same in every lane but for what is said to be the lane's own).
 struct Feed {
-    const uint8_t* src;            // next step of the current chunk (of the whole run, where chunks carry no scales)
+    const uint8_t* src;            // next step of the current chunk (of the whole run, where chunks carry no scales); this lane's bytes
     int steps, left;               // steps left in it, chunks left in the run behind it
-    int eoff;                      // from src to the scales of that step
+    int eoff;                      // from src to the scales of that step (this lane's)
     int ebps, cs;                  // scale bytes per step, steps per chunk
     int ahead;                     // blocks requested and not yet multiplied
-    uint32_t rd, wr;               // shared-memory addresses (this lane's part) of the next block to multiply, the next to request
+    uint32_t rd;                   // shared-memory address of the next block to multiply (this lane's part)
 };
 // Where a consumer warp's weight stream stands: ahead of the multiplication by up to the ring's depth.
 struct Cur {
@@ -123,7 +123,7 @@ struct Cur {
     uint32_t gn, now;              // stages entered; the stage the warp multiplies in
     int b, nb;                     // batches of the stage begun, all of them
     // the registers of the stream between two GEMV stages
-    Feed f;                        // (rd, wr without the lane's part)
+    Feed f;                        // (the first lane's)
 };
 
 struct Shared {
@@ -474,6 +474,12 @@ __device__ __noinline__ bool next_run(Shared& S) {
     __syncwarp();
     return left > 0;
 }
+__device__ __forceinline__ void next_chunk(Feed& f) {
+    f.src += f.cs * f.ebps;                                    // past the scales of the chunk before
+    f.left--;
+    f.steps = f.cs;
+    f.eoff = f.cs * 512 - lane_() * 12;
+}
 // Fill the warp's free slots.  The caller has ordered the warp's reads of the freed slots before this (a warp barrier).
 // Every free slot gets a group of copies, an empty one when there is nothing to request: then at least ring_depth - 1
 // groups lie behind the next block to multiply, and waiting for all but that many waits for the block.
@@ -483,41 +489,49 @@ __device__ __forceinline__ void feed(Shared& S, Feed& f, int depth, uint32_t rin
     for (; n_free > 0; n_free--) {
         if (f.steps == 0) {
             if (f.left > 0) {
-                f.src += f.cs * f.ebps;                        // past the scales of the chunk before
-                f.left--;
+                next_chunk(f);
             } else {
                 if (!next_run(S)) break;
                 const Cur& c = S.cur[warp_()];
-                f.src = c.src; f.ebps = c.ebps; f.cs = c.chunk_steps; f.left = c.left;
-                if (f.ebps == 0) f.cs *= f.left;
-                f.left = f.ebps == 0 ? 0 : f.left - 1;
+                f.ebps = c.ebps;
+                f.cs = f.ebps ? c.chunk_steps : c.chunk_steps * c.left;
+                f.left = f.ebps ? c.left : 1;
+                f.src = c.src + lane_() * 16 - f.cs * f.ebps;
+                next_chunk(f);
             }
-            f.steps = f.cs;
-            f.eoff = f.cs * 512;
         }
         const int n = min(BLOCK_STEPS, f.steps);
-        const uint8_t* src = f.src + lane_() * 16;
-#pragma unroll
-        for (int u = 0; u < BLOCK_STEPS; u++)
-            if (u < n) cp_async16(f.wr + u * 512, src + u * 512);
-        if (lane_() * 4 < n * f.ebps) cp_async4(f.wr + BLOCK_STEPS * 512 - lane_() * 12, f.src + f.eoff + lane_() * 4);
+        uint32_t wr = f.rd + f.ahead * BLOCK_BYTES;
+        if (wr >= ring_end) wr -= depth * BLOCK_BYTES;
+#pragma unroll 1
+        for (int u = 0; u < n; u++) cp_async16(wr + u * 512, f.src + u * 512);
+        if (lane_() * 4 < n * f.ebps) cp_async4(wr + BLOCK_STEPS * 512 - lane_() * 12, f.src + f.eoff);
         cp_async_commit();
         f.src += n * 512;
         f.steps -= n;
         f.eoff += n * (f.ebps - 512);
         f.ahead++;
-        f.wr += BLOCK_BYTES;
-        if (f.wr >= ring_end) f.wr -= depth * BLOCK_BYTES;
     }
 #pragma unroll 1
     for (; n_free > 0; n_free--) cp_async_commit();
 }
+// The same where only slot `wr` is free and a whole block can be requested (nearly always).
+__device__ __forceinline__ void feed_one(Feed& f, uint32_t wr) {
+#pragma unroll
+    for (int u = 0; u < BLOCK_STEPS; u++) cp_async16(wr + u * 512, f.src + u * 512);
+    if (lane_() < f.ebps) cp_async4(wr + BLOCK_STEPS * 512 - lane_() * 12, f.src + f.eoff);
+    cp_async_commit();
+    f.src += BLOCK_STEPS * 512;
+    f.eoff += BLOCK_STEPS * (f.ebps - 512);
+    f.steps -= BLOCK_STEPS;
+    f.ahead++;
+    if (f.steps == 0 && f.left > 0) next_chunk(f);
+}
 // All but depth - 1 groups of copies have landed.
 __device__ __forceinline__ void wait_block(int depth) {
-    static_assert(MIN_RING_DEPTH == 4 && MAX_RING_DEPTH == 6, "one wait per ring depth");
+    static_assert(MIN_RING_DEPTH == 4 && MAX_RING_DEPTH == 5, "one wait per ring depth");
     if (depth == 4) cp_async_wait<3>();
-    else if (depth == 5) cp_async_wait<4>();
-    else cp_async_wait<5>();
+    else cp_async_wait<4>();
 }
 
 // ---- scout ---------------------------------------------------------------------------------------------------
@@ -904,8 +918,7 @@ __device__ __forceinline__ void tile_step(uint32_t sl, uint32_t sc, int st, cons
         // The conversion unit (cvt ... e2m1x2) is the scarcest pipe of this loop, so only half of the
         // values go through it.  The 32 columns of scale group 0 (MMAs 0 and 1) arrive with their bits
         // pre-arranged by the packer: every 32-bit word yields four f16x2 registers with shifts and masks
-        // alone (sign at bit 15, the three magnitude bits at 11..9 of each half: the value times 2^-14,
-        // which the group's scale takes back).  Scale group 1 (MMAs 2 and 3) keeps plain nibbles.
+        // alone (sign at bit 15, the three magnitude bits at 11..9 of each half: the value times 2^-14).  Scale group 1 (MMAs 2 and 3) keeps plain nibbles.
         const uint32_t scw = lds_u32(sc);
         float t0[4] = {0.f, 0.f, 0.f, 0.f};                                    // scale group 0: MMAs 0, 1
         float u0[4] = {0.f, 0.f, 0.f, 0.f};                                    // scale group 1: MMAs 2, 3
@@ -940,9 +953,10 @@ __device__ __forceinline__ void tile_step(uint32_t sl, uint32_t sc, int st, cons
             a[3] = cvt_e2m1x2(hi >> 24);
             mma_f16(u0, a, b[3].x, b[3].y);
         }
-        // e8m0 scales: bytes [row g: group 0, group 1, row g + 8: group 0, group 1]; group 0 also takes 2^14
-        const float s00 = __uint_as_float(((scw & 0xFFu) + 14u) << 23), s01 = __uint_as_float(((scw >> 8) & 0xFFu) << 23);
-        const float s10 = __uint_as_float((((scw >> 16) & 0xFFu) + 14u) << 23), s11 = __uint_as_float((scw >> 24) << 23);
+        // e8m0 scales: bytes [row g: group 0, group 1, row g + 8: group 0, group 1]; group 0 is collected in `acc`, which takes
+        // back the 2^14 at the end of the tile
+        const float s00 = __uint_as_float((scw << 23) & 0x7F800000u), s01 = __uint_as_float((scw << 15) & 0x7F800000u);
+        const float s10 = __uint_as_float((scw << 7) & 0x7F800000u), s11 = __uint_as_float((scw >> 1) & 0x7F800000u);
         acc[0] = fmaf(t0[0], s00, acc[0]); acc[1] = fmaf(t0[1], s00, acc[1]);
         acc[2] = fmaf(t0[2], s10, acc[2]); acc[3] = fmaf(t0[3], s10, acc[3]);
         acc2[0] = fmaf(u0[0], s01, acc2[0]); acc2[1] = fmaf(u0[1], s01, acc2[1]);
@@ -1110,9 +1124,11 @@ __device__ __forceinline__ bool multiply(Shared& S, const mk_stage_desc& d, cons
     constexpr int STEP_BYTES = (FMT == MKS_FMT_MXFP4 ? 4 : (FMT == MKS_FMT_BF16 ? 1 : 2)) * 32;   // staged input bytes of one tile step
     const int depth = S.A.ring_depth;
     Feed f = S.cur[warp_()].f;
+    f.src += lane_() * 16;
+    f.eoff -= lane_() * 12;
     f.rd += lane_() * 16;
-    f.wr += lane_() * 16;
-    const uint32_t ring_end = smem_u32(S.ring()) + (warp_() + 1) * depth * BLOCK_BYTES;
+    const int ring_bytes = depth * BLOCK_BYTES;
+    const uint32_t ring_end = smem_u32(S.ring()) + (warp_() + 1) * ring_bytes;
     __syncwarp();
     if (lane_() == 0) S.cur[warp_()].now = n_stage;
     __syncwarp();
@@ -1156,46 +1172,48 @@ __device__ __forceinline__ bool multiply(Shared& S, const mk_stage_desc& d, cons
             // lanes beyond the staged columns read a live one (their accumulators are never used): predicated zeros cost a tenth of the loop
             const uint8_t* xk = S.xs() + min(lane_() >> 2, S.A.M * d.i[MKS_I_PIECES] - 1) * stride + (lane_() & 3) * 8 + k * chunk_steps * STEP_BYTES;
             // the stream's blocks end where a chunk with scales, or a run of chunks, ends
-            int chunks = run;
+            int steps = run * chunk_steps, in = scales ? chunk_steps : steps;
+            const uint32_t sc_off = BLOCK_STEPS * 512 - lane_() * 16 + (lane_() >> 2) * 4;
 #pragma unroll 1
-            while (chunks > 0 && ok) {
-                const int take = scales ? 1 : chunks;
-                int steps = take * chunk_steps;
-                chunks -= take;
-#pragma unroll 1
-                while (steps > 0) {
-                    __syncwarp();
+            while (steps > 0) {
+                __syncwarp();                                  // the warp has read the block before
+                if (f.ahead == depth - 1 && f.steps >= BLOCK_STEPS) {
+                    feed_one(f, f.rd == ring_end - ring_bytes + lane_() * 16 ? ring_end - BLOCK_BYTES + lane_() * 16 : f.rd - BLOCK_BYTES);
+                } else {
                     feed(S, f, depth, ring_end);
                     if (f.ahead == 0) {                        // (a stream that was refused: the launch has failed)
                         ok = false;
                         break;
                     }
-                    wait_block(depth);
-                    __syncwarp();
-                    const uint32_t sl = f.rd;
-                    if (steps >= BLOCK_STEPS) {
-#pragma unroll
-                        for (int st = 0; st < BLOCK_STEPS; st++, xk += STEP_BYTES) tile_step<FMT>(sl + st * 512, sl + BLOCK_STEPS * 512 + st * 32 - lane_() * 16 + (lane_() >> 2) * 4, st, xk, acc, acc2);
-                    } else {
-#pragma unroll 1
-                        for (int st = 0; st < steps; st++, xk += STEP_BYTES) tile_step<FMT>(sl + st * 512, sl + BLOCK_STEPS * 512 + st * 32 - lane_() * 16 + (lane_() >> 2) * 4, st, xk, acc, acc2);
-                    }
-                    if (FMT == MKS_FMT_FP8 && scales) {
-                        // one scale per 128 k for rows 0-7 of the tile and one for rows 8-15 (a GLU tile pairs two matrices)
-                        const float2 bs = lds_f2(sl + BLOCK_STEPS * 512 - lane_() * 16);
-                        tot[0] = fmaf(acc[0] + acc2[0], bs.x, tot[0]); tot[1] = fmaf(acc[1] + acc2[1], bs.x, tot[1]);
-                        tot[2] = fmaf(acc[2] + acc2[2], bs.y, tot[2]); tot[3] = fmaf(acc[3] + acc2[3], bs.y, tot[3]);
-                        acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-                        acc2[0] = acc2[1] = acc2[2] = acc2[3] = 0.f;
-                    }
-                    steps -= BLOCK_STEPS;
-                    f.ahead--;
-                    f.rd += BLOCK_BYTES;
-                    if (f.rd >= ring_end) f.rd -= depth * BLOCK_BYTES;
                 }
+                wait_block(depth);
+                __syncwarp();
+                const uint32_t sl = f.rd;
+                const int ns = min(BLOCK_STEPS, in);
+                if (ns == BLOCK_STEPS) {
+#pragma unroll
+                    for (int st = 0; st < BLOCK_STEPS; st++, xk += STEP_BYTES) tile_step<FMT>(sl + st * 512, sl + sc_off + st * 32, st, xk, acc, acc2);
+                } else {
+#pragma unroll 1
+                    for (int st = 0; st < ns; st++, xk += STEP_BYTES) tile_step<FMT>(sl + st * 512, sl + sc_off + st * 32, st, xk, acc, acc2);
+                }
+                if (FMT == MKS_FMT_FP8 && scales) {
+                    // one scale per 128 k for rows 0-7 of the tile and one for rows 8-15 (a GLU tile pairs two matrices)
+                    const float2 bs = lds_f2(sl + BLOCK_STEPS * 512 - lane_() * 16);
+                    tot[0] = fmaf(acc[0] + acc2[0], bs.x, tot[0]); tot[1] = fmaf(acc[1] + acc2[1], bs.x, tot[1]);
+                    tot[2] = fmaf(acc[2] + acc2[2], bs.y, tot[2]); tot[3] = fmaf(acc[3] + acc2[3], bs.y, tot[3]);
+                    acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+                    acc2[0] = acc2[1] = acc2[2] = acc2[3] = 0.f;
+                }
+                steps -= ns;
+                in -= ns;
+                if (in == 0) in = chunk_steps;
+                f.ahead--;
+                f.rd += BLOCK_BYTES;
+                if (f.rd >= ring_end) f.rd -= ring_bytes;
             }
 #pragma unroll
-            for (int i = 0; i < 4; i++) acc[i] = acc[i] + acc2[i] + (FMT == MKS_FMT_FP8 ? tot[i] : 0.f);
+            for (int i = 0; i < 4; i++) acc[i] = acc[i] * (FMT == MKS_FMT_MXFP4 ? 16384.f : 1.f) + acc2[i] + (FMT == MKS_FMT_FP8 ? tot[i] : 0.f);
         }
         __syncwarp();
         // undo the input scaling, fold the second piece's columns onto the first
@@ -1243,8 +1261,6 @@ __device__ __forceinline__ bool multiply(Shared& S, const mk_stage_desc& d, cons
     __syncwarp();
     feed(S, f, depth, ring_end);
     if (lane_() == 0) {
-        f.rd -= lane_() * 16;
-        f.wr -= lane_() * 16;
         S.cur[warp_()].f = f;
     }
     __syncwarp();
