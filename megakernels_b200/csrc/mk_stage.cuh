@@ -95,6 +95,7 @@ struct Geo {
     int g0, ng;                    // groups these tiles lie in, when every group has an input of its own (else 0, 1)
     int nb;                        // batches: one staged input each
     uint32_t stage;                // the stage this entry describes (counted over the launch)
+    int beside;                    // CTAs this stage leaves to the one behind it (0: it has the whole grid, or the rest of it)
 };
 // A warp's share of a batch: chunks [c, c1), tile by tile.
 struct Share {
@@ -119,7 +120,7 @@ struct Cur {
     int run, jump;                 // chunks of a whole run, bytes from one's end to the next
     int chunk_bytes, chunk_steps;
     int ebps;                      // scale bytes per tile step (behind a chunk's steps)
-    int tile, seg;                 // the run behind the current one, if the runs belong to several matrices
+    int tile, seg, seg0, seg1;     // the run behind the current one, if the runs belong to several matrices; the batch's K splits
     uint32_t gn, now;              // stages entered; the stage the warp multiplies in
     int b, nb;                     // batches of the stage begun, all of them
     // the registers of the stream between two GEMV stages
@@ -398,9 +399,9 @@ __device__ __noinline__ bool next_run(Shared& S) {
             src = split_weights(S, g, tile, seg);
             __syncwarp();
             if (lane_() == 0) {
-                const Batch bt = geo_batch(g, c.b - 1);
-                c.seg = !g.reduce || seg + 1 == bt.seg1 ? bt.seg0 : seg + 1;
-                c.tile = c.seg == bt.seg0 ? tile + 1 : tile;
+                const bool end = !g.reduce || seg + 1 == c.seg1;
+                c.seg = end ? c.seg0 : seg + 1;
+                c.tile = end ? tile + 1 : tile;
             }
         }
         left = min(run, rest);
@@ -459,7 +460,7 @@ __device__ __noinline__ bool next_run(Shared& S) {
                 c.run = run;
                 c.jump = (g.S * g.n_chunks - sh.cpt) * g.chunk_bytes;
                 c.chunk_bytes = g.chunk_bytes; c.chunk_steps = g.chunk_steps; c.ebps = g.ebps;
-                c.tile = tile; c.seg = seg;
+                c.tile = tile; c.seg = seg; c.seg0 = bt.seg0; c.seg1 = bt.seg1;
             }
         }
         __syncwarp();
@@ -551,10 +552,23 @@ __device__ __forceinline__ bool scout_wait(Shared& S, volatile unsigned* word, u
     __syncwarp();
     return true;
 }
+// Two GEMV stages without a barrier between them do not depend on each other, and a small one is all latency: they share the
+// grid in proportion to their weights, at least a CTA per tile of a small second one (up to a tenth of the grid).  One after
+// the other the router of a 35B-A3B layer's neighbours cost 17 us behind 13 to 21.  -> CTAs of the second.
+__device__ __forceinline__ int side_by_side(const mk_stage_desc& a, const mk_stage_desc& b, int n_groups, int grid) {
+    const float ta = (float)a.i[MKS_I_TILES] * (a.i[MKS_I_GROUPS] < 0 ? n_groups : a.i[MKS_I_GROUPS]);
+    const float tb = (float)b.i[MKS_I_TILES] * (b.i[MKS_I_GROUPS] < 0 ? n_groups : b.i[MKS_I_GROUPS]);
+    const float ba = ta * a.i[MKS_I_SPLITS] * (a.i[MKS_I_UNIT_STEPS] / a.i[MKS_I_CHUNK_STEPS]) * a.i[MKS_I_CHUNK_BYTES];
+    const float bb = tb * b.i[MKS_I_SPLITS] * (b.i[MKS_I_UNIT_STEPS] / b.i[MKS_I_CHUNK_STEPS]) * b.i[MKS_I_CHUNK_BYTES];
+    const int least = max(2, grid / 10);
+    int k = (int)((float)grid * bb / (ba + bb));
+    k = max(k, min((int)tb, least));
+    k = min(k, grid - min((int)ta, least));
+    return max(1, min(grid - 1, k));
+}
 __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
     constexpr int DESC_WORDS = (int)(sizeof(mk_stage_desc) / 4);
     unsigned n = 0, routes = 0;
-    const int grid = grid_(), cta = cta_();
 #pragma unroll 1
     for (int step = 0; step < A.n_steps; step++) {
 #pragma unroll 1
@@ -575,6 +589,7 @@ __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
             if (d.op != MKS_OP_GEMV) {
                 if (lane_() == 0) {
                     g.nb = 0;
+                    g.beside = 0;
                     g.stage = n;
                     __threadfence_block();
                     S.described = n + 1;
@@ -588,8 +603,22 @@ __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
             const int n_chunks = d.i[MKS_I_UNIT_STEPS] / d.i[MKS_I_CHUNK_STEPS], cb = d.i[MKS_I_CHUNK_BYTES];
             const int R = reduce ? T : G * T, Q = reduce ? G * Sp : Sp;
             const int w = max_panel_splits(A.xs_bytes, kc, A.M * pieces, pieces, reduce);
-            int P = 1, panel = 0, c0 = 0, nc = grid, nb = 0, t0 = 0, t1 = 0;
-            if (R > 0 && Q > 0) {
+            int P = 1, panel = 0, c0 = 0, nc = 0, nb = 0, t0 = 0, t1 = 0;
+            // the CTAs of this stage: all of them, unless it runs beside its neighbour
+            int grid = grid_(), cta = cta_(), beside = 0;
+            const int before = si > 0 ? S.geo[(n - 1) % GEO_RING].beside : 0;
+            if (before > 0) {
+                cta -= grid - before;
+                grid = before;
+            } else if ((d.flags & MKS_FLAG_NO_BARRIER) && si + 1 < A.n_stages && R > 0 && Q > 0) {
+                const mk_stage_desc& nx = A.prog[si + 1];
+                if (nx.op == MKS_OP_GEMV && __ldg(&nx.i[MKS_I_TILES]) > 0) {
+                    beside = side_by_side(d, nx, *reinterpret_cast<const volatile int*>(&S.n_groups), grid);
+                    grid -= beside;
+                }
+            }
+            nc = grid;
+            if (R > 0 && Q > 0 && cta >= 0 && cta < grid) {
                 const int P0 = (Q + w - 1) / w;
                 P = pick_panels(R, Q, P0, n_chunks, cb, kc, A.M, grid);
                 if (P == 0) {
@@ -628,6 +657,7 @@ __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
                 }
                 g.nb = nb * g.ng;
                 g.stage = n;
+                g.beside = beside;
             }
             __syncwarp();
             if (g.nb && lane_() < NCW) S.share[n % GEO_RING][lane_()] = batch_share(S, g, geo_batch(g, 0), lane_());
@@ -654,6 +684,109 @@ constexpr int XB = 4;       // float4 groups per thread and round
 __device__ __forceinline__ int scale_exponent(int bits) {
     const int e = bits > 0 && bits < 0x7f800000 ? ((bits >> 23) & 0xff) - 126 : 0;
     return max(-100, min(100, 14 - e));
+}
+// Four and more sequences, one piece, no adding up of groups: four sequences' values of one column group at a time, the next
+// four requested before the present ones are used.  (All 8 x 5120 values of a 27B layer: 10.5 us with a round trip per four.)
+__device__ __noinline__ void stage_wide(Shared& S, const mk_stage_desc& d, int seg0, int seg1, int grp0) {
+    const int kc = d.i[MKS_I_KC], M = S.A.M, cols = (seg1 - seg0) * kc, stride = xs_stride_bytes(cols);
+    const bool norm = d.i[MKS_I_PROLOGUE] == MKS_P_NORM, bf16 = d.i[MKS_I_FMT] == MKS_FMT_BF16;
+    const int xstride = d.i[MKS_I_X_STRIDE], c4n = cols >> 2;
+    const float* x = reinterpret_cast<const float*>(d.p[MKS_P_X]) + (size_t)grp0 * d.i[MKS_I_X_GSTRIDE] + (size_t)seg0 * kc;
+    const float* nw = reinterpret_cast<const float*>(d.p[MKS_P_NORM_W]) + (size_t)seg0 * kc;
+    const float noff = d.f[MKS_F_NORM_OFF], bound = d.f[MKS_F_IN_BOUND];
+    const bool final_form = bf16 || bound > 0.f;               // see stage_x
+    float fscale = 1.f;
+    if (tid_() < 8) {
+        S.xmax[tid_()] = 0;
+        if (bf16) S.xinv[tid_()] = 1.f;
+    }
+    if (!bf16 && final_form) {
+        const int be = ((__float_as_int(bound) >> 23) & 0xff) - 126;          // bound < 2^be
+        const int e = max(-100, min(100, 15 - be));
+        fscale = __int_as_float((127 + e) << 23);
+        if (tid_() < 8) S.xinv[tid_()] = __int_as_float((127 - e) << 23);
+    }
+    const int total = (c4n + NCT - 1) / NCT * ((M + 3) >> 2);
+    float4 xn[4], wn = make_float4(0.f, 0.f, 0.f, 0.f);
+    int li = tid_(), lm = 0;
+    auto request = [&]() {
+        if (norm && lm == 0 && li < c4n) wn = __ldg(reinterpret_cast<const float4*>(nw) + li);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            xn[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (li < c4n && lm + u < M) xn[u] = __ldcg(reinterpret_cast<const float4*>(x + (size_t)(lm + u) * xstride) + li);
+        }
+    };
+    request();
+    if (norm && warp_() < M) {
+        const int K = d.i[MKS_I_K_TOTAL], n16 = K / 16;
+        const float* row = reinterpret_cast<const float*>(d.p[MKS_P_X_SSQ]) + (size_t)warp_() * n16;
+        float s = 0.f;
+#pragma unroll 8
+        for (int j = lane_(); j < n16; j += 32) s += ldcg_f(row + j);
+        s = warp_sum(s);
+        if (lane_() == 0) S.rstd[warp_()] = rsqrtf(s / (float)K + d.f[MKS_F_EPS]) * (d.f[MKS_F_IN_SCALE] != 0.f ? d.f[MKS_F_IN_SCALE] : 1.f);
+    }
+    __syncwarp();
+    consumer_sync();
+    prof_mark(S, 4);
+#pragma unroll 1
+    for (int it = 0; it < total; it++) {
+        float4 xv[4];
+        const float4 w = wn;
+        const int c4 = li, m0 = lm;
+#pragma unroll
+        for (int u = 0; u < 4; u++) xv[u] = xn[u];
+        lm += 4;
+        if (lm >= M) {
+            lm = 0;
+            li += NCT;
+        }
+        if (it + 1 < total) request();
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int m = m0 + u;
+            if (m >= M) break;
+            float v[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w};
+            if (norm) {
+                const float r = S.rstd[m];
+                v[0] = v[0] * r * (noff + w.x); v[1] = v[1] * r * (noff + w.y);
+                v[2] = v[2] * r * (noff + w.z); v[3] = v[3] * r * (noff + w.w);
+            }
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+            uint2 out = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            if (final_form) {
+                if (!bf16) {
+                    const __half2 a2 = __floats2half2_rn(bf_lo(out.x) * fscale, bf_hi(out.x) * fscale);
+                    const __half2 b2 = __floats2half2_rn(bf_lo(out.y) * fscale, bf_hi(out.y) * fscale);
+                    out = make_uint2(*reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&b2));
+                }
+            } else {
+                // magnitudes of bf16 values compare like their bits
+                const uint32_t a = max(max(out.x & 0x7FFFu, (out.x >> 16) & 0x7FFFu), max(out.y & 0x7FFFu, (out.y >> 16) & 0x7FFFu));
+                const uint32_t mx = __reduce_max_sync(0xffffffffu, a);
+                if (lane_() == 0) atomicMax(&S.xmax[m], (int)(mx << 16));
+            }
+            if (c4 < c4n) *reinterpret_cast<uint2*>(S.xs() + m * stride + c4 * 8) = out;
+        }
+    }
+    if (final_form) return;                                    // the caller's barrier publishes it
+    __syncwarp();
+    consumer_sync();
+    prof_mark(S, 5);
+    if (tid_() < M) S.xinv[tid_()] = __int_as_float((127 - scale_exponent(S.xmax[tid_()])) << 23);
+    // bf16 -> scaled fp16 in place, each thread its own column groups
+#pragma unroll 1
+    for (int c4 = tid_(); c4 < c4n; c4 += NCT) {
+#pragma unroll 4
+        for (int m = 0; m < M; m++) {
+            const float sc = __int_as_float((127 + scale_exponent(S.xmax[m])) << 23);
+            uint2* q = reinterpret_cast<uint2*>(S.xs() + m * stride + c4 * 8);
+            const uint2 b = *q;
+            const __half2 a2 = __floats2half2_rn(bf_lo(b.x) * sc, bf_hi(b.x) * sc), b2 = __floats2half2_rn(bf_lo(b.y) * sc, bf_hi(b.y) * sc);
+            *q = make_uint2(*reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&b2));
+        }
+    }
 }
 // (PLAIN: one piece, no adding up of groups: nearly every stage)
 template <bool PLAIN>
@@ -1147,9 +1280,9 @@ __device__ __forceinline__ bool multiply(Shared& S, const mk_stage_desc& d, cons
         {
             int sg = 0, grp = 0, tile = bt.t0 + tl;
             if (gm.reduce) {
-                sg = k / n_chunks;
+                sg = n_chunks == 1 ? k : k / n_chunks;
                 ke = (sg + 1) * n_chunks;
-                grp = (bt.seg0 + sg) / gm.S;
+                grp = gm.S == 1 ? bt.seg0 + sg : (bt.seg0 + sg) / gm.S;
                 f0 = S.coef[grp * 8 + 2 * (lane_() & 3)];
                 f1 = S.coef[grp * 8 + 2 * (lane_() & 3) + 1];
             } else if (tile >= gm.T) {
@@ -1293,7 +1426,8 @@ __device__ __forceinline__ void gemv_stage(Shared& S, const mk_stage_desc& d, co
         const Batch bt = geo_batch(gm, b);
         __syncwarp();
         if (b) consumer_sync();                                  // everybody is done with the staging area
-        if (d.i[MKS_I_PIECES] == 1 && !gm.reduce) stage_x<true>(S, d, bt.seg0, bt.seg1, bt.grp, gm.S);
+        if (d.i[MKS_I_PIECES] == 1 && !gm.reduce && S.A.M >= 4) stage_wide(S, d, bt.seg0, bt.seg1, bt.grp);
+        else if (d.i[MKS_I_PIECES] == 1 && !gm.reduce) stage_x<true>(S, d, bt.seg0, bt.seg1, bt.grp, gm.S);
         else stage_x<false>(S, d, bt.seg0, bt.seg1, bt.grp, gm.S);
         __syncwarp();
         consumer_sync();
