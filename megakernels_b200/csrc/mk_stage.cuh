@@ -290,26 +290,30 @@ __host__ __device__ __forceinline__ int max_panel_splits(int xs_bytes, int kc, i
 // panels: the weights of its tiles (whole chunks per warp count half: the other warps keep the memory busy); the input it
 // stages (every CTA reads its panel's fp32 columns from L2: about 0.12 ns a value); and with more than one panel the exchange:
 // one round trip through L2 (about 1.5 us) and 16-byte words of partial tiles, written once and read once.
-__host__ __device__ __forceinline__ u64 panel_cost(int R, int Q, int P, int n_chunks, int chunk_bytes, int kc, int M, int grid) {
-    const u64 tiles = ((u64)R * P + grid - 1) / grid, w = (Q + P - 1) / P;
-    const u64 chunks = tiles * w * n_chunks, even = (chunks + NCW - 1) / NCW * NCW;
-    return (chunks + even) / 2 * chunk_bytes + w * kc * M * 10 + (P > 1 ? 120000 + tiles * M * 256 : 0);
+// (In floats: the scout compares them while the CTA waits for a routed stage.)
+__host__ __device__ __forceinline__ float panel_cost(int R, int Q, int P, int n_chunks, int chunk_bytes, int kc, int M, int grid) {
+    const int tiles = (R * P + grid - 1) / grid, w = (Q + P - 1) / P;
+    const int chunks = tiles * w * n_chunks, even = (chunks + NCW - 1) / NCW * NCW;
+    return 0.5f * (float)(chunks + even) * (float)chunk_bytes + (float)(w * kc) * (float)M * 10.f + (P > 1 ? 120000.f + (float)(tiles * M) * 256.f : 0.f);
 }
 
 // Every lane of the scout calls this: the number of panels, from P0 (what the staging area allows) up to half the grid
 // (each panel then has a CTA).
 __device__ __forceinline__ int pick_panels(int R, int Q, int P0, int n_chunks, int chunk_bytes, int kc, int M, int grid) {
-    u64 best = ~0ull;
-    for (int P = P0 + lane_(); P <= min(Q, grid / 2); P += 32) {
-        const u64 k = panel_cost(R, Q, P, n_chunks, chunk_bytes, kc, M, grid) << 8 | (u64)P;
-        best = k < best ? k : best;
+    const int P1 = min(Q, grid / 2);
+    if (P0 >= P1) return P0 == P1 ? P0 : 0;
+    float best = 3.0e38f;
+    int at = 0;
+    for (int P = P0 + lane_(); P <= P1; P += 32) {
+        const float k = panel_cost(R, Q, P, n_chunks, chunk_bytes, kc, M, grid);
+        if (k < best) {
+            best = k;
+            at = P;
+        }
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
-        best = other < best ? other : best;
-    }
-    return best == ~0ull ? 0 : (int)(best & 255u);
+    __syncwarp();
+    const int low = __reduce_min_sync(0xffffffffu, __float_as_int(best));          // (positive floats compare like their bits)
+    return (int)__reduce_min_sync(0xffffffffu, __float_as_int(best) == low ? (unsigned)at : ~0u);
 }
 
 // One batch of a stage: a staged input (K splits [seg0, seg1) of a panel) and the tiles [t0, t1) it multiplies.
@@ -627,7 +631,7 @@ __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
                 }
                 if (P > 1 && panel >= 0) {
                     // panel p has the CTAs [grid q0 / Q, grid q1 / Q), q0 and q1 its first split and the next panel's
-                    panel = (int)((long long)cta * P / grid);
+                    panel = cta * P / grid;
                     auto first = [&](int p) { return (grid * (Q * p / P) + Q - 1) / Q; };
                     while (panel > 0 && first(panel) > cta) panel--;
                     while (panel + 1 < P && first(panel + 1) <= cta) panel++;
@@ -635,8 +639,8 @@ __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
                     nc = first(panel + 1) - c0;
                 }
                 const int k = cta - c0;
-                t0 = (int)((long long)R * k / nc);
-                t1 = (int)((long long)R * (k + 1) / nc);
+                t0 = (int)((unsigned)R * (unsigned)k / (unsigned)nc);   // (fewer than 2^24 units)
+                t1 = (int)((unsigned)R * (unsigned)(k + 1) / (unsigned)nc);
                 nb = t1 > t0 ? (panel < 0 ? P : 1) : 0;
             }
             if (lane_() == 0) {
@@ -680,6 +684,22 @@ __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
 // behind 1/rms.  And the size of the code: every stage runs through it once, at the speed of instruction fetch.
 constexpr int XB = 4;       // float4 groups per thread and round
 
+// 1/rms of sequence `warp` from the 16-element sums of squares of the whole input vector: all loads of a lane in flight
+// together (up to 8192 elements), added in a fixed order.
+__device__ __forceinline__ float row_rstd(const mk_stage_desc& d, int m) {
+    const int K = d.i[MKS_I_K_TOTAL], n16 = K / 16;
+    const float* row = reinterpret_cast<const float*>(d.p[MKS_P_X_SSQ]) + (size_t)m * n16;
+    float s = 0.f;
+#pragma unroll 1
+    for (int j0 = lane_(); j0 < n16; j0 += 512) {
+        float v[16];
+#pragma unroll
+        for (int u = 0; u < 16; u++) v[u] = j0 + 32 * u < n16 ? ldcg_f(row + j0 + 32 * u) : 0.f;
+#pragma unroll
+        for (int u = 0; u < 16; u++) s += v[u];
+    }
+    return rsqrtf(warp_sum(s) / (float)K + d.f[MKS_F_EPS]) * (d.f[MKS_F_IN_SCALE] != 0.f ? d.f[MKS_F_IN_SCALE] : 1.f);
+}
 // Exponent of the scale of a column whose largest magnitude has these bits: a = f * 2^e with f in [0.5, 1), the scale 2^(14 - e).
 __device__ __forceinline__ int scale_exponent(int bits) {
     const int e = bits > 0 && bits < 0x7f800000 ? ((bits >> 23) & 0xff) - 126 : 0;
@@ -719,13 +739,8 @@ __device__ __noinline__ void stage_wide(Shared& S, const mk_stage_desc& d, int s
     };
     request();
     if (norm && warp_() < M) {
-        const int K = d.i[MKS_I_K_TOTAL], n16 = K / 16;
-        const float* row = reinterpret_cast<const float*>(d.p[MKS_P_X_SSQ]) + (size_t)warp_() * n16;
-        float s = 0.f;
-#pragma unroll 8
-        for (int j = lane_(); j < n16; j += 32) s += ldcg_f(row + j);
-        s = warp_sum(s);
-        if (lane_() == 0) S.rstd[warp_()] = rsqrtf(s / (float)K + d.f[MKS_F_EPS]) * (d.f[MKS_F_IN_SCALE] != 0.f ? d.f[MKS_F_IN_SCALE] : 1.f);
+        const float r = row_rstd(d, warp_());
+        if (lane_() == 0) S.rstd[warp_()] = r;
     }
     __syncwarp();
     consumer_sync();
@@ -788,6 +803,54 @@ __device__ __noinline__ void stage_wide(Shared& S, const mk_stage_desc& d, int s
         }
     }
 }
+// Routed groups that are added up (an expert's down projection), one piece, no norm: few sequences give a group any weight, so
+// a warp takes one (K split, sequence) pair at a time, finds its scale by itself and leaves the other columns zero.  The
+// general staging below went through all of them: 11 us for the ten experts of a panel at eight sequences.
+__device__ __noinline__ void stage_routed(Shared& S, const mk_stage_desc& d, int seg0, int seg1, int n_splits) {
+    const int kc = d.i[MKS_I_KC], M = S.A.M, nseg = seg1 - seg0, stride = xs_stride_bytes(nseg * kc);
+    const bool bf16 = d.i[MKS_I_FMT] == MKS_FMT_BF16;
+    const float* x = reinterpret_cast<const float*>(d.p[MKS_P_X]);
+    for (int i = tid_(); i < M * stride / 16; i += NCT) reinterpret_cast<uint4*>(S.xs())[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid_() < nseg * 8) S.xinv[tid_()] = 1.f;
+    __syncwarp();
+    consumer_sync();
+    prof_mark(S, 4);
+#pragma unroll 1
+    for (int p = warp_(); p < nseg * M; p += NCW) {
+        const int sg = p / M, m = p - sg * M, grp = n_splits == 1 ? seg0 + sg : (seg0 + sg) / n_splits;
+        if (S.coef[grp * 8 + m] == 0.f) continue;
+        const float* src = x + (size_t)grp * d.i[MKS_I_X_GSTRIDE] + (size_t)m * d.i[MKS_I_X_STRIDE] + (size_t)(seg0 + sg - grp * n_splits) * kc;
+        uint8_t* dst = S.xs() + m * stride + sg * kc * 2;
+        uint32_t mx = 0;
+#pragma unroll 1
+        for (int e = lane_() * 4; e < kc; e += 512) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = e + u * 128 < kc ? __ldcg(reinterpret_cast<const float4*>(src + e + u * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(v[u].x, v[u].y), hi = __floats2bfloat162_rn(v[u].z, v[u].w);
+                const uint2 b = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                mx = max(max(mx, max(b.x & 0x7FFFu, (b.x >> 16) & 0x7FFFu)), max(b.y & 0x7FFFu, (b.y >> 16) & 0x7FFFu));   // magnitudes compare like their bits
+                if (e + u * 128 < kc) *reinterpret_cast<uint2*>(dst + (e + u * 128) * 2) = b;
+            }
+        }
+        __syncwarp();
+        if (!bf16) {
+            const int ex = scale_exponent((int)(__reduce_max_sync(0xffffffffu, mx) << 16));
+            const float sc = __int_as_float((127 + ex) << 23);
+            if (lane_() == 0) S.xinv[sg * 8 + m] = __int_as_float((127 - ex) << 23);
+#pragma unroll 2
+            for (int e = lane_() * 4; e < kc; e += 128) {      // the lane's own values
+                uint2* q = reinterpret_cast<uint2*>(dst + e * 2);
+                const uint2 b = *q;
+                const __half2 a2 = __floats2half2_rn(bf_lo(b.x) * sc, bf_hi(b.x) * sc), b2 = __floats2half2_rn(bf_lo(b.y) * sc, bf_hi(b.y) * sc);
+                *q = make_uint2(*reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&b2));
+            }
+        }
+        __syncwarp();
+    }
+}
 // (PLAIN: one piece, no adding up of groups: nearly every stage)
 template <bool PLAIN>
 __device__ __forceinline__ void stage_x(Shared& S, const mk_stage_desc& d, int seg0, int seg1, int grp0, int n_splits) {
@@ -848,17 +911,9 @@ __device__ __forceinline__ void stage_x(Shared& S, const mk_stage_desc& d, int s
             }
             if (first) {
                 first = false;
-                if (norm && warp_() < M) {
-                    // 1/rms of every sequence from the 16-element sums of squares of the whole input vector: warp m adds up
-                    // sequence m's sums (a lane's loads in flight together, fixed order) while the other warps only wait for x
-                    const int K = d.i[MKS_I_K_TOTAL], n16 = K / 16;
-                    const float* row = reinterpret_cast<const float*>(d.p[MKS_P_X_SSQ]) + (size_t)warp_() * n16;
-                    float s = 0.f;
-#pragma unroll 8
-                    for (int j = lane_(); j < n16; j += 32) s += ldcg_f(row + j);
-                    s = warp_sum(s);
-                    if (lane_() == 0)
-                        S.rstd[warp_()] = rsqrtf(s / (float)K + d.f[MKS_F_EPS]) * (d.f[MKS_F_IN_SCALE] != 0.f ? d.f[MKS_F_IN_SCALE] : 1.f);
+                if (norm && warp_() < M) {                         // while the other warps only wait for x
+                    const float r = row_rstd(d, warp_());
+                    if (lane_() == 0) S.rstd[warp_()] = r;
                 }
                 __syncwarp();
                 consumer_sync();
@@ -1427,6 +1482,7 @@ __device__ __forceinline__ void gemv_stage(Shared& S, const mk_stage_desc& d, co
         __syncwarp();
         if (b) consumer_sync();                                  // everybody is done with the staging area
         if (d.i[MKS_I_PIECES] == 1 && !gm.reduce && S.A.M >= 4) stage_wide(S, d, bt.seg0, bt.seg1, bt.grp);
+        else if (d.i[MKS_I_PIECES] == 1 && gm.reduce && d.i[MKS_I_PROLOGUE] != MKS_P_NORM) stage_routed(S, d, bt.seg0, bt.seg1, gm.S);
         else if (d.i[MKS_I_PIECES] == 1 && !gm.reduce) stage_x<true>(S, d, bt.seg0, bt.seg1, bt.grp, gm.S);
         else stage_x<false>(S, d, bt.seg0, bt.seg1, bt.grp, gm.S);
         __syncwarp();

@@ -105,9 +105,9 @@ static int64_t scratch_bytes(const mk_stage_desc* prog, int n_stages, int batch)
             const int R = reduce ? d.i[MKS_I_TILES] : d.i[MKS_I_TILES] * G, Q = reduce ? d.i[MKS_I_SPLITS] * G : d.i[MKS_I_SPLITS];
             const int w = max_panel_splits(XS_BYTES, kc, ncols, d.i[MKS_I_PIECES], reduce), P0 = (Q + w - 1) / w;
             int P = P0;
-            uint64_t best = ~0ull;
+            float best = 3.0e38f;
             for (int p = P0; p <= Q && p <= 148 / 2; p++) {
-                const uint64_t k = panel_cost(R, Q, p, d.i[MKS_I_UNIT_STEPS] / d.i[MKS_I_CHUNK_STEPS], d.i[MKS_I_CHUNK_BYTES], kc, batch, 148);
+                const float k = panel_cost(R, Q, p, d.i[MKS_I_UNIT_STEPS] / d.i[MKS_I_CHUNK_STEPS], d.i[MKS_I_CHUNK_BYTES], kc, batch, 148);
                 if (k < best) { best = k; P = p; }
             }
             b = (int64_t)xs_stride_bytes((Q + P - 1) / P * kc) * ncols;

@@ -881,35 +881,33 @@ __device__ __noinline__ void route_stage(Shared& S, const mk_stage_desc& d) {
     consumer_sync();
     if (warp_() < S.A.M && S.valid_s[warp_()]) {              // a padding row selects no expert
         const int m = warp_();
-        float v[8];
-        bool used[8];
+        // a score as an unsigned word in the same order (0: taken, or none): one reduction finds the best, a second the lowest id
         const int per = E / 32;                                   // 8 (256 experts) or 4 (128)
+        float v[8];
+        uint32_t key[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = i < per ? ldcg_f(logits + (size_t)m * stride + lane_() + 32 * i) : 0.f;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            v[i] = i < per ? ldcg_f(logits + (size_t)m * stride + lane_() + 32 * i) : 0.f;
-            used[i] = i >= per;
+            const uint32_t b = __float_as_uint(v[i] == 0.f ? 0.f : v[i]);                    // (-0 and 0 are equal scores)
+            key[i] = i < per ? max((b & 0x80000000u) ? ~b : b | 0x80000000u, 1u) : 0u;
         }
         float top0 = 0.f, wsum = 0.f, myw = 0.f;
 #pragma unroll 1
         for (int k = 0; k < topk; k++) {
-            u64 best = 0;
+            uint32_t mine = key[0];
+#pragma unroll
+            for (int i = 1; i < 8; i++) mine = max(mine, key[i]);
+            const uint32_t best = __reduce_max_sync(0xffffffffu, mine);
+            unsigned at = ~0u;
+#pragma unroll
+            for (int i = 7; i >= 0; i--)
+                if (key[i] == best) at = (unsigned)(lane_() + 32 * i);
+            const int id = min((int)__reduce_min_sync(0xffffffffu, at), E - 1);
 #pragma unroll
             for (int i = 0; i < 8; i++)
-                if (!used[i]) {
-                    const u64 key = score_key(v[i], lane_() + 32 * i);
-                    best = key > best ? key : best;
-                }
-            best = warp_max_u64(best);
-            int id = key_index(best);
-            id = max(0, min(E - 1, id));
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-                if (lane_() + 32 * i == id) used[i] = true;
-            float mine = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-                if (i == (id >> 5)) mine = v[i];
-            const float sc = __shfl_sync(0xffffffffu, mine, id & 31);
+                if (lane_() + 32 * i == id) key[i] = 0u;
+            const float sc = __uint_as_float((best & 0x80000000u) ? best & 0x7FFFFFFFu : ~best);
             if (k == 0) top0 = sc;
             const float w = __expf(sc - top0);
             wsum += w;
@@ -919,6 +917,7 @@ __device__ __noinline__ void route_stage(Shared& S, const mk_stage_desc& d) {
                 atomicOr(&S.gmask[id >> 5], 1u << (id & 31));
             }
         }
+        __syncwarp();
         if (lane_() < topk) {
             const int id = S.r_ids[m * 8 + lane_()];
             S.r_w[m * 8 + lane_()] = myw / wsum * (kind == 1 && pes ? pes[id] : 1.f);
@@ -964,6 +963,20 @@ __device__ __noinline__ void vec_stage(Shared& S, const mk_stage_desc& d) {
     float* out_ssq = reinterpret_cast<float*>(d.p[MKS_P_VEC_OUT_SSQ]);
     const float eps = d.f[MKS_F_EPS], off = d.f[MKS_F_NORM_OFF];
     const float scale = d.f[MKS_F_SCALE] != 0.f ? d.f[MKS_F_SCALE] : 1.f;
+    const int g0 = ng * cta_() / grid_(), g1 = ng * (cta_() + 1) / grid_();
+    const int n = g1 - g0;
+    // the first round's terms are requested before the sums of squares are added up
+    float4 av = make_float4(0.f, 0.f, 0.f, 0.f), bv = av, hv = av;
+    auto request = [&](int idx) {
+        if (idx < n * M * 4) {
+            const int gi = idx >> 2, m = gi / n;
+            const size_t o = (size_t)m * N + (g0 + gi - m * n) * 16 + (idx & 3) * 4;
+            av = __ldcg(reinterpret_cast<const float4*>(a + o));
+            if (b) bv = __ldcg(reinterpret_cast<const float4*>(b + o));
+            if (base) hv = __ldcg(reinterpret_cast<const float4*>(base + o));
+        }
+    };
+    request(tid_());
     // warps 0..M-1: rstd of a; warps 8..8+M-1: rstd of b
     {
         const int m = warp_() & 7;
@@ -971,17 +984,23 @@ __device__ __noinline__ void vec_stage(Shared& S, const mk_stage_desc& d) {
         const float* ssq = reinterpret_cast<const float*>(d.p[second ? MKS_P_VEC_B_SSQ : MKS_P_VEC_A_SSQ]);
         if (m < M && (!second || b)) {
             float s = 0.f;
-#pragma unroll 4
-            for (int j = lane_(); j < ng; j += 32) s += ldcg_f(ssq + (size_t)m * ng + j);
+#pragma unroll 1
+            for (int j0 = lane_(); j0 < ng; j0 += 256) {
+                float v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = j0 + 32 * u < ng ? ldcg_f(ssq + (size_t)m * ng + j0 + 32 * u) : 0.f;
+#pragma unroll
+                for (int u = 0; u < 8; u++) s += v[u];
+            }
             s = warp_sum(s);
             if (lane_() == 0) S.red[(second ? 8 : 0) + m] = rsqrtf(s / (float)N + eps);
         }
     }
+    __syncwarp();
     consumer_sync();
-    const int g0 = ng * cta_() / grid_(), g1 = ng * (cta_() + 1) / grid_();
-    const int n = g1 - g0;
 #pragma unroll 1
     for (int idx0 = 0; idx0 < n * M * 4; idx0 += NCT) {
+        if (idx0) request(idx0 + tid_());
         // four threads share a 16-element group: each takes a float4 and the group's sum of squares is shuffled together
         // (every lane of a warp takes part in the shuffles; the ones past the end carry zeros)
         const int idx = idx0 + tid_();
@@ -991,18 +1010,15 @@ __device__ __noinline__ void vec_stage(Shared& S, const mk_stage_desc& d) {
         const size_t o = (size_t)m * N + grp * 16 + q4 * 4;
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
         if (live) {
-            const float4 av = __ldcg(reinterpret_cast<const float4*>(a + o));
             const float4 aw = __ldg(reinterpret_cast<const float4*>(wa + grp * 16 + q4 * 4));
             const float ra = S.red[m];
             r = make_float4(av.x * ra * (off + aw.x), av.y * ra * (off + aw.y), av.z * ra * (off + aw.z), av.w * ra * (off + aw.w));
             if (b) {
-                const float4 bv = __ldcg(reinterpret_cast<const float4*>(b + o));
                 const float4 bw = __ldg(reinterpret_cast<const float4*>(wb + grp * 16 + q4 * 4));
                 const float rb = S.red[8 + m];
                 r.x += bv.x * rb * (off + bw.x); r.y += bv.y * rb * (off + bw.y); r.z += bv.z * rb * (off + bw.z); r.w += bv.w * rb * (off + bw.w);
             }
             if (base) {
-                const float4 hv = __ldcg(reinterpret_cast<const float4*>(base + o));
                 r.x += hv.x; r.y += hv.y; r.z += hv.z; r.w += hv.w;
             }
             r.x *= scale; r.y *= scale; r.z *= scale; r.w *= scale;
