@@ -100,7 +100,7 @@ struct Geo {
 // A warp's share of a batch: chunks [c, c1), tile by tile.
 struct Share {
     const uint8_t* src;            // chunk c
-    int c, c1, n;                  // and all of the batch's chunks
+    int c, c1, per;                // per: chunks of every warp's share but the last ones'
     int cpt, tl, k;                // chunks of one tile; chunk c as tile of the batch and chunk of the tile
 };
 // The stream's registers (the same in every lane but for what is said to be the lane's own).
@@ -375,13 +375,18 @@ __device__ __forceinline__ const uint8_t* split_weights(const Shared& S, const G
     }
     return group_weights(S, g, grp) + (size_t)((tile * g.S + seg) * g.n_chunks) * g.chunk_bytes;
 }
-// Warp w's share of batch b.
+constexpr int FEW_WARPS = 4;
+// Warp w's share of a batch.
 __device__ __forceinline__ Share batch_share(const Shared& S, const Geo& g, const Batch& bt, int w) {
     Share r;
     r.cpt = (bt.seg1 - bt.seg0) * g.n_chunks;
-    r.n = (bt.t1 - bt.t0) * r.cpt;
-    r.c = r.n * w / NCW;
-    r.c1 = r.n * (w + 1) / NCW;
+    // Equal shares of whole chunks, the first warps first: as long as the longest share is no longer, every warp without one
+    // is a partial tile less to add.  Fewer chunks than warps go to FEW_WARPS: two or three chunks in a row cost less than
+    // the exchange (27B x1 per step 1417 -> 1382 us, 35B-A3B x8 1531 -> 1494 us).
+    const int n = (bt.t1 - bt.t0) * r.cpt, warps = n < NCW && n > FEW_WARPS ? FEW_WARPS : NCW;
+    r.per = (n + warps - 1) / warps;
+    r.c = min(n, w * r.per);
+    r.c1 = min(n, r.c + r.per);
     r.tl = r.c / r.cpt;
     r.k = r.c - r.tl * r.cpt;
     const int sg = r.k / g.n_chunks;
@@ -1098,7 +1103,7 @@ __device__ __forceinline__ float2 lds_f2(uint32_t a) {
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
     return v;
 }
-// One tile step: accumulates into acc / acc2 (two chains: consecutive MMAs never wait for each other).
+// One tile step: accumulates into acc / acc2 (two chains where a warp's own MMAs would wait for each other).
 template <int FMT>
 __device__ __forceinline__ void tile_step(uint32_t sl, uint32_t sc, int st, const uint8_t* xk, float (&acc)[4], float (&acc2)[4]) {
     const uint4 wq = lds_u4(sl);
@@ -1159,7 +1164,7 @@ __device__ __forceinline__ void tile_step(uint32_t sl, uint32_t sc, int st, cons
             a[1] = cvt_e4m3x2(hi);
             a[3] = cvt_e4m3x2(hi >> 16);
             const uint2 b = *reinterpret_cast<const uint2*>(xk + j * 32);
-            mma_f16(j == 0 ? acc : acc2, a, b.x, b.y);
+            mma_f16(acc, a, b.x, b.y);
         }
     } else if (FMT == MKS_FMT_INT8) {
         const uint32_t x0 = wq.x ^ 0x80808080u, x1 = wq.y ^ 0x80808080u, x2 = wq.z ^ 0x80808080u, x3 = wq.w ^ 0x80808080u;
@@ -1177,7 +1182,7 @@ __device__ __forceinline__ void tile_step(uint32_t sl, uint32_t sc, int st, cons
     } else {
         uint32_t a[4] = {wq.x, wq.z, wq.y, wq.w};                 // row g: (x, y), row g + 8: (z, w)
         const uint2 b = *reinterpret_cast<const uint2*>(xk);
-        if (st & 1) mma_bf16(acc2, a, b.x, b.y);
+        if (st & 2) mma_bf16(acc2, a, b.x, b.y);
         else mma_bf16(acc, a, b.x, b.y);
     }
 }
@@ -1459,7 +1464,7 @@ __device__ __forceinline__ bool multiply(Shared& S, const mk_stage_desc& d, cons
     consumer_sync();
     if (k > 0 && c == c1 && c > sh.c && ok) {
         // the warps behind this one, up to the one that has the tile's last chunk
-        const int last = (16 * ((tl + 1) * cpt - 1) + 15) / sh.n;
+        const int last = ((tl + 1) * cpt - 1) / sh.per;
 #pragma unroll 4
         for (int v = warp_() + 1; v <= last; v++) {
             const float4 x = tiles[v * 32];
