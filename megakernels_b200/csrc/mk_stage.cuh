@@ -387,6 +387,12 @@ __device__ __forceinline__ Share batch_share(const Shared& S, const Geo& g, cons
     r.per = (n + warps - 1) / warps;
     r.c = min(n, w * r.per);
     r.c1 = min(n, r.c + r.per);
+    if (g.routed && !g.reduce) {
+        // many tiles of many experts: cut as evenly as chunks allow (per < 0: minus all of the batch's chunks)
+        r.per = -n;
+        r.c = n * w / NCW;
+        r.c1 = n * (w + 1) / NCW;
+    }
     r.tl = r.c / r.cpt;
     r.k = r.c - r.tl * r.cpt;
     const int sg = r.k / g.n_chunks;
@@ -1464,7 +1470,7 @@ __device__ __forceinline__ bool multiply(Shared& S, const mk_stage_desc& d, cons
     consumer_sync();
     if (k > 0 && c == c1 && c > sh.c && ok) {
         // the warps behind this one, up to the one that has the tile's last chunk
-        const int last = ((tl + 1) * cpt - 1) / sh.per;
+        const int end = (tl + 1) * cpt - 1, last = sh.per > 0 ? end / sh.per : (NCW * end + NCW - 1) / -sh.per;
 #pragma unroll 4
         for (int v = warp_() + 1; v <= last; v++) {
             const float4 x = tiles[v * 32];
