@@ -35,6 +35,8 @@ MAX_STEPS_PER_LAUNCH = 1024
 # Prompt tokens from which the token-parallel path takes a prompt in: it passes over the weights once (about 2 ms with its
 # launches) where stepping costs 0.4 ms per token.  Shorter ones keep the step path and its bits.
 MIN_PROMPT_ROWS = 16
+# ... and a run that returns logits keeps prompts up to this long on the step path: its logits are those of `mk_launch`.
+EXACT_PROMPT = 96
 # Positions of one pass of that path: bounds its workspace (about 150 KB per position).
 MAX_PROMPT_ROWS = 4096
 
@@ -429,7 +431,8 @@ class Megakernel:
         hidden = torch.empty(n_steps, cfg.hidden, device=dev) if want_hidden else None
         # a long prompt goes in all at once, except its last token (whoever wants logits or times per token gets steps)
         taken = 0
-        if n_given > MIN_PROMPT_ROWS and not all_logits and not timing and prof is None:
+        # (a caller who asks for logits gets those of `mk_launch`, bit for bit, up to EXACT_PROMPT tokens)
+        if n_given > (max(EXACT_PROMPT, MIN_PROMPT_ROWS) if return_logits else MIN_PROMPT_ROWS) and not all_logits and not timing and prof is None:
             taken = n_given - 1
             self._take_in(given[:taken], self.pos, hidden)
             self.pos += taken
