@@ -604,9 +604,13 @@ __device__ __noinline__ void attn_stage(Shared& S, const mk_stage_desc& d) {
 //     of a lane's 16 bytes spread over eight MMAs; pairs of positions are put together with byte permutes;
 //   * 256 positions at a time with a running maximum; one CTA barrier per 256.
 constexpr int ATTN_SUB = 256;             // positions between two barriers: one tile per warp
+// Buffers of cache-row offsets.  Sub-chunk s + 1's are written between the barriers of s - 1 and s, when a slower warp still
+// reads s - 1's for its V rows and every warp reads s's for its scores: three.  (Scores and maxima are written and read on
+// either side of their own barrier: two.)
+constexpr int ATTN_ROWS = 3;
 __host__ __device__ __forceinline__ int attn_mma_bytes(int QPK, int HD) {
-    // q fp32 [QPK][HD] | new K, V rows | q bf16 [8][HD + 8] | scores [2][8][ATTN_SUB + 4] | tile maxima [2][8][16] | rows [2][ATTN_SUB]
-    const int a = QPK * HD * 4 + 2 * HD * 4 + 8 * (HD + 8) * 2 + 2 * 8 * (ATTN_SUB + 4) * 4 + 2 * 8 * 16 * 4 + 2 * ATTN_SUB * 4;
+    // q fp32 [QPK][HD] | new K, V rows | q bf16 [8][HD + 8] | scores [2][8][ATTN_SUB + 4] | tile maxima [2][8][16] | rows [ATTN_ROWS][ATTN_SUB]
+    const int a = QPK * HD * 4 + 2 * HD * 4 + 8 * (HD + 8) * 2 + 2 * 8 * (ATTN_SUB + 4) * 4 + 2 * 8 * 16 * 4 + ATTN_ROWS * ATTN_SUB * 4;
     // at the end: output pieces [16 warps][8][64] | sums [4][8] | merge weights
     const int b = NCW * 8 * 64 * 4 + 4 * 8 * 4 + 8 * ATTN_MAX_CHUNKS * 4;
     return a > b ? a : b;
@@ -634,7 +638,7 @@ __device__ __noinline__ void attn_mma_stage(Shared& S, const mk_stage_desc& d) {
     const int qb_stride = (HD + 8) * 2;
     float* sc_s = reinterpret_cast<float*>(qb + 8 * qb_stride);   // [2][8][ATTN_SUB + 4]
     float* wm_s = sc_s + 2 * 8 * (ATTN_SUB + 4);               // [2][8][16]
-    uint32_t* row_s = reinterpret_cast<uint32_t*>(wm_s + 2 * 8 * 16);   // [2][ATTN_SUB] element offsets of the cache rows
+    uint32_t* row_s = reinterpret_cast<uint32_t*>(wm_s + 2 * 8 * 16);   // [ATTN_ROWS][ATTN_SUB] element offsets of the cache rows
     const int g = lane_() >> 2, t = lane_() & 3;
     const int ndg = HD / 64, nres = NCW / ndg, dg = warp_() % ndg, res = warp_() / ndg;
     int maxn = 1;
@@ -663,7 +667,7 @@ __device__ __noinline__ void attn_mma_stage(Shared& S, const mk_stage_desc& d) {
         // cache rows of sub-chunk `sub` (past the end: its last row), by `nt` threads from `t0`; the first touch of a page after
         // the weight stream costs microseconds (TLB), so one line per cache block is requested as soon as it is known
         auto rows = [&](int sub, int i0, int step) {
-            uint32_t* r = row_s + (sub & 1) * ATTN_SUB;
+            uint32_t* r = row_s + (sub % ATTN_ROWS) * ATTN_SUB;
 #pragma unroll 1
             for (int i = i0; i < ATTN_SUB; i += step) {
                 const int p = min(first + sub * ATTN_SUB + i, last - 1);
@@ -713,7 +717,7 @@ __device__ __noinline__ void attn_mma_stage(Shared& S, const mk_stage_desc& d) {
 #pragma unroll 1
         for (int sub = 0; sub < nsub; sub++) {
             const int ns = min(ATTN_SUB, np - sub * ATTN_SUB), ntile = (ns + 15) >> 4;
-            const uint32_t* row = row_s + (sub & 1) * ATTN_SUB;
+            const uint32_t* row = row_s + (sub % ATTN_ROWS) * ATTN_SUB;
             float* sc = sc_s + (sub & 1) * 8 * (ATTN_SUB + 4);
             float* wm = wm_s + (sub & 1) * 8 * 16;
             {
