@@ -105,10 +105,11 @@ struct Share {
 };
 // The stream's registers (the same in every lane but for what is said to be the lane's own).
 struct Feed {
-    const uint8_t* src;            // next step of the current chunk (of the whole run, where chunks carry no scales); this lane's bytes
+    const uint8_t* src;            // next step of the current chunk (of the whole run, where chunks are steps alone); this lane's bytes
     int steps, left;               // steps left in it, chunks left in the run behind it
     int eoff;                      // from src to the scales of that step (this lane's)
     int ebps, cs;                  // scale bytes per step, steps per chunk
+    int gap;                       // bytes from a chunk's last step to the next chunk: its scales and padding
     int ahead;                     // blocks requested and not yet multiplied
     uint32_t rd;                   // shared-memory address of the next block to multiply (this lane's part)
 };
@@ -491,7 +492,7 @@ __device__ __noinline__ bool next_run(Shared& S) {
     return left > 0;
 }
 __device__ __forceinline__ void next_chunk(Feed& f) {
-    f.src += f.cs * f.ebps;                                    // past the scales of the chunk before
+    f.src += f.gap;
     f.left--;
     f.steps = f.cs;
     f.eoff = f.cs * 512 - lane_() * 12;
@@ -510,9 +511,10 @@ __device__ __forceinline__ void feed(Shared& S, Feed& f, int depth, uint32_t rin
                 if (!next_run(S)) break;
                 const Cur& c = S.cur[warp_()];
                 f.ebps = c.ebps;
-                f.cs = f.ebps ? c.chunk_steps : c.chunk_steps * c.left;
-                f.left = f.ebps ? c.left : 1;
-                f.src = c.src + lane_() * 16 - f.cs * f.ebps;
+                f.gap = c.chunk_bytes - c.chunk_steps * 512;
+                f.cs = f.gap ? c.chunk_steps : c.chunk_steps * c.left;
+                f.left = f.gap ? c.left : 1;
+                f.src = c.src + lane_() * 16 - f.gap;
                 next_chunk(f);
             }
         }
@@ -1370,8 +1372,8 @@ __device__ __forceinline__ bool multiply(Shared& S, const mk_stage_desc& d, cons
             float tot[4] = {0.f, 0.f, 0.f, 0.f};                // block-scaled FP8: the sum over 128-column blocks
             // lanes beyond the staged columns read a live one (their accumulators are never used): predicated zeros cost a tenth of the loop
             const uint8_t* xk = S.xs() + min(lane_() >> 2, S.A.M * d.i[MKS_I_PIECES] - 1) * stride + (lane_() & 3) * 8 + k * chunk_steps * STEP_BYTES;
-            // the stream's blocks end where a chunk with scales, or a run of chunks, ends
-            int steps = run * chunk_steps, in = scales ? chunk_steps : steps;
+            // the stream's blocks end where a chunk with scales or padding, or a run of chunks, ends
+            int steps = run * chunk_steps, in = gm.chunk_bytes != chunk_steps * 512 ? chunk_steps : steps;
             const uint32_t sc_off = BLOCK_STEPS * 512 - lane_() * 16 + (lane_() >> 2) * 4;
 #pragma unroll 1
             while (steps > 0) {

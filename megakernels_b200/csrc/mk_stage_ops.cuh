@@ -1064,7 +1064,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) stage_kernel(const __grid_constan
     if (warp_() < NCW && lane_() == 0) {
         Cur& c = S.cur[warp_()];
         c.src = nullptr; c.left = c.rest = c.run = c.ebps = 0; c.gn = c.now = 0; c.b = 0; c.nb = 0;
-c.f.src = nullptr; c.f.steps = c.f.left = c.f.eoff = c.f.ebps = c.f.cs = c.f.ahead = 0;
+        c.f.src = nullptr; c.f.steps = c.f.left = c.f.eoff = c.f.ebps = c.f.cs = c.f.gap = c.f.ahead = 0;
         c.f.rd = smem_u32(smem_raw + MISC_BYTES + A_in.xs_bytes) + warp_() * A_in.ring_depth * BLOCK_BYTES;
     }
     __syncthreads();

@@ -34,7 +34,7 @@ def _weights(fmt, N, K, seed, block=False):
     return wq, kw, rs, deq.double()
 
 
-def _run(fmt, N, K, M, splits, *, block=False, prologue="plain", epilogue="store", seed=0, softcap=0.0, act="silu"):
+def _run(fmt, N, K, M, splits, *, block=False, prologue="plain", epilogue="store", seed=0, softcap=0.0, act="silu", chunk_pad=0):
     dev = torch.device("cuda", 0)
     grid = torch.cuda.get_device_properties(dev).multi_processor_count
     glu = epilogue == "glu"
@@ -42,6 +42,10 @@ def _run(fmt, N, K, M, splits, *, block=False, prologue="plain", epilogue="store
     wq, kw, rs, deq = _weights(fmt, rows, K, seed, block)
     order = P.glu_row_order(N) if glu else None
     packed, meta = P.pack_matrix(fmt, splits, wq, row_order=order, **kw)
+    if chunk_pad:                                        # the record's chunk_bytes may exceed the chunk's contents
+        chunks = packed.reshape(-1, meta["chunk_bytes"])
+        packed = torch.cat([chunks, torch.full((chunks.shape[0], chunk_pad), 0x7F, dtype=torch.uint8, device=dev)], 1).reshape(-1)
+        meta = dict(meta, chunk_bytes=meta["chunk_bytes"] + chunk_pad, bytes=packed.numel())
     if rs is not None and order is not None:
         rs = rs[order.cuda()].contiguous()
     if rs is not None and rs.numel() < meta["tiles"] * 16:
@@ -128,6 +132,20 @@ def test_norm_prologue_and_residual_epilogue(fmt, block):
 def test_glu_epilogue(fmt, block, act):
     out, want, *_ = _run(fmt, 768, 1024, 2, 2, block=block, prologue="norm", epilogue="glu", act=act, seed=7)
     assert float((out.double() - want).abs().max()) <= _tol(want) + 1e-3 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("kc", [384, 640])
+@pytest.mark.parametrize("M,splits", [(3, 1), (8, 5)])
+def test_block_scaled_chunks_of_four_steps(kc, M, splits):
+    """An odd number of 128-column blocks per split: chunks of four steps, whose 2056 bytes are padded to 2064."""
+    out, want, *_ = _run(P.FMT_FP8, 640, kc * splits, M, splits, block=True, seed=15)
+    assert float((out.double() - want).abs().max()) <= _tol(want)
+
+
+@pytest.mark.parametrize("fmt,block", FORMATS, ids=IDS)
+def test_chunks_with_padding(fmt, block):
+    out, want, *_ = _run(fmt, 640, 1536, 3, 2, block=block, seed=17, chunk_pad=48)
+    assert float((out.double() - want).abs().max()) <= _tol(want)
 
 
 @pytest.mark.parametrize("softcap", [0.0, 30.0])
