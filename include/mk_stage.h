@@ -165,8 +165,8 @@ enum {
     MKS_P_OUT,
     MKS_P_OUT_SSQ,       /* E_RESID: fp32 [M][N/16]                                                */
     MKS_P_CNT,           /* u32 [output tiles] (per group unless REDUCE_GROUPS): not read, kept for the record's layout */
-    MKS_P_PART,          /* u64 partial tiles [output tile][K split][16 x 8], zero before the first launch: a value and the
-                            launch's tag in one word                                               */
+    MKS_P_PART,          /* u64 partial tiles [output tile][K split][16 x 8], zero before the first launch: a value and a
+                            tag of the launch's own in one word                                    */
     MKS_P_KEYS,          /* E_LOGITS: u64 [M][grid] best (score, ~row) key of every CTA            */
     MKS_P_ROW_BASE,      /* E_LOGITS: first vocabulary row of this rank (a value)                  */
     MKS_P_W_BYTES,       /* bytes of one group's matrix (a value; 0: unchecked): a copy that would leave it

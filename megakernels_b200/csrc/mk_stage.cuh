@@ -75,6 +75,8 @@ struct Args {
     int prof_cta;            // the CTA whose timestamps go to `prof`
     int xs_bytes;            // input staging / mixer scratch area of this launch
     int ring_depth;          // ring slots per consumer warp
+    uint32_t tile_tag;       // tag of this launch's first partial tiles
+    int clear_tiles;         // 1: words of partial tiles are left zero (a captured launch, which runs again with the same tags)
 };
 
 // Everything the threads of a CTA share lives in shared memory, behind the ring and the input staging
@@ -1196,9 +1198,19 @@ __device__ __forceinline__ void tile_step(uint32_t sl, uint32_t sc, int st, cons
 }
 
 // Partial tiles of a stage with several panels: [tile][panel][8 sequences][8 row pairs][2] words (value | tag << 32); only
-// live sequences' columns are written and read.
+// live sequences' columns are written and read.  A launch's tags are its own (the host counts them over all launches, apart
+// from the barrier counter, which a caller may start over); a captured launch runs again with the same ones, so there the
+// words are left zero, which no tag is (cleared in every launch: 1 to 2.5 % of a step).
 __device__ __forceinline__ unsigned long long* tile_words(unsigned long long* part, int tile_panel) {
     return part + (size_t)tile_panel * 128 + (lane_() & 3) * 32 + (lane_() >> 2) * 2;
+}
+__device__ __noinline__ void clear_tile(Shared& S, unsigned long long* src, int P) {
+    const int m0 = 2 * (lane_() & 3);
+#pragma unroll 1
+    for (int p = 0; p < P; p++, src += 128) {
+        if (m0 < S.A.M) __stcg(reinterpret_cast<ulonglong2*>(src), make_ulonglong2(0ull, 0ull));
+        if (m0 + 1 < S.A.M) __stcg(reinterpret_cast<ulonglong2*>(src + 16), make_ulonglong2(0ull, 0ull));
+    }
 }
 __device__ __forceinline__ void publish_tile(unsigned long long* dst, uint32_t tag, int M, const float (&v)[4]) {
     chaos_delay();
@@ -1511,8 +1523,10 @@ __device__ __forceinline__ void gemv_stage(Shared& S, const mk_stage_desc& d, co
 #pragma unroll 1
         for (int tl = first + warp_() * step; tl < gm.t1 && ok; tl += NCW * step) {
             float sum[4];
-            ok = collect_tile(S, tile_words(reinterpret_cast<unsigned long long*>(d.p[MKS_P_PART]), tl * gm.P), tag, gm.P, sum) &&
-                 finish_tile(S, d, ar_seq, tl, make_float4(sum[0], sum[1], sum[2], sum[3]));
+            unsigned long long* words = tile_words(reinterpret_cast<unsigned long long*>(d.p[MKS_P_PART]), tl * gm.P);
+            ok = collect_tile(S, words, tag, gm.P, sum);
+            if (ok && S.A.clear_tiles) clear_tile(S, words, gm.P);
+            ok = ok && finish_tile(S, d, ar_seq, tl, make_float4(sum[0], sum[1], sum[2], sum[3]));
         }
     }
     __syncwarp();

@@ -1,4 +1,5 @@
 // C ABI of the stage-machine megakernel (declarations and reference citations: include/mk_stage.h).
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -202,6 +203,12 @@ extern "C" int mk_stage_launch(const mk_stage_args* a, void* stream) {
     if (depth < MIN_RING_DEPTH) return sfail(MK_ERR_BADARG, "mk_stage_launch: no room for %d ring slots per warp", MIN_RING_DEPTH);
     A.xs_bytes = xs;
     A.ring_depth = depth;
+    // Tags of partial tiles: no two launches of a process share one (a stage's is tile_tag + the barriers passed before it).
+    static std::atomic<uint32_t> next_tag{1};
+    A.tile_tag = next_tag.fetch_add((uint32_t)a->n_steps * (uint32_t)a->n_stages + 1u, std::memory_order_relaxed);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capture) != cudaSuccess) (void)cudaGetLastError();     // (then the launch says why)
+    A.clear_tiles = capture != cudaStreamCaptureStatusNone;
 
     const int smem = MISC_BYTES + xs + 16 * depth * BLOCK_BYTES;
     MKS_CUDA(cudaFuncSetAttribute(stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

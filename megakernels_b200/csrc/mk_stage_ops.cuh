@@ -1113,10 +1113,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) stage_kernel(const __grid_constan
                 case MKS_OP_GEMV:
                     if (d.i[MKS_I_ALLREDUCE] != 0 && A.tp > 1) ar_seq++;
                     switch (d.i[MKS_I_FMT]) {
-                        case MKS_FMT_MXFP4: gemv_stage<MKS_FMT_MXFP4>(S, d, S.geo[n % GEO_RING], ar_seq, S.tag0 + (uint32_t)bar_n + 1u, n); break;
-                        case MKS_FMT_FP8: gemv_stage<MKS_FMT_FP8>(S, d, S.geo[n % GEO_RING], ar_seq, S.tag0 + (uint32_t)bar_n + 1u, n); break;
-                        case MKS_FMT_INT8: gemv_stage<MKS_FMT_INT8>(S, d, S.geo[n % GEO_RING], ar_seq, S.tag0 + (uint32_t)bar_n + 1u, n); break;
-                        default: gemv_stage<MKS_FMT_BF16>(S, d, S.geo[n % GEO_RING], ar_seq, S.tag0 + (uint32_t)bar_n + 1u, n); break;
+                        case MKS_FMT_MXFP4: gemv_stage<MKS_FMT_MXFP4>(S, d, S.geo[n % GEO_RING], ar_seq, max(A.tile_tag + (uint32_t)bar_n, 1u), n); break;
+                        case MKS_FMT_FP8: gemv_stage<MKS_FMT_FP8>(S, d, S.geo[n % GEO_RING], ar_seq, max(A.tile_tag + (uint32_t)bar_n, 1u), n); break;
+                        case MKS_FMT_INT8: gemv_stage<MKS_FMT_INT8>(S, d, S.geo[n % GEO_RING], ar_seq, max(A.tile_tag + (uint32_t)bar_n, 1u), n); break;
+                        default: gemv_stage<MKS_FMT_BF16>(S, d, S.geo[n % GEO_RING], ar_seq, max(A.tile_tag + (uint32_t)bar_n, 1u), n); break;
                     }
                     break;
                 case MKS_OP_GDN: gdn_stage(S, d); break;

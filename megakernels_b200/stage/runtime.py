@@ -169,7 +169,7 @@ class Runtime:
         self.bar, self.status = z(1, torch.int64), z(4, torch.int32)
         self.bar_base = 0
         self.ar_base = 0
-        for t in program.shared.values():          # partial tiles carry tags that count from bar_base
+        for t in program.shared.values():          # counters and partial tiles start at zero
             t.zero_()
         self.tp, self.rank, self.mailbox = tp, rank, mailbox
         self.spin_limit_ns = int(spin_limit_ms * 1e6)

@@ -176,3 +176,30 @@ def test_a_stage_runs_twice_with_the_same_counters():
     torch.cuda.synchronize()
     rt.check()
     assert torch.equal(out, first)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_a_counter_that_starts_over_meets_no_old_partial_tiles(captured):
+    """A host may zero the barrier counter and pass base 0 for every launch, also in a graph that it replays."""
+    out, want, _, _, rt = _run(P.FMT_FP8, 512, 4096, 8, 8, seed=19)
+    assert float((out.double() - want).abs().max()) <= _tol(want)
+    assert bool(rt.prog.shared["t.part"].any())                   # the stage is cut into panels
+    x = rt.prog.keep[3]
+    assert x.shape == (8, 4096)
+
+    def launch():
+        rt.bar.zero_()
+        rt.bar_base = 0
+        rt.launch(1)
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            launch()
+    for k in range(20):
+        factor = -2.0 if k % 2 == 0 else -0.5                     # exact: the products follow bit for bit
+        x.mul_(factor)
+        first = out.clone()
+        graph.replay() if captured else launch()
+        torch.cuda.synchronize()
+        rt.check()
+        assert torch.equal(out, first * factor), k
