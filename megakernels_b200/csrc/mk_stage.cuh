@@ -629,7 +629,7 @@ __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
             if (before > 0) {
                 cta -= grid - before;
                 grid = before;
-            } else if ((d.flags & MKS_FLAG_NO_BARRIER) && si + 1 < A.n_stages && R > 0 && Q > 0) {
+            } else if ((d.flags & MKS_FLAG_NO_BARRIER) && si + 1 < A.n_stages && R > 0 && Q > 0 && grid > 1) {     // (one CTA cannot be shared)
                 const mk_stage_desc& nx = A.prog[si + 1];
                 if (nx.op == MKS_OP_GEMV && __ldg(&nx.i[MKS_I_TILES]) > 0) {
                     beside = side_by_side(d, nx, *reinterpret_cast<const volatile int*>(&S.n_groups), grid);

@@ -203,3 +203,26 @@ def test_a_counter_that_starts_over_meets_no_old_partial_tiles(captured):
         torch.cuda.synchronize()
         rt.check()
         assert torch.equal(out, first * factor), k
+
+
+@pytest.mark.parametrize("grid", [1, 2, 3])
+def test_stages_without_a_barrier_between_them_on_few_ctas(grid):
+    """Two stages share the grid when nothing separates them; one CTA runs both."""
+    dev = torch.device("cuda", 0)
+    g = torch.Generator().manual_seed(23)
+    x = (torch.randn(2, 1024, generator=g) * 1.5).cuda()
+    pr = Program(dev, 2, grid)
+    pr.embed(pr.zeros(4, 256, dtype=torch.bfloat16), pr.zeros(2, 256), pr.zeros(2, 16), None, 256, 4, keys_valid=False)
+    xb, outs, wants = pr.hold(x.clone()), [], []
+    for i, N in enumerate((256, 48)):
+        wq, kw, _, deq = _weights(P.FMT_MXFP4, N, 1024, 30 + i)
+        packed, meta = P.pack_matrix(P.FMT_MXFP4, 1, wq, **kw)
+        outs.append(pr.zeros(2, N))
+        pr.gemv(f"t{i}", pr.hold(packed), meta, xb, outs[i], x_stride=1024, out_stride=N, no_barrier=i == 0)
+        wants.append(x.to(torch.bfloat16).double() @ deq.t())
+    rt = Runtime(pr, spin_limit_ms=1000)
+    rt.launch(1)
+    torch.cuda.synchronize()
+    rt.check()
+    for out, want in zip(outs, wants):
+        assert float((out.double() - want).abs().max()) <= _tol(want)
