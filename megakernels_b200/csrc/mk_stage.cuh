@@ -632,6 +632,8 @@ __device__ __noinline__ void scout_main(Shared& S, const Args& A) {
             } else if ((d.flags & MKS_FLAG_NO_BARRIER) && si + 1 < A.n_stages && R > 0 && Q > 0 && grid > 1) {     // (one CTA cannot be shared)
                 const mk_stage_desc& nx = A.prog[si + 1];
                 if (nx.op == MKS_OP_GEMV && __ldg(&nx.i[MKS_I_TILES]) > 0) {
+                    // every CTA must see the same number of groups, also when only the second stage is a routed one
+                    if (nx.i[MKS_I_GROUPS] < 0 && !scout_wait(S, &S.route_seq, routes)) return;
                     beside = side_by_side(d, nx, *reinterpret_cast<const volatile int*>(&S.n_groups), grid);
                     grid -= beside;
                 }

@@ -226,3 +226,48 @@ def test_stages_without_a_barrier_between_them_on_few_ctas(grid):
     rt.check()
     for out, want in zip(outs, wants):
         assert float((out.double() - want).abs().max()) <= _tol(want)
+
+
+def test_a_dense_stage_before_the_routed_one():
+    """ROUTE, a dense stage without a barrier, a routed stage: both share the grid by their weights, so the split follows the
+    number of routed groups (8 in the first layer here, 64 in the second)."""
+    dev, M, K, N, E, top = torch.device("cuda", 0), 8, 512, 1024, 128, 8
+    grid = torch.cuda.get_device_properties(dev).multi_processor_count
+    g = torch.Generator().manual_seed(29)
+    wq, kw, rs, deq = _weights(P.FMT_FP8, E * N, K, 31)
+    mats = [P.pack_matrix(P.FMT_FP8, 1, wq[e * N: (e + 1) * N]) for e in range(E)]
+    experts, meta = torch.cat([m[0] for m in mats]), mats[0][1]
+    dq, dkw, drs, ddeq = _weights(P.FMT_FP8, 512, K, 32)
+    dense, dmeta = P.pack_matrix(P.FMT_FP8, 1, dq)
+    pr = Program(dev, M, grid)
+    pr.embed(pr.zeros(4, 256, dtype=torch.bfloat16), pr.zeros(M, 256), pr.zeros(M, 16), None, 256, 4, keys_valid=False)
+    experts, dense, rs, drs = pr.hold(experts), pr.hold(dense), pr.hold(rs), pr.hold(drs)
+    x, xg = pr.hold(torch.randn(M, K, generator=g).cuda()), pr.hold(torch.randn(72, M, K, generator=g).cuda())
+    outs, wants, chosen = [], [], []
+    for layer in range(2):
+        lg = torch.full((M, E), -20.0, device=dev)
+        for m in range(M):
+            lg[m, (torch.arange(top) + (8 * m if layer else 0)).tolist()] = torch.randn(top, generator=g).cuda()
+        lg = pr.hold(lg)
+        pr.add(D.desc(D.MKS_OP_ROUTE, D.MKS_FLAG_NO_BARRIER, i=dict(EXPERTS=E, TOPK=top, LOGIT_STRIDE=E, ROUTE_KIND=1), p=dict(LOGITS=lg.data_ptr())))
+        a, b = pr.zeros(M, 512), pr.zeros(M, N)
+        pr.gemv("dense", dense, dmeta, x, a, x_stride=K, out_stride=512, row_scale=drs, no_barrier=True)
+        pr.gemv("routed", experts, meta, xg, b, x_stride=K, x_gstride=M * K, out_stride=N, n_valid=N, groups=-1, w_gstride=meta["bytes"],
+                row_scale=rs, rs_gstride=N, reduce_groups=True)
+        ids = sorted({(8 * m if layer else 0) + k for m in range(M) for k in range(top)})
+        coef = torch.softmax(lg.double(), -1)
+        want = torch.zeros(M, N, dtype=torch.float64, device=dev)
+        for i, e in enumerate(ids):
+            y = xg[i].to(torch.bfloat16).double() @ deq[e * N: (e + 1) * N].t()
+            want += torch.where(coef[:, e: e + 1] > 1e-6, coef[:, e: e + 1], 0.0) * y
+        outs += [a, b]
+        wants += [x.to(torch.bfloat16).double() @ ddeq.t(), want]
+    rt = Runtime(pr, spin_limit_ms=1000)
+    for _ in range(5):
+        for o in outs:
+            o.zero_()
+        rt.launch(1)
+        torch.cuda.synchronize()
+        rt.check()
+        for out, want in zip(outs, wants):
+            assert float((out.double() - want).abs().max()) <= _tol(want)
