@@ -88,7 +88,8 @@ enum {
     MKS_I_ALLREDUCE,     /* 1: sum over tensor-parallel ranks before the epilogue                  */
     MKS_I_ACT,           /* MKS_ACT_* of E_GLU                                                     */
     MKS_I_K_TOTAL,       /* columns of the whole input vector (the mean of P_NORM divides by it)    */
-    MKS_I_BLOCK_SCALES,  /* FP8: fp32 scales per 128 k inside each chunk (0: none)                 */
+    MKS_I_BLOCK_SCALES,  /* FP8: fp32 scales per 128 k inside each chunk (0: none; 2: and all of them, of every group, are
+                            bf16 values, which lets a prompt's products take two weight pieces instead of three) */
     MKS_I_PIECES,        /* 1: input rounded to bf16 (the model dtype); 2: hi + lo pieces, fp16 (bf16 for bf16 weights):
                             inputs exact to 16+ bits, two MMA columns per sequence, M <= 4       */
     MKS_I_GEMV_END,

@@ -71,7 +71,7 @@ struct Exec {
     static int format(const mk_stage_desc& d) {
         switch (d.i[MKS_I_FMT]) {
             case MKS_FMT_MXFP4: return W_MXFP4;
-            case MKS_FMT_FP8: return d.i[MKS_I_BLOCK_SCALES] ? W_FP8_PIECES : W_FP8;
+            case MKS_FMT_FP8: return d.i[MKS_I_BLOCK_SCALES] == 2 ? W_FP8_PIECES2 : (d.i[MKS_I_BLOCK_SCALES] ? W_FP8_PIECES3 : W_FP8);
             case MKS_FMT_BF16: return W_BF16;
             default: return -1;
         }
@@ -178,12 +178,14 @@ struct Exec {
 
     int gemm(const mk_stage_desc& d, GemmArgs& A, int out, int items) {
         const int blocks = (d.i[MKS_I_TILES] + 7) / 8;
-        switch (format(d)) {
+        const int fmt = format(d);
+        if ((fmt == W_FP8_PIECES2 || fmt == W_FP8_PIECES3) && A.ksplit == 1 && A.nt * (A.kbs / 2) <= 512 && A.kbs % 2 == 0)
+            return launch_gemm<W_FP8_BLOCK, 1>(A, out, blocks, ntiles, items, st);
+        switch (fmt) {
             case W_MXFP4: return launch_gemm<W_MXFP4, 1>(A, out, blocks, ntiles, items, st);
             case W_FP8: return launch_gemm<W_FP8, 1>(A, out, blocks, ntiles, items, st);
-            case W_FP8_PIECES:
-                if (A.ksplit == 1 && A.nt * (A.kbs / 2) <= 512 && A.kbs % 2 == 0) return launch_gemm<W_FP8_BLOCK, 1>(A, out, blocks, ntiles, items, st);
-                return launch_gemm<W_FP8_PIECES, 1>(A, out, blocks, ntiles, items, st);
+            case W_FP8_PIECES2: return launch_gemm<W_FP8_PIECES2, 1>(A, out, blocks, ntiles, items, st);
+            case W_FP8_PIECES3: return launch_gemm<W_FP8_PIECES3, 1>(A, out, blocks, ntiles, items, st);
             default: return launch_gemm<W_BF16, 1>(A, out, blocks, ntiles, items, st);
         }
     }

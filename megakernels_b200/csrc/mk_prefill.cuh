@@ -64,11 +64,13 @@ __device__ __forceinline__ void store_slab8(uint8_t* x, size_t piece_stride, int
 }
 
 // ---- matrix product ----------------------------------------------------------------------------------------
-// How the weights come: packed tiles of a format, or bf16 slabs.  Block-scaled FP8 has two forms: few tokens per tile leave
+// How the weights come: packed tiles of a format, or bf16 slabs.  Block-scaled FP8 has three forms: few tokens per tile leave
 // room in tensor memory for an accumulator per 128-column block, and the epilogue adds them with their scales
-// (W_FP8_BLOCK, the decode kernel's arithmetic); many tokens do not, and the scaled weights enter as two exact bf16 pieces
-// (W_FP8_PIECES), at twice the MMAs.
-enum { W_MXFP4 = 0, W_FP8, W_FP8_BLOCK, W_FP8_PIECES, W_BF16, W_SLAB };
+// (W_FP8_BLOCK, the decode kernel's arithmetic); many tokens do not, and the scaled weights enter as bf16 pieces.  A value
+// has 4 bits: with scales that are bf16 values (8 bits; the record says so) two pieces hold the product exactly
+// (W_FP8_PIECES2), at twice the MMAs; with any fp32 scale three hold its fp32 value (W_FP8_PIECES3).
+enum { W_MXFP4 = 0, W_FP8, W_FP8_BLOCK, W_FP8_PIECES2, W_FP8_PIECES3, W_BF16, W_SLAB };
+template <int FMT> constexpr int weight_pieces = FMT == W_FP8_PIECES3 ? 3 : (FMT == W_FP8_PIECES2 ? 2 : 1);
 enum { OUT_STORE = 0, OUT_ADD, OUT_GLU };
 
 struct GemmArgs {
@@ -168,7 +170,7 @@ __device__ __forceinline__ uint32_t e4m3_as_bf16(uint32_t w, uint32_t sel) {
 __device__ __forceinline__ uint32_t f16_as_bf16(uint32_t h) { return (h & 0x80008000u) | ((h >> 3) & 0x0FFF0FFFu); }
 
 // Raw bytes of one 64-column block of a 16-row tile, as lane (g, q) holds them.
-template <int FMT> struct Raw { uint4 q[FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2)]; uint32_t s[FMT == W_FP8_PIECES ? 2 : 1]; };
+template <int FMT> struct Raw { uint4 q[FMT == W_BF16 ? 4 : (FMT == W_MXFP4 ? 1 : 2)]; uint32_t s[weight_pieces<FMT> > 1 ? 2 : 1]; };
 
 // Walks the 64-column blocks of one tile: its units follow one another.
 template <int FMT>
@@ -188,10 +190,10 @@ struct Walk {
     }
     __device__ __forceinline__ void load(const GemmArgs& A, Raw<FMT>& r) {
         if (FMT == W_MXFP4) r.s[0] = __ldg(reinterpret_cast<const uint32_t*>(s));
-        if (FMT == W_FP8_PIECES) {
+        if constexpr (weight_pieces<FMT> > 1) {
             const uint2 x = __ldg(reinterpret_cast<const uint2*>(s));
             r.s[0] = x.x;
-            r.s[FMT == W_FP8_PIECES ? 1 : 0] = x.y;
+            r.s[1] = x.y;
         }
 #pragma unroll
         for (int i = 0; i < STEPS; i++) {
@@ -206,7 +208,7 @@ struct Walk {
     __device__ __forceinline__ void step(const GemmArgs& A) {
         p += 512;
         if (FMT == W_MXFP4) s += 32;
-        if (FMT == W_FP8_PIECES && (left & 3) == 1) s += 8;
+        if (weight_pieces<FMT> > 1 && (left & 3) == 1) s += 8;
         if (--left == 0) {
             left = A.chunk_steps;
             p += A.chunk_bytes - A.chunk_steps * 512;
@@ -215,11 +217,19 @@ struct Walk {
     }
 };
 
-// One lane's share of a block as bf16: v[row half][j] holds columns 16 j + 4 q + {0 .. 3}; for block-scaled weights
-// `lo` takes what the product of a value (4 bits) and its bf16 scale (8 bits) keeps behind the first eight bits, so that
-// the two pieces together are exact.
+// Two scaled values as bf16 pieces: each takes the first eight bits of what the ones before it left.
+__device__ __forceinline__ void split_scaled(uint32_t e, float s, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    float a = bf_lo(e) * s, b = bf_hi(e) * s;
+    p0 = pack_bf16(a, b);
+    a -= bf_lo(p0); b -= bf_hi(p0);
+    p1 = pack_bf16(a, b);
+    a -= bf_lo(p1); b -= bf_hi(p1);
+    p2 = pack_bf16(a, b);
+}
+// One lane's share of a block as bf16: piece 0's v[row half][j] holds columns 16 j + 4 q + {0 .. 3}.
 template <int FMT>
-__device__ __forceinline__ void convert(const Raw<FMT>& r, uint2 (&v)[2][4], uint2 (&lo)[2][4]) {
+__device__ __forceinline__ void convert(const Raw<FMT>& r, uint2 (&pieces)[weight_pieces<FMT>][2][4]) {
+    uint2 (&v)[2][4] = pieces[0];
     if constexpr (FMT == W_BF16) {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -265,13 +275,19 @@ __device__ __forceinline__ void convert(const Raw<FMT>& r, uint2 (&v)[2][4], uin
                 const int h = k >> 1, j = 2 * i + (k & 1);
                 v[h][j].x = mul_bf16x2(e4m3_as_bf16(w[k], 0x1404), UP);
                 v[h][j].y = mul_bf16x2(e4m3_as_bf16(w[k], 0x3424), UP);
-                if constexpr (FMT == W_FP8_PIECES) {
-                    const uint32_t s = r.s[h] >> 16, ss = s | (s << 16), neg = 0xBF80BF80u;
+                if constexpr (FMT == W_FP8_PIECES2) {
+                    const uint32_t s = r.s[h] >> 16, ss = s | (s << 16), neg = 0xBF80BF80u;      // (a bf16 value: the lower half is zero)
                     const uint2 e = v[h][j];
+                    uint2& lo = pieces[1][h][j];
                     v[h][j].x = mul_bf16x2(e.x, ss);
                     v[h][j].y = mul_bf16x2(e.y, ss);
-                    lo[h][j].x = fma_bf16x2(e.x, ss, mul_bf16x2(v[h][j].x, neg));
-                    lo[h][j].y = fma_bf16x2(e.y, ss, mul_bf16x2(v[h][j].y, neg));
+                    lo.x = fma_bf16x2(e.x, ss, mul_bf16x2(v[h][j].x, neg));
+                    lo.y = fma_bf16x2(e.y, ss, mul_bf16x2(v[h][j].y, neg));
+                } else if constexpr (FMT == W_FP8_PIECES3) {
+                    const float s = __uint_as_float(r.s[h]);
+                    const uint2 e = v[h][j];
+                    split_scaled(e.x, s, v[h][j].x, pieces[1][h][j].x, pieces[2][h][j].x);
+                    split_scaled(e.y, s, v[h][j].y, pieces[1][h][j].y, pieces[2][h][j].y);
                 }
             }
         }
@@ -311,14 +327,14 @@ __device__ __forceinline__ float block_scale(const GemmArgs& A, int group, int n
 //   warp 8 CG + 1        one lane issues the MMAs.
 // grid: x = token tile (neighbouring CTAs share weights, so HBM reads them once), y = 128-row weight block, z = K split;
 // routed groups: x = weight block, y = work item.
-// PX: bf16 pieces of the token operand (3: fp32-exact inputs); weight pieces: 2 for W_FP8_PIECES, else 1.
+// PX: bf16 pieces of the token operand (3: fp32-exact inputs); weight pieces: see the formats.
 // Three-piece inputs keep the products of the first piece in an accumulator of their own: an accumulation rounds its sum
 // towards zero, and the small terms of pieces 2 and 3 would add two more such roundings per step to the large sum.
 template <int FMT, int PX, int OUT, int CG>
 static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) rows_gemm(const __grid_constant__ GemmArgs A) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    constexpr int PW = FMT == W_FP8_PIECES ? 2 : 1, CW = 8 * CG;
-    constexpr int DIST = FMT == W_BF16 ? 2 : (FMT == W_MXFP4 ? 6 : 4);        // blocks a lane requests ahead
+    constexpr int PW = weight_pieces<FMT>, CW = 8 * CG;
+    constexpr int DIST = FMT == W_BF16 || FMT == W_FP8_PIECES3 ? 2 : (FMT == W_MXFP4 ? 6 : 4);        // blocks a lane requests ahead
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int group = 0, row0, rows, block, z = 0;
@@ -458,14 +474,14 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
 #pragma unroll
                 for (int i = 0; i < DIST; i++) {
                     if (kb + i * CG < kb1 && ok) {
-                        uint2 v[2][4], lo[2][4];
-                        convert<FMT>(raw[i], v, lo);
+                        uint2 v[PW][2][4];
+                        convert<FMT>(raw[i], v);
                         request(raw[i]);
                         ok = __all_sync(0xffffffffu, wait(B, A, &B.empty[slot], phase ^ 1u, WP_EMPTY));   // the warp leaves together
                         if (ok && have) {
                             uint8_t* st = smem + (size_t)slot * stage_bytes;
-                            store_operand(st, off, g & 1, v);
-                            if (PW == 2) store_operand(st + A_BYTES, off, g & 1, lo);
+#pragma unroll
+                            for (int p = 0; p < PW; p++) store_operand(st + p * A_BYTES, off, g & 1, v[p]);
                         }
                         mk::fence_proxy_async();
                         __syncwarp();

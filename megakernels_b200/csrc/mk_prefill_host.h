@@ -52,7 +52,7 @@ int launch_gemm_cg(GemmArgs& A, int out, dim3 grid, int smem, cudaStream_t st) {
 
 template <int FMT, int PX>
 int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaStream_t st) {
-    constexpr int PW = FMT == W_FP8_PIECES ? 2 : 1;
+    constexpr int PW = weight_pieces<FMT>;
     const int stage = PW * A_BYTES + PX * A.nt * 128, fixed = (int)sizeof(GemmBars) + 1024;
     // Narrow tiles leave room for two CTAs per SM with three stages each: one's start and end hide behind the other.  Wide
     // ones have the SM to themselves, with sixteen warps to convert weights (eight cannot keep up with the MMAs).

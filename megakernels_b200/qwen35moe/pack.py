@@ -98,6 +98,9 @@ class Packed:
             se = m + "shared_expert."
             pack((i, "sh_gu"), cat([get(i, se + "gate_proj"), get(i, se + "up_proj")]), FP8_KC, row_order=tile.glu_row_order(s.sfi), splits=1)
             pack((i, "sh_down"), get(i, se + "down_proj"), FP8_KC, splits=1)
+            for n in ("gu", "down"):                                       # one record describes the routed and the shared matrices
+                ex, sh = self.mats[(i, "ex_" + n)][1], self.mats[(i, "sh_" + n)][1]
+                ex["bf16_scales"] = sh["bf16_scales"] = ex["bf16_scales"] and sh["bf16_scales"]
             assert s.sfi == s.fi, "the shared expert rides the routed stages as one more group: same geometry"
             names = ["input_layernorm.weight", "post_attention_layernorm.weight"]
             names += ["self_attn.q_norm.weight", "self_attn.k_norm.weight"] if s.is_attn(i) else \

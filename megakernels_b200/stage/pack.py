@@ -87,6 +87,7 @@ def pack_matrix(fmt, splits, w, scales=None, block_scales=None, row_order=None):
     nch = unit_steps // cs
     cb = chunk_bytes(fmt, cs, block_scaled)
     dev = w.device
+    bf16_scales = False
     if fmt == FMT_BF16:
         x = _pad_rows(w.contiguous().view(torch.int16), T * 16)
         v = _steps_view(x, splits, 16).reshape(T, 2, 8, splits, unit_steps, 4, 4)          # t h g s st q sl
@@ -127,6 +128,7 @@ def pack_matrix(fmt, splits, w, scales=None, block_scales=None, row_order=None):
             per_row = block_scales.float()[(src_rows // 128)]                                 # [T*16, K/128]
             per_row = per_row[:, : K // 128].reshape(T, 2, 8, splits, kc // 128)[:, :, 0]     # [T, h, s, blocks]
             extra = per_row.permute(2, 0, 3, 1).contiguous()                                  # s t blk h
+            bf16_scales = bool((extra == extra.to(torch.bfloat16).float()).all())
             extra = extra.reshape(splits, T, nch, (cs // 4) * 2).view(torch.uint8).reshape(splits, T, nch, (cs // 4) * 8)
     parts = [body] if extra is None else [body, extra]
     used = sum(p.shape[-1] for p in parts)
@@ -134,7 +136,7 @@ def pack_matrix(fmt, splits, w, scales=None, block_scales=None, row_order=None):
         parts.append(torch.zeros(splits, T, nch, cb - used, dtype=torch.uint8, device=dev))
     out = torch.cat(parts, dim=-1).transpose(0, 1).reshape(-1)
     meta = dict(fmt=fmt, tiles=T, splits=splits, unit_steps=unit_steps, chunk_steps=cs, chunk_bytes=cb, kc=kc, rows=N,
-                block_scaled=block_scaled, bytes=out.numel())
+                block_scaled=block_scaled, bf16_scales=bf16_scales, bytes=out.numel())
     return out, meta
 
 

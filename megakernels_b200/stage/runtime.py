@@ -83,7 +83,7 @@ class Program:
                  CHUNK_BYTES=meta["chunk_bytes"], KC=meta["kc"], PROLOGUE=prologue, EPILOGUE=epilogue,
                  N_VALID=n_valid if n_valid is not None else meta["rows"], X_STRIDE=x_stride, X_GSTRIDE=x_gstride,
                  OUT_STRIDE=out_stride, OUT_GSTRIDE=out_gstride, REDUCE_GROUPS=int(reduce_groups), ALLREDUCE=int(allreduce), ACT=act,
-                 K_TOTAL=k_total if k_total is not None else meta["kc"] * S, BLOCK_SCALES=int(meta["block_scaled"]), PIECES=pieces)
+                 K_TOTAL=k_total if k_total is not None else meta["kc"] * S, BLOCK_SCALES=int(meta["block_scaled"]) + int(meta.get("bf16_scales", False)), PIECES=pieces)
         in_bound = 0.0
         if prologue == D.MKS_P_NORM and norm_w is not None:
             # |x_i| / rms(x) <= sqrt(K): a bound on every normed value, with a margin for the roundings

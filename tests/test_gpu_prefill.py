@@ -2,7 +2,8 @@
 
 The first layer's recurrent state sees no earlier bf16 rounding, so there the two must agree to fp32 sums; behind it
 roundings of GEMV inputs flip, so logits and states are held to the bars the decode tests use.  Lengths: the shortest
-this path takes, one row short of / past a 16-row tile and a 256-row tile, several passes, and a start behind a context."""
+this path takes, one row short of / past a 16-row tile and a 256-row tile, several passes, and a start behind a context.
+Block-scaled FP8 with scales that are bf16 values and with others, in tiles with and without room for an accumulator per block."""
 
 import pytest
 import torch
@@ -21,7 +22,7 @@ SHAPES = {
     "26b": (gemma26b, FULL26.with_(hidden=512, vocab=4096, layers=6, ffn=256, experts=128, eff=128, window=64)),
 }
 CASES = [("27b", {}, 1, 12, 0), ("27b", {}, 1, 258, 0), ("27b", {}, 3, 86, 37), ("27b", {"fmt": "bf16"}, 2, 41, 0),
-         ("35b", {}, 1, 18, 0), ("35b", {}, 2, 129, 21), ("26b", {}, 1, 17, 0), ("26b", {}, 3, 150, 21)]
+         ("35b", {}, 1, 18, 0), ("35b", {}, 2, 129, 21), ("35b", {"fp32_scales": True}, 1, 18, 0), ("35b", {"fp32_scales": True}, 2, 129, 0), ("26b", {}, 1, 17, 0), ("26b", {}, 3, 150, 21)]
 
 
 def rel(a, b):
@@ -36,7 +37,13 @@ def packed():
         key = (model, tuple(fmt.items()))
         if key not in made:
             pkg, shape = SHAPES[model]
-            made[key] = pkg.Packed(pkg.SynthWeights(shape, layers=shape.layers, init="realistic", device="cuda", **fmt), "cuda")
+            kw = dict(fmt)
+            fp32_scales = kw.pop("fp32_scales", False)
+            W = pkg.SynthWeights(shape, layers=shape.layers, init="realistic", device="cuda", **kw)
+            if fp32_scales:                                  # block scales that are not bf16 values: just below the next one
+                W.raw = {k: (q, sc.float() * 1.0037) for k, (q, sc) in W.raw.items()}
+                W.exs = {k: sc.float() * 1.0037 for k, sc in W.exs.items()}
+            made[key] = pkg.Packed(W, "cuda")
         return made[key]
     return get
 

@@ -112,3 +112,11 @@ def test_chunk_geometry():
     assert P.pick_chunk_steps(12, P.FMT_FP8, block_scaled=True) % 4 == 0
     assert P.chunk_bytes(P.FMT_MXFP4, 8) == 8 * 512 + 8 * 32
     assert P.chunk_bytes(P.FMT_FP8, 8, True) == 8 * 512 + 16
+
+
+def test_packing_says_whether_block_scales_are_bf16_values():
+    q, sc = Q.quantize_fp8_block(torch.randn(256, 256, generator=torch.Generator().manual_seed(1)))
+    assert P.pack_matrix(P.FMT_FP8, 1, q, block_scales=sc)[1]["bf16_scales"]
+    odd = sc.float()
+    odd[1, 1] *= 1.0 + 2.0 ** -12
+    assert not P.pack_matrix(P.FMT_FP8, 1, q, block_scales=odd)[1]["bf16_scales"]
