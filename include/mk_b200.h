@@ -220,7 +220,7 @@ int mk_launch_batch(mk_engine* e, const mk_batch_args* args, void* stream);
  * a prompt token by token inside its kernel (qwen3.5-0.8b/qwen_mk/engine.py:296-301). */
 typedef struct mk_prefill_args {
     uint64_t tokens;         /* int32[positions] in device memory                                  */
-    int32_t positions;
+    int32_t positions;       /* at most 65535 a call                                               */
     int32_t start_pos;       /* position of the first token                                        */
     int32_t sequence;        /* which of the engine's sequences (0 for single-sequence launches)   */
     int32_t batched;         /* 1: for mk_launch_batch (MK_L_CONV_HIST_B), 0: for mk_launch        */

@@ -268,13 +268,15 @@ int mk_stage_launch(const mk_stage_args* args, void* stream);
 /* A prompt through `program`, all positions at once: what `positions` decode steps with given tokens leave in the
  * states, caches and `pos`, computed as matrix products over batch x positions token rows (tcgen05) instead of step by
  * step.  The LM head is not run: either feed the prompt's last token to mk_stage_launch, or let this call take it in too
- * (`last`) and launch the LM head's record alone.  `program` is a HOST copy of the records.  Programs with two-piece inputs, int8 weights, an fp32 KV cache or all-reduces are MK_ERR_UNSUPPORTED.
+ * (`last`) and launch the LM head's record alone.  `program` is a HOST copy of the records.  MK_ERR_UNSUPPORTED (step through
+ * the prompt instead): two-piece inputs, int8 weights, an fp32 KV cache, all-reduces, and records that read anything but what
+ * earlier records of the program have written.
  * The reference takes a prompt in by one `step` per position (qwen3.8-27b-gfx942/mk/reference.py:378-386). */
 typedef struct mk_stage_prefill_args {
     uint64_t program;        /* host address of mk_stage_desc[n_stages]                             */
     int32_t n_stages;
     int32_t batch;           /* M, 1..8                                                            */
-    int32_t positions;       /* L: prompt tokens per sequence                                      */
+    int32_t positions;       /* L: prompt tokens per sequence; at most 65535 / batch a call        */
     int32_t device;
     uint64_t tokens;         /* int32[positions][batch] in device memory                           */
     uint64_t pos;            /* int32[M]: positions of the first token; advanced by `positions`    */

@@ -4,6 +4,7 @@
 // the kernels of mk_prefill.cuh.  The program's per-step activation buffers ([M][width]) become arrays of M x L rows in
 // the caller's workspace; weights, states and caches are used where they are.  Everything the LM head needs is left to
 // one ordinary decode step with the prompt's last token, so the caller sees exactly what stepping through would leave.
+#include <utility>
 #include <vector>
 
 #include "mk_prefill_host.h"
@@ -12,7 +13,175 @@ using namespace mkp;
 
 namespace {
 
+// What this path does not do exactly as the decode kernel does is refused as a whole, and the caller steps through the prompt.
+// A record is taken only if all it reads is what earlier records of the program have written in the same form: here the
+// per-step buffers are arrays of their own, with nothing in them that was there before, and products' inputs are kept as bf16
+// slabs.  The check follows the records through the buffers without touching the device.
+struct Flow {
+    struct Rows { uint64_t base; int width; uint64_t ssq; std::vector<std::pair<int, int>> cols; };   // fp32 [M][width]; written columns; sums of squares of all of it
+    struct Made { uint64_t key; int stride, width; };                                                 // slabs
+    int M;
+    std::vector<Rows> rows;
+    std::vector<Made> slabs;
+
+    Rows* find(uint64_t p) {
+        for (auto& r : rows)
+            if (p >= r.base && p < r.base + (uint64_t)r.width * 4) return &r;
+        return nullptr;
+    }
+    bool reads(uint64_t p, int stride, int off, int n) {
+        Rows* r = find(p);
+        if (!r || r->width != stride || (p - r->base) % 16) return false;
+        int at = (int)((p - r->base) / 4) + off;
+        const int end = at + n;
+        if (at < 0 || end > r->width) return false;
+        for (bool more = true; more && at < end;) {
+            more = false;
+            for (auto& c : r->cols)
+                if (c.first <= at && c.second > at) {
+                    at = c.second;
+                    more = true;
+                }
+        }
+        return at >= end;
+    }
+    static bool apart(uint64_t a, uint64_t a_bytes, uint64_t b, uint64_t b_bytes) { return a + a_bytes <= b || b + b_bytes <= a; }
+    bool writes(uint64_t p, int stride, int n, uint64_t ssq) {
+        if (n > stride || stride % 4) return false;
+        const uint64_t bytes = ((uint64_t)(M - 1) * stride + n) * 4;
+        for (auto& m : slabs)
+            if (!apart(p, bytes, m.key, (uint64_t)M * m.stride * 4)) return false;
+        Rows* r = find(p);
+        if (r) {
+            const int at = (int)((p - r->base) / 4);
+            if (r->width != stride || (p - r->base) % 16 || at + n > stride) return false;
+            r->cols.push_back({at, at + n});
+            r->ssq = at == 0 && n == stride ? ssq : 0;
+            return true;
+        }
+        for (auto& o : rows)
+            if (!apart(p, bytes, o.base, (uint64_t)M * o.width * 4)) return false;
+        rows.push_back({p, stride, n == stride ? ssq : 0, {{0, n}}});
+        return true;
+    }
+    bool makes(uint64_t key, int stride, int width) {
+        if (width > stride || width % 64) return false;
+        const uint64_t bytes = (uint64_t)M * stride * 4;
+        for (auto& r : rows)
+            if (!apart(key, bytes, r.base, (uint64_t)M * r.width * 4)) return false;
+        for (auto& m : slabs) {
+            if (m.key == key && m.stride == stride) {
+                m.width = width;
+                return true;
+            }
+            if (!apart(key, bytes, m.key, (uint64_t)M * m.stride * 4)) return false;
+        }
+        slabs.push_back({key, stride, width});
+        return true;
+    }
+    // all columns of a vector, and the sums of squares its norm is computed from
+    bool normed(uint64_t p, int n, uint64_t ssq) {
+        Rows* r = find(p);
+        return r && r->base == p && r->width == n && ssq && r->ssq == ssq;
+    }
+    // a product's input
+    bool operand(const mk_stage_desc& d, int K) {
+        for (auto& m : slabs)
+            if (m.key == d.p[MKS_P_X]) return d.i[MKS_I_PROLOGUE] == MKS_P_PLAIN && m.stride == d.i[MKS_I_X_STRIDE] && m.width == K;
+        if (!reads(d.p[MKS_P_X], d.i[MKS_I_X_STRIDE], 0, K)) return false;
+        return d.i[MKS_I_PROLOGUE] == MKS_P_PLAIN || (d.i[MKS_I_PROLOGUE] == MKS_P_NORM && normed(d.p[MKS_P_X], K, d.p[MKS_P_X_SSQ]));
+    }
+};
+
+const char* refuse(const mk_stage_desc* prog, int n_stages, int M) {
+    Flow F;
+    F.M = M;
+    const mk_stage_desc& e = prog[0];
+    const int H = e.i[MKS_I_HIDDEN];
+    if (H < 16 || H % 16 || !F.writes(e.p[MKS_P_H], H, H, e.p[MKS_P_H_SSQ])) return "the embedding's width";
+    const mk_stage_desc *route = nullptr, *up = nullptr;       // the last routing, and the routed gate and up products behind it
+    for (int s = 1; s < n_stages; s++) {
+        const mk_stage_desc& d = prog[s];
+        if (d.op == MKS_OP_GEMV) {
+            const int kc = d.i[MKS_I_KC], K = kc * d.i[MKS_I_SPLITS], n = d.i[MKS_I_N_VALID], epi = d.i[MKS_I_EPILOGUE];
+            const bool routed = d.i[MKS_I_GROUPS] < 0, glu = epi == MKS_E_GLU;
+            if (d.i[MKS_I_PIECES] != 1) return "two-piece inputs";
+            if (d.i[MKS_I_ALLREDUCE]) return "tensor parallelism";
+            if (d.i[MKS_I_FMT] == MKS_FMT_INT8) return "int8 weights";
+            if (kc % 64) return "columns per split are not whole 64-column blocks";
+            if (d.i[MKS_I_GROUPS] != 1 && d.i[MKS_I_GROUPS] != -1) return "fixed groups";
+            if (d.i[MKS_I_PROLOGUE] == MKS_P_NORM && d.i[MKS_I_K_TOTAL] != K) return "a norm over more than the stage's columns";
+            if (epi == MKS_E_LOGITS) {
+                // the head runs behind the prompt, on the last position's residual alone
+                if (s != n_stages - 1 || routed || d.p[MKS_P_X] != e.p[MKS_P_H] || d.i[MKS_I_X_STRIDE] != H || K != H ||
+                    (d.i[MKS_I_PROLOGUE] == MKS_P_NORM && d.p[MKS_P_X_SSQ] != e.p[MKS_P_H_SSQ])) return "an LM head that does not end the program on its residual";
+                continue;
+            }
+            if (n < 1 || n > d.i[MKS_I_TILES] * (glu ? 8 : 16)) return "more output columns than tiles";
+            if (!routed) {
+                if (d.i[MKS_I_REDUCE_GROUPS]) return "one group to add up";
+                if (!F.operand(d, K)) return "an input that no earlier stage leaves in this form";
+                if (glu) {
+                    if (!F.makes(d.p[MKS_P_OUT], d.i[MKS_I_OUT_STRIDE], n)) return "activations that overlap another buffer or are not whole 64-column blocks";
+                    continue;
+                }
+            } else {
+                if (!route) return "routed products without a routing";
+                if (d.i[MKS_I_SPLITS] != 1) return "split experts";
+                if (d.p[MKS_P_W_SHARED] && route->i[MKS_I_ROUTE_KIND] != 0) return "a shared expert without a gate";
+                if (glu) {
+                    if (d.i[MKS_I_REDUCE_GROUPS] || d.i[MKS_I_X_GSTRIDE] || n % 64 || !F.operand(d, K)) return "routed gate and up products of another form";
+                    up = &d;
+                    continue;
+                }
+                if (!up || !d.i[MKS_I_REDUCE_GROUPS] || d.i[MKS_I_PROLOGUE] != MKS_P_PLAIN || d.p[MKS_P_X] != up->p[MKS_P_OUT] || K != up->i[MKS_I_N_VALID] ||
+                    d.i[MKS_I_X_STRIDE] != up->i[MKS_I_OUT_STRIDE] || d.i[MKS_I_X_GSTRIDE] != up->i[MKS_I_OUT_GSTRIDE] ||
+                    !d.p[MKS_P_W_SHARED] != !up->p[MKS_P_W_SHARED]) return "routed products that do not follow their gate and up products";
+                if (n % 4) return "routed outputs that are not whole float4s";
+            }
+            if (epi == MKS_E_RESID && !F.reads(d.p[MKS_P_OUT], d.i[MKS_I_OUT_STRIDE], 0, n)) return "a sum onto something no earlier stage writes";
+            if (!F.writes(d.p[MKS_P_OUT], d.i[MKS_I_OUT_STRIDE], n, d.p[MKS_P_OUT_SSQ])) return "an output that overlaps another buffer";
+        } else if (d.op == MKS_OP_GDN) {
+            const int key = d.i[MKS_I_NKH] * 128, val = d.i[MKS_I_NVH] * 128, stride = d.i[MKS_I_Y_STRIDE];
+            const uint64_t y = d.p[MKS_P_Y];
+            if (d.i[MKS_I_CONV_DIM] != 2 * key + val || (d.i[MKS_I_Q_OFF] | d.i[MKS_I_K_OFF] | d.i[MKS_I_V_OFF]) % 4) return "DeltaNet channels";
+            if (!F.reads(y, stride, d.i[MKS_I_Q_OFF], key) || !F.reads(y, stride, d.i[MKS_I_K_OFF], key) || !F.reads(y, stride, d.i[MKS_I_V_OFF], val) ||
+                !F.reads(y, stride, d.i[MKS_I_Z_OFF], val) || !F.reads(y, stride, d.i[MKS_I_B_OFF], d.i[MKS_I_NVH]) || !F.reads(y, stride, d.i[MKS_I_A_OFF], d.i[MKS_I_NVH]))
+                return "DeltaNet inputs that no earlier stage writes";
+            if (!F.makes(d.p[MKS_P_Y2], d.i[MKS_I_Y2_STRIDE], val)) return "DeltaNet outputs that overlap another buffer";
+        } else if (d.op == MKS_OP_ATTN) {
+            const int nq = d.i[MKS_I_NQ], nkv = d.i[MKS_I_NKV], HD = d.i[MKS_I_HD], rot = d.i[MKS_I_ROT], stride = d.i[MKS_I_A_Y_STRIDE];
+            const uint64_t y = d.p[MKS_P_A_Y];
+            if (d.i[MKS_I_KV_F32] || !d.i[MKS_I_Q_BF16]) return "fp32 attention";
+            if (nq % nkv) return "query heads per KV head";
+            if (rot < 64 || rot > HD || rot % 64 || d.i[MKS_I_ROPE_PAIRS] > rot / 2) return "rotated dims that are not whole 64-dim blocks";
+            bool ok = F.reads(y, stride, d.i[MKS_I_A_K_OFF], nkv * HD) && (d.i[MKS_I_A_V_OFF] < 0 || F.reads(y, stride, d.i[MKS_I_A_V_OFF], nkv * HD));
+            for (int h = 0; h < nq; h++) {
+                const int q = d.i[MKS_I_A_Q_OFF] + h * d.i[MKS_I_A_Q_HSTRIDE];
+                ok = ok && F.reads(y, stride, q, HD) && (d.i[MKS_I_A_GATE_OFF] < 0 || F.reads(y, stride, q + d.i[MKS_I_A_GATE_OFF], HD));
+            }
+            if (!ok) return "attention inputs that no earlier stage writes";
+            if (!F.makes(d.p[MKS_P_A_Y2], d.i[MKS_I_A_Y2_STRIDE], nq * HD)) return "attention outputs that overlap another buffer";
+        } else if (d.op == MKS_OP_ROUTE) {
+            if (!F.reads(d.p[MKS_P_LOGITS], d.i[MKS_I_LOGIT_STRIDE], 0, d.i[MKS_I_EXPERTS] + (d.i[MKS_I_ROUTE_KIND] == 0))) return "router logits that no earlier stage writes";
+            route = &d;
+            up = nullptr;
+        } else if (d.op == MKS_OP_VEC) {
+            const int N = d.i[MKS_I_VEC_N];
+            if (N == 0) continue;
+            if (!F.normed(d.p[MKS_P_VEC_A], N, d.p[MKS_P_VEC_A_SSQ]) || (d.p[MKS_P_VEC_B] && !F.normed(d.p[MKS_P_VEC_B], N, d.p[MKS_P_VEC_B_SSQ])))
+                return "a vector step's term without its sums of squares";
+            if (d.p[MKS_P_VEC_BASE] && (!F.reads(d.p[MKS_P_VEC_BASE], N, 0, N))) return "a vector step's base that no earlier stage writes";
+            if (!F.writes(d.p[MKS_P_VEC_OUT], N, N, d.p[MKS_P_VEC_OUT_SSQ]) || F.find(d.p[MKS_P_VEC_OUT])->base != d.p[MKS_P_VEC_OUT]) return "a vector step's output";
+        } else {
+            return "an embedding inside the program";
+        }
+    }
+    return nullptr;
+}
+
 struct Buffer { uint64_t base; int width; float* rows; };
+struct Have { uint64_t key; const void* norm; float in_scale, eps, off; int K; };      // what x_scratch holds
 struct Slab { uint64_t key; const void* norm; float in_scale; uint8_t* x; int rows, width; };
 
 struct Exec {
@@ -28,7 +197,7 @@ struct Exec {
     std::vector<Buffer> bufs;
     std::vector<Slab> slabs;
     uint8_t* x_scratch = nullptr;        // slabs made from fp32 rows; reused by every stage that needs new ones
-    Slab x_have = {0, nullptr, 0.f, nullptr, 0, 0};
+    Have x_have = {};
     float* part = nullptr;
     size_t part_floats = 0;
     // DeltaNet / attention / routing scratch
@@ -75,29 +244,6 @@ struct Exec {
             case MKS_FMT_BF16: return W_BF16;
             default: return -1;
         }
-    }
-
-    // What this path cannot do is refused as a whole, and the caller steps through the prompt instead.
-    const char* refuse() const {
-        if (prog[0].op != MKS_OP_EMBED) return "the program does not start with the embedding";
-        for (int s = 0; s < n_stages; s++) {
-            const mk_stage_desc& d = prog[s];
-            if (d.op == MKS_OP_GEMV) {
-                if (d.i[MKS_I_PIECES] != 1) return "two-piece inputs";
-                if (d.i[MKS_I_ALLREDUCE]) return "tensor parallelism";
-                if (format(d) < 0) return "int8 weights";
-                if (d.i[MKS_I_KC] % 64) return "columns per split are not whole 64-column blocks";
-                if (d.i[MKS_I_GROUPS] != 1 && d.i[MKS_I_GROUPS] != -1) return "fixed groups";
-                if (d.i[MKS_I_GROUPS] < 0 && d.i[MKS_I_SPLITS] != 1) return "split experts";
-                if (d.i[MKS_I_FMT] == MKS_FMT_BF16 && d.i[MKS_I_KC] / 16 % 4) return "bf16 blocks";
-                if (d.i[MKS_I_EPILOGUE] != MKS_E_LOGITS && d.i[MKS_I_OUT_STRIDE] % 4) return "unaligned outputs";
-                if (d.i[MKS_I_X_STRIDE] % 4) return "unaligned inputs";
-            } else if (d.op == MKS_OP_ATTN) {
-                if (d.i[MKS_I_KV_F32] || !d.i[MKS_I_Q_BF16]) return "fp32 attention";
-                if (d.i[MKS_I_NQ] / d.i[MKS_I_NKV] > 8) return "query heads per KV head";
-            }
-        }
-        return nullptr;
     }
 
     void layout() {
@@ -221,13 +367,14 @@ struct Exec {
         const bool norm = d.i[MKS_I_PROLOGUE] == MKS_P_NORM;
         const void* nw = norm ? reinterpret_cast<const void*>(d.p[MKS_P_NORM_W]) : nullptr;
         const float in_scale = d.f[MKS_F_IN_SCALE] != 0.f ? d.f[MKS_F_IN_SCALE] : 1.f;
-        if (x_have.key != d.p[MKS_P_X] || x_have.norm != nw || x_have.in_scale != in_scale) {
+        const Have want = {d.p[MKS_P_X], nw, in_scale, d.f[MKS_F_EPS], d.f[MKS_F_NORM_OFF], d.i[MKS_I_KC] * d.i[MKS_I_SPLITS]};
+        const bool same = x_have.key == want.key && x_have.norm == nw && x_have.K == want.K && (!norm || (x_have.in_scale == in_scale && x_have.eps == want.eps && x_have.off == want.off));
+        if (!same) {
             const float* src = at(d.p[MKS_P_X]);
-            if (!src) return pfail(MK_ERR_BADARG, "prefill: a stage reads a buffer no earlier stage writes");
             rows_in<1><<<rows, 256, 0, st>>>(src, d.i[MKS_I_X_STRIDE], d.i[MKS_I_KC] * d.i[MKS_I_SPLITS], reinterpret_cast<const float*>(nw), d.f[MKS_F_NORM_OFF],
                                              d.f[MKS_F_EPS], in_scale, x_scratch, 0, xrows);
             MKP_CUDA(cudaGetLastError());
-            x_have = {d.p[MKS_P_X], nw, in_scale, x_scratch, xrows, 0};
+            x_have = want;
         }
         *x = x_scratch;
         *x_rows = xrows;
@@ -312,7 +459,6 @@ struct Exec {
         GdnArgs G;
         memset(&G, 0, sizeof G);
         G.y = at(d.p[MKS_P_Y]);
-        if (!G.y) return pfail(MK_ERR_BADARG, "prefill: the DeltaNet stage reads a buffer no earlier stage writes");
         G.y_stride = d.i[MKS_I_Y_STRIDE];
         G.M = M; G.L = L;
         G.nkh = d.i[MKS_I_NKH]; G.nvh = d.i[MKS_I_NVH]; G.conv_dim = d.i[MKS_I_CONV_DIM];
@@ -351,7 +497,6 @@ struct Exec {
         memset(&T, 0, sizeof T);
         const int HD = d.i[MKS_I_HD];
         T.y = at(d.p[MKS_P_A_Y]);
-        if (!T.y) return pfail(MK_ERR_BADARG, "prefill: the attention stage reads a buffer no earlier stage writes");
         T.y_stride = d.i[MKS_I_A_Y_STRIDE];
         T.M = M; T.L = L; T.nq = d.i[MKS_I_NQ]; T.nkv = d.i[MKS_I_NKV];
         T.q_off = d.i[MKS_I_A_Q_OFF]; T.q_hs = d.i[MKS_I_A_Q_HSTRIDE]; T.gate_off = d.i[MKS_I_A_GATE_OFF];
@@ -383,7 +528,6 @@ struct Exec {
 
     int routing(const mk_stage_desc& d) {
         route.logits = at(d.p[MKS_P_LOGITS]);
-        if (!route.logits) return pfail(MK_ERR_BADARG, "prefill: the routing stage reads a buffer no earlier stage writes");
         route.rows = rows;
         route.stride = d.i[MKS_I_LOGIT_STRIDE];
         route.experts = d.i[MKS_I_EXPERTS];
@@ -451,9 +595,11 @@ int prepare(Exec& E, const mk_stage_desc* prog, int n_stages, int batch, int pos
     E.rows = batch * positions;
     token_tiles(E.rows, &E.ntiles, &E.nt);
     E.xrows = E.ntiles * E.nt;
+    const int rc = mk_stage_validate(prog, n_stages, batch);
+    if (rc != MK_OK) return rc;
+    if (const char* why = refuse(prog, n_stages, batch)) return pfail(MK_ERR_UNSUPPORTED, "prefill: %s", why);
     if (cudaDeviceGetAttribute(&E.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return pfail(MK_ERR_CUDA, "prefill: no device %d", device);
     E.arena.base = static_cast<uint8_t*>(workspace);
-    if (const char* why = E.refuse()) return pfail(MK_ERR_UNSUPPORTED, "prefill: %s", why);
     E.layout();
     return MK_OK;
 }
@@ -461,7 +607,7 @@ int prepare(Exec& E, const mk_stage_desc* prog, int n_stages, int batch, int pos
 }  // namespace
 
 extern "C" int64_t mk_stage_prefill_bytes(const mk_stage_desc* program, int n_stages, int batch, int positions, int device) {
-    if (!program || n_stages < 1 || batch < 1 || batch > MKS_MAX_BATCH || positions < 1) return pfail(MK_ERR_BADARG, "mk_stage_prefill_bytes: bad argument");
+    if (!program || n_stages < 1 || batch < 1 || batch > MKS_MAX_BATCH || positions < 1 || positions > MAX_ROWS / batch) return pfail(MK_ERR_BADARG, "mk_stage_prefill_bytes: bad argument");
     Exec E;
     const int rc = prepare(E, program, n_stages, batch, positions, device, nullptr);
     return rc == MK_OK ? (int64_t)E.arena.off + 1024 : rc;
@@ -469,7 +615,8 @@ extern "C" int64_t mk_stage_prefill_bytes(const mk_stage_desc* program, int n_st
 
 extern "C" int mk_stage_prefill(const mk_stage_prefill_args* a, void* stream) {
     if (!a || !a->program || a->n_stages < 1) return pfail(MK_ERR_BADARG, "mk_stage_prefill: no program");
-    if (a->batch < 1 || a->batch > MKS_MAX_BATCH || a->positions < 1) return pfail(MK_ERR_BADARG, "mk_stage_prefill: batch %d, positions %d", a->batch, a->positions);
+    if (a->batch < 1 || a->batch > MKS_MAX_BATCH || a->positions < 1 || a->positions > MAX_ROWS / a->batch)
+        return pfail(MK_ERR_BADARG, "mk_stage_prefill: batch %d, positions %d (at most %d rows a call)", a->batch, a->positions, MAX_ROWS);
     if (!a->tokens || !a->pos || !a->status || !a->workspace) return pfail(MK_ERR_BADARG, "mk_stage_prefill: tokens / pos / status / workspace missing");
     MKP_CUDA(cudaSetDevice(a->device));
     Exec E;

@@ -283,7 +283,7 @@ extern "C" int mk_prefill_weights(mk_engine* e, uint64_t weights, int64_t bytes,
 }
 
 extern "C" int64_t mk_prefill_bytes(int positions) {
-    if (positions < 1) return pfail(MK_ERR_BADARG, "mk_prefill_bytes: %d positions", positions);
+    if (positions < 1 || positions > MAX_ROWS) return pfail(MK_ERR_BADARG, "mk_prefill_bytes: %d positions", positions);
     Run R;
     memset(&R, 0, sizeof R);
     R.rows = positions;
@@ -296,7 +296,7 @@ extern "C" int mk_prefill(mk_engine* e, const mk_prefill_args* a, void* stream) 
     Run R;
     memset(&R, 0, sizeof R);
     if (mk_engine_view(e, &R.desc, &R.P) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill: mk_set_params has not succeeded on this engine");
-    if (a->positions < 1 || !a->tokens || !a->workspace || !a->weights) return pfail(MK_ERR_BADARG, "mk_prefill: positions %d, tokens / weights / workspace missing", a->positions);
+    if (a->positions < 1 || a->positions > MAX_ROWS || !a->tokens || !a->workspace || !a->weights) return pfail(MK_ERR_BADARG, "mk_prefill: positions %d, tokens / weights / workspace missing", a->positions);
     if (a->start_pos < 0 || (int64_t)a->start_pos + a->positions > R.desc->max_seq) return pfail(MK_ERR_BADARG, "mk_prefill: sequence would exceed max_seq=%d", R.desc->max_seq);
     if (a->sequence < 0 || a->sequence >= (R.desc->max_batch > 1 ? R.desc->max_batch : 1)) return pfail(MK_ERR_BADARG, "mk_prefill: sequence %d", a->sequence);
     for (int l = 0; l < R.P->n_layers; l++)

@@ -27,6 +27,7 @@ inline int pfail(int code, const char* fmt, ...) {
     } while (0)
 
 constexpr int SMEM_MAX = 232448;
+constexpr int MAX_ROWS = 65535;                     // token rows of a call: one grid coordinate of several kernels
 
 // Hands out the workspace; with base == nullptr it only counts.
 struct Arena {

@@ -64,6 +64,7 @@ def test_prompt_rows_equal_stepping(packed, monkeypatch, model, fmt, M, length, 
             launches = eng.rt.launches
             logits = eng.prefill([q[context:] for q in prompts]).clone()
             assert eng.rt.launches == launches + 1
+            assert (eng.rt._workspace is not None) == rows           # one arm took the token-parallel path, the other stepped
         eng.check()
         engines.append((eng, logits))
     (a, la), (b, lb) = engines
