@@ -1194,13 +1194,14 @@ static __global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant
     const int m = blockIdx.z, kvh = blockIdx.y, l0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * bq;      // long ones first
     const int np = min(bq, T.L - l0), pos0 = T.pos[m] + l0;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp & 3, dh = warp >> 2, g = lane >> 2, t = lane & 3;
-    const int last = pos0 + np - 1, first = (T.window ? max(0, pos0 - T.window + 1) : 0) & ~(AT_KEYS - 1);
+    // keys outside [low, last] are zeros and their pages are not touched: before a window there may be anything
+    const int last = pos0 + np - 1, low = T.window ? max(0, pos0 - T.window + 1) : 0, first = low & ~(AT_KEYS - 1);
     const __nv_bfloat16 *kc = reinterpret_cast<const __nv_bfloat16*>(T.k_cache), *vc = reinterpret_cast<const __nv_bfloat16*>(T.v_cache);
     auto load_kv = [&](uint8_t* dst, const __nv_bfloat16* cache, int k0) {
 #pragma unroll 4
         for (int i = tid; i < AT_KEYS * CH; i += 256) {
             const int key = i / CH, c = i - key * CH, p = k0 + key;
-            cp16_zfill(smem_u32(dst + (size_t)key * RB + (((c & ~7) | ((c ^ key) & 7)) << 4)), cache + kv_offset(T, m, kvh, min(p, last)) + c * 8, p <= last);
+            cp16_zfill(smem_u32(dst + (size_t)key * RB + (((c & ~7) | ((c ^ key) & 7)) << 4)), cache + kv_offset(T, m, kvh, min(max(p, low), last)) + c * 8, p >= low && p <= last);
         }
         mk::cp_async_commit();
     };

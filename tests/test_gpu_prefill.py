@@ -78,6 +78,27 @@ def test_prompt_rows_equal_stepping(packed, monkeypatch, model, fmt, M, length, 
         assert rel(a.k_cache, b.k_cache) < 2e-2 and rel(a.v_cache, b.v_cache) < 2e-2
 
 
+def test_prompt_rows_see_no_key_before_their_window(packed):
+    """What lies before the first row's window in its cache page may be anything: a page another sequence used, or never
+    written.  The decode kernel does not touch it."""
+    pkg, shape = SHAPES["26b"]
+    prompt, got = pkg.make_prompt(shape.vocab, 40, seed=3), []
+    for poisoned in (False, True):
+        eng = pkg.Engine(packed("26b", {}), 1, maxlen=200)
+        for t in (eng.ks, eng.vs):
+            t.normal_(0.0, 0.5, generator=torch.Generator(device="cuda").manual_seed(5))
+        if poisoned:
+            bt = eng.bt[0].long()
+            for p in range(100 - shape.window + 1):                   # positions 0 .. 36: the prompt starts at 100, the window is 64
+                eng.ks[:, bt[p // 64], :, p % 64] = float("inf")
+                eng.vs[:, bt[p // 64], :, p % 64] = float("nan")
+        eng.pos[0] = 100
+        got.append(eng.prefill([prompt]).clone())
+        assert eng.rt._workspace is not None
+        eng.check()
+    assert torch.isfinite(got[0]).all() and torch.equal(*got)
+
+
 def test_programs_without_the_row_path_step(packed):
     pkg, shape = SHAPES["35b"]
     eng = pkg.Engine(packed("35b", {}), 1, maxlen=64, exact_inputs=True)
