@@ -246,7 +246,8 @@ int mk_status(mk_engine* e, int32_t* where);
 enum {
     MK_Q_SMEM_BYTES = 0, MK_Q_N_THREADS, MK_Q_CONV_RING, MK_Q_KV_BLOCK, MK_Q_MAX_SPLITS, MK_Q_PART_STRIDE,
     MK_Q_OPS_PER_LAYER, MK_Q_PROF_MAX_OPS, MK_Q_PROF_FIELDS, MK_Q_SPEC_T, MK_Q_MAX_LAYERS, MK_Q_LAYER_FIELDS,
-    MK_Q_GLOBAL_FIELDS, MK_Q_SLOT_BYTES, MK_Q_STAGES, MK_Q_MAX_LM_ROWS, MK_Q_MAX_BATCH, MK_Q_BATCH_SMEM_BYTES
+    MK_Q_GLOBAL_FIELDS, MK_Q_SLOT_BYTES, MK_Q_STAGES, MK_Q_MAX_LM_ROWS, MK_Q_MAX_BATCH, MK_Q_BATCH_SMEM_BYTES,
+    MK_Q_MAX_CHUNK_POS
 };
 int64_t mk_query(int what);
 

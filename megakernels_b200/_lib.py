@@ -26,7 +26,7 @@ GLOBAL_FIELDS = ["embed", "embed_scale", "lm_head", "lm_scale", "final_norm", "r
                  "mtp_norm_e", "mtp_norm_h", "mtp_norm", "draft_head", "draft_scale", "draft_ids", "xml", "partl"]
 QUERIES = ["SMEM_BYTES", "N_THREADS", "CONV_RING", "KV_BLOCK", "MAX_SPLITS", "PART_STRIDE", "OPS_PER_LAYER",
            "PROF_MAX_OPS", "PROF_FIELDS", "SPEC_T", "MAX_LAYERS", "LAYER_FIELDS", "GLOBAL_FIELDS", "SLOT_BYTES",
-           "STAGES", "MAX_LM_ROWS", "MAX_BATCH", "BATCH_SMEM_BYTES"]
+           "STAGES", "MAX_LM_ROWS", "MAX_BATCH", "BATCH_SMEM_BYTES", "MAX_CHUNK_POS"]
 EXPORTS = ["mk_create", "mk_destroy", "mk_set_params", "mk_launch", "mk_launch_static", "mk_launch_batch", "mk_prefill", "mk_prefill_bytes", "mk_prefill_weights", "mk_prefill_weight_bytes", "mk_status", "mk_query", "mk_bw_probe",
            "mk_plan_rows", "mk_plan_attn_chunk", "mk_last_error"]
 

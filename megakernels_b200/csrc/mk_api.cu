@@ -37,10 +37,11 @@ int mk_set_error(int code, const char* text) {
     return code;
 }
 // the library's other translation units see an engine through this
-int mk_engine_view(mk_engine* e, const mk_model_desc** desc, const Params** params) {
+int mk_engine_view(mk_engine* e, const mk_model_desc** desc, const Params** params, bool* static_only) {
     if (!e->params_set) return MK_ERR_BADARG;
     *desc = &e->desc;
     *params = &e->host;
+    *static_only = e->static_only;
     return MK_OK;
 }
 #define MK_CUDA(call)                                                                      \
@@ -498,6 +499,7 @@ extern "C" int64_t mk_query(int what) {
         case MK_Q_MAX_LM_ROWS: return MAX_LM_ROWS;
         case MK_Q_MAX_BATCH: return NB;
         case MK_Q_BATCH_SMEM_BYTES: return GeoB::SMEM;
+        case MK_Q_MAX_CHUNK_POS: return MAX_CHUNK_POS;
         default: return -1;
     }
 }

@@ -11,7 +11,7 @@ using namespace mkp;
 typedef mk::Qwen35_08B S;
 
 // mk_api.cu: the engine's description and parameter block
-int mk_engine_view(mk_engine* e, const mk_model_desc** desc, const mk::Params** params);
+int mk_engine_view(mk_engine* e, const mk_model_desc** desc, const mk::Params** params, bool* static_only);
 
 namespace {
 
@@ -252,14 +252,16 @@ struct Run {
 extern "C" int64_t mk_prefill_weight_bytes(mk_engine* e) {
     const mk_model_desc* desc;
     const mk::Params* P;
-    if (!e || mk_engine_view(e, &desc, &P) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill_weight_bytes: mk_set_params has not succeeded on this engine");
+    bool bare;
+    if (!e || mk_engine_view(e, &desc, &P, &bare) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill_weight_bytes: mk_set_params has not succeeded on this engine");
     return (int64_t)(LayerSlabs(nullptr, P, P->n_layers - 1).end - static_cast<const uint8_t*>(nullptr)) + 1024;
 }
 
 extern "C" int mk_prefill_weights(mk_engine* e, uint64_t weights, int64_t bytes, void* stream) {
     const mk_model_desc* desc;
     const mk::Params* P;
-    if (!e || !weights || mk_engine_view(e, &desc, &P) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill_weights: null argument or no parameters");
+    bool bare;
+    if (!e || !weights || mk_engine_view(e, &desc, &P, &bare) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill_weights: null argument or no parameters");
     if (bytes < mk_prefill_weight_bytes(e)) return pfail(MK_ERR_BADARG, "mk_prefill_weights: %lld bytes, %lld needed", (long long)bytes, (long long)mk_prefill_weight_bytes(e));
     const uint8_t* base = reinterpret_cast<const uint8_t*>((weights + 1023) & ~(uint64_t)1023);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -295,12 +297,18 @@ extern "C" int mk_prefill(mk_engine* e, const mk_prefill_args* a, void* stream) 
     if (!e || !a) return pfail(MK_ERR_BADARG, "mk_prefill: null argument");
     Run R;
     memset(&R, 0, sizeof R);
-    if (mk_engine_view(e, &R.desc, &R.P) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill: mk_set_params has not succeeded on this engine");
+    bool bare;
+    if (mk_engine_view(e, &R.desc, &R.P, &bare) != MK_OK) return pfail(MK_ERR_BADARG, "mk_prefill: mk_set_params has not succeeded on this engine");
     if (a->positions < 1 || a->positions > MAX_ROWS || !a->tokens || !a->workspace || !a->weights) return pfail(MK_ERR_BADARG, "mk_prefill: positions %d, tokens / weights / workspace missing", a->positions);
     if (a->start_pos < 0 || (int64_t)a->start_pos + a->positions > R.desc->max_seq) return pfail(MK_ERR_BADARG, "mk_prefill: sequence would exceed max_seq=%d", R.desc->max_seq);
     if (a->sequence < 0 || a->sequence >= (R.desc->max_batch > 1 ? R.desc->max_batch : 1)) return pfail(MK_ERR_BADARG, "mk_prefill: sequence %d", a->sequence);
+    // what the launches behind a prompt refuse
+    if (bare) return pfail(MK_ERR_BADARG, "mk_prefill: this engine was given no hand-off buffers; only mk_launch_static can run it");
+    if (a->batched && R.desc->quant != MK_QUANT_INT8) return pfail(MK_ERR_UNSUPPORTED, "mk_prefill: batched decoding is built for int8 weights only");
+    if (a->batched && !R.P->actl) return pfail(MK_ERR_BADARG, "mk_prefill: the engine was given no MLP activation words (MK_G_ACTL)");
     for (int l = 0; l < R.P->n_layers; l++)
-        if (R.P->layer[l].kind == 0 && a->batched && !R.P->layer[l].conv_hist_b) return pfail(MK_ERR_BADARG, "mk_prefill: layer %d lacks the batched conv history", l);
+        if (a->batched && ((R.P->layer[l].kind == 0 && (!R.P->layer[l].conv_hist_b || !R.P->layer[l].w_out_rows)) || !R.P->layer[l].w_down_rows))
+            return pfail(MK_ERR_BADARG, "mk_prefill: layer %d lacks the batched kernel's buffers (MK_L_CONV_HIST_B, MK_L_W_OUT_ROWS, MK_L_W_DOWN_ROWS)", l);
     MKP_CUDA(cudaSetDevice(R.desc->device));
     MKP_CUDA(cudaDeviceGetAttribute(&R.sms, cudaDevAttrMultiProcessorCount, R.desc->device));
     R.rows = a->positions;

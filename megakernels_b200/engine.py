@@ -363,9 +363,7 @@ class Megakernel:
         _lib.check(self.lib.mk_launch(self._h, ctypes.byref(record), ctypes.c_void_p(stream)))
         self.launches += 1
         words = info.tolist()
-        if int(self.status[0]) != 0:                       # a device-side wait ran out: raises with the wait site
-            where = ctypes.c_int32()
-            _lib.check(self.lib.mk_status(self._h, ctypes.byref(where)))
+        self._raise_if_timed_out()
         self.epoch = words[1] & 0xFFFFFFFF
         if self.epoch > 0xFFFF0000:
             raise RuntimeError("epoch counter exhausted; call reset()")
@@ -375,12 +373,23 @@ class Megakernel:
             self.last_step_ns = (t[1:] - t[:-1]).tolist()
         return words
 
+    def _raise_if_timed_out(self):
+        """Waits for the device; if a device-side wait ran out, raises with the wait site."""
+        if int(self.status[0]) != 0:
+            where = ctypes.c_int32()
+            _lib.check(self.lib.mk_status(self._h, ctypes.byref(where)))
+
     @staticmethod
     def _sampling(temperature, seed, stop_ids, device):
         """The LaunchArgs members that describe how a token is chosen and which ids end a launch."""
         stops = torch.tensor(list(stop_ids) or [-1], dtype=torch.int32, device=device)
         return dict(seed=seed & 0xFFFFFFFF, inv_temperature=(1.0 / temperature) if temperature > 0 else 0.0,
                     n_stop=len(stop_ids)), stops
+
+    def _attention_fits(self, last_pos, sequences=1):
+        """Whether a launch of so many sequences accepts this context; one that does not is left to say so before anything ran."""
+        splits = min(self.grid // sequences // self.cfg.n_kv_heads, _lib.query("MAX_SPLITS"))
+        return splits > 0 and 0 < self.lib.mk_plan_attn_chunk(last_pos, splits) <= _lib.query("MAX_CHUNK_POS")
 
     def _take_in(self, tokens, start, hidden=None, seq=0, batched=False):
         """`tokens` enter positions start, start + 1, ... of sequence `seq`, all at once (`mk_prefill`); `hidden` [n, hidden]
@@ -426,24 +435,24 @@ class Megakernel:
         n_steps = n_given - 1 + n_generate
         if self.pos + n_steps > self.max_seq:
             raise ValueError(f"sequence would exceed max_seq={self.max_seq}")
-        dev, cfg = self.device, self.cfg
+        dev, cfg, start = self.device, self.cfg, self.pos
         want_hidden = track_mtp or return_resid
-        hidden = torch.empty(n_steps, cfg.hidden, device=dev) if want_hidden else None
         # a long prompt goes in all at once, except its last token (whoever wants logits or times per token gets steps)
-        taken = 0
         # (a caller who asks for logits gets those of `mk_launch`, bit for bit, up to EXACT_PROMPT tokens)
-        if n_given > (max(EXACT_PROMPT, MIN_PROMPT_ROWS) if return_logits else MIN_PROMPT_ROWS) and not all_logits and not timing and prof is None:
-            taken = n_given - 1
-            self._take_in(given[:taken], self.pos, hidden)
-            self.pos += taken
+        long = n_given > (max(EXACT_PROMPT, MIN_PROMPT_ROWS) if return_logits else MIN_PROMPT_ROWS)
+        taken = n_given - 1 if long and not all_logits and not timing and prof is None and self._attention_fits(start + n_steps) else 0
         left, n_left = n_given - taken, n_steps - taken
+        # everything that can be refused comes before the prompt changes the state
+        hidden = torch.empty(n_steps, cfg.hidden, device=dev) if want_hidden else None
         how, stops = self._sampling(temperature, seed, stop_ids, dev)
         bufs = dict(forced=torch.tensor(given[taken:], dtype=torch.int32).pin_memory().to(dev, non_blocking=True),
                     stop_ids=stops, tokens_out=torch.zeros(n_left, dtype=torch.int64, device=dev),
                     logits_out=torch.empty(n_left, cfg.vocab, device=dev) if (return_logits or all_logits) else None,
                     resid_out=hidden[taken:] if want_hidden else None, prof=prof)
         first_choice = 0 if all_logits else left - 1               # the first step whose LM head runs
-        words = self._submit(n_left, dict(how, n_forced=left, lm_from=first_choice, prof_step=prof_step), bufs, timing)
+        if taken:
+            self._take_in(given[:taken], start, hidden)
+        words = self._submit(n_left, dict(how, start_pos=start + taken, n_forced=left, lm_from=first_choice, prof_step=prof_step), bufs, timing)
         ran = words[0]
         # tokens_out holds keys (ordered score << 32 | ~id): the low word, complemented, is the id
         chosen = (0xFFFFFFFF - (bufs["tokens_out"][left - 1: ran] & 0xFFFFFFFF)).tolist()
@@ -451,11 +460,11 @@ class Megakernel:
             hidden = hidden[: taken + ran]
         if taken + ran:
             if track_mtp and self.mtp is not None:
-                entered = (given + chosen)[: taken + ran]          # what positions pos - taken .. pos + ran - 1 were fed
-                self.mtp_fed(self.pos - taken, mtp_mod.rmsnorm(hidden, self.final_norm, cfg.eps), entered)
+                entered = (given + chosen)[: taken + ran]          # what positions start .. start + taken + ran - 1 were fed
+                self.mtp_fed(start, mtp_mod.rmsnorm(hidden, self.final_norm, cfg.eps), entered)
             else:
                 self.mtp_h = None                                  # the draft head's cache no longer follows the sequence
-        self.pos += ran
+        self.pos = start + taken + ran
         self.last_resid = hidden
         if all_logits:
             return chosen, bufs["logits_out"][:ran]
@@ -492,11 +501,10 @@ class Megakernel:
             raise ValueError(f"a sequence would exceed max_seq={self.max_seq}")
         dev = self.device
         # long prompts go in all at once, except their last tokens (times per step are times of steps)
-        for j, p in enumerate(prompts):
-            if len(p) > MIN_PROMPT_ROWS and not timing and prof is None:
-                self._take_in(p[:-1], self.bpos[j], seq=j, batched=True)
-                self.bpos[j] += len(p) - 1
-                prompts[j] = p[-1:]
+        rows = not timing and prof is None and self._attention_fits(max(self.bpos[:B]) + n_steps, B)
+        bodies = [p[:-1] if rows and len(p) > MIN_PROMPT_ROWS else [] for p in prompts]
+        prompts = [p[len(b):] for p, b in zip(prompts, bodies)]
+        pos0 = [self.bpos[j] + len(b) for j, b in enumerate(bodies)]
         n_forced = [len(p) for p in prompts]
         n_total = [n + n_generate - 1 for n in n_forced]
         n_steps = max(n_total)
@@ -512,19 +520,20 @@ class Megakernel:
         ptr = lambda t: t.data_ptr() if t is not None else 0
         pad = lambda v: (ctypes.c_int32 * NBW)(*(list(v) + [0] * (NBW - len(v))))
         a = _lib.BatchArgs(forced=forced.data_ptr(), n_forced=pad(n_forced), n_total=pad(n_total),
-                           pos0=pad(self.bpos[:B]), batch=B, n_steps=n_steps, lm_from=min(n_forced) - 1,
+                           pos0=pad(pos0), batch=B, n_steps=n_steps, lm_from=min(n_forced) - 1,
                            epoch_base=self.epoch, seed=seed & 0xFFFFFFFF,
                            inv_temperature=1.0 / temperature if temperature > 0 else 0.0, n_stop=len(stop_ids),
                            prof_step=prof_step, stop_ids=stops.data_ptr(), tokens_out=out.data_ptr(),
                            logits_out=ptr(logits), step_ts=ptr(ts), out_info=info.data_ptr(), prof=ptr(prof),
                            spin_limit_ns=self.spin_limit_ns)
+        for j, body in enumerate(bodies):                  # behind everything that can be refused
+            if body:
+                self._take_in(body, self.bpos[j], seq=j, batched=True)
         stream = torch.cuda.current_stream(dev).cuda_stream
         _lib.check(self.lib.mk_launch_batch(self._h, ctypes.byref(a), ctypes.c_void_p(stream)))
         self.launches += 1
         done, epoch, _ = info[:3].tolist()          # synchronises with the launch
-        if int(self.status[0]) != 0:
-            where = ctypes.c_int32()
-            _lib.check(self.lib.mk_status(self._h, ctypes.byref(where)))
+        self._raise_if_timed_out()
         self.epoch = epoch & 0xFFFFFFFF
         if self.epoch > 0xFFFF0000:
             raise RuntimeError("epoch counter exhausted; call reset()")
@@ -542,7 +551,7 @@ class Megakernel:
                     ids = ids[: i + 1]
                     last = first + i + 1
                     break
-            self.bpos[j] += last
+            self.bpos[j] = pos0[j] + last
             result.append(ids)
             if return_logits:
                 result_logits.append(logits[first:last, j])
@@ -567,13 +576,14 @@ class Megakernel:
         launches of `chunk` steps), keeping the draft head's cache in step; the last token is handed back for the caller to
         feed with the first generation launch, as the reference's `prefill` does (`qwen_mk/engine.py:296-301`)."""
         *body, tail = [int(t) for t in tokens]
-        if len(body) >= MIN_PROMPT_ROWS:
+        n, start = len(body), self.pos
+        if n >= MIN_PROMPT_ROWS and self._attention_fits(start + n):
             self._enter_mode("single")
-            n, start = len(body), self.pos
             if start + n > self.max_seq:
                 raise ValueError(f"sequence would exceed max_seq={self.max_seq}")
             hidden = torch.empty(n, self.cfg.hidden, device=self.device) if self.mtp is not None else None
             self._take_in(body, start, hidden)
+            self._raise_if_timed_out()
             self.pos += n
             if hidden is not None:
                 self.mtp_fed(start, mtp_mod.rmsnorm(hidden, self.final_norm, self.cfg.eps), body)

@@ -157,3 +157,48 @@ def test_small_model_batched_prompts_equal_stepping(small, monkeypatch):
     assert ia == ib and a.bpos == b.bpos
     for x, y in zip(a.bstate + a.bconv_hist, b.bstate + b.bconv_hist):
         assert rel(x, y) < 2e-5
+
+
+def test_small_model_refused_calls_leave_the_state_alone(small):
+    """What a call refuses it refuses before the prompt goes in: bad arguments, formats and contexts the launch does not take."""
+    from megakernels_b200 import _lib
+    from megakernels_b200 import engine as E
+    from megakernels_b200.synth import make_prompt
+    prompt = make_prompt(small[0], 40)
+
+    def untouched(mk):
+        return mk.bpos == [0] * mk.batch and not any(bool(t.any()) for t in mk.bstate + mk.conv_hist + mk.bconv_hist + mk.k_cache)
+    mk = E.Megakernel(small[:2], max_seq=256, quant="bf16")
+    with pytest.raises((TypeError, ValueError)):
+        mk.run(prompt, n_generate=2, stop_ids=["end"])
+    assert untouched(mk)
+    mk.reset()
+    with pytest.raises(_lib.MkError, match="int8"):
+        mk.run_batch([prompt], n_generate=2)
+    assert untouched(mk)
+    mk = E.Megakernel(small[:2], max_seq=4096, quant="int8", batch=8)
+    with pytest.raises(_lib.MkError, match="too long"):
+        mk.run_batch([make_prompt(small[0], 4060)] * 8, n_generate=8)
+    assert untouched(mk)
+    lv, _, g = mk._tables
+    bare = dict(g, **dict.fromkeys(("xl", "projl", "mixl", "actl", "lml", "attn_part", "partl"), 0))
+    gv = _lib.i64_array([bare[f] for f in _lib.GLOBAL_FIELDS])
+    _lib.check(mk.lib.mk_set_params(mk._h, _lib.i64_array(lv), len(lv), None, 0, gv, len(gv)))
+    mk.reset()
+    with pytest.raises(_lib.MkError, match="hand-off"):
+        mk.prefill(prompt)
+    assert untouched(mk)
+
+
+def test_small_model_prefill_reports_a_wait_that_ran_out(small):
+    from megakernels_b200 import _lib
+    from megakernels_b200 import engine as E
+    from megakernels_b200.synth import make_prompt
+    mk = E.Megakernel(small[:2], max_seq=256, quant="int8")
+    mk.status[0] = _lib.MK_ERR_TIMEOUT                                # what a kernel leaves whose wait ran out
+    with pytest.raises(_lib.MkError) as err:
+        mk.prefill(make_prompt(small[0], 40))
+    assert err.value.code == _lib.MK_ERR_TIMEOUT and mk.pos == 0
+    mk.reset()
+    mk.prefill(make_prompt(small[0], 40))
+    assert mk.pos == 39
