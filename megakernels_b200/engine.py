@@ -327,7 +327,8 @@ class Megakernel:
 
     def reset(self):
         """Start a new sequence (cached K/V need no clearing: positions are rewritten)."""
-        torch._foreach_zero_(self.conv_hist + self.bconv_hist + self.bstate)      # a handful of launches for 54 tensors
+        if self.bstate:                                    # (a model may have no DeltaNet layer)
+            torch._foreach_zero_(self.conv_hist + self.bconv_hist + self.bstate)  # a handful of launches for 54 tensors
         torch._foreach_zero_(self.ll)
         self._mode = None              # "single" or "batch": the two kinds of launch keep separate conv histories
         self.bpos = [0] * self.batch   # position of every sequence; `pos` is that of sequence 0
@@ -749,6 +750,7 @@ class Megakernel:
 
     def restore(self, snap):
         tensors, pos, mode = snap
-        torch._foreach_copy_(self.conv_hist + self.bconv_hist + self.bstate, tensors)
+        if tensors:
+            torch._foreach_copy_(self.conv_hist + self.bconv_hist + self.bstate, tensors)
         self.bpos = list(pos)
         self._mode = mode

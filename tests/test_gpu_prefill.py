@@ -202,3 +202,32 @@ def test_small_model_prefill_reports_a_wait_that_ran_out(small):
     mk.reset()
     mk.prefill(make_prompt(small[0], 40))
     assert mk.pos == 39
+
+
+def test_small_model_without_a_deltanet_layer(lib_built):
+    """A model of attention layers alone has no recurrent state to clear, keep or put back."""
+    import dataclasses
+    from megakernels_b200 import engine as E
+    from megakernels_b200.config import qwen35_08b
+    from megakernels_b200.synth import make_prompt, make_weights
+    cfg = dataclasses.replace(qwen35_08b(n_layers=2, vocab=4096), layer_types=["full_attention"] * 2)
+    mk = E.Megakernel((cfg, make_weights(cfg, 0, init="realistic")), max_seq=128, quant="bf16")
+    prompt = make_prompt(cfg, 30)
+    first = mk.run(prompt, n_generate=4)
+    mk.reset()
+    tail = mk.prefill(prompt)
+    snap = mk.snapshot()
+    assert mk.run([tail], n_generate=4) == first
+    mk.restore(snap)
+    assert mk.pos == 29 and mk.run([tail], n_generate=4) == first
+
+
+def test_small_model_snapshots_kept_on_the_host(small):
+    from megakernels_b200 import engine as E
+    from megakernels_b200.synth import make_prompt
+    mk = E.Megakernel(small[:2], max_seq=128, quant="int8")
+    tail = mk.prefill(make_prompt(small[0], 30))
+    tensors, pos, mode = mk.snapshot()
+    first = mk.run([tail], n_generate=4)
+    mk.restore(([t.cpu() for t in tensors], pos, mode))
+    assert mk.run([tail], n_generate=4) == first
