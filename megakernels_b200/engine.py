@@ -392,21 +392,30 @@ class Megakernel:
         splits = min(self.grid // sequences // self.cfg.n_kv_heads, _lib.query("MAX_SPLITS"))
         return splits > 0 and 0 < self.lib.mk_plan_attn_chunk(last_pos, splits) <= _lib.query("MAX_CHUNK_POS")
 
+    def _prompt_room(self, n):
+        """Makes room for taking `n` tokens in at once: the path's workspace and its copy of the matrices (1 GB), both kept.
+        False where the device has no memory left for them: steps need neither."""
+        need = int(self.lib.mk_prefill_bytes(min(n, MAX_PROMPT_ROWS)))
+        try:
+            if self._workspace is None or self._workspace.numel() < need:
+                self._workspace = None
+                self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
+            if self._prompt_weights is None:
+                w = torch.empty(int(self.lib.mk_prefill_weight_bytes(self._h)), dtype=torch.uint8, device=self.device)
+                stream = torch.cuda.current_stream(self.device)
+                _lib.check(self.lib.mk_prefill_weights(self._h, w.data_ptr(), w.numel(), ctypes.c_void_p(stream.cuda_stream)))
+                stream.synchronize()                       # complete before a launch on any stream reads it
+                self._prompt_weights = w
+        except torch.cuda.OutOfMemoryError:
+            return False
+        return True
+
     def _take_in(self, tokens, start, hidden=None, seq=0, batched=False):
-        """`tokens` enter positions start, start + 1, ... of sequence `seq`, all at once (`mk_prefill`); `hidden` [n, hidden]
+        """`tokens` enter positions start, start + 1, ... of sequence `seq`, all at once (`mk_prefill`, behind `_prompt_room`); `hidden` [n, hidden]
         fp32 receives the residuals after the last layer.  Asynchronous; positions are the caller's to advance."""
         n = len(tokens)
-        need = int(self.lib.mk_prefill_bytes(min(n, MAX_PROMPT_ROWS)))
-        if self._workspace is None or self._workspace.numel() < need:
-            self._workspace = None
-            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
         ids = torch.tensor(tokens, dtype=torch.int32).to(self.device)
         stream = torch.cuda.current_stream(self.device).cuda_stream
-        if self._prompt_weights is None:
-            w = torch.empty(int(self.lib.mk_prefill_weight_bytes(self._h)), dtype=torch.uint8, device=self.device)
-            _lib.check(self.lib.mk_prefill_weights(self._h, w.data_ptr(), w.numel(), ctypes.c_void_p(stream)))
-            torch.cuda.current_stream(self.device).synchronize()      # complete before a launch on any stream reads it
-            self._prompt_weights = w
         for lo in range(0, n, MAX_PROMPT_ROWS):
             rows = min(MAX_PROMPT_ROWS, n - lo)
             a = _lib.PrefillArgs(tokens=ids.data_ptr() + 4 * lo, positions=rows, start_pos=start + lo, sequence=seq, batched=int(batched),
@@ -441,7 +450,7 @@ class Megakernel:
         # a long prompt goes in all at once, except its last token (whoever wants logits or times per token gets steps)
         # (a caller who asks for logits gets those of `mk_launch`, bit for bit, up to EXACT_PROMPT tokens)
         long = n_given > (max(EXACT_PROMPT, MIN_PROMPT_ROWS) if return_logits else MIN_PROMPT_ROWS)
-        taken = n_given - 1 if long and not all_logits and not timing and prof is None and self._attention_fits(start + n_steps) else 0
+        taken = n_given - 1 if long and not all_logits and not timing and prof is None and self._attention_fits(start + n_steps) and self._prompt_room(n_given - 1) else 0
         left, n_left = n_given - taken, n_steps - taken
         # everything that can be refused comes before the prompt changes the state
         hidden = torch.empty(n_steps, cfg.hidden, device=dev) if want_hidden else None
@@ -502,7 +511,8 @@ class Megakernel:
             raise ValueError(f"a sequence would exceed max_seq={self.max_seq}")
         dev = self.device
         # long prompts go in all at once, except their last tokens (times per step are times of steps)
-        rows = not timing and prof is None and self._attention_fits(max(self.bpos[:B]) + n_steps, B)
+        longest = max(n_forced)
+        rows = longest > MIN_PROMPT_ROWS and not timing and prof is None and self._attention_fits(max(self.bpos[:B]) + n_steps, B) and self._prompt_room(longest - 1)
         bodies = [p[:-1] if rows and len(p) > MIN_PROMPT_ROWS else [] for p in prompts]
         prompts = [p[len(b):] for p, b in zip(prompts, bodies)]
         pos0 = [self.bpos[j] + len(b) for j, b in enumerate(bodies)]
@@ -578,7 +588,7 @@ class Megakernel:
         feed with the first generation launch, as the reference's `prefill` does (`qwen_mk/engine.py:296-301`)."""
         *body, tail = [int(t) for t in tokens]
         n, start = len(body), self.pos
-        if n >= MIN_PROMPT_ROWS and self._attention_fits(start + n):
+        if n >= MIN_PROMPT_ROWS and self._attention_fits(start + n) and self._prompt_room(n):
             self._enter_mode("single")
             if start + n > self.max_seq:
                 raise ValueError(f"sequence would exceed max_seq={self.max_seq}")

@@ -215,8 +215,9 @@ class Runtime:
 
     def prefill(self, tokens):
         """A prompt of every sequence: `tokens` int32 [L, M] on the device.  Long ones go through the token-parallel path in
-        passes of at most MAX_ROWS rows, and only the LM head runs in the decode kernel; short ones, and programs that path
-        cannot run (two-piece inputs, tensor parallelism), step through the decode kernel."""
+        passes of at most MAX_ROWS rows, and only the LM head runs in the decode kernel; short ones, programs that path does
+        not run (two-piece inputs, tensor parallelism, records of another form), and prompts for whose workspace there is no
+        memory, step through the decode kernel."""
         L = tokens.shape[0]
         passes = -(-L * self.M // MAX_ROWS)
         each = -(-L // passes)
@@ -225,12 +226,15 @@ class Runtime:
             need = int(self.lib.mk_stage_prefill_bytes(self.host, self.n_stages, self.M, each, self.device.index))
             if need < 0 and need != _lib.MK_ERR_UNSUPPORTED:
                 _lib.check(need)
+        if need > 0 and (self._workspace is None or self._workspace.numel() < need):
+            self._workspace = None
+            try:
+                self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
+            except torch.cuda.OutOfMemoryError:
+                need = -1                       # no memory left for it: steps need none
         self.tok[: self.M].copy_(tokens[0])
         if need < 0:
             return self.launch(L, tokens_in=tokens)
-        if self._workspace is None or self._workspace.numel() < need:
-            self._workspace = None
-            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
         stream = torch.cuda.current_stream(self.device).cuda_stream
         for lo in range(0, L, each):
             part = tokens[lo: min(lo + each, L)]

@@ -231,3 +231,35 @@ def test_small_model_snapshots_kept_on_the_host(small):
     first = mk.run([tail], n_generate=4)
     mk.restore(([t.cpu() for t in tensors], pos, mode))
     assert mk.run([tail], n_generate=4) == first
+
+
+def test_prompts_step_where_no_memory_is_left(packed, small, monkeypatch):
+    from megakernels_b200 import engine as E
+    from megakernels_b200.synth import make_prompt
+    pkg, shape = SHAPES["27b"]
+    prompt, small_prompt = pkg.make_prompt(shape.vocab, 40, seed=3), make_prompt(small[0], 40)
+    engines = [pkg.Engine(packed("27b", {}), 1, maxlen=128) for _ in range(2)]
+    minis = [E.Megakernel(small[:2], max_seq=128, quant="int8") for _ in range(2)]
+    real = torch.empty
+
+    def full(*a, **k):
+        if k.get("dtype") == torch.uint8:
+            raise torch.cuda.OutOfMemoryError("no memory left")
+        return real(*a, **k)
+    got = []
+    for eng, mk, arm in zip(engines, minis, ("full", "stepping")):
+        with monkeypatch.context() as mp:
+            if arm == "full":
+                mp.setattr(torch, "empty", full)
+            else:
+                mp.setattr(runtime, "MIN_ROWS_PATH", 1 << 30)
+                mp.setattr(E, "MIN_PROMPT_ROWS", 1 << 30)
+            logits = eng.prefill([prompt]).clone()
+            tail = mk.prefill(small_prompt)
+            ids = mk.run([tail], n_generate=3)
+            mk.reset()
+            got.append((logits, ids, mk.run(small_prompt, n_generate=3), mk.bstate))
+        assert eng.rt._workspace is None and mk._workspace is None
+    (la, ia, ja, sa), (lb, ib, jb, sb) = got
+    assert torch.equal(la, lb) and ia == ib and ja == jb and all(torch.equal(x, y) for x, y in zip(sa, sb))
+    assert minis[0].run([1] * 30, n_generate=1) and minis[0]._workspace is not None     # memory again
