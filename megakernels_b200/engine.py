@@ -35,7 +35,9 @@ MAX_STEPS_PER_LAUNCH = 1024
 # Prompt tokens from which the token-parallel path takes a prompt in: it passes over the weights once (about 2 ms with its
 # launches) where stepping costs 0.4 ms per token.  Shorter ones keep the step path and its bits.
 MIN_PROMPT_ROWS = 16
-# ... and a run that returns logits keeps prompts up to this long on the step path: its logits are those of `mk_launch`.
+# ... and a single-sequence run that returns logits keeps prompts up to this long on the step path, at 0.4 ms per token: its
+# logits are then the bits of `mk_launch`, which `mk_launch_static` and logits kept from other runs can be compared with.
+# (Not a measured line: a page and a half.  Longer prompts differ from those bits by fp32 rounding, 1e-5 of their norm.)
 EXACT_PROMPT = 96
 # Positions of one pass of that path: bounds its workspace (about 150 KB per position).
 MAX_PROMPT_ROWS = 4096
@@ -428,7 +430,10 @@ class Megakernel:
     @torch.no_grad()
     def run(self, tokens, n_generate=1, temperature=0.0, seed=0, stop_ids=(), return_logits=False, prof=None,
             prof_step=0, timing=False, all_logits=False, track_mtp=False, return_resid=False):
-        """Feed `tokens`, then continue with up to `n_generate` tokens of the model's own choosing, in one launch.
+        """Feed `tokens`, then continue with up to `n_generate` tokens of the model's own choosing: one launch, behind the
+        passes of a prompt of more than MIN_PROMPT_ROWS tokens, which goes in all at once up to its last token.  (Such a
+        pass sums in another order than steps do, so chosen ids can differ from those of a call that steps where two logits
+        are equal to fp32 rounding; calls that ask for times, a profile, all logits, or logits of at most EXACT_PROMPT tokens step.)
 
         The contract is the reference's (`qwen_mk/engine.py:198-250`): the given tokens enter one per step; from the
         last of them on, every step's choice is fed to the next step on the GPU; choosing a stop id ends the launch,

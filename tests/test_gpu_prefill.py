@@ -132,8 +132,10 @@ def test_small_model_prompt_equals_stepping(small, monkeypatch, quant, kv, lengt
             if context:
                 mk.run(prompt[:context])
             mp.setattr(E, "MIN_PROMPT_ROWS", 16 if rows else 1 << 30)
+            mp.setattr(E, "EXACT_PROMPT", 0)                 # logits are asked for here
             mp.setattr(E, "MAX_PROMPT_ROWS", 120)            # several passes
             ids, logits = mk.run(prompt[context:], n_generate=6, return_logits=True, track_mtp=True)
+        assert (mk._workspace is not None) == rows           # one arm took the prompt in at once, the other stepped
         got.append((mk, ids, logits))
     (a, ia, la), (b, ib, lb) = got
     tol = 2e-5 if kv == "fp32" else 2e-4                      # a bf16 cache rounds
@@ -153,6 +155,7 @@ def test_small_model_batched_prompts_equal_stepping(small, monkeypatch):
         mk = E.Megakernel(small[:2], max_seq=256, quant="int8", batch=4)
         monkeypatch.setattr(E, "MIN_PROMPT_ROWS", rows)
         got.append((mk.run_batch(prompts, n_generate=8), mk))
+        assert (mk._workspace is not None) == (rows == 16)
     (ia, a), (ib, b) = got
     assert ia == ib and a.bpos == b.bpos
     for x, y in zip(a.bstate + a.bconv_hist, b.bstate + b.bconv_hist):
