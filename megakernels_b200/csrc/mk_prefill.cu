@@ -593,7 +593,7 @@ int prepare(Exec& E, const mk_stage_desc* prog, int n_stages, int batch, int pos
     E.M = batch;
     E.L = positions;
     E.rows = batch * positions;
-    token_tiles(E.rows, &E.ntiles, &E.nt);
+    token_tiles(E.rows, 256, &E.ntiles, &E.nt);
     E.xrows = E.ntiles * E.nt;
     const int rc = mk_stage_validate(prog, n_stages, batch);
     if (rc != MK_OK) return rc;

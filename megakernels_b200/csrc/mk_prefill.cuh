@@ -112,6 +112,7 @@ constexpr int A_BYTES = 128 * 128;                     // one 64-column block of
 constexpr int MAX_STAGES = 8;
 struct GemmBars {
     uint64_t full[MAX_STAGES], empty[MAX_STAGES], done;
+    uint64_t block_full[2], block_read[2];      // drained products: the two accumulators of the first piece
     uint32_t tmem;
     volatile int dead;
 };
@@ -328,10 +329,15 @@ __device__ __forceinline__ float block_scale(const GemmArgs& A, int group, int n
 // grid: x = token tile (neighbouring CTAs share weights, so HBM reads them once), y = 128-row weight block, z = K split;
 // routed groups: x = weight block, y = work item.
 // PX: bf16 pieces of the token operand (3: fp32-exact inputs); weight pieces: see the formats.
-// Three-piece inputs keep the products of the first piece in an accumulator of their own: an accumulation rounds its sum
-// towards zero, and the small terms of pieces 2 and 3 would add two more such roundings per step to the large sum.
-template <int FMT, int PX, int OUT, int CG>
-static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) rows_gemm(const __grid_constant__ GemmArgs A) {
+// An accumulation in tensor memory rounds its sum towards zero, once per instruction.  Three-piece inputs stand for fp32 ones,
+// and one accumulator for all of K left a 24-layer bf16 prompt five times as far from 64 bits as stepping (logits 1.9e-5 of
+// their norm against 4.0e-6).  So the small products of pieces 2 and 3 have an accumulator of their own, and the first piece's
+// sums are short:
+//   DG = 0  as many accumulators as tensor memory has room for, each over its share of K;
+//   DG > 0  two accumulators of one 64-column block each, in turn: the conversion warps, which have no weights to convert, add
+//           them up in registers, DG groups of sixteen tokens per warp, while the other one is filled.
+template <int FMT, int PX, int OUT, int CG, int DG>
+static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ? 2 : 1) rows_gemm(const __grid_constant__ GemmArgs A) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     constexpr int PW = weight_pieces<FMT>, CW = 8 * CG;
     constexpr int DIST = FMT == W_BF16 || FMT == W_FP8_PIECES3 ? 2 : (FMT == W_MXFP4 ? 6 : 4);        // blocks a lane requests ahead
@@ -356,14 +362,19 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
     const uint32_t x_bytes = (uint32_t)nt * 128u, stage_bytes = PW * A_BYTES + PX * (uint32_t)A.nt * 128u;
     GemmBars& B = *reinterpret_cast<GemmBars*>(smem + (size_t)A.stages * stage_bytes);
     const int blocks128 = FMT == W_FP8_BLOCK ? A.kbs / 2 : 1;   // (K splits do not occur with per-block accumulators)
+    const int first_accs = DG ? 2 : (PX > 1 ? min(512 / nt - 1, kb1 - kb0) : 1);
     int cols = 32;
-    while (cols < nt * (PX > 1 ? 2 : blocks128)) cols *= 2;
+    while (cols < nt * (PX > 1 ? 1 + first_accs : blocks128)) cols *= 2;
     if (threadIdx.x == 0) {
         for (int i = 0; i < A.stages; i++) {
             mbar_init(&B.full[i], FMT == W_SLAB ? 1 : 8 + 1);
             mbar_init(&B.empty[i], 1);
         }
         mbar_init(&B.done, 1);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&B.block_full[i], 1);
+            mbar_init(&B.block_read[i], 8);
+        }
         B.dead = 0;
         mk::fence_barrier_init();
     }
@@ -407,10 +418,11 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
         if (lane == 0) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | (8u << 24);   // f32 <- bf16 x bf16, M 128
             uint32_t slot = 0, phase = 0, first = 1;
-            bool ok = true;
+            int chunk = 0;                                        // of the first piece: its accumulator
+            bool ok = true, begin = true;
 #pragma unroll 1
             for (int kb = kb0; kb < kb1; kb++) {
-                if (!wait(B, A, &B.full[slot], phase, WP_FULL)) {
+                if ((DG && !wait(B, A, &B.block_read[(kb - kb0) & 1], (((kb - kb0) >> 1) & 1) ^ 1, WP_DRAIN)) || !wait(B, A, &B.full[slot], phase, WP_FULL)) {
                     ok = false;
                     break;
                 }
@@ -421,15 +433,24 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
 #pragma unroll
                     for (int pw = 0; pw < PW; pw++) {
                         const uint64_t da = operand_desc(st + pw * A_BYTES), db = operand_desc(st + PW * A_BYTES + px * (uint32_t)A.nt * 128u);
-                        const uint32_t d = tmem + (px ? (uint32_t)nt : 0u) + (FMT == W_FP8_BLOCK ? (uint32_t)((kb >> 1) * nt) : 0u);
+                        const uint32_t d = tmem + (PX > 1 ? (uint32_t)(px ? 0 : (1 + chunk) * nt) : 0u) + (FMT == W_FP8_BLOCK ? (uint32_t)((kb >> 1) * nt) : 0u);
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
-                            const uint32_t accumulate = !((FMT == W_FP8_BLOCK ? !(kb & 1) : first != 0) && k == 0 && pw == 0 && px <= 1);
+                            const bool starts = FMT == W_FP8_BLOCK ? !(kb & 1) : (PX > 1 && px == 0 ? begin : first != 0);
+                            const uint32_t accumulate = !(starts && k == 0 && pw == 0 && px <= 1);
                             asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
                                          ::"r"(d), "l"(da + 2 * k), "l"(db + 2 * k), "r"(idesc), "r"(accumulate));
                         }
                     }
                 first = 0;
+                if (DG) {
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&B.block_full[chunk])) : "memory");
+                    chunk ^= 1;
+                } else if (PX > 1) {
+                    const int next = (kb + 1 - kb0) * first_accs / (kb1 - kb0);
+                    begin = next != chunk;
+                    chunk = next;
+                }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&B.empty[slot])) : "memory");
                 if (++slot == (uint32_t)A.stages) {
                     slot = 0;
@@ -495,15 +516,45 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
                 }
             }
         }
+        // the sums of drained products: this lane's row, group g of sixteen tokens
+        float sums[DG ? DG : 1][16];
+        bool drained = true;
+        if constexpr (DG > 0) {
+#pragma unroll
+            for (int g = 0; g < DG; g++)
+#pragma unroll
+                for (int i = 0; i < 16; i++) sums[g][i] = 0.f;
+#pragma unroll 1
+            for (int b = 0; b < kb1 - kb0 && drained; b++) {
+                drained = __all_sync(0xffffffffu, wait(B, A, &B.block_full[b & 1], (b >> 1) & 1, WP_DRAIN));
+                if (!drained) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int g = 0; g < DG; g++) {
+                    const int c0 = (warp >> 2) * 16 + 32 * g;
+                    if (c0 < nt) {
+                        uint32_t r[16];
+                        load16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((1 + (b & 1)) * nt + c0), r);
+#pragma unroll
+                        for (int i = 0; i < 16; i++) sums[g][i] += __uint_as_float(r[i]);
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&B.block_read[b & 1]);
+            }
+        }
         // ---- epilogue: lane = weight row, columns = tokens; each set of four warps takes every 2 CG-th group of 16 tokens
-        const bool ok = __all_sync(0xffffffffu, wait(B, A, &B.done, 0, WP_DONE));
+        const bool ok = drained && __all_sync(0xffffffffu, wait(B, A, &B.done, 0, WP_DONE));
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int sub = warp & 3, n = block * 128 + sub * 32 + lane;
             float rs = 1.f;
             if (A.row_scale && n < A.n_valid) rs = __ldg(A.row_scale + (size_t)group * A.rs_gstride + (A.rs_pairs ? 2 * ((n >> 4) * 8 + (n & 7)) + ((n >> 3) & 1) : n));
-#pragma unroll 1
-            for (int c0 = (warp >> 2) * 16; c0 < nt; c0 += 32 * CG) {
+#pragma unroll(DG ? DG : 1)
+            for (int g = 0; g < (DG ? DG : 16); g++) {
+                const int c0 = (warp >> 2) * 16 + 32 * CG * g;
+                if (c0 >= nt) break;
                 float v[16];
                 {
                     uint32_t r[16];
@@ -520,10 +571,16 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 ? 2 : 1) row
                             for (int i = 0; i < 16; i++) v[i] = fmaf(__uint_as_float(r[i]), s, v[i]);
                         }
                     }
-                    if (PX > 1) {
-                        load16(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)(nt + c0), r);
+                    if constexpr (DG > 0) {
 #pragma unroll
-                        for (int i = 0; i < 16; i++) v[i] += __uint_as_float(r[i]);
+                        for (int i = 0; i < 16; i++) v[i] += sums[g][i];
+                    } else if (PX > 1) {
+#pragma unroll 1
+                        for (int a = 1; a <= first_accs; a++) {
+                            load16(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)(a * nt + c0), r);
+#pragma unroll
+                            for (int i = 0; i < 16; i++) v[i] += __uint_as_float(r[i]);
+                        }
                     }
                 }
 #pragma unroll

@@ -16,6 +16,8 @@ int mk_engine_view(mk_engine* e, const mk_model_desc** desc, const mk::Params** 
 namespace {
 
 constexpr int PX = 3;
+// Most tokens per tile: what rows_gemm adds up in registers (bf16 weights), or what leaves two accumulators for the first piece.
+int tile_tokens(int quant) { return quant == MK_QUANT_INT8 ? 160 : 32 * DRAIN_GROUPS; }
 
 // Weight rows in the decode layout (groups of up to eight rows, 64-byte k-blocks; pack.py: pack_rows) -> slabs.
 // A lane takes 16 bytes of a row; `glu` moves alternating gate / up rows into tiles of eight gates and their eight ups.
@@ -123,7 +125,7 @@ int to_slabs(const mk_model_desc* desc, const uint8_t* src, int N, int K, int un
 struct Run {
     const mk_model_desc* desc;
     const mk::Params* P;
-    int rows, nt, ntiles, xrows, sms, start, seq, batched;
+    int rows, nt, ntiles, xrows, sms, start, seq, batched, tile_most;
     const int* tokens;
     long long spin;
     cudaStream_t st;
@@ -136,7 +138,7 @@ struct Run {
     int* pos;
 
     void layout(float* resid) {
-        token_tiles(rows, &ntiles, &nt);
+        token_tiles(rows, tile_most, &ntiles, &nt);
         xrows = ntiles * nt;
         h = resid ? resid : arena.take<float>((size_t)rows * S::HID);
         y = arena.take<float>((size_t)rows * S::PROJ_MAX);
@@ -289,8 +291,14 @@ extern "C" int64_t mk_prefill_bytes(int positions) {
     Run R;
     memset(&R, 0, sizeof R);
     R.rows = positions;
-    R.layout(nullptr);
-    return (int64_t)R.arena.off + 1024;
+    size_t most = 0;
+    for (int quant : {MK_QUANT_BF16, MK_QUANT_INT8}) {
+        R.arena.off = 0;
+        R.tile_most = tile_tokens(quant);
+        R.layout(nullptr);
+        most = R.arena.off > most ? R.arena.off : most;
+    }
+    return (int64_t)most + 1024;
 }
 
 extern "C" int mk_prefill(mk_engine* e, const mk_prefill_args* a, void* stream) {
@@ -312,6 +320,7 @@ extern "C" int mk_prefill(mk_engine* e, const mk_prefill_args* a, void* stream) 
     MKP_CUDA(cudaSetDevice(R.desc->device));
     MKP_CUDA(cudaDeviceGetAttribute(&R.sms, cudaDevAttrMultiProcessorCount, R.desc->device));
     R.rows = a->positions;
+    R.tile_most = tile_tokens(R.desc->quant);
     R.start = a->start_pos;
     R.seq = a->sequence;
     R.batched = a->batched;

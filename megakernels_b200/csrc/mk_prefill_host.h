@@ -27,6 +27,7 @@ inline int pfail(int code, const char* fmt, ...) {
     } while (0)
 
 constexpr int SMEM_MAX = 232448;
+constexpr int DRAIN_GROUPS = 4;                     // rows_gemm: three-piece products in tiles of up to 32 x 4 tokens
 constexpr int MAX_ROWS = 65535;                     // token rows of a call: one grid coordinate of several kernels
 
 // Hands out the workspace; with base == nullptr it only counts.
@@ -42,9 +43,9 @@ struct Arena {
     }
 };
 
-template <int FMT, int PX, int CG>
+template <int FMT, int PX, int CG, int DG>
 int launch_gemm_cg(GemmArgs& A, int out, dim3 grid, int smem, cudaStream_t st) {
-    auto fn = out == OUT_STORE ? rows_gemm<FMT, PX, OUT_STORE, CG> : (out == OUT_ADD ? rows_gemm<FMT, PX, OUT_ADD, CG> : rows_gemm<FMT, PX, OUT_GLU, CG>);
+    auto fn = out == OUT_STORE ? rows_gemm<FMT, PX, OUT_STORE, CG, DG> : (out == OUT_ADD ? rows_gemm<FMT, PX, OUT_ADD, CG, DG> : rows_gemm<FMT, PX, OUT_GLU, CG, DG>);
     MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     fn<<<grid, (8 * CG + 2) * 32, smem, st>>>(A);
     MKP_CUDA(cudaGetLastError());
@@ -65,7 +66,18 @@ int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaSt
     A.stages = stages;
     const int smem = stages * stage + fixed;
     const dim3 grid = items ? dim3(blocks, items, 1) : dim3(tiles_x, blocks, A.ksplit);
-    const int rc = two || FMT == W_SLAB ? launch_gemm_cg<FMT, PX, 1>(A, out, grid, smem, st) : launch_gemm_cg<FMT, PX, FMT == W_SLAB ? 1 : 2>(A, out, grid, smem, st);
+    int rc;
+    if constexpr (FMT == W_SLAB) {
+        // Adding up in registers costs 3 % of a 512-token prompt and is what bf16 weights need.  Those of an int8 matrix (the ones
+        // with row scales) are integers of seven bits, whose products leave less to round away: with two accumulators for the
+        // first piece such a prompt is as close to 64 bits as stepping (logits 3.8e-6 of their norm against 3.7e-6 at 300
+        // tokens and 24 layers; with one 4.8e-6).
+        const bool drain = A.nt > 64 && !A.row_scale;
+        if (A.nt > (drain ? 32 * DRAIN_GROUPS : 160)) return pfail(MK_ERR_BADARG, "prefill: %d tokens per tile", A.nt);
+        rc = drain ? launch_gemm_cg<FMT, PX, 1, DRAIN_GROUPS>(A, out, grid, smem, st) : launch_gemm_cg<FMT, PX, 1, 0>(A, out, grid, smem, st);
+    } else {
+        rc = two ? launch_gemm_cg<FMT, PX, 1, 0>(A, out, grid, smem, st) : launch_gemm_cg<FMT, PX, 2, 0>(A, out, grid, smem, st);
+    }
     if (rc != MK_OK) return rc;
     if (A.ksplit > 1) {
         const dim3 fgrid(out == OUT_GLU ? (A.act_cols + 255) / 256 : (A.n_valid + 1023) / 1024, A.rows);
@@ -91,9 +103,9 @@ inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), int sms, cudaStre
     return MK_OK;
 }
 
-// Token tiles of `rows` rows: equal tiles of at most 256, multiples of 16.
-inline void token_tiles(int rows, int* n, int* nt) {
-    *n = (rows + 255) / 256;
+// Token tiles of `rows` rows: equal tiles of at most `most`, multiples of 16.
+inline void token_tiles(int rows, int most, int* n, int* nt) {
+    *n = (rows + most - 1) / most;
     *nt = ((rows + *n - 1) / *n + 15) / 16 * 16;
 }
 

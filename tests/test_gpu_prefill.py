@@ -266,3 +266,36 @@ def test_prompts_step_where_no_memory_is_left(packed, small, monkeypatch):
     (la, ia, ja, sa), (lb, ib, jb, sb) = got
     assert torch.equal(la, lb) and ia == ib and ja == jb and all(torch.equal(x, y) for x, y in zip(sa, sb))
     assert minis[0].run([1] * 30, n_generate=1) and minis[0]._workspace is not None     # memory again
+
+
+@pytest.mark.parametrize("quant,length", [("bf16", 30), ("bf16", 150), ("bf16", 260), ("int8", 170), ("int8", 320)])
+def test_small_model_prompts_are_as_exact_as_stepping(small, monkeypatch, quant, length):
+    """Both paths against the decoder in 64 bits: sums in tensor memory round towards zero, so long ones drift (a single
+    accumulator per product left a bf16 prompt five times as far from 64 bits as stepping).  Lengths: tiles of 32 and 80 to
+    160 tokens, one to three of them."""
+    from megakernels_b200 import engine as E
+    from megakernels_b200.quant import dequantized_weights
+    from megakernels_b200.synth import make_prompt
+    from oracle import decoder
+
+    def rms_norm(x, w, eps):
+        return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps) * (w + 1.0)
+    monkeypatch.setattr(decoder, "rms_norm", rms_norm)
+    cfg, w = small[:2]
+    prompt = make_prompt(cfg, length)
+    d = decoder.Decoder(cfg, dequantized_weights(w, quant), max_seq=length)
+    d.w, d.cos, d.sin = {k: v.double() for k, v in d.w.items()}, d.cos.double(), d.sin.double()
+    for kept in (d.conv_hist, d.state, d.k_cache, d.v_cache):
+        for k in kept:
+            kept[k] = kept[k].double()
+    for t in prompt[:-1]:
+        d.hidden_step(t)
+    off = []
+    for rows in (16, 1 << 30):
+        mk = E.Megakernel((cfg, w), max_seq=512, quant=quant)
+        monkeypatch.setattr(E, "MIN_PROMPT_ROWS", rows)
+        mk.prefill(prompt)
+        assert (mk._workspace is not None) == (rows == 16)
+        states = [rel(mk.deltanet_state(i).cpu(), s) for i, s in enumerate(d.state[i] for i in sorted(d.state))]
+        off.append(sum(states) / len(states))
+    assert off[0] < 1.5 * off[1] and off[0] < 5e-6, off
