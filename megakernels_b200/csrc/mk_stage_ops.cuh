@@ -600,8 +600,12 @@ __device__ __noinline__ void attn_stage(Shared& S, const mk_stage_desc& d) {
 //   * a warp scores a tile of 16 positions: A = 16 rows of K straight from global memory (the dot product may take the dims in
 //     any order, so a lane's 16-byte loads are its fragments), B = the query heads;
 //   * a warp then owns 64 dims of the output and every nres-th tile: A = the heads' probabilities (rows 0-7 their first bf16
-//     piece, rows 8-15 the second; the third in an MMA of its own: fp32-exact), B = V, again from global memory with the dims
-//     of a lane's 16 bytes spread over eight MMAs; pairs of positions are put together with byte permutes;
+//     piece, rows 8-15 the second; the third in an MMA of its own, also in rows 8-15: fp32-exact), B = V, again from global
+//     memory with the dims of a lane's 16 bytes spread over eight MMAs; pairs of positions are put together with byte permutes;
+//   * an MMA rounds its sums towards zero, so chains are short where that costs nothing: scores are folded every four MMAs, and
+//     the large sums of the first piece take one MMA per tile.  Off 64 bits by 1.9e-7 in a task of 250 positions and 256 dims
+//     (3.3e-7 with one chain per operand half and the third piece in rows 0-7; fp32 FMAs: 1.6e-7), growing with the tiles per
+//     warp: 4.2e-7 at 800 positions and 512 dims; fresh accumulators per tile would end that for 1 % of a step;
 //   * 256 positions at a time with a running maximum; one CTA barrier per 256.
 constexpr int ATTN_SUB = 256;             // positions between two barriers: one tile per warp
 // Buffers of cache-row offsets.  Sub-chunk s + 1's are written between the barriers of s - 1 and s, when a slower warp still
@@ -728,7 +732,7 @@ __device__ __noinline__ void attn_mma_stage(Shared& S, const mk_stage_desc& d) {
                     const __nv_bfloat16* ra = kc + row[ia] + t * 8;
                     const __nv_bfloat16* rb = kc + row[ib] + t * 8;
                     const uint8_t* q = qb + g * qb_stride + t * 16;
-                    float c2[4] = {0.f, 0.f, 0.f, 0.f};
+                    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
                     for (int e = 0; e < HD; e += 256) {
                         uint4 ka[8], kb[8];
@@ -741,12 +745,18 @@ __device__ __noinline__ void attn_mma_stage(Shared& S, const mk_stage_desc& d) {
                         for (int j = 0; j < 8; j++) {
                             const uint4 qv = *reinterpret_cast<const uint4*>(q + (e + j * 32) * 2);
                             const uint32_t a0[4] = {ka[j].x, kb[j].x, ka[j].y, kb[j].y}, a1[4] = {ka[j].z, kb[j].z, ka[j].w, kb[j].w};
-                            mma_bf16(c, a0, qv.x, qv.y);
-                            mma_bf16(c2, a1, qv.z, qv.w);
+                            mma_bf16(s0, a0, qv.x, qv.y);
+                            mma_bf16(s1, a1, qv.z, qv.w);
+                            if ((j & 3) == 3)
+#pragma unroll
+                                for (int i = 0; i < 4; i++) {
+                                    c[i] += s0[i] + s1[i];
+                                    s0[i] = s1[i] = 0.f;
+                                }
                         }
                     }
 #pragma unroll
-                    for (int i = 0; i < 4; i++) c[i] = (c[i] + c2[i]) * scale;
+                    for (int i = 0; i < 4; i++) c[i] *= scale;
                 }
                 if (ia >= ns) c[0] = c[1] = -3.0e38f;
                 if (ib >= ns) c[2] = c[3] = -3.0e38f;
@@ -816,7 +826,7 @@ __device__ __noinline__ void attn_mma_stage(Shared& S, const mk_stage_desc& d) {
                     pr[0] -= bf_lo(w0); pr[1] -= bf_hi(w0); pr[2] -= bf_lo(w1); pr[3] -= bf_hi(w1);
                     if (piece == 0) { hi[0] = w0; hi[2] = w1; }
                     if (piece == 1) { hi[1] = w0; hi[3] = w1; }
-                    if (piece == 2) { lw[0] = w0; lw[2] = w1; }
+                    if (piece == 2) { lw[1] = w0; lw[3] = w1; }
                 }
 #pragma unroll
                 for (int j = 0; j < 8; j++) {

@@ -26,7 +26,8 @@ def _head(x, w, cos, sin):
     return _bf(torch.cat([a * cos - b * sin, b * cos + a * sin, n[..., 2 * h:]], -1))
 
 
-def _run(M, nkv, qpk, HD, lengths, window=0, seed=0):
+def _run(M, nkv, qpk, HD, lengths, window=0, seed=0, exact=False):
+    """`exact`: queries and new keys of +-1 and no rotation, so that nothing but the attention itself rounds."""
     dev = torch.device("cuda", 0)
     grid = torch.cuda.get_device_properties(dev).multi_processor_count
     g = torch.Generator(device=dev).manual_seed(seed)
@@ -36,10 +37,14 @@ def _run(M, nkv, qpk, HD, lengths, window=0, seed=0):
     pr = Program(dev, M, grid)
     pr.embed(pr.zeros(4, 256, dtype=torch.bfloat16), pr.zeros(M, 256), pr.zeros(M, 16), None, 256, 4, keys_valid=False)
     width = nq * HD + 2 * nkv * HD
-    y, y2 = pr.hold(rnd(M, width)), pr.zeros(M, nq * HD)
+    y, y2 = rnd(M, width), pr.zeros(M, nq * HD)
     qn, kn = pr.hold(0.1 * rnd(HD)), pr.hold(0.1 * rnd(HD))
+    if exact:
+        y[:, : nq * HD + nkv * HD].sign_()
+        qn.zero_(), kn.zero_()
+    y = pr.hold(y)
     ang = torch.arange(maxlen, device=dev)[:, None] * (0.01 ** (torch.arange(rot // 2, device=dev) / (rot // 2)))[None]
-    cos, sin = pr.hold(ang.cos()), pr.hold(ang.sin())
+    cos, sin = (pr.hold((ang * (not exact)).cos()), pr.hold((ang * (not exact)).sin()))
     kc, vc = (pr.hold(rnd(M * nb, nkv, 64, HD).to(torch.bfloat16)) for _ in range(2))
     bt = pr.hold(torch.randperm(M * nb, device=dev, generator=g).reshape(M, nb).to(torch.int32))
     rec = -(-qpk * (HD + 2) // 4) * 4
@@ -70,6 +75,7 @@ def _run(M, nkv, qpk, HD, lengths, window=0, seed=0):
         err = float((y2.double() - want).norm() / want.norm())
         # a norm and a rotation in fp32 may round a query or key dim to the neighbouring bf16: 2^-9 of one of HD terms
         assert err < 1e-3, err
+    return err
 
 
 @pytest.mark.parametrize("M,nkv,qpk,HD,lengths,window", [
@@ -81,3 +87,10 @@ def _run(M, nkv, qpk, HD, lengths, window=0, seed=0):
 ])
 def test_attention_stage_matches_fp64(M, nkv, qpk, HD, lengths, window):
     _run(M, nkv, qpk, HD, lengths, window)
+
+
+@pytest.mark.parametrize("M,nkv,qpk,HD,n,bound", [(8, 4, 6, 256, 1000, 1.6e-7), (8, 8, 6, 256, 1600, 3e-7), (8, 8, 8, 512, 1600, 6e-7)])
+def test_attention_sums_round_towards_zero_in_short_chains(M, nkv, qpk, HD, n, bound):
+    """250, 800 and 800 positions per task: 1.2e-7, 2.1e-7 and 4.2e-7 measured; chains twice as long gave 1.9e-7, 4.6e-7 and
+    9.0e-7."""
+    assert _run(M, nkv, qpk, HD, [n] * M, seed=4, exact=True) < bound
