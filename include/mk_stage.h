@@ -253,7 +253,7 @@ typedef struct mk_stage_args {
     uint64_t tokens_in;      /* optional i32[n_tokens_in][batch]: the inputs of the first n_tokens_in steps (a prompt);
                                 step s < n_tokens_in feeds tokens_in[s] instead of `tok` / the previous choice    */
     int32_t xs_bytes;        /* shared staging area the program needs (mk_stage_scratch_bytes; 0: the maximum);
-                                what it leaves of the SM's shared memory becomes ring slots (2..4 per warp) */
+                                what it leaves of the SM's shared memory becomes ring slots (4 or 5 per warp) */
     int32_t n_tokens_in;
     uint64_t row_valid;      /* optional i32[batch]: 0 marks a padding row for this launch.  Its recurrent state, conv
                                 history, KV cache and position stay as they are and it selects no routed expert;

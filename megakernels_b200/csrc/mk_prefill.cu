@@ -300,6 +300,7 @@ struct Exec {
         if (q_w) q = arena.take<__nv_bfloat16>((size_t)rows * q_w);
         if (experts) {
             // tile width of the routed products: about twice the mean load, so that most experts are one tile
+            // (by estimate: narrower tiles leave fewer columns of padding, wider ones convert an expert's weights fewer times)
             const int mean = (int)((long long)rows * topk / experts);
             memset(&route, 0, sizeof route);
             route.nt = mean > 96 ? 256 : (mean > 40 ? 128 : (mean > 16 ? 64 : 32));

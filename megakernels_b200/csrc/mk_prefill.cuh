@@ -3,9 +3,10 @@
 //
 // The contractions are matrix products here, so they run on the 5th-generation tensor cores: `rows_gemm` keeps 128
 // weight rows as the A operand of tcgen05.mma and up to 256 token rows as its N columns, accumulators in tensor
-// memory.  The weights stay in the decode kernel's packed tiles: eight warps read a tile step each with one 128-bit
-// load per lane, convert it to bf16 (exact for every format) and write the swizzled operand into shared memory, so
-// a prompt reads the same bytes from HBM as a decode step does and no second copy of the model exists.
+// memory.  The weights of a stage program stay in the decode kernel's packed tiles: eight or sixteen warps read a tile
+// step each with one 128-bit load per lane, convert it to bf16 pieces that hold its value and write the swizzled operand
+// into shared memory, so a prompt reads the same bytes from HBM as a decode step does and needs no second copy of the
+// model.  (The 0.8B model does keep one: mk_prefill_08b.cu.)
 //
 // Operand layout in global memory ("slabs"): a matrix of R token rows and K columns is stored as K / 64 slabs of R
 // rows x 128 bytes, the 16-byte pieces of a row swizzled with its number (piece p of row r sits at p ^ (r & 7)).

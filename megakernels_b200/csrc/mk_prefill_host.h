@@ -110,7 +110,8 @@ inline void token_tiles(int rows, int most, int* n, int* nt) {
 }
 
 // CTAs that share the K range of one tile: the count with the shortest schedule (rounds of one CTA per SM, each 64-column
-// block counted once and the start and end of a CTA as six), at least eight blocks each.
+// block counted once, the start and end of a CTA as six and the pass that adds the partials as 4 + z: estimates), at least
+// eight blocks each.
 inline int pick_ksplit(int ctas, int kbs, int sms) {
     int best = 1;
     double cost = 1e30;

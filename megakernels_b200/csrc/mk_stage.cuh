@@ -169,7 +169,7 @@ __device__ __forceinline__ int warp_() { return (int)(threadIdx.x >> 5); }
 __device__ __forceinline__ int lane_() { return (int)(threadIdx.x & 31); }
 __device__ __forceinline__ int cta_() { return (int)blockIdx.x; }
 __device__ __forceinline__ int grid_() { return (int)gridDim.x; }
-constexpr int PROF_FIELDS = 8;  // per stage: entered, input staged, units done, barrier passed, ring-wait ns of warp 0
+constexpr int PROF_FIELDS = 8;  // per stage: entered, input staged, work done, barrier passed, then up to three marks inside staging or attention
 __device__ __forceinline__ void prof_mark(Shared& S, int field) {
     if (S.prof && tid_() == 0) S.prof[field] = globaltimer();
 }
@@ -353,11 +353,10 @@ __device__ __forceinline__ const float* group_row_scale(const Shared& S, const m
 
 // ---- the weight stream of a consumer warp --------------------------------------------------------------------
 // A warp requests its own weights, block by block (four tile steps), in the order it multiplies them: lane j copies the 16
-// bytes per step that lane j will read, and right after a block has been read the slot takes the next request.  Earlier,
-// a producer warp filled two slots of a whole chunk per consumer warp and polled sixteen release barriers for free ones; with
-// half of the ring in flight at most, and the polls sharing issue slots with the multiplication, a 95 MB MXFP4 matrix
-// streamed at 3.0 TB/s where the same loop with the data in place runs at 5.9.
-//
+// bytes per step that lane j will read, and right after a block has been read the slot takes the next request.  So all of the
+// ring but one block is in flight, and nobody polls for free slots.  (A 95 MB MXFP4 matrix: 34 us for its stage; a producer
+// warp that filled two slots of a whole chunk per consumer warp streamed at 3.0 TB/s where the same loop with the data in
+// place runs at 5.9.)
 __device__ __noinline__ void stream_error(Shared& S, uint32_t stage, int where) {
     if (atomicCAS(S.A.status, 0, -5) == 0) {
         S.A.status[1] = (int)stage;
@@ -385,13 +384,15 @@ __device__ __forceinline__ Share batch_share(const Shared& S, const Geo& g, cons
     r.cpt = (bt.seg1 - bt.seg0) * g.n_chunks;
     // Equal shares of whole chunks, the first warps first: as long as the longest share is no longer, every warp without one
     // is a partial tile less to add.  Fewer chunks than warps go to FEW_WARPS: two or three chunks in a row cost less than
-    // the exchange (27B x1 per step 1417 -> 1382 us, 35B-A3B x8 1531 -> 1494 us).
+    // the exchange.  (Both rules together, 8 and 6 layers: 27B x1 per step 1417 -> 1373 us, x8 1699 -> 1656 us, 35B-A3B x8
+    // 1531 -> 1493 us, 26B x4 1419 -> 1413 us; the second one's own part was not measured.)
     const int n = (bt.t1 - bt.t0) * r.cpt, warps = n < NCW && n > FEW_WARPS ? FEW_WARPS : NCW;
     r.per = (n + warps - 1) / warps;
     r.c = min(n, w * r.per);
     r.c1 = min(n, r.c + r.per);
     if (g.routed && !g.reduce) {
-        // many tiles of many experts: cut as evenly as chunks allow (per < 0: minus all of the batch's chunks)
+        // many tiles of many experts: cut as evenly as chunks allow.  `per` then holds minus the batch's chunks, from which
+        // multiply() finds the warp that has a tile's last chunk.
         r.per = -n;
         r.c = n * w / NCW;
         r.c1 = n * (w + 1) / NCW;
@@ -572,8 +573,9 @@ __device__ __forceinline__ bool scout_wait(Shared& S, volatile unsigned* word, u
     return true;
 }
 // Two GEMV stages without a barrier between them do not depend on each other, and a small one is all latency: they share the
-// grid in proportion to their weights, at least a CTA per tile of a small second one (up to a tenth of the grid).  One after
-// the other the router of a 35B-A3B layer's neighbours cost 17 us behind 13 to 21.  -> CTAs of the second.
+// grid in proportion to their weights, at least a CTA per tile of a small one (up to a tenth of the grid: an estimate).  One
+// after the other, the gates' projection behind a 35B-A3B DeltaNet layer's qkvz, and in a 26B layer the router behind the
+// dense gate and up and the experts' down behind the dense one, cost their whole latency, 13 to 20 us each.  -> CTAs of the second.
 __device__ __forceinline__ int side_by_side(const mk_stage_desc& a, const mk_stage_desc& b, int n_groups, int grid) {
     const float ta = (float)a.i[MKS_I_TILES] * (a.i[MKS_I_GROUPS] < 0 ? n_groups : a.i[MKS_I_GROUPS]);
     const float tb = (float)b.i[MKS_I_TILES] * (b.i[MKS_I_GROUPS] < 0 ? n_groups : b.i[MKS_I_GROUPS]);
@@ -821,8 +823,8 @@ __device__ __noinline__ void stage_wide(Shared& S, const mk_stage_desc& d, int s
     }
 }
 // Routed groups that are added up (an expert's down projection), one piece, no norm: few sequences give a group any weight, so
-// a warp takes one (K split, sequence) pair at a time, finds its scale by itself and leaves the other columns zero.  The
-// general staging below went through all of them: 11 us for the ten experts of a panel at eight sequences.
+// a warp takes one (K split, sequence) pair at a time, finds its scale by itself and leaves the other columns zero.  (The
+// general staging below goes through all of them: 11 us for the ten experts of a panel at eight sequences.)
 __device__ __noinline__ void stage_routed(Shared& S, const mk_stage_desc& d, int seg0, int seg1, int n_splits) {
     const int kc = d.i[MKS_I_KC], M = S.A.M, nseg = seg1 - seg0, stride = xs_stride_bytes(nseg * kc);
     const bool bf16 = d.i[MKS_I_FMT] == MKS_FMT_BF16;

@@ -593,9 +593,9 @@ __device__ __noinline__ void attn_stage(Shared& S, const mk_stage_desc& d) {
     }
 }
 
-// bf16 caches and bf16 queries (every model's default): the same task on the tensor cores.  What bounded it: a task of 220
-// positions spent 65 us on fp32 FMAs with one shared-memory read per eight of them, three CTA barriers and two trips through
-// global scratch, and a chunk size fixed for the longest context left some CTAs a second task.  Here
+// bf16 caches and bf16 queries (every model's default): the same task on the tensor cores.  (attn_stage takes 65 us for 220
+// positions: fp32 FMAs with one shared-memory read per eight of them, three CTA barriers and two trips through global scratch,
+// and its chunk size, fixed for the longest context, can leave some CTAs a second task.)  Here
 //   * the chunks of a (sequence, KV head) are as many as give every CTA one task at the present lengths;
 //   * a warp scores a tile of 16 positions: A = 16 rows of K straight from global memory (the dot product may take the dims in
 //     any order, so a lane's 16-byte loads are its fragments), B = the query heads;
