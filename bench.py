@@ -45,7 +45,7 @@ NCU_CONTEXT = 64
 # stage_kernel: dram bytes of the captured launch (8 of 64 layers, vocabulary 32768, batch 8, 8 steps) over the
 # algorithmic bytes of that launch; the bench scales its own algorithmic bytes by it (the capture of the full model
 # would hold 20 GB on the device under the profiler)
-NCU_STAGE_TRAFFIC_RATIO = (17.065627e9 + 2.102116e9) / 18.072158208e9
+NCU_STAGE_TRAFFIC_RATIO = (17.162017e9 + 3.451152e9) / 18.072158208e9
 
 
 def measured_peak_gbs():
