@@ -186,7 +186,8 @@ struct Slab { uint64_t key; const void* norm; float in_scale; uint8_t* x; int ro
 
 struct Exec {
     const mk_stage_desc* prog;
-    int n_stages, M, L, rows, xrows, ntiles, nt, sms;
+    int n_stages, M, L, rows, xrows = 0, sms;
+    struct Tiling { int n, nt, ksplit; } tile[2];          // of the token rows: at most 256 and at most 384 a tile
     const int* tokens;
     int* pos;
     int* status;
@@ -246,6 +247,27 @@ struct Exec {
         }
     }
 
+    // How a dense product is cut.  A CTA converts its weights once for all tokens of its tile, which takes sixteen warps about 860
+    // cycles per 64 columns; up to 256 tokens hide behind that (MXFP4, 192 tokens: the tensor cores are busy 43 % of the time).  Wider
+    // tiles convert less often, and what then counts is shared memory: about 10 / 3 cycles per token (384 tokens: 1270).
+    static constexpr int CONVERT = 860;
+    Tiling tiling(const mk_stage_desc& d) const {
+        const int blocks = (d.i[MKS_I_TILES] + 7) / 8, kbs = d.i[MKS_I_KC] * d.i[MKS_I_SPLITS] / 64, fmt = format(d);
+        Tiling best = tile[0];
+        double cost = 0.;
+        for (int i = 0; i < (fmt == W_FP8_PIECES2 || fmt == W_FP8_PIECES3 ? 1 : 2); i++) {
+            Tiling t = tile[i];
+            t.ksplit = pick_ksplit(blocks * t.n, kbs, sms);
+            const int per = (kbs + t.ksplit - 1) / t.ksplit + 6;
+            const double c = (double)((blocks * t.n * t.ksplit + sms - 1) / sms) * per * (10 * t.nt > 3 * CONVERT ? 10. * t.nt / 3 : (double)CONVERT);
+            if (!i || c < cost) {
+                best = t;
+                cost = c;
+            }
+        }
+        return best;
+    }
+
     void layout() {
         for (int s = 0; s < n_stages; s++) {
             const mk_stage_desc& d = prog[s];
@@ -272,7 +294,7 @@ struct Exec {
                 if (routed && d.i[MKS_I_EPILOGUE] != MKS_E_GLU) up(ex_n, d.i[MKS_I_N_VALID]);
                 if (K > kmax) kmax = K;
                 if (!routed) {
-                    const int blocks = (d.i[MKS_I_TILES] + 7) / 8, z = pick_ksplit(blocks * ntiles, K / 64, sms);
+                    const int z = tiling(d).ksplit;
                     if (z > 1) up(part_floats, (size_t)z * rows * (d.i[MKS_I_EPILOGUE] == MKS_E_GLU ? d.i[MKS_I_TILES] * 16 : d.i[MKS_I_N_VALID]));
                 }
             } else if (d.op == MKS_OP_GDN) {
@@ -324,7 +346,7 @@ struct Exec {
     }
 
     int gemm(const mk_stage_desc& d, GemmArgs& A, int out, int items) {
-        const int blocks = (d.i[MKS_I_TILES] + 7) / 8;
+        const int blocks = (d.i[MKS_I_TILES] + 7) / 8, ntiles = (A.rows + A.nt - 1) / A.nt;
         const int fmt = format(d);
         if ((fmt == W_FP8_PIECES2 || fmt == W_FP8_PIECES3) && A.ksplit == 1 && A.nt * (A.kbs / 2) <= 512 && A.kbs % 2 == 0)
             return launch_gemm<W_FP8_BLOCK, 1>(A, out, blocks, ntiles, items, st);
@@ -349,7 +371,7 @@ struct Exec {
         A.kbs = d.i[MKS_I_KC] * d.i[MKS_I_SPLITS] / 64;
         A.ksplit = 1;
         A.rows = rows;
-        A.nt = nt;
+        A.nt = tile[0].nt;
         A.gelu = d.i[MKS_I_ACT] == MKS_ACT_GELU_TANH;
         A.n_valid = d.i[MKS_I_EPILOGUE] == MKS_E_GLU ? d.i[MKS_I_TILES] * 16 : d.i[MKS_I_N_VALID];
         A.act_cols = d.i[MKS_I_N_VALID];
@@ -386,7 +408,9 @@ struct Exec {
         GemmArgs A = args(d);
         int rc = operand(d, &A.x, &A.x_rows);
         if (rc != MK_OK) return rc;
-        A.ksplit = pick_ksplit((d.i[MKS_I_TILES] + 7) / 8 * ntiles, A.kbs, sms);
+        const Tiling t = tiling(d);
+        A.nt = t.nt;
+        A.ksplit = t.ksplit;
         A.part = part;
         A.part_rows = rows;
         int out;
@@ -594,8 +618,9 @@ int prepare(Exec& E, const mk_stage_desc* prog, int n_stages, int batch, int pos
     E.M = batch;
     E.L = positions;
     E.rows = batch * positions;
-    token_tiles(E.rows, 256, &E.ntiles, &E.nt);
-    E.xrows = E.ntiles * E.nt;
+    token_tiles(E.rows, 256, &E.tile[0].n, &E.tile[0].nt);
+    token_tiles(E.rows, 384, &E.tile[1].n, &E.tile[1].nt);
+    for (auto& t : E.tile) E.xrows = E.xrows > t.n * t.nt ? E.xrows : t.n * t.nt;
     const int rc = mk_stage_validate(prog, n_stages, batch);
     if (rc != MK_OK) return rc;
     if (const char* why = refuse(prog, n_stages, batch)) return pfail(MK_ERR_UNSUPPORTED, "prefill: %s", why);

@@ -95,7 +95,7 @@ struct GemmArgs {
     int act_rows, act_cols;      // activation columns (n_valid pairs)
     int n_valid;                 // weight rows that exist
     int rows;                    // token rows that exist (dense)
-    int nt;                      // tokens per tile (a multiple of 16, <= 256)
+    int nt;                      // tokens per tile (a multiple of 16; <= 384, with pieces or per-block accumulators 256)
     int kbs;                     // 64-column blocks of K
     int ksplit;                  // CTAs that share K; > 1: fp32 partials [split][part_rows][n_valid] in `part`
     float* part;
@@ -337,7 +337,7 @@ __device__ __forceinline__ float block_scale(const GemmArgs& A, int group, int n
 //   DG = 0  as many accumulators as tensor memory has room for, each over its share of K;
 //   DG > 0  two accumulators of one 64-column block each, in turn: the conversion warps, which have no weights to convert, add
 //           them up in registers, DG groups of sixteen tokens per warp, while the other one is filled.
-template <int FMT, int PX, int OUT, int CG, int DG>
+template <int FMT, int PX, int OUT, int CG, int DG, bool WIDE = false>
 static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ? 2 : 1) rows_gemm(const __grid_constant__ GemmArgs A) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     constexpr int PW = weight_pieces<FMT>, CW = 8 * CG;
@@ -417,7 +417,9 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ?
         }
     } else if (warp == CW + 1) {
         if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | (8u << 24);   // f32 <- bf16 x bf16, M 128
+            // f32 <- bf16 x bf16, M 128; an instruction has at most 256 columns, so a wide tile takes two
+            const uint32_t n0 = WIDE ? (uint32_t)((nt / 2 + 15) & ~15) : (uint32_t)nt, n1 = (uint32_t)nt - n0;
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((n0 >> 3) << 17) | (8u << 24), idesc1 = (1u << 4) | (1u << 7) | (1u << 10) | ((n1 >> 3) << 17) | (8u << 24);
             uint32_t slot = 0, phase = 0, first = 1;
             int chunk = 0;                                        // of the first piece: its accumulator
             bool ok = true, begin = true;
@@ -441,6 +443,9 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ?
                             const uint32_t accumulate = !(starts && k == 0 && pw == 0 && px <= 1);
                             asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
                                          ::"r"(d), "l"(da + 2 * k), "l"(db + 2 * k), "r"(idesc), "r"(accumulate));
+                            if constexpr (WIDE)              // the rows past n0 (whole groups of eight)
+                                asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                                             ::"r"(d + n0), "l"(da + 2 * k), "l"(db + (uint64_t)(n0 * 8) + 2 * k), "r"(idesc1), "r"(accumulate));
                         }
                     }
                 first = 0;

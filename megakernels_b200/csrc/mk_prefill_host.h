@@ -43,9 +43,9 @@ struct Arena {
     }
 };
 
-template <int FMT, int PX, int CG, int DG>
+template <int FMT, int PX, int CG, int DG, bool WIDE = false>
 int launch_gemm_cg(GemmArgs& A, int out, dim3 grid, int smem, cudaStream_t st) {
-    auto fn = out == OUT_STORE ? rows_gemm<FMT, PX, OUT_STORE, CG, DG> : (out == OUT_ADD ? rows_gemm<FMT, PX, OUT_ADD, CG, DG> : rows_gemm<FMT, PX, OUT_GLU, CG, DG>);
+    auto fn = out == OUT_STORE ? rows_gemm<FMT, PX, OUT_STORE, CG, DG, WIDE> : (out == OUT_ADD ? rows_gemm<FMT, PX, OUT_ADD, CG, DG, WIDE> : rows_gemm<FMT, PX, OUT_GLU, CG, DG, WIDE>);
     MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     fn<<<grid, (8 * CG + 2) * 32, smem, st>>>(A);
     MKP_CUDA(cudaGetLastError());
@@ -76,7 +76,12 @@ int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaSt
         if (A.nt > (drain ? 32 * DRAIN_GROUPS : 160)) return pfail(MK_ERR_BADARG, "prefill: %d tokens per tile", A.nt);
         rc = drain ? launch_gemm_cg<FMT, PX, 1, DRAIN_GROUPS>(A, out, grid, smem, st) : launch_gemm_cg<FMT, PX, 1, 0>(A, out, grid, smem, st);
     } else {
-        rc = two ? launch_gemm_cg<FMT, PX, 1, 0>(A, out, grid, smem, st) : launch_gemm_cg<FMT, PX, 2, 0>(A, out, grid, smem, st);
+        if (A.nt > 256) {
+            if constexpr (PW == 1 && FMT != W_FP8_BLOCK) rc = launch_gemm_cg<FMT, PX, 2, 0, true>(A, out, grid, smem, st);
+            else return pfail(MK_ERR_BADARG, "prefill: %d tokens per tile", A.nt);
+        } else {
+            rc = two ? launch_gemm_cg<FMT, PX, 1, 0>(A, out, grid, smem, st) : launch_gemm_cg<FMT, PX, 2, 0>(A, out, grid, smem, st);
+        }
     }
     if (rc != MK_OK) return rc;
     if (A.ksplit > 1) {
