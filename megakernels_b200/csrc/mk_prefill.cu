@@ -208,6 +208,7 @@ struct Exec {
     RouteArgs route;
     uint8_t* xg = nullptr;               // gathered slabs
     int slot_rows = 0, max_items = 0;
+    bool few = false;                                     // the routed products are those of experts_gemm
     float *yg = nullptr, *ys = nullptr;
     uint8_t *act_g = nullptr, *act_s = nullptr;
 
@@ -277,6 +278,7 @@ struct Exec {
         }
         for (auto& b : bufs) b.rows = arena.take<float>((size_t)rows * b.width);
         int kmax = 0, experts = 0, topk = 0;
+        bool fp8 = true, scaled = false;      // the experts' weights
         size_t conv = 0, heads = 0, vals = 0, q_w = 0, ex_k = 0, ex_n = 0, ex_f = 0, sh = 0;
         for (int s = 0; s < n_stages; s++) {
             const mk_stage_desc& d = prog[s];
@@ -284,6 +286,10 @@ struct Exec {
             if (d.op == MKS_OP_GEMV && d.i[MKS_I_EPILOGUE] != MKS_E_LOGITS) {
                 const int K = d.i[MKS_I_KC] * d.i[MKS_I_SPLITS];
                 const bool routed = d.i[MKS_I_GROUPS] < 0;
+                if (routed) {
+                    fp8 &= d.i[MKS_I_FMT] == MKS_FMT_FP8;
+                    scaled |= d.i[MKS_I_BLOCK_SCALES] != 0;
+                }
                 if (d.i[MKS_I_EPILOGUE] == MKS_E_GLU) {
                     if (routed) {
                         up(ex_k, K);
@@ -325,7 +331,9 @@ struct Exec {
             // (by estimate: narrower tiles leave fewer columns of padding, wider ones convert an expert's weights fewer times)
             const int mean = (int)((long long)rows * topk / experts);
             memset(&route, 0, sizeof route);
-            route.nt = mean > 96 ? 256 : (mean > 40 ? 128 : (mean > 16 ? 64 : 32));
+            few = fp8 && mean <= (scaled ? 32 : 16);
+            if (few) route.nt = 32;
+            else route.nt = mean > 96 ? 256 : (mean > 40 ? 128 : (mean > 16 ? 64 : 32));
             slot_rows = (rows * topk + experts * 15 + route.nt + 15) / 16 * 16;
             max_items = experts + rows * topk / route.nt + 1;
             if (max_items > rows * topk) max_items = rows * topk;
@@ -444,7 +452,8 @@ struct Exec {
                 rc = gemm(d, S, OUT_GLU, 0);
                 if (rc != MK_OK) return rc;
             }
-            gather_rows<<<rows, 256, 0, st>>>(A.x, A.x_rows, route.slot, route.topk, A.kbs, xg, slot_rows);
+            auto gather = few ? gather_rows<true> : gather_rows<false>;
+            gather<<<rows, 256, 0, st>>>(A.x, A.x_rows, route.slot, route.topk, A.kbs, xg, slot_rows);
             MKP_CUDA(cudaGetLastError());
             A.x = xg;
             A.act = act_g;
@@ -471,7 +480,10 @@ struct Exec {
         A.nt = route.nt;
         A.items = route.items;
         A.n_items = route.n_items;
-        rc = gemm(d, A, up ? OUT_GLU : OUT_STORE, max_items);
+        const int out = up ? OUT_GLU : OUT_STORE;
+        A.blocks = (d.i[MKS_I_TILES] + 7) / 8;
+        if (!few) rc = gemm(d, A, out, max_items);
+        else rc = d.i[MKS_I_BLOCK_SCALES] ? launch_experts<true, 4>(A, out, max_items, sms, st) : launch_experts<false, 4>(A, out, max_items, sms, st);
         if (rc != MK_OK || up) return rc;
         combine_rows<<<rows, 256, 0, st>>>(yg, d.i[MKS_I_N_VALID], route.slot, route.weight, route.topk, shared ? ys : nullptr, route.gate,
                                            d.i[MKS_I_EPILOGUE] == MKS_E_RESID, at(d.p[MKS_P_OUT]), d.i[MKS_I_OUT_STRIDE]);

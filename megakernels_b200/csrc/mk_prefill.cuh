@@ -97,6 +97,7 @@ struct GemmArgs {
     int rows;                    // token rows that exist (dense)
     int nt;                      // tokens per tile (a multiple of 16; <= 384, with pieces or per-block accumulators 256)
     int kbs;                     // 64-column blocks of K
+    int blocks;                  // experts_gemm: 128-row blocks of a group
     int ksplit;                  // CTAs that share K; > 1: fp32 partials [split][part_rows][n_valid] in `part`
     float* part;
     int part_rows;
@@ -118,17 +119,17 @@ struct GemmBars {
     volatile int dead;
 };
 
-static __device__ __noinline__ bool wait_slow(GemmBars& B, const GemmArgs& A, uint64_t* b, uint32_t parity, int site) {
+static __device__ __noinline__ bool wait_slow(volatile int* dead, const GemmArgs& A, uint64_t* b, uint32_t parity, int site) {
     u64 t0 = 0;
 #pragma unroll 1
     for (unsigned it = 0;; it++) {
         if (mbar_try_wait(b, parity)) return true;
         if ((it & 63u) == 63u) {
-            if (B.dead) return false;
+            if (*dead) return false;
             const u64 now = mk::globaltimer();
             if (!t0) t0 = now;
             else if (now - t0 > (u64)A.spin_limit_ns) {
-                B.dead = 1;
+                *dead = 1;
                 if (atomicCAS(A.status, 0, ERR_TIMEOUT) == 0) {
                     A.status[1] = site;
                     A.status[2] = (int)blockIdx.x;
@@ -139,8 +140,9 @@ static __device__ __noinline__ bool wait_slow(GemmBars& B, const GemmArgs& A, ui
         }
     }
 }
-__device__ __forceinline__ bool wait(GemmBars& B, const GemmArgs& A, uint64_t* b, uint32_t parity, int site) {
-    return mbar_try_wait(b, parity) || wait_slow(B, A, b, parity, site);
+template <class Bars>
+__device__ __forceinline__ bool wait(Bars& B, const GemmArgs& A, uint64_t* b, uint32_t parity, int site) {
+    return mbar_try_wait(b, parity) || wait_slow(&B.dead, A, b, parity, site);
 }
 
 // K-major SWIZZLE_128B operand: rows of 128 bytes, eight-row groups 1024 bytes apart
@@ -1590,6 +1592,207 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
     }
 }
 
+// ---- products of a few rows per expert -----------------------------------------------------------------------
+// A routed group has a few dozen token rows, so its product is a stream of weights, and what limits it is what happens to a weight on
+// the way: through shared memory into the tensor cores' operand (rows_gemm) it costs some 300 instructions per 16 x 64 tile,
+// which kept the stream at 1.5 of 6.5 TB/s.  The packed tiles are the register fragments of mma.sync, so here they stay in the
+// warp that loaded them: 9 instructions turn four fp8 bytes into two bf16 pairs and the MMA takes them as they are.
+//   A unit is 128 weight rows (eight warps, a tile each) times the rows of a work item; CTAs take units in turn and warps run on
+// from unit to unit, each at its own pace.  Token rows come in stages of 128 columns by bulk copies of a ninth warp.
+//   Columns of a token row are stored (gather_rows, the epilogue below) in the order in which the fragments hold those of the
+// weights: of sixteen columns the even ones, then the odd ones.  Block-scaled FP8 adds an accumulator per 128 columns with the
+// block's scale to fp32 sums (the decode kernel's arithmetic); row scales are applied at the end.
+//   Bound by issue slots (58 % used) and then by the stream: 256 experts x 15.6 rows, block-scaled, a layer's gate and up products (537 MB)
+// 198 us, down (268 MB) 120 us, against 348 and 174 through the operand (83 and 42 at the measured copy bandwidth).
+// NT8: groups of eight tokens of the widest item.
+constexpr int EX_STAGES = 6;
+struct ExpertBars {
+    uint64_t full[EX_STAGES], empty[EX_STAGES];
+    volatile int dead;
+};
+// Four fp8 bytes as two pairs of bf16: bytes 0 and 2, bytes 1 and 3.
+__device__ __forceinline__ void e4m3x4_bf16(uint32_t w, uint32_t& even, uint32_t& odd) {
+    constexpr uint32_t UP = 0x7B807B80u;           // 2^120: the bits moved into the bf16 fields are the values times 2^-120, subnormals included
+    even = mul_bf16x2(((w << 4) & 0x07F007F0u) | ((w << 8) & 0x80008000u), UP);
+    odd = mul_bf16x2(((w >> 4) & 0x07F007F0u) | (w & 0x80008000u), UP);
+}
+// Offset of column c of a row whose sixteens are stored even columns first.
+__device__ __forceinline__ size_t slab_offset_eo(int rows, int row, int c) { return slab_offset(rows, row, (c & ~15) | ((c & 1) << 3) | ((c & 15) >> 1)); }
+
+template <bool BLOCKS, int OUT, int NT8>
+static __global__ void __launch_bounds__(256, 2) experts_gemm(const __grid_constant__ GemmArgs A) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    constexpr int X_KB = NT8 * 8 * 128;
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    ExpertBars& B = *reinterpret_cast<ExpertBars*>(smem + EX_STAGES * 2 * X_KB);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, units = __ldg(A.n_items) * A.blocks;
+    auto item = [&](int u) { return __ldg(A.items + min(u, units - 1) / A.blocks); };
+    if ((int)blockIdx.x >= units) return;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < EX_STAGES; i++) {
+            mbar_init(&B.full[i], 1);
+            mbar_init(&B.empty[i], 8);
+        }
+        B.dead = 0;
+        mk::fence_barrier_init();
+    }
+    __syncthreads();
+    const int g = lane >> 2, t = lane & 3;
+    // Requests run ahead of the products, across units, two blocks of 64 columns at a time; warp 0 asks for the token rows too.
+    // (Block-scaled: the two are four steps of one chunk with a scale each for the tile's upper and lower eight rows.)
+    Walk<W_FP8> walk;
+    Raw<W_FP8> raw[4];
+    float2 scale[2];
+    int ask_u = blockIdx.x, ask_kb = 0;
+    uint32_t ask_slot = 0, ask_phase = 0;
+    int4 ask_it = item(blockIdx.x);
+    auto ask_start = [&]() { walk.start(A, A.w + (size_t)ask_it.x * A.w_gstride, min(ask_u % A.blocks * 8 + warp, A.tiles - 1), 0, lane); };
+    auto request2 = [&](Raw<W_FP8>& a, Raw<W_FP8>& b, float2& sc) {
+        if (ask_u < units) {
+            if (ask_kb < A.kbs) {
+                const bool two = BLOCKS || ask_kb + 1 < A.kbs;
+                if (BLOCKS) {
+                    const uint4* q = reinterpret_cast<const uint4*>(walk.p);
+                    a.q[0] = __ldg(q); a.q[1] = __ldg(q + 32); b.q[0] = __ldg(q + 64); b.q[1] = __ldg(q + 96);
+                    sc = __ldg(reinterpret_cast<const float2*>(walk.s));
+                    walk.p += 2048;
+                    walk.s += 8;
+                    if ((walk.left -= 4) == 0) {
+                        walk.left = A.chunk_steps;
+                        walk.p += A.chunk_bytes - A.chunk_steps * 512;
+                        walk.s += A.chunk_bytes - A.chunk_steps * 2;
+                    }
+                } else {
+                    walk.load(A, a);
+                    if (two) walk.load(A, b);
+                }
+                if (warp == 0 && lane == 0 && wait(B, A, &B.empty[ask_slot], ask_phase ^ 1u, WP_EMPTY)) {
+                    const uint32_t bytes = (uint32_t)((ask_it.z + 7) & ~7) * 128u;
+                    mbar_expect_tx(&B.full[ask_slot], two ? 2 * bytes : bytes);
+                    for (int i = 0; i < (two ? 2 : 1); i++)
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                     ::"r"(smem_u32(smem + (size_t)(2 * ask_slot + i) * X_KB)), "l"(A.x + ((size_t)(ask_kb + i) * A.x_rows + ask_it.y) * 128), "r"(bytes),
+                                       "r"(smem_u32(&B.full[ask_slot])) : "memory");
+                }
+                if (++ask_slot == EX_STAGES) {
+                    ask_slot = 0;
+                    ask_phase ^= 1u;
+                }
+            }
+            ask_kb += 2;
+            if (ask_kb >= A.kbs && !(ask_kb & 2)) {                // (a unit is a whole number of turns of the two buffers)
+                ask_kb = 0;
+                ask_u += gridDim.x;
+                ask_it = item(ask_u);
+                if (ask_u < units) ask_start();
+            }
+        }
+    };
+    ask_start();
+    request2(raw[0], raw[1], scale[0]);
+    request2(raw[2], raw[3], scale[1]);
+    uint32_t slot = 0, phase = 0;
+    const uint32_t frag = smem_u32(smem) + (uint32_t)(lane & 7) * 128, piece = lane >> 3, sw = lane & 7;
+    int4 it = item(blockIdx.x);
+#pragma unroll 1
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        const int4 next = item(u + gridDim.x);
+        const int n8 = (it.z + 7) >> 3, tile = u % A.blocks * 8 + warp;
+        float acc[NT8][4], sums[BLOCKS ? NT8 : 1][4];
+#pragma unroll
+        for (int n = 0; n < NT8; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[n][i] = sums[BLOCKS ? n : 0][i] = 0.f;
+        bool ok = true;
+        auto product = [&](const Raw<W_FP8>& r, uint32_t x, bool fresh) {           // fresh: the accumulators start over
+            uint32_t a[4][4];                        // [16 columns][row g even, row g + 8 even, row g odd, row g + 8 odd]
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                e4m3x4_bf16(r.q[i].x, a[2 * i][0], a[2 * i][2]);
+                e4m3x4_bf16(r.q[i].y, a[2 * i + 1][0], a[2 * i + 1][2]);
+                e4m3x4_bf16(r.q[i].z, a[2 * i][1], a[2 * i][3]);
+                e4m3x4_bf16(r.q[i].w, a[2 * i + 1][1], a[2 * i + 1][3]);
+            }
+#pragma unroll
+            for (int n = 0; n < NT8; n++) {
+                if (n >= n8) break;
+                uint32_t b[2][4];
+#pragma unroll
+                for (int h = 0; h < 2; h++) ldsm4(b[h], x + n * 1024 + (((4 * h + piece) ^ sw) << 4));
+                if (fresh) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma16816(acc[n], a[j], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+            }
+        };
+        auto pair = [&](int kb, Raw<W_FP8>& ra, Raw<W_FP8>& rb, float2& sc) {
+            if (kb < A.kbs) {
+                ok = ok && __all_sync(0xffffffffu, wait(B, A, &B.full[slot], phase, WP_FULL));     // the warp leaves together
+                if (!ok) return;
+                const uint32_t x = frag + 2 * slot * X_KB;
+                product(ra, x, BLOCKS);
+                if (BLOCKS || kb + 1 < A.kbs) product(rb, x + X_KB, false);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&B.empty[slot]);
+                if (++slot == EX_STAGES) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+                if constexpr (BLOCKS) {
+#pragma unroll
+                    for (int n = 0; n < NT8; n++) {
+                        if (n >= n8) break;
+                        sums[n][0] = fmaf(acc[n][0], sc.x, sums[n][0]);
+                        sums[n][1] = fmaf(acc[n][1], sc.x, sums[n][1]);
+                        sums[n][2] = fmaf(acc[n][2], sc.y, sums[n][2]);
+                        sums[n][3] = fmaf(acc[n][3], sc.y, sums[n][3]);
+                    }
+                }
+            }
+            request2(ra, rb, sc);
+        };
+#pragma unroll 1
+        for (int kb = 0; kb < A.kbs && ok; kb += 4) {
+            pair(kb, raw[0], raw[1], scale[0]);
+            pair(kb + 2, raw[2], raw[3], scale[1]);
+        }
+        if (!ok) {
+            if (warp == 0) {                     // copies in flight must land before the CTA leaves (see rows_gemm)
+                const u64 t0 = mk::globaltimer();
+                while (mk::globaltimer() - t0 < 1000000ull) {}
+            }
+            break;
+        }
+        // lane (g, t): rows g and g + 8 of the tile, tokens 2 t and 2 t + 1 of every eight
+        const int r0 = tile * 16 + g;
+        float rs0 = 1.f, rs1 = 1.f;
+        if (A.row_scale && tile < A.tiles) {
+            const float* rs = A.row_scale + (size_t)it.x * A.rs_gstride;
+            if (r0 < A.n_valid) rs0 = __ldg(rs + r0);
+            if (r0 + 8 < A.n_valid) rs1 = __ldg(rs + r0 + 8);
+        }
+        if (tile < A.tiles) {
+#pragma unroll
+            for (int n = 0; n < NT8; n++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int tok = 8 * n + 2 * t + i;
+                    if (tok >= it.z) continue;
+                    const float lo = (BLOCKS ? sums[n][i] : acc[n][i]) * rs0, hi = (BLOCKS ? sums[n][2 + i] : acc[n][2 + i]) * rs1;
+                    if (OUT == OUT_GLU) {            // rows 0-7 of a tile are gates, rows 8-15 their up rows
+                        const int col = tile * 8 + g;
+                        const float y = (A.gelu ? 0.5f * lo * (1.f + tanhf(0.7978845608028654f * (lo + 0.044715f * lo * lo * lo))) : silu_f(lo)) * hi;
+                        if (col < A.act_cols) *reinterpret_cast<__nv_bfloat16*>(A.act + slab_offset_eo(A.act_rows, it.y + tok, col)) = __float2bfloat16_rn(y);
+                    } else {
+                        float* o = A.out + (size_t)(it.y + tok) * A.out_stride + r0;
+                        if (r0 < A.n_valid) o[0] = lo;
+                        if (r0 + 8 < A.n_valid) o[8] = hi;
+                    }
+                }
+        }
+        it = next;
+    }
+}
+
 // ---- expert routing --------------------------------------------------------------------------------------------
 struct RouteArgs {
     const float* logits;
@@ -1691,15 +1894,25 @@ static __global__ void __launch_bounds__(256) route_slots(const __grid_constant_
     R.slot[i] = R.counts[2 * R.experts + e] + atomicAdd(R.counts + R.experts + e, 1);
 }
 
-// Copies every token's slab row to the rows of its experts.
+// Copies every token's slab row to the rows of its experts.  EO: of every sixteen columns the even ones first, as experts_gemm
+// reads them.
+template <bool EO>
 static __global__ void __launch_bounds__(256) gather_rows(const uint8_t* x, int x_rows, const int* slot, int topk, int kbs, uint8_t* out, int out_rows) {
     const int row = blockIdx.x;
-    for (int i = threadIdx.x; i < kbs * 8; i += 256) {
-        const int kb = i >> 3, c = i & 7;
-        const uint4 v = *reinterpret_cast<const uint4*>(x + ((size_t)kb * x_rows + row) * 128 + ((c ^ (row & 7)) << 4));
+    for (int i = threadIdx.x; i < kbs * 4; i += 256) {
+        const int kb = i >> 2, c = 2 * (i & 3);
+        const uint8_t* src = x + ((size_t)kb * x_rows + row) * 128;
+        uint4 a = *reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4)), b = *reinterpret_cast<const uint4*>(src + (((c + 1) ^ (row & 7)) << 4));
+        if (EO) {
+            const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            a = make_uint4(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410), __byte_perm(w[4], w[5], 0x5410), __byte_perm(w[6], w[7], 0x5410));
+            b = make_uint4(__byte_perm(w[0], w[1], 0x7632), __byte_perm(w[2], w[3], 0x7632), __byte_perm(w[4], w[5], 0x7632), __byte_perm(w[6], w[7], 0x7632));
+        }
         for (int k = 0; k < topk; k++) {
             const int s = slot[(size_t)row * 8 + k];
-            *reinterpret_cast<uint4*>(out + ((size_t)kb * out_rows + s) * 128 + ((c ^ (s & 7)) << 4)) = v;
+            uint8_t* dst = out + ((size_t)kb * out_rows + s) * 128;
+            *reinterpret_cast<uint4*>(dst + ((c ^ (s & 7)) << 4)) = a;
+            *reinterpret_cast<uint4*>(dst + (((c + 1) ^ (s & 7)) << 4)) = b;
         }
     }
 }

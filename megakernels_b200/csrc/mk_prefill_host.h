@@ -94,6 +94,18 @@ int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaSt
     return MK_OK;
 }
 
+// FP8 products of routed groups with at most 8 NT8 rows per work item; `items` bounds the number of items.
+template <bool BLOCKS, int NT8>
+int launch_experts(GemmArgs& A, int out, int items, int sms, cudaStream_t st) {
+    const int smem = EX_STAGES * 2 * NT8 * 8 * 128 + (int)sizeof(ExpertBars) + 1024;
+    const long long units = (long long)items * A.blocks;
+    auto fn = out == OUT_GLU ? experts_gemm<BLOCKS, OUT_GLU, NT8> : experts_gemm<BLOCKS, OUT_STORE, NT8>;
+    MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    fn<<<(int)(units < 2 * sms ? units : 2 * sms), 256, smem, st>>>(A);
+    MKP_CUDA(cudaGetLastError());
+    return MK_OK;
+}
+
 // The DeltaNet mixer of M sequences of L rows; `gate` is gdn_gate of the wanted number of pieces.
 inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), int sms, cudaStream_t st) {
     const int rows = G.M * G.L, chunks = (G.L + SCAN - 1) / SCAN;

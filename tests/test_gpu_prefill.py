@@ -299,3 +299,23 @@ def test_small_model_prompts_are_as_exact_as_stepping(small, monkeypatch, quant,
         states = [rel(mk.deltanet_state(i).cpu(), s) for i, s in enumerate(d.state[i] for i in sorted(d.state))]
         off.append(sum(states) / len(states))
     assert off[0] < 1.5 * off[1] and off[0] < 5e-6, off
+
+
+@pytest.mark.parametrize("model,M,length", [("26b", 5, 30), ("26b", 8, 50), ("26b", 8, 101), ("26b", 8, 200), ("35b", 8, 49), ("35b", 8, 101), ("35b", 8, 200)])
+def test_prompt_rows_of_crowded_experts(model, M, length):
+    """Routed products by the width of a work item (the mean load of 128 experts: 32, 64, 128 and 256 tokens; block-scaled ones at
+    most 128, several items an expert); 26b: 11 blocks of 64 columns in the down-projection, the last weight block past the matrix."""
+    pkg, shape = SHAPES[model]
+    shape = shape.with_(eff=704, hidden=576) if model == "26b" else shape.with_(experts=128)
+    PK = pkg.Packed(pkg.SynthWeights(shape, layers=shape.layers, init="realistic", device="cuda"), "cuda")
+    prompts = [pkg.make_prompt(shape.vocab, length, seed=j) for j in range(M)]
+    out = []
+    for rows in (True, False):
+        eng = pkg.Engine(PK, M, maxlen=length + 64)
+        with pytest.MonkeyPatch.context() as mp:
+            if not rows:
+                mp.setattr(runtime, "MIN_ROWS_PATH", 1 << 30)
+            out.append(eng.prefill(prompts).clone())
+        assert (eng.rt._workspace is not None) == rows
+        eng.check()
+    assert rel(*out) < 3e-2
