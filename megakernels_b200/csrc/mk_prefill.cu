@@ -323,7 +323,7 @@ struct Exec {
             qkv = arena.take<float>((size_t)rows * conv);
             scal = arena.take<float4>((size_t)rows * heads);
             o = arena.take<float>((size_t)rows * vals);
-            gram = arena.take<float>((size_t)M * ((L + SCAN - 1) / SCAN) * heads * 80);
+            gram = arena.take<float>((size_t)M * ((L + SCAN - 1) / SCAN) * heads * GRAM);
         }
         if (q_w) q = arena.take<__nv_bfloat16>((size_t)rows * q_w);
         if (experts) {
@@ -517,7 +517,7 @@ struct Exec {
         G.out = s->x;
         G.out_rows = s->rows;
         G.gram = gram;
-        return launch_gdn(G, gdn_gate<1>, sms, st);
+        return launch_gdn(G, gdn_gate<1>, st);
     }
 
     template <int HD>

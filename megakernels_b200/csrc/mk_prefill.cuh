@@ -802,7 +802,7 @@ struct GdnArgs {
     // scratch
     float* qkv;                  // [rows][conv_dim]: normalised q, k, and v
     float4* scal;                // [rows][nvh]: decay, beta
-    float* gram;                 // [M][blocks of 8 positions][nvh][80]: see gdn_gram
+    float* gram;                 // [M][blocks of 8 positions][nvh][GRAM]: see gdn_gram
     float* o;                    // [rows][nvh * 128]
     uint8_t* out;                // slabs of the gated output
     size_t out_piece;
@@ -908,7 +908,8 @@ static __global__ void __launch_bounds__(256) gdn_history(const __grid_constant_
 // scalar steps.
 constexpr int SCAN = 8;
 // Per block and value head: k_i k_t (i < t) and q_i k_t (i >= t) with the decays between the two positions, [t][i], then
-// P_t and P_8 / P_t.  One warp per block and key head.
+// P_t, P_8 / P_t and beta_t (a position past the end decays by 1 and corrects by 0).  One warp per block and key head.
+constexpr int GRAM = SCAN * SCAN + 3 * SCAN;
 static __global__ void __launch_bounds__(128) gdn_gram(const __grid_constant__ GdnArgs G) {
     const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, chunks = (G.L + SCAN - 1) / SCAN;
     if (w >= G.M * chunks * G.nkh) return;
@@ -942,10 +943,11 @@ static __global__ void __launch_bounds__(128) gdn_gram(const __grid_constant__ G
                 v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
     }
-    // per value head: entry (t, i) takes the decays between the two positions; a position past the end decays by 1
+    // per value head: entry (t, i) takes the decays between the two positions
     for (int r = 0; r < rep; r++) {
         const int h = kh * rep + r, l = c * SCAN + (lane & 7);
-        const float dec = l < G.L ? G.scal[((size_t)m * G.L + l) * G.nvh + h].x : 1.f;
+        const float4 sc = l < G.L ? G.scal[((size_t)m * G.L + l) * G.nvh + h] : make_float4(1.f, 0.f, 0.f, 0.f);
+        const float dec = sc.x;
         float d0 = 1.f, d1 = 1.f, p = 1.f;
         const int t = lane >> 2, i = (lane & 3) * 2;
 #pragma unroll
@@ -955,9 +957,9 @@ static __global__ void __launch_bounds__(128) gdn_gram(const __grid_constant__ G
             d1 *= j > min(t, i + 1) && j <= max(t, i + 1) ? dj : 1.f;
             p *= (lane < 8 ? j <= lane : j > (lane & 7)) ? dj : 1.f;
         }
-        float* out = G.gram + (((size_t)m * chunks + c) * G.nvh + h) * 80;
+        float* out = G.gram + (((size_t)m * chunks + c) * G.nvh + h) * GRAM;
         *reinterpret_cast<float2*>(out + 2 * lane) = make_float2(v[0] * d0, v[1] * d1);
-        if (lane < 16) out[64 + lane] = p;
+        if (lane < 24) out[64 + lane] = lane < 16 ? p : sc.y;
     }
 }
 __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
@@ -973,35 +975,32 @@ __device__ __forceinline__ u64 mul2(u64 a, u64 b) {
 __device__ __forceinline__ u64 both(float a) { return ((u64)__float_as_uint(a) << 32) | __float_as_uint(a); }
 __device__ __forceinline__ float sum2(u64 a) { return __uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32)); }
 
-// Four warps; eight lanes share R value rows of one head of one sequence (16 keys each, in registers, packed in pairs), so
-// a CTA holds 16 R rows and a head is 8 / R CTAs: R = 1 spreads a few heads over the chip, R = 2 reads shared memory once
-// for two rows when there are enough heads.  16 heads x 511 positions: 70 us (207 position by position; 145 with the decay
-// products formed here instead of in gdn_gram, where their branches serialised 64 threads per block).
-template <int R>
+// Four warps; sixteen lanes share two value rows of one head of one sequence (eight keys each, in registers, packed in pairs), so
+// a CTA holds 16 rows and a head is eight CTAs.  What bounds a block is shared memory: a 16-byte read is four of its cycles, and
+// every lane reads its keys of eight k and eight q.  Two rows a lane halve the reads per product, and the k's stay in registers
+// for the update.  16 heads x 511 positions: 54 us (69 with eight lanes to one row; 207 position by position).
 static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ GdnArgs G) {
-    constexpr int ROWS = 16 * R, IN = 256 + ROWS;
+    constexpr int ROWS = 16, IN = 256 + ROWS;
     __shared__ __align__(16) float in_s[2][SCAN][IN];        // q | k | values
-    __shared__ __align__(16) float4 sc_s[2][SCAN];           // decay, beta
-    __shared__ __align__(16) float mats[2][80];           // what gdn_gram left for the block
+    __shared__ __align__(16) float mats[2][GRAM];            // what gdn_gram left for the block
     const int rep = G.nvh / G.nkh;
     const int m = blockIdx.z, h = blockIdx.y, v0 = blockIdx.x * ROWS, kh = h / rep;
-    const int tid = threadIdx.x, part = tid & 7, rr = (tid >> 3) * R;
+    const int tid = threadIdx.x, part = tid & 15, r0 = (tid >> 4) * 2;       // the lanes' rows r0, r0 + 1; keys part * 4 + 64 i + {0..3}
     const int chunks = (G.L + SCAN - 1) / SCAN, key_dim = G.nkh * 128;
-    float* st = G.ssm + (((size_t)m * G.nvh + h) * 128 + v0 + rr) * 128 + part * 4;     // keys part * 4 + 32 i + {0..3}
-    u64 s[R][8];
+    float* st = G.ssm + (((size_t)m * G.nvh + h) * 128 + v0 + r0) * 128 + part * 4;
+    u64 s[2][4];
 #pragma unroll
-    for (int r = 0; r < R; r++)
+    for (int r = 0; r < 2; r++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(st + r * 128 + 32 * i);
+        for (int i = 0; i < 2; i++) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(st + r * 128 + 64 * i);
             s[r][2 * i] = a.x;
             s[r][2 * i + 1] = a.y;
         }
     const size_t row0 = (size_t)m * G.L;
     const float* qk_src = G.qkv + row0 * G.conv_dim + ((tid & 32) ? key_dim : 0) + kh * 128 + 4 * (tid & 31);
-    const float* v_src = G.qkv + row0 * G.conv_dim + 2 * key_dim + h * 128 + v0 + 4 * (tid % (ROWS / 4));
-    const float* m_src = G.gram + ((size_t)m * chunks * G.nvh + h) * 80 + 4 * (tid - 64);
-    const float4* s_src = G.scal + row0 * G.nvh + h;
+    const float* v_src = G.qkv + row0 * G.conv_dim + 2 * key_dim + h * 128 + v0 + 4 * (tid & 3);
+    const float* m_src = G.gram + ((size_t)m * chunks * G.nvh + h) * GRAM + 4 * (tid - 64);
     auto request = [&](int buf, int c) {
         const int l0 = c * SCAN;
 #pragma unroll
@@ -1009,119 +1008,83 @@ static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ G
             const int b = (tid >> 6) + 2 * j;
             mk::cp_async16(&in_s[buf][b][4 * (tid & 63)], qk_src + (size_t)min(l0 + b, G.L - 1) * G.conv_dim);
         }
-        if (tid < 2 * ROWS) {
-            const int b = tid / (ROWS / 4);
-            mk::cp_async16(&in_s[buf][b][256 + 4 * (tid % (ROWS / 4))], v_src + (size_t)min(l0 + b, G.L - 1) * G.conv_dim);
-        }
-        if (tid >= 64 && tid < 84) mk::cp_async16(&mats[buf][4 * (tid - 64)], m_src + (size_t)c * G.nvh * 80);
-        if (tid >= 96 && tid < 96 + SCAN) mk::cp_async16(&sc_s[buf][tid - 96], s_src + (size_t)min(l0 + tid - 96, G.L - 1) * G.nvh);
+        if (tid < 4 * SCAN) mk::cp_async16(&in_s[buf][tid >> 2][256 + 4 * (tid & 3)], v_src + (size_t)min(l0 + (tid >> 2), G.L - 1) * G.conv_dim);
+        if (tid >= 64 && tid < 64 + GRAM / 4) mk::cp_async16(&mats[buf][4 * (tid - 64)], m_src + (size_t)c * G.nvh * GRAM);
         mk::cp_async_commit();
     };
     request(0, 0);
-    float* o = G.o + row0 * (size_t)(G.nvh * 128) + h * 128 + v0 + rr;
+    const int mine = (part >> 3) & 1, mt = part & 7;                        // the row and the position whose products this lane ends up with
+    float* o = G.o + row0 * (size_t)(G.nvh * 128) + h * 128 + v0 + r0 + mine;
 #pragma unroll 1
     for (int c = 0, buf = 0; c < chunks; c++, buf ^= 1) {
         mk::cp_async_wait_all();
         __syncthreads();
         if (c + 1 < chunks) request(buf ^ 1, c + 1);
-        const int nb = min(SCAN, G.L - c * SCAN);
-        // a position past the end decays by 1 and corrects by 0
-        const float *mat_s = mats[buf], *p_s = mats[buf] + 64, *e_s = mats[buf] + 72;
-        // s k_t, s q_t over this lane's keys
-        float u[R][16];
+        const float* mat_s = mats[buf];
+        // s k_t, s q_t of both rows over this lane's keys: value r * 16 + 2 t (k) and + 1 (q)
+        u64 k[SCAN][4];
+        float u[32];
 #pragma unroll
         for (int t = 0; t < SCAN; t++) {
             const float* q = in_s[buf][t] + part * 4;
-            u64 a[R], b[R];
+            const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(q + 128), k1 = *reinterpret_cast<const ulonglong2*>(q + 192);
+            const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(q), q1 = *reinterpret_cast<const ulonglong2*>(q + 64);
+            k[t][0] = k0.x; k[t][1] = k0.y; k[t][2] = k1.x; k[t][3] = k1.y;
 #pragma unroll
-            for (int r = 0; r < R; r++) a[r] = b[r] = 0ull;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(q + 128 + 32 * i), qv = *reinterpret_cast<const ulonglong2*>(q + 32 * i);
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    a[r] = fma2(s[r][2 * i], kv.x, a[r]);
-                    b[r] = fma2(s[r][2 * i], qv.x, b[r]);
-                    a[r] = fma2(s[r][2 * i + 1], kv.y, a[r]);
-                    b[r] = fma2(s[r][2 * i + 1], qv.y, b[r]);
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                u[r][2 * t] = sum2(a[r]);
-                u[r][2 * t + 1] = sum2(b[r]);
+            for (int r = 0; r < 2; r++) {
+                u[16 * r + 2 * t] = sum2(fma2(s[r][3], k1.y, fma2(s[r][2], k1.x, fma2(s[r][1], k0.y, mul2(s[r][0], k0.x)))));
+                u[16 * r + 2 * t + 1] = sum2(fma2(s[r][3], q1.y, fma2(s[r][2], q1.x, fma2(s[r][1], q0.y, mul2(s[r][0], q0.x)))));
             }
         }
-        // lane t of the eight ends up with s k_t and s q_t
+        // sums over the sixteen lanes; every step halves what a lane carries
 #pragma unroll
-        for (int x = 4, n = 8; x; x >>= 1, n >>= 1) {
+        for (int x = 8, n = 16; x; x >>= 1, n >>= 1) {
             const bool up = part & x;
 #pragma unroll
-            for (int r = 0; r < R; r++)
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    if (j < n) {
-                        const float send = up ? u[r][j] : u[r][j + n], keep = up ? u[r][j + n] : u[r][j];
-                        u[r][j] = keep + __shfl_xor_sync(0xffffffffu, send, x);
-                    }
+            for (int j = 0; j < 16; j++)
+                if (j < n) {
+                    const float send = up ? u[j] : u[j + n], keep = up ? u[j + n] : u[j];
+                    u[j] = keep + __shfl_xor_sync(0xffffffffu, send, x);
+                }
         }
-        float delta[R][SCAN];
+        // the eight corrections of this lane's row, one after the other
+        float delta[SCAN];
 #pragma unroll
         for (int t = 0; t < SCAN; t++) {
-            float mrow[SCAN];
-#pragma unroll
-            for (int i = 0; i < SCAN; i += 4) {
-                if (i >= t) continue;
-                const float4 a = *reinterpret_cast<const float4*>(mat_s + t * 8 + i);
-                mrow[i] = a.x; mrow[i + 1] = a.y; mrow[i + 2] = a.z; mrow[i + 3] = a.w;
-            }
-            const float beta = t < nb ? sc_s[buf][t].y : 0.f, p = p_s[t];
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                float recall = __shfl_sync(0xffffffffu, u[r][0], (tid & 24) | t) * p;
-#pragma unroll
-                for (int i = 0; i < SCAN; i++)
-                    if (i < t) recall = fmaf(mrow[i], delta[r][i], recall);
-                delta[r][t] = (in_s[buf][t][256 + rr + r] - recall) * beta;
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            float y = u[r][1] * p_s[part];
+            float recall = __shfl_sync(0xffffffffu, u[0], (tid & 24) | t) * mat_s[64 + t];
 #pragma unroll
             for (int i = 0; i < SCAN; i++)
-                if (i <= part) y = fmaf(mat_s[i * 8 + part], delta[r][i], y);
-            if (part < nb) o[(size_t)(c * SCAN + part) * (G.nvh * 128) + r] = y;
+                if (i < t) recall = fmaf(mat_s[t * 8 + i], delta[i], recall);
+            delta[t] = (in_s[buf][t][256 + r0 + mine] - recall) * mat_s[80 + t];
         }
         {
-            const u64 p = both(p_s[SCAN - 1]);
+            float y = u[1] * mat_s[64 + mt];
 #pragma unroll
-            for (int r = 0; r < R; r++)
-#pragma unroll
-                for (int i = 0; i < 8; i++) s[r][i] = mul2(s[r][i], p);
+            for (int i = 0; i < SCAN; i++)
+                if (i <= mt) y = fmaf(mat_s[i * 8 + mt], delta[i], y);
+            if (c * SCAN + mt < G.L) o[(size_t)(c * SCAN + mt) * (G.nvh * 128)] = y;
         }
+        const u64 p = both(mat_s[64 + SCAN - 1]);
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) s[r][i] = mul2(s[r][i], p);
 #pragma unroll
         for (int t = 0; t < SCAN; t++) {
-            const float* k = in_s[buf][t] + 128 + part * 4;
-            u64 f[R];
+            const float e = delta[t] * mat_s[72 + t], other = __shfl_xor_sync(0xffffffffu, e, 8);
 #pragma unroll
-            for (int r = 0; r < R; r++) f[r] = both(delta[r][t] * e_s[t]);
+            for (int r = 0; r < 2; r++) {
+                const u64 f = both(mine == r ? e : other);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k + 32 * i);
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    s[r][2 * i] = fma2(kv.x, f[r], s[r][2 * i]);
-                    s[r][2 * i + 1] = fma2(kv.y, f[r], s[r][2 * i + 1]);
-                }
+                for (int i = 0; i < 4; i++) s[r][i] = fma2(k[t][i], f, s[r][i]);
             }
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int r = 0; r < R; r++)
+    for (int r = 0; r < 2; r++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) *reinterpret_cast<ulonglong2*>(st + r * 128 + 32 * i) = make_ulonglong2(s[r][2 * i], s[r][2 * i + 1]);
+        for (int i = 0; i < 2; i++) *reinterpret_cast<ulonglong2*>(st + r * 128 + 64 * i) = make_ulonglong2(s[r][2 * i], s[r][2 * i + 1]);
 }
 
 // Gated RMSNorm per head, into slabs: one half warp per head and row (eight columns per lane).

@@ -152,7 +152,7 @@ struct Run {
         scal = arena.take<float4>((size_t)rows * S::LIN_H);
         o = arena.take<float>((size_t)rows * S::LIN_V);
         q = arena.take<float>((size_t)rows * S::MIX);
-        gram = arena.take<float>((size_t)((rows + SCAN - 1) / SCAN) * S::LIN_H * 80);
+        gram = arena.take<float>((size_t)((rows + SCAN - 1) / SCAN) * S::LIN_H * GRAM);
         part = arena.take<float>((size_t)8 * rows * S::HID);
         pos = arena.take<int>(1);
     }
@@ -237,7 +237,7 @@ struct Run {
                 G.ssm = L.state + (size_t)seq * S::LIN_H * S::LIN_DV * S::LIN_DK;
                 G.pos = pos; G.l2_clamp = 1; G.eps = 1e-6f; G.norm_eps = S::EPS;
                 G.qkv = qkv; G.scal = scal; G.gram = gram; G.o = o; G.out = mix; G.out_piece = mix_piece; G.out_rows = xrows;
-                if ((rc = launch_gdn(G, gdn_gate<PX>, sms, st)) != MK_OK) return rc;
+                if ((rc = launch_gdn(G, gdn_gate<PX>, st)) != MK_OK) return rc;
             }
             MKP_CUDA(cudaGetLastError());
             if ((rc = product(W.out, S::HID, S::MIX, mix, mix_piece, L.s_out, OUT_ADD, h, S::HID)) != MK_OK) return rc;

@@ -107,14 +107,12 @@ int launch_experts(GemmArgs& A, int out, int items, int sms, cudaStream_t st) {
 }
 
 // The DeltaNet mixer of M sequences of L rows; `gate` is gdn_gate of the wanted number of pieces.
-inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), int sms, cudaStream_t st) {
+inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), cudaStream_t st) {
     const int rows = G.M * G.L, chunks = (G.L + SCAN - 1) / SCAN;
     gdn_conv<<<dim3((G.conv_dim / 128 + 7) / 8, G.M * ((G.L + CONV_ROWS - 1) / CONV_ROWS)), 256, 0, st>>>(G);
     gdn_history<<<dim3((G.conv_dim + 255) / 256, G.M, G.ring), 256, 0, st>>>(G);
     gdn_gram<<<(G.M * chunks * G.nkh + 3) / 4, 128, 0, st>>>(G);
-    // one row per lane while that is about one CTA per SM (latency decides); with more, shared-memory reads do: two rows
-    if (2 * G.M * G.nvh * 8 > 3 * sms) gdn_scan<2><<<dim3(4, G.nvh, G.M), 128, 0, st>>>(G);
-    else gdn_scan<1><<<dim3(8, G.nvh, G.M), 128, 0, st>>>(G);
+    gdn_scan<<<dim3(8, G.nvh, G.M), 128, 0, st>>>(G);
     gate<<<dim3((G.nvh + 15) / 16, rows), 256, 0, st>>>(G);
     MKP_CUDA(cudaGetLastError());
     return MK_OK;
