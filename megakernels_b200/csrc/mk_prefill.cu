@@ -199,6 +199,7 @@ struct Exec {
     std::vector<Slab> slabs;
     uint8_t* x_scratch = nullptr;        // slabs made from fp32 rows; reused by every stage that needs new ones
     Have x_have = {};
+    struct { uint64_t key; int ksplit; } left = {};       // a residual whose last addend waits as partial products in `part`
     float* part = nullptr;
     size_t part_floats = 0;
     // DeltaNet / attention / routing scratch
@@ -401,10 +402,10 @@ struct Exec {
         const Have want = {d.p[MKS_P_X], nw, in_scale, d.f[MKS_F_EPS], d.f[MKS_F_NORM_OFF], d.i[MKS_I_KC] * d.i[MKS_I_SPLITS]};
         const bool same = x_have.key == want.key && x_have.norm == nw && x_have.K == want.K && (!norm || (x_have.in_scale == in_scale && x_have.eps == want.eps && x_have.off == want.off));
         if (!same) {
-            const float* src = at(d.p[MKS_P_X]);
-            rows_in<1><<<rows, 256, 0, st>>>(src, d.i[MKS_I_X_STRIDE], d.i[MKS_I_KC] * d.i[MKS_I_SPLITS], reinterpret_cast<const float*>(nw), d.f[MKS_F_NORM_OFF],
-                                             d.f[MKS_F_EPS], in_scale, x_scratch, 0, xrows);
-            MKP_CUDA(cudaGetLastError());
+            const int splits = left.key == want.key ? left.ksplit : 0;
+            const RowsIn R = {at(d.p[MKS_P_X]), d.i[MKS_I_X_STRIDE], want.K, splits, rows, part, reinterpret_cast<const float*>(nw), d.f[MKS_F_NORM_OFF], d.f[MKS_F_EPS], in_scale, x_scratch, 0, xrows};
+            MKP_CUDA(launch(splits ? rows_in<1, true> : rows_in<1, false>, dim3(rows), 256, 0, st, R));
+            left = {};
             x_have = want;
         }
         *x = x_scratch;
@@ -432,6 +433,12 @@ struct Exec {
             A.out = at(d.p[MKS_P_OUT]);
             A.out_stride = d.i[MKS_I_OUT_STRIDE];
             written(d.p[MKS_P_OUT]);
+            // the next record norms this residual: it adds the K splits' partials on the way
+            const mk_stage_desc* n = &d + 1;
+            A.leave = out == OUT_ADD && A.ksplit > 1 && n < prog + n_stages && n->op == MKS_OP_GEMV && n->i[MKS_I_EPILOGUE] != MKS_E_LOGITS && n->i[MKS_I_PROLOGUE] == MKS_P_NORM &&
+                      n->p[MKS_P_X] == d.p[MKS_P_OUT] && n->i[MKS_I_KC] * n->i[MKS_I_SPLITS] == A.n_valid && n->i[MKS_I_X_STRIDE] == A.out_stride &&
+                      (n->i[MKS_I_GROUPS] == 1 || n->i[MKS_I_EPILOGUE] == MKS_E_GLU);
+            if (A.leave) left = {d.p[MKS_P_OUT], A.ksplit};
         }
         return gemm(d, A, out, 0);
     }
@@ -453,7 +460,7 @@ struct Exec {
                 if (rc != MK_OK) return rc;
             }
             auto gather = few ? gather_rows<true> : gather_rows<false>;
-            gather<<<rows, 256, 0, st>>>(A.x, A.x_rows, route.slot, route.topk, A.kbs, xg, slot_rows);
+            MKP_CUDA(launch(gather, dim3(rows), 256, 0, st, A.x, A.x_rows, route.slot, route.topk, A.kbs, xg, slot_rows));
             MKP_CUDA(cudaGetLastError());
             A.x = xg;
             A.act = act_g;
@@ -485,8 +492,8 @@ struct Exec {
         if (!few) rc = gemm(d, A, out, max_items);
         else rc = d.i[MKS_I_BLOCK_SCALES] ? launch_experts<true, 4>(A, out, max_items, sms, st) : launch_experts<false, 4>(A, out, max_items, sms, st);
         if (rc != MK_OK || up) return rc;
-        combine_rows<<<rows, 256, 0, st>>>(yg, d.i[MKS_I_N_VALID], route.slot, route.weight, route.topk, shared ? ys : nullptr, route.gate,
-                                           d.i[MKS_I_EPILOGUE] == MKS_E_RESID, at(d.p[MKS_P_OUT]), d.i[MKS_I_OUT_STRIDE]);
+        MKP_CUDA(launch(combine_rows, dim3(rows), 256, 0, st, yg, d.i[MKS_I_N_VALID], route.slot, route.weight, route.topk, shared ? ys : nullptr, route.gate,
+                                           d.i[MKS_I_EPILOGUE] == MKS_E_RESID, at(d.p[MKS_P_OUT]), d.i[MKS_I_OUT_STRIDE]));
         MKP_CUDA(cudaGetLastError());
         written(d.p[MKS_P_OUT]);
         return MK_OK;
@@ -517,15 +524,15 @@ struct Exec {
         G.out = s->x;
         G.out_rows = s->rows;
         G.gram = gram;
-        return launch_gdn(G, gdn_gate<1>, st);
+        return launch_gdn(G, gdn_gate<1>, sms, st);
     }
 
     template <int HD>
     int attn_hd(const AttnArgs& T) {
         const int bq = AT_ROWS / (T.nq / T.nkv);
-        attn_prepare<HD, false, false><<<dim3((T.nq + 2 * T.nkv + 7) / 8, rows), 256, 0, st>>>(T);
+        MKP_CUDA(launch((attn_prepare<HD, false, false>), dim3((T.nq + 2 * T.nkv + 7) / 8, rows), 256, 0, st, T));
         MKP_CUDA(cudaFuncSetAttribute(attn_rows<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem<HD>()));
-        attn_rows<HD><<<dim3((L + bq - 1) / bq, T.nkv, M), 256, attn_smem<HD>(), st>>>(T);
+        MKP_CUDA(launch(attn_rows<HD>, dim3((L + bq - 1) / bq, T.nkv, M), 256, attn_smem<HD>(), st, T));
         MKP_CUDA(cudaGetLastError());
         return MK_OK;
     }
@@ -574,18 +581,18 @@ struct Exec {
         MKP_CUDA(cudaMemsetAsync(route.counts, 0, (3 * route.experts + 1) * sizeof(int), st));
         route.ids_out = h_last ? reinterpret_cast<int*>(d.p[MKS_P_ROUTE_OUT]) : nullptr;
         route.L = L;
-        route_rows<<<(rows + 7) / 8, 256, 0, st>>>(route);
-        route_plan<<<1, 256, 0, st>>>(route);
-        route_slots<<<(rows * 8 + 255) / 256, 256, 0, st>>>(route);
+        MKP_CUDA(launch(route_rows, dim3((rows + 7) / 8), 256, 0, st, route));
+        MKP_CUDA(launch(route_plan, dim3(1), 256, 0, st, route));
+        MKP_CUDA(launch(route_slots, dim3((rows * 8 + 255) / 256), 256, 0, st, route));
         MKP_CUDA(cudaGetLastError());
         return MK_OK;
     }
 
     int vec(const mk_stage_desc& d) {
         if (!d.i[MKS_I_VEC_N]) return MK_OK;
-        vec_rows<<<rows, 256, 0, st>>>(d.i[MKS_I_VEC_N], at(d.p[MKS_P_VEC_BASE]), at(d.p[MKS_P_VEC_A]), reinterpret_cast<const float*>(d.p[MKS_P_VEC_A_W]),
+        MKP_CUDA(launch(vec_rows, dim3(rows), 256, 0, st, d.i[MKS_I_VEC_N], at(d.p[MKS_P_VEC_BASE]), at(d.p[MKS_P_VEC_A]), reinterpret_cast<const float*>(d.p[MKS_P_VEC_A_W]),
                                        at(d.p[MKS_P_VEC_B]), reinterpret_cast<const float*>(d.p[MKS_P_VEC_B_W]), d.f[MKS_F_NORM_OFF], d.f[MKS_F_EPS],
-                                       d.f[MKS_F_SCALE] != 0.f ? d.f[MKS_F_SCALE] : 1.f, at(d.p[MKS_P_VEC_OUT]));
+                                       d.f[MKS_F_SCALE] != 0.f ? d.f[MKS_F_SCALE] : 1.f, at(d.p[MKS_P_VEC_OUT])));
         MKP_CUDA(cudaGetLastError());
         written(d.p[MKS_P_VEC_OUT]);
         return MK_OK;
@@ -597,8 +604,8 @@ struct Exec {
             int rc = MK_OK;
             switch (d.op) {
                 case MKS_OP_EMBED:
-                    embed_rows<<<rows, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(d.p[MKS_P_TABLE]), tokens, M, L, d.i[MKS_I_HIDDEN], d.i[MKS_I_VOCAB],
-                                                     d.f[MKS_F_SCALE], at(d.p[MKS_P_H]));
+                    MKP_CUDA(launch(embed_rows, dim3(rows), 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(d.p[MKS_P_TABLE]), tokens, M, L, d.i[MKS_I_HIDDEN], d.i[MKS_I_VOCAB],
+                                                     d.f[MKS_F_SCALE], at(d.p[MKS_P_H])));
                     MKP_CUDA(cudaGetLastError());
                     written(d.p[MKS_P_H]);
                     break;
@@ -616,9 +623,9 @@ struct Exec {
         }
         if (h_last) {
             const mk_stage_desc& d = prog[0];
-            last_rows<<<M, 256, 0, st>>>(at(d.p[MKS_P_H]), L, d.i[MKS_I_HIDDEN], reinterpret_cast<float*>(d.p[MKS_P_H]), reinterpret_cast<float*>(d.p[MKS_P_H_SSQ]));
+            MKP_CUDA(launch(last_rows, dim3(M), 256, 0, st, at(d.p[MKS_P_H]), L, d.i[MKS_I_HIDDEN], reinterpret_cast<float*>(d.p[MKS_P_H]), reinterpret_cast<float*>(d.p[MKS_P_H_SSQ])));
         }
-        advance_pos<<<1, 32, 0, st>>>(pos, M, h_last ? L - 1 : L);
+        MKP_CUDA(launch(advance_pos, dim3(1), 32, 0, st, pos, M, h_last ? L - 1 : L));
         MKP_CUDA(cudaGetLastError());
         return MK_OK;
     }

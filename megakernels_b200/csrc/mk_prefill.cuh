@@ -33,6 +33,15 @@ using mk::u64;
 using mk::warp_max;
 using mk::warp_sum;
 
+// A pass is a chain of some hundred short kernels, launched with programmatic stream serialisation: a kernel's CTAs come up
+// while the one before drains, and wait here for its end before they touch memory that any kernel of the chain writes.  Every
+// kernel of the chain calls this first thing (a CTA that left without it would let the next kernel start too early), or behind a
+// prologue that reads nothing but the packed weights.  (512 tokens of the 0.8B model, 231 launches: 5.79 ms without the attribute, 5.28 with it.)
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 constexpr int ERR_TIMEOUT = -2;
 enum { WP_EMPTY = 301, WP_FULL, WP_DONE, WP_DRAIN };
 
@@ -101,6 +110,7 @@ struct GemmArgs {
     int ksplit;                  // CTAs that share K; > 1: fp32 partials [split][part_rows][n_valid] in `part`
     float* part;
     int part_rows;
+    bool leave;                  // the partials are left to rows_in
     int gelu;
     // routed groups: items[i] = {group, first row, rows, 0}, n_items on the device
     const int4* items;
@@ -348,8 +358,9 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ?
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int group = 0, row0, rows, block, z = 0;
     if (A.items) {
-        if ((int)blockIdx.y >= __ldg(A.n_items)) return;
-        const int4 it = __ldg(A.items + blockIdx.y);
+        chain_wait();
+        if ((int)blockIdx.y >= __ldcg(A.n_items)) return;
+        const int4 it = __ldcg(A.items + blockIdx.y);
         group = it.x;
         row0 = it.y;
         rows = it.z;
@@ -389,6 +400,7 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ?
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = B.tmem;
+    if (!A.items && (FMT == W_SLAB || warp >= CW)) chain_wait();
 
     if (warp == CW) {
         if (lane == 0) {
@@ -496,6 +508,7 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ?
             };
 #pragma unroll
             for (int i = 0; i < DIST; i++) request(raw[i]);
+            if (!A.items) chain_wait();
             uint32_t slot = (uint32_t)(warp >> 3), phase = 0;
             bool ok = true;
 #pragma unroll 1
@@ -644,6 +657,7 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ?
 // Adds the K splits' partials in split order and runs the epilogue.
 template <int PX, int OUT>
 static __global__ void __launch_bounds__(256) rows_finish(const __grid_constant__ GemmArgs A) {
+    chain_wait();
     const int t = blockIdx.y;
     const float* p = A.part + (size_t)t * A.n_valid;
     const size_t ss = (size_t)A.part_rows * A.n_valid;
@@ -701,37 +715,61 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // fp32 rows -> slabs: optional RMSNorm, rounding to bf16 (PIECES = 1, the model's activation type) or fp32-exact pieces.
-template <int PIECES>
-static __global__ void __launch_bounds__(256) rows_in(const float* x, long long stride, int K, const float* norm_w, float norm_off, float eps, float in_scale,
-                                               uint8_t* out, size_t piece, int out_rows) {
+// PARTS: the row is `x` plus the K splits' partial products `part` [split][rows][K], in split order, and is stored back first:
+// the end of one product and the input of the next in one pass over the residual (511 x 1024, eight splits: 5.6 us against 5.4 + 4.3).
+struct RowsIn {
+    float* x;
+    long long stride;
+    int K, ksplit, rows;
+    const float* part;
+    const float* norm_w;
+    float norm_off, eps, in_scale;
+    uint8_t* out;
+    size_t piece;
+    int out_rows;
+};
+template <int PIECES, bool PARTS>
+static __global__ void __launch_bounds__(256) rows_in(const __grid_constant__ RowsIn R) {
+    chain_wait();
     __shared__ float red[8];
-    const int row = blockIdx.x;
-    const float* src = x + (size_t)row * stride;
+    const int row = blockIdx.x, K = R.K;
+    float* src = R.x + (size_t)row * R.stride;
     float r = 1.f;
-    if (norm_w) {
+    if (R.norm_w) {
         float s = 0.f;
         for (int c = threadIdx.x * 4; c < K; c += 1024) {
-            const float4 a = *reinterpret_cast<const float4*>(src + c);
+            float4 a = *reinterpret_cast<const float4*>(src + c);
+            if (PARTS) {
+                const float* p = R.part + (size_t)row * K + c;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int z = 0; z < R.ksplit; z++, p += (size_t)R.rows * K) {
+                    const float4 b = *reinterpret_cast<const float4*>(p);
+                    v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+                }
+                a = make_float4(v.x + a.x, v.y + a.y, v.z + a.z, v.w + a.w);
+                *reinterpret_cast<float4*>(src + c) = a;
+            }
             s += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
         }
-        s = block_sum(s, red);
-        r = rsqrtf(s / (float)K + eps) * in_scale;
+        s = block_sum(s, red);                     // (its barriers also publish the stored row to the block)
+        r = rsqrtf(s / (float)K + R.eps) * R.in_scale;
     }
     for (int c = threadIdx.x * 8; c < K; c += 2048) {
         const float4 a = *reinterpret_cast<const float4*>(src + c), b = *reinterpret_cast<const float4*>(src + c + 4);
         float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        if (norm_w) {
-            const float4 wa = __ldg(reinterpret_cast<const float4*>(norm_w + c)), wb = __ldg(reinterpret_cast<const float4*>(norm_w + c + 4));
+        if (R.norm_w) {
+            const float4 wa = __ldg(reinterpret_cast<const float4*>(R.norm_w + c)), wb = __ldg(reinterpret_cast<const float4*>(R.norm_w + c + 4));
             const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = v[i] * r * (norm_off + w[i]);
+            for (int i = 0; i < 8; i++) v[i] = v[i] * r * (R.norm_off + w[i]);
         }
-        store_slab8<PIECES>(out, piece, out_rows, row, c, v);
+        store_slab8<PIECES>(R.out, R.piece, R.out_rows, row, c, v);
     }
 }
 
 // Row r = sequence * L + position of every array below; tokens are [L][M] (step-major, as mk_stage_args.tokens_in).
 static __global__ void __launch_bounds__(256) embed_rows(const __nv_bfloat16* table, const int* tokens, int M, int L, int H, int vocab, float scale, float* h) {
+    chain_wait();
     const int row = blockIdx.x, m = row / L, l = row - m * L;
     const int tok = max(0, min(vocab - 1, tokens[(size_t)l * M + m]));
     const uint32_t* src = reinterpret_cast<const uint32_t*>(table + (size_t)tok * H);
@@ -749,6 +787,7 @@ static __global__ void __launch_bounds__(256) embed_rows(const __nv_bfloat16* ta
 
 // The last position of every sequence: its residual and the sums of squares per 16 elements, where a decode step leaves them.
 static __global__ void __launch_bounds__(256) last_rows(const float* h, int L, int H, float* out, float* ssq) {
+    chain_wait();
     const int m = blockIdx.x;
     const float* src = h + ((size_t)m * L + L - 1) * H;
     for (int g = threadIdx.x; g < H / 16; g += 256) {
@@ -763,12 +802,14 @@ static __global__ void __launch_bounds__(256) last_rows(const float* h, int L, i
 }
 
 static __global__ void advance_pos(int* pos, int M, int L) {
+    chain_wait();
     if ((int)threadIdx.x < M) pos[threadIdx.x] += L;
 }
 
 // out = (base + rms(a) w_a [+ rms(b) w_b]) * scale
 static __global__ void __launch_bounds__(256) vec_rows(int N, const float* base, const float* a, const float* wa, const float* b, const float* wb, float off, float eps,
                                                 float scale, float* out) {
+    chain_wait();
     __shared__ float red[8];
     const size_t o = (size_t)blockIdx.x * N;
     float sa = 0.f, sb = 0.f;
@@ -825,6 +866,7 @@ __device__ __forceinline__ float* conv_slot(const GdnArgs& G, int m, int ch, int
 // once per CONV_ROWS + 3 rows instead of four times.
 constexpr int CONV_ROWS = 8;
 static __global__ void __launch_bounds__(256) gdn_conv(const __grid_constant__ GdnArgs G) {
+    chain_wait();
     const int groups = (G.L + CONV_ROWS - 1) / CONV_ROWS, m = blockIdx.y / groups, l0 = (blockIdx.y - m * groups) * CONV_ROWS, lane = threadIdx.x & 31;
     const int blk = blockIdx.x * 8 + (threadIdx.x >> 5);                    // 128-channel block: q heads, k heads, v heads
     if (blk * 128 >= G.conv_dim) return;
@@ -888,9 +930,10 @@ static __global__ void __launch_bounds__(256) gdn_conv(const __grid_constant__ G
     }
 }
 
-// The last `ring` inputs of every channel go back into the history rings.  Runs after gdn_conv has read them.
-static __global__ void __launch_bounds__(256) gdn_history(const __grid_constant__ GdnArgs G) {
-    const int ch = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y, l = G.L - 1 - (int)blockIdx.z;
+// The last `ring` inputs of every channel go back into the history rings, 128 channels of one ring slot per block.  Only after
+// gdn_conv has read them: gdn_gram's last blocks do it.
+__device__ __forceinline__ void put_history(const GdnArgs& G, int block) {
+    const int per = (G.conv_dim + 127) / 128, ch = block % per * 128 + threadIdx.x, z = block / per % G.ring, m = block / (per * G.ring), l = G.L - 1 - z;
     if (ch >= G.conv_dim || l < 0) return;
     const int qk = G.nkh * 128, part = ch < qk ? 0 : (ch < 2 * qk ? 1 : 2);
     const int col = (part == 0 ? G.q_off : (part == 1 ? G.k_off : G.v_off)) + ch - part * qk;
@@ -911,7 +954,12 @@ constexpr int SCAN = 8;
 // P_t, P_8 / P_t and beta_t (a position past the end decays by 1 and corrects by 0).  One warp per block and key head.
 constexpr int GRAM = SCAN * SCAN + 3 * SCAN;
 static __global__ void __launch_bounds__(128) gdn_gram(const __grid_constant__ GdnArgs G) {
-    const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, chunks = (G.L + SCAN - 1) / SCAN;
+    chain_wait();
+    const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, chunks = (G.L + SCAN - 1) / SCAN, blocks = (G.M * chunks * G.nkh + 3) / 4;
+    if ((int)blockIdx.x >= blocks) {
+        put_history(G, blockIdx.x - blocks);
+        return;
+    }
     if (w >= G.M * chunks * G.nkh) return;
     const int kh = w % G.nkh, c = (w / G.nkh) % chunks, m = w / (G.nkh * chunks), rep = G.nvh / G.nkh;
     float4 q[SCAN], k[SCAN];
@@ -980,6 +1028,7 @@ __device__ __forceinline__ float sum2(u64 a) { return __uint_as_float((uint32_t)
 // every lane reads its keys of eight k and eight q.  Two rows a lane halve the reads per product, and the k's stay in registers
 // for the update.  16 heads x 511 positions: 54 us (69 with eight lanes to one row; 207 position by position).
 static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ GdnArgs G) {
+    chain_wait();
     constexpr int ROWS = 16, IN = 256 + ROWS;
     __shared__ __align__(16) float in_s[2][SCAN][IN];        // q | k | values
     __shared__ __align__(16) float mats[2][GRAM];            // what gdn_gram left for the block
@@ -1090,6 +1139,7 @@ static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ G
 // Gated RMSNorm per head, into slabs: one half warp per head and row (eight columns per lane).
 template <int PIECES>
 static __global__ void __launch_bounds__(256) gdn_gate(const __grid_constant__ GdnArgs G) {
+    chain_wait();
     const int row = blockIdx.y, h = blockIdx.x * 16 + (threadIdx.x >> 4), i = (threadIdx.x & 15) * 8;
     if (h >= G.nvh) return;
     const float* o = G.o + (size_t)row * (G.nvh * 128) + h * 128 + i;
@@ -1139,6 +1189,7 @@ __device__ __forceinline__ size_t kv_offset(const AttnArgs& T, int m, int kvh, i
 // One warp per head vector; lane i holds dims i + 32 j, so both halves of a rotated pair are in one lane.
 template <int HD, bool QF32, bool KVF32>
 static __global__ void __launch_bounds__(256) attn_prepare(const __grid_constant__ AttnArgs T) {
+    chain_wait();
     constexpr int N = HD / 32;
     const int row = blockIdx.y, m = row / T.L, lane = threadIdx.x & 31;
     const int hv = blockIdx.x * 8 + (threadIdx.x >> 5);                 // q heads, k heads, v heads
@@ -1214,6 +1265,7 @@ constexpr int AT_ROWS = 64, AT_KEYS = 64, AT_PIECES = 3;
 template <int HD> constexpr int attn_smem() { return 3 * AT_ROWS * HD * 2 + AT_PIECES * AT_ROWS * AT_KEYS * 2 + 4 * AT_ROWS * 4; }
 template <int HD>
 static __global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant__ AttnArgs T) {
+    chain_wait();
     extern __shared__ __align__(128) uint8_t sm[];
     constexpr int RB = HD * 2, CH = RB / 16;                             // bytes and 16-byte pieces of a row
     uint8_t *q_s = sm, *k_s = q_s + AT_ROWS * RB, *v_s = k_s + AT_KEYS * RB, *p_s = v_s + AT_KEYS * RB;
@@ -1384,6 +1436,7 @@ __device__ __forceinline__ void split4(uint8_t* base, size_t piece, int row, int
 }
 template <bool KVF32>
 static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_constant__ AttnArgs T) {
+    chain_wait();
     extern __shared__ __align__(128) uint8_t sm[];
     constexpr int KP = KVF32 ? 3 : 1, QB = AF_ROWS * AF_RB, KB = AF_KEYS * AF_RB, PB = AF_ROWS * AF_KEYS * 2;
     constexpr int PER = AF_KEYS * AF_HD / 4 / 256;                        // groups of four columns per thread and block
@@ -1588,8 +1641,10 @@ static __global__ void __launch_bounds__(256, 2) experts_gemm(const __grid_const
     constexpr int X_KB = NT8 * 8 * 128;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     ExpertBars& B = *reinterpret_cast<ExpertBars*>(smem + EX_STAGES * 2 * X_KB);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, units = __ldg(A.n_items) * A.blocks;
-    auto item = [&](int u) { return __ldg(A.items + min(u, units - 1) / A.blocks); };
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    chain_wait();
+    const int units = __ldcg(A.n_items) * A.blocks;
+    auto item = [&](int u) { return __ldcg(A.items + min(u, units - 1) / A.blocks); };
     if ((int)blockIdx.x >= units) return;
     if (threadIdx.x == 0) {
         for (int i = 0; i < EX_STAGES; i++) {
@@ -1774,6 +1829,7 @@ struct RouteArgs {
 
 // One warp per token: the top-k experts (ties to the lower id), their weights, and the count per expert.
 static __global__ void __launch_bounds__(256) route_rows(const __grid_constant__ RouteArgs R) {
+    chain_wait();
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= R.rows) return;
     const float* lg = R.logits + (size_t)row * R.stride;
@@ -1829,6 +1885,7 @@ static __global__ void __launch_bounds__(256) route_rows(const __grid_constant__
 
 // Lays the experts' tokens out one after the other (each expert from a multiple of 16 rows) and lists the tiles.
 static __global__ void __launch_bounds__(256) route_plan(const __grid_constant__ RouteArgs R) {
+    chain_wait();
     __shared__ int rows_s[256], tiles_s[256];
     const int e = threadIdx.x, n = e < R.experts ? R.counts[e] : 0;
     const int rows = (n + 15) & ~15, tiles = (n + R.nt - 1) / R.nt;
@@ -1851,6 +1908,7 @@ static __global__ void __launch_bounds__(256) route_plan(const __grid_constant__
 }
 
 static __global__ void __launch_bounds__(256) route_slots(const __grid_constant__ RouteArgs R) {
+    chain_wait();
     const int i = blockIdx.x * 256 + threadIdx.x, row = i >> 3, k = i & 7;
     if (row >= R.rows || k >= R.topk) return;
     const int e = R.slot[i];
@@ -1861,6 +1919,7 @@ static __global__ void __launch_bounds__(256) route_slots(const __grid_constant_
 // reads them.
 template <bool EO>
 static __global__ void __launch_bounds__(256) gather_rows(const uint8_t* x, int x_rows, const int* slot, int topk, int kbs, uint8_t* out, int out_rows) {
+    chain_wait();
     const int row = blockIdx.x;
     for (int i = threadIdx.x; i < kbs * 4; i += 256) {
         const int kb = i >> 2, c = 2 * (i & 3);
@@ -1883,6 +1942,7 @@ static __global__ void __launch_bounds__(256) gather_rows(const uint8_t* x, int 
 // Weighted sum of a token's expert outputs (ascending expert id, then the shared expert), stored or added.
 static __global__ void __launch_bounds__(256) combine_rows(const float* y, int N, const int* slot, const float* weight, int topk, const float* shared, const float* gate,
                                                     int add, float* out, long long out_stride) {
+    chain_wait();
     const int row = blockIdx.x;
     for (int c = threadIdx.x * 4; c < N; c += 1024) {
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);

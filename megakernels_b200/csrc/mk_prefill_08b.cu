@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(256) slabs_from_cols(const uint8_t* w, int sli
 
 template <bool Q8>
 __global__ void __launch_bounds__(256) embed_rows_08b(const uint8_t* table, const float* scale, const int* tokens, int vocab, float* h) {
+    chain_wait();
     const int tok = max(0, min(vocab - 1, tokens[blockIdx.x])), c = threadIdx.x * 4;
     float4 v;
     if (Q8) {
@@ -96,7 +97,10 @@ __global__ void __launch_bounds__(256) embed_rows_08b(const uint8_t* table, cons
     *reinterpret_cast<float4*>(h + (size_t)blockIdx.x * S::HID + c) = v;
 }
 
-__global__ void put_pos(int* p, int v) { *p = v; }
+__global__ void put_pos(int* p, int v) {
+    chain_wait();
+    *p = v;
+}
 
 // Where a layer's four matrices lie among the slabs (rows rounded up to whole 128-row blocks).
 struct LayerSlabs {
@@ -157,7 +161,18 @@ struct Run {
         pos = arena.take<int>(1);
     }
 
-    int product(const uint8_t* w, int N, int K, const uint8_t* xs, size_t piece, const float* scale, int out, float* dst, int dst_stride) {
+    int left = 0;                // K splits of a product whose partials wait in `part` to be added to the residual
+
+    // The normed residual as operand slabs; adds what the product before left.
+    int norm(const float* w) {
+        const RowsIn R = {h, S::HID, S::HID, left, rows, part, w, 1.f, S::EPS, 1.f, x, x_piece, xrows};
+        MKP_CUDA(launch(left ? rows_in<PX, true> : rows_in<PX, false>, dim3(rows), 256, 0, st, R));
+        left = 0;
+        return MK_OK;
+    }
+
+    // `leave`: the residual's next reader is norm(), which adds the K splits' partials.
+    int product(const uint8_t* w, int N, int K, const uint8_t* xs, size_t piece, const float* scale, int out, float* dst, int dst_stride, bool leave = false) {
         GemmArgs A;
         memset(&A, 0, sizeof A);
         A.w = w;
@@ -182,6 +197,8 @@ struct Run {
         A.ksplit = N == S::HID ? pick_ksplit(blocks * ntiles, A.kbs, sms) : 1;     // `part` holds the narrow products only
         A.part = part;
         A.part_rows = rows;
+        A.leave = leave;
+        if (leave && A.ksplit > 1) left = A.ksplit;
         A.status = P->status;
         A.spin_limit_ns = spin;
         return launch_gemm<W_SLAB, PX>(A, out, blocks, ntiles, 0, st);
@@ -190,15 +207,15 @@ struct Run {
     int run() {
         const bool q8 = desc->quant == MK_QUANT_INT8, kv32 = desc->kv_dtype == MK_KV_F32;
         int rc;
-        put_pos<<<1, 1, 0, st>>>(pos, start);
-        if (q8) embed_rows_08b<true><<<rows, 256, 0, st>>>(P->embed, P->embed_scale, tokens, P->vocab, h);
-        else embed_rows_08b<false><<<rows, 256, 0, st>>>(P->embed, nullptr, tokens, P->vocab, h);
+        MKP_CUDA(launch(put_pos, dim3(1), 1, 0, st, pos, start));
+        if (q8) MKP_CUDA(launch(embed_rows_08b<true>, dim3(rows), 256, 0, st, P->embed, P->embed_scale, tokens, P->vocab, h));
+        else MKP_CUDA(launch(embed_rows_08b<false>, dim3(rows), 256, 0, st, P->embed, nullptr, tokens, P->vocab, h));
         MKP_CUDA(cudaGetLastError());
         for (int l = 0; l < P->n_layers; l++) {
             const mk::LayerP& L = P->layer[l];
             const bool attn = L.kind != 0;
             const int in_rows = attn ? S::ATT_IN : S::GDN_IN;
-            rows_in<PX><<<rows, 256, 0, st>>>(h, S::HID, S::HID, L.in_norm, 1.f, S::EPS, 1.f, x, x_piece, xrows);
+            if ((rc = norm(L.in_norm)) != MK_OK) return rc;
             const LayerSlabs W(slabs, P, l);
             if ((rc = product(W.in, in_rows, S::HID, x, x_piece, L.s_in, OUT_STORE, y, S::PROJ_MAX)) != MK_OK) return rc;
             if (attn) {
@@ -217,13 +234,13 @@ struct Run {
                 T.pos = pos; T.q = q; T.out = mix; T.out_piece = mix_piece; T.out_rows = xrows;
                 const dim3 pg((S::NQ + 2 * S::NKV + 7) / 8, rows), ag((rows + AF_ROWS / S::QPK - 1) / (AF_ROWS / S::QPK), S::NKV, 1);
                 if (kv32) {
-                    attn_prepare<256, true, true><<<pg, 256, 0, st>>>(T);
+                    MKP_CUDA(launch((attn_prepare<256, true, true>), pg, 256, 0, st, T));
                     MKP_CUDA(cudaFuncSetAttribute(attn_rows_f32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_f32_smem<true>()));
-                    attn_rows_f32<true><<<ag, 256, attn_f32_smem<true>(), st>>>(T);
+                    MKP_CUDA(launch(attn_rows_f32<true>, ag, 256, attn_f32_smem<true>(), st, T));
                 } else {
-                    attn_prepare<256, true, false><<<pg, 256, 0, st>>>(T);
+                    MKP_CUDA(launch((attn_prepare<256, true, false>), pg, 256, 0, st, T));
                     MKP_CUDA(cudaFuncSetAttribute(attn_rows_f32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_f32_smem<false>()));
-                    attn_rows_f32<false><<<ag, 256, attn_f32_smem<false>(), st>>>(T);
+                    MKP_CUDA(launch(attn_rows_f32<false>, ag, 256, attn_f32_smem<false>(), st, T));
                 }
             } else {
                 GdnArgs G;
@@ -237,13 +254,13 @@ struct Run {
                 G.ssm = L.state + (size_t)seq * S::LIN_H * S::LIN_DV * S::LIN_DK;
                 G.pos = pos; G.l2_clamp = 1; G.eps = 1e-6f; G.norm_eps = S::EPS;
                 G.qkv = qkv; G.scal = scal; G.gram = gram; G.o = o; G.out = mix; G.out_piece = mix_piece; G.out_rows = xrows;
-                if ((rc = launch_gdn(G, gdn_gate<PX>, st)) != MK_OK) return rc;
+                if ((rc = launch_gdn(G, gdn_gate<PX>, sms, st)) != MK_OK) return rc;
             }
             MKP_CUDA(cudaGetLastError());
-            if ((rc = product(W.out, S::HID, S::MIX, mix, mix_piece, L.s_out, OUT_ADD, h, S::HID)) != MK_OK) return rc;
-            rows_in<PX><<<rows, 256, 0, st>>>(h, S::HID, S::HID, L.post_norm, 1.f, S::EPS, 1.f, x, x_piece, xrows);
+            if ((rc = product(W.out, S::HID, S::MIX, mix, mix_piece, L.s_out, OUT_ADD, h, S::HID, true)) != MK_OK) return rc;
+            if ((rc = norm(L.post_norm)) != MK_OK) return rc;
             if ((rc = product(W.gu, 2 * S::INTER, S::HID, x, x_piece, L.s_gu, OUT_GLU, nullptr, 0)) != MK_OK) return rc;
-            if ((rc = product(W.down, S::HID, S::INTER, act, act_piece, L.s_down, OUT_ADD, h, S::HID)) != MK_OK) return rc;
+            if ((rc = product(W.down, S::HID, S::INTER, act, act_piece, L.s_down, OUT_ADD, h, S::HID, l + 1 < P->n_layers)) != MK_OK) return rc;
         }
         return MK_OK;
     }

@@ -26,6 +26,22 @@ inline int pfail(int code, const char* fmt, ...) {
             return pfail(MK_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(err__));   \
     } while (0)
 
+// Launches a kernel of the chain (see chain_wait).
+template <class Kernel, class... Args>
+inline cudaError_t launch(Kernel fn, dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
 constexpr int SMEM_MAX = 232448;
 constexpr int DRAIN_GROUPS = 4;                     // rows_gemm: three-piece products in tiles of up to 32 x 4 tokens
 constexpr int MAX_ROWS = 65535;                     // token rows of a call: one grid coordinate of several kernels
@@ -47,7 +63,7 @@ template <int FMT, int PX, int CG, int DG, bool WIDE = false>
 int launch_gemm_cg(GemmArgs& A, int out, dim3 grid, int smem, cudaStream_t st) {
     auto fn = out == OUT_STORE ? rows_gemm<FMT, PX, OUT_STORE, CG, DG, WIDE> : (out == OUT_ADD ? rows_gemm<FMT, PX, OUT_ADD, CG, DG, WIDE> : rows_gemm<FMT, PX, OUT_GLU, CG, DG, WIDE>);
     MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    fn<<<grid, (8 * CG + 2) * 32, smem, st>>>(A);
+    MKP_CUDA(launch(fn, grid, (8 * CG + 2) * 32, smem, st, A));
     MKP_CUDA(cudaGetLastError());
     return MK_OK;
 }
@@ -84,11 +100,11 @@ int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaSt
         }
     }
     if (rc != MK_OK) return rc;
-    if (A.ksplit > 1) {
+    if (A.ksplit > 1 && !A.leave) {
         const dim3 fgrid(out == OUT_GLU ? (A.act_cols + 255) / 256 : (A.n_valid + 1023) / 1024, A.rows);
-        if (out == OUT_STORE) rows_finish<PX, OUT_STORE><<<fgrid, 256, 0, st>>>(A);
-        else if (out == OUT_ADD) rows_finish<PX, OUT_ADD><<<fgrid, 256, 0, st>>>(A);
-        else rows_finish<PX, OUT_GLU><<<fgrid, 256, 0, st>>>(A);
+        if (out == OUT_STORE) MKP_CUDA(launch((rows_finish<PX, OUT_STORE>), fgrid, 256, 0, st, A));
+        else if (out == OUT_ADD) MKP_CUDA(launch((rows_finish<PX, OUT_ADD>), fgrid, 256, 0, st, A));
+        else MKP_CUDA(launch((rows_finish<PX, OUT_GLU>), fgrid, 256, 0, st, A));
         MKP_CUDA(cudaGetLastError());
     }
     return MK_OK;
@@ -101,19 +117,24 @@ int launch_experts(GemmArgs& A, int out, int items, int sms, cudaStream_t st) {
     const long long units = (long long)items * A.blocks;
     auto fn = out == OUT_GLU ? experts_gemm<BLOCKS, OUT_GLU, NT8> : experts_gemm<BLOCKS, OUT_STORE, NT8>;
     MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    fn<<<(int)(units < 2 * sms ? units : 2 * sms), 256, smem, st>>>(A);
+    MKP_CUDA(launch(fn, dim3((int)(units < 2 * sms ? units : 2 * sms)), 256, smem, st, A));
     MKP_CUDA(cudaGetLastError());
     return MK_OK;
 }
 
 // The DeltaNet mixer of M sequences of L rows; `gate` is gdn_gate of the wanted number of pieces.
-inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), cudaStream_t st) {
+inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), int sms, cudaStream_t st) {
     const int rows = G.M * G.L, chunks = (G.L + SCAN - 1) / SCAN;
-    gdn_conv<<<dim3((G.conv_dim / 128 + 7) / 8, G.M * ((G.L + CONV_ROWS - 1) / CONV_ROWS)), 256, 0, st>>>(G);
-    gdn_history<<<dim3((G.conv_dim + 255) / 256, G.M, G.ring), 256, 0, st>>>(G);
-    gdn_gram<<<(G.M * chunks * G.nkh + 3) / 4, 128, 0, st>>>(G);
-    gdn_scan<<<dim3(8, G.nvh, G.M), 128, 0, st>>>(G);
-    gate<<<dim3((G.nvh + 15) / 16, rows), 256, 0, st>>>(G);
+    MKP_CUDA(launch(gdn_conv, dim3((G.conv_dim / 128 + 7) / 8, G.M * ((G.L + CONV_ROWS - 1) / CONV_ROWS)), 256, 0, st, G));
+    MKP_CUDA(launch(gdn_gram, dim3((G.M * chunks * G.nkh + 3) / 4 + G.M * G.ring * ((G.conv_dim + 127) / 128)), 128, 0, st, G));
+    // One CTA per SM or less: not with the chain's attribute.  Brought up while gdn_gram's many small CTAs drain, several of them
+    // land on one SM and share its shared memory, which is what they are bound by (16 heads x 511 positions: the pass takes 6.41 instead
+    // of 5.27 ms).  With more CTAs than SMs they share anyway.
+    const dim3 scan(8, G.nvh, G.M);
+    if (8 * G.nvh * G.M <= sms) gdn_scan<<<scan, 128, 0, st>>>(G);
+    else MKP_CUDA(launch(gdn_scan, scan, 128, 0, st, G));
+    MKP_CUDA(cudaGetLastError());
+    MKP_CUDA(launch(gate, dim3((G.nvh + 15) / 16, rows), 256, 0, st, G));
     MKP_CUDA(cudaGetLastError());
     return MK_OK;
 }
