@@ -586,7 +586,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) batch_kernel(const __grid_constan
         c.sm.wsc_s = reinterpret_cast<float*>(p); p += NB * NCW * 4;                           // 512
         c.sm.full = reinterpret_cast<uint64_t*>(p); p += 6 * 8;
         c.sm.empty = reinterpret_cast<uint64_t*>(p); p += 6 * 8;
-        c.sm.xscale_s = reinterpret_cast<float*>(p); p += 8;
         c.sm.abort_flag = reinterpret_cast<volatile int*>(p); p += 4;
         c.sm.quit_flag = reinterpret_cast<volatile int*>(p); p += 4;
     }

@@ -41,10 +41,9 @@ struct Smem {
     float* xown;        // fp32 master copy of the residual rows this CTA owns, [T][16]
     u64* best_s;        // [NCW] block-reduction scratch for 64-bit keys
     float* scale_s;     // per-row scales: two 128-row buffers for layer GEMVs, then the streaming ring
-    float* xscale_s;    // [T] power-of-two factors that undo the fixed-point scaling of the staged inputs
     float* act_s;       // [T][DOWN_K] this CTA's SwiGLU outputs (entries past its slice stay zero)
     float* mix_s;       // [T][DOWN_K] this DeltaNet task's gated outputs (16 value columns, the rest zero)
-    float* ssq_s;       // batched decoding: [sequence][NCW] per-warp sums of squares of the RMSNorm input staged last
+    float* ssq_s;       // [token or sequence][NCW] per-warp sums of squares of the RMSNorm input staged last
     float* wsc_s;       // batched decoding: [NCW][sequence] inverse fixed-point scales of each warp's k-slice
     uint64_t* full;     // [ring stages]
     uint64_t* empty;    // [ring stages]
@@ -276,8 +275,18 @@ template <int T> struct Geo {
     static constexpr int RING = NS * SLOT_BYTES;
     static constexpr int XQ = (T == 1 ? 3 : 7) * 2 * 3584;          // input planes: bf16 pieces of K = 3584 are the largest
     static constexpr int PART = NCW * T * 64 * 4;                   // per-warp partial sums
-    static constexpr int SMEM = RING + XQ + PART + MAX_BLOCKS * 4 + 2048 + 2048;
+    static constexpr int SMEM = RING + XQ + PART + MAX_BLOCKS * 4 + 2048 + 2304;
 };
+
+// Sum of one value per consumer warp (16-byte aligned), in a fixed order of short chains.
+__device__ __forceinline__ float sum_warps(const float* v) {
+    static_assert(NCW == 16, "four vectors");
+    const float4 a = *reinterpret_cast<const float4*>(v), b = *reinterpret_cast<const float4*>(v + 4);
+    const float4 c = *reinterpret_cast<const float4*>(v + 8), d = *reinterpret_cast<const float4*>(v + 12);
+    return (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) + (((c.x + c.y) + (c.z + c.w)) + ((d.x + d.y) + (d.z + d.w)));
+}
+// Largest of the lanes' magnitudes: their bits order like the values.
+__device__ __forceinline__ float warp_absmax(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v) & 0x7fffffffu)); }
 
 // Sums and maxima over all consumer threads in one barrier, fixed order; one pair per token.
 template <int T>
@@ -294,13 +303,13 @@ __device__ __forceinline__ void consumer_sum_max(Ctx& c, float (&sum)[T], float 
     consumer_sync();
 #pragma unroll
     for (int j = 0; j < T; j++) {
-        float t = 0.f, m = 0.f;
+        float m = 0.f;
 #pragma unroll
-        for (int i = 0; i < NCW; i++) {
-            t += buf[(2 * j) * NCW + i];
-            m = fmaxf(m, buf[(2 * j + 1) * NCW + i]);
+        for (int i = 0; i < NCW; i += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(buf + (2 * j + 1) * NCW + i);
+            m = fmaxf(fmaxf(m, fmaxf(a.x, a.y)), fmaxf(a.z, a.w));
         }
-        sum[j] = t;
+        sum[j] = sum_warps(buf + (2 * j) * NCW);
         mx[j] = m;
     }
 }
@@ -443,12 +452,13 @@ __device__ __forceinline__ void mma_blocks(const uint8_t* buf, const uint8_t* xr
 //                   warps 2 * token and 2 * token + 1 finish that token's rows;
 //   STREAM = true   (LM head, draft head): one barrier per chunk, warp `token` finishes that token's
 //                   rows of the chunk while the other warps move on.
+// `unscale[token]` undoes the fixed-point scale of this warp's k-slice of the input.  `rms`: the input was x (1 + w) of an
+// RMSNorm, and the finishing warps apply the 1 / rms that follows from the warps' sums of squares in `ssq_s`.
 // A finishing warp calls sink(lane, row, token, value, valid) on all of its lanes; `value` already
-// carries the row's scale and the input's fixed-point scale.  A layer GEMV ends with one more barrier
-// after the sink (`tail_barrier`).
-template <bool Q8, int T, bool STREAM, class Sink>
+// carries the row's scale.  A layer GEMV ends with one more barrier after the sink.
+template <class S, bool Q8, int T, bool STREAM, class Sink>
 __device__ __forceinline__ void gemv_mma(Ctx& c, int r0, int r1, int rb, const float* __restrict__ row_scale,
-                                         Sink&& sink, bool tail_barrier = true) {
+                                         const float (&unscale)[T], bool rms, Sink&& sink) {
     constexpr int NS = Geo<T>::NS;
     const int rpc = SLOT_BYTES / rb;
     const int nkb = rb >> 6;
@@ -456,6 +466,9 @@ __device__ __forceinline__ void gemv_mma(Ctx& c, int r0, int r1, int rb, const f
     const uint8_t* xrow = c.sm.xq + g * rb + t * 16;                      // plane g = column g of the B operand
     const bool xlive = (g >> 2) < T && (g & 3) < Planes<Q8>::N;
     const int tok = t >> 1;                                               // token whose sums this lane ends up with
+    const float us = unscale[T > 1 && tok ? T - 1 : 0];
+    auto post_factor = [&](int j) { return rms ? rsqrtf(sum_warps(c.sm.ssq_s + j * NCW) * (1.0f / S::HID) + S::EPS) : 1.0f; };
+    float post = 1.f;
     const float* scales = STREAM ? c.sm.scale_s + 2 * SCALE_BODY : c.sm.scale_s + (c.gemv_n & 1) * SCALE_BODY;
     c.gemv_n++;
     float pend = 1.f;                            // scale fetched for the chunk four ahead (STREAM)
@@ -487,7 +500,7 @@ __device__ __forceinline__ void gemv_mma(Ctx& c, int r0, int r1, int rb, const f
             if ((t & 1) == 0 && tok < T) {
 #pragma unroll
                 for (int q = 0; q < 4; q++)
-                    if (b0 + 8 * q + g < nr) part[b0 + 8 * q + g] = v[q];
+                    if (b0 + 8 * q + g < nr) part[b0 + 8 * q + g] = Q8 ? v[q] * us : v[q];
             }
         }
         __syncwarp();
@@ -498,11 +511,12 @@ __device__ __forceinline__ void gemv_mma(Ctx& c, int r0, int r1, int rb, const f
             consumer_sync();
             if (c.warp < T) {
                 const float* pp = c.sm.part_s + ((n & 1) * NCW * T + c.warp) * 32 + c.lane;
-                float v = 0.f;
+                float p[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int w = 0; w < NCW; w++) v += pp[w * T * 32];
+                for (int w = 0; w < NCW; w++) p[w & 3] += pp[w * T * 32];
+                if (chunk == 0) post = post_factor(c.warp);
                 const float rs = row_scale ? scales[(chunk & 7) * 32 + c.lane] : 1.f;
-                sink(c.lane, base + c.lane, c.warp, v * rs * c.sm.xscale_s[c.warp], c.lane < nr);
+                sink(c.lane, base + c.lane, c.warp, ((p[0] + p[1]) + (p[2] + p[3])) * post * rs, c.lane < nr);
             }
         }
     }
@@ -513,18 +527,18 @@ __device__ __forceinline__ void gemv_mma(Ctx& c, int r0, int r1, int rb, const f
         if (c.warp < 2 * T) {
             const int tk = c.warp >> 1, idx = (c.warp & 1) * 32 + c.lane;
             const float* pp = c.sm.part_s + tk * 64 + idx;
-            float v = 0.f;
+            float p[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int w = 0; w < NCW; w++) v += pp[w * T * 64];
+            for (int w = 0; w < NCW; w++) p[w & 3] += pp[w * T * 64];
+            post = post_factor(tk);
             const float rs = row_scale ? scales[idx] : 1.f;
-            sink(c.lane, r0 + idx, tk, v * rs * c.sm.xscale_s[tk], idx < r1 - r0);
+            sink(c.lane, r0 + idx, tk, ((p[0] + p[1]) + (p[2] + p[3])) * post * rs, idx < r1 - r0);
             MK_MARK(c, 11);
         }
         // Without a barrier here the other warps run ahead into the next op's prologue and poll for its
         // inputs; their loads then sit in this SM's memory pipeline in front of the stores the finishing
         // warps are about to issue, and every CTA's outputs reach the others later (3 % of the step).
-        // A caller that follows up with a barrier of its own passes tail_barrier = false.
-        if (tail_barrier) consumer_sync();
+        consumer_sync();
     }
 }
 
@@ -622,61 +636,29 @@ __device__ void producer_main(Ctx& c, const Params& P, const Args& A) {
 }
 
 // ---- prologues ---------------------------------------------------------------------------------------
-// RMSNorm of T residual vectors into the GEMV input planes.  `x[j]` are this thread's two elements
-// (2*tid, 2*tid+1) of token j.  One block reduction yields, per token, the sum of squares and the
-// largest |x (1 + w)|, from which the fixed-point scale follows without a second pass.  `y` returns
-// the normalised values.
+// RMSNorm of T residual vectors into the GEMV input planes: x[j] are this thread's two elements (2 * tid, 2 * tid + 1) of
+// token j.  A warp stages elements [64 w, 64 w + 64), which is the k-slice it multiplies, with a power-of-two scale of its own
+// (`unscale` undoes it on its partial sums), and leaves its sum of squares in `ssq_s`; the 1 / rms factor is applied to the
+// finished rows.  So nothing block-wide sits between the arrival of the residual and the MMAs (with a block reduction for the norm
+// and the scale, half a microsecond twice per layer, a step took 519 instead of 475 us: int8, 700 positions).
 template <class S, bool Q8, int T>
-__device__ __forceinline__ void stage_rmsnorm(Ctx& c, const float (&x)[T][2], float2 g, float (&y)[T][2]) {
+__device__ __forceinline__ void stage_rmsnorm(Ctx& c, const float (&x)[T][2], float2 g, float (&unscale)[T]) {
     static_assert(S::HID == 2 * NCT, "two residual elements per consumer thread");
     constexpr int RB = Q8 ? S::HID : 2 * S::HID;
-    const int k = 2 * c.tid;
-    float ss[T], mx[T];
-#pragma unroll
-    for (int j = 0; j < T; j++) {
-        y[j][0] = x[j][0] * (1.0f + g.x);
-        y[j][1] = x[j][1] * (1.0f + g.y);
-        ss[j] = x[j][0] * x[j][0] + x[j][1] * x[j][1];
-        mx[j] = fmaxf(fabsf(y[j][0]), fabsf(y[j][1]));
-    }
     MK_MARK(c, 6);
-    consumer_sum_max<T>(c, ss, mx);
-    MK_MARK(c, 7);
 #pragma unroll
     for (int j = 0; j < T; j++) {
-        const float inv = rsqrtf(ss[j] * (1.0f / S::HID) + S::EPS);
-        const float scale = Q8 ? fixed_scale(mx[j] * inv) : 1.0f;
-        y[j][0] *= inv;
-        y[j][1] *= inv;
-        stage_pair<Q8>(c.sm.xq + (size_t)(4 * j) * RB, RB, k, y[j][0], y[j][1], scale);
-        if (c.tid == 0) c.sm.xscale_s[j] = 1.0f / scale;
-    }
-    // No block barrier: a warp stages elements [64 w, 64 w + 64), which is the k-slice it multiplies;
-    // the inverse scales are read after the barrier that follows the MMAs.
-    __syncwarp();
-}
-
-// For inputs that need no norm: per-token fixed-point scales from this thread's largest magnitudes
-// (one block reduction on the int8 path, nothing on the bf16 path) ...
-template <bool Q8, int T>
-__device__ __forceinline__ void block_scale(Ctx& c, float (&mx)[T], float (&scale)[T]) {
-    if (Q8) {
-        float dummy[T];
-#pragma unroll
-        for (int j = 0; j < T; j++) dummy[j] = 0.f;
-        consumer_sum_max<T>(c, dummy, mx);
+        const float y0 = x[j][0] * (1.0f + g.x), y1 = x[j][1] * (1.0f + g.y);
+        const float scale = Q8 ? fixed_scale(warp_absmax(fmaxf(fabsf(y0), fabsf(y1)))) : 1.0f;
+        stage_pair<Q8>(c.sm.xq + (size_t)(4 * j) * RB, RB, 2 * c.tid, y0, y1, scale);
+        unscale[j] = 1.0f / scale;
     }
 #pragma unroll
-    for (int j = 0; j < T; j++) scale[j] = Q8 ? fixed_scale(mx[j]) : 1.0f;
-}
-// ... and the end of a staging phase: publish the inverse scales.  The caller's threads staged 4
-// consecutive inputs each, so a warp wrote exactly the k-slice it multiplies: no block barrier.
-template <int T>
-__device__ __forceinline__ void finish_stage(Ctx& c, const float (&scale)[T]) {
-    if (c.tid == 0) {
-#pragma unroll
-        for (int j = 0; j < T; j++) c.sm.xscale_s[j] = 1.0f / scale[j];
+    for (int j = 0; j < T; j++) {
+        const float ss = warp_sum(x[j][0] * x[j][0] + x[j][1] * x[j][1]);
+        if (c.lane == 0) c.sm.ssq_s[j * NCW + c.warp] = ss;
     }
+    MK_MARK(c, 7);
     __syncwarp();
 }
 
@@ -871,25 +853,27 @@ __device__ bool gdn_op(Ctx& c, const Params& P, const LayerP& L, int pos, uint32
         const float* qs_ = qkv_s + tk * QS;
         const float4 q4 = *reinterpret_cast<const float4*>(qs_ + 4 * c.lane);
         const float4 k4 = *reinterpret_cast<const float4*>(qs_ + S::LIN_DK + 4 * c.lane);
+        // One round of sums for the norms and all products with the state: with s the state before the token and k, q
+        // before their norms, the output s' q of the updated state s' = d s + delta k is d (s q) + delta (k q).
         const float qn = warp_sum(q4.x * q4.x + q4.y * q4.y + q4.z * q4.z + q4.w * q4.w);
         const float kn = warp_sum(k4.x * k4.x + k4.y * k4.y + k4.z * k4.z + k4.w * k4.w);
+        const float kq = warp_sum(fmaf(k4.w, q4.w, fmaf(k4.z, q4.z, fmaf(k4.y, q4.y, k4.x * q4.x))));
+        const float sk = warp_sum(fmaf(s3, k4.w, fmaf(s2, k4.z, fmaf(s1, k4.y, s0 * k4.x))));
+        const float sq = warp_sum(fmaf(s3, q4.w, fmaf(s2, q4.z, fmaf(s1, q4.y, s0 * q4.x))));
         // x / max(|x|, 1e-6), and the 1/sqrt(dk) query scale
         const float qs = 0.08838834764831845f / fmaxf(sqrtf(qn), 1e-6f);
         const float ks = 1.0f / fmaxf(sqrtf(kn), 1e-6f);
         const float vval = qs_[2 * S::LIN_DK + c.warp];
         const float beta = sigmoid_f(qs_[NCH]);
         const float decay = expf(-expf(a_log) * softplus_f(qs_[NCH + 1] + dt_bias));
-        const float kx = k4.x * ks, ky = k4.y * ks, kz = k4.z * ks, kw = k4.w * ks;
-        s0 *= decay; s1 *= decay; s2 *= decay; s3 *= decay;
-        const float recalled = warp_sum(fmaf(s3, kw, fmaf(s2, kz, fmaf(s1, ky, s0 * kx))));
-        const float delta = (vval - recalled) * beta;
-        s0 = fmaf(kx, delta, s0);
-        s1 = fmaf(ky, delta, s1);
-        s2 = fmaf(kz, delta, s2);
-        s3 = fmaf(kw, delta, s3);
+        const float delta = (vval - decay * ks * sk) * beta * ks;
+        const float o = fmaf(delta, kq, decay * sq) * qs;
+        s0 = fmaf(k4.x, delta, s0 * decay);
+        s1 = fmaf(k4.y, delta, s1 * decay);
+        s2 = fmaf(k4.z, delta, s2 * decay);
+        s3 = fmaf(k4.w, delta, s3 * decay);
         float* sout = (T == 2 && tk == 0) ? L.state_bak + soff : L.state + soff;
         *reinterpret_cast<float4*>(sout) = make_float4(s0, s1, s2, s3);
-        const float o = warp_sum(fmaf(s3, q4.w, fmaf(s2, q4.z, fmaf(s1, q4.y, s0 * q4.x)))) * qs;
         // The elementwise part of the gated norm (weight, silu(z)) is applied here; the head's 1 / rms
         // needs the squared outputs of the head's eight tasks and is applied by whoever sums the tasks'
         // partial out-projections: this task publishes its sum of squares beside them.
@@ -1333,7 +1317,7 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
     constexpr int WB = Q8 ? 1 : 2;                       // bytes per weight
     const uint32_t eB = eA + 1, eC = eA + 2, eD = eA + 3, eE = eA + 4;
     const bool attn = L.kind != 0;
-    float y[T][2];
+    float unscale[T];
     // ---- A: in-projection
     {
         prof_stamp(c, op0, 0);
@@ -1349,9 +1333,9 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
 #pragma unroll
             for (int j = 0; j < T; j++) { x[j][0] = v[2 * j]; x[j][1] = v[2 * j + 1]; }
         }
-        stage_rmsnorm<S, Q8, T>(c, x, nw, y);
+        stage_rmsnorm<S, Q8, T>(c, x, nw, unscale);
         prof_stamp(c, op0, 1);
-        gemv_mma<Q8, T, false>(c, r0, r1, S::HID * WB, L.s_in, [&](int, int row, int tk, float v, bool ok) {
+        gemv_mma<S, Q8, T, false>(c, r0, r1, S::HID * WB, L.s_in, unscale, true, [&](int, int row, int tk, float v, bool ok) {
             if (ok) ll_store(P.projl + (size_t)tk * S::PROJ_MAX + row, eA, v);
         });
         prof_stamp(c, op0, 3);
@@ -1452,19 +1436,18 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
                 }
             }
         }
-        float mx[T], scale[T];
-#pragma unroll
-        for (int j = 0; j < T; j++) mx[j] = fmaxf(fmaxf(fabsf(m[j][0]), fabsf(m[j][1])), fmaxf(fabsf(m[j][2]), fabsf(m[j][3])));
-        block_scale<Q8, T>(c, mx, scale);
+        // the warp's 128 inputs are the k-slice it multiplies: a scale of its own, no block barrier
 #pragma unroll
         for (int j = 0; j < T; j++) {
+            const float scale = Q8 ? fixed_scale(warp_absmax(fmaxf(fmaxf(fabsf(m[j][0]), fabsf(m[j][1])), fmaxf(fabsf(m[j][2]), fabsf(m[j][3]))))) : 1.0f;
             uint8_t* xq = c.sm.xq + (size_t)(4 * j) * (S::MIX * WB);
-            stage_pair<Q8>(xq, S::MIX * WB, k, m[j][0], m[j][1], scale[j]);
-            stage_pair<Q8>(xq, S::MIX * WB, k + 2, m[j][2], m[j][3], scale[j]);
+            stage_pair<Q8>(xq, S::MIX * WB, k, m[j][0], m[j][1], scale);
+            stage_pair<Q8>(xq, S::MIX * WB, k + 2, m[j][2], m[j][3], scale);
+            unscale[j] = 1.0f / scale;
         }
-        finish_stage<T>(c, scale);
+        __syncwarp();
         prof_stamp(c, op, 1);
-        gemv_mma<Q8, T, false>(c, xr0, xr1, S::MIX * WB, L.s_out, [&](int, int row, int tk, float v, bool ok) {
+        gemv_mma<S, Q8, T, false>(c, xr0, xr1, S::MIX * WB, L.s_out, unscale, false, [&](int, int row, int tk, float v, bool ok) {
             if (ok) {
                 const float xn = c.sm.xown[tk * 16 + row - xr0] + v;
                 c.sm.xown[tk * 16 + row - xr0] = xn;
@@ -1488,9 +1471,9 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
 #pragma unroll
             for (int j = 0; j < T; j++) { x[j][0] = v[2 * j]; x[j][1] = v[2 * j + 1]; }
         }
-        stage_rmsnorm<S, Q8, T>(c, x, nw, y);
+        stage_rmsnorm<S, Q8, T>(c, x, nw, unscale);
         prof_stamp(c, op, 1);
-        gemv_mma<Q8, T, false>(c, r0, r1, S::HID * WB, L.s_gu, [&](int lane, int row, int tk, float v, bool ok) {
+        gemv_mma<S, Q8, T, false>(c, r0, r1, S::HID * WB, L.s_gu, unscale, true, [&](int lane, int row, int tk, float v, bool ok) {
             // rows alternate gate, up; chunks hold whole pairs, so the partner is the next lane.  The
             // SwiGLU outputs stay in this CTA: it multiplies them with its column slice of the
             // down-projection itself.
@@ -1576,7 +1559,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
         c.sm.best_s = reinterpret_cast<u64*>(p); p += NCW * 8;                     // 128
         c.sm.full = reinterpret_cast<uint64_t*>(p); p += 6 * 8;
         c.sm.empty = reinterpret_cast<uint64_t*>(p); p += 6 * 8;
-        c.sm.xscale_s = reinterpret_cast<float*>(p); p += 8;
+        c.sm.ssq_s = reinterpret_cast<float*>(p); p += SPEC_T * NCW * 4;            // 128
         c.sm.abort_flag = reinterpret_cast<volatile int*>(p); p += 4;
         c.sm.quit_flag = reinterpret_cast<volatile int*>(p); p += 4;
         c.sm.act_s = reinterpret_cast<float*>(p); p += SPEC_T * DOWN_K * 4;
@@ -1595,7 +1578,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
         }
         *c.sm.abort_flag = 0;
         *c.sm.quit_flag = 0;
-        c.sm.xscale_s[0] = c.sm.xscale_s[1] = 1.0f;
         fence_barrier_init();
         fence_proxy_async();
     }
@@ -1661,11 +1643,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
 #pragma unroll
             for (int j = 0; j < T; j++) { x[j][0] = v[2 * j]; x[j][1] = v[2 * j + 1]; }
         }
-        stage_rmsnorm<S, Q8, T>(c, x, nw, hn);
+        float unscale[T];
+        stage_rmsnorm<S, Q8, T>(c, x, nw, unscale);
         prof_stamp(c, op, 1);
         u64 best = 0;                                    // warp j tracks token j
         const float invT = A.inv_temperature;
-        gemv_mma<Q8, T, true>(c, lr0, lr1, S::HID * WB, P.lm_scale, [&](int, int row, int tk, float v, bool ok) {
+        gemv_mma<S, Q8, T, true>(c, lr0, lr1, S::HID * WB, P.lm_scale, unscale, true, [&](int, int row, int tk, float v, bool ok) {
             if (!ok) return;
             if (logits) logits[(size_t)tk * P.vocab + row] = v;
             float score = v;
@@ -1677,6 +1660,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
             const u64 key = score_key(score, row);
             best = key > best ? key : best;
         });
+        if (T > 1) {                                     // the draft head's input
+#pragma unroll
+            for (int j = 0; j < T; j++) {
+                const float inv = rsqrtf(sum_warps(c.sm.ssq_s + j * NCW) * (1.0f / S::HID) + S::EPS);
+                hn[j][0] = x[j][0] * (1.0f + nw.x) * inv;
+                hn[j][1] = x[j][1] * (1.0f + nw.y) * inv;
+            }
+        }
         if (c.warp < T) {
             best = warp_max_u64(best);
             if (c.lane == 0) {
@@ -1813,6 +1804,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
                 }
                 consumer_sum_max<2 * T>(c, ss, mx);
                 constexpr int RB = 2 * S::HID * WB;
+                float unscale[T];
 #pragma unroll
                 for (int j = 0; j < T; j++) {
                     const float inv_e = rsqrtf(ss[2 * j] * (1.0f / S::HID) + S::EPS);
@@ -1821,11 +1813,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
                     uint8_t* xq = c.sm.xq + (size_t)(4 * j) * RB;
                     stage_pair<Q8>(xq, RB, 2 * c.tid, ye[j][0] * inv_e, ye[j][1] * inv_e, scale);
                     stage_pair<Q8>(xq, RB, S::HID + 2 * c.tid, yh[j][0] * inv_h, yh[j][1] * inv_h, scale);
-                    if (c.tid == 0) c.sm.xscale_s[j] = 1.0f / scale;
+                    unscale[j] = 1.0f / scale;
                 }
                 consumer_sync();
                 prof_stamp(c, op, 1);
-                gemv_mma<Q8, T, false>(c, xr0, xr1, RB, P.mtp_fc_scale, [&](int, int row, int tk, float v, bool ok) {
+                gemv_mma<S, Q8, T, false>(c, xr0, xr1, RB, P.mtp_fc_scale, unscale, false, [&](int, int row, int tk, float v, bool ok) {
                     if (ok) {
                         c.sm.xown[tk * 16 + row - xr0] = v;
                         ll_store(P.xml + (size_t)tk * S::HID + row, eF, v);
@@ -1845,7 +1837,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
                 cta_rows(P.draft_vocab, 1, c.cta, c.grid, dr0, dr1);
                 scale_prefetch(c, P.draft_scale, dr0, dr1, true);
                 const float2 nw = *reinterpret_cast<const float2*>(P.mtp_norm + 2 * c.tid);
-                float u[T][2], un[T][2];
+                float u[T][2], unscale[T];
                 {
                     const u64* ptrs[T];
                     uint32_t eps[T];
@@ -1856,11 +1848,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
 #pragma unroll
                     for (int j = 0; j < T; j++) { u[j][0] = v[2 * j]; u[j][1] = v[2 * j + 1]; }
                 }
-                stage_rmsnorm<S, Q8, T>(c, u, nw, un);
+                stage_rmsnorm<S, Q8, T>(c, u, nw, unscale);
                 prof_stamp(c, op, 1);
                 u64 best = 0;
                 const int want = n_new - 1;              // token slot whose draft counts
-                gemv_mma<Q8, T, true>(c, dr0, dr1, S::HID * WB, P.draft_scale, [&](int, int row, int tk, float v, bool ok) {
+                gemv_mma<S, Q8, T, true>(c, dr0, dr1, S::HID * WB, P.draft_scale, unscale, true, [&](int, int row, int tk, float v, bool ok) {
                     if (!ok || tk != want) return;
                     const u64 key = score_key(v, row);
                     best = key > best ? key : best;
