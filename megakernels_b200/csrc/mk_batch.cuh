@@ -28,16 +28,6 @@
 namespace mk {
 
 constexpr int NB = 8;                       // sequences per pass = columns of one MMA
-// Cached K rows a warp, and cached V elements a thread, requests together in batched attention.  More
-// loads in flight (2 or 4 rows, 16 elements) measured 3 to 14 % slower per step: at 96 registers per
-// thread they turn into spills, and spills are served by L2 because shared memory leaves the L1
-// almost nothing.
-#ifndef MK_B_KU
-#define MK_B_KU 1
-#endif
-#ifndef MK_B_VU
-#define MK_B_VU 8
-#endif
 
 struct BatchArgs {
     const int* forced;                      // [steps][NB] prompt tokens, step-major
@@ -415,6 +405,25 @@ __device__ void producer_batch(Ctx& c, const Params& P, const BatchArgs& A) {
     pr.drain();
 }
 
+// Asks the L2 for the cached rows this CTA's attention task is going to scan, an op ahead: a task of a shared grid has more rows
+// than its threads' registers hold, and from HBM every round of them would cost its latency.  A page holds a KV head's
+// positions one after the other, so a task's share of a page is one request.
+template <class S, bool KVF32>
+__device__ void request_kv(const Ctx& c, const Params& P, const LayerP& L, const BatchArgs& A, int step) {
+    const int per = c.grid / A.nb, q = c.cta / per;
+    if (q >= A.nb) return;
+    const int cta = c.cta - q * per, pos = A.pos0[q] + step, n = pos + 1;
+    const int ch = attn_chunk(n, min(per / S::NKV, MAX_SPLITS)), g = cta % S::NKV, p0 = cta / S::NKV * ch, p1 = min(pos, p0 + ch);
+    constexpr uint32_t ROW = S::HD * (KVF32 ? 4 : 2);
+    const int* bt = c.sm.bt_s + q * (P.max_seq / KV_BLOCK);
+    for (int p = p0; p < p1; p = (p / KV_BLOCK + 1) * KV_BLOCK) {
+        const size_t off = (((size_t)bt[p / KV_BLOCK] * S::NKV + g) * KV_BLOCK + p % KV_BLOCK) * ROW;
+        const uint32_t bytes = (uint32_t)(min(p1, (p / KV_BLOCK + 1) * KV_BLOCK) - p) * ROW;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)L.k_cache + off), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)L.v_cache + off), "r"(bytes) : "memory");
+    }
+}
+
 // One decoder layer for every live sequence (ops A..E as in `run_layer`).  `x` holds this thread's
 // residual elements when `x_in_regs` (first layer), otherwise they are awaited at epoch eA - 1.
 template <class S, bool KVF32>
@@ -430,6 +439,7 @@ __device__ __forceinline__ bool run_layer_b(Ctx& c, const Params& P, const Layer
         cta_rows(attn ? S::ATT_IN : S::GDN_IN, 1, c.cta, c.grid, r0, r1);
         scale_prefetch(c, L.s_in, r0, r1, false);
         const float2 nw = *reinterpret_cast<const float2*>(L.in_norm + 2 * c.tid);
+        if (attn && c.tid == 0) request_kv<S, KVF32>(c, P, L, A, step);
         if (!x_in_regs) wait_residual_b<S>(c, P.xl, eA - 1, nb, x);
         stage_rms_b<S>(c, x, nw);
         prof_stamp(c, op0, 1);
@@ -448,7 +458,7 @@ __device__ __forceinline__ bool run_layer_b(Ctx& c, const Params& P, const Layer
             const AttnView view = {c.cta - q * per, per, P.projl + (size_t)q * S::PROJ_MAX, P.mixl + (size_t)q * S::MIX,
                                    P.attn_part + (size_t)q * S::NKV * MAX_SPLITS * S::PART_STRIDE,
                                    c.sm.bt_s + q * (P.max_seq / KV_BLOCK), true};
-            had_task = attn_op<S, KVF32, 1, MK_B_KU, MK_B_VU>(c, P, L, view, A.pos0[q] + step, eA, eB, op0 + 1);
+            had_task = attn_op<S, KVF32, 1>(c, P, L, view, A.pos0[q] + step, eA, eB, op0 + 1);
         }
     } else {
         had_task = gdn_batch<S>(c, P, L, A, step, frozen, eA, eB, op0 + 1);

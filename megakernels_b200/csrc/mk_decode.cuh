@@ -959,15 +959,16 @@ struct AttnView {
     bool gate;              // publish o * sigmoid(gate) instead of o (otherwise the out-projection's prologue applies the gate)
 };
 
-// KU cached K rows per warp and VU cached V elements per thread are requested together before they are
-// used: 1 and 8 suit the short chunks of a sequence that has the whole grid; tasks that scan 64 or more
-// positions (several sequences sharing the grid) want more loads in flight.
-template <class S, bool KVF32, int T, int KU = 1, int VU = 8>
+// Scores: a warp takes every 16th position and requests its next K row before it scores the present one.  Values: two threads
+// share a dim, one takes the even, one the odd positions of the task for all four heads (a V element is loaded once), and
+// they exchange halves at the end, after which thread (d, hp) holds heads 2 hp and 2 hp + 1.  (A step at 4000 positions 522 -> 509 us; of
+// eight sequences at 640, with request_kv, 906 -> 869.)
+template <class S, bool KVF32, int T>
 __device__ bool attn_op(Ctx& c, const Params& P, const LayerP& L, const AttnView& V, int pos, uint32_t e_proj,
                         uint32_t e_out, int op) {
     static_assert(S::HD == 256 && S::QPK == 4 && NCW == 16 && S::ROT == 64, "thread mapping below");
     constexpr int NOUT = S::QPK * S::HD;        // outputs per KV head and token
-    constexpr int PFV = 16;                     // V rows requested early per thread
+    constexpr int PFV = 8, VU = 8;              // V elements a thread requests before the wait, and together later on
     const int n = pos + T;
     const int max_splits = min(V.grid / S::NKV, MAX_SPLITS);
     const int ch = attn_chunk(n, max_splits);
@@ -1005,7 +1006,7 @@ __device__ bool attn_op(Ctx& c, const Params& P, const LayerP& L, const AttnView
     }
 #pragma unroll
     for (int i = 0; i < PFV; i++) {
-        const int p = p0 + i;
+        const int p = p0 + 2 * i + hp;
         vpre[i] = (p < p1 && p < pos) ? load1<KVF32>(L.v_cache, kv_elem(p) + d) : 0.f;
     }
 
@@ -1109,35 +1110,35 @@ __device__ bool attn_op(Ctx& c, const Params& P, const LayerP& L, const AttnView
                     float a = x.x * kk[0];
                     a = fmaf(x.y, kk[1], a); a = fmaf(x.z, kk[2], a); a = fmaf(x.w, kk[3], a);
                     a = fmaf(y.x, kk[4], a); a = fmaf(y.y, kk[5], a); a = fmaf(y.z, kk[6], a); a = fmaf(y.w, kk[7], a);
-                    dsum[hh] = warp_sum(a);
+                    dsum[hh] = a;
                 }
-                if (c.lane == 0) {
-                    const bool seen = p <= pos + tk;
+                // the four heads' sums in six shuffles: lane l ends up with head 2 (l & 1) + ((l >> 1) & 1)
+                const bool b0 = c.lane & 1, b1 = c.lane & 2;
+                const float e0 = (b0 ? dsum[2] : dsum[0]) + __shfl_xor_sync(0xffffffffu, b0 ? dsum[0] : dsum[2], 1);
+                const float e1 = (b0 ? dsum[3] : dsum[1]) + __shfl_xor_sync(0xffffffffu, b0 ? dsum[1] : dsum[3], 1);
+                float r = (b1 ? e1 : e0) + __shfl_xor_sync(0xffffffffu, b1 ? e0 : e1, 2);
 #pragma unroll
-                    for (int hh = 0; hh < S::QPK; hh++)
-                        sc_s[(tk * S::QPK + hh) * ch + (p - p0)] = seen ? dsum[hh] : -INFINITY;
-                }
+                for (int x = 4; x <= 16; x *= 2) r += __shfl_xor_sync(0xffffffffu, r, x);
+                if (c.lane < S::QPK)
+                    sc_s[(tk * S::QPK + 2 * (c.lane & 1) + (c.lane >> 1)) * ch + (p - p0)] = p <= pos + tk ? r : -INFINITY;
             }
         };
-        for (int pb = p0 + c.warp; pb < p1; pb += KU * NCW) {
-            float kk[KU][8];
+        float kk[8];
 #pragma unroll
-            for (int u = 0; u < KU; u++) {
-                const int p = pb + u * NCW;
-                if (p >= p1) continue;
-                if (p >= pos) {
+        for (int i = 0; i < 8; i++) kk[i] = kpre[i];
+#pragma unroll 1
+        for (int p = p0 + c.warp; p < p1; p += NCW) {
+            float next[8];
 #pragma unroll
-                    for (int i = 0; i < 8; i++) kk[u][i] = knew_s[(p - pos) * S::HD + 8 * c.lane + i];
-                } else if (p == p0 + c.warp) {
+            for (int i = 0; i < 8; i++) next[i] = 0.f;
+            if (p + NCW < min(p1, pos)) load8<KVF32>(L.k_cache, kv_elem(p + NCW) + 8 * c.lane, next);
+            if (p >= pos) {
 #pragma unroll
-                    for (int i = 0; i < 8; i++) kk[u][i] = kpre[i];
-                } else {
-                    load8<KVF32>(L.k_cache, kv_elem(p) + 8 * c.lane, kk[u]);
-                }
+                for (int i = 0; i < 8; i++) kk[i] = knew_s[(p - pos) * S::HD + 8 * c.lane + i];
             }
+            score(p, kk);
 #pragma unroll
-            for (int u = 0; u < KU; u++)
-                if (pb + u * NCW < p1) score(pb + u * NCW, kk[u]);
+            for (int i = 0; i < 8; i++) kk[i] = next[i];
         }
     }
     consumer_sync();
@@ -1160,40 +1161,49 @@ __device__ bool attn_op(Ctx& c, const Params& P, const LayerP& L, const AttnView
         }
     }
     consumer_sync();
-    // -- 5. weighted values: thread -> dim d, heads 2*hp and 2*hp+1, every token
+    // -- 5. weighted values: thread -> dim d, positions p0 + hp, p0 + hp + 2, ..., every head and token
     float acc[T][2];
-#pragma unroll
-    for (int tk = 0; tk < T; tk++) acc[tk][0] = acc[tk][1] = 0.f;
     {
+        float part[T][S::QPK];
+#pragma unroll
+        for (int tk = 0; tk < T; tk++)
+#pragma unroll
+            for (int hh = 0; hh < S::QPK; hh++) part[tk][hh] = 0.f;
         auto accumulate = [&](int i, float v) {
 #pragma unroll
-            for (int tk = 0; tk < T; tk++) {
-                acc[tk][0] = fmaf(sc_s[(tk * S::QPK + 2 * hp) * ch + i], v, acc[tk][0]);
-                acc[tk][1] = fmaf(sc_s[(tk * S::QPK + 2 * hp + 1) * ch + i], v, acc[tk][1]);
-            }
+            for (int tk = 0; tk < T; tk++)
+#pragma unroll
+                for (int hh = 0; hh < S::QPK; hh++) part[tk][hh] = fmaf(sc_s[(tk * S::QPK + hh) * ch + i], v, part[tk][hh]);
         };
 #pragma unroll
-        for (int i = 0; i < PFV; i++) {
-            if (i < np) {
-                const int p = p0 + i;
-                accumulate(i, p >= pos ? vnew_s[(p - pos) * S::HD + d] : vpre[i]);
-            }
+        for (int u = 0; u < PFV; u++) {
+            const int i = 2 * u + hp, p = p0 + i;
+            if (i < np) accumulate(i, p >= pos ? vnew_s[(p - pos) * S::HD + d] : vpre[u]);
         }
-        int i = PFV;
-        for (; i + VU <= np; i += VU) {
+#pragma unroll 1
+        for (int i0 = 2 * PFV + hp; i0 < np; i0 += 2 * VU) {
             float v[VU];
 #pragma unroll
             for (int u = 0; u < VU; u++) {
-                const int p = p0 + i + u;
-                v[u] = p >= pos ? vnew_s[(p - pos) * S::HD + d] : load1<KVF32>(L.v_cache, kv_elem(p) + d);
+                const int i = i0 + 2 * u, p = p0 + i;
+                v[u] = 0.f;
+                if (i < np) v[u] = p >= pos ? vnew_s[(p - pos) * S::HD + d] : load1<KVF32>(L.v_cache, kv_elem(p) + d);
             }
 #pragma unroll
-            for (int u = 0; u < VU; u++) accumulate(i + u, v[u]);
+            for (int u = 0; u < VU; u++)
+                if (i0 + 2 * u < np) accumulate(i0 + 2 * u, v[u]);
         }
-        for (; i < np; i++) {
-            const int p = p0 + i;
-            accumulate(i, p >= pos ? vnew_s[(p - pos) * S::HD + d] : load1<KVF32>(L.v_cache, kv_elem(p) + d));
-        }
+        // (every score is read: the queries' scratch is free since the barrier before the statistics)
+        float* swap = q_s;                          // [token][head][dim]: what the other thread of the dim keeps
+#pragma unroll
+        for (int tk = 0; tk < T; tk++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) swap[(tk * S::QPK + 2 * (hp ^ 1) + k) * S::HD + d] = hp ? part[tk][k] : part[tk][2 + k];
+        consumer_sync();
+#pragma unroll
+        for (int tk = 0; tk < T; tk++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) acc[tk][k] = (hp ? part[tk][2 + k] : part[tk][k]) + swap[(tk * S::QPK + 2 * hp + k) * S::HD + d];
     }
     prof_stamp(c, op, 2);
     if (nsplit == 1) {
