@@ -1316,6 +1316,18 @@ __device__ bool attn_op(Ctx& c, const Params& P, const LayerP& L, const AttnView
     return true;
 }
 
+// Calls f(token, row, row is owned, row + 1 is owned) for every pair of rows (row even) with a row in [r0, r1), a warp per pair
+// and token.  The partial sums of a row are one word from every CTA, each in a sector of its own, and the requests for them are
+// what the L2 is busy with: reading the words of two rows at once halves them (a step 469 -> 451 us).  Two tokens go to different warps.
+template <int T, class F>
+__device__ __forceinline__ void own_rows(const Ctx& c, int r0, int r1, F&& f) {
+    const int first = r0 >> 1, pairs = ((r1 + 1) >> 1) - first, span = T > 1 && pairs <= NCW / 2 ? NCW / 2 : NCW;
+    const int row = 2 * (first + c.warp % span);
+    if (c.warp % span < pairs)
+#pragma unroll 1
+        for (int j = c.warp / span; j < T; j += NCW / span) f(j, row, row >= r0, row + 1 < r1);
+}
+
 // ---- one decoder layer -----------------------------------------------------------------------------------
 // Runs ops A..E of layer `L` for T tokens at positions pos .. pos + T - 1 on the residual stream `xbuf`
 // (words [T][HID]).  `x` holds this thread's residual elements when `x_in_regs` (first layer: they come
@@ -1358,56 +1370,55 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
     prof_stamp(c, op0 + 1, 3);
     // ---- C: out-projection + residual
     if (!attn) {
-        // DeltaNet: the tasks have already multiplied their outputs with their column slices.  Warp r
-        // sums the 128 partial sums of owned row r, each weighted with its head's 1 / rms: lane l takes
+        // DeltaNet: the tasks have already multiplied their outputs with their column slices.  A warp
+        // sums the 128 partial sums of two owned rows, each weighted with its head's 1 / rms: lane l takes
         // tasks l, l + 32, l + 64, l + 96, whose heads' eight tasks are eight consecutive lanes.
         const int op = op0 + 2;
         prof_stamp(c, op, 0);
         static_assert(S::GDN_TASKS == 128 && S::LIN_DV / S::GDN_SLICE == 8, "four tasks per lane, eight per head");
-        if (c.warp < xr1 - xr0) {
-            const int row = xr0 + c.warp;
-            const float rs = Q8 ? L.s_out[row] : 1.0f;           // requested before the wait
+        own_rows<T>(c, xr0, xr1, [&](int j, int row, bool a_own, bool b_own) {
+            const float rs0 = Q8 && a_own ? L.s_out[row] : 1.0f, rs1 = Q8 && b_own ? L.s_out[row + 1] : 1.0f;   // requested before the wait
+            const u64* psrc = P.partl + (size_t)j * c.grid * S::HID + row + (size_t)c.lane * S::HID;
+            const u64* ssrc = P.mixl + (size_t)j * S::MIX + c.lane;
+            u64 w[4][2], sw[4];
 #pragma unroll
-            for (int j = 0; j < T; j++) {
-                const u64* psrc = P.partl + (size_t)j * c.grid * S::HID + row;
-                const u64* ssrc = P.mixl + (size_t)j * S::MIX;
-                u64 w[4], sw[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    w[i] = ll_load(psrc + (size_t)(c.lane + 32 * i) * S::HID);
-                    sw[i] = ll_load(ssrc + c.lane + 32 * i);
-                }
-                Spin sp;
-                while (true) {
-                    bool ok = true;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        if ((uint32_t)(w[i] >> 32) != eB) { ok = false; w[i] = ll_load(psrc + (size_t)(c.lane + 32 * i) * S::HID); }
-                        if ((uint32_t)(sw[i] >> 32) != eB) { ok = false; sw[i] = ll_load(ssrc + c.lane + 32 * i); }
-                    }
-                    if (ok) break;
-                    if (MK_SPIN_FAIL(c, sp, W_MIX)) {
-                        c.dead = true;
-                        break;
-                    }
-                }
-                float acc = 0.f;
+            for (int i = 0; i < 4; i++) {
+                ll_load2(psrc + (size_t)32 * i * S::HID, w[i][0], w[i][1]);
+                sw[i] = ll_load(ssrc + 32 * i);
+            }
+            Spin sp;
+            while (true) {
+                bool ok = true;
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    float hs = __uint_as_float((uint32_t)sw[i]);      // sum of squares over the head: 8 lanes
-                    hs += __shfl_xor_sync(0xffffffffu, hs, 1);
-                    hs += __shfl_xor_sync(0xffffffffu, hs, 2);
-                    hs += __shfl_xor_sync(0xffffffffu, hs, 4);
-                    acc += __uint_as_float((uint32_t)w[i]) * rsqrtf(hs * (1.0f / S::LIN_DV) + S::EPS);
+                    if ((uint32_t)(w[i][0] >> 32) != eB || (uint32_t)(w[i][1] >> 32) != eB) { ok = false; ll_load2(psrc + (size_t)32 * i * S::HID, w[i][0], w[i][1]); }
+                    if ((uint32_t)(sw[i] >> 32) != eB) { ok = false; sw[i] = ll_load(ssrc + 32 * i); }
                 }
-                const float tot = warp_sum(acc);
-                if (c.lane == 0) {
-                    const float xn = c.sm.xown[j * 16 + c.warp] + tot * rs;
-                    c.sm.xown[j * 16 + c.warp] = xn;
-                    ll_store(xbuf + (size_t)j * S::HID + row, eC, xn);
+                if (ok) break;
+                if (MK_SPIN_FAIL(c, sp, W_MIX)) {
+                    c.dead = true;
+                    break;
                 }
             }
-        }
+            float acc0 = 0.f, acc1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                float hs = __uint_as_float((uint32_t)sw[i]);      // sum of squares over the head: 8 lanes
+                hs += __shfl_xor_sync(0xffffffffu, hs, 1);
+                hs += __shfl_xor_sync(0xffffffffu, hs, 2);
+                hs += __shfl_xor_sync(0xffffffffu, hs, 4);
+                const float inv = rsqrtf(hs * (1.0f / S::LIN_DV) + S::EPS);
+                acc0 += __uint_as_float((uint32_t)w[i][0]) * inv;
+                acc1 += __uint_as_float((uint32_t)w[i][1]) * inv;
+            }
+            const float t0 = warp_sum(acc0) * rs0, t1 = warp_sum(acc1) * rs1;
+            if (c.lane < 2 && (c.lane ? b_own : a_own)) {
+                float* own = c.sm.xown + j * 16 + row + c.lane - xr0;
+                const float xn = *own + (c.lane ? t1 : t0);
+                *own = xn;
+                ll_store(xbuf + (size_t)j * S::HID + row + c.lane, eC, xn);
+            }
+        });
         prof_stamp(c, op, 3);
         consumer_sync();   // keep the other warps' polls for the next op behind these stores
     } else {
@@ -1499,51 +1510,51 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
     {
         const int op = op0 + 4;
         prof_stamp(c, op, 0);
-        if (c.warp < xr1 - xr0) {
-            const int row = xr0 + c.warp;
-            const float rs = Q8 ? L.s_down[row] : 1.0f;         // requested before the wait
+        own_rows<T>(c, xr0, xr1, [&](int j, int row, bool a_own, bool b_own) {
+            const float rs0 = Q8 && a_own ? L.s_down[row] : 1.0f, rs1 = Q8 && b_own ? L.s_down[row + 1] : 1.0f;   // requested before the wait
+            // lane l takes CTAs l, l + 32, ...; fixed order, then the shuffle tree
+            constexpr int PER = 5;                          // grids of up to 160 CTAs
+            const u64* src = P.partl + (size_t)j * c.grid * S::HID + row + (size_t)c.lane * S::HID;
+            u64 w[PER][2];
 #pragma unroll
-            for (int j = 0; j < T; j++) {
-                // lane l takes CTAs l, l + 32, ...; fixed order, then the shuffle tree
-                constexpr int PER = 5;                          // grids of up to 160 CTAs
-                const u64* src = P.partl + (size_t)j * c.grid * S::HID + row;
-                u64 w[PER];
-#pragma unroll
-                for (int i = 0; i < PER; i++) {
-                    const int cta = c.lane + 32 * i;
-                    w[i] = cta < c.grid ? ll_load(src + (size_t)cta * S::HID) : 0;
-                }
-                Spin sp;
-                while (true) {
-                    bool ok = true;
-#pragma unroll
-                    for (int i = 0; i < PER; i++) {
-                        const int cta = c.lane + 32 * i;
-                        if (cta < c.grid && (uint32_t)(w[i] >> 32) != eD) {
-                            ok = false;
-                            w[i] = ll_load(src + (size_t)cta * S::HID);
-                        }
-                    }
-                    if (ok) break;
-                    if (MK_SPIN_FAIL(c, sp, W_ACT)) {
-                        c.dead = true;
-                        break;
-                    }
-                }
-                float acc = 0.f;
+            for (int i = 0; i < PER; i++) {
+                w[i][0] = w[i][1] = 0;
+                if (c.lane + 32 * i < c.grid) ll_load2(src + (size_t)32 * i * S::HID, w[i][0], w[i][1]);
+            }
+            Spin sp;
+            while (true) {
+                bool ok = true;
 #pragma unroll
                 for (int i = 0; i < PER; i++)
-                    if (c.lane + 32 * i < c.grid) acc += __uint_as_float((uint32_t)w[i]);
-                const float tot = warp_sum(acc);
-                if (c.lane == 0) {
-                    const float xn = c.sm.xown[j * 16 + c.warp] + tot * rs;
-                    c.sm.xown[j * 16 + c.warp] = xn;
-                    ll_store(xbuf + (size_t)j * S::HID + row, eE, xn);
-                    if (resid_out) resid_out[(size_t)j * S::HID + row] = xn;
+                    if (c.lane + 32 * i < c.grid && ((uint32_t)(w[i][0] >> 32) != eD || (uint32_t)(w[i][1] >> 32) != eD)) {
+                        ok = false;
+                        ll_load2(src + (size_t)32 * i * S::HID, w[i][0], w[i][1]);
+                    }
+                if (ok) break;
+                if (MK_SPIN_FAIL(c, sp, W_ACT)) {
+                    c.dead = true;
+                    break;
                 }
             }
-        }
-        prof_stamp(c, op, 3);
+            float acc0 = 0.f, acc1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < PER; i++)
+                if (c.lane + 32 * i < c.grid) {
+                    acc0 += __uint_as_float((uint32_t)w[i][0]);
+                    acc1 += __uint_as_float((uint32_t)w[i][1]);
+                }
+            const float t0 = warp_sum(acc0) * rs0, t1 = warp_sum(acc1) * rs1;
+            if (c.lane < 2 && (c.lane ? b_own : a_own)) {
+                float* own = c.sm.xown + j * 16 + row + c.lane - xr0;
+                const float xn = *own + (c.lane ? t1 : t0);
+                *own = xn;
+                ll_store(xbuf + (size_t)j * S::HID + row + c.lane, eE, xn);
+                if (resid_out) resid_out[(size_t)j * S::HID + row + c.lane] = xn;
+            }
+        });
+    }
+    {
+        prof_stamp(c, op0 + 4, 3);
         failed = consumer_any(c.dead);
     }
     return failed;
