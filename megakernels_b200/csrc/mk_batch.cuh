@@ -398,11 +398,76 @@ __device__ void producer_batch(Ctx& c, const Params& P, const BatchArgs& A) {
             pr.stream(L.w_in, L.kind ? S::ATT_IN : S::GDN_IN, 1, S::HID);
             pr.stream(L.kind ? L.w_out : L.w_out_rows, S::HID, 1, S::MIX);
             pr.stream(L.w_gu, 2 * S::INTER, 2, S::HID);
-            pr.stream(L.w_down_rows, S::HID, 1, S::INTER);
+            pr.stream(L.w_down, (S::HID / 16) * c.grid, S::HID / 16, 16 * DOWN_K);   // this CTA's column slice: 64 tiles
         }
         if (s >= A.lm_from) pr.stream(P.lm_head, P.vocab, 1, S::HID);
     }
     pr.drain();
+}
+
+// Partial down-projections are handed over as words [cta][row][sequences, an even number].  They share the attention partials'
+// buffer, which is as large from two sequences on: either op writes only after every CTA has read what the other left there
+// (between them lie the exchanges of the residual that all CTAs take part in).
+__device__ __forceinline__ u64* down_words(const Params& P, int nb) { return nb > 1 ? P.attn_part : P.partl; }
+
+// The batched partial_cols: `act` ([NB][DOWN_K] in shared memory, zero past the CTA's slice) times the CTA's column slice of the
+// down-projection: 1024 partial sums per sequence.  Handing activations over instead would have every CTA read all 3584 of
+// every sequence (34 MB of words per layer at eight sequences, which is what the L2 was busy with); the sums of the rows a CTA owns
+// are 10 MB over all CTAs (a step at 640 positions 869 -> 789 us).  Inputs are signed 24-bit integers with a scale per sequence, cut into bytes as everywhere here.
+template <class S>
+__device__ __forceinline__ void partial_cols_b(Ctx& c, const float* act, u64* out, int nbp, uint32_t epoch) {
+    constexpr int TILES = S::HID / 16;
+    static_assert(TILES * 16 * DOWN_K == SLOT_BYTES && TILES % NCW == 0, "one ring chunk, whole rounds of 16 tiles");
+    const int g = c.lane >> 2, t = c.lane & 3;
+    uint32_t b[3][2];                               // B fragments of sequence g: digit, low or high 16 columns
+    float inv;
+    {
+        const float4 lo = *reinterpret_cast<const float4*>(act + g * DOWN_K + 4 * t), hi = *reinterpret_cast<const float4*>(act + g * DOWN_K + 16 + 4 * t);
+        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        float mx = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; i++) mx = fmaxf(mx, fabsf(v[i]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float scale = fixed_scale24(mx);
+        inv = 1.0f / scale;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            uint32_t q[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) q[i] = (uint32_t)__float2int_rn(v[4 * h + i] * scale);
+#pragma unroll
+            for (int d = 0; d < 3; d++) b[d][h] = __byte_perm(__byte_perm(q[0], q[1], 0x0040 + d * 0x0011), __byte_perm(q[2], q[3], 0x0040 + d * 0x0011), 0x5410);
+        }
+    }
+    const float is0 = __shfl_sync(0xffffffffu, inv, 8 * t), is1 = __shfl_sync(0xffffffffu, inv, 8 * t + 4);    // of sequences 2 t, 2 t + 1
+    const uint32_t n = c.cons_n++;
+    const int slot = (int)(n % GeoB::NS);
+    mbar_wait(c, &c.sm.full[slot], (n / GeoB::NS) & 1, W_FULL);
+    const uint8_t* buf = c.sm.ring + (size_t)slot * SLOT_BYTES;
+#pragma unroll
+    for (int i = 0; i < TILES / NCW; i++) {
+        const int tile = c.warp + NCW * i;
+        const uint4 w = *reinterpret_cast<const uint4*>(buf + (size_t)tile * 16 * DOWN_K + c.lane * 16);
+        int ci[3][4];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) ci[d][k] = 0;
+        mma_s8u8(ci[0], w.x, w.y, w.z, w.w, b[0][0], b[0][1]);
+        mma_s8u8(ci[1], w.x, w.y, w.z, w.w, b[1][0], b[1][1]);
+        mma_s8(ci[2], w.x, w.y, w.z, w.w, b[2][0], b[2][1]);
+        float v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = fmaf((float)ci[2][k], 65536.f, fmaf((float)ci[1][k], 256.f, (float)ci[0][k])) * ((k & 1) ? is1 : is0);
+        if (2 * t < nbp) {
+            u64* dst = out + (size_t)(tile * 16 + g) * nbp + 2 * t;
+            ll_store2(dst, epoch, v[0], v[1]);
+            ll_store2(dst + (size_t)8 * nbp, epoch, v[2], v[3]);
+        }
+    }
+    __syncwarp();
+    if (c.lane == 0 && !c.dead) mbar_arrive(&c.sm.empty[slot]);
 }
 
 // Asks the L2 for the cached rows this CTA's attention task is going to scan, an op ahead: a task of a shared grid has more rows
@@ -519,58 +584,72 @@ __device__ __forceinline__ bool run_layer_b(Ctx& c, const Params& P, const Layer
         stage_rms_b<S>(c, x, nw);
         prof_stamp(c, op, 1);
         gemv_b<S, false>(c, r0, r1, S::HID, L.s_gu, true, [&](int lane, int row, int j, float v, bool ok) {
-            // rows alternate gate, up; chunks hold whole pairs, so the partner is the next lane
+            // rows alternate gate, up; chunks hold whole pairs, so the partner is the next lane.  The outputs stay in this
+            // CTA, which multiplies them with its column slice of the down-projection.
             const float up = __shfl_down_sync(0xffffffffu, v, 1);
-            if (ok && j < nb && !(lane & 1)) ll_store(P.actl + (size_t)j * S::INTER + (row >> 1), eD, silu_f(v) * up);
+            if (ok && !(lane & 1)) c.sm.act_s[j * DOWN_K + ((row - r0) >> 1)] = silu_f(v) * up;
         });
+        partial_cols_b<S>(c, c.sm.act_s, down_words(P, nb) + (size_t)c.cta * S::HID * ((nb + 1) & ~1), (nb + 1) & ~1, eD);
         prof_stamp(c, op, 3);
     }
-    // ---- E: down-projection + residual
+    // ---- E: sum of the CTAs' partial down-projections + residual, for the rows this CTA owns
     bool failed;
     {
-        const int op = op0 + 4;
+        // Two warps per row, half of the CTAs each: eight CTAs per request, four lanes with two sequences each
+        const int op = op0 + 4, rows = xr1 - xr0, nbp = (nb + 1) & ~1, half = c.warp & 1, t = c.lane & 3;
         prof_stamp(c, op, 0);
-        scale_prefetch(c, L.s_down, xr0, xr1, false);
-        // the warp stages the inputs of the k-blocks it multiplies (3 or 4): pairs e0 + 2 lane + 64 i
-        int kb0, kb1;
-        warp_kslice(S::INTER / 64, c.warp, kb0, kb1);
-        const int e0 = kb0 * 64, e1 = kb1 * 64;
-        const int np = (e1 - e0) / 64;                           // 3 or 4 pairs per lane and sequence
-        // Two sequences per round (8 word pairs in flight).  Keeping the next round's loads in flight
-        // while this one is staged measured slower: the registers it takes end up as spills.
+        const float rs = c.tid < rows * NB ? L.s_down[xr0 + (c.tid >> 3)] : 0.f;      // requested before the wait
+        const int c0 = half ? (c.grid + 1) / 2 : 0, c1 = half ? c.grid : (c.grid + 1) / 2;
 #pragma unroll 1
-        for (int jj = 0; jj < NB; jj += 2) {
-            float v[16];
-            const u64* act0 = P.actl + (size_t)jj * S::INTER + e0 + 2 * c.lane;
-            ll_wait_pairs_fn<8>(c,
-                                [&](int i) -> const u64* {
-                                    if (jj + (i >> 2) >= nb || (i & 3) >= np) return nullptr;
-                                    return act0 + (size_t)(i >> 2) * S::INTER + 64 * (i & 3);
-                                },
-                                [&](int) { return eD; }, v, W_ACT);
-            float mx = 0.f;
+        for (int r = c.warp >> 1; r < rows; r += NCW / 2) {
+            constexpr int PER = 10;                          // grids of up to 160 CTAs
+            const u64* src = down_words(P, nb) + ((size_t)(c0 + (c.lane >> 2)) * S::HID + xr0 + r) * nbp + 2 * t;
+            const size_t stride = (size_t)8 * S::HID * nbp;
+            const int n = 2 * t < nbp ? (c1 - c0 - (c.lane >> 2) + 7) >> 3 : 0;      // words of this lane
+            u64 w[PER][2];
 #pragma unroll
-            for (int i = 0; i < 16; i++) mx = fmaxf(mx, fabsf(v[i]));
-            const float scale = fixed_scale24(warp_max(mx));        // one scale for the pair of sequences
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int k = e0 + 2 * c.lane + 64 * i;
-                    if (k < e1) stage_pair_b(c.sm.xq, S::INTER, jj + u, k, v[8 * u + 2 * i], v[8 * u + 2 * i + 1], scale);
-                }
-            if (c.lane == 0) c.sm.wsc_s[c.warp * 4 + (jj >> 1)] = 1.0f / scale;
-        }
-        __syncwarp();
-        prof_stamp(c, op, 1);
-        failed = gemv_b<S, false>(c, xr0, xr1, S::INTER, L.s_down, false, [&](int, int row, int j, float v, bool ok) {
-            if (ok && j < nb) {
-                const float xn = c.sm.xown[j * 16 + row - xr0] + v;
-                c.sm.xown[j * 16 + row - xr0] = xn;
-                ll_store(P.xl + (size_t)j * S::HID + row, eE, xn);
+            for (int i = 0; i < PER; i++) {
+                w[i][0] = w[i][1] = (u64)eD << 32;           // (no word: a zero)
+                if (i < n) ll_load2(src + i * stride, w[i][0], w[i][1]);
             }
-        });
+            Spin sp;
+            while (true) {
+                bool ok = true;
+#pragma unroll
+                for (int i = 0; i < PER; i++)
+                    if ((uint32_t)(w[i][0] >> 32) != eD || (uint32_t)(w[i][1] >> 32) != eD) {
+                        ok = false;
+                        ll_load2(src + i * stride, w[i][0], w[i][1]);
+                    }
+                if (ok) break;
+                if (MK_SPIN_FAIL(c, sp, W_ACT)) {
+                    c.dead = true;
+                    break;
+                }
+            }
+            float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                a0 += __uint_as_float((uint32_t)w[i][0]);
+                a1 += __uint_as_float((uint32_t)w[i][1]);
+            }
+#pragma unroll
+            for (int x = 4; x < 32; x *= 2) {
+                a0 += __shfl_xor_sync(0xffffffffu, a0, x);
+                a1 += __shfl_xor_sync(0xffffffffu, a1, x);
+            }
+            if (c.lane < 4) *reinterpret_cast<float2*>(c.sm.part_s + (2 * r + half) * NB + 2 * t) = make_float2(a0, a1);
+        }
+        prof_stamp(c, op, 1);
+        failed = consumer_any(c.dead);
+        if (c.tid < rows * NB && (c.tid & 7) < nb) {
+            const int r = c.tid >> 3, j = c.tid & 7;
+            const float xn = c.sm.xown[j * 16 + r] + (c.sm.part_s[2 * r * NB + j] + c.sm.part_s[(2 * r + 1) * NB + j]) * rs;
+            c.sm.xown[j * 16 + r] = xn;
+            ll_store(P.xl + (size_t)j * S::HID + xr0 + r, eE, xn);
+        }
         prof_stamp(c, op, 3);
+        consumer_sync();                                     // the partial sums are free again
     }
     return failed;
 }
@@ -594,6 +673,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) batch_kernel(const __grid_constan
         c.sm.best_s = reinterpret_cast<u64*>(p); p += NCW * 8;                                 // 128
         c.sm.ssq_s = reinterpret_cast<float*>(p); p += NB * NCW * 4;                           // 512
         c.sm.wsc_s = reinterpret_cast<float*>(p); p += NB * NCW * 4;                           // 512
+        c.sm.act_s = reinterpret_cast<float*>(p); p += NB * DOWN_K * 4;                        // 1024
         c.sm.full = reinterpret_cast<uint64_t*>(p); p += 6 * 8;
         c.sm.empty = reinterpret_cast<uint64_t*>(p); p += 6 * 8;
         c.sm.abort_flag = reinterpret_cast<volatile int*>(p); p += 4;
@@ -605,6 +685,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) batch_kernel(const __grid_constan
     c.limit_ns = (u64)A.spin_limit_ns;
     c.status = P.status;
     const int nb = A.nb;
+    if (c.tid < NB * DOWN_K) c.sm.act_s[c.tid] = 0.f;
     if (c.tid == 0) {
         for (int i = 0; i < NS; i++) {
             mbar_init(&c.sm.full[i], 1);

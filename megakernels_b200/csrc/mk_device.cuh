@@ -105,6 +105,12 @@ __device__ __forceinline__ void ll_store(u64* p, uint32_t epoch, float v) {
     const u64 w = ((u64)epoch << 32) | __float_as_uint(v);
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
 }
+// Two neighbouring words (16-byte aligned).
+__device__ __forceinline__ void ll_store2(u64* p, uint32_t epoch, float a, float b) {
+    chaos_delay();
+    const u64 w0 = ((u64)epoch << 32) | __float_as_uint(a), w1 = ((u64)epoch << 32) | __float_as_uint(b);
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(w0), "l"(w1) : "memory");
+}
 __device__ __forceinline__ void ll_store_bits(u64* p, uint32_t epoch, uint32_t bits) {
     chaos_delay();
     const u64 w = ((u64)epoch << 32) | bits;
