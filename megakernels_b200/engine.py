@@ -51,6 +51,46 @@ def rope_tables(cfg, max_seq, device):
     return ang.cos().to(device), ang.sin().to(device)
 
 
+class _CallBuffers:
+    """What one launch takes in and hands back as integers, in one device array: `words` (name -> count of int64 results, zero
+    at first), the eight info words and `ints` (name -> int32 inputs).  One pinned copy brings it to the device and one, with the
+    status words, brings the results back; a copy, a fill and a blocking read for each were a quarter of a one-token call."""
+
+    INFO = 8
+
+    def __init__(self, device, words, ints):
+        self.at, n = {}, 0                              # name -> (first int32, count of int32)
+        for name, count in words.items():
+            self.at[name] = (n, 2 * count)
+            n += 2 * count
+        self.at["info"] = (n, self.INFO)
+        self.n_out = n + self.INFO
+        n = self.n_out
+        for name, values in ints.items():
+            self.at[name] = (n, len(values))
+            n += len(values)
+        host = torch.zeros(n, dtype=torch.int32, pin_memory=True)
+        host[self.n_out:] = torch.tensor([v for values in ints.values() for v in values], dtype=torch.int32)
+        self.dev = host.to(device, non_blocking=True)
+
+    def ptr(self, name):
+        return self.dev.data_ptr() + 4 * self.at[name][0]
+
+    def read(self, status):
+        """Waits for the launch.  Returns the status words; `out(name)` has the results."""
+        back = torch.empty(self.n_out + status.numel(), dtype=torch.int32, pin_memory=True)
+        back[: self.n_out].copy_(self.dev[: self.n_out], non_blocking=True)
+        back[self.n_out:].copy_(status, non_blocking=True)
+        torch.cuda.current_stream(self.dev.device).synchronize()
+        self._back = back
+        return back[self.n_out:].tolist()
+
+    def out(self, name):
+        first, count = self.at[name]
+        t = self._back[first: first + count]
+        return t if name == "info" else t.view(torch.int64)
+
+
 class Megakernel:
     def __init__(self, model, max_seq=8192, device="cuda", quant="bf16", mtp=False,
                  draft_vocab=0, kv_dtype="fp32", spin_limit_ms=2000, draft_ids=None, batch=1, pack_device=None):
@@ -350,31 +390,39 @@ class Megakernel:
     # One place builds the launch record, submits it and settles the host-side bookkeeping that every kind of
     # single-sequence launch shares (status, epoch); the public methods differ in what they ask for and in how
     # they read the result.
-    def _submit(self, n_steps, fields, buffers, timing):
+    def _submit(self, n_steps, fields, buffers, io, timing):
         """Launch `n_steps` steps (or cycles).  `fields`: LaunchArgs members by name; `buffers`: name -> device tensor
-        or None, passed by address under the same name.  Returns the launch's info words as a list (reading them
-        waits for the kernel)."""
+        or None, `io`: _CallBuffers, both passed by address under their names.  Returns the launch's info words as a list (reading
+        them waits for the kernel)."""
         dev = self.device
-        info = torch.zeros(8, dtype=torch.int32, device=dev)
         stamps = torch.zeros(n_steps + 1, dtype=torch.int64, device=dev) if timing else None
         args = dict(n_steps=n_steps, start_pos=self.pos, epoch_base=self.epoch, grid=self.grid,
-                    spin_limit_ns=self.spin_limit_ns, out_info=info.data_ptr(), step_ts=stamps.data_ptr() if timing else 0)
+                    spin_limit_ns=self.spin_limit_ns, step_ts=stamps.data_ptr() if timing else 0)
         args.update(fields)
+        args.update({"out_info" if name == "info" else name: io.ptr(name) for name in io.at})
         args.update({name: (t.data_ptr() if t is not None else 0) for name, t in buffers.items()})
         record = _lib.LaunchArgs(**args)
         stream = torch.cuda.current_stream(dev).cuda_stream
         _lib.check(self.lib.mk_launch(self._h, ctypes.byref(record), ctypes.c_void_p(stream)))
         self.launches += 1
-        words = info.tolist()
-        self._raise_if_timed_out()
-        self.epoch = words[1] & 0xFFFFFFFF
-        if self.epoch > 0xFFFF0000:
-            raise RuntimeError("epoch counter exhausted; call reset()")
+        self._settle(io)
+        words = io.out("info").tolist()
+        self._set_epoch(words[1])
         if timing:
             n_run = words[5] if fields.get("spec") else words[0]
             t = stamps[: n_run + 1].cpu()
             self.last_step_ns = (t[1:] - t[:-1]).tolist()
         return words
+
+    def _settle(self, io):
+        """Waits for the launch behind `io`; raises if a device-side wait of it ran out."""
+        if io.read(self.status)[0] != 0:
+            self._raise_if_timed_out()
+
+    def _set_epoch(self, word):
+        self.epoch = word & 0xFFFFFFFF
+        if self.epoch > 0xFFFF0000:
+            raise RuntimeError("epoch counter exhausted; call reset()")
 
     def _raise_if_timed_out(self):
         """Waits for the device; if a device-side wait ran out, raises with the wait site."""
@@ -383,11 +431,10 @@ class Megakernel:
             _lib.check(self.lib.mk_status(self._h, ctypes.byref(where)))
 
     @staticmethod
-    def _sampling(temperature, seed, stop_ids, device):
-        """The LaunchArgs members that describe how a token is chosen and which ids end a launch."""
-        stops = torch.tensor(list(stop_ids) or [-1], dtype=torch.int32, device=device)
+    def _sampling(temperature, seed, stop_ids):
+        """The LaunchArgs members that describe how a token is chosen, and the ids that end a launch."""
         return dict(seed=seed & 0xFFFFFFFF, inv_temperature=(1.0 / temperature) if temperature > 0 else 0.0,
-                    n_stop=len(stop_ids)), stops
+                    n_stop=len(stop_ids)), list(stop_ids) or [-1]
 
     def _attention_fits(self, last_pos, sequences=1):
         """Whether a launch of so many sequences accepts this context; one that does not is left to say so before anything ran."""
@@ -459,18 +506,17 @@ class Megakernel:
         left, n_left = n_given - taken, n_steps - taken
         # everything that can be refused comes before the prompt changes the state
         hidden = torch.empty(n_steps, cfg.hidden, device=dev) if want_hidden else None
-        how, stops = self._sampling(temperature, seed, stop_ids, dev)
-        bufs = dict(forced=torch.tensor(given[taken:], dtype=torch.int32).pin_memory().to(dev, non_blocking=True),
-                    stop_ids=stops, tokens_out=torch.zeros(n_left, dtype=torch.int64, device=dev),
-                    logits_out=torch.empty(n_left, cfg.vocab, device=dev) if (return_logits or all_logits) else None,
+        how, stops = self._sampling(temperature, seed, stop_ids)
+        io = _CallBuffers(dev, dict(tokens_out=n_left), dict(forced=given[taken:], stop_ids=stops))
+        bufs = dict(logits_out=torch.empty(n_left, cfg.vocab, device=dev) if (return_logits or all_logits) else None,
                     resid_out=hidden[taken:] if want_hidden else None, prof=prof)
         first_choice = 0 if all_logits else left - 1               # the first step whose LM head runs
         if taken:
             self._take_in(given[:taken], start, hidden)
-        words = self._submit(n_left, dict(how, start_pos=start + taken, n_forced=left, lm_from=first_choice, prof_step=prof_step), bufs, timing)
+        words = self._submit(n_left, dict(how, start_pos=start + taken, n_forced=left, lm_from=first_choice, prof_step=prof_step), bufs, io, timing)
         ran = words[0]
         # tokens_out holds keys (ordered score << 32 | ~id): the low word, complemented, is the id
-        chosen = (0xFFFFFFFF - (bufs["tokens_out"][left - 1: ran] & 0xFFFFFFFF)).tolist()
+        chosen = (0xFFFFFFFF - (io.out("tokens_out")[left - 1: ran] & 0xFFFFFFFF)).tolist()
         if want_hidden:
             hidden = hidden[: taken + ran]
         if taken + ran:
@@ -524,23 +570,18 @@ class Megakernel:
         n_forced = [len(p) for p in prompts]
         n_total = [n + n_generate - 1 for n in n_forced]
         n_steps = max(n_total)
-        forced = torch.zeros(max(n_forced), NBW, dtype=torch.int32)
-        for j, p in enumerate(prompts):
-            forced[: len(p), j] = torch.tensor(p, dtype=torch.int32)
-        forced = forced.pin_memory().to(dev, non_blocking=True)
-        stops = torch.tensor(list(stop_ids) or [-1], dtype=torch.int32, device=dev)
-        out = torch.zeros(n_steps, NBW, dtype=torch.int64, device=dev)
-        info = torch.zeros(8, dtype=torch.int32, device=dev)
+        forced = [[p[i] if i < len(p) else 0 for p in prompts] + [0] * (NBW - B) for i in range(max(n_forced))]
+        io = _CallBuffers(dev, dict(tokens_out=n_steps * NBW), dict(forced=[t for row in forced for t in row], stop_ids=list(stop_ids) or [-1]))
         ts = torch.zeros(n_steps + 1, dtype=torch.int64, device=dev) if timing else None
         logits = torch.empty(n_steps, NBW, self.cfg.vocab, device=dev) if return_logits else None
         ptr = lambda t: t.data_ptr() if t is not None else 0
         pad = lambda v: (ctypes.c_int32 * NBW)(*(list(v) + [0] * (NBW - len(v))))
-        a = _lib.BatchArgs(forced=forced.data_ptr(), n_forced=pad(n_forced), n_total=pad(n_total),
+        a = _lib.BatchArgs(forced=io.ptr("forced"), n_forced=pad(n_forced), n_total=pad(n_total),
                            pos0=pad(pos0), batch=B, n_steps=n_steps, lm_from=min(n_forced) - 1,
                            epoch_base=self.epoch, seed=seed & 0xFFFFFFFF,
                            inv_temperature=1.0 / temperature if temperature > 0 else 0.0, n_stop=len(stop_ids),
-                           prof_step=prof_step, stop_ids=stops.data_ptr(), tokens_out=out.data_ptr(),
-                           logits_out=ptr(logits), step_ts=ptr(ts), out_info=info.data_ptr(), prof=ptr(prof),
+                           prof_step=prof_step, stop_ids=io.ptr("stop_ids"), tokens_out=io.ptr("tokens_out"),
+                           logits_out=ptr(logits), step_ts=ptr(ts), out_info=io.ptr("info"), prof=ptr(prof),
                            spin_limit_ns=self.spin_limit_ns)
         for j, body in enumerate(bodies):                  # behind everything that can be refused
             if body:
@@ -548,15 +589,13 @@ class Megakernel:
         stream = torch.cuda.current_stream(dev).cuda_stream
         _lib.check(self.lib.mk_launch_batch(self._h, ctypes.byref(a), ctypes.c_void_p(stream)))
         self.launches += 1
-        done, epoch, _ = info[:3].tolist()          # synchronises with the launch
-        self._raise_if_timed_out()
-        self.epoch = epoch & 0xFFFFFFFF
-        if self.epoch > 0xFFFF0000:
-            raise RuntimeError("epoch counter exhausted; call reset()")
+        self._settle(io)
+        done, epoch = io.out("info")[:2].tolist()
+        self._set_epoch(epoch)
         if timing:
             t = ts[: done + 1].cpu()
             self.last_step_ns = (t[1:] - t[:-1]).tolist()
-        ids_all = (0xFFFFFFFF - (out[:done] & 0xFFFFFFFF)).cpu()
+        ids_all = 0xFFFFFFFF - (io.out("tokens_out").view(n_steps, NBW)[:done] & 0xFFFFFFFF)
         stop_set = set(int(s) for s in stop_ids)
         result, result_logits = [], []
         for j in range(B):
@@ -661,15 +700,14 @@ class Megakernel:
             raise ValueError(f"sequence would exceed max_seq={self.max_seq}")
         self._mtp_close(self.pos, token)
         dev = self.device
-        how, stops = self._sampling(temperature, seed, stop_ids, dev)
-        bufs = dict(stop_ids=stops, spec_out=torch.zeros(n_generate, dtype=torch.int32, device=dev),
-                    cycle_out=torch.zeros(2 * cycles, dtype=torch.int32, device=dev),
-                    logits_out=torch.empty(cycles, 2, self.cfg.vocab, device=dev) if return_logits else None, prof=prof)
+        how, stops = self._sampling(temperature, seed, stop_ids)
+        io = _CallBuffers(dev, dict(spec_out=(n_generate + 1) // 2, cycle_out=cycles), dict(stop_ids=stops))     # int32 ids, and pairs of them
+        bufs = dict(logits_out=torch.empty(cycles, 2, self.cfg.vocab, device=dev) if return_logits else None, prof=prof)
         words = self._submit(cycles, dict(how, forced=0, n_forced=0, lm_from=0, tokens_out=0, spec=1, first_tok=int(token),
-                                          first_draft=int(draft), limit=n_generate, prof_step=prof_step), bufs, timing)
+                                          first_draft=int(draft), limit=n_generate, prof_step=prof_step), bufs, io, timing)
         emitted, _, self.pos, pending, next_draft, cycles_run = words[:6]
-        self.last_cycles = bufs["cycle_out"][: 2 * cycles_run].view(-1, 2).tolist()
-        ids = bufs["spec_out"][:emitted].tolist()
+        self.last_cycles = io.out("cycle_out").view(torch.int32)[: 2 * cycles_run].view(-1, 2).tolist()
+        ids = io.out("spec_out").view(torch.int32)[:emitted].tolist()
         assert ids[-1] == pending
         if return_logits:
             self.last_logits = bufs["logits_out"][:cycles_run]
