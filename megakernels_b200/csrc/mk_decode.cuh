@@ -884,12 +884,7 @@ __device__ bool gdn_op(Ctx& c, const Params& P, const LayerP& L, int pos, uint32
     }
     prof_stamp(c, op, 2);
     consumer_sync();  // the scratch aliases the GEMV input vector that the next prologue writes
-    if (c.tid < T) {
-        float tot = 0.f;
-#pragma unroll
-        for (int w = 0; w < NCW; w++) tot += osq[c.tid * NCW + w];
-        ll_store(P.mixl + (size_t)c.tid * S::MIX + c.cta, e_out, tot);
-    }
+    if (c.tid < T) ll_store(P.mixl + (size_t)c.tid * S::MIX + c.cta, e_out, sum_warps(osq + c.tid * NCW));
     // out-projection, split over K: this task's 16 gated outputs times its column slice -> 1024 partial sums
     partial_cols<S, Q8, T, 1>(c, c.sm.mix_s, P.partl + (size_t)c.cta * S::HID, (size_t)c.grid * S::HID, e_out);
     return true;
@@ -1376,6 +1371,9 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
         const int op = op0 + 2;
         prof_stamp(c, op, 0);
         static_assert(S::GDN_TASKS == 128 && S::LIN_DV / S::GDN_SLICE == 8, "four tasks per lane, eight per head");
+        // The CTAs without a task have been here since the in-projection.  Polling the one kilobyte of sums of squares all the while,
+        // they made a hot spot of it: a step took 389 or 451 us (int8, 700 positions) depending on where in memory it lay.
+        if (!had_task) gate_on_samples(c, P.mixl + (size_t)(T - 1) * S::MIX, S::GDN_TASKS, eB);
         own_rows<T>(c, xr0, xr1, [&](int j, int row, bool a_own, bool b_own) {
             const float rs0 = Q8 && a_own ? L.s_out[row] : 1.0f, rs1 = Q8 && b_own ? L.s_out[row + 1] : 1.0f;   // requested before the wait
             const u64* psrc = P.partl + (size_t)j * c.grid * S::HID + row + (size_t)c.lane * S::HID;
