@@ -1027,7 +1027,8 @@ __device__ __forceinline__ float sum2(u64 a) { return __uint_as_float((uint32_t)
 // a CTA holds 16 rows and a head is eight CTAs.  What bounds a block is shared memory: a 16-byte read is four of its cycles, and
 // every lane reads its keys of eight k and eight q.  Two rows a lane halve the reads per product, and the k's stay in registers
 // for the update.  16 heads x 511 positions: 54 us (69 with eight lanes to one row; 207 position by position).
-static __global__ void __launch_bounds__(128) gdn_scan(const __grid_constant__ GdnArgs G) {
+template <bool FOUR>      // four CTAs per SM
+static __global__ void __launch_bounds__(128, FOUR ? 4 : 0) gdn_scan(const __grid_constant__ GdnArgs G) {
     chain_wait();
     constexpr int ROWS = 16, IN = 256 + ROWS;
     __shared__ __align__(16) float in_s[2][SCAN][IN];        // q | k | values

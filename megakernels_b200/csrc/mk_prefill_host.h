@@ -131,8 +131,9 @@ inline int launch_gdn(const GdnArgs& G, void (*gate)(GdnArgs), int sms, cudaStre
     // land on one SM and share its shared memory, which is what they are bound by (16 heads x 511 positions: the pass takes 6.41 instead
     // of 5.27 ms).  With more CTAs than SMs they share anyway.
     const dim3 scan(8, G.nvh, G.M);
-    if (8 * G.nvh * G.M <= sms) gdn_scan<<<scan, 128, 0, st>>>(G);
-    else MKP_CUDA(launch(gdn_scan, scan, 128, 0, st, G));
+    // (More than three CTAs per SM: fewer registers each instead of a second round.)
+    if (8 * G.nvh * G.M <= sms) gdn_scan<false><<<scan, 128, 0, st>>>(G);
+    else MKP_CUDA(launch(8 * G.nvh * G.M <= 3 * sms ? gdn_scan<false> : gdn_scan<true>, scan, 128, 0, st, G));
     MKP_CUDA(cudaGetLastError());
     MKP_CUDA(launch(gate, dim3((G.nvh + 15) / 16, rows), 256, 0, st, G));
     MKP_CUDA(cudaGetLastError());
