@@ -606,6 +606,9 @@ __device__ __noinline__ void attn_stage(Shared& S, const mk_stage_desc& d) {
 //     the large sums of the first piece take one MMA per tile.  Off 64 bits by 1.9e-7 in a task of 250 positions and 256 dims
 //     (3.3e-7 with one chain per operand half and the third piece in rows 0-7; fp32 FMAs: 1.6e-7), growing with the tiles per
 //     warp: 4.2e-7 at 800 positions and 512 dims; fresh accumulators per tile would end that for 1 % of a step;
+//   * K goes by 128 dims: with 256 a lane asked for sixteen 16-byte pieces at once, and at 96 registers a thread the outputs'
+//     accumulators went to local memory and back around them (652 instead of 404 bytes of spill stores, four sequences at
+//     8000 positions and 256 dims 65 instead of 72 us);
 //   * 256 positions at a time with a running maximum; one CTA barrier per 256.
 constexpr int ATTN_SUB = 256;             // positions between two barriers: one tile per warp
 // Buffers of cache-row offsets.  Sub-chunk s + 1's are written between the barriers of s - 1 and s, when a slower warp still
@@ -734,25 +737,24 @@ __device__ __noinline__ void attn_mma_stage(Shared& S, const mk_stage_desc& d) {
                     const uint8_t* q = qb + g * qb_stride + t * 16;
                     float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-                    for (int e = 0; e < HD; e += 256) {
-                        uint4 ka[8], kb[8];
+                    for (int e = 0; e < HD; e += 128) {
+                        uint4 ka[4], kb[4];
 #pragma unroll
-                        for (int j = 0; j < 8; j++) {
+                        for (int j = 0; j < 4; j++) {
                             ka[j] = __ldcg(reinterpret_cast<const uint4*>(ra + e + j * 32));
                             kb[j] = __ldcg(reinterpret_cast<const uint4*>(rb + e + j * 32));
                         }
 #pragma unroll
-                        for (int j = 0; j < 8; j++) {
+                        for (int j = 0; j < 4; j++) {
                             const uint4 qv = *reinterpret_cast<const uint4*>(q + (e + j * 32) * 2);
                             const uint32_t a0[4] = {ka[j].x, kb[j].x, ka[j].y, kb[j].y}, a1[4] = {ka[j].z, kb[j].z, ka[j].w, kb[j].w};
                             mma_bf16(s0, a0, qv.x, qv.y);
                             mma_bf16(s1, a1, qv.z, qv.w);
-                            if ((j & 3) == 3)
+                        }
 #pragma unroll
-                                for (int i = 0; i < 4; i++) {
-                                    c[i] += s0[i] + s1[i];
-                                    s0[i] = s1[i] = 0.f;
-                                }
+                        for (int i = 0; i < 4; i++) {
+                            c[i] += s0[i] + s1[i];
+                            s0[i] = s1[i] = 0.f;
                         }
                     }
 #pragma unroll
