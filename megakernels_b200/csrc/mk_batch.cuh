@@ -69,7 +69,7 @@ __device__ __forceinline__ void mma_s8u8(int (&c)[4], uint32_t a0, uint32_t a1, 
 
 // Power of two that maps a vector whose largest magnitude is `mx` below 2^22: with rounding the
 // integers stay inside the signed 24-bit range.
-__device__ __forceinline__ float fixed_scale24(float mx) { return fixed_scale(mx) * 0.03125f; }
+__device__ __forceinline__ float fixed_scale24(float mx) { return fixed_scale(mx) * 0.00390625f; }
 
 // Stage inputs k, k + 1 of sequence `seq` into the three digit planes: byte d of both integers is one
 // byte permute and one 16-bit store.
