@@ -478,7 +478,7 @@ __device__ void request_kv(const Ctx& c, const Params& P, const LayerP& L, const
     const int per = c.grid / A.nb, q = c.cta / per;
     if (q >= A.nb) return;
     const int cta = c.cta - q * per, pos = A.pos0[q] + step, n = pos + 1;
-    const int ch = attn_chunk(n, min(per / S::NKV, MAX_SPLITS)), g = cta % S::NKV, p0 = cta / S::NKV * ch, p1 = min(pos, p0 + ch);
+    const int ch = attn_chunk_shared(n, min(per / S::NKV, MAX_SPLITS)), g = cta % S::NKV, p0 = cta / S::NKV * ch, p1 = min(pos, p0 + ch);
     constexpr uint32_t ROW = S::HD * (KVF32 ? 4 : 2);
     const int* bt = c.sm.bt_s + q * (P.max_seq / KV_BLOCK);
     for (int p = p0; p < p1; p = (p / KV_BLOCK + 1) * KV_BLOCK) {
@@ -522,7 +522,7 @@ __device__ __forceinline__ bool run_layer_b(Ctx& c, const Params& P, const Layer
         if (q < nb) {
             const AttnView view = {c.cta - q * per, per, P.projl + (size_t)q * S::PROJ_MAX, P.mixl + (size_t)q * S::MIX,
                                    P.attn_part + (size_t)q * S::NKV * MAX_SPLITS * S::PART_STRIDE,
-                                   c.sm.bt_s + q * (P.max_seq / KV_BLOCK), true};
+                                   c.sm.bt_s + q * (P.max_seq / KV_BLOCK), true, true};
             had_task = attn_op<S, KVF32, 1>(c, P, L, view, A.pos0[q] + step, eA, eB, op0 + 1);
         }
     } else {

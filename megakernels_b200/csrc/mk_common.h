@@ -144,5 +144,12 @@ __host__ __device__ inline int attn_chunk(int n, int max_splits) {
     while ((n + ch - 1) / ch > max_splits) ch = ch < KV_BLOCK ? ch * 2 : ch + KV_BLOCK;
     return ch;
 }
+// The same for a sequence that shares the grid, in steps of 16 positions: with a few CTAs per KV head a step of a whole page leaves
+// a third of them idle (641 positions, nine tasks: 80 each instead of six of 128).  Never more than attn_chunk gives, and more than
+// MAX_CHUNK_POS for the same n.
+__host__ __device__ inline int attn_chunk_shared(int n, int max_splits) {
+    const int ch = ((n + max_splits - 1) / max_splits + 15) / 16 * 16;
+    return ch < 16 ? 16 : ch;
+}
 
 }  // namespace mk

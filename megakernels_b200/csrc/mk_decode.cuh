@@ -950,6 +950,7 @@ struct AttnView {
     u64* mixl;              // mixer output words of that slot
     u64* part;              // split partials of that slot
     const int* bt;          // the sequence's block table (shared memory)
+    bool shared;            // several sequences share the grid (positions per task: attn_chunk_shared)
     bool gate;              // publish o * sigmoid(gate) instead of o (otherwise the out-projection's prologue applies the gate)
 };
 
@@ -965,7 +966,7 @@ __device__ bool attn_op(Ctx& c, const Params& P, const LayerP& L, const AttnView
     constexpr int PFV = 8, VU = 8;              // V elements a thread requests before the wait, and together later on
     const int n = pos + T;
     const int max_splits = min(V.grid / S::NKV, MAX_SPLITS);
-    const int ch = attn_chunk(n, max_splits);
+    const int ch = V.shared ? attn_chunk_shared(n, max_splits) : attn_chunk(n, max_splits);
     const int nsplit = (n + ch - 1) / ch;
     if (V.cta >= nsplit * S::NKV) return false;
     const int g = V.cta % S::NKV, sp = V.cta / S::NKV;
@@ -1358,7 +1359,7 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
     }
     // ---- B: mixer
     prof_stamp(c, op0 + 1, 0);
-    const AttnView view = {c.cta, c.grid, P.projl, P.mixl, P.attn_part, c.sm.bt_s, false};
+    const AttnView view = {c.cta, c.grid, P.projl, P.mixl, P.attn_part, c.sm.bt_s, false, false};
     const bool had_task = attn ? attn_op<S, KVF32, T>(c, P, L, view, pos, eA, eB, op0 + 1)
                                : gdn_op<S, Q8, T>(c, P, L, pos, eA, eB, op0 + 1, from_bak);
     prof_stamp(c, op0 + 1, 3);

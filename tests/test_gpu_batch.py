@@ -248,3 +248,19 @@ def test_long_context_where_attention_chunks_grow(tiny, lib_built):
             assert got == pick_token(ref), (j, i)
             if i + 1 < len(ids[j]):
                 ref = dec.step(got)
+
+
+@pytest.mark.parametrize("batch,length", [(8, 144), (8, 577), (5, 230), (3, 400), (2, 593)])
+def test_attention_tasks_of_any_size_equal_a_sequence_alone(tiny, batch, length, lib_built):
+    """Positions per attention task grow in steps of 16 when sequences share the grid: contexts on either side of such a step
+    (9, 14, 24 and 37 tasks per KV head), of a page and of one task, against the same sequences decoded alone."""
+    cfg, w = tiny
+    prompts = [make_prompt(cfg, max(2, length - 3 * j), seed=100 + j) for j in range(batch)]
+    ids, logits = engine(cfg, w, batch=batch, max_seq=1024).run_batch(prompts, n_generate=8, return_logits=True)
+    alone = engine(cfg, w, max_seq=1024)
+    for j, prompt in enumerate(prompts):
+        alone.reset()
+        one, want = alone.run(prompt, n_generate=8, return_logits=True)
+        assert ids[j] == one
+        # integer products, fp32 sums in another order
+        assert float((logits[j].double() - want.double()).norm() / want.double().norm()) < 2e-5
