@@ -863,8 +863,9 @@ __device__ __forceinline__ float* conv_slot(const GdnArgs& G, int m, int ch, int
 
 // Causal conv1d + SiLU of every channel, L2 norms of q and k, and the scalars of the recurrence.  One warp per 128
 // channels and CONV_ROWS consecutive rows, four channels per lane: the window slides through registers, so an input is read
-// once per CONV_ROWS + 3 rows instead of four times.
-constexpr int CONV_ROWS = 8;
+// CONV_ROWS + 3 times in CONV_ROWS rows instead of four times a row.  (Eight rows a warp were a chain of 16 us whatever the shape; two are
+// 1 to 3 % of a pass, one takes longer again.)
+constexpr int CONV_ROWS = 2;
 static __global__ void __launch_bounds__(256) gdn_conv(const __grid_constant__ GdnArgs G) {
     chain_wait();
     const int groups = (G.L + CONV_ROWS - 1) / CONV_ROWS, m = blockIdx.y / groups, l0 = (blockIdx.y - m * groups) * CONV_ROWS, lane = threadIdx.x & 31;

@@ -319,3 +319,21 @@ def test_prompt_rows_of_crowded_experts(model, M, length):
         assert (eng.rt._workspace is not None) == rows
         eng.check()
     assert rel(*out) < 3e-2
+
+
+@pytest.mark.parametrize("fmt,M,length", [({}, 1, 258), ({}, 1, 386), ({}, 2, 386), ({"fmt": "bf16"}, 3, 130)])
+def test_prompt_rows_in_wide_tiles(packed, fmt, M, length):
+    """Tiles of more than 256 tokens (two MMAs per step): just over that, the widest one and a row past it, two of them.  The first
+    layer's state sees no earlier bf16 rounding, so it agrees to fp32 sums."""
+    pkg, shape = SHAPES["27b"]
+    prompts, engines = [pkg.make_prompt(shape.vocab, length, seed=j) for j in range(M)], []
+    for rows in (True, False):
+        eng = pkg.Engine(packed("27b", fmt), M, maxlen=length + 64)
+        with pytest.MonkeyPatch.context() as mp:
+            if not rows:
+                mp.setattr(runtime, "MIN_ROWS_PATH", 1 << 30)
+            engines.append((eng, eng.prefill(prompts).clone()))
+        assert (eng.rt._workspace is not None) == rows
+        eng.check()
+    (a, la), (b, lb) = engines
+    assert rel(la, lb) < 3e-2 and rel(a.ssm[0], b.ssm[0]) < 2e-4 and rel(a.ssm, b.ssm) < 1e-2
