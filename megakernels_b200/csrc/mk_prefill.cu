@@ -332,7 +332,10 @@ struct Exec {
             // (by estimate: narrower tiles leave fewer columns of padding, wider ones convert an expert's weights fewer times)
             const int mean = (int)((long long)rows * topk / experts);
             memset(&route, 0, sizeof route);
-            few = fp8 && mean <= (scaled ? 32 : 16);
+            // Few rows per expert go straight from the packed tiles.  Passes through the operand against these, ms, at a mean load of
+            // block scales (256 experts): 40 9.37 / 7.62, 64 11.77 / 11.00, 78 13.71 / 13.21, 93 15.38 / 15.14; beyond, the operand's
+            // tiles are 256 tokens wide.  Row scales (128 experts): 20 3.52 / 3.42, 24 3.57 / 3.58, 32 3.79 / 4.07.
+            few = fp8 && mean <= (scaled ? 96 : 20);
             if (few) route.nt = 32;
             else route.nt = mean > 96 ? 256 : (mean > 40 ? 128 : (mean > 16 ? 64 : 32));
             slot_rows = (rows * topk + experts * 15 + route.nt + 15) / 16 * 16;

@@ -2,8 +2,8 @@
 // one step, done for all positions of a prompt at once.
 //
 // The contractions are matrix products here, so they run on the 5th-generation tensor cores: `rows_gemm` keeps 128
-// weight rows as the A operand of tcgen05.mma and up to 256 token rows as its N columns, accumulators in tensor
-// memory.  The weights of a stage program stay in the decode kernel's packed tiles: eight or sixteen warps read a tile
+// weight rows as the A operand of tcgen05.mma and up to 384 token rows as its N columns, accumulators in tensor
+// memory.  (FP8 experts with few rows each: `experts_gemm`, where the weights stay in registers for mma.sync.)  The weights of a stage program stay in the decode kernel's packed tiles: eight or sixteen warps read a tile
 // step each with one 128-bit load per lane, convert it to bf16 pieces that hold its value and write the swizzled operand
 // into shared memory, so a prompt reads the same bytes from HBM as a decode step does and needs no second copy of the
 // model.  (The 0.8B model does keep one: mk_prefill_08b.cu.)
@@ -1616,18 +1616,34 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
 // which kept the stream at 1.5 of 6.5 TB/s.  The packed tiles are the register fragments of mma.sync, so here they stay in the
 // warp that loaded them: 9 instructions turn four fp8 bytes into two bf16 pairs and the MMA takes them as they are.
 //   A unit is 128 weight rows (eight warps, a tile each) times the rows of a work item; CTAs take units in turn and warps run on
-// from unit to unit, each at its own pace.  Token rows come in stages of 128 columns by bulk copies of a ninth warp.
+// from unit to unit, each at its own pace.  Token rows come in stages of 128 columns by bulk copies that warp 0 asks for.
 //   Columns of a token row are stored (gather_rows, the epilogue below) in the order in which the fragments hold those of the
 // weights: of sixteen columns the even ones, then the odd ones.  Block-scaled FP8 adds an accumulator per 128 columns with the
 // block's scale to fp32 sums (the decode kernel's arithmetic); row scales are applied at the end.
-//   Bound by issue slots (58 % used) and then by the stream: 256 experts x 15.6 rows, block-scaled, a layer's gate and up products (537 MB)
-// 198 us, down (268 MB) 120 us, against 348 and 174 through the operand (83 and 42 at the measured copy bandwidth).
+//   Each warp's weights come through a ring of its own in shared memory, four pairs of blocks ahead.  (In registers, two pairs: 47 %
+// of the issue slots used and gate and up 190 us, down 103.)
+//   Bound by issue slots (60 % used, a fifth of the rest math-pipe throttle) and then by the stream: 256 experts x 15.6 rows,
+// block-scaled, a layer's gate and up products (537 MB) 151 us, down (268 MB) 91 us, against 348 and 174 through the operand (83
+// and 42 at the measured copy bandwidth).
 // NT8: groups of eight tokens of the widest item.
-constexpr int EX_STAGES = 6;
+constexpr int EX_STAGES = 5, EX_AHEAD = 4;
+constexpr int EX_PAIR = 2048 + 16, EX_BARS = 128;      // bytes of two blocks of a tile and their scales; of the barriers
 struct ExpertBars {
     uint64_t full[EX_STAGES], empty[EX_STAGES];
     volatile int dead;
 };
+static_assert(sizeof(ExpertBars) <= EX_BARS, "");
+constexpr int experts_smem(int nt8) { return 1024 + EX_STAGES * 2 * nt8 * 8 * 128 + EX_BARS + 8 * EX_AHEAD * EX_PAIR; }
+__device__ __forceinline__ uint4 lds16(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 lds8(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    return v;
+}
 // Four fp8 bytes as two pairs of bf16: bytes 0 and 2, bytes 1 and 3.
 __device__ __forceinline__ void e4m3x4_bf16(uint32_t w, uint32_t& even, uint32_t& odd) {
     constexpr uint32_t UP = 0x7B807B80u;           // 2^120: the bits moved into the bf16 fields are the values times 2^-120, subnormals included
@@ -1658,123 +1674,141 @@ static __global__ void __launch_bounds__(256, 2) experts_gemm(const __grid_const
     }
     __syncthreads();
     const int g = lane >> 2, t = lane & 3;
-    // Requests run ahead of the products, across units, two blocks of 64 columns at a time; warp 0 asks for the token rows too.
-    // (Block-scaled: the two are four steps of one chunk with a scale each for the tile's upper and lower eight rows.)
+    // Requests run EX_AHEAD pairs of blocks (64 columns each) ahead of the products, across units: each lane copies the bytes that it
+    // will read to the warp's ring, and warp 0 asks for the token rows too.  (Block-scaled: a pair is four steps of one chunk with a
+    // scale each for the tile's upper and lower eight rows.)
     Walk<W_FP8> walk;
-    Raw<W_FP8> raw[4];
-    float2 scale[2];
     int ask_u = blockIdx.x, ask_kb = 0;
     uint32_t ask_slot = 0, ask_phase = 0;
-    int4 ask_it = item(blockIdx.x);
+    const uint32_t ring = smem_u32(smem + EX_STAGES * 2 * X_KB + EX_BARS + warp * (EX_AHEAD * EX_PAIR));
+    uint32_t ask_at = 0, at = 0;                   // ring places of the next pair to ask for and to multiply
+    int4 ask_it = item(blockIdx.x), ask_next = item(blockIdx.x + gridDim.x);
     auto ask_start = [&]() { walk.start(A, A.w + (size_t)ask_it.x * A.w_gstride, min(ask_u % A.blocks * 8 + warp, A.tiles - 1), 0, lane); };
-    auto request2 = [&](Raw<W_FP8>& a, Raw<W_FP8>& b, float2& sc) {
+    auto request = [&]() {
         if (ask_u < units) {
-            if (ask_kb < A.kbs) {
-                const bool two = BLOCKS || ask_kb + 1 < A.kbs;
-                if (BLOCKS) {
-                    const uint4* q = reinterpret_cast<const uint4*>(walk.p);
-                    a.q[0] = __ldg(q); a.q[1] = __ldg(q + 32); b.q[0] = __ldg(q + 64); b.q[1] = __ldg(q + 96);
-                    sc = __ldg(reinterpret_cast<const float2*>(walk.s));
-                    walk.p += 2048;
-                    walk.s += 8;
-                    if ((walk.left -= 4) == 0) {
-                        walk.left = A.chunk_steps;
-                        walk.p += A.chunk_bytes - A.chunk_steps * 512;
-                        walk.s += A.chunk_bytes - A.chunk_steps * 2;
-                    }
-                } else {
-                    walk.load(A, a);
-                    if (two) walk.load(A, b);
+            const bool two = BLOCKS || ask_kb + 1 < A.kbs;
+            const uint32_t to = ring + ask_at + lane * 16;
+            if (BLOCKS) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) mk::cp_async16(to + i * 512, walk.p + i * 512);
+                if (lane == 0) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to + 2048), "l"(walk.s) : "memory");
+                walk.p += 2048;
+                walk.s += 8;
+                if ((walk.left -= 4) == 0) {
+                    walk.left = A.chunk_steps;
+                    walk.p += A.chunk_bytes - A.chunk_steps * 512;
+                    walk.s += A.chunk_bytes - A.chunk_steps * 2;
                 }
-                if (warp == 0 && lane == 0 && wait(B, A, &B.empty[ask_slot], ask_phase ^ 1u, WP_EMPTY)) {
-                    const uint32_t bytes = (uint32_t)((ask_it.z + 7) & ~7) * 128u;
-                    mbar_expect_tx(&B.full[ask_slot], two ? 2 * bytes : bytes);
-                    for (int i = 0; i < (two ? 2 : 1); i++)
-                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                     ::"r"(smem_u32(smem + (size_t)(2 * ask_slot + i) * X_KB)), "l"(A.x + ((size_t)(ask_kb + i) * A.x_rows + ask_it.y) * 128), "r"(bytes),
-                                       "r"(smem_u32(&B.full[ask_slot])) : "memory");
-                }
-                if (++ask_slot == EX_STAGES) {
-                    ask_slot = 0;
-                    ask_phase ^= 1u;
+            } else {
+                for (int i = 0; i < (two ? 4 : 2); i++) {
+                    mk::cp_async16(to + i * 512, walk.p);
+                    walk.step(A);
                 }
             }
-            ask_kb += 2;
-            if (ask_kb >= A.kbs && !(ask_kb & 2)) {                // (a unit is a whole number of turns of the two buffers)
+            if (warp == 0 && lane == 0 && wait(B, A, &B.empty[ask_slot], ask_phase ^ 1u, WP_EMPTY)) {
+                const uint32_t bytes = (uint32_t)((ask_it.z + 7) & ~7) * 128u;
+                mbar_expect_tx(&B.full[ask_slot], two ? 2 * bytes : bytes);
+                for (int i = 0; i < (two ? 2 : 1); i++)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 ::"r"(smem_u32(smem + (size_t)(2 * ask_slot + i) * X_KB)), "l"(A.x + ((size_t)(ask_kb + i) * A.x_rows + ask_it.y) * 128), "r"(bytes),
+                                   "r"(smem_u32(&B.full[ask_slot])) : "memory");
+            }
+            if (++ask_slot == EX_STAGES) {
+                ask_slot = 0;
+                ask_phase ^= 1u;
+            }
+            if ((ask_at += EX_PAIR) == EX_AHEAD * EX_PAIR) ask_at = 0;
+            if ((ask_kb += 2) >= A.kbs) {
                 ask_kb = 0;
                 ask_u += gridDim.x;
-                ask_it = item(ask_u);
+                ask_it = ask_next;
+                ask_next = item(ask_u + gridDim.x);
                 if (ask_u < units) ask_start();
             }
         }
+        mk::cp_async_commit();                     // (also when there is nothing left: waiting for all but EX_AHEAD - 1 then still waits for the pair)
     };
     ask_start();
-    request2(raw[0], raw[1], scale[0]);
-    request2(raw[2], raw[3], scale[1]);
+#pragma unroll 1
+    for (int i = 0; i < EX_AHEAD; i++) request();
     uint32_t slot = 0, phase = 0;
     const uint32_t frag = smem_u32(smem) + (uint32_t)(lane & 7) * 128, piece = lane >> 3, sw = lane & 7;
     int4 it = item(blockIdx.x);
 #pragma unroll 1
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
         const int4 next = item(u + gridDim.x);
-        const int n8 = (it.z + 7) >> 3, tile = u % A.blocks * 8 + warp;
-        float acc[NT8][4], sums[BLOCKS ? NT8 : 1][4];
-#pragma unroll
-        for (int n = 0; n < NT8; n++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) acc[n][i] = sums[BLOCKS ? n : 0][i] = 0.f;
+        const int tile = u % A.blocks * 8 + warp;
+        float sums[NT8][4];
         bool ok = true;
-        auto product = [&](const Raw<W_FP8>& r, uint32_t x, bool fresh) {           // fresh: the accumulators start over
-            uint32_t a[4][4];                        // [16 columns][row g even, row g + 8 even, row g odd, row g + 8 odd]
+        // The unit's products for N8 groups of eight tokens, written out for each number: a loop that leaves at the number in hand took
+        // a fifth more instructions, most of them branches (gate and up 200 us instead of 190).
+        auto products = [&](auto n8) {
+            constexpr int N8 = decltype(n8)::value;
+            float acc[N8][4];
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
-                e4m3x4_bf16(r.q[i].x, a[2 * i][0], a[2 * i][2]);
-                e4m3x4_bf16(r.q[i].y, a[2 * i + 1][0], a[2 * i + 1][2]);
-                e4m3x4_bf16(r.q[i].z, a[2 * i][1], a[2 * i][3]);
-                e4m3x4_bf16(r.q[i].w, a[2 * i + 1][1], a[2 * i + 1][3]);
-            }
+            for (int n = 0; n < N8; n++)
 #pragma unroll
-            for (int n = 0; n < NT8; n++) {
-                if (n >= n8) break;
-                uint32_t b[2][4];
+                for (int i = 0; i < 4; i++) acc[n][i] = sums[n][i] = 0.f;
+            auto product = [&](uint32_t w, uint32_t x, bool fresh) {                     // fresh: the accumulators start over
+                uint32_t a[4][4];                        // [16 columns][row g even, row g + 8 even, row g odd, row g + 8 odd]
 #pragma unroll
-                for (int h = 0; h < 2; h++) ldsm4(b[h], x + n * 1024 + (((4 * h + piece) ^ sw) << 4));
-                if (fresh) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-#pragma unroll
-                for (int j = 0; j < 4; j++) mma16816(acc[n], a[j], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
-            }
-        };
-        auto pair = [&](int kb, Raw<W_FP8>& ra, Raw<W_FP8>& rb, float2& sc) {
-            if (kb < A.kbs) {
-                ok = ok && __all_sync(0xffffffffu, wait(B, A, &B.full[slot], phase, WP_FULL));     // the warp leaves together
-                if (!ok) return;
-                const uint32_t x = frag + 2 * slot * X_KB;
-                product(ra, x, BLOCKS);
-                if (BLOCKS || kb + 1 < A.kbs) product(rb, x + X_KB, false);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&B.empty[slot]);
-                if (++slot == EX_STAGES) {
-                    slot = 0;
-                    phase ^= 1u;
+                for (int i = 0; i < 2; i++) {
+                    const uint4 q = lds16(w + i * 512);
+                    e4m3x4_bf16(q.x, a[2 * i][0], a[2 * i][2]);
+                    e4m3x4_bf16(q.y, a[2 * i + 1][0], a[2 * i + 1][2]);
+                    e4m3x4_bf16(q.z, a[2 * i][1], a[2 * i][3]);
+                    e4m3x4_bf16(q.w, a[2 * i + 1][1], a[2 * i + 1][3]);
                 }
-                if constexpr (BLOCKS) {
 #pragma unroll
-                    for (int n = 0; n < NT8; n++) {
-                        if (n >= n8) break;
+                for (int n = 0; n < N8; n++) {
+                    uint32_t b[2][4];
+#pragma unroll
+                    for (int h = 0; h < 2; h++) ldsm4(b[h], x + n * 1024 + (((4 * h + piece) ^ sw) << 4));
+                    if (fresh) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 4; j++) mma16816(acc[n], a[j], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+                }
+            };
+#pragma unroll 1
+            for (int kb = 0; kb < A.kbs; kb += 2) {
+                ok = __all_sync(0xffffffffu, wait(B, A, &B.full[slot], phase, WP_FULL));               // the warp leaves together
+                if (!ok) break;
+                cp_wait<EX_AHEAD - 1>();
+                __syncwarp();
+                const uint32_t x = frag + 2 * slot * X_KB, w = ring + at + lane * 16;
+                product(w, x, BLOCKS);
+                if (BLOCKS || kb + 1 < A.kbs) product(w + 1024, x + X_KB, false);
+                if constexpr (BLOCKS) {
+                    const float2 sc = lds8(ring + at + 2048);
+#pragma unroll
+                    for (int n = 0; n < N8; n++) {
                         sums[n][0] = fmaf(acc[n][0], sc.x, sums[n][0]);
                         sums[n][1] = fmaf(acc[n][1], sc.x, sums[n][1]);
                         sums[n][2] = fmaf(acc[n][2], sc.y, sums[n][2]);
                         sums[n][3] = fmaf(acc[n][3], sc.y, sums[n][3]);
                     }
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&B.empty[slot]);
+                if (++slot == EX_STAGES) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+                if ((at += EX_PAIR) == EX_AHEAD * EX_PAIR) at = 0;
+                request();
             }
-            request2(ra, rb, sc);
+            if constexpr (!BLOCKS)
+#pragma unroll
+                for (int n = 0; n < N8; n++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) sums[n][i] = acc[n][i];
         };
-#pragma unroll 1
-        for (int kb = 0; kb < A.kbs && ok; kb += 4) {
-            pair(kb, raw[0], raw[1], scale[0]);
-            pair(kb + 2, raw[2], raw[3], scale[1]);
-        }
+        static_assert(NT8 == 4, "one case for every number of groups");
+        const int groups = __shfl_sync(0xffffffffu, (it.z + 7) >> 3, 0);
+        if (groups <= 1) products(std::integral_constant<int, 1>{});
+        else if (groups == 2) products(std::integral_constant<int, 2>{});
+        else if (groups == 3) products(std::integral_constant<int, 3>{});
+        else products(std::integral_constant<int, 4>{});
         if (!ok) {
             if (warp == 0) {                     // copies in flight must land before the CTA leaves (see rows_gemm)
                 const u64 t0 = mk::globaltimer();
@@ -1797,7 +1831,7 @@ static __global__ void __launch_bounds__(256, 2) experts_gemm(const __grid_const
                 for (int i = 0; i < 2; i++) {
                     const int tok = 8 * n + 2 * t + i;
                     if (tok >= it.z) continue;
-                    const float lo = (BLOCKS ? sums[n][i] : acc[n][i]) * rs0, hi = (BLOCKS ? sums[n][2 + i] : acc[n][2 + i]) * rs1;
+                    const float lo = sums[n][i] * rs0, hi = sums[n][2 + i] * rs1;
                     if (OUT == OUT_GLU) {            // rows 0-7 of a tile are gates, rows 8-15 their up rows
                         const int col = tile * 8 + g;
                         const float y = (A.gelu ? 0.5f * lo * (1.f + tanhf(0.7978845608028654f * (lo + 0.044715f * lo * lo * lo))) : silu_f(lo)) * hi;
@@ -1811,6 +1845,7 @@ static __global__ void __launch_bounds__(256, 2) experts_gemm(const __grid_const
         }
         it = next;
     }
+    mk::cp_async_wait_all();                       // (a warp that gave up has copies in flight)
 }
 
 // ---- expert routing --------------------------------------------------------------------------------------------

@@ -113,7 +113,7 @@ int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaSt
 // FP8 products of routed groups with at most 8 NT8 rows per work item; `items` bounds the number of items.
 template <bool BLOCKS, int NT8>
 int launch_experts(GemmArgs& A, int out, int items, int sms, cudaStream_t st) {
-    const int smem = EX_STAGES * 2 * NT8 * 8 * 128 + (int)sizeof(ExpertBars) + 1024;
+    const int smem = experts_smem(NT8);
     const long long units = (long long)items * A.blocks;
     auto fn = out == OUT_GLU ? experts_gemm<BLOCKS, OUT_GLU, NT8> : experts_gemm<BLOCKS, OUT_STORE, NT8>;
     MKP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
