@@ -56,7 +56,7 @@ enum {
     MK_L_KIND,          /* 0 = Gated DeltaNet, 1 = gated full attention (a value, not a pointer) */
     MK_L_CONV_HIST_B,   /* fp32 [batch, 16 heads, 384 channels, 8]: conv history of batched decoding (0 if unused) */
     MK_L_W_OUT_ROWS,    /* DeltaNet layers: out-projection in the row-slice layout, the batched kernel's copy (0 if unused) */
-    MK_L_W_DOWN_ROWS,   /* down-projection in the row-slice layout of the other matrices: the batched kernel's copy (0 if unused) */
+    MK_L_W_DOWN_ROWS,   /* down-projection in the row-slice layout of the other matrices: read by mk_prefill_weights, asked for by mk_launch_batch (0 if unused) */
     MK_LAYER_FIELDS
 };
 
@@ -73,7 +73,7 @@ enum {
     MK_G_XL,            /* u64 [tokens, hidden]        residual stream, (epoch<<32)|fp32 words */
     MK_G_PROJL,         /* u64 [tokens, in_rows_max]   input-projection output                 */
     MK_G_MIXL,          /* u64 [tokens, 2048]          mixer (DeltaNet / attention) output     */
-    MK_G_ACTL,          /* u64 [tokens, intermediate]  MLP activation: mk_launch_batch only (0: never batched) */
+    MK_G_ACTL,          /* u64 [tokens, intermediate]  MLP activation: asked for by mk_launch_batch only (0: never batched), no longer read or written */
     MK_G_LML,           /* u64 [tokens, grid, 2]       per-CTA LM-head winners                 */
     MK_G_ATTN_PART,     /* u64 [tokens, kv_heads, MK_MAX_SPLITS, MK_PART_STRIDE] split partials, flag-in-data words */
     MK_G_BLOCK_TABLE,   /* int32 [max_seq / MK_KV_BLOCK]: logical KV block -> physical block   */

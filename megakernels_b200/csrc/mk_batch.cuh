@@ -1,7 +1,7 @@
 // Batched decoding: up to eight independent sequences share every pass over the weights (int8 weights).
 //
 // The kernel keeps the structure of the single-sequence kernel (mk_decode.cuh): one resident CTA per
-// SM, a producer lane that streams this CTA's row slices through a shared-memory ring, flag-in-data
+// SM, a producer lane that streams this CTA's weight slices through a shared-memory ring, flag-in-data
 // words between ops.  What changes:
 //   * The eight sequences are the eight columns of the MMA B operand.  An input is x * 2^s rounded to a
 //     signed 24-bit integer and cut into three bytes (two's complement: the top byte signed, the lower

@@ -55,7 +55,7 @@ struct LayerP {
     const uint8_t* w_out;
     const uint8_t* w_gu;
     const uint8_t* w_down;        // single-sequence kernels: column slices per CTA in fragment order (pack_down_cols)
-    const uint8_t* w_down_rows;   // batched kernel: row slices per CTA (pack_rows)
+    const uint8_t* w_down_rows;   // row slices per CTA (pack_rows): source of the prompt path's operand; batched launches ask for it
     const uint8_t* w_out_rows;    // batched kernel, DeltaNet layers: row slices (single-sequence kernels: w_out holds column slices per task)
     const float* s_in;
     const float* s_out;
@@ -91,7 +91,7 @@ struct Params {
     unsigned long long* xl;
     unsigned long long* projl;
     unsigned long long* mixl;
-    unsigned long long* actl;
+    unsigned long long* actl;     // no kernel reads it any more; batched launches ask for it
     unsigned long long* lml;
     unsigned long long* attn_part;
     const int* block_table;

@@ -181,8 +181,8 @@ class Megakernel:
             rec = dict.fromkeys(F, 0)
             gu = torch.stack([w[m + "mlp.gate_proj.weight"], w[m + "mlp.up_proj.weight"]], dim=1).reshape(-1, cfg.hidden)
             rec["w_gu"], rec["s_gu"] = mat(gu, unit=2)
-            # the single-sequence kernels take the down-projection as column slices (the CTA that produces
-            # SwiGLU outputs multiplies them itself); the batched kernel takes row slices like every other matrix
+            # the kernels take the down-projection as column slices (the CTA that produces SwiGLU outputs
+            # multiplies them itself); the prompt path makes its operand from row slices, which int8 engines keep
             dm, ds = plain(w[m + "mlp.down_proj.weight"])
             rec["w_down"] = keep(pack_down_cols(dm, self.grid))
             rec["s_down"] = keep(ds) if ds is not None else 0
@@ -270,8 +270,7 @@ class Megakernel:
         g = dict.fromkeys(_lib.GLOBAL_FIELDS, 0)
         g.update(embed=embed_ptr, embed_scale=embed_scale, lm_head=lm_ptr, lm_scale=lm_scale,
                  final_norm=f32(self.final_norm), rope_cos=keep(cos), rope_sin=keep(sin),
-                 xl=keep(self.ll[0]), projl=keep(self.ll[1]), mixl=keep(self.ll[2]), actl=keep(self.ll[3]) if quant == "int8" else 0,      # only batched launches (int8 engines) hand activations over in words
-                
+                 xl=keep(self.ll[0]), projl=keep(self.ll[1]), mixl=keep(self.ll[2]), actl=keep(self.ll[3]) if quant == "int8" else 0,      # batched launches ask for them
                  lml=keep(self.ll[4]), attn_part=keep(self.attn_part),
                  block_table=keep(self.block_table), status=keep(self.status))
         g["xml"] = keep(self.ll[5])
