@@ -1423,6 +1423,29 @@ static __global__ void __launch_bounds__(256, 1) attn_rows(const __grid_constant
 // bf16 cache is one piece: three products).  32 query rows per CTA (a 500-token prompt is then one CTA per SM), blocks of 32
 // keys: warp (r, d) takes rows 16 r .. 16 r + 15, scores keys 8 d .. 8 d + 7 and accumulates head dims 64 d .. 64 d + 63.
 // The fp32 rows of the next block wait in registers.
+//   A block of keys takes 6 us, bound by the chain load - split - two products with a barrier each at one CTA per SM, and the last
+// rows see all of them.  So the CTAs of a cluster share a row block's keys (attn_splits), and the first one adds the others'
+// sums through distributed shared memory.
+__device__ __forceinline__ int cluster_size() { uint32_t v; asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v)); return (int)v; }
+__device__ __forceinline__ int cluster_rank() { uint32_t v; asm("mov.u32 %0, %%cluster_ctaid.x;" : "=r"(v)); return (int)v; }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float cluster_f1(const float* p, int rank) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr(p, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 cluster_f2(const float* p, int rank) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(cluster_addr(p, rank)) : "memory");
+    return v;
+}
 constexpr int AF_ROWS = 32, AF_KEYS = 32, AF_HD = 256, AF_RB = AF_HD * 2;
 template <bool KVF32> constexpr int attn_f32_smem() { return 3 * AF_ROWS * AF_RB + 2 * (KVF32 ? 3 : 1) * AF_KEYS * AF_RB + 3 * AF_ROWS * AF_KEYS * 2 + 8 * AF_ROWS * 4; }
 // Four consecutive columns c .. c + 3 of a row, as NP pieces of swizzled rows
@@ -1445,8 +1468,10 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
     uint8_t *q_s = sm, *k_s = q_s + 3 * QB, *v_s = k_s + KP * KB, *p_s = v_s + KP * KB;
     float* st_s = reinterpret_cast<float*>(p_s + 3 * PB);
     const int qpk = T.nq / T.nkv, bq = AF_ROWS / qpk;
-    const int m = blockIdx.z, kvh = blockIdx.y, l0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * bq;
+    const int ranks = cluster_size(), rank = cluster_rank();
+    const int m = blockIdx.z, kvh = blockIdx.y, l0 = ((int)(gridDim.x - 1 - blockIdx.x) / ranks) * bq;
     const int np = min(bq, T.L - l0), pos0 = T.pos[m] + l0, last = pos0 + np - 1;
+    const int share = (last / AF_KEYS + ranks) / ranks * AF_KEYS, first = rank * share, end = min(last + 1, first + share);    // this CTA's keys
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp & 1, dh = warp >> 1, g = lane >> 2, t = lane & 3;
     auto fetch = [&](const void* cache, int k0, float4 (&r)[PER]) {
 #pragma unroll
@@ -1468,7 +1493,7 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
         for (int i = 0; i < PER; i++) split4<KP>(dst, KB, (tid >> 6) + 4 * i, (tid & 63) * 4, r[i]);
     };
     float4 kr[PER];
-    fetch(T.k_cache, 0, kr);
+    fetch(T.k_cache, first, kr);
     for (int i = tid; i < AF_ROWS * AF_HD / 4; i += 256) {
         const int r = i / (AF_HD / 4), c = (i - r * (AF_HD / 4)) * 4, p = r / qpk, hq = r - p * qpk;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1483,7 +1508,7 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
     for (int i = 0; i < 2; i++) qp[i] = pos0 + min((16 * rg + g + 8 * i) / qpk, np - 1);
     const uint32_t qa = smem_u32(q_s) + (uint32_t)(16 * rg + (lane & 15)) * AF_RB, qx = lane & 7;
 #pragma unroll 1
-    for (int k0 = 0; k0 <= last; k0 += AF_KEYS) {
+    for (int k0 = first; k0 < end; k0 += AF_KEYS) {
         __syncthreads();                                                 // everybody is done with the previous block
         place(k_s, kr);
         float4 vr[PER];
@@ -1555,7 +1580,7 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
             o[i][2] *= f[1]; o[i][3] *= f[1];
         }
         place(v_s, vr);
-        if (k0 + AF_KEYS <= last) fetch(T.k_cache, k0 + AF_KEYS, kr);
+        if (k0 + AF_KEYS < end) fetch(T.k_cache, k0 + AF_KEYS, kr);
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < AF_KEYS / 16; kk++) {
@@ -1589,9 +1614,52 @@ static __global__ void __launch_bounds__(256, 1) attn_rows_f32(const __grid_cons
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < 2; r++) {
+        const int rr = 16 * rg + g + 8 * r;
+        sum[r] = (st_s[4 * AF_ROWS + rr] + st_s[5 * AF_ROWS + rr]) + (st_s[6 * AF_ROWS + rr] + st_s[7 * AF_ROWS + rr]);
+    }
+    if (ranks > 1) {                             // the first CTA adds the others' sums to its own
+        float* part = reinterpret_cast<float*>(k_s);
+        constexpr int PR = AF_HD + 8;            // padded against bank conflicts
+        static_assert(AF_ROWS * PR * 4 <= 2 * KP * KB + 3 * PB, "K, V and probabilities are read by now");
+        if (rank) {
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int rr = 16 * rg + g + 8 * r;
+#pragma unroll
+                for (int n = 0; n < AF_HD / 32; n++)
+                    *reinterpret_cast<float2*>(part + rr * PR + dh * (AF_HD / 4) + 8 * n + 2 * t) = make_float2(o[n][2 * r], o[n][2 * r + 1]);
+                if (dh == 0 && t == 0) st_s[rr] = mx[r];
+                if (dh == 1 && t == 0) st_s[AF_ROWS + rr] = sum[r];
+            }
+        }
+        cluster_sync();
+        if (rank == 0) {
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int rr = 16 * rg + g + 8 * r;
+#pragma unroll 1
+                for (int c = 1; c < ranks; c++) {
+                    const float2 ms = make_float2(cluster_f1(st_s + rr, c), cluster_f1(st_s + AF_ROWS + rr, c));
+                    const float nm = fmaxf(mx[r], ms.x), f = __expf(mx[r] - nm), fc = __expf(ms.x - nm);
+                    mx[r] = nm;
+                    sum[r] = fmaf(sum[r], f, ms.y * fc);
+#pragma unroll
+                    for (int n = 0; n < AF_HD / 32; n++) {
+                        const float2 v = cluster_f2(part + rr * PR + dh * (AF_HD / 4) + 8 * n + 2 * t, c);
+                        o[n][2 * r] = fmaf(o[n][2 * r], f, v.x * fc);
+                        o[n][2 * r + 1] = fmaf(o[n][2 * r + 1], f, v.y * fc);
+                    }
+                }
+            }
+        }
+        cluster_sync();                          // their shared memory has been read
+        if (rank) return;
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
         const int rr = 16 * rg + g + 8 * r, p = rr / qpk, hq = kvh * qpk + rr - p * qpk;
         if (p >= np) continue;
-        const float inv = 1.f / ((st_s[4 * AF_ROWS + rr] + st_s[5 * AF_ROWS + rr]) + (st_s[6 * AF_ROWS + rr] + st_s[7 * AF_ROWS + rr]));
+        const float inv = 1.f / sum[r];
         const int row = m * T.L + l0 + p;
         const float* gate = T.y + (size_t)row * T.y_stride + T.q_off + (size_t)hq * T.q_hs + T.gate_off;
 #pragma unroll

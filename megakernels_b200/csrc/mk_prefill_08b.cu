@@ -232,15 +232,17 @@ struct Run {
                 T.max_pages = P->max_seq / mk::KV_BLOCK; T.kv_shift = 6;
                 T.s_page = S::NKV * mk::KV_BLOCK * S::HD; T.s_head = mk::KV_BLOCK * S::HD; T.s_pos = S::HD;
                 T.pos = pos; T.q = q; T.out = mix; T.out_piece = mix_piece; T.out_rows = xrows;
-                const dim3 pg((S::NQ + 2 * S::NKV + 7) / 8, rows), ag((rows + AF_ROWS / S::QPK - 1) / (AF_ROWS / S::QPK), S::NKV, 1);
+                const dim3 pg((S::NQ + 2 * S::NKV + 7) / 8, rows), blocks((rows + AF_ROWS / S::QPK - 1) / (AF_ROWS / S::QPK), S::NKV, 1);
+                const int splits = attn_splits(blocks.x * blocks.y, start + rows, sms);
+                const dim3 ag(blocks.x * splits, blocks.y, 1);
                 if (kv32) {
                     MKP_CUDA(launch((attn_prepare<256, true, true>), pg, 256, 0, st, T));
                     MKP_CUDA(cudaFuncSetAttribute(attn_rows_f32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_f32_smem<true>()));
-                    MKP_CUDA(launch(attn_rows_f32<true>, ag, 256, attn_f32_smem<true>(), st, T));
+                    MKP_CUDA(launch_cluster(attn_rows_f32<true>, ag, 256, attn_f32_smem<true>(), splits, st, T));
                 } else {
                     MKP_CUDA(launch((attn_prepare<256, true, false>), pg, 256, 0, st, T));
                     MKP_CUDA(cudaFuncSetAttribute(attn_rows_f32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_f32_smem<false>()));
-                    MKP_CUDA(launch(attn_rows_f32<false>, ag, 256, attn_f32_smem<false>(), st, T));
+                    MKP_CUDA(launch_cluster(attn_rows_f32<false>, ag, 256, attn_f32_smem<false>(), splits, st, T));
                 }
             } else {
                 GdnArgs G;

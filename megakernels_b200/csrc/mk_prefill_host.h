@@ -42,6 +42,25 @@ inline cudaError_t launch(Kernel fn, dim3 grid, int threads, size_t smem, cudaSt
     return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
+// The same in clusters of `ranks` CTAs along x.
+template <class Kernel, class... Args>
+inline cudaError_t launch_cluster(Kernel fn, dim3 grid, int threads, size_t smem, int ranks, cudaStream_t st, const Args&... args) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = ranks;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
 constexpr int SMEM_MAX = 232448;
 constexpr int DRAIN_GROUPS = 4;                     // rows_gemm: three-piece products in tiles of up to 32 x 4 tokens
 constexpr int MAX_ROWS = 65535;                     // token rows of a call: one grid coordinate of several kernels
@@ -108,6 +127,17 @@ int launch_gemm(GemmArgs& A, int out, int blocks, int tiles_x, int items, cudaSt
         MKP_CUDA(cudaGetLastError());
     }
     return MK_OK;
+}
+
+// CTAs that share a row block's keys in attn_rows_f32: `ctas` row blocks, the longest sees `keys` keys.  While the SMs have room
+// for all of them, two blocks of keys each are enough; up to two CTAs per SM, one after the other, pay where the longest share is four
+// blocks (they even out the causal triangle).  Passes of the int8 model without and with, ms: 120 rows (2 each) 2.82 / 2.78, 250 (2)
+// 3.32 / 3.22 (with 4 3.27), 400 (2) 4.64 / 4.50, 511 (2) 5.06 / 4.91; no room: 600 with 2 all the same 5.82 / 5.75, 1000 8.28 / 8.43.
+inline int attn_splits(int ctas, int keys, int sms) {
+    const int blocks = (keys + AF_KEYS - 1) / AF_KEYS;
+    int s = 1;
+    while (s < 8 && ((2 * s * ctas <= sms && blocks >= 4 * s) || (2 * s * ctas <= 2 * sms && blocks >= 8 * s))) s *= 2;
+    return s;
 }
 
 // FP8 products of routed groups with at most 8 NT8 rows per work item; `items` bounds the number of items.

@@ -147,6 +147,26 @@ def test_small_model_prompt_equals_stepping(small, monkeypatch, quant, kv, lengt
         assert rel(a.mtp_k_cache, b.mtp_k_cache) < 50 * tol and a.mtp_h[0] == b.mtp_h[0]
 
 
+@pytest.mark.parametrize("kv,context,length", [("fp32", 0, 130), ("fp32", 310, 20), ("fp32", 500, 17), ("bf16", 500, 17)])
+def test_small_model_rows_share_their_keys(small, monkeypatch, kv, context, length):
+    """Row blocks whose keys are shared by 2, 4 and 8 CTAs: whole shares, a last one that is short, and two empty ones."""
+    from megakernels_b200 import engine as E
+    from megakernels_b200.synth import make_prompt
+    prompt, got = make_prompt(small[0], context + length), []
+    for rows in (True, False):
+        mk = E.Megakernel(small[:2], max_seq=576, quant="int8", kv_dtype=kv)
+        with monkeypatch.context() as mp:
+            mp.setattr(E, "MIN_PROMPT_ROWS", 1 << 30)
+            if context:
+                mk.run(prompt[:context])
+            mp.setattr(E, "MIN_PROMPT_ROWS", 16 if rows else 1 << 30)
+            mp.setattr(E, "EXACT_PROMPT", 0)
+            got.append(mk.run(prompt[context:], n_generate=4, return_logits=True))
+        assert (mk._workspace is not None) == rows
+    (ia, la), (ib, lb) = got
+    assert ia == ib and rel(la, lb) < (2e-5 if kv == "fp32" else 2e-4)              # a bf16 cache rounds
+
+
 def test_small_model_batched_prompts_equal_stepping(small, monkeypatch):
     from megakernels_b200 import engine as E
     from megakernels_b200.synth import make_prompt
