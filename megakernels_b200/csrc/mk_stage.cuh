@@ -377,16 +377,15 @@ __device__ __forceinline__ const uint8_t* split_weights(const Shared& S, const G
     }
     return group_weights(S, g, grp) + (size_t)((tile * g.S + seg) * g.n_chunks) * g.chunk_bytes;
 }
-constexpr int FEW_WARPS = 8;
+constexpr int FEW_WARPS = 4;
 // Warp w's share of a batch.
 __device__ __forceinline__ Share batch_share(const Shared& S, const Geo& g, const Batch& bt, int w) {
     Share r;
     r.cpt = (bt.seg1 - bt.seg0) * g.n_chunks;
     // Equal shares of whole chunks, the first warps first: as long as the longest share is no longer, every warp without one
-    // is a partial tile less to add.  Fewer chunks than warps go to FEW_WARPS: two chunks in a row cost less than the exchange,
-    // four no longer do where a stage is one tile of a small matrix.  (Per step, 8 and 6 layers: both rules with 4 warps 27B x1
-    // 1417 -> 1373 us, x8 1699 -> 1656 us, 35B-A3B x8 1531 -> 1493 us, 26B x4 1419 -> 1413 us.  8 or 16 warps instead of 4, ratio
-    // of speeds: 27B x1 1.000 and 0.998, x8 1.000 and 0.998, 35B-A3B x8 1.007 and 1.008, 26B x4 0.999 and 0.995.)
+    // is a partial tile less to add.  Fewer chunks than warps go to FEW_WARPS: two or three chunks in a row cost less than
+    // the exchange.  (Both rules together, 8 and 6 layers: 27B x1 per step 1417 -> 1373 us, x8 1699 -> 1656 us, 35B-A3B x8
+    // 1531 -> 1493 us, 26B x4 1419 -> 1413 us; the second one's own part was not measured.)
     const int n = (bt.t1 - bt.t0) * r.cpt, warps = n < NCW && n > FEW_WARPS ? FEW_WARPS : NCW;
     r.per = (n + warps - 1) / warps;
     r.c = min(n, w * r.per);
