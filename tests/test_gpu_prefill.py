@@ -323,8 +323,8 @@ def test_small_model_prompts_are_as_exact_as_stepping(small, monkeypatch, quant,
 
 @pytest.mark.parametrize("model,M,length", [("26b", 5, 30), ("26b", 8, 50), ("26b", 8, 101), ("26b", 8, 200), ("35b", 8, 49), ("35b", 8, 101), ("35b", 8, 200)])
 def test_prompt_rows_of_crowded_experts(model, M, length):
-    """Routed products by the width of a work item (the mean load of 128 experts: 32, 64, 128 and 256 tokens; block-scaled ones at
-    most 128, several items an expert); 26b: 11 blocks of 64 columns in the down-projection, the last weight block past the matrix."""
+    """Routed products by the width of a work item (the mean load of 128 experts: 32, 64, 128 and 256 tokens; block-scaled ones up to a
+    mean of 96 in items of 32, several an expert); 26b: 11 blocks of 64 columns in the down-projection, the last weight block past the matrix."""
     pkg, shape = SHAPES[model]
     shape = shape.with_(eff=704, hidden=576) if model == "26b" else shape.with_(experts=128)
     PK = pkg.Packed(pkg.SynthWeights(shape, layers=shape.layers, init="realistic", device="cuda"), "cuda")
