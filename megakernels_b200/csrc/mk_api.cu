@@ -112,8 +112,10 @@ extern "C" int mk_create(const mk_model_desc* d, mk_engine** out) {
     if (d->max_batch < 0 || d->max_batch > MK_MAX_BATCH) return fail(MK_ERR_BADARG, "mk_create: max_batch %d out of [0, %d]", d->max_batch, (int)MK_MAX_BATCH);
     if ((int64_t)(d->max_batch > 1 ? d->max_batch : 1) * (d->max_seq / KV_BLOCK) > MAX_BLOCKS)
         return fail(MK_ERR_BADARG, "mk_create: %d sequences of %d positions need more than %d KV pages", d->max_batch, d->max_seq, MAX_BLOCKS);
+    if (d->grid > MAX_GRID) return fail(MK_ERR_BADARG, "mk_create: grid %d, the kernels take %d CTAs at most", d->grid, MAX_GRID);
     int n_sm = 0;
     MK_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d->device));
+    if (d->grid == 0 && n_sm > MAX_GRID) return fail(MK_ERR_BADARG, "mk_create: %d SMs, pack for a grid of %d CTAs at most", n_sm, MAX_GRID);
     if (d->grid < 0 || d->grid > n_sm) return fail(MK_ERR_BADARG, "mk_create: grid %d exceeds the %d SMs (every CTA must be resident)", d->grid, n_sm);
     mk_engine* e = new mk_engine();
     e->desc = *d;

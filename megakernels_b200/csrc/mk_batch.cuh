@@ -602,7 +602,7 @@ __device__ __forceinline__ bool run_layer_b(Ctx& c, const Params& P, const Layer
         const int c0 = half ? (c.grid + 1) / 2 : 0, c1 = half ? c.grid : (c.grid + 1) / 2;
 #pragma unroll 1
         for (int r = c.warp >> 1; r < rows; r += NCW / 2) {
-            constexpr int PER = 10;                          // grids of up to 160 CTAs
+            constexpr int PER = (MAX_GRID + 15) / 16;            // (of the larger half)
             const u64* src = down_words(P, nb) + ((size_t)(c0 + (c.lane >> 2)) * S::HID + xr0 + r) * nbp + 2 * t;
             const size_t stride = (size_t)8 * S::HID * nbp;
             const int n = 2 * t < nbp ? (c1 - c0 - (c.lane >> 2) + 7) >> 3 : 0;      // words of this lane

@@ -17,6 +17,7 @@ constexpr int MAX_SPLITS = 128;           // attention split-K chunks per KV hea
 constexpr int MAX_CHUNK_POS = 448;        // positions one attention task scans at most
 constexpr int MAX_LM_ROWS = 1 << 20;      // LM-head rows one CTA can own (no per-CTA staging limits it)
 constexpr int MAX_BODY_ROWS = 64;         // rows of a layer GEMV one CTA can own
+constexpr int MAX_GRID = 160;             // CTAs whose partial sums a warp adds: whole words per lane, all of them requested at once
 constexpr int OPS_PER_LAYER = 5;
 #ifdef MK_TRACE
 constexpr int PROF_FIELDS = 12;         // + fine-grained marks of a trace build

@@ -1511,7 +1511,7 @@ __device__ __forceinline__ bool run_layer(Ctx& c, const Params& P, const LayerP&
         own_rows<T>(c, xr0, xr1, [&](int j, int row, bool a_own, bool b_own) {
             const float rs0 = Q8 && a_own ? L.s_down[row] : 1.0f, rs1 = Q8 && b_own ? L.s_down[row + 1] : 1.0f;   // requested before the wait
             // lane l takes CTAs l, l + 32, ...; fixed order, then the shuffle tree
-            constexpr int PER = 5;                          // grids of up to 160 CTAs
+            constexpr int PER = (MAX_GRID + 31) / 32;
             const u64* src = P.partl + (size_t)j * c.grid * S::HID + row + (size_t)c.lane * S::HID;
             u64 w[PER][2];
 #pragma unroll

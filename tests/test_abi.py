@@ -99,6 +99,9 @@ def test_bad_arguments_are_refused_without_a_gpu(lib_built):
         desc = _lib.ModelDesc(**d)
         assert lib.mk_create(ctypes.byref(desc), ctypes.byref(h)) == _lib.MK_ERR_BADARG, kw
         assert b"max_batch" in lib.mk_last_error() or b"KV pages" in lib.mk_last_error()
+    # more CTAs than the kernels add partial sums of
+    desc = _lib.ModelDesc(shape=_lib.MK_SHAPE_QWEN35_08B, n_layers=4, vocab=4096, max_seq=64, quant=1, kv_dtype=1, draft_vocab=0, device=0, grid=161)
+    assert lib.mk_create(ctypes.byref(desc), ctypes.byref(h)) == _lib.MK_ERR_BADARG and b"160" in lib.mk_last_error()
     assert lib.mk_launch(None, None, None) == _lib.MK_ERR_BADARG
     assert lib.mk_launch_batch(None, None, None) == _lib.MK_ERR_BADARG
     assert lib.mk_destroy(None) == _lib.MK_OK
