@@ -264,3 +264,28 @@ def test_attention_tasks_of_any_size_equal_a_sequence_alone(tiny, batch, length,
         assert ids[j] == one
         # integer products, fp32 sums in another order
         assert float((logits[j].double() - want.double()).norm() / want.double().norm()) < 2e-5
+
+
+@pytest.mark.parametrize("batch", [1, 2, 3, 7])
+def test_hand_off_words_stay_inside_their_buffers(tiny, batch, lib_built):
+    """Buffers of exactly the sizes mk_b200.h gives them, with a pattern behind: partial projection sums of one token (a host that never
+    speculates), split partials of `batch` sequences."""
+    from megakernels_b200 import _lib
+    cfg, w = tiny
+    prompts = [make_prompt(cfg, 40 - 3 * j, seed=100 + j) for j in range(batch)]
+    want = engine(cfg, w, batch=batch).run_batch(prompts, n_generate=6, return_logits=True)
+    mk = engine(cfg, w, batch=batch)
+    sizes = dict(partl=mk.grid * cfg.hidden, attn_part=batch * cfg.n_kv_heads * _lib.query("MAX_SPLITS") * _lib.query("PART_STRIDE"))
+    guarded, spare = {}, 1 << 20
+    for name, n in sizes.items():
+        guarded[name] = torch.full((n + spare,), 0x5A5A5A5A, dtype=torch.int64, device=mk.device)
+        guarded[name][:n] = 0
+    layers, _, g = mk._tables
+    g = dict(g, **{name: t.data_ptr() for name, t in guarded.items()})
+    lv, gv = _lib.i64_array(layers), _lib.i64_array([g[f] for f in _lib.GLOBAL_FIELDS])
+    _lib.check(mk.lib.mk_set_params(mk._h, lv, len(lv), None, 0, gv, len(gv)))
+    ids, logits = mk.run_batch(prompts, n_generate=6, return_logits=True)
+    assert ids == want[0] and all(torch.equal(a, b) for a, b in zip(logits, want[1]))
+    for name, n in sizes.items():
+        assert bool((guarded[name][n:] == 0x5A5A5A5A).all()), name
+    assert not bool(guarded["partl"][: sizes["partl"]].any())          # no hand-off of a batched launch
