@@ -76,14 +76,14 @@ enum {
     MK_G_ACTL,          /* u64 [tokens, intermediate]  MLP activation: asked for by mk_launch_batch only (0: never batched), no longer read or written */
     MK_G_LML,           /* u64 [tokens, grid, 2]       per-CTA LM-head winners                 */
     MK_G_ATTN_PART,     /* u64 [tokens, kv_heads, MK_MAX_SPLITS, MK_PART_STRIDE] split partials, flag-in-data words;
-                           mk_launch_batch also hands its partial down-projection sums over in it */
+                           mk_launch_batch hands its partial down-projection sums over in it too */
     MK_G_BLOCK_TABLE,   /* int32 [max_seq / MK_KV_BLOCK]: logical KV block -> physical block   */
     MK_G_STATUS,        /* int32 [4]: [0] error code of the first wait that ran out, [1] where */
     MK_G_MTP_FC, MK_G_MTP_FC_SCALE, MK_G_MTP_NORM_E, MK_G_MTP_NORM_H, MK_G_MTP_NORM,
     MK_G_DRAFT_HEAD, MK_G_DRAFT_SCALE, MK_G_DRAFT_IDS,
     MK_G_XML,           /* u64 [tokens, hidden] MTP residual stream                            */
     MK_G_PARTL,         /* u64 [tokens, grid, hidden] partial projection sums of every CTA; tokens = 2 for speculative
-                           cycles, else 1 (mk_launch_batch does not use it) */
+                           cycles, else 1 (mk_launch_batch uses it for a batch of one only) */
     MK_GLOBAL_FIELDS
 };
 

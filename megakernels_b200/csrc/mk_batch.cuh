@@ -405,16 +405,22 @@ __device__ void producer_batch(Ctx& c, const Params& P, const BatchArgs& A) {
     pr.drain();
 }
 
-// Partial down-projections are handed over as words [cta][row][sequences, one or an even number].  They share the attention partials'
-// buffer (attn_part), which is large enough for any number of sequences: either op writes only after every CTA has read what the other left there
-// (between them lie the exchanges of the residual that all CTAs take part in).
-__device__ __forceinline__ int down_stride(int nb) { return nb > 1 ? (nb + 1) & ~1 : 1; }
+// Partial down-projections are handed over as words [cta][row][sequences, an even number].  From two sequences on they share the attention
+// partials' buffer, which is large enough: either op writes only after every CTA has read what the other left there (between them lie
+// the exchanges of the residual that all CTAs take part in).  Of one sequence's buffers neither is large enough alone, so
+// the first half of the CTAs has its words where single-sequence launches have theirs.  (A word per row instead, for
+// one sequence, cost every larger batch 1 % of a step in registers and branches; pointers from the host 2 to 3 %.)
 template <class S>
-constexpr bool down_words_fit() {       // one sequence, two, and three, which have most padding
+__device__ __forceinline__ u64* down_words(const Params& P, int nb, int grid, int cta) {
+    const int half = nb > 1 ? 0 : grid / 2;
+    return cta < half ? P.partl + (size_t)cta * (2 * S::HID) : P.attn_part + (size_t)(cta - half) * S::HID * ((nb + 1) & ~1);
+}
+template <class S>
+constexpr bool down_words_fit() {       // the larger half of one sequence's; two sequences; three, which have most padding
     constexpr size_t ROWS = (size_t)MAX_GRID * S::HID, PER = (size_t)S::NKV * MAX_SPLITS * S::PART_STRIDE;
     return ROWS <= PER && ROWS * 2 <= PER * 2 && ROWS * 4 <= PER * 3;
 }
-static_assert(down_words_fit<Qwen35_08B>(), "the largest grid");
+static_assert(down_words_fit<Qwen35_08B>() && MAX_GRID % 2 == 0, "the largest grid");
 
 // The batched partial_cols: `act` ([NB][DOWN_K] in shared memory, zero past the CTA's slice) times the CTA's column slice of the
 // down-projection: 1024 partial sums per sequence.  Handing activations over instead would have every CTA read all 3584 of
@@ -468,13 +474,8 @@ __device__ __forceinline__ void partial_cols_b(Ctx& c, const float* act, u64* ou
         for (int k = 0; k < 4; k++) v[k] = fmaf((float)ci[2][k], 65536.f, fmaf((float)ci[1][k], 256.f, (float)ci[0][k])) * ((k & 1) ? is1 : is0);
         if (2 * t < nbp) {
             u64* dst = out + (size_t)(tile * 16 + g) * nbp + 2 * t;
-            if (nbp == 1) {
-                ll_store(dst, epoch, v[0]);
-                ll_store(dst + 8, epoch, v[2]);
-            } else {
-                ll_store2(dst, epoch, v[0], v[1]);
-                ll_store2(dst + (size_t)8 * nbp, epoch, v[2], v[3]);
-            }
+            ll_store2(dst, epoch, v[0], v[1]);
+            ll_store2(dst + (size_t)8 * nbp, epoch, v[2], v[3]);
         }
     }
     __syncwarp();
@@ -600,32 +601,29 @@ __device__ __forceinline__ bool run_layer_b(Ctx& c, const Params& P, const Layer
             const float up = __shfl_down_sync(0xffffffffu, v, 1);
             if (ok && !(lane & 1)) c.sm.act_s[j * DOWN_K + ((row - r0) >> 1)] = silu_f(v) * up;
         });
-        partial_cols_b<S>(c, c.sm.act_s, P.attn_part + (size_t)c.cta * S::HID * down_stride(nb), down_stride(nb), eD);
+        partial_cols_b<S>(c, c.sm.act_s, down_words<S>(P, nb, c.grid, c.cta), (nb + 1) & ~1, eD);
         prof_stamp(c, op, 3);
     }
     // ---- E: sum of the CTAs' partial down-projections + residual, for the rows this CTA owns
     bool failed;
     {
         // Two warps per row, half of the CTAs each: eight CTAs per request, four lanes with two sequences each
-        const int op = op0 + 4, rows = xr1 - xr0, nbp = down_stride(nb), half = c.warp & 1, t = c.lane & 3;
+        const int op = op0 + 4, rows = xr1 - xr0, nbp = (nb + 1) & ~1, half = c.warp & 1, t = c.lane & 3;
         prof_stamp(c, op, 0);
         const float rs = c.tid < rows * NB ? L.s_down[xr0 + (c.tid >> 3)] : 0.f;      // requested before the wait
-        const int c0 = half ? (c.grid + 1) / 2 : 0, c1 = half ? c.grid : (c.grid + 1) / 2;
+        const int c0 = half ? c.grid / 2 : 0, c1 = half ? c.grid : c.grid / 2;
+        const u64* words = down_words<S>(P, nb, c.grid, c0);
 #pragma unroll 1
         for (int r = c.warp >> 1; r < rows; r += NCW / 2) {
             constexpr int PER = (MAX_GRID + 15) / 16;            // (of the larger half)
-            const u64* src = P.attn_part + ((size_t)(c0 + (c.lane >> 2)) * S::HID + xr0 + r) * nbp + 2 * t;
+            const u64* src = words + ((size_t)(c.lane >> 2) * S::HID + xr0 + r) * nbp + 2 * t;
             const size_t stride = (size_t)8 * S::HID * nbp;
             const int n = 2 * t < nbp ? (c1 - c0 - (c.lane >> 2) + 7) >> 3 : 0;      // words of this lane
             u64 w[PER][2];
-            auto load = [&](int i) {
-                if (nbp == 1) w[i][0] = ll_load(src + i * stride);
-                else ll_load2(src + i * stride, w[i][0], w[i][1]);
-            };
 #pragma unroll
             for (int i = 0; i < PER; i++) {
                 w[i][0] = w[i][1] = (u64)eD << 32;           // (no word: a zero)
-                if (i < n) load(i);
+                if (i < n) ll_load2(src + i * stride, w[i][0], w[i][1]);
             }
             Spin sp;
             while (true) {
@@ -634,7 +632,7 @@ __device__ __forceinline__ bool run_layer_b(Ctx& c, const Params& P, const Layer
                 for (int i = 0; i < PER; i++)
                     if ((uint32_t)(w[i][0] >> 32) != eD || (uint32_t)(w[i][1] >> 32) != eD) {
                         ok = false;
-                        load(i);
+                        ll_load2(src + i * stride, w[i][0], w[i][1]);
                     }
                 if (ok) break;
                 if (MK_SPIN_FAIL(c, sp, W_ACT)) {

@@ -288,4 +288,3 @@ def test_hand_off_words_stay_inside_their_buffers(tiny, batch, lib_built):
     assert ids == want[0] and all(torch.equal(a, b) for a, b in zip(logits, want[1]))
     for name, n in sizes.items():
         assert bool((guarded[name][n:] == 0x5A5A5A5A).all()), name
-    assert not bool(guarded["partl"][: sizes["partl"]].any())          # no hand-off of a batched launch
