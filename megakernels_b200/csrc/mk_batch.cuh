@@ -407,9 +407,10 @@ __device__ void producer_batch(Ctx& c, const Params& P, const BatchArgs& A) {
 
 // Partial down-projections are handed over as words [cta][row][sequences, an even number].  From two sequences on they share the attention
 // partials' buffer, which is large enough: either op writes only after every CTA has read what the other left there (between them lie
-// the exchanges of the residual that all CTAs take part in).  Of one sequence's buffers neither is large enough alone, so
-// the first half of the CTAs has its words where single-sequence launches have theirs.  (A word per row instead, for
-// one sequence, cost every larger batch 1 % of a step in registers and branches; pointers from the host 2 to 3 %.)
+// the exchanges of the residual that all CTAs take part in; a step without an LM head ends with a wait for its own).
+//   Of one sequence's buffers neither is large enough alone, so the first half of the CTAs has its words where single-sequence launches
+// have theirs.  (A word per row instead, for one sequence, cost every larger batch 1 % of a step in registers and branches; pointers
+// from the host 2 to 3 %.)
 template <class S>
 __device__ __forceinline__ u64* down_words(const Params& P, int nb, int grid, int cta) {
     const int half = nb > 1 ? 0 : grid / 2;
@@ -830,6 +831,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) batch_kernel(const __grid_constan
             }
             prof_stamp(c, NL5, 3);
             if (consumer_any(c.dead)) break;
+        } else {
+            wait_residual_b<S>(c, P.xl, e0 + (uint32_t)NL5 - 1, nb, x);      // no exchange ends this step (see decode_kernel)
         }
         steps_done = s + 1;
     }

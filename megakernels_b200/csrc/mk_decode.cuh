@@ -1733,6 +1733,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
             if (s >= A.lm_from) {
                 float* logits = A.logits_out ? A.logits_out + (size_t)s * P.vocab : nullptr;
                 if (lm_head(e0 + (uint32_t)OPS - 1, NL5, pos, logits, x, hn)) break;
+            } else {
+                // No exchange that every CTA takes part in ends this step, and the next one's first layer writes partial sums where a slow
+                // CTA may still read this one's: wait for its residual, published behind the last read.  (A residual word is
+                // overwritten only when every CTA is past this wait: the first layer's needs all of its in-projection.)
+                const u64* base = P.xl + 2 * c.tid;
+                float v[2];
+                ll_wait_pairs_fn<1>(c, [&](int) { return base; }, [&](int) { return e0 + (uint32_t)NL5 - 1; }, v, W_X);
             }
             steps_done = s + 1;
         }

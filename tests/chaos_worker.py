@@ -43,6 +43,18 @@ def main():
     ids, logits = mk.run_batch([make_prompt(cfg, n, seed=20 + j) for j, n in enumerate((9, 4, 6, 2))], n_generate=8, return_logits=True)
     out["batch_int8"] = digest(*[torch.tensor(x) for x in ids], *logits)
     del mk
+    # prompts that step through a first layer of either kind: steps that end without an LM head
+    import dataclasses
+    first = dataclasses.replace(cfg, n_layers=2, layer_types=["full_attention", "linear_attention"])
+    mk = Megakernel((first, make_weights(first, 0, init="realistic")), max_seq=128, quant="int8", batch=3)
+    ids, logits = mk.run_batch([make_prompt(cfg, 15, seed=30 + j) for j in range(3)], n_generate=2, return_logits=True)
+    out["batch_int8_attention_first"] = digest(*[torch.tensor(x) for x in ids], *logits, mk.deltanet_state(0, seq=2))
+    del mk
+    thin = dataclasses.replace(cfg, n_layers=1, layer_types=["linear_attention"])
+    mk = Megakernel((thin, make_weights(thin, 0, init="realistic")), max_seq=128, quant="int8")
+    ids, logits = mk.run(make_prompt(cfg, 15, seed=40), n_generate=2, return_logits=True)
+    out["run_int8_one_layer"] = digest(ids, logits, mk.deltanet_state(0))
+    del mk
     # ---- the stage machine: dense hybrid with K splits, and the MoE hybrid with routed groups, eight sequences
     from megakernels_b200 import qwen27b, qwen35moe
     s27 = qwen27b.FULL.with_(hidden=1024, ffn=2048, vocab=4096, layers=4, nkh=4, nvh=12, nq=8, nkv=2)

@@ -288,3 +288,25 @@ def test_hand_off_words_stay_inside_their_buffers(tiny, batch, lib_built):
     assert ids == want[0] and all(torch.equal(a, b) for a, b in zip(logits, want[1]))
     for name, n in sizes.items():
         assert bool((guarded[name][n:] == 0x5A5A5A5A).all()), name
+
+
+def test_stepped_prompts_behind_a_first_layer_of_attention(lib_built):
+    """Steps of a prompt run no LM head, so only the residual separates one step's down-projection sums from the next step's attention
+    partials in the same words: many such steps in a row, against the oracle."""
+    import dataclasses
+    from oracle.decoder import pick_token
+    cfg = dataclasses.replace(qwen35_08b(n_layers=2, vocab=4096), layer_types=["full_attention", "linear_attention"])
+    w = make_weights(cfg, 0, init="realistic")
+    mk = engine(cfg, w, batch=4)
+    prompts = [make_prompt(cfg, 15, seed=50 + j) for j in range(4)]
+    ids, logits = mk.run_batch(prompts, n_generate=4, return_logits=True)
+    for j, prompt in enumerate(prompts):
+        dec = oracle(cfg, w)
+        for t in prompt[:-1]:
+            dec.step(t)
+        ref = dec.step(prompt[-1])
+        for i, got in enumerate(ids[j]):
+            assert float((logits[j][i].cpu() - ref).abs().max()) < LOGIT_TOL, (j, i)
+            assert got == pick_token(ref), (j, i)
+            if i + 1 < len(ids[j]):
+                ref = dec.step(got)
