@@ -60,7 +60,7 @@ enum {
     MK_LAYER_FIELDS
 };
 
-/* Field order of the model-wide pointer record (MK_GLOBAL_FIELDS int64 values).
+/* Field order of the model-wide pointer record (MK_GLOBAL_FIELDS int64 values).  Buffers of words (u64) start on 16 bytes.
  * Replaces the 20-entry list of qwen3.5-0.8b/csrc/binding.cpp:47-66. */
 enum {
     MK_G_EMBED = 0,     /* token embedding table, plain row-major [vocab, hidden], int8 or bf16 */

@@ -193,7 +193,7 @@ extern "C" int mk_set_params(mk_engine* e, const int64_t* layers, int64_t n_laye
             return fail(MK_ERR_BADARG, "activation word buffers null or not 16-byte aligned (all of them, or none for a static-only engine)");
         // the MLP activation words are a hand-off of the batched kernel only: mk_launch_batch refuses an engine without them
         if (p.actl != nullptr && bad16(p.actl)) return fail(MK_ERR_BADARG, "MLP activation words not 16-byte aligned");
-        if (!p.attn_part) return fail(MK_ERR_BADARG, "attention scratch missing");
+        if (bad16(p.attn_part)) return fail(MK_ERR_BADARG, "attention scratch null or not 16-byte aligned");
     }
     if (!p.block_table || !p.status) return fail(MK_ERR_BADARG, "block table / status missing");
     e->static_only = no_handoff;

@@ -290,6 +290,17 @@ def test_hand_off_words_stay_inside_their_buffers(tiny, batch, lib_built):
         assert bool((guarded[name][n:] == 0x5A5A5A5A).all()), name
 
 
+@pytest.mark.parametrize("name", ["attn_part", "partl"])
+def test_misaligned_hand_off_words_are_refused(tiny, name, lib_built):
+    """Pairs of words are read and written at once, so their buffers start on 16 bytes; nothing is launched."""
+    from megakernels_b200 import _lib
+    mk = engine(*tiny, batch=2)
+    lv, _, g = mk._tables
+    gv = _lib.i64_array([g[f] + 8 * (f == name) for f in _lib.GLOBAL_FIELDS])
+    assert mk.lib.mk_set_params(mk._h, _lib.i64_array(lv), len(lv), None, 0, gv, len(gv)) == _lib.MK_ERR_BADARG
+    assert b"16-byte" in mk.lib.mk_last_error()
+
+
 def test_stepped_prompts_behind_a_first_layer_of_attention(lib_built):
     """Steps of a prompt run no LM head, so only the residual separates one step's down-projection sums from the next step's attention
     partials in the same words: many such steps in a row, against the oracle."""
