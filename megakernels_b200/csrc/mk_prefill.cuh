@@ -37,9 +37,14 @@ using mk::warp_sum;
 // while the one before drains, and wait here for its end before they touch memory that any kernel of the chain writes.  Every
 // kernel of the chain calls this first thing (a CTA that left without it would let the next kernel start too early), or behind a
 // prologue that reads nothing but the packed weights.  (512 tokens of the 0.8B model, 231 launches: 5.79 ms without the attribute, 5.28 with it.)
+//   The next kernel's CTAs come up once every CTA has called chain_release or left.  A kernel that needs tensor memory calls it only
+// when it owns it: the next one may allocate before it waits (rows_gemm of dense products does), an allocation waits without a
+// limit, and columns that it took ahead of a CTA still to allocate would never come free.
+__device__ __forceinline__ void chain_acquire() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    chain_acquire();
+    chain_release();
 }
 
 constexpr int ERR_TIMEOUT = -2;
@@ -358,7 +363,7 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ?
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int group = 0, row0, rows, block, z = 0;
     if (A.items) {
-        chain_wait();
+        chain_acquire();
         if ((int)blockIdx.y >= __ldcg(A.n_items)) return;
         const int4 it = __ldcg(A.items + blockIdx.y);
         group = it.x;
@@ -400,7 +405,8 @@ static __global__ void __launch_bounds__((8 * CG + 2) * 32, CG == 1 && DG == 0 ?
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = B.tmem;
-    if (!A.items && (FMT == W_SLAB || warp >= CW)) chain_wait();
+    if (A.items) chain_release();
+    else if (FMT == W_SLAB || warp >= CW) chain_wait();
 
     if (warp == CW) {
         if (lane == 0) {

@@ -115,3 +115,27 @@ def test_malformed_programs_and_sizes_are_errors(lib_built):
     assert _answer(stages) == _lib.MK_ERR_BADARG
     a = D.PrefillArgs(program=ctypes.addressof((D.StageDesc * 1)(prog["embed"])), n_stages=1, batch=2, positions=40000, tokens=16, pos=16, status=16, workspace=1024)
     assert D.lib().mk_stage_prefill(ctypes.byref(a), None) == _lib.MK_ERR_BADARG
+
+
+def test_prompt_kernels_own_tensor_memory_before_the_next_one_starts():
+    """Read in the source: every kernel of the chain waits for the one before, and one that allocates tensor memory lets the next kernel's CTAs
+    come up only behind the barrier that follows the allocation.  (What breaks the rule would hang a GPU, so no run can show it.)"""
+    import os
+    import re
+    csrc = os.path.join(os.path.dirname(_lib.__file__), "csrc")
+    text = open(os.path.join(csrc, "mk_prefill.cuh")).read() + open(os.path.join(csrc, "mk_prefill_08b.cu")).read()
+    heads = [m.start() for m in re.finditer(r"__global__ void", text)]
+    allocating = 0
+    for at, end in zip(heads, heads[1:] + [len(text)]):
+        body = text[at: re.compile(r"^}", re.M).search(text, at).end()]
+        name = re.search(r"(\w+)\(", body[body.index(")") if "__launch_bounds__" in body.split("\n")[0] else 0:]).group(1)
+        if name.startswith("slabs_from"):                    # lays the weights out once, not a kernel of a pass
+            continue
+        assert re.search(r"chain_(wait|acquire)\(\)", body), name
+        alloc = body.find("tcgen05.alloc")
+        if alloc < 0:
+            continue
+        allocating += 1
+        owned = body.index("__syncthreads()", alloc)
+        assert all(m.start() > owned for m in re.finditer(r"chain_(wait|release)\(\)", body)), name
+    assert allocating == 1
