@@ -191,7 +191,7 @@ extern "C" int mk_set_params(mk_engine* e, const int64_t* layers, int64_t n_laye
     if (!no_handoff) {
         if (bad16(p.xl) || bad16(p.projl) || bad16(p.mixl) || bad16(p.lml) || bad16(p.partl))
             return fail(MK_ERR_BADARG, "activation word buffers null or not 16-byte aligned (all of them, or none for a static-only engine)");
-        // the MLP activation words are a hand-off of the batched kernel only: mk_launch_batch refuses an engine without them
+        // (mk_launch_batch refuses an engine without the MLP activation words, though no kernel uses them any more)
         if (p.actl != nullptr && bad16(p.actl)) return fail(MK_ERR_BADARG, "MLP activation words not 16-byte aligned");
         if (bad16(p.attn_part)) return fail(MK_ERR_BADARG, "attention scratch null or not 16-byte aligned");
     }

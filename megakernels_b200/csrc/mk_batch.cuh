@@ -8,9 +8,12 @@
 //     two unsigned); byte d of sequence j is plane d * 8 + j, so digit d of all sequences is one
 //     s8 x s8 (top) or s8 x u8 (lower) MMA.  Integer MMAs are exact; the digits recombine in fp32.
 //   * Every warp owns a contiguous k-slice of the rows and stages exactly the inputs of that slice,
-//     with its own power-of-two scale per pair of sequences (undone on its partial sums), so nothing
+//     with its own power-of-two scale (of all sequences behind a norm, of each pair in front of the out-projection, of each
+//     sequence in front of the down-projection), undone on its partial sums, so nothing
 //     block-wide sits between the arrival of the inputs and the MMAs.  The 1 / rms factor of an
 //     RMSNorm is applied to the finished rows from per-warp sums of squares.
+//   * The down-projection is split over K: a CTA multiplies its own SwiGLU outputs with its column slice
+//     (partial_cols_b), and the owner of a residual row adds the CTAs' sums.
 //   * Every CTA stages all inputs of all sequences, so whatever can be done once is done by the op
 //     that produces a value: the mixers publish gated outputs (DeltaNet: per-head RMSNorm times
 //     silu(z); attention: times the sigmoid gate), and the out-projection only quantises them.
@@ -50,7 +53,7 @@ struct BatchArgs {
 struct GeoB {
     static constexpr int NS = 3;                                   // ring stages: the input planes take the rest
     static constexpr int RING = NS * SLOT_BYTES;
-    static constexpr int XQ = 3 * NB * 3584;                       // 24 byte planes of K = 3584 at most
+    static constexpr int XQ = 3 * NB * 3584;                       // 24 byte planes of K = 2048 take 48 KB of it, the mixer's scratch 68 KB
     static constexpr int PL = 68;                                  // row stride of a (warp, sequence) partial-sum line: 64 rows, padded against bank conflicts
     static constexpr int PS = 36;                                  // same for the 32-row lines of the streaming GEMV
     static constexpr int PART = 2 * NCW * NB * PS * 4;             // >= NCW * NB * PL * 4

@@ -55,7 +55,7 @@ struct LayerP {
     const uint8_t* w_in;
     const uint8_t* w_out;
     const uint8_t* w_gu;
-    const uint8_t* w_down;        // single-sequence kernels: column slices per CTA in fragment order (pack_down_cols)
+    const uint8_t* w_down;        // column slices per CTA in fragment order (pack_down_cols)
     const uint8_t* w_down_rows;   // row slices per CTA (pack_rows): source of the prompt path's operand; batched launches ask for it
     const uint8_t* w_out_rows;    // batched kernel, DeltaNet layers: row slices (single-sequence kernels: w_out holds column slices per task)
     const float* s_in;
@@ -106,7 +106,7 @@ struct Params {
     const float* draft_scale;
     const int* draft_ids;
     unsigned long long* xml;
-    unsigned long long* partl;    // [token][cta][hidden] partial down-projection sums
+    unsigned long long* partl;    // [token][cta][hidden] partial projection sums (batched launches: a batch of one only)
     int n_layers, vocab, max_seq, draft_vocab;
 };
 

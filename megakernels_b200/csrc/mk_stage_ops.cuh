@@ -607,8 +607,8 @@ __device__ __noinline__ void attn_stage(Shared& S, const mk_stage_desc& d) {
 //     (3.3e-7 with one chain per operand half and the third piece in rows 0-7; fp32 FMAs: 1.6e-7), growing with the tiles per
 //     warp: 4.2e-7 at 800 positions and 512 dims; fresh accumulators per tile would end that for 1 % of a step;
 //   * K goes by 128 dims: with 256 a lane asked for sixteen 16-byte pieces at once, and at 96 registers a thread the outputs'
-//     accumulators went to local memory and back around them (652 instead of 404 bytes of spill stores, four sequences at
-//     8000 positions and 256 dims 65 instead of 72 us);
+//     accumulators went to local memory and back around them (612 bytes of spill stores, 404 by 128; eight sequences at 8192
+//     positions, mean of five sliding layers and a full one, 72 us, 65 by 128);
 //   * 256 positions at a time with a running maximum; one CTA barrier per 256.
 constexpr int ATTN_SUB = 256;             // positions between two barriers: one tile per warp
 // Buffers of cache-row offsets.  Sub-chunk s + 1's are written between the barriers of s - 1 and s, when a slower warp still
